@@ -71,6 +71,22 @@ class Af3kError(RuntimeError):
 
 
 _lib: Optional[ctypes.CDLL] = None
+_host_module = None
+
+
+def host():
+    """The native host path (``_host.so``), bound to the library ``load()`` loads."""
+    global _host_module
+    if _host_module is None:
+        load()
+        try:
+            from . import _host
+        except ImportError as exc:
+            raise ImportError(f"the native host path cannot be imported ({exc}): build it with "
+                              "`python -m af3_kernels_b200.build`.  There is no fallback.") from exc
+        _host.bind_library(LIB_PATH)
+        _host_module = _host
+    return _host_module
 
 
 def load() -> ctypes.CDLL:

@@ -1,4 +1,4 @@
-"""Builds ``libaf3k.so`` in-tree with nvcc for sm_100a.
+"""Builds ``libaf3k.so`` (nvcc, sm_100a) and ``_host.so`` (g++, torch headers) in-tree.
 
 Usage: ``python -m af3_kernels_b200.build [--force]``.  nvcc cross-compiles, so this works on a
 host without a GPU; the resulting library needs a compute-capability-10.x device to run.
@@ -36,23 +36,53 @@ def _nvcc() -> str:
     return exe
 
 
-def is_stale() -> bool:
-    if not os.path.exists(LIB_PATH):
+# the host path on at::Tensor: an extension module beside the binding (it looks the library's entry
+# points up at run time, so it does not link against libaf3k.so)
+HOST_SRC = os.path.join(CSRC, "host_torch.cpp")
+HOST_PATH = os.path.join(_HERE, "_host.so")
+
+
+def _older(path, sources) -> bool:
+    if not os.path.exists(path):
         return True
-    t = os.path.getmtime(LIB_PATH)
-    return any(os.path.getmtime(f) > t for f in SOURCES + HEADERS)
+    t = os.path.getmtime(path)
+    return any(os.path.getmtime(f) > t for f in sources)
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    """Compiles the library when it is missing or older than its sources; returns its path."""
-    if not force and not is_stale():
-        return LIB_PATH
-    cmd = [_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", LIB_PATH] + SOURCES
+def is_stale() -> bool:
+    return _older(LIB_PATH, SOURCES + HEADERS) or _older(HOST_PATH, [HOST_SRC, HEADERS[-1]])
+
+
+def _run(cmd, what, verbose):
     res = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or res.returncode != 0:
         sys.stderr.write(res.stdout + res.stderr)
     if res.returncode != 0:
-        raise RuntimeError("nvcc failed building libaf3k.so")
+        raise RuntimeError(f"building {what} failed")
+
+
+def build_host(verbose: bool = False) -> None:
+    import sysconfig
+
+    import torch
+
+    tdir = os.path.dirname(torch.__file__)
+    inc = [os.path.join(tdir, "include"), os.path.join(tdir, "include", "torch", "csrc", "api", "include"),
+           os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include"), sysconfig.get_paths()["include"]]
+    lib = os.path.join(tdir, "lib")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_host",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+    cmd += [f"-I{d}" for d in inc] + [HOST_SRC, "-o", HOST_PATH, f"-L{lib}"]
+    cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-ldl"]
+    _run(cmd, "_host.so", verbose)
+
+
+def build(force: bool = False, verbose: bool = False) -> str:
+    """Compiles what is missing or older than its sources; returns the library's path."""
+    if force or _older(LIB_PATH, SOURCES + HEADERS):
+        _run([_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", LIB_PATH] + SOURCES, "libaf3k.so", verbose)
+    if force or _older(HOST_PATH, [HOST_SRC, HEADERS[-1]]):
+        build_host(verbose)
     return LIB_PATH
 
 

@@ -1,0 +1,414 @@
+// Native host path: what a call of the operator does between Python and the C ABI - argument checks,
+// dtype and layout conversions, output allocation, the cache of staged biases, stream look-up - on
+// at::Tensor, without the interpreter.  A small attention call is bound by its host time: through
+// Python and ctypes it took 37 - 44 us on the host whatever the size (kernel: 5 - 20 us), through this
+// file about 7 us, of which the launch itself is 3.
+//
+// Nothing here computes: every result comes from a kernel of libaf3k.so, whose entry points are looked
+// up in the library the Python binding loaded (bind_library).
+#include <ATen/cuda/CUDAEvent.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/extension.h>
+
+#include <cmath>
+#include <cstring>
+#include <list>
+#include <mutex>
+
+#include "../../include/af3k.h"
+
+namespace {
+
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+// ------------------------------------------------------------------ library and errors
+struct Library {
+  decltype(&af3k_dot_product_attention) attention = nullptr;
+  decltype(&af3k_dot_product_attention_workspace) workspace = nullptr;
+  decltype(&af3k_stage_bias) stage_bias = nullptr;
+};
+Library g_lib;
+
+void bind_library(const std::string& path) {
+  void* h = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+  TORCH_CHECK(h != nullptr, "cannot load ", path, ": ", dlerror());
+  auto find = [&](const char* name) {
+    void* p = dlsym(h, name);
+    TORCH_CHECK(p != nullptr, path, " does not export ", name);
+    return p;
+  };
+  g_lib.attention = reinterpret_cast<decltype(g_lib.attention)>(find("af3k_dot_product_attention"));
+  g_lib.workspace = reinterpret_cast<decltype(g_lib.workspace)>(find("af3k_dot_product_attention_workspace"));
+  g_lib.stage_bias = reinterpret_cast<decltype(g_lib.stage_bias)>(find("af3k_stage_bias"));
+}
+
+// Return codes become the Python binding's Af3kError.
+void check(int code) {
+  if (code == AF3K_OK) return;
+  py::gil_scoped_acquire gil;
+  py::module_::import("af3_kernels_b200._capi").attr("check")(code);
+}
+
+[[noreturn]] void value_error(const std::string& what) { throw py::value_error(what); }
+[[noreturn]] void type_error(const std::string& what) { throw py::type_error(what); }
+
+// Status words {bits, 1 + barrier, block, warp} of a device, shared by all calls on it; kept for the
+// life of the process.
+Tensor status_buffer(int64_t device) {
+  static std::mutex mu;
+  static std::vector<Tensor>* bufs = new std::vector<Tensor>(64);
+  std::lock_guard<std::mutex> lock(mu);
+  Tensor& t = bufs->at(device);
+  if (!t.defined()) t = at::zeros({4}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
+  return t;
+}
+
+// ------------------------------------------------------------------ staged biases
+// A bias the kernel cannot read in place (fp32, rows that are not 16-byte multiples) or, with fp8 q/k,
+// not before it was divided by each head's logit scale, is converted once; the copy is used again
+// while the very same tensor object is alive and unmodified (its version counter) and, for fp8, the
+// scales are the same.  Four copies are kept; copies of dead tensors are dropped when another is made.
+struct TensorId {
+  c10::weak_intrusive_ptr<c10::TensorImpl> impl;
+  int64_t version = -1;
+  explicit TensorId(const Tensor& t) : impl(t.getIntrusivePtr()), version(t._version()) {}
+  bool is(const Tensor& t) const { return !impl.expired() && impl._unsafe_get_target() == t.unsafeGetTensorImpl() && version == (int64_t)t._version(); }
+};
+
+struct Staged {
+  TensorId bias;
+  std::vector<int64_t> sizes, strides;
+  const void* data;
+  int64_t B2, Sq, Sk;
+  std::optional<TensorId> q_scale, k_scale;
+  float scale;
+  Tensor copy;
+  at::cuda::CUDAEvent made;                 // behind the conversion kernel
+  std::vector<c10::StreamId> ordered;       // streams that are behind it already
+};
+
+std::mutex g_staged_mu;
+std::list<Staged>* g_staged = new std::list<Staged>();
+constexpr size_t kStagedMost = 4;
+
+Tensor make_staged(const Tensor& bias_in, int64_t B2, int64_t Sq, int64_t Sk, int64_t D, const float* q_scale,
+                   const float* k_scale, float scale, cudaStream_t stream) {
+  Tensor bias = bias_in;
+  if (bias.scalar_type() != at::kBFloat16 && bias.scalar_type() != at::kFloat) bias = bias.to(at::kFloat);
+  if (bias.dim() != 3) bias = bias.reshape({B2, Sq, Sk});
+  if ((Sk > 1 && bias.stride(2) != 1) || (B2 > 1 && bias.stride(0) == 0) || (Sq > 1 && bias.stride(1) == 0)) bias = bias.contiguous();
+  af3k_attention_desc d{};
+  d.B1 = 1; d.B2 = B2; d.Sq = Sq; d.Sk = Sk; d.D = (D + 15) / 16 * 16;
+  const int64_t most = std::max(Sq, Sk) * 64;
+  for (int64_t* s : {d.q_stride, d.k_stride, d.v_stride, d.out_stride}) { s[0] = B2 * most; s[1] = most; s[2] = 64; }
+  d.bias_stride[0] = bias.stride(0); d.bias_stride[1] = bias.stride(1);
+  d.qk_dtype = q_scale != nullptr ? AF3K_FP8_E4M3 : AF3K_BF16;
+  d.bias_dtype = bias.scalar_type() == at::kBFloat16 ? AF3K_BF16 : AF3K_F32;
+  d.softmax_scale = scale;
+  Tensor staged = at::empty({B2, Sq, (Sk + 7) / 8 * 8}, bias.options().dtype(at::kBFloat16));
+  check(g_lib.stage_bias(&d, bias.data_ptr(), q_scale, k_scale, staged.data_ptr(), staged.numel() * 2, stream));
+  return staged;
+}
+
+Tensor staged_bias(const Tensor& bias, int64_t B2, int64_t Sq, int64_t Sk, int64_t D, const OptTensor& qs_id,
+                   const OptTensor& ks_id, const float* q_scale, const float* k_scale, float scale) {
+  const auto stream = c10::cuda::getCurrentCUDAStream(bias.device().index());
+  const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+  const bool cacheable = !bias.is_inference() && !(qs_id && (qs_id->is_inference() || ks_id->is_inference()));
+  std::lock_guard<std::mutex> lock(g_staged_mu);
+  if (cacheable) {
+    for (auto it = g_staged->begin(); it != g_staged->end(); ++it) {
+      Staged& e = *it;
+      if (!e.bias.is(bias) || e.B2 != B2 || e.Sq != Sq || e.Sk != Sk || e.data != bias.data_ptr() || bias.sizes() != e.sizes ||
+          bias.strides() != e.strides || e.q_scale.has_value() != qs_id.has_value())
+        continue;
+      if (qs_id && (!e.q_scale->is(*qs_id) || !e.k_scale->is(*ks_id) || e.scale != scale)) continue;
+      if (std::find(e.ordered.begin(), e.ordered.end(), stream.id()) == e.ordered.end()) {
+        if (capturing) break;              // a captured stream cannot wait for work outside the graph: convert inside it
+        e.made.block(stream);
+        c10::cuda::CUDACachingAllocator::recordStream(e.copy.storage().data_ptr(), stream);
+        e.ordered.push_back(stream.id());
+      }
+      if (it != g_staged->begin()) g_staged->splice(g_staged->begin(), *g_staged, it);
+      return e.copy;
+    }
+  }
+  Tensor copy = make_staged(bias, B2, Sq, Sk, D, q_scale, k_scale, scale, stream);
+  if (!cacheable || capturing) return copy;     // a copy made inside a graph exists only while the graph replays
+  g_staged->remove_if([&](const Staged& e) { return e.bias.impl.expired() || e.bias.impl._unsafe_get_target() == bias.unsafeGetTensorImpl(); });
+  while (g_staged->size() >= kStagedMost) g_staged->pop_back();
+  Staged e{TensorId(bias), bias.sizes().vec(), bias.strides().vec(), bias.data_ptr(), B2, Sq, Sk, std::nullopt, std::nullopt, scale, copy,
+           at::cuda::CUDAEvent(), {stream.id()}};
+  if (qs_id) { e.q_scale.emplace(*qs_id); e.k_scale.emplace(*ks_id); }
+  e.made.record(stream);
+  g_staged->push_front(std::move(e));
+  return copy;
+}
+
+// ------------------------------------------------------------------ the operator
+// unit innermost stride; a broadcast (zero-stride) view cannot be described to TMA
+Tensor inner_contiguous(const Tensor& t) {
+  bool bad = t.size(3) != 1 && t.stride(3) != 1;
+  for (int i = 0; i < 3; ++i) bad = bad || (t.stride(i) == 0 && t.size(i) > 1);
+  return bad ? t.contiguous() : t;
+}
+
+std::string shape_text(const Tensor& t) {
+  std::ostringstream s;
+  s << t.sizes();
+  return s.str();
+}
+
+// bias_form: 0 an ordinary bias tensor, 1 the copy of a StagedBias, 2 the same divided by fp8 scales
+Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor bias, const OptTensor& q_scale_in,
+                 const OptTensor& k_scale_in, std::optional<double> softmax_scale, int64_t rows_per_item, const OptTensor& out_in,
+                 bool use_workspace, bool cache_bias, int64_t max_ctas, int64_t bias_form, int* status = nullptr) {
+  if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4) value_error("q, k, v must be 4-D [B1, B2, S, D]");
+  if (!q.is_cuda()) throw std::runtime_error("af3_kernels_b200 runs on CUDA tensors only (no CPU fallback)");
+  const auto dev = q.device();
+  if (k.device() != dev || v.device() != dev || bias.device() != dev) value_error("q, k, v, bias must live on the same device");
+  const int64_t B1 = q.size(0), B2 = q.size(1), Sq = q.size(2), D = q.size(3), Sk = k.size(2);
+  for (const Tensor* t : {&k, &v})
+    if (t->size(0) != B1 || t->size(1) != B2 || t->size(2) != Sk || t->size(3) != D) value_error("k and v must be [B1, B2, Sk, D] matching q");
+  const c10::cuda::CUDAGuard guard(dev);
+  const bool fp8 = q.scalar_type() == at::kFloat8_e4m3fn;
+  bool f32_result = false;
+  Tensor q_scale, k_scale;
+  if (fp8) {
+    if (k.scalar_type() != at::kFloat8_e4m3fn || !q_scale_in || !k_scale_in) type_error("fp8 q needs fp8 k and q_scale / k_scale");
+    q_scale = q_scale_in->to(dev, at::kFloat).contiguous();
+    k_scale = k_scale_in->to(dev, at::kFloat).contiguous();
+    if (q_scale.numel() != B2 || k_scale.numel() != B2) value_error("q_scale / k_scale must have one entry per head");
+  } else {
+    if (q.scalar_type() == at::kFloat) {
+      // the reference has an fp32 instantiation (src/csrc/dot_product_attention.cpp:554-558); here fp32
+      // callers get the bf16 kernel (operands rounded once) and an fp32 result
+      if (out_in) value_error("`out` must be omitted with fp32 q (the result is converted from the kernel's bf16 output)");
+      q = q.to(at::kBFloat16);
+      f32_result = true;
+    }
+    if (q.scalar_type() != at::kBFloat16) type_error(std::string("q must be bfloat16, float32 or float8_e4m3fn, got ") + c10::toString(q.scalar_type()));
+    if ((q_scale_in || k_scale_in) && !f32_result) type_error("q_scale / k_scale are only valid with fp8 q and k");
+    if (k.scalar_type() != at::kBFloat16) k = k.to(at::kBFloat16);
+  }
+  if (v.scalar_type() != at::kBFloat16) v = v.to(at::kBFloat16);
+  const float scale = softmax_scale ? (float)*softmax_scale : (float)(1.0 / std::sqrt((double)D));
+
+  bool prescaled = bias_form == 2;
+  if (bias_form == 0) {
+    if (bias.numel() != B2 * Sq * Sk) {
+      value_error("bias must have B2*Sq*Sk = " + std::to_string(B2 * Sq * Sk) + " elements, got " + std::to_string(bias.numel()));
+    }
+    const bool needs_copy = bias.scalar_type() != at::kBFloat16 || bias.dim() != 3 || bias.stride(2) != 1 ||
+                            (bias.stride(1) * 2) % 16 != 0 || (bias.stride(0) * 2) % 16 != 0 ||
+                            reinterpret_cast<uintptr_t>(bias.data_ptr()) % 16 != 0;
+    if (use_workspace && cache_bias && (needs_copy || fp8) && bias.numel() != 0) {
+      bias = staged_bias(bias, B2, Sq, Sk, D, fp8 ? q_scale_in : std::nullopt, fp8 ? k_scale_in : std::nullopt,
+                         fp8 ? q_scale.data_ptr<float>() : nullptr, fp8 ? k_scale.data_ptr<float>() : nullptr, scale);
+      prescaled = fp8;
+    } else {
+      if (bias.scalar_type() != at::kBFloat16 && bias.scalar_type() != at::kFloat) bias = bias.to(at::kFloat);
+      if (bias.dim() != 3) bias = bias.reshape({B2, Sq, Sk});
+      if ((Sk > 1 && bias.stride(2) != 1) || (B2 > 1 && bias.stride(0) == 0) || (Sq > 1 && bias.stride(1) == 0)) bias = bias.contiguous();
+    }
+  }
+  q = inner_contiguous(q); k = inner_contiguous(k); v = inner_contiguous(v);
+
+  Tensor mask;
+  int64_t mask_stride = 0;
+  if (mask_in) {      // bool, [Sk] or [1 | B1, Sk] (the Python side brings other forms to this one)
+    mask = *mask_in;
+    if (mask.size(-1) != Sk || (mask.dim() == 2 && mask.size(0) != 1 && mask.size(0) != B1) || mask.dim() > 2)
+      value_error("mask of shape " + shape_text(mask) + " does not match B1=" + std::to_string(B1) + ", Sk=" + std::to_string(Sk));
+    mask = mask.contiguous();
+    if (mask.device() != dev) mask = mask.to(dev);
+    mask_stride = mask.dim() == 2 && !(mask.size(0) == 1 && B1 != 1) ? Sk : 0;
+  }
+
+  Tensor out;
+  if (!out_in) {
+    out = at::empty({B1, B2, Sq, D}, at::TensorOptions().dtype(at::kBFloat16).device(dev));
+  } else {
+    out = *out_in;
+    if (out.dim() != 4 || out.size(0) != B1 || out.size(1) != B2 || out.size(2) != Sq || out.size(3) != D ||
+        out.scalar_type() != at::kBFloat16 || out.stride(3) != 1)
+      value_error("out must be a bf16 [B1, B2, Sq, D] tensor with unit inner stride");
+  }
+  if (out.numel() == 0) return f32_result ? out.to(at::kFloat) : out;
+
+  af3k_attention_desc d{};
+  d.B1 = B1; d.B2 = B2; d.Sq = Sq; d.Sk = Sk; d.D = D;
+  for (int i = 0; i < 3; ++i) {
+    d.q_stride[i] = q.stride(i); d.k_stride[i] = k.stride(i); d.v_stride[i] = v.stride(i); d.out_stride[i] = out.stride(i);
+  }
+  d.bias_stride[0] = bias.stride(0); d.bias_stride[1] = bias.stride(1);
+  d.mask_row_stride = mask_stride;
+  d.qk_dtype = fp8 ? AF3K_FP8_E4M3 : AF3K_BF16;
+  d.bias_dtype = bias.scalar_type() == at::kBFloat16 ? AF3K_BF16 : AF3K_F32;
+  d.softmax_scale = scale;
+  d.rows_per_item = (int32_t)rows_per_item;
+  d.bias_prescaled = prescaled ? 1 : 0;
+  d.max_ctas = (int32_t)max_ctas;
+  Tensor ws;
+  if (use_workspace) {
+    const size_t bytes = g_lib.workspace(&d, bias.data_ptr());
+    if (bytes != 0) ws = at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(dev));
+  }
+  check(g_lib.attention(&d, q.data_ptr(), k.data_ptr(), v.data_ptr(), bias.data_ptr(),
+                        mask.defined() ? static_cast<const uint8_t*>(mask.data_ptr()) : nullptr, out.data_ptr(),
+                        fp8 ? q_scale.data_ptr<float>() : nullptr, fp8 ? k_scale.data_ptr<float>() : nullptr,
+                        ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? (size_t)ws.numel() : 0,
+                        status != nullptr ? status : status_buffer(dev.index()).data_ptr<int>(), c10::cuda::getCurrentCUDAStream(dev.index())));
+  return f32_result ? out.to(at::kFloat) : out;
+}
+
+// ------------------------------------------------------------------ the operator on host tensors
+// The batch rows are independent problems, so the call is a pipeline over row blocks on three streams:
+// host-to-device copies of block i + 1, the kernel on block i, the device-to-host copy of block i - 1
+// (the link carries both directions at once).  Bias, mask and scales go over once, first.  What bounds it
+// is the link: at 256 rows of 256 keys 51 MB in at 55 GB/s is 0.93 ms.  Only the last block's kernel and
+// copy back stick out behind the input copies, while every block costs three more copies (4 us each on the
+// copy engine) and about 20 us of host time, so each block takes half of the rows that are left, down to
+// kHostBlockBytes of input; a call that small runs on the caller's stream alone.  (Eight equal blocks
+// at this size: 1.34 ms; 1.40 with the loop in Python.)
+constexpr int64_t kHostBlockBytes = 2 << 20;
+
+#define AF3K_CUDA_CHECK(call)                                                                  \
+  do {                                                                                         \
+    const cudaError_t e_ = (call);                                                             \
+    if (e_ != cudaSuccess) {                                                                   \
+      (void)cudaGetLastError();                                                                \
+      throw std::runtime_error(std::string(#call) + ": " + cudaGetErrorString(e_));            \
+    }                                                                                          \
+  } while (0)
+
+void host_attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor bias, const OptTensor& q_scale,
+                    const OptTensor& k_scale, std::optional<double> softmax_scale, Tensor out, int64_t device, int64_t chunks) {
+  const int64_t B1 = q.size(0), B2 = q.size(1), Sq = q.size(2), D = q.size(3), Sk = k.dim() == 4 ? k.size(2) : 0;
+  for (const Tensor* t : {&k, &v})
+    if (t->dim() != 4 || t->size(0) != B1 || t->size(1) != B2 || t->size(2) != Sk || t->size(3) != D)
+      value_error("k and v must be [B1, B2, Sk, D] matching q");
+  if (bias.numel() != B2 * Sq * Sk)
+    value_error("bias must have B2*Sq*Sk = " + std::to_string(B2 * Sq * Sk) + " elements, got " + std::to_string(bias.numel()));
+  const at::Device dev(at::kCUDA, (c10::DeviceIndex)device);
+  const c10::cuda::CUDAGuard guard(dev);
+  q = q.contiguous(); k = k.contiguous(); v = v.contiguous();
+  const int64_t row_bytes = (int64_t)((q.nbytes() + k.nbytes() + v.nbytes()) / B1);
+  std::vector<int64_t> bounds{0};
+  while ((int64_t)bounds.size() < chunks && (B1 - bounds.back()) * row_bytes >= 2 * kHostBlockBytes && B1 - bounds.back() >= 2)
+    bounds.push_back(bounds.back() + (B1 - bounds.back() + 1) / 2);
+  bounds.push_back(B1);
+  const int64_t blocks = (int64_t)bounds.size() - 1;
+  const auto main = c10::cuda::getCurrentCUDAStream(dev.index());
+  const auto s_in = blocks > 1 ? c10::cuda::getStreamFromPool(false, dev.index()) : main;
+  const auto s_out = blocks > 1 ? c10::cuda::getStreamFromPool(false, dev.index()) : main;
+
+  auto on_device = [&](const Tensor& t) { return at::empty(t.sizes(), t.options().device(dev).pinned_memory(false)); };
+  auto copy = [&](void* dst, const void* src, size_t bytes, cudaMemcpyKind kind, cudaStream_t s) {
+    if (bytes != 0) AF3K_CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, kind, s));
+  };
+  auto send = [&](const Tensor& host) {
+    if (host.is_cuda()) return host.to(dev);
+    Tensor t = on_device(host);
+    copy(t.data_ptr(), host.data_ptr(), host.nbytes(), cudaMemcpyHostToDevice, s_in);
+    return t;
+  };
+  // the call may only return (or throw) once nothing on the device touches the host tensors or the
+  // buffers below any more
+  struct Drain {
+    cudaStream_t s[3];
+    bool done = false;
+    ~Drain() {
+      if (!done)
+        for (cudaStream_t t : s) (void)cudaStreamSynchronize(t);
+    }
+  };
+  // buffers come from the caller's stream: what used their memory before is ordered ahead of that stream
+  Tensor dq = on_device(q), dk = on_device(k), dv = on_device(v), dout = on_device(out);
+  Tensor bias_sent, bias_d, mask_d;
+  // the kernels' status words live in pinned host memory here: only a wait that ran out writes them, and
+  // reading them after the call's own synchronisation costs no copy
+  Tensor status = at::empty({4}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+  int* st = status.data_ptr<int>();
+  std::memset(st, 0, 16);
+  OptTensor qs, ks;
+  const bool fp8 = q.scalar_type() == at::kFloat8_e4m3fn;
+  {
+    Drain drain{{s_in, main, s_out}};
+    std::vector<at::cuda::CUDAEvent> ev(2 * blocks + 2);
+    if (blocks > 1) {
+      ev[2 * blocks].record(main);
+      ev[2 * blocks].block(s_in);
+      ev[2 * blocks].block(s_out);
+    }
+    int64_t form = 0;
+    {
+      const c10::cuda::CUDAStreamGuard on_in(s_in);
+      if (q_scale) qs = send(q_scale->to(at::kFloat).contiguous());
+      if (k_scale) ks = send(k_scale->to(at::kFloat).contiguous());
+      bias_d = send(bias.contiguous());
+      if (mask_in) mask_d = send(mask_in->contiguous());
+    }
+    bias_sent = bias_d;
+    const bool aligned = bias_d.scalar_type() == at::kBFloat16 && Sk % 8 == 0;
+    if (fp8 ? (qs && ks && qs->numel() == B2 && ks->numel() == B2) : !aligned) {
+      // converted on the caller's stream, under the copies of the first block
+      if (blocks > 1) {
+        ev[2 * blocks + 1].record(s_in);
+        ev[2 * blocks + 1].block(main);
+      }
+      const float scale = softmax_scale ? (float)*softmax_scale : (float)(1.0 / std::sqrt((double)D));
+      bias_d = make_staged(bias_d, B2, Sq, Sk, D, fp8 ? qs->data_ptr<float>() : nullptr, fp8 ? ks->data_ptr<float>() : nullptr, scale, main)
+                   .slice(2, 0, Sk);
+      form = fp8 ? 2 : 1;
+    }
+    const bool row_mask = mask_d.defined() && mask_d.dim() == 2 && mask_d.size(0) == B1 && B1 != 1;
+    for (int64_t i = 0; i < blocks; ++i) {
+      const int64_t lo = bounds[i], hi = bounds[i + 1];
+      auto part = [&](const Tensor& t) { return t.slice(0, lo, hi); };
+      for (auto [d, h] : {std::pair<Tensor*, Tensor*>{&dq, &q}, {&dk, &k}, {&dv, &v}}) {
+        const size_t row = h->nbytes() / B1;
+        copy(static_cast<char*>(d->data_ptr()) + lo * row, static_cast<const char*>(h->data_ptr()) + lo * row, (hi - lo) * row,
+             cudaMemcpyHostToDevice, s_in);
+      }
+      if (blocks > 1) {
+        ev[2 * i].record(s_in);
+        ev[2 * i].block(main);
+      }
+      attention(part(dq), part(dk), part(dv), row_mask ? OptTensor(part(mask_d)) : (mask_d.defined() ? OptTensor(mask_d) : std::nullopt),
+                bias_d, qs, ks, softmax_scale, 0, part(dout), true, false, 0, form, st);
+      if (blocks > 1) {
+        ev[2 * i + 1].record(main);
+        ev[2 * i + 1].block(s_out);
+      }
+      const size_t row = out.nbytes() / B1;
+      copy(static_cast<char*>(out.data_ptr()) + lo * row, static_cast<const char*>(dout.data_ptr()) + lo * row, (hi - lo) * row,
+           cudaMemcpyDeviceToHost, s_out);
+    }
+    AF3K_CUDA_CHECK(cudaStreamSynchronize(s_out));     // behind the last kernel and, through it, the last copy in
+    drain.done = true;
+  }
+  if (st[0] != 0) {
+    throw std::runtime_error("af3k kernel reported status " + std::to_string(st[0]) + " (wait timeout: barrier slot " +
+                             std::to_string(st[1] - 1) + ", block " + std::to_string(st[2]) + ", warp " + std::to_string(st[3]) +
+                             "); the output is not valid");
+  }
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_host, m) {
+  m.def("host_attention", &host_attention, py::call_guard<py::gil_scoped_release>());
+  m.def("bind_library", &bind_library);
+  m.def("status_buffer", &status_buffer);
+  m.def("attention", [](const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& mask, const Tensor& bias, const OptTensor& q_scale,
+                        const OptTensor& k_scale, std::optional<double> softmax_scale, int64_t rows_per_item, const OptTensor& out,
+                        bool use_workspace, bool cache_bias, int64_t max_ctas, int64_t bias_form) {
+    return attention(q, k, v, mask, bias, q_scale, k_scale, softmax_scale, rows_per_item, out, use_workspace, cache_bias, max_ctas, bias_form);
+  }, py::call_guard<py::gil_scoped_release>());
+}

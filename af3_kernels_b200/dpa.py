@@ -3,15 +3,15 @@
 Mirrors what the reference does between its Python wrapper and its C++ entry
 (src/af3_kernels/__init__.py:31-52 -> src/csrc/dot_product_attention.cpp:545-559): rank-lifts
 the mask, checks dtypes and shapes, allocates the output, and calls the C ABI of libaf3k.so
-with raw device pointers on the current CUDA stream.  There is no CPU path.
+with raw device pointers on the current CUDA stream.  For CUDA tensors all of that is native code
+(``csrc/host_torch.cpp``); what is left here are the rare forms of the arguments and the pipelined
+call on host tensors.  There is no CPU path.
 """
 from __future__ import annotations
 
-import collections
 import ctypes
 import math
 import os
-import weakref
 from typing import Optional
 
 import torch
@@ -19,16 +19,11 @@ import torch
 from . import _capi
 
 _DEBUG = os.environ.get("AF3K_DEBUG", "0") == "1"
-_status_buffers: dict = {}
 
 
 def _status_buffer(device: torch.device) -> torch.Tensor:
-    key = (device.type, device.index)
-    buf = _status_buffers.get(key)
-    if buf is None:
-        buf = torch.zeros(4, dtype=torch.int32, device=device)
-        _status_buffers[key] = buf
-    return buf
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    return _capi.host().status_buffer(index)
 
 
 def read_status(device: torch.device) -> list:
@@ -85,33 +80,6 @@ def stage_bias(bias: torch.Tensor, B2: int, Sq: int, Sk: int, *, q_scale=None, k
     return StagedBias(staged, B2, Sq, Sk, fp8)
 
 
-# Staged copies of recently used biases, so that a caller that applies one bias tensor in many
-# calls (every pair row block of a grid attention, every step of the diffusion transformer) pays
-# for the conversion once.  An entry is valid while the very same tensor object is alive and
-# unmodified (its version counter) and, for fp8, the same scale tensors and softmax scale are used.
-_STAGED_CACHE_SIZE = 4
-_staged_cache: "collections.OrderedDict" = collections.OrderedDict()
-
-
-def _version(t) -> int:
-    return -1 if t is None else t._version
-
-
-def _cached_stage(bias, B2, Sq, Sk, D, q_scale, k_scale, scale) -> StagedBias:
-    key = id(bias)
-    sig = (_version(bias), tuple(bias.shape), tuple(bias.stride()), bias.dtype, bias.data_ptr(), B2, Sq, Sk,
-           None if q_scale is None else (id(q_scale), q_scale._version, id(k_scale), k_scale._version, scale))
-    hit = _staged_cache.get(key)
-    if hit is not None and hit[0]() is bias and hit[1] == sig:
-        _staged_cache.move_to_end(key)
-        return hit[2]
-    staged = stage_bias(bias, B2, Sq, Sk, q_scale=q_scale, k_scale=k_scale, softmax_scale=scale, head_dim=D)
-    _staged_cache[key] = (weakref.ref(bias), sig, staged, q_scale, k_scale)
-    while len(_staged_cache) > _STAGED_CACHE_SIZE:
-        _staged_cache.popitem(last=False)
-    return staged
-
-
 def _mask_rows(mask: Optional[torch.Tensor], B1: int, Sk: int):
     """-> (uint8 tensor [rows, Sk] with unit inner stride, row stride in bytes) or (None, 0).
 
@@ -166,126 +134,26 @@ def dot_product_attention(
     tensor object keeps being passed (``cache_bias=False`` stages inside every call instead).
     ``max_ctas`` > 0 caps the kernel's grid, leaving the other SMs to a kernel that runs beside it.
     """
-    if q.dim() != 4 or k.dim() != 4 or v.dim() != 4:
-        raise ValueError("q, k, v must be 4-D [B1, B2, S, D]")
-    if not q.is_cuda:
-        raise RuntimeError("af3_kernels_b200 runs on CUDA tensors only (no CPU fallback)")
-    bias_dev = bias.data.device if isinstance(bias, StagedBias) else bias.device
-    if k.device != q.device or v.device != q.device or bias_dev != q.device:
-        raise ValueError("q, k, v, bias must live on the same device")
-    B1, B2, Sq, D = q.shape
-    Sk = k.shape[2]
-    if k.shape != (B1, B2, Sk, D) or v.shape != (B1, B2, Sk, D):
-        raise ValueError("k and v must be [B1, B2, Sk, D] matching q")
-    fp8 = q.dtype == torch.float8_e4m3fn
-    if fp8:
-        if k.dtype != torch.float8_e4m3fn or q_scale is None or k_scale is None:
-            raise TypeError("fp8 q needs fp8 k and q_scale / k_scale")
-        q_scale = q_scale.to(device=q.device, dtype=torch.float32).contiguous()
-        k_scale = k_scale.to(device=q.device, dtype=torch.float32).contiguous()
-        if q_scale.numel() != B2 or k_scale.numel() != B2:
-            raise ValueError("q_scale / k_scale must have one entry per head")
-    else:
-        if q.dtype == torch.float32:
-            # the reference has an fp32 instantiation (src/csrc/dot_product_attention.cpp:554-558);
-            # here fp32 callers get the bf16 kernel (operands rounded once) and an fp32 result
-            if out is not None:
-                raise ValueError("`out` must be omitted with fp32 q (the result is converted from the kernel's bf16 output)")
-            return dot_product_attention(
-                q.to(torch.bfloat16), k, v, mask, bias, softmax_scale=softmax_scale,
-                rows_per_item=rows_per_item, check_status=check_status, use_workspace=use_workspace,
-                max_ctas=max_ctas,
-            ).to(torch.float32)
-        if q.dtype != torch.bfloat16:
-            raise TypeError(f"q must be bfloat16, float32 or float8_e4m3fn, got {q.dtype}")
-        if q_scale is not None or k_scale is not None:
-            raise TypeError("q_scale / k_scale are only valid with fp8 q and k")
-        if k.dtype != torch.bfloat16:
-            k = k.to(torch.bfloat16)
-    if v.dtype != torch.bfloat16:
-        v = v.to(torch.bfloat16)
-    scale = float(softmax_scale) if softmax_scale is not None else 1.0 / math.sqrt(D)
-    prescaled = False
-    if not isinstance(bias, StagedBias):
-        if bias.numel() != B2 * Sq * Sk:
-            raise ValueError(f"bias must have B2*Sq*Sk = {B2 * Sq * Sk} elements, got {bias.numel()}")
-        needs_copy = (bias.dtype != torch.bfloat16 or bias.dim() != 3 or bias.stride(-1) != 1
-                      or (bias.stride(-2) * 2) % 16 != 0 or (bias.stride(0) * 2) % 16 != 0
-                      or bias.data_ptr() % 16 != 0)
-        if use_workspace and cache_bias and (needs_copy or fp8):
-            bias = _cached_stage(bias, B2, Sq, Sk, D, q_scale if fp8 else None, k_scale if fp8 else None, scale)
+    if mask is not None and (mask.dtype is not torch.bool or mask.dim() not in (1, 2)):
+        if q.dim() != 4 or k.dim() != 4:
+            raise ValueError("q, k, v must be 4-D [B1, B2, S, D]")
+        mask = _mask_rows(mask, q.shape[0], k.shape[2])[0].view(torch.bool)
+    form = 0
     if isinstance(bias, StagedBias):
-        if (bias.B2, bias.Sq, bias.Sk) != (B2, Sq, Sk) or bias.prescaled != fp8:
+        fp8 = q.dtype == torch.float8_e4m3fn
+        if q.dim() != 4 or (bias.B2, bias.Sq, bias.Sk) != (q.shape[1], q.shape[2], k.shape[2]) or bias.prescaled != fp8:
             raise ValueError("staged bias was made for another shape or another q/k type")
-        prescaled = bias.prescaled
-        bias = bias.data[:, :, :Sk]
-    else:
-        if bias.dtype not in (torch.bfloat16, torch.float32):
-            bias = bias.to(torch.float32)
-        bias = bias.reshape(B2, Sq, Sk) if bias.dim() != 3 else bias
-        if (Sk > 1 and bias.stride(2) != 1) or (B2 > 1 and bias.stride(0) == 0) or (Sq > 1 and bias.stride(1) == 0):
-            bias = bias.contiguous()
-
-    def _inner_contig(t):
-        # unit innermost stride; a broadcast (zero-stride) view cannot be described to TMA
-        if t.shape[3] != 1 and t.stride(3) != 1:
-            return t.contiguous()
-        if any(t.stride(i) == 0 and t.shape[i] > 1 for i in range(3)):
-            return t.contiguous()
-        return t
-
-    q, k, v = _inner_contig(q), _inner_contig(k), _inner_contig(v)
-    mask_u8, mask_stride = _mask_rows(mask, B1, Sk)
-    if mask_u8 is not None and mask_u8.device != q.device:
-        mask_u8 = mask_u8.to(q.device)
-
-    if out is None:
-        out = torch.empty((B1, B2, Sq, D), dtype=torch.bfloat16, device=q.device)
-    elif out.shape != (B1, B2, Sq, D) or out.dtype != torch.bfloat16 or out.stride(3) != 1:
-        raise ValueError("out must be a bf16 [B1, B2, Sq, D] tensor with unit inner stride")
-    if out.numel() == 0:
-        return out
-
-    desc = _capi.AttentionDesc()
-    desc.B1, desc.B2, desc.Sq, desc.Sk, desc.D = B1, B2, Sq, Sk, D
-    for name, t in (("q_stride", q), ("k_stride", k), ("v_stride", v), ("out_stride", out)):
-        getattr(desc, name)[:] = [t.stride(0), t.stride(1), t.stride(2)]
-    desc.bias_stride[:] = [bias.stride(0), bias.stride(1)]
-    desc.mask_row_stride = mask_stride
-    desc.qk_dtype = _capi.AF3K_FP8_E4M3 if fp8 else _capi.AF3K_BF16
-    desc.bias_dtype = _capi.AF3K_BF16 if bias.dtype == torch.bfloat16 else _capi.AF3K_F32
-    desc.softmax_scale = scale
-    desc.rows_per_item = int(rows_per_item)
-    desc.bias_prescaled = 1 if prescaled else 0
-    desc.max_ctas = int(max_ctas)
-
-    lib = _capi.load()
-    with torch.cuda.device(q.device):
-        ws_bytes = lib.af3k_dot_product_attention_workspace(ctypes.byref(desc), bias.data_ptr())
-        if not use_workspace:
-            ws_bytes = 0
-        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device) if ws_bytes else None
-        status = _status_buffer(q.device)
-        code = lib.af3k_dot_product_attention(
-            ctypes.byref(desc),
-            q.data_ptr(), k.data_ptr(), v.data_ptr(), bias.data_ptr(),
-            mask_u8.data_ptr() if mask_u8 is not None else None,
-            out.data_ptr(),
-            q_scale.data_ptr() if fp8 else None,
-            k_scale.data_ptr() if fp8 else None,
-            ws.data_ptr() if ws is not None else None,
-            ws_bytes,
-            status.data_ptr(),
-            torch.cuda.current_stream().cuda_stream,
-        )
-        _capi.check(code)
-        if check_status if check_status is not None else _DEBUG:
-            st = read_status(q.device)
-            if st[0] != 0:
-                raise RuntimeError(
-                    f"af3k kernel reported status {st[0]} (wait timeout: barrier slot {st[1] - 1}, "
-                    f"block {st[2]}, warp {st[3]})"
-                )
+        form = 2 if bias.prescaled else 1
+        bias = bias.data[:, :, :bias.Sk]
+    out = _capi.host().attention(q, k, v, mask, bias, q_scale, k_scale, softmax_scale, rows_per_item, out,
+                                 use_workspace, cache_bias, max_ctas, form)
+    if check_status if check_status is not None else _DEBUG:
+        st = read_status(q.device)
+        if st[0] != 0:
+            raise RuntimeError(
+                f"af3k kernel reported status {st[0]} (wait timeout: barrier slot {st[1] - 1}, "
+                f"block {st[2]}, warp {st[3]})"
+            )
     return out
 
 
@@ -306,10 +174,11 @@ def dot_product_attention_host(
     """The same operator for HOST tensors (what a caller of the reference, a CPU library, holds):
     q, k, v ``[B1, B2, S, D]`` in host memory, result in host memory.
 
-    The batch rows are independent problems, so the call is a three-stage pipeline over ``chunks``
-    row blocks on three CUDA streams: host-to-device copies of block *i + 1*, the kernel on block
-    *i* and the device-to-host copy of block *i - 1* run at the same time (PCIe is full duplex), so
-    the call costs about the time of the larger transfer instead of the sum of all three.  Bias and
+    The batch rows are independent problems, so the call is a three-stage pipeline over up to
+    ``chunks`` row blocks (fewer when the blocks would get small) on three CUDA streams:
+    host-to-device copies of block *i + 1*, the kernel on block *i* and the device-to-host copy of
+    block *i - 1* run at the same time (PCIe is full duplex), so the call costs about the time of
+    the larger transfer instead of the sum of all three.  Bias and
     mask go over once.  Pinned host tensors (``tensor.pin_memory()``) are what makes the copies
     asynchronous; pageable ones work but serialise.  ``out`` may be a preallocated (pinned) host
     tensor.  The call returns after the result has arrived in host memory.
@@ -330,83 +199,7 @@ def dot_product_attention_host(
         raise ValueError("out must be a contiguous bf16 host tensor [B1, B2, Sq, D]")
     if B1 == 0 or out.numel() == 0:
         return out
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    n_chunks = max(1, min(int(chunks), B1))
-    bounds = [B1 * i // n_chunks for i in range(n_chunks + 1)]
-
-    with torch.cuda.device(dev):
-        main = torch.cuda.current_stream()
-        st = _host_path_state(dev, q, k, v, (B1, B2, Sq, D))
-        s_in, s_out = st["s_in"], st["s_out"]
-        dq, dk, dv, do = st["q"], st["k"], st["v"], st["o"]
-        s_in.wait_stream(main)
-        s_out.wait_stream(main)
-        # Bias, mask and scales go over once, on the copy stream and ahead of the row blocks; an
-        # fp32 bias is rounded to bf16 there too.  (Issued on the compute stream instead, the small
-        # conversion kernel held the first attention kernel back until every row block had landed:
-        # 11.3 ms per call at N = 768 instead of 9.5.)
-        with torch.cuda.stream(s_in):
-            bias_d = bias.to(dev, non_blocking=True)
-            if bias_d.dtype not in (torch.bfloat16,):
-                bias_d = bias_d.to(torch.bfloat16)
-            mask_d = None if mask is None else mask.to(dev, non_blocking=True)
-            qs = None if q_scale is None else q_scale.to(dev, non_blocking=True)
-            ks = None if k_scale is None else k_scale.to(dev, non_blocking=True)
-            for t in (bias_d, mask_d, qs, ks):
-                if t is not None:
-                    t.record_stream(main)
-        per_row_mask = mask_d is not None and mask_d.dim() >= 2 and mask_d.reshape(-1, mask_d.shape[-1]).shape[0] == B1 \
-            and B1 != 1
-        if per_row_mask:
-            mask_d = mask_d.reshape(B1, mask_d.shape[-1])
-        for i in range(n_chunks):
-            lo, hi = bounds[i], bounds[i + 1]
-            if lo == hi:
-                continue
-            with torch.cuda.stream(s_in):
-                dq[lo:hi].copy_(q[lo:hi], non_blocking=True)
-                dk[lo:hi].copy_(k[lo:hi], non_blocking=True)
-                dv[lo:hi].copy_(v[lo:hi], non_blocking=True)
-                landed = torch.cuda.Event()
-                landed.record(s_in)
-            main.wait_event(landed)
-            dot_product_attention(dq[lo:hi], dk[lo:hi], dv[lo:hi],
-                                  mask_d[lo:hi] if per_row_mask else mask_d, bias_d,
-                                  q_scale=qs, k_scale=ks, softmax_scale=softmax_scale, out=do[lo:hi])
-            done = torch.cuda.Event()
-            done.record(main)
-            with torch.cuda.stream(s_out):
-                s_out.wait_event(done)
-                out[lo:hi].copy_(do[lo:hi], non_blocking=True)
-        main.wait_stream(s_out)
-        s_out.synchronize()
-        # the call synchronised anyway: the device status word costs nothing to read here
-        status = read_status(dev)
-        if status[0] != 0:
-            raise RuntimeError(
-                f"af3k kernel reported status {status[0]} (wait timeout: barrier slot {status[1] - 1}, "
-                f"block {status[2]}, warp {status[3]}); the output is not valid")
+    if mask is not None and (mask.dtype is not torch.bool or mask.dim() not in (1, 2)):
+        mask = _mask_rows(mask, B1, k.shape[2])[0].view(torch.bool)
+    _capi.host().host_attention(q, k, v, mask, bias, q_scale, k_scale, softmax_scale, out, dev.index, max(1, int(chunks)))
     return out
-
-
-# Copy streams and device staging buffers of the host-tensor path, kept between calls (per device
-# and problem shape) so that a caller in a loop does not create streams and allocate 4 buffers
-# per call.  Calls on one device are serialised by the synchronisation at the end of each call.
-_host_state: dict = {}
-
-
-def _host_path_state(dev, q, k, v, out_shape):
-    key = (dev.index, tuple(q.shape), q.dtype, tuple(k.shape), k.dtype, tuple(v.shape), v.dtype)
-    st = _host_state.get(key)
-    if st is None:
-        if len(_host_state) >= 2:          # keep at most two shapes' worth of buffers alive
-            _host_state.pop(next(iter(_host_state)))
-        st = {
-            "s_in": torch.cuda.Stream(device=dev), "s_out": torch.cuda.Stream(device=dev),
-            "q": torch.empty(q.shape, dtype=q.dtype, device=dev),
-            "k": torch.empty(k.shape, dtype=k.dtype, device=dev),
-            "v": torch.empty(v.shape, dtype=v.dtype, device=dev),
-            "o": torch.empty(out_shape, dtype=torch.bfloat16, device=dev),
-        }
-        _host_state[key] = st
-    return st

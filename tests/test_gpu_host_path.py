@@ -38,3 +38,17 @@ def test_host_path_rejects_cuda_tensors(cuda_device):
     q = torch.zeros(1, 1, 8, 32, dtype=torch.bfloat16, device=cuda_device)
     with pytest.raises(ValueError):
         A.dot_product_attention_host(q, q, q, None, torch.zeros(1, 8, 8))
+
+
+@pytest.mark.parametrize("B1,chunks", [(40, 8), (41, 3), (40, 1)])
+def test_host_row_blocks_give_the_device_result(cuda_device, B1, chunks):
+    """Enough rows that the call is cut into halving row blocks on three streams (10 MB of q, k, v; blocks
+    of at least 2 MB), with a bias the kernel cannot read in place and one mask row per batch row."""
+    g = torch.Generator().manual_seed(7)
+    B2, S, D = 4, 331, 32
+    q, k, v = (torch.randn(B1, B2, S, D, generator=g).to(torch.bfloat16).pin_memory() for _ in range(3))
+    bias = torch.randn(B2, S, S, generator=g).to(torch.bfloat16)
+    mask = torch.rand(B1, S, generator=g) >= 0.1
+    out = A.dot_product_attention_host(q, k, v, mask, bias, chunks=chunks)
+    ref = A.dot_product_attention_cpp(*(t.to(cuda_device) for t in (q, k, v, mask, bias)))
+    assert torch.equal(out, ref.cpu())
