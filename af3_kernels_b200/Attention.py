@@ -10,8 +10,9 @@ import torch
 import torch.distributed as dist
 import torch.nn as nn
 
-from . import pair_bias
-from .fused_ops import attention_block, grid_block_from_raw_pair, pair_front_ok
+from . import _capi, pair_bias
+from .dpa import bool_mask
+from .fused_ops import attention_block
 from .tools import profile
 
 
@@ -32,13 +33,6 @@ class GridSelfAttentionCpp(nn.Module):
         self.gating_query = nn.Linear(self.c_pair, self.c_pair, bias=False)
         self.output_projection = nn.Linear(self.c_pair, self.c_pair, bias=False)
 
-    # One pass over the raw pair for LayerNorm + pair bias + q/k/v/gate projections (af3k_pair_front).
-    # Off by default: at N = 768 it takes 0.232 ms against 0.073 + 0.140 ms for the two kernels it
-    # replaces - it saves the normalised pair's round trip through HBM, but only two tiles per SM are
-    # being normalised at a time (against five CTAs of the stand-alone producer), and the row walks are
-    # latency-bound.
-    fused_front = False
-
     def _weights(self):
         # [in, out] views of the Linear weights: what the reference hands to its operator
         return (self.q_projection.weight.T, self.k_projection.weight.T, self.v_projection.weight.T,
@@ -56,12 +50,14 @@ class GridSelfAttentionCpp(nn.Module):
 
     @profile("B200 GridSelfAttention")
     def forward(self, pair: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
+        host = _capi.host()
+        if host.grid_fused(pair, self.num_head, self.num_head) and mask is not None:
+            # c_pair 64 or 128, up to four heads: three launches, LayerNorm to output projection
+            lin = (self.q_projection, self.k_projection, self.v_projection, self.gating_query, self.output_projection)
+            return host.grid_module(pair, bool_mask(mask, *pair.shape[:2]),
+                                    [m.weight for m in lin] + [self.act_norm.weight, self.act_norm.bias, self.pair_bias_projection.weight],
+                                    self.act_norm.eps, self.num_head, self.transpose)
         dtype = pair.dtype
-        if self.fused_front and not self.transpose and pair_front_ok(pair, self.num_head, self.num_head):
-            # bf16 pair, c_pair = 128, up to four heads: LayerNorm, pair bias and the four projections
-            # in one pass over the raw pair
-            return grid_block_from_raw_pair(pair, mask, self.act_norm.weight, self.act_norm.bias, self.act_norm.eps,
-                                            self.pair_bias_projection.weight, *self._weights(), self.num_head).to(dtype)
         pair, bias = self._norm_and_bias(pair)
         if self.transpose:
             pair = pair.permute(1, 0, 2)

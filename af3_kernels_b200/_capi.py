@@ -37,6 +37,9 @@ EXPORTED_SYMBOLS = (
     "af3k_pair_bias",
     "af3k_sigmoid_gate",
     "af3k_qkvg_projection",
+    "af3k_grid_front",
+    "af3k_grid_out",
+    "af3k_grid_pack",
 )
 
 

@@ -6,14 +6,15 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <utility>
 
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
 #include "attn_sm100.cuh"
+#include "grid_sm100.cuh"
 #include "pair_bias_sm100.cuh"
-#include "proj_sm100.cuh"
 
 namespace {
 
@@ -104,9 +105,16 @@ int device_info(DeviceInfo** out) {
       return cuda_fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize, pair_bias)", e);
     if ((e = cudaFuncSetAttribute(pair_bias_mma_kernel, attr, kPbmSmemBytes)) != cudaSuccess)
       return cuda_fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize, pair_bias_mma)", e);
-    if ((e = cudaFuncSetAttribute(qkvg_projection_kernel<false>, attr, (int)kProjSmemBytes)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(qkvg_projection_kernel<true>, attr, (int)kProjSmemBytes)) != cudaSuccess)
-      return cuda_fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize, qkvg_projection)", e);
+    const std::pair<const void*, uint32_t> grid_kernels[] = {
+        {(const void*)grid_front_kernel<128, __nv_bfloat16, true>, FrontTile<128>::kSmem}, {(const void*)grid_front_kernel<128, float, true>, FrontTile<128>::kSmem},
+        {(const void*)grid_front_kernel<128, __nv_bfloat16, false>, FrontTile<128>::kSmem}, {(const void*)grid_front_kernel<64, __nv_bfloat16, true>, FrontTile<64>::kSmem},
+        {(const void*)grid_front_kernel<64, float, true>, FrontTile<64>::kSmem}, {(const void*)grid_front_kernel<64, __nv_bfloat16, false>, FrontTile<64>::kSmem},
+        {(const void*)grid_out_kernel<128, __nv_bfloat16>, OutTile<128>::kSmem}, {(const void*)grid_out_kernel<128, float>, OutTile<128>::kSmem},
+        {(const void*)grid_out_kernel<64, __nv_bfloat16>, OutTile<64>::kSmem}, {(const void*)grid_out_kernel<64, float>, OutTile<64>::kSmem},
+    };
+    for (const auto& k : grid_kernels)
+      if ((e = cudaFuncSetAttribute(k.first, attr, (int)k.second)) != cudaSuccess)
+        return cuda_fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize, grid)", e);
     d.attr_set = true;
   }
   *out = &d;
@@ -349,7 +357,7 @@ int static_scratch_address(void** out) {
 
 extern "C" {
 
-int af3k_version(void) { return 1002; }
+int af3k_version(void) { return 1003; }
 
 const char* af3k_strerror(int code) {
   switch (code) {
@@ -648,82 +656,149 @@ int af3k_pair_bias_status(int32_t* out4) {
 }  // extern "C"
 
 namespace {
-// Shared by af3k_qkvg_projection (x already layer-normed) and af3k_pair_front (x is the raw pair:
-// the kernel's LayerNorm warpgroup normalises every tile in shared memory and writes the bias).
-int launch_projection(const void* x, const void* w4, int64_t R, int64_t N, int64_t H, float q_scale, void* q,
-                      void* k, void* v, void* gate, int* status_dev, void* stream_v, bool with_ln,
-                      const float* gamma, const float* beta, const float* bias_w, int64_t Hb, float eps,
-                      void* bias, int64_t bias_pitch) {
-  t_last_launches = 0;
-  if (R < 0 || N < 0 || H < 1 || kProjC % H != 0 || (kProjC / H) % 8 != 0) return AF3K_ERR_BAD_SHAPE;
-  if (R > 0x7fffffff || N > 0x7fffffff || R * N > 0x7fffff00LL * 128) return AF3K_ERR_BAD_SHAPE;
-  if (with_ln && (Hb < 1 || Hb > 4)) return AF3K_ERR_BAD_SHAPE;
-  if (with_ln && (bias_pitch < N || (bias_pitch & 7) != 0)) return AF3K_ERR_BAD_STRIDE;
-  if (R == 0 || N == 0) return AF3K_OK;
-  if (!x || !w4 || !q || !k || !v || !gate) return AF3K_ERR_NULL_POINTER;
-  if (with_ln && (!gamma || !beta || !bias_w || !bias)) return AF3K_ERR_NULL_POINTER;
-  if (!aligned16(x) || !aligned16(w4) || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(gate))
-    return AF3K_ERR_BAD_ALIGNMENT;
-  if (with_ln && (!aligned16(gamma) || !aligned16(beta) || !aligned16(bias_w) || !aligned16(bias)))
-    return AF3K_ERR_BAD_ALIGNMENT;
-  DeviceInfo* dev = nullptr;
-  int rc = device_info(&dev);
-  if (rc != AF3K_OK) return rc;
+int encode_weight_map(CUtensorMap* tm, const void* w, int64_t C, int64_t rows) {
   auto enc = tensor_map_encoder();
   if (!enc) return driver_fail("cuTensorMapEncodeTiled entry point", -1);
-  const long long M = R * N;
-  if (M * kProjC > 0x7fffffffLL) return AF3K_ERR_BAD_SHAPE;    // 32-bit element offsets in the epilogue, 32-bit TMA coordinates
-  CUtensorMap tm_x, tm_w;
-  {
-    cuuint64_t dims[2] = {(cuuint64_t)kProjC, (cuuint64_t)M};
-    cuuint64_t strides[1] = {(cuuint64_t)kProjC * 2};
-    cuuint32_t box[2] = {64, 128};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(&tm_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return driver_fail("cuTensorMapEncodeTiled(x)", (int)r);
-    cuuint64_t wdims[2] = {(cuuint64_t)kProjC, (cuuint64_t)kProjOut};
-    cuuint32_t wbox[2] = {64, 256};
-    r = enc(&tm_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(w4), wdims, strides, wbox, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return driver_fail("cuTensorMapEncodeTiled(w4)", (int)r);
-  }
-  ProjParams p;
-  std::memset(&p, 0, sizeof(p));
-  p.M = M; p.N = (int)N; p.H = (int)H; p.D = kProjC / (int)H; p.q_scale = q_scale;
-  p.q = static_cast<__nv_bfloat16*>(q); p.k = static_cast<__nv_bfloat16*>(k);
-  p.v = static_cast<__nv_bfloat16*>(v); p.g = static_cast<__nv_bfloat16*>(gate);
-  p.status = status_dev;
-  p.wait_limit = wait_limit_cycles();
-  p.gamma = gamma; p.beta = beta; p.bias_w = bias_w; p.bias = static_cast<__nv_bfloat16*>(bias);
-  p.bias_pitch = bias_pitch; p.Hb = (int)Hb; p.R = (int)R; p.eps = eps;
-  const long long n_tiles = (M + 127) / 128;
-  const unsigned grid = (unsigned)(n_tiles < dev->sm_count ? n_tiles : dev->sm_count);
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
-  if (with_ln) qkvg_projection_kernel<true><<<grid, kProjLnThreads, kProjSmemBytes, stream>>>(p, tm_x, tm_w);
-  else         qkvg_projection_kernel<false><<<grid, kProjThreads, kProjSmemBytes, stream>>>(p, tm_x, tm_w);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail("launch qkvg_projection_kernel", e);
-  t_last_launches = 1;
-  return AF3K_OK;
+  cuuint64_t dims[2] = {(cuuint64_t)C, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)C * 2};
+  cuuint32_t box[2] = {64, 64};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(w), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? AF3K_OK : driver_fail("cuTensorMapEncodeTiled(weights)", (int)r);
+}
+
+template <int C>
+void launch_front(const GridParams& p, const CUtensorMap& tm, unsigned grid, bool f32, bool ln, cudaStream_t stream) {
+  constexpr uint32_t smem = FrontTile<C>::kSmem;
+  if (!ln)      grid_front_kernel<C, __nv_bfloat16, false><<<grid, kGridThreads, smem, stream>>>(p, tm);
+  else if (f32) grid_front_kernel<C, float, true><<<grid, kGridThreads, smem, stream>>>(p, tm);
+  else          grid_front_kernel<C, __nv_bfloat16, true><<<grid, kGridThreads, smem, stream>>>(p, tm);
 }
 }  // namespace
 
 extern "C" {
 
+int af3k_grid_front(const void* pair, int32_t pair_dtype, const float* gamma, const float* beta, float eps, const float* bias_w,
+                    int64_t Hb, const void* w4, int64_t R, int64_t N, int64_t C, int64_t H, float q_scale, int32_t transpose,
+                    void* bias, int64_t bias_pitch, void* q, void* k, void* v, void* gate, int* status_dev, void* stream_v) {
+  t_last_launches = 0;
+  const bool ln = gamma != nullptr;
+  if (pair_dtype != AF3K_BF16 && !(pair_dtype == AF3K_F32 && ln)) return AF3K_ERR_BAD_DTYPE;
+  if (C != 64 && C != 128) return AF3K_ERR_BAD_SHAPE;
+  if (R < 0 || N < 0 || H < 1 || C % H != 0 || (C / H) % 8 != 0 || Hb < 0 || Hb > 4 || (Hb > 0 && !ln)) return AF3K_ERR_BAD_SHAPE;
+  if (R > 0x7fffffff || N > 0x7fffffff || R * N * C > 0x7fffffffLL) return AF3K_ERR_BAD_SHAPE;    // 32-bit element offsets
+  if (Hb > 0 && (bias_pitch < N || (bias_pitch & 7) != 0)) return AF3K_ERR_BAD_STRIDE;
+  if (R == 0 || N == 0) return AF3K_OK;
+  if (!pair || !w4 || !q || !k || !v || !gate || (ln && !beta) || (Hb > 0 && (!bias_w || !bias))) return AF3K_ERR_NULL_POINTER;
+  for (const void* ptr : {pair, w4, (const void*)q, (const void*)k, (const void*)v, (const void*)gate})
+    if (!aligned16(ptr)) return AF3K_ERR_BAD_ALIGNMENT;
+  if (Hb > 0 && (!aligned16(bias_w) || !aligned16(bias))) return AF3K_ERR_BAD_ALIGNMENT;
+  DeviceInfo* dev = nullptr;
+  int rc = device_info(&dev);
+  if (rc != AF3K_OK) return rc;
+  CUtensorMap tm;
+  if ((rc = encode_weight_map(&tm, w4, C, 4 * C)) != AF3K_OK) return rc;
+  GridParams p;
+  std::memset(&p, 0, sizeof(p));
+  p.M = R * N; p.R = (int)R; p.N = (int)N; p.H = (int)H; p.D = (int)(C / H); p.transpose = transpose ? 1 : 0;
+  p.q_scale = q_scale; p.pair = pair; p.gamma = gamma; p.beta = beta; p.bias_w = bias_w; p.eps = eps; p.Hb = (int)Hb;
+  p.bias = static_cast<__nv_bfloat16*>(bias); p.bias_pitch = bias_pitch;
+  p.q = static_cast<__nv_bfloat16*>(q); p.k = static_cast<__nv_bfloat16*>(k);
+  p.v = static_cast<__nv_bfloat16*>(v); p.g = static_cast<__nv_bfloat16*>(gate);
+  p.status = status_dev; p.wait_limit = wait_limit_cycles();
+  // Few tiles: several CTAs take a tile, each a part of the output columns (and the weights' rows).  They
+  // repeat the row work, which costs less than the part of the epilogue and of the weights' load it saves.
+  const long long n_tiles = (p.M + 127) / 128;
+  p.split = 1;
+  while (p.split < (C == 128 ? 4 : 2) && n_tiles * p.split * 2 <= dev->sm_count) p.split *= 2;
+  const long long ctas = n_tiles * p.split, most = dev->sm_count / p.split * p.split;
+  const unsigned grid = (unsigned)(ctas < most ? ctas : most);
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
+  if (C == 128) launch_front<128>(p, tm, grid, pair_dtype == AF3K_F32, ln, stream);
+  else          launch_front<64>(p, tm, grid, pair_dtype == AF3K_F32, ln, stream);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail("launch grid_front_kernel", e);
+  t_last_launches = 1;
+  return AF3K_OK;
+}
+
+int af3k_grid_out(const void* weighted, const void* gate, const void* wo, void* out, int32_t out_dtype, int64_t M, int64_t C,
+                  int* status_dev, void* stream_v) {
+  t_last_launches = 0;
+  if (out_dtype != AF3K_BF16 && out_dtype != AF3K_F32) return AF3K_ERR_BAD_DTYPE;
+  if ((C != 64 && C != 128) || M < 0 || M > 0x7fffffff) return AF3K_ERR_BAD_SHAPE;
+  if (M == 0) return AF3K_OK;
+  if (!weighted || !gate || !wo || !out) return AF3K_ERR_NULL_POINTER;
+  if (!aligned16(weighted) || !aligned16(gate) || !aligned16(wo) || !aligned16(out)) return AF3K_ERR_BAD_ALIGNMENT;
+  DeviceInfo* dev = nullptr;
+  int rc = device_info(&dev);
+  if (rc != AF3K_OK) return rc;
+  CUtensorMap tm;
+  if ((rc = encode_weight_map(&tm, wo, C, C)) != AF3K_OK) return rc;
+  GridParams p;
+  std::memset(&p, 0, sizeof(p));
+  p.M = M; p.weighted = static_cast<const __nv_bfloat16*>(weighted); p.gate = static_cast<const __nv_bfloat16*>(gate);
+  p.out = out; p.status = status_dev; p.wait_limit = wait_limit_cycles();
+  const long long n_tiles = (M + 127) / 128;
+  const unsigned grid = (unsigned)(n_tiles < dev->sm_count ? n_tiles : dev->sm_count);
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
+  const bool f32 = out_dtype == AF3K_F32;
+  if (C == 128) {
+    if (f32) grid_out_kernel<128, float><<<grid, kGridThreads, OutTile<128>::kSmem, stream>>>(p, tm);
+    else     grid_out_kernel<128, __nv_bfloat16><<<grid, kGridThreads, OutTile<128>::kSmem, stream>>>(p, tm);
+  } else {
+    if (f32) grid_out_kernel<64, float><<<grid, kGridThreads, OutTile<64>::kSmem, stream>>>(p, tm);
+    else     grid_out_kernel<64, __nv_bfloat16><<<grid, kGridThreads, OutTile<64>::kSmem, stream>>>(p, tm);
+  }
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail("launch grid_out_kernel", e);
+  t_last_launches = 1;
+  return AF3K_OK;
+}
+
+int af3k_grid_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void* gamma, const void* beta, int32_t ln_dtype,
+                   int64_t C, int64_t Hb, void* w4, void* wo, float* vec, void* stream_v) {
+  t_last_launches = 0;
+  if (C < 1 || C > 1024 || Hb < 0 || Hb > 1024 || (Hb > 0 && bias_w == nullptr)) return AF3K_ERR_BAD_SHAPE;
+  if (!w5 || !w4 || !wo || !vec) return AF3K_ERR_NULL_POINTER;
+  PackParams p;
+  std::memset(&p, 0, sizeof(p));
+  auto matrix = [](const af3k_matrix& m) { return PackMatrix{m.data, m.stride_out, m.stride_in, m.dtype == AF3K_F32 ? 1 : 0}; };
+  for (int i = 0; i < 5; ++i) {
+    if (!w5[i].data) return AF3K_ERR_NULL_POINTER;
+    if (w5[i].dtype != AF3K_F32 && w5[i].dtype != AF3K_BF16) return AF3K_ERR_BAD_DTYPE;
+    p.w[i] = matrix(w5[i]);
+  }
+  if (Hb > 0) {
+    if (bias_w->dtype != AF3K_F32 && bias_w->dtype != AF3K_BF16) return AF3K_ERR_BAD_DTYPE;
+    p.bias_w = matrix(*bias_w);
+  }
+  p.gamma = gamma; p.beta = beta; p.gamma_f32 = p.beta_f32 = ln_dtype == AF3K_F32 ? 1 : 0;
+  p.C = (int)C; p.Hb = (int)Hb;
+  p.w4 = static_cast<__nv_bfloat16*>(w4); p.wo = static_cast<__nv_bfloat16*>(wo); p.vec = vec;
+  const int n = (int)(5 * C * C + (2 + Hb) * C);
+  grid_pack_kernel<<<(n + 255) / 256, 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(p);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail("launch grid_pack_kernel", e);
+  t_last_launches = 1;
+  return AF3K_OK;
+}
+
 int af3k_qkvg_projection(const void* x, const void* w4, int64_t R, int64_t N, int64_t H, float q_scale,
                          void* q, void* k, void* v, void* gate, int* status_dev, void* stream_v) {
-  return launch_projection(x, w4, R, N, H, q_scale, q, k, v, gate, status_dev, stream_v, false, nullptr, nullptr,
-                           nullptr, 0, 0.f, nullptr, 0);
+  return af3k_grid_front(x, AF3K_BF16, nullptr, nullptr, 0.f, nullptr, 0, w4, R, N, 128, H, q_scale, 0, nullptr, 0, q, k, v, gate,
+                         status_dev, stream_v);
 }
 
 int af3k_pair_front(const void* pair, const float* gamma, const float* beta, float eps, const float* bias_w,
                     int64_t Hb, const void* w4, int64_t R, int64_t N, int64_t H, float q_scale, void* bias,
                     int64_t bias_pitch, void* q, void* k, void* v, void* gate, int* status_dev, void* stream_v) {
-  return launch_projection(pair, w4, R, N, H, q_scale, q, k, v, gate, status_dev, stream_v, true, gamma, beta,
-                           bias_w, Hb, eps, bias, bias_pitch);
+  if (Hb < 1) return AF3K_ERR_BAD_SHAPE;
+  if (!gamma) return AF3K_ERR_NULL_POINTER;
+  return af3k_grid_front(pair, AF3K_BF16, gamma, beta, eps, bias_w, Hb, w4, R, N, 128, H, q_scale, 0, bias, bias_pitch, q, k, v, gate,
+                         status_dev, stream_v);
 }
 
 int af3k_sigmoid_gate(const void* weighted, const void* gate, void* out, int64_t n, void* stream_v) {

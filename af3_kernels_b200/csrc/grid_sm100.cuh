@@ -1,0 +1,626 @@
+// The two GEMM-shaped passes around the attention core of the grid / triangle attention block, for sm_100a.
+//
+//   grid_front_kernel   x = LayerNorm(pair);  bias = (x Wb^T) permuted to [Hb, R, N];
+//                       [q | k | v | gate] = x [Wq; Wk; Wv; Wg]^T          (or x = pair as it is)
+//   grid_out_kernel     out = (weighted * sigmoid(gate)) Wo^T
+//
+// They stand in for the statements in front of the core in the reference's modules
+// (src/af3_kernels/Attention.py:51-52, :152-153) and for the projection BRGEMMs, the SigmoidFwdTPP + MulTPP
+// pair and the output BRGEMM inside its fused block (src/csrc/dot_product_attention.cpp:285-345, :347-372).
+//
+// Both are the same machine: persistent CTAs over tiles of 128 rows, the weights resident in shared memory,
+//
+//   warps 12-19  row producers: global -> registers -> (LayerNorm and pair bias | gate product) -> bf16 ->
+//                shared memory in the layout of a tcgen05.mma A operand (K-major, 128-byte swizzle,
+//                panels of 64 channels).  A row is spread over C / 8 lanes, 8 channels each, so global
+//                reads are full 16-byte pieces of consecutive lanes, the LayerNorm reductions are four
+//                (C = 64: three) shuffles and its parameters stay in registers.  The next rows are
+//                requested before the current ones are worked on.
+//   warp 0       TMEM allocation, the weights' TMA loads, the MMAs (fp32 accumulators in TMEM)
+//   warps 4-11   epilogue, one TMEM lane quarter x one half of the columns each: TMEM -> registers -> bf16 or
+//                fp32 -> a private XOR-swizzled patch of shared memory -> 16-byte stores in runs of 128 bytes
+//   warps 1-3    unused (they give their registers to the other roles)
+//
+// What bounds them is HBM: per row of a bf16 pair with C = 128 the front reads 256 bytes and writes 1 024
+// (+ 2 Hb), the output pass reads 512 and writes 256.  The normalised pair and the gated product never
+// reach HBM.  One tile of the front is about 7 300 cycles of an SM's share of HBM time, against 2 400 issue
+// slots per scheduler for the LayerNorm + bias and 1 500 for the epilogue.
+#pragma once
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <cstdint>
+
+#include "pair_bias_sm100.cuh"
+#include "ptx_sm100.cuh"
+
+namespace af3k {
+
+constexpr int kGridThreads = 640;
+constexpr int kGridProducerWarps = 8, kGridRowsPerWarp = 16;
+// Registers: launched with 96 per thread (61440, the pool setmaxnreg works in), then 128 x 32 (warps 0-3)
+// + 256 x 104 (epilogue) + 256 x 120 (row producers) = 61440.
+constexpr int kGridRegsMisc = 32, kGridRegsEpi = 104, kGridRegsRows = 120;
+static_assert(128 * kGridRegsMisc + 256 * kGridRegsEpi + 256 * kGridRegsRows <= 96 * kGridThreads,
+              "setmaxnreg totals exceed the launch allocation");
+
+template <int C, int kOutC, int kStagesT>
+struct GridTile {
+  static constexpr int kStages = kStagesT;
+  static constexpr uint32_t kX = 128 * C * 2;              // one A tile: C / 64 panels of 128 rows x 128 bytes
+  static constexpr uint32_t kW = kOutC * C * 2;            // weights: C / 64 panels of kOutC rows x 128 bytes
+  static constexpr uint32_t kPatch = 8 * 32 * 128;         // per epilogue warp: 32 rows x 128 bytes
+  static constexpr uint32_t kBiasPatch = kGridProducerWarps * 4 * kGridRowsPerWarp * 2;
+  static constexpr uint32_t off_x = kW, off_patch = off_x + kStages * kX, off_bias = off_patch + kPatch,
+                            off_bar = off_bias + kBiasPatch;
+  static constexpr uint32_t kSmem = off_bar + 128 + 1024 /*alignment*/;
+};
+template <int C> using FrontTile = GridTile<C, 4 * C, C == 128 ? 2 : 4>;
+template <int C> using OutTile = GridTile<C, C, 4>;
+
+struct GridBar {
+  static constexpr int w_full = 0, x_ready = 1 /*[4]*/, x_empty = 5 /*[4]*/, acc_full = 9 /*[2]*/, acc_empty = 11 /*[2]*/, count = 13;
+};
+
+struct GridParams {
+  long long M;             // rows (= R * N)
+  int R, N;                // the pair is [R, N, C]
+  int H, D;                // heads and head width, H * D == C
+  int transpose;           // 1: q, k, v are those of the pair with its two positions exchanged: [N, H, R, D]
+  int split;               // front: CTAs that share a tile's 4 C output columns (small problems)
+  float q_scale;
+  const void* pair;        // front: input rows
+  const float* gamma;      // front with LayerNorm
+  const float* beta;
+  const float* bias_w;     // [Hb, C]
+  float eps;
+  int Hb;
+  __nv_bfloat16* bias;     // [Hb, R, bias_pitch]
+  long long bias_pitch;
+  __nv_bfloat16 *q, *k, *v, *g;   // front: outputs; g [M, C]
+  const __nv_bfloat16* weighted;  // out: attention result [M, C]
+  const __nv_bfloat16* gate;      // out: gate [M, C]
+  void* out;               // out: [M, C] bf16 or fp32
+  int* status;
+  long long wait_limit;
+};
+
+#define AF3K_GRID_WAIT(idx, parity)                                                              \
+  do {                                                                                           \
+    const bool ok_ = mbar_wait_bounded(bars + 8u * (idx), (parity), p.wait_limit, &abort_flag);   \
+    if (!__all_sync(0xffffffffu, ok_)) {                                                         \
+      grid_timeout(p, &abort_flag, (idx));                                                       \
+      goto done;                                                                                 \
+    }                                                                                            \
+  } while (0)
+
+__device__ __forceinline__ void grid_timeout(const GridParams& p, volatile int* abort_flag, int bar) {
+  *abort_flag = 1;
+  if (p.status != nullptr) {
+    atomicOr(p.status, 1 /* wait timeout */);
+    if (atomicCAS(p.status + 1, 0, 2000 + bar + 1) == 0) {
+      p.status[2] = blockIdx.x;
+      p.status[3] = threadIdx.x >> 5;
+    }
+  }
+}
+
+// eight channels of one row as they sit in memory
+template <typename T> struct Raw8 { uint4 v[sizeof(T) / 2]; };
+template <typename T>
+__device__ __forceinline__ Raw8<T> load_raw8(const T* src, bool live) {
+  Raw8<T> r;
+#pragma unroll
+  for (int i = 0; i < (int)sizeof(T) / 2; ++i)
+    r.v[i] = live ? __ldg(reinterpret_cast<const uint4*>(src) + i) : make_uint4(0u, 0u, 0u, 0u);
+  return r;
+}
+template <typename T>
+__device__ __forceinline__ void unpack_raw8(const Raw8<T>& r, float (&x)[8]) {
+  if constexpr (sizeof(T) == 4) pb_unpack8<T>(r.v[0], r.v[1], x);
+  else                          pb_unpack8<T>(r.v[0], r.v[0], x);
+}
+
+__device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// Position of the 16-byte piece c8 (channels 8 c8 ..) of a row in an A tile.
+__device__ __forceinline__ uint32_t grid_piece(uint32_t tile, int row, int c8) {
+  return tile + (uint32_t)((c8 >> 3) * (128 * 128) + row * 128 + (((c8 & 7) ^ (row & 7)) << 4));
+}
+
+// Barrier set-up, TMEM allocation and weight loads shared by both kernels (all threads; ends with a block barrier).
+template <class Tile, int C, int kOutRows>
+__device__ __forceinline__ uint32_t grid_prologue(uint32_t smem, uint32_t bars, uint32_t* slot, int* abort_flag, uint32_t tmem_cols,
+                                                  const CUtensorMap* tm_w, int w_row0, int w_rows) {
+  const int warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    prefetch_tensormap(tm_w);
+    mbar_init(bars + 8u * GridBar::w_full, 1);
+    for (int i = 0; i < Tile::kStages; ++i) {
+      mbar_init(bars + 8u * (GridBar::x_ready + i), kGridProducerWarps);
+      mbar_init(bars + 8u * (GridBar::x_empty + i), 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bars + 8u * (GridBar::acc_full + i), 1);
+      mbar_init(bars + 8u * (GridBar::acc_empty + i), 4);
+    }
+    fence_barrier_init();
+    // the weights: rows [w_row0, w_row0 + w_rows) of the packed matrix, panel by panel, in boxes of 64 rows
+    mbar_arrive_expect_tx(bars + 8u * GridBar::w_full, (uint32_t)w_rows * C * 2);
+    for (int kb = 0; kb < C / 64; ++kb)
+      for (int r = 0; r < w_rows; r += 64)
+        tma_load_2d(smem + kb * (kOutRows * 128) + r * 128, tm_w, bars + 8u * GridBar::w_full, kb * 64, w_row0 + r);
+  }
+  if (warp == 0) {
+    __syncwarp();
+    tmem_alloc(smem_u32(slot), tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  return *slot;
+}
+
+// Block-wide end of both kernels.
+__device__ __forceinline__ void grid_epilogue_common(volatile int* abort_flag, uint32_t tmem, uint32_t tmem_cols) {
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag != 0) {
+    for (int i = 0; i < 200; ++i) __nanosleep(10000);
+    __syncthreads();
+  }
+  if ((threadIdx.x >> 5) == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem, tmem_cols);
+  }
+}
+
+template <int C, typename T, bool kLn>
+__global__ void __launch_bounds__(kGridThreads, 1)
+grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CUtensorMap tm_w) {
+  using Tile = FrontTile<C>;
+  extern __shared__ uint8_t grid_smem_raw[];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t smem = (smem_u32(grid_smem_raw) + 1023u) & ~1023u;
+  const uint32_t bars = smem + Tile::off_bar;
+  constexpr uint32_t kTmem = 4 * C;
+  // this CTA's share of the columns (all of them unless split): two accumulator halves of `width` columns
+  const int part = blockIdx.x % p.split, first = blockIdx.x / p.split, step = gridDim.x / p.split;
+  const int width = 2 * C / p.split, col_base = part * 2 * width;
+  const long long n_tiles = (p.M + 127) / 128;
+  const uint32_t tmem = grid_prologue<Tile, C, 4 * C>(smem, bars, &tmem_slot, &abort_flag, kTmem, &tm_w, col_base, 2 * width);
+
+  if (warp < 4) {
+    setmaxnreg_dec<kGridRegsMisc>();
+    if (warp == 0) {
+      // ---- MMA issuer
+      const bool leader = elect_one();
+      const uint32_t idesc = make_idesc(1u, 1u, 0u, 0u, (uint32_t)width);
+      const uint64_t ad0 = make_smem_desc(smem + Tile::off_x, 16, 8 * 128, 2), bd0 = make_smem_desc(smem, 16, 8 * 128, 2);
+      const uint32_t ad_lo = (uint32_t)ad0, ad_hi = (uint32_t)(ad0 >> 32), bd_lo = (uint32_t)bd0, bd_hi = (uint32_t)(bd0 >> 32);
+      AF3K_GRID_WAIT(GridBar::w_full, 0);
+      uint32_t n = 0;
+      for (long long tile = first; tile < n_tiles; tile += step, ++n) {
+        const uint32_t st = n % Tile::kStages;
+        AF3K_GRID_WAIT(GridBar::x_ready + st, (n / Tile::kStages) & 1);
+        for (int nh = 0; nh < 2; ++nh) {
+          // the epilogue warps of this half must have read the previous tile's columns
+          if (n >= 1) AF3K_GRID_WAIT(GridBar::acc_empty + nh, (n - 1) & 1);
+          tc_fence_after();
+          if (leader) {
+#pragma unroll
+            for (int ks = 0; ks < C / 16; ++ks) {   // 16 channels = 32 bytes of a 128-byte panel row; panel ks / 4
+              const uint32_t a = ad_lo + ((st * Tile::kX + (ks >> 2) * (128 * 128)) >> 4) + 2 * (ks & 3);
+              const uint32_t b = bd_lo + (((ks >> 2) * (4 * C * 128) + nh * width * 128) >> 4) + 2 * (ks & 3);
+              mma_ss_f16(tmem + nh * width, a, ad_hi, b, bd_hi, idesc, ks > 0 ? 1u : 0u);
+            }
+            tc_commit(bars + 8u * (GridBar::acc_full + nh));
+            if (nh == 1) tc_commit(bars + 8u * (GridBar::x_empty + st));
+          }
+          __syncwarp();
+        }
+      }
+    }
+  } else if (warp < 12) {
+    // ---- epilogue: TMEM lane quarter x column half
+    setmaxnreg_inc<kGridRegsEpi>();
+    const int quarter = warp & 3, half = (warp - 4) >> 2;
+    const uint32_t t_base = tmem + ((uint32_t)(quarter * 32) << 16) + half * width;
+    const uint32_t patch = smem + Tile::off_patch + (uint32_t)(warp - 4) * (32 * 128);
+    const int log2d = 31 - __clz(p.D);
+    const int tokens = p.transpose ? p.R : p.N;
+    uint32_t n = 0;
+    for (long long tile = first; tile < n_tiles; tile += step, ++n) {
+      const long long m0 = tile * 128 + quarter * 32;                 // the warp's first row
+      const int i0 = (int)(m0 / p.N), j0 = (int)(m0 - (long long)i0 * p.N);
+      // Element offsets of the eight rows this lane stores in every 64-column piece (rows (lane >> 3)
+      // + 4 it), worked out once per tile: into [rows, H, tokens, D] at head 0.
+      uint32_t off_qkv[8], row_ok = 0;
+#pragma unroll
+      for (int it = 0; it < 8; ++it) {
+        const int row = it * 4 + (lane >> 3);
+        int i = i0, j = j0 + row;
+        while (j >= p.N) { j -= p.N; ++i; }
+        off_qkv[it] = (uint32_t)(p.transpose ? (long long)j * p.H * p.R + i : (long long)i * p.H * p.N + j) << log2d;
+        if (m0 + row < p.M) row_ok |= 1u << it;
+      }
+      AF3K_GRID_WAIT(GridBar::acc_full + half, n & 1);
+      tc_fence_after();
+#pragma unroll 1
+      for (int c0 = 0; c0 < width; c0 += 64) {
+        const int col0 = col_base + half * width + c0;                // 64 columns of one output tensor
+        const int which = col0 / C, within = col0 % C;                // 0 q, 1 k, 2 v, 3 gate
+        const float mul = which == 0 ? p.q_scale : 1.0f;
+#pragma unroll
+        for (int hc = 0; hc < 2; ++hc) {
+          uint32_t acc[32];
+          tmem_ld_x32(t_base + c0 + 32 * hc, acc);
+          tc_wait_ld();
+          // own row -> shared, piece at position piece ^ (row & 7): conflict-free both ways
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(acc[8 * j + e]) * mul;
+            sts128(patch + lane * 128 + (((4 * hc + j) ^ (lane & 7)) << 4), pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]),
+                   pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+          }
+        }
+        if (c0 + 64 >= width) {
+          // the last columns are in registers: the MMAs of the next tile may overwrite this half
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bars + 8u * (GridBar::acc_empty + half));
+        } else {
+          __syncwarp();
+        }
+        // shared -> global: lane l takes piece l & 7 of rows (l >> 3) + 4 it
+        const int ch = within + 8 * (lane & 7);
+        __nv_bfloat16* dst;
+        if (which == 3) dst = p.g + m0 * C + (lane >> 3) * C + ch;
+        else dst = (which == 0 ? p.q : (which == 1 ? p.k : p.v)) + (((long long)(ch >> log2d) * tokens) << log2d) + (ch & (p.D - 1));
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+          const int row = it * 4 + (lane >> 3);
+          uint4 o;
+          asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
+                       : "r"(patch + row * 128 + (((lane & 7) ^ (row & 7)) << 4)));
+          if ((row_ok >> it) & 1u) *reinterpret_cast<uint4*>(dst + (which == 3 ? (uint32_t)(it * 4 * C) : off_qkv[it])) = o;
+        }
+        __syncwarp();      // the patch is rewritten by the next 64 columns
+      }
+    }
+  } else {
+    // ---- row producers: warp w normalises rows 16 w .. 16 w + 15 of every tile
+    setmaxnreg_inc<kGridRegsRows>();
+    const int w = warp - 12;
+    constexpr int kLanes = C / 8;                       // lanes per row
+    constexpr int kRowsIt = 32 / kLanes;                // rows per step of the warp
+    constexpr int kIts = kGridRowsPerWarp / kRowsIt;    // steps per tile
+    constexpr int kBatch = sizeof(T) == 2 ? 4 : 2;      // steps in flight (and worked on together)
+    static_assert(kIts % kBatch == 0, "whole batches per tile");
+    const int c8 = lane % kLanes, sub = lane / kLanes;  // channels 8 c8 .., row within the step
+    float g[8], b[8];
+    if (kLn) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) { g[e] = p.gamma[8 * c8 + e]; b[e] = p.beta[8 * c8 + e]; }
+    }
+    const T* src = static_cast<const T*>(p.pair) + 8 * c8;
+    const uint32_t bias_patch = smem + Tile::off_bias + w * (4 * kGridRowsPerWarp * 2);
+    const bool with_bias = kLn && p.Hb > 0 && part == 0;
+    Raw8<T> next[kBatch];
+    auto request = [&](long long tile, int it0) {
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) {
+        const long long m = tile * 128 + w * kGridRowsPerWarp + (it0 + u) * kRowsIt + sub;
+        next[u] = load_raw8<T>(src + m * C, m < p.M);
+      }
+    };
+    if (first < n_tiles) request(first, 0);
+    uint32_t n = 0;
+    for (long long tile = first; tile < n_tiles; tile += step, ++n) {
+      const uint32_t st = n % Tile::kStages;
+      const uint32_t x_tile = smem + Tile::off_x + st * Tile::kX;
+      if (n >= (uint32_t)Tile::kStages) AF3K_GRID_WAIT(GridBar::x_empty + st, ((n / Tile::kStages) - 1) & 1);
+#pragma unroll
+      for (int it0 = 0; it0 < kIts; it0 += kBatch) {
+        Raw8<T> cur[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) cur[u] = next[u];
+        if (it0 + kBatch < kIts) request(tile, it0 + kBatch);
+        else if (tile + step < n_tiles) request(tile + step, 0);
+        float y[kBatch][8];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) unpack_raw8<T>(cur[u], y[u]);
+        if (kLn) {
+          // mean, then the (biased) variance of the deviations, over the row's kLanes lanes
+          float s[kBatch];
+#pragma unroll
+          for (int u = 0; u < kBatch; ++u) s[u] = ((y[u][0] + y[u][1]) + (y[u][2] + y[u][3])) + ((y[u][4] + y[u][5]) + (y[u][6] + y[u][7]));
+#pragma unroll
+          for (int o = kLanes / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+#pragma unroll
+          for (int u = 0; u < kBatch; ++u) {
+            const float mean = s[u] * (1.0f / C);
+            float q = 0.f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) { y[u][e] -= mean; q = fmaf(y[u][e], y[u][e], q); }
+            s[u] = q;
+          }
+#pragma unroll
+          for (int o = kLanes / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+#pragma unroll
+          for (int u = 0; u < kBatch; ++u) {
+            const float rstd = rsqrtf(s[u] * (1.0f / C) + p.eps);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) y[u][e] = fmaf(y[u][e] * rstd, g[e], b[e]);
+          }
+        }
+        uint32_t yw[kBatch][4];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) yw[u][e] = pack_bf16x2(y[u][2 * e], y[u][2 * e + 1]);
+          const int row = w * kGridRowsPerWarp + (it0 + u) * kRowsIt + sub;
+          sts128(grid_piece(x_tile, row, c8), yw[u][0], yw[u][1], yw[u][2], yw[u][3]);
+        }
+        if (with_bias) {
+          // the bias projection sees the rounded values; four heads' sums over the row's lanes by
+          // exchanging halves: after two exchanges a lane holds one head's partial sum
+          float acc[4][kBatch];
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            float wt[8];
+            if (h < p.Hb) {
+              const float4 w0 = __ldg(reinterpret_cast<const float4*>(p.bias_w + h * C + 8 * c8));
+              const float4 w1 = __ldg(reinterpret_cast<const float4*>(p.bias_w + h * C + 8 * c8) + 1);
+              wt[0] = w0.x; wt[1] = w0.y; wt[2] = w0.z; wt[3] = w0.w; wt[4] = w1.x; wt[5] = w1.y; wt[6] = w1.z; wt[7] = w1.w;
+            } else {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) wt[e] = 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+              float a = 0.f, c = 0.f;
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                a = fmaf(__uint_as_float(yw[u][e] << 16), wt[2 * e], a);
+                c = fmaf(__uint_as_float(yw[u][e] & 0xffff0000u), wt[2 * e + 1], c);
+              }
+              acc[h][u] = a + c;
+            }
+          }
+          const bool hi1 = (lane & (kLanes / 2)) != 0, hi2 = (lane & (kLanes / 4)) != 0;
+#pragma unroll
+          for (int u = 0; u < kBatch; ++u) {
+            float k0 = hi1 ? acc[2][u] : acc[0][u], k1 = hi1 ? acc[3][u] : acc[1][u];
+            const float s0 = hi1 ? acc[0][u] : acc[2][u], s1 = hi1 ? acc[1][u] : acc[3][u];
+            k0 += __shfl_xor_sync(0xffffffffu, s0, kLanes / 2);
+            k1 += __shfl_xor_sync(0xffffffffu, s1, kLanes / 2);
+            float k = (hi2 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, hi2 ? k0 : k1, kLanes / 4);
+#pragma unroll
+            for (int o = kLanes / 8; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
+            if ((lane & (kLanes / 4 - 1)) == 0) {
+              const int h = (hi1 ? 2 : 0) + (hi2 ? 1 : 0);
+              asm volatile("st.shared.b16 [%0], %1;" ::"r"(bias_patch + (h * kGridRowsPerWarp + (it0 + u) * kRowsIt + sub) * 2),
+                           "h"(__bfloat16_as_ushort(__float2bfloat16_rn(k))) : "memory");
+            }
+          }
+        }
+      }
+      fence_proxy_async_smem();     // the tile was written through the generic proxy; the tensor core reads it
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bars + 8u * (GridBar::x_ready + st));
+      if (with_bias) {
+        // the warp's 16 rows x 4 heads: consecutive lanes are consecutive rows
+        const int r = lane & 15;
+        const long long m = tile * 128 + w * kGridRowsPerWarp + r;
+        if (m < p.M) {
+          const int i = (int)(m / p.N), j = (int)(m - (long long)i * p.N);
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            const int h = (lane >> 4) + 2 * hh;
+            if (h < p.Hb) {
+              unsigned short v;
+              asm volatile("ld.shared.b16 %0, [%1];" : "=h"(v) : "r"(bias_patch + (h * kGridRowsPerWarp + r) * 2));
+              p.bias[((long long)h * p.R + i) * p.bias_pitch + j] = __ushort_as_bfloat16(v);
+            }
+          }
+        }
+        __syncwarp();
+      }
+    }
+  }
+
+done:
+  grid_epilogue_common(&abort_flag, tmem, kTmem);
+}
+
+template <int C, typename TOut>
+__global__ void __launch_bounds__(kGridThreads, 1)
+grid_out_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CUtensorMap tm_w) {
+  using Tile = OutTile<C>;
+  extern __shared__ uint8_t grid_smem_raw[];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t smem = (smem_u32(grid_smem_raw) + 1023u) & ~1023u;
+  const uint32_t bars = smem + Tile::off_bar;
+  constexpr uint32_t kTmem = 2 * C;               // two accumulators, taken in turn
+  const long long n_tiles = (p.M + 127) / 128;
+  const uint32_t tmem = grid_prologue<Tile, C, C>(smem, bars, &tmem_slot, &abort_flag, kTmem, &tm_w, 0, C);
+
+  if (warp < 4) {
+    setmaxnreg_dec<kGridRegsMisc>();
+    if (warp == 0) {
+      const bool leader = elect_one();
+      const uint32_t idesc = make_idesc(1u, 1u, 0u, 0u, (uint32_t)C);
+      const uint64_t ad0 = make_smem_desc(smem + Tile::off_x, 16, 8 * 128, 2), bd0 = make_smem_desc(smem, 16, 8 * 128, 2);
+      const uint32_t ad_lo = (uint32_t)ad0, ad_hi = (uint32_t)(ad0 >> 32), bd_lo = (uint32_t)bd0, bd_hi = (uint32_t)(bd0 >> 32);
+      AF3K_GRID_WAIT(GridBar::w_full, 0);
+      uint32_t n = 0;
+      for (long long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++n) {
+        const uint32_t st = n % Tile::kStages, buf = n & 1;
+        AF3K_GRID_WAIT(GridBar::x_ready + st, (n / Tile::kStages) & 1);
+        if (n >= 2) AF3K_GRID_WAIT(GridBar::acc_empty + buf, ((n >> 1) - 1) & 1);
+        tc_fence_after();
+        if (leader) {
+#pragma unroll
+          for (int ks = 0; ks < C / 16; ++ks) {
+            const uint32_t a = ad_lo + ((st * Tile::kX + (ks >> 2) * (128 * 128)) >> 4) + 2 * (ks & 3);
+            const uint32_t b = bd_lo + (((ks >> 2) * (C * 128)) >> 4) + 2 * (ks & 3);
+            mma_ss_f16(tmem + buf * C, a, ad_hi, b, bd_hi, idesc, ks > 0 ? 1u : 0u);
+          }
+          tc_commit(bars + 8u * (GridBar::acc_full + buf));
+          tc_commit(bars + 8u * (GridBar::x_empty + st));
+        }
+        __syncwarp();
+      }
+    }
+  } else if (warp < 12) {
+    // ---- epilogue: warps 4-7 take the even tiles (accumulator 0), warps 8-11 the odd ones
+    setmaxnreg_inc<kGridRegsEpi>();
+    const int quarter = warp & 3, buf = (warp - 4) >> 2;
+    const uint32_t t_base = tmem + ((uint32_t)(quarter * 32) << 16) + buf * C;
+    const uint32_t patch = smem + Tile::off_patch + (uint32_t)(warp - 4) * (32 * 128);
+    constexpr int kCols = 128 / (int)sizeof(TOut);      // columns per 128-byte piece of a row
+    uint32_t n = (uint32_t)buf;
+    for (long long tile = blockIdx.x + (long long)buf * gridDim.x; tile < n_tiles; tile += 2LL * gridDim.x, n += 2) {
+      const long long m0 = tile * 128 + quarter * 32;
+      AF3K_GRID_WAIT(GridBar::acc_full + buf, (n >> 1) & 1);
+      tc_fence_after();
+#pragma unroll 1
+      for (int c0 = 0; c0 < C; c0 += kCols) {
+#pragma unroll
+        for (int hc = 0; hc < kCols / 32; ++hc) {
+          uint32_t acc[32];
+          tmem_ld_x32(t_base + c0 + 32 * hc, acc);
+          tc_wait_ld();
+          if constexpr (sizeof(TOut) == 2) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              sts128(patch + lane * 128 + (((4 * hc + j) ^ (lane & 7)) << 4),
+                     pack_bf16x2(__uint_as_float(acc[8 * j]), __uint_as_float(acc[8 * j + 1])),
+                     pack_bf16x2(__uint_as_float(acc[8 * j + 2]), __uint_as_float(acc[8 * j + 3])),
+                     pack_bf16x2(__uint_as_float(acc[8 * j + 4]), __uint_as_float(acc[8 * j + 5])),
+                     pack_bf16x2(__uint_as_float(acc[8 * j + 6]), __uint_as_float(acc[8 * j + 7])));
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              sts128(patch + lane * 128 + ((j ^ (lane & 7)) << 4), acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
+          }
+        }
+        if (c0 + kCols >= C) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bars + 8u * (GridBar::acc_empty + buf));
+        } else {
+          __syncwarp();
+        }
+        TOut* dst = static_cast<TOut*>(p.out) + m0 * C + c0 + (lane & 7) * (16 / (int)sizeof(TOut));
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+          const int row = it * 4 + (lane >> 3);
+          uint4 o;
+          asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
+                       : "r"(patch + row * 128 + (((lane & 7) ^ (row & 7)) << 4)));
+          if (m0 + row < p.M) *reinterpret_cast<uint4*>(dst + row * C) = o;
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    // ---- row producers: weighted * sigmoid(gate), sigmoid in fp32, rounded once
+    setmaxnreg_inc<kGridRegsRows>();
+    const int w = warp - 12;
+    constexpr int kLanes = C / 8, kRowsIt = 32 / kLanes, kIts = kGridRowsPerWarp / kRowsIt, kBatch = 4;
+    static_assert(kIts % kBatch == 0, "whole batches per tile");
+    const int c8 = lane % kLanes, sub = lane / kLanes;
+    uint4 na[kBatch], ng[kBatch];
+    auto request = [&](long long tile, int it0) {
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) {
+        const long long m = tile * 128 + w * kGridRowsPerWarp + (it0 + u) * kRowsIt + sub;
+        na[u] = load_raw8<__nv_bfloat16>(p.weighted + m * C + 8 * c8, m < p.M).v[0];
+        ng[u] = load_raw8<__nv_bfloat16>(p.gate + m * C + 8 * c8, m < p.M).v[0];
+      }
+    };
+    if ((long long)blockIdx.x < n_tiles) request(blockIdx.x, 0);
+    uint32_t n = 0;
+    for (long long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++n) {
+      const uint32_t st = n % Tile::kStages;
+      const uint32_t x_tile = smem + Tile::off_x + st * Tile::kX;
+      if (n >= (uint32_t)Tile::kStages) AF3K_GRID_WAIT(GridBar::x_empty + st, ((n / Tile::kStages) - 1) & 1);
+#pragma unroll
+      for (int it0 = 0; it0 < kIts; it0 += kBatch) {
+        uint4 ca[kBatch], cg[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) { ca[u] = na[u]; cg[u] = ng[u]; }
+        if (it0 + kBatch < kIts) request(tile, it0 + kBatch);
+        else if (tile + gridDim.x < n_tiles) request(tile + gridDim.x, 0);
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          const uint32_t aw[4] = {ca[u].x, ca[u].y, ca[u].z, ca[u].w}, gw[4] = {cg[u].x, cg[u].y, cg[u].z, cg[u].w};
+          uint32_t r[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            r[e] = pack_bf16x2(__uint_as_float(aw[e] << 16) * sigmoid_fast(__uint_as_float(gw[e] << 16)),
+                               __uint_as_float(aw[e] & 0xffff0000u) * sigmoid_fast(__uint_as_float(gw[e] & 0xffff0000u)));
+          const int row = w * kGridRowsPerWarp + (it0 + u) * kRowsIt + sub;
+          sts128(grid_piece(x_tile, row, c8), r[0], r[1], r[2], r[3]);
+        }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bars + 8u * (GridBar::x_ready + st));
+    }
+  }
+
+done:
+  grid_epilogue_common(&abort_flag, tmem, kTmem);
+}
+
+// ------------------------------------------------------------------ packed weights
+// One launch that lays a block's parameters out for the two kernels: W4 [4 C, C] = q, k, v, gate rows, Wo [C, C]
+// (rows = output channels, bf16), gamma, beta, bias projection (fp32).  Sources may be bf16 or fp32 and
+// carry any strides (nn.Linear.weight or its transpose).
+struct PackMatrix { const void* src; long long so, si; int f32; };   // element (out, in) at so * out + si * in
+struct PackParams {
+  PackMatrix w[5];         // q, k, v, gate, output projection
+  PackMatrix bias_w;       // [Hb, C]; src == nullptr: absent
+  const void* gamma; const void* beta; int gamma_f32, beta_f32;
+  int C, Hb;
+  __nv_bfloat16* w4; __nv_bfloat16* wo; float* vec;    // vec: gamma [C], beta [C], bias_w [Hb, C]
+};
+__device__ __forceinline__ float pack_at(const void* src, long long i, int f32) {
+  return f32 ? static_cast<const float*>(src)[i] : __bfloat162float(static_cast<const __nv_bfloat16*>(src)[i]);
+}
+__global__ void grid_pack_kernel(const __grid_constant__ PackParams p) {
+  const int C = p.C, n_mat = 5 * C * C, n = n_mat + (2 + p.Hb) * C;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    if (e < n_mat) {
+      const int m = e / (C * C), r = e % (C * C) / C, c = e % C;
+      const __nv_bfloat16 v = __float2bfloat16_rn(pack_at(p.w[m].src, p.w[m].so * r + p.w[m].si * c, p.w[m].f32));
+      if (m < 4) p.w4[(m * C + r) * C + c] = v; else p.wo[r * C + c] = v;
+    } else {
+      const int v = (e - n_mat) / C, c = e % C;
+      if (v == 0) { if (p.gamma) p.vec[c] = pack_at(p.gamma, c, p.gamma_f32); }
+      else if (v == 1) { if (p.beta) p.vec[C + c] = pack_at(p.beta, c, p.beta_f32); }
+      else p.vec[v * C + c] = pack_at(p.bias_w.src, p.bias_w.so * (v - 2) + p.bias_w.si * c, p.bias_w.f32);
+    }
+  }
+}
+
+}  // namespace af3k

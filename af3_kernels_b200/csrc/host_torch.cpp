@@ -31,6 +31,9 @@ struct Library {
   decltype(&af3k_dot_product_attention) attention = nullptr;
   decltype(&af3k_dot_product_attention_workspace) workspace = nullptr;
   decltype(&af3k_stage_bias) stage_bias = nullptr;
+  decltype(&af3k_grid_front) grid_front = nullptr;
+  decltype(&af3k_grid_out) grid_out = nullptr;
+  decltype(&af3k_grid_pack) grid_pack = nullptr;
 };
 Library g_lib;
 
@@ -42,9 +45,14 @@ void bind_library(const std::string& path) {
     TORCH_CHECK(p != nullptr, path, " does not export ", name);
     return p;
   };
-  g_lib.attention = reinterpret_cast<decltype(g_lib.attention)>(find("af3k_dot_product_attention"));
-  g_lib.workspace = reinterpret_cast<decltype(g_lib.workspace)>(find("af3k_dot_product_attention_workspace"));
-  g_lib.stage_bias = reinterpret_cast<decltype(g_lib.stage_bias)>(find("af3k_stage_bias"));
+#define AF3K_BIND(field, name) g_lib.field = reinterpret_cast<decltype(g_lib.field)>(find(#name))
+  AF3K_BIND(attention, af3k_dot_product_attention);
+  AF3K_BIND(workspace, af3k_dot_product_attention_workspace);
+  AF3K_BIND(stage_bias, af3k_stage_bias);
+  AF3K_BIND(grid_front, af3k_grid_front);
+  AF3K_BIND(grid_out, af3k_grid_out);
+  AF3K_BIND(grid_pack, af3k_grid_pack);
+#undef AF3K_BIND
 }
 
 // Return codes become the Python binding's Af3kError.
@@ -267,6 +275,184 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
   return f32_result ? out.to(at::kFloat) : out;
 }
 
+// ------------------------------------------------------------------ packed block weights
+// A block's parameters laid out for its kernels (bf16 matrices with output rows, fp32 vectors): made in one
+// launch, used again while the same storages are alive and unmodified.  Sixteen blocks' worth is kept
+// (C = 128: 164 KB each), the least recently used one goes first, those of dead parameters with the next
+// one made.
+struct ParamId {
+  c10::weak_intrusive_ptr<c10::StorageImpl> storage;
+  int64_t version, offset;
+  std::vector<int64_t> strides;
+  at::ScalarType dtype;
+  explicit ParamId(const Tensor& t)
+      : storage(t.storage().getWeakStorageImpl()), version(t._version()), offset(t.storage_offset()), strides(t.strides().vec()), dtype(t.scalar_type()) {}
+  bool is(const Tensor& t) const {
+    return !storage.expired() && storage._unsafe_get_target() == t.storage().unsafeGetStorageImpl() && version == (int64_t)t._version() &&
+           offset == t.storage_offset() && t.strides() == at::IntArrayRef(strides) && dtype == t.scalar_type();
+  }
+};
+
+struct Packed {
+  std::vector<ParamId> of;
+  Tensor w4, wo, vec;
+  at::cuda::CUDAEvent made;
+  std::vector<c10::StreamId> ordered;
+};
+std::mutex g_packed_mu;
+std::list<Packed>* g_packed = new std::list<Packed>();
+constexpr size_t kPackedMost = 16;
+
+// params: q, k, v, gate, output projection [C, C] as (out, in) matrices, then (all or none) LayerNorm weight and
+// bias [C], bias projection [Hb, C]
+Packed packed_weights(const std::vector<Tensor>& params, int64_t C) {
+  const at::Device dev = params[0].device();
+  const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+  bool cacheable = true;
+  for (const Tensor& t : params) cacheable = cacheable && !t.is_inference();
+  std::lock_guard<std::mutex> lock(g_packed_mu);
+  if (cacheable) {
+    for (auto it = g_packed->begin(); it != g_packed->end(); ++it) {
+      bool same = it->of.size() == params.size();
+      for (size_t i = 0; same && i < params.size(); ++i) same = it->of[i].is(params[i]);
+      if (!same) continue;
+      if (std::find(it->ordered.begin(), it->ordered.end(), stream.id()) == it->ordered.end()) {
+        if (capturing) break;
+        it->made.block(stream);
+        for (const Tensor* t : {&it->w4, &it->wo, &it->vec}) c10::cuda::CUDACachingAllocator::recordStream(t->storage().data_ptr(), stream);
+        it->ordered.push_back(stream.id());
+      }
+      if (it != g_packed->begin()) g_packed->splice(g_packed->begin(), *g_packed, it);
+      Packed r;
+      r.w4 = it->w4; r.wo = it->wo; r.vec = it->vec;
+      return r;
+    }
+  }
+  const bool with_ln = params.size() > 5;
+  const int64_t Hb = with_ln ? params[7].size(0) : 0;
+  std::vector<Tensor> src;
+  for (const Tensor& t : params) {
+    Tensor x = t.detach();
+    if (x.device() != dev || (x.scalar_type() != at::kFloat && x.scalar_type() != at::kBFloat16)) x = x.to(dev, at::kFloat);
+    src.push_back(x);
+  }
+  if (with_ln) {
+    if (src[5].scalar_type() != src[6].scalar_type()) { src[5] = src[5].to(at::kFloat); src[6] = src[6].to(at::kFloat); }
+    src[5] = src[5].contiguous(); src[6] = src[6].contiguous();
+  }
+  auto dtype_of = [](const Tensor& t) { return t.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16; };
+  auto matrix = [&](const Tensor& t) { return af3k_matrix{t.data_ptr(), t.stride(0), t.stride(1), dtype_of(t)}; };
+  af3k_matrix w5[5], bw{};
+  for (int i = 0; i < 5; ++i) w5[i] = matrix(src[i]);
+  if (with_ln) bw = matrix(src[7]);
+  Packed e;
+  const auto options = at::TensorOptions().device(dev);
+  e.w4 = at::empty({4 * C, C}, options.dtype(at::kBFloat16));
+  e.wo = at::empty({C, C}, options.dtype(at::kBFloat16));
+  e.vec = at::empty({(2 + Hb) * C}, options.dtype(at::kFloat));
+  check(g_lib.grid_pack(w5, with_ln ? &bw : nullptr, with_ln ? src[5].data_ptr() : nullptr, with_ln ? src[6].data_ptr() : nullptr,
+                        with_ln ? dtype_of(src[5]) : AF3K_F32, C, Hb, e.w4.data_ptr(), e.wo.data_ptr(), e.vec.data_ptr<float>(), stream));
+  Packed r;
+  r.w4 = e.w4; r.wo = e.wo; r.vec = e.vec;
+  if (!cacheable || capturing) return r;
+  g_packed->remove_if([](const Packed& o) {
+    for (const ParamId& id : o.of) if (id.storage.expired()) return true;
+    return false;
+  });
+  while (g_packed->size() >= kPackedMost) g_packed->pop_back();
+  for (const Tensor& t : params) e.of.emplace_back(t);
+  e.made.record(stream);
+  e.ordered.push_back(stream.id());
+  g_packed->push_front(std::move(e));
+  return r;
+}
+
+// ------------------------------------------------------------------ the grid attention block
+bool grid_fused(const Tensor& pair, int64_t head, int64_t bias_heads) {
+  if (!pair.is_cuda() || pair.dim() != 3 || pair.numel() == 0) return false;
+  const int64_t C = pair.size(2);
+  return (C == 64 || C == 128) && head > 0 && C % head == 0 && (C / head) % 8 == 0 && bias_heads <= 4 &&
+         (pair.scalar_type() == at::kBFloat16 || pair.scalar_type() == at::kFloat);
+}
+
+std::vector<Tensor> matrices(const std::vector<Tensor>& w, int64_t C) {
+  for (const Tensor& t : w)
+    if (t.dim() != 2 || t.size(0) != C || t.size(1) != C) value_error("projection weights must be [C, C]");
+  return w;
+}
+
+// The whole module: raw pair [N, N, C] -> front (LayerNorm, bias, q / k / v / gate) -> attention -> gate and output
+// projection, three launches.  weights: nn.Linear.weight of q, k, v, gate, output; then LayerNorm weight and bias,
+// bias projection.  transpose: attention along the columns of the pair; q, k, v are written, and the result is
+// read back, in the exchanged order, so nothing is permuted in memory.
+Tensor grid_module(Tensor pair, const Tensor& mask_in, const std::vector<Tensor>& params, double eps, int64_t head, bool transpose) {
+  const at::Device dev = pair.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  const int64_t R = pair.size(0), N = pair.size(1), C = pair.size(2), D = C / head, M = R * N;
+  if (R != N) value_error("pair must be [N, N, c_pair]");
+  matrices({params.begin(), params.begin() + 5}, C);
+  if (params[7].dim() != 2 || params[7].size(0) != head || params[7].size(1) != C || params[5].numel() != C || params[6].numel() != C)
+    value_error("LayerNorm and bias projection do not match the pair");
+  pair = pair.contiguous();
+  if (reinterpret_cast<uintptr_t>(pair.data_ptr()) % 16 != 0) pair = pair.clone();
+  Tensor mask = mask_in.device() == dev ? mask_in.contiguous() : mask_in.to(dev).contiguous();
+  if (mask.size(-1) != N || (mask.dim() == 2 && mask.size(0) != 1 && mask.size(0) != N))
+    value_error("mask of shape " + shape_text(mask) + " does not match B1=" + std::to_string(N) + ", Sk=" + std::to_string(N));
+  const Packed w = packed_weights(params, C);
+  const float* vec = w.vec.data_ptr<float>();
+  const auto bf16 = pair.options().dtype(at::kBFloat16);
+  const int64_t pitch = (N + 7) / 8 * 8;
+  Tensor bias = at::empty({head, N, pitch}, bf16);
+  Tensor buf = at::empty({5, M, C}, bf16);           // q, k, v, gate, attention result
+  Tensor out = at::empty({R, N, C}, pair.options());
+  char* b = static_cast<char*>(buf.data_ptr());
+  const size_t part = (size_t)M * C * 2;
+  void *q = b, *k = b + part, *v = b + 2 * part, *gate = b + 3 * part, *weighted = b + 4 * part;
+  const bool f32 = pair.scalar_type() == at::kFloat;
+  int* status = status_buffer(dev.index()).data_ptr<int>();
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  check(g_lib.grid_front(pair.data_ptr(), f32 ? AF3K_F32 : AF3K_BF16, vec, vec + C, (float)eps, vec + 2 * C, head, w.w4.data_ptr(), R, N,
+                         C, head, 1.0f / std::sqrt((float)D), transpose, bias.data_ptr(), pitch, q, k, v, gate, status, stream));
+  af3k_attention_desc d{};
+  d.B1 = N; d.B2 = head; d.Sq = N; d.Sk = N; d.D = D;
+  for (int64_t* st : {d.q_stride, d.k_stride, d.v_stride}) { st[0] = head * N * D; st[1] = N * D; st[2] = D; }
+  d.out_stride[0] = transpose ? C : N * C; d.out_stride[1] = D; d.out_stride[2] = transpose ? N * C : C;
+  d.bias_stride[0] = N * pitch; d.bias_stride[1] = pitch;
+  d.mask_row_stride = mask.dim() == 2 && mask.size(0) == N ? N : 0;
+  d.qk_dtype = AF3K_BF16; d.bias_dtype = AF3K_BF16;
+  d.softmax_scale = 1.0f;                            // q left the projection scaled
+  check(g_lib.attention(&d, q, k, v, bias.data_ptr(), static_cast<const uint8_t*>(mask.data_ptr()), weighted, nullptr, nullptr, nullptr, 0,
+                        status, stream));
+  check(g_lib.grid_out(weighted, gate, w.wo.data_ptr(), out.data_ptr(), f32 ? AF3K_F32 : AF3K_BF16, M, C, status, stream));
+  return out;
+}
+
+// The block on an already normalised pair [R, N, C] with a bias of the caller's.  weights: q, k, v, gate, output as
+// [out, in].
+Tensor grid_block(const Tensor& pair, const OptTensor& mask, const Tensor& bias, const std::vector<Tensor>& weights, int64_t head) {
+  const at::Device dev = pair.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  const int64_t R = pair.size(0), N = pair.size(1), C = pair.size(2), D = C / head, M = R * N;
+  matrices(weights, C);
+  Tensor x = pair.to(at::kBFloat16).contiguous();
+  if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0) x = x.clone();
+  const Packed w = packed_weights(weights, C);
+  Tensor buf = at::empty({5, M, C}, x.options());
+  auto at_part = [&](int i, at::IntArrayRef sizes) { return buf.select(0, i).view(sizes); };
+  Tensor q = at_part(0, {R, head, N, D}), k = at_part(1, {R, head, N, D}), v = at_part(2, {R, head, N, D});
+  Tensor gate = at_part(3, {M, C}), weighted = at_part(4, {R, N, head, D});
+  Tensor out = at::empty({R, N, C}, x.options().dtype(pair.scalar_type()));
+  int* status = status_buffer(dev.index()).data_ptr<int>();
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  check(g_lib.grid_front(x.data_ptr(), AF3K_BF16, nullptr, nullptr, 0.f, nullptr, 0, w.w4.data_ptr(), R, N, C, head, 1.0f / std::sqrt((float)D), 0,
+                         nullptr, 0, q.data_ptr(), k.data_ptr(), v.data_ptr(), gate.data_ptr(), status, stream));
+  attention(q, k, v, mask, bias, std::nullopt, std::nullopt, 1.0, 0, weighted.permute({0, 2, 1, 3}), true, true, 0, 0);
+  check(g_lib.grid_out(weighted.data_ptr(), gate.data_ptr(), w.wo.data_ptr(), out.data_ptr(), pair.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16,
+                       M, C, status, stream));
+  return out;
+}
+
 // ------------------------------------------------------------------ the operator on host tensors
 // The batch rows are independent problems, so the call is a pipeline over row blocks on three streams:
 // host-to-device copies of block i + 1, the kernel on block i, the device-to-host copy of block i - 1
@@ -275,7 +461,9 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
 // copy back stick out behind the input copies, while every block costs three more copies (4 us each on the
 // copy engine) and about 20 us of host time, so each block takes half of the rows that are left, down to
 // kHostBlockBytes of input; a call that small runs on the caller's stream alone.  (Eight equal blocks
-// at this size: 1.34 ms; 1.40 with the loop in Python.)
+// at this size: 1.34 ms, this schedule: 1.20, eight blocks issued from Python: 1.40; 64 rows of 64 keys:
+// 1.05 -> 0.15 ms.  A kernel that stores straight into the pinned result, without the copy back, was
+// slower, 2.1 ms: such stores reach 16 GB/s.)
 constexpr int64_t kHostBlockBytes = 2 << 20;
 
 #define AF3K_CUDA_CHECK(call)                                                                  \
@@ -403,6 +591,9 @@ void host_attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tens
 }  // namespace
 
 PYBIND11_MODULE(_host, m) {
+  m.def("grid_fused", &grid_fused);
+  m.def("grid_module", &grid_module, py::call_guard<py::gil_scoped_release>());
+  m.def("grid_block", &grid_block, py::call_guard<py::gil_scoped_release>());
   m.def("host_attention", &host_attention, py::call_guard<py::gil_scoped_release>());
   m.def("bind_library", &bind_library);
   m.def("status_buffer", &status_buffer);

@@ -555,6 +555,14 @@ __global__ void __launch_bounds__(kPbmRows, 5) pair_bias_mma_kernel(const PairBi
 }
 
 // ---------------------------------------------------------------- sigmoid gate
+// sigmoid(x) = 1 / (1 + 2^(-x log2 e)), by the two approximate instructions (a few fp32 ulps; every use rounds
+// the product to bf16)
+__device__ __forceinline__ float sigmoid_fast(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + ex2_approx(-1.4426950408889634f * x)));
+  return r;
+}
+
 // out = weighted * sigmoid(gate), elementwise over bf16 tensors of n elements (n a multiple of 8,
 // pointers 16-byte aligned).  Stands in for the SigmoidFwdTPP + MulTPP pair behind the core in the
 // reference's fused blocks (src/csrc/dot_product_attention.cpp:339-345 and :522-528).  The
@@ -572,10 +580,7 @@ __global__ void __launch_bounds__(256) sigmoid_gate_kernel(const uint4* __restri
     for (int e = 0; e < 4; ++e) {
       const float a0 = __uint_as_float(aw[e] << 16), a1 = __uint_as_float(aw[e] & 0xffff0000u);
       const float g0 = __uint_as_float(gw[e] << 16), g1 = __uint_as_float(gw[e] & 0xffff0000u);
-      // sigmoid(x) = 1 / (1 + 2^(-x log2 e))
-      const float s0 = __frcp_rn(1.0f + ex2_approx(-1.4426950408889634f * g0));
-      const float s1 = __frcp_rn(1.0f + ex2_approx(-1.4426950408889634f * g1));
-      r[e] = pb_pack_bf16x2(a0 * s0, a1 * s1);
+      r[e] = pb_pack_bf16x2(a0 * sigmoid_fast(g0), a1 * sigmoid_fast(g1));
     }
     out[i] = make_uint4(r[0], r[1], r[2], r[3]);
   }

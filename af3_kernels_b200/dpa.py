@@ -105,6 +105,13 @@ def _mask_rows(mask: Optional[torch.Tensor], B1: int, Sk: int):
     return mask, stride
 
 
+def bool_mask(mask: Optional[torch.Tensor], B1: int, Sk: int) -> Optional[torch.Tensor]:
+    """The mask as the native path takes it: None, or bool ``[Sk]`` or ``[1 | B1, Sk]``."""
+    if mask is None or (mask.dtype is torch.bool and mask.dim() in (1, 2)):
+        return mask
+    return _mask_rows(mask, B1, Sk)[0].view(torch.bool)
+
+
 def dot_product_attention(
     q: torch.Tensor,
     k: torch.Tensor,
@@ -134,10 +141,8 @@ def dot_product_attention(
     tensor object keeps being passed (``cache_bias=False`` stages inside every call instead).
     ``max_ctas`` > 0 caps the kernel's grid, leaving the other SMs to a kernel that runs beside it.
     """
-    if mask is not None and (mask.dtype is not torch.bool or mask.dim() not in (1, 2)):
-        if q.dim() != 4 or k.dim() != 4:
-            raise ValueError("q, k, v must be 4-D [B1, B2, S, D]")
-        mask = _mask_rows(mask, q.shape[0], k.shape[2])[0].view(torch.bool)
+    if mask is not None and q.dim() == 4 and k.dim() == 4:
+        mask = bool_mask(mask, q.shape[0], k.shape[2])
     form = 0
     if isinstance(bias, StagedBias):
         fp8 = q.dtype == torch.float8_e4m3fn
@@ -199,7 +204,6 @@ def dot_product_attention_host(
         raise ValueError("out must be a contiguous bf16 host tensor [B1, B2, Sq, D]")
     if B1 == 0 or out.numel() == 0:
         return out
-    if mask is not None and (mask.dtype is not torch.bool or mask.dim() not in (1, 2)):
-        mask = _mask_rows(mask, B1, k.shape[2])[0].view(torch.bool)
+    mask = bool_mask(mask, B1, k.shape[2])
     _capi.host().host_attention(q, k, v, mask, bias, q_scale, k_scale, softmax_scale, out, dev.index, max(1, int(chunks)))
     return out

@@ -232,6 +232,42 @@ int af3k_pair_front(const void* pair, const float* gamma, const float* beta, flo
                     int64_t Hb, const void* w4, int64_t R, int64_t N, int64_t H, float q_scale, void* bias,
                     int64_t bias_pitch, void* q, void* k, void* v, void* gate, int* status_dev, void* stream);
 
+/* The front of the grid / triangle attention block for pairs of 64 or 128 channels, bf16 or fp32, in one
+ * pass over the pair: af3k_pair_front (gamma non-NULL) or af3k_qkvg_projection (gamma, beta NULL, Hb 0: x
+ * is taken as it is, bf16 only) with these additions:
+ *   pair_dtype AF3K_BF16 or AF3K_F32;  C 64 or 128;  Hb 0..4 (0: no bias is computed)
+ *   transpose non-zero: q, k and v are those of the pair with its two positions exchanged, [N, H, R, C / H]
+ *     (what the reference's module does with pair.permute(1, 0, 2), src/af3_kernels/Attention.py:57-58);
+ *     the bias and the gate stay in the order of the pair
+ * Everything else as there. */
+int af3k_grid_front(const void* pair, int32_t pair_dtype, const float* gamma, const float* beta, float eps,
+                    const float* bias_w, int64_t Hb, const void* w4, int64_t R, int64_t N, int64_t C, int64_t H,
+                    float q_scale, int32_t transpose, void* bias, int64_t bias_pitch, void* q, void* k, void* v,
+                    void* gate, int* status_dev, void* stream);
+
+/* The end of the block in one pass:  out = (weighted * sigmoid(gate)) Wo^T.
+ * Stands in for the SigmoidFwdTPP + MulTPP pair and the output projection BRGEMM of the reference's fused
+ * block (src/csrc/dot_product_attention.cpp:339-372).
+ *   weighted, gate [M, C] bf16 contiguous, C 64 or 128;  wo [C, C] bf16 (out x in);  out [M, C], out_dtype
+ *   AF3K_BF16 or AF3K_F32.  The gated product is rounded to bf16 (the GEMM's operand), as af3k_sigmoid_gate does.
+ * All pointers 16-byte aligned. */
+int af3k_grid_out(const void* weighted, const void* gate, const void* wo, void* out, int32_t out_dtype, int64_t M,
+                  int64_t C, int* status_dev, void* stream);
+
+/* A weight matrix of the block: element (out, in) at data[out * stride_out + in * stride_in], bf16 or fp32. */
+typedef struct af3k_matrix {
+  const void* data;
+  int64_t stride_out, stride_in;
+  int32_t dtype;
+} af3k_matrix;
+
+/* Lays a block's parameters out for af3k_grid_front / af3k_grid_out in one launch: w5 = q, k, v, gate, output
+ * projection -> w4 [4 C, C] and wo [C, C] bf16;  gamma, beta (both of ln_dtype, may be NULL) and bias_w [Hb, C]
+ * (NULL with Hb 0) -> vec: fp32 gamma [C], beta [C], bias_w [Hb, C].  No counterpart in the reference (which
+ * repacks its weights for its CPU GEMM, src/csrc/tools.cpp:151-176). */
+int af3k_grid_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void* gamma, const void* beta,
+                   int32_t ln_dtype, int64_t C, int64_t Hb, void* w4, void* wo, float* vec, void* stream);
+
 /* out = weighted * sigmoid(gate), elementwise over n bf16 elements (n a multiple of 8; all three
  * pointers 16-byte aligned; out may be weighted).  Stands in for the SigmoidFwdTPP + MulTPP pair
  * behind the attention core in the reference's fused blocks

@@ -202,3 +202,41 @@ def test_fused_front_matches_the_two_kernels_it_replaces(cuda_device):
             assert (a.float() - b.float()).abs().mean().item() <= 2.0 ** -10 * s_
         scale = bias_ref.float().abs().max().item()
         assert (bias.float() - bias_ref.float()).abs().max().item() <= 2.0 ** -7 * scale + 1e-3
+
+
+@pytest.mark.parametrize("N,C,H,dtype,transpose", [
+    (1, 128, 4, torch.bfloat16, False), (5, 64, 4, torch.float32, True), (64, 128, 4, torch.bfloat16, True),
+    (100, 64, 2, torch.bfloat16, False), (129, 128, 2, torch.float32, False), (131, 128, 4, torch.float32, True),
+    (192, 64, 4, torch.bfloat16, True), (261, 128, 1, torch.bfloat16, False), (261, 64, 4, torch.float32, True)])
+def test_fused_grid_module_against_oracle(cuda_device, N, C, H, dtype, transpose):
+    """The three-launch module over what its kernels branch on: one row tile and less, tiles that straddle
+    pair rows, tiles shared by four / two CTAs and several tiles per CTA, both widths, both pair types, both
+    orientations, one to four heads of bias (H = 1 with C = 128 has D = 128: the unfused path)."""
+    if C // H > 64:
+        H = 2
+    torch.manual_seed(N + C)
+    m = A.GridSelfAttentionCpp(C, H, transpose)
+    with torch.no_grad():
+        m.act_norm.weight.add_(0.2 * torch.randn(C))
+        m.act_norm.bias.add_(0.1 * torch.randn(C))
+        for lin in (m.q_projection, m.k_projection):
+            lin.weight.mul_(3.0)
+        m.pair_bias_projection.weight.mul_(4.0)
+    m = m.to(dtype).eval()
+    pair = (torch.randn(N, N, C) * 2.0 + 0.5).to(dtype)
+    mask = torch.rand(N, N) >= 0.1
+    mask[:, 0] = True
+    sd = m.state_dict()
+    ref = O.grid_block_fp32(pair, mask, *(sd[k].float() for k in (
+        "act_norm.weight", "act_norm.bias", "pair_bias_projection.weight", "q_projection.weight", "k_projection.weight",
+        "v_projection.weight", "gating_query.weight", "output_projection.weight")), H, transpose)
+    m = m.to(cuda_device)
+    with torch.no_grad():
+        out = m(pair.to(cuda_device), mask.to(cuda_device))
+        # new values in the same parameters are seen (the packed copy follows the version counter)
+        m.output_projection.weight.neg_()
+        flipped = m(pair.to(cuda_device), mask.to(cuda_device))
+    assert out.dtype == dtype and out.shape == (N, N, C)
+    _close(out, ref, (N, C, H, dtype, transpose))
+    assert torch.equal(flipped, -out)
+    assert read_status(cuda_device)[0] == 0
