@@ -60,7 +60,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-constexpr int kStaticSmemReserve = 256;
+constexpr int kStaticSmemReserve = 1024;   // the kernels' few static bytes, padded to the dynamic part's alignment
 
 struct DeviceInfo {
   int sm_count = 0;
@@ -199,7 +199,7 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   p.v_tile_bytes = kTile * p.v_row_bytes;
   p.scale = d.softmax_scale;
 
-  const int budget = dev.max_smem_optin - 1024 /*alignment slack*/ - kStaticSmemReserve;
+  const int budget = dev.max_smem_optin - kStaticSmemReserve;
   p.mask_col = 1;   // set for real in the launch path once the mask pointer is known
   const int fixed = kBiasStages * kBiasTileBytes + (int)kBarrierBlockBytes +
                     (kMaxKvStages + 2) * (int)kMaskPanelBytes /*ones column, mask ring, zero block*/ +
@@ -261,7 +261,7 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   p.off_mcol = off;   off += kMaxKvStages * kMaskPanelBytes;
   p.off_zero = off;   off += kMaskPanelBytes;
   p.off_ident = off;  off += kIdentBytes;
-  size_t smem = off + 1024;
+  size_t smem = off;
   // One CTA per SM is required (each CTA allocates all of TMEM): ask for more than half the SM's
   // shared memory even when the tiles need less.
   if (smem < 120 * 1024) smem = 120 * 1024;

@@ -926,7 +926,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                  const __grid_constant__ CUtensorMap tm_bias) {
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
 
@@ -935,7 +935,7 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
 
   Ctx c;
   c.p = &p;
-  c.smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  c.smem = smem_u32(smem_raw);
   c.bars = c.smem + p.off_bar;
   c.abort_flag = &abort_flag;
 

@@ -10,21 +10,23 @@
 //
 // Both are the same machine: persistent CTAs over tiles of 128 rows, the weights resident in shared memory,
 //
-//   warps 12-19  row producers: global -> registers -> (LayerNorm and pair bias | gate product) -> bf16 ->
+//   warps 12-19  row producers: global -> registers -> (LayerNorm | gate product) -> bf16 ->
 //                shared memory in the layout of a tcgen05.mma A operand (K-major, 128-byte swizzle,
 //                panels of 64 channels).  A row is spread over C / 8 lanes, 8 channels each, so global
 //                reads are full 16-byte pieces of consecutive lanes, the LayerNorm reductions are four
 //                (C = 64: three) shuffles and its parameters stay in registers.  The next rows are
 //                requested before the current ones are worked on.
 //   warp 0       TMEM allocation, the weights' TMA loads, the MMAs (fp32 accumulators in TMEM)
-//   warps 4-11   epilogue, one TMEM lane quarter x one half of the columns each: TMEM -> registers -> bf16 or
-//                fp32 -> a private XOR-swizzled patch of shared memory -> 16-byte stores in runs of 128 bytes
+//   warps 4-11   epilogue, one TMEM lane quarter each, the two warpgroups taking the accumulators in turn: TMEM ->
+//                registers -> bf16 or fp32 -> a private XOR-swizzled patch of shared memory -> 16-byte stores
+//                in runs of 128 bytes
 //   warps 1-3    unused (they give their registers to the other roles)
 //
 // What bounds them is HBM: per row of a bf16 pair with C = 128 the front reads 256 bytes and writes 1 024
 // (+ 2 Hb), the output pass reads 512 and writes 256.  The normalised pair and the gated product never
-// reach HBM.  One tile of the front is about 7 300 cycles of an SM's share of HBM time, against 2 400 issue
-// slots per scheduler for the LayerNorm + bias and 1 500 for the epilogue.
+// reach HBM.  The pair bias is part of the GEMM: as arithmetic of the row producers (32 FMAs and five
+// shuffles per row piece) it made their chain the limit, 185 us against 148 (768 x 768 x 128 bf16; 116 us at
+// the copy rate).  The output pass takes 82 us there (69 at the copy rate).
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -44,22 +46,27 @@ constexpr int kGridRegsMisc = 32, kGridRegsEpi = 104, kGridRegsRows = 120;
 static_assert(128 * kGridRegsMisc + 256 * kGridRegsEpi + 256 * kGridRegsRows <= 96 * kGridThreads,
               "setmaxnreg totals exceed the launch allocation");
 
-template <int C, int kOutC, int kStagesT>
+// Shared memory: kRows weight rows per panel of 64 channels, the A tiles, the epilogue patches, barriers.
+template <int C, int kRowsT, int kStagesT>
 struct GridTile {
-  static constexpr int kStages = kStagesT;
+  static constexpr int kStages = kStagesT, kRows = kRowsT;
   static constexpr uint32_t kX = 128 * C * 2;              // one A tile: C / 64 panels of 128 rows x 128 bytes
-  static constexpr uint32_t kW = kOutC * C * 2;            // weights: C / 64 panels of kOutC rows x 128 bytes
+  static constexpr uint32_t kW = kRows * C * 2;            // weights: C / 64 panels of kRows rows x 128 bytes
   static constexpr uint32_t kPatch = 8 * 32 * 128;         // per epilogue warp: 32 rows x 128 bytes
-  static constexpr uint32_t kBiasPatch = kGridProducerWarps * 4 * kGridRowsPerWarp * 2;
-  static constexpr uint32_t off_x = kW, off_patch = off_x + kStages * kX, off_bias = off_patch + kPatch,
-                            off_bar = off_bias + kBiasPatch;
-  static constexpr uint32_t kSmem = off_bar + 128 + 1024 /*alignment*/;
+  static constexpr uint32_t off_x = kW, off_patch = off_x + kStages * kX, off_bar = off_patch + kPatch;
+  static constexpr uint32_t off_slot = off_bar + 120;      // TMEM address, abort flag
+  static constexpr uint32_t kSmem = off_bar + 128;
 };
-template <int C> using FrontTile = GridTile<C, 4 * C, C == 128 ? 2 : 4>;
+// Front: the q rows, then kBiasRows rows of the bias projection (each fp32 weight as a bf16 high part, rows
+// 0-3, plus a bf16 low part, rows 4-7, so that it is not rounded to bf16), then the k, v and gate rows: the
+// bias comes out of the q rows' MMAs as 16 more columns (the upper eight read k rows and are not used).
+constexpr int kBiasRows = 8;
+template <int C> using FrontTile = GridTile<C, 4 * C + kBiasRows, C == 128 ? 2 : 4>;
 template <int C> using OutTile = GridTile<C, C, 4>;
+constexpr int kFrontAcc = 3;     // accumulators of C + 16 (rounded up to C + 32) TMEM columns, taken in turn
 
 struct GridBar {
-  static constexpr int w_full = 0, x_ready = 1 /*[4]*/, x_empty = 5 /*[4]*/, acc_full = 9 /*[2]*/, acc_empty = 11 /*[2]*/, count = 13;
+  static constexpr int w_full = 0, x_ready = 1 /*[4]*/, x_empty = 5 /*[4]*/, acc_full = 9 /*[3]*/, acc_empty = 12 /*[3]*/, count = 15;
 };
 
 struct GridParams {
@@ -67,7 +74,7 @@ struct GridParams {
   int R, N;                // the pair is [R, N, C]
   int H, D;                // heads and head width, H * D == C
   int transpose;           // 1: q, k, v are those of the pair with its two positions exchanged: [N, H, R, D]
-  int split;               // front: CTAs that share a tile's 4 C output columns (small problems)
+  int split;               // front: CTAs that share a tile's four outputs (small problems): 1, 2 or 4
   float q_scale;
   const void* pair;        // front: input rows
   const float* gamma;      // front with LayerNorm
@@ -87,9 +94,9 @@ struct GridParams {
 
 #define AF3K_GRID_WAIT(idx, parity)                                                              \
   do {                                                                                           \
-    const bool ok_ = mbar_wait_bounded(bars + 8u * (idx), (parity), p.wait_limit, &abort_flag);   \
+    const bool ok_ = mbar_wait_bounded(bars + 8u * (idx), (parity), p.wait_limit, abort_flag);    \
     if (!__all_sync(0xffffffffu, ok_)) {                                                         \
-      grid_timeout(p, &abort_flag, (idx));                                                       \
+      grid_timeout(p, abort_flag, (idx));                                                        \
       goto done;                                                                                 \
     }                                                                                            \
   } while (0)
@@ -130,10 +137,12 @@ __device__ __forceinline__ uint32_t grid_piece(uint32_t tile, int row, int c8) {
   return tile + (uint32_t)((c8 >> 3) * (128 * 128) + row * 128 + (((c8 & 7) ^ (row & 7)) << 4));
 }
 
-// Barrier set-up, TMEM allocation and weight loads shared by both kernels (all threads; ends with a block barrier).
-template <class Tile, int C, int kOutRows>
-__device__ __forceinline__ uint32_t grid_prologue(uint32_t smem, uint32_t bars, uint32_t* slot, int* abort_flag, uint32_t tmem_cols,
-                                                  const CUtensorMap* tm_w, int w_row0, int w_rows) {
+// Barrier set-up, TMEM allocation and weight loads shared by both kernels (all threads; ends with a block
+// barrier).  The weights are `chunks` blocks of C rows from row w_row0 of the packed matrix on; `gap` rows are left
+// free behind the first one.
+template <class Tile, int C>
+__device__ __forceinline__ uint32_t grid_prologue(uint32_t smem, uint32_t bars, volatile uint32_t* slot, volatile int* abort_flag,
+                                                  uint32_t tmem_cols, const CUtensorMap* tm_w, int w_row0, int chunks, int gap) {
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -143,22 +152,24 @@ __device__ __forceinline__ uint32_t grid_prologue(uint32_t smem, uint32_t bars, 
       mbar_init(bars + 8u * (GridBar::x_ready + i), kGridProducerWarps);
       mbar_init(bars + 8u * (GridBar::x_empty + i), 1);
     }
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < 3; ++i) {
       mbar_init(bars + 8u * (GridBar::acc_full + i), 1);
       mbar_init(bars + 8u * (GridBar::acc_empty + i), 4);
     }
     fence_barrier_init();
-    // the weights: rows [w_row0, w_row0 + w_rows) of the packed matrix, panel by panel, in boxes of 64 rows
-    mbar_arrive_expect_tx(bars + 8u * GridBar::w_full, (uint32_t)w_rows * C * 2);
-    for (int kb = 0; kb < C / 64; ++kb)
-      for (int r = 0; r < w_rows; r += 64)
-        tma_load_2d(smem + kb * (kOutRows * 128) + r * 128, tm_w, bars + 8u * GridBar::w_full, kb * 64, w_row0 + r);
+    mbar_arrive_expect_tx(bars + 8u * GridBar::w_full, (uint32_t)chunks * C * C * 2);
+    for (int c = 0; c < chunks; ++c)
+      for (int kb = 0; kb < C / 64; ++kb)
+        for (int r = 0; r < C; r += 64)
+          tma_load_2d(smem + kb * (Tile::kRows * 128) + (c * C + (c > 0 ? gap : 0) + r) * 128, tm_w, bars + 8u * GridBar::w_full,
+                      kb * 64, w_row0 + c * C + r);
   }
   if (warp == 0) {
     __syncwarp();
-    tmem_alloc(smem_u32(slot), tmem_cols);
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(slot)), tmem_cols);
     tmem_relinquish();
   }
+  fence_proxy_async_smem();      // whatever the caller stored for the tensor core
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -183,60 +194,85 @@ template <int C, typename T, bool kLn>
 __global__ void __launch_bounds__(kGridThreads, 1)
 grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CUtensorMap tm_w) {
   using Tile = FrontTile<C>;
-  extern __shared__ uint8_t grid_smem_raw[];
-  __shared__ uint32_t tmem_slot;
-  __shared__ int abort_flag;
+  extern __shared__ __align__(1024) uint8_t grid_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t smem = (smem_u32(grid_smem_raw) + 1023u) & ~1023u;
+  const uint32_t smem = smem_u32(grid_smem);
   const uint32_t bars = smem + Tile::off_bar;
-  constexpr uint32_t kTmem = 4 * C;
-  // this CTA's share of the columns (all of them unless split): two accumulator halves of `width` columns
+  volatile uint32_t* slot = reinterpret_cast<volatile uint32_t*>(grid_smem + Tile::off_slot);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(grid_smem + Tile::off_slot + 4);
+  constexpr uint32_t kAccCols = C + 32, kTmem = C == 128 ? 512 : 512;
+  static_assert(kFrontAcc * kAccCols <= kTmem, "accumulators exceed TMEM");
+  // this CTA's outputs out of {q + bias, k, v, gate}: all of them unless split
   const int part = blockIdx.x % p.split, first = blockIdx.x / p.split, step = gridDim.x / p.split;
-  const int width = 2 * C / p.split, col_base = part * 2 * width;
+  const int chunks = 4 / p.split, chunk0 = part * chunks;
+  const bool with_bias = kLn && p.Hb > 0 && part == 0;
   const long long n_tiles = (p.M + 127) / 128;
-  const uint32_t tmem = grid_prologue<Tile, C, 4 * C>(smem, bars, &tmem_slot, &abort_flag, kTmem, &tm_w, col_base, 2 * width);
+  if (with_bias && threadIdx.x >= 128) {
+    // bias projection rows, 16 bytes (8 channels) per thread
+    for (int k = threadIdx.x - 128; k < kBiasRows * (C / 8); k += kGridThreads - 128) {
+      const int r = k / (C / 8), c8 = k % (C / 8), h = r & 3;
+      uint32_t w[4] = {0u, 0u, 0u, 0u};
+      if (h < p.Hb) {
+        const float* src = p.bias_w + h * C + c8 * 8;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float x = src[2 * e], y = src[2 * e + 1];
+          if (r >= 4) {   // what the bf16 high part leaves over
+            x -= __bfloat162float(__float2bfloat16_rn(x));
+            y -= __bfloat162float(__float2bfloat16_rn(y));
+          }
+          w[e] = pack_bf16x2(x, y);
+        }
+      }
+      sts128(smem + (c8 >> 3) * (Tile::kRows * 128) + (C + r) * 128 + (((c8 & 7) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+    }
+  }
+  const uint32_t tmem = grid_prologue<Tile, C>(smem, bars, slot, abort_flag, kTmem, &tm_w, chunk0 * C, chunks, kBiasRows);
 
   if (warp < 4) {
     setmaxnreg_dec<kGridRegsMisc>();
     if (warp == 0) {
-      // ---- MMA issuer
+      // ---- MMA issuer: the tile's outputs one after the other, into the accumulators in turn
       const bool leader = elect_one();
-      const uint32_t idesc = make_idesc(1u, 1u, 0u, 0u, (uint32_t)width);
+      const uint32_t idesc = make_idesc(1u, 1u, 0u, 0u, C), idesc_q = make_idesc(1u, 1u, 0u, 0u, C + 16);
       const uint64_t ad0 = make_smem_desc(smem + Tile::off_x, 16, 8 * 128, 2), bd0 = make_smem_desc(smem, 16, 8 * 128, 2);
       const uint32_t ad_lo = (uint32_t)ad0, ad_hi = (uint32_t)(ad0 >> 32), bd_lo = (uint32_t)bd0, bd_hi = (uint32_t)(bd0 >> 32);
       AF3K_GRID_WAIT(GridBar::w_full, 0);
-      uint32_t n = 0;
+      uint32_t n = 0, buf = 0, lap = 0;
       for (long long tile = first; tile < n_tiles; tile += step, ++n) {
         const uint32_t st = n % Tile::kStages;
         AF3K_GRID_WAIT(GridBar::x_ready + st, (n / Tile::kStages) & 1);
-        for (int nh = 0; nh < 2; ++nh) {
-          // the epilogue warps of this half must have read the previous tile's columns
-          if (n >= 1) AF3K_GRID_WAIT(GridBar::acc_empty + nh, (n - 1) & 1);
+        for (int c = 0; c < chunks; ++c) {
+          // the epilogue warps must have read this accumulator's previous columns
+          if (lap > 0) AF3K_GRID_WAIT(GridBar::acc_empty + buf, (lap - 1) & 1);
           tc_fence_after();
           if (leader) {
+            const uint32_t id = c == 0 && with_bias ? idesc_q : idesc;
+            const uint32_t row = (uint32_t)(c * C + (c > 0 ? kBiasRows : 0));
 #pragma unroll
             for (int ks = 0; ks < C / 16; ++ks) {   // 16 channels = 32 bytes of a 128-byte panel row; panel ks / 4
               const uint32_t a = ad_lo + ((st * Tile::kX + (ks >> 2) * (128 * 128)) >> 4) + 2 * (ks & 3);
-              const uint32_t b = bd_lo + (((ks >> 2) * (4 * C * 128) + nh * width * 128) >> 4) + 2 * (ks & 3);
-              mma_ss_f16(tmem + nh * width, a, ad_hi, b, bd_hi, idesc, ks > 0 ? 1u : 0u);
+              const uint32_t b = bd_lo + (((ks >> 2) * (Tile::kRows * 128) + row * 128) >> 4) + 2 * (ks & 3);
+              mma_ss_f16(tmem + buf * kAccCols, a, ad_hi, b, bd_hi, id, ks > 0 ? 1u : 0u);
             }
-            tc_commit(bars + 8u * (GridBar::acc_full + nh));
-            if (nh == 1) tc_commit(bars + 8u * (GridBar::x_empty + st));
+            tc_commit(bars + 8u * (GridBar::acc_full + buf));
+            if (c == chunks - 1) tc_commit(bars + 8u * (GridBar::x_empty + st));
           }
           __syncwarp();
+          if (++buf == kFrontAcc) { buf = 0; ++lap; }
         }
       }
     }
   } else if (warp < 12) {
-    // ---- epilogue: TMEM lane quarter x column half
+    // ---- epilogue: TMEM lane quarter; warps 4-7 take the CTA's even outputs, 8-11 the odd ones
     setmaxnreg_inc<kGridRegsEpi>();
-    const int quarter = warp & 3, half = (warp - 4) >> 2;
-    const uint32_t t_base = tmem + ((uint32_t)(quarter * 32) << 16) + half * width;
+    const int quarter = warp & 3, wg = (warp - 4) >> 2;
+    const uint32_t t_lane = tmem + ((uint32_t)(quarter * 32) << 16);
     const uint32_t patch = smem + Tile::off_patch + (uint32_t)(warp - 4) * (32 * 128);
     const int log2d = 31 - __clz(p.D);
     const int tokens = p.transpose ? p.R : p.N;
-    uint32_t n = 0;
-    for (long long tile = first; tile < n_tiles; tile += step, ++n) {
+    uint32_t count = 0, buf = 0, lap = 0;            // outputs of this CTA so far, their accumulator
+    for (long long tile = first; tile < n_tiles; tile += step) {
       const long long m0 = tile * 128 + quarter * 32;                 // the warp's first row
       const int i0 = (int)(m0 / p.N), j0 = (int)(m0 - (long long)i0 * p.N);
       // Element offsets of the eight rows this lane stores in every 64-column piece (rows (lane >> 3)
@@ -250,51 +286,71 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
         off_qkv[it] = (uint32_t)(p.transpose ? (long long)j * p.H * p.R + i : (long long)i * p.H * p.N + j) << log2d;
         if (m0 + row < p.M) row_ok |= 1u << it;
       }
-      AF3K_GRID_WAIT(GridBar::acc_full + half, n & 1);
-      tc_fence_after();
-#pragma unroll 1
-      for (int c0 = 0; c0 < width; c0 += 64) {
-        const int col0 = col_base + half * width + c0;                // 64 columns of one output tensor
-        const int which = col0 / C, within = col0 % C;                // 0 q, 1 k, 2 v, 3 gate
+      for (int c = 0; c < chunks; ++c, ++count) {
+        const uint32_t b = buf, l = lap;
+        if (++buf == kFrontAcc) { buf = 0; ++lap; }
+        if ((count & 1u) != (uint32_t)wg) continue;
+        const int which = chunk0 + c;                                   // 0 q, 1 k, 2 v, 3 gate
+        const uint32_t t_base = t_lane + b * kAccCols;
         const float mul = which == 0 ? p.q_scale : 1.0f;
-#pragma unroll
-        for (int hc = 0; hc < 2; ++hc) {
-          uint32_t acc[32];
-          tmem_ld_x32(t_base + c0 + 32 * hc, acc);
+        AF3K_GRID_WAIT(GridBar::acc_full + b, l & 1);
+        tc_fence_after();
+        if (c == 0 && with_bias) {
+          // lane = row: consecutive lanes are consecutive j of one pair row (or the next one)
+          uint32_t acc[16];
+          tmem_ld_x16(t_base + C, acc);
           tc_wait_ld();
-          // own row -> shared, piece at position piece ^ (row & 7): conflict-free both ways
+          int i = i0, j = j0 + lane;
+          while (j >= p.N) { j -= p.N; ++i; }
+          if (m0 + lane < p.M) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float f[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(acc[8 * j + e]) * mul;
-            sts128(patch + lane * 128 + (((4 * hc + j) ^ (lane & 7)) << 4), pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]),
-                   pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+            for (int h = 0; h < 4; ++h)
+              if (h < p.Hb)
+                p.bias[((long long)h * p.R + i) * p.bias_pitch + j] =
+                    __float2bfloat16_rn(__uint_as_float(acc[h]) + __uint_as_float(acc[4 + h]));
           }
         }
-        if (c0 + 64 >= width) {
-          // the last columns are in registers: the MMAs of the next tile may overwrite this half
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bars + 8u * (GridBar::acc_empty + half));
-        } else {
-          __syncwarp();
-        }
-        // shared -> global: lane l takes piece l & 7 of rows (l >> 3) + 4 it
-        const int ch = within + 8 * (lane & 7);
-        __nv_bfloat16* dst;
-        if (which == 3) dst = p.g + m0 * C + (lane >> 3) * C + ch;
-        else dst = (which == 0 ? p.q : (which == 1 ? p.k : p.v)) + (((long long)(ch >> log2d) * tokens) << log2d) + (ch & (p.D - 1));
+#pragma unroll 1
+        for (int c0 = 0; c0 < C; c0 += 64) {
 #pragma unroll
-        for (int it = 0; it < 8; ++it) {
-          const int row = it * 4 + (lane >> 3);
-          uint4 o;
-          asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                       : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
-                       : "r"(patch + row * 128 + (((lane & 7) ^ (row & 7)) << 4)));
-          if ((row_ok >> it) & 1u) *reinterpret_cast<uint4*>(dst + (which == 3 ? (uint32_t)(it * 4 * C) : off_qkv[it])) = o;
+          for (int hc = 0; hc < 2; ++hc) {
+            uint32_t acc[32];
+            tmem_ld_x32(t_base + c0 + 32 * hc, acc);
+            tc_wait_ld();
+            // own row -> shared, piece at position piece ^ (row & 7): conflict-free both ways
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float f[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(acc[8 * j + e]) * mul;
+              sts128(patch + lane * 128 + (((4 * hc + j) ^ (lane & 7)) << 4), pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]),
+                     pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+            }
+          }
+          if (c0 + 64 >= C) {
+            // the last columns are in registers: the next MMAs may overwrite this accumulator
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + 8u * (GridBar::acc_empty + b));
+          } else {
+            __syncwarp();
+          }
+          // shared -> global: lane l takes piece l & 7 of rows (l >> 3) + 4 it
+          const int ch = c0 + 8 * (lane & 7);
+          __nv_bfloat16* dst;
+          if (which == 3) dst = p.g + (m0 + (lane >> 3)) * C + ch;
+          else dst = (which == 0 ? p.q : (which == 1 ? p.k : p.v)) + (((long long)(ch >> log2d) * tokens) << log2d) + (ch & (p.D - 1));
+#pragma unroll
+          for (int it = 0; it < 8; ++it) {
+            const int row = it * 4 + (lane >> 3);
+            uint4 o;
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
+                         : "r"(patch + row * 128 + (((lane & 7) ^ (row & 7)) << 4)));
+            if ((row_ok >> it) & 1u) *reinterpret_cast<uint4*>(dst + (which == 3 ? (uint32_t)(it * 4 * C) : off_qkv[it])) = o;
+          }
+          __syncwarp();      // the patch is rewritten by the next 64 columns
         }
-        __syncwarp();      // the patch is rewritten by the next 64 columns
       }
     }
   } else {
@@ -313,8 +369,6 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
       for (int e = 0; e < 8; ++e) { g[e] = p.gamma[8 * c8 + e]; b[e] = p.beta[8 * c8 + e]; }
     }
     const T* src = static_cast<const T*>(p.pair) + 8 * c8;
-    const uint32_t bias_patch = smem + Tile::off_bias + w * (4 * kGridRowsPerWarp * 2);
-    const bool with_bias = kLn && p.Hb > 0 && part == 0;
     Raw8<T> next[kBatch];
     auto request = [&](long long tile, int it0) {
 #pragma unroll
@@ -375,91 +429,30 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
           const int row = w * kGridRowsPerWarp + (it0 + u) * kRowsIt + sub;
           sts128(grid_piece(x_tile, row, c8), yw[u][0], yw[u][1], yw[u][2], yw[u][3]);
         }
-        if (with_bias) {
-          // the bias projection sees the rounded values; four heads' sums over the row's lanes by
-          // exchanging halves: after two exchanges a lane holds one head's partial sum
-          float acc[4][kBatch];
-#pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            float wt[8];
-            if (h < p.Hb) {
-              const float4 w0 = __ldg(reinterpret_cast<const float4*>(p.bias_w + h * C + 8 * c8));
-              const float4 w1 = __ldg(reinterpret_cast<const float4*>(p.bias_w + h * C + 8 * c8) + 1);
-              wt[0] = w0.x; wt[1] = w0.y; wt[2] = w0.z; wt[3] = w0.w; wt[4] = w1.x; wt[5] = w1.y; wt[6] = w1.z; wt[7] = w1.w;
-            } else {
-#pragma unroll
-              for (int e = 0; e < 8; ++e) wt[e] = 0.f;
-            }
-#pragma unroll
-            for (int u = 0; u < kBatch; ++u) {
-              float a = 0.f, c = 0.f;
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                a = fmaf(__uint_as_float(yw[u][e] << 16), wt[2 * e], a);
-                c = fmaf(__uint_as_float(yw[u][e] & 0xffff0000u), wt[2 * e + 1], c);
-              }
-              acc[h][u] = a + c;
-            }
-          }
-          const bool hi1 = (lane & (kLanes / 2)) != 0, hi2 = (lane & (kLanes / 4)) != 0;
-#pragma unroll
-          for (int u = 0; u < kBatch; ++u) {
-            float k0 = hi1 ? acc[2][u] : acc[0][u], k1 = hi1 ? acc[3][u] : acc[1][u];
-            const float s0 = hi1 ? acc[0][u] : acc[2][u], s1 = hi1 ? acc[1][u] : acc[3][u];
-            k0 += __shfl_xor_sync(0xffffffffu, s0, kLanes / 2);
-            k1 += __shfl_xor_sync(0xffffffffu, s1, kLanes / 2);
-            float k = (hi2 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, hi2 ? k0 : k1, kLanes / 4);
-#pragma unroll
-            for (int o = kLanes / 8; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
-            if ((lane & (kLanes / 4 - 1)) == 0) {
-              const int h = (hi1 ? 2 : 0) + (hi2 ? 1 : 0);
-              asm volatile("st.shared.b16 [%0], %1;" ::"r"(bias_patch + (h * kGridRowsPerWarp + (it0 + u) * kRowsIt + sub) * 2),
-                           "h"(__bfloat16_as_ushort(__float2bfloat16_rn(k))) : "memory");
-            }
-          }
-        }
       }
       fence_proxy_async_smem();     // the tile was written through the generic proxy; the tensor core reads it
       __syncwarp();
       if (lane == 0) mbar_arrive(bars + 8u * (GridBar::x_ready + st));
-      if (with_bias) {
-        // the warp's 16 rows x 4 heads: consecutive lanes are consecutive rows
-        const int r = lane & 15;
-        const long long m = tile * 128 + w * kGridRowsPerWarp + r;
-        if (m < p.M) {
-          const int i = (int)(m / p.N), j = (int)(m - (long long)i * p.N);
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            const int h = (lane >> 4) + 2 * hh;
-            if (h < p.Hb) {
-              unsigned short v;
-              asm volatile("ld.shared.b16 %0, [%1];" : "=h"(v) : "r"(bias_patch + (h * kGridRowsPerWarp + r) * 2));
-              p.bias[((long long)h * p.R + i) * p.bias_pitch + j] = __ushort_as_bfloat16(v);
-            }
-          }
-        }
-        __syncwarp();
-      }
     }
   }
 
 done:
-  grid_epilogue_common(&abort_flag, tmem, kTmem);
+  grid_epilogue_common(abort_flag, tmem, kTmem);
 }
 
 template <int C, typename TOut>
 __global__ void __launch_bounds__(kGridThreads, 1)
 grid_out_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CUtensorMap tm_w) {
   using Tile = OutTile<C>;
-  extern __shared__ uint8_t grid_smem_raw[];
-  __shared__ uint32_t tmem_slot;
-  __shared__ int abort_flag;
+  extern __shared__ __align__(1024) uint8_t grid_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t smem = (smem_u32(grid_smem_raw) + 1023u) & ~1023u;
+  const uint32_t smem = smem_u32(grid_smem);
   const uint32_t bars = smem + Tile::off_bar;
+  volatile uint32_t* slot = reinterpret_cast<volatile uint32_t*>(grid_smem + Tile::off_slot);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(grid_smem + Tile::off_slot + 4);
   constexpr uint32_t kTmem = 2 * C;               // two accumulators, taken in turn
   const long long n_tiles = (p.M + 127) / 128;
-  const uint32_t tmem = grid_prologue<Tile, C, C>(smem, bars, &tmem_slot, &abort_flag, kTmem, &tm_w, 0, C);
+  const uint32_t tmem = grid_prologue<Tile, C>(smem, bars, slot, abort_flag, kTmem, &tm_w, 0, 1, 0);
 
   if (warp < 4) {
     setmaxnreg_dec<kGridRegsMisc>();
@@ -589,7 +582,7 @@ grid_out_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CU
   }
 
 done:
-  grid_epilogue_common(&abort_flag, tmem, kTmem);
+  grid_epilogue_common(abort_flag, tmem, kTmem);
 }
 
 // ------------------------------------------------------------------ packed weights

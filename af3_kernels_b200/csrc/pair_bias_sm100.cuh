@@ -349,14 +349,14 @@ __global__ void __launch_bounds__(PbTile<T>::kRows, 640 / PbTile<T>::kRows) pair
 constexpr int kPbmRows = 128;                       // vectors per tile = threads per CTA
 constexpr int kPbmHalfBytes = kPbmRows * 128;       // one 64-channel half of the tile
 constexpr uint32_t kPbmTmemCols = 32;
-// dynamic shared memory from a 1024-aligned base: tile, weights (same layout, 16 rows), gamma / beta,
+// dynamic shared memory: tile, weights (same layout, 16 rows), gamma / beta,
 // bias staging [16][128] bf16, mbarrier + TMEM address slot
 constexpr int kPbmOffW = 2 * kPbmHalfBytes;
 constexpr int kPbmWRows = 32;                       // B operand rows: 16 heads x {high, low} part
 constexpr int kPbmOffC = kPbmOffW + 2 * kPbmWRows * 128;
 constexpr int kPbmOffBias = kPbmOffC + 2 * kPbChannels * 4;
 constexpr int kPbmOffBar = kPbmOffBias + kPbMaxHeads * kPbmRows * 2;
-constexpr int kPbmSmemBytes = kPbmOffBar + 16 + 1024;
+constexpr int kPbmSmemBytes = kPbmOffBar + 16;
 
 __device__ int g_pair_bias_status[4];   // {1 = a bounded wait ran out, block, tile (low word), 0}
 
@@ -365,9 +365,9 @@ __device__ __forceinline__ uint32_t pbm_swz(int row, int piece) {   // byte offs
 }
 
 __global__ void __launch_bounds__(kPbmRows, 5) pair_bias_mma_kernel(const PairBiasParams p, long long wait_limit) {
-  extern __shared__ uint8_t pbm_raw[];
-  const uint32_t base = (smem_u32(pbm_raw) + 1023u) & ~1023u;
-  uint8_t* gbase = pbm_raw + (base - smem_u32(pbm_raw));
+  extern __shared__ __align__(1024) uint8_t pbm_raw[];
+  const uint32_t base = smem_u32(pbm_raw);
+  uint8_t* gbase = pbm_raw;
   float* s_c = reinterpret_cast<float*>(gbase + kPbmOffC);                       // gamma, beta
   __nv_bfloat16* s_bias = reinterpret_cast<__nv_bfloat16*>(gbase + kPbmOffBias);  // [16][128]
   const uint32_t bar = base + kPbmOffBar;
