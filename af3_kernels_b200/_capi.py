@@ -40,6 +40,7 @@ EXPORTED_SYMBOLS = (
     "af3k_grid_front",
     "af3k_grid_out",
     "af3k_grid_pack",
+    "af3k_token_projection",
 )
 
 
@@ -64,6 +65,8 @@ class AttentionDesc(ctypes.Structure):
         ("rows_per_item", ctypes.c_int32),
         ("bias_prescaled", ctypes.c_int32),
         ("max_ctas", ctypes.c_int32),
+        ("gate", ctypes.c_void_p),
+        ("gate_stride", ctypes.c_int64 * 3),
     ]
 
 

@@ -19,6 +19,7 @@ HEADERS = [
     os.path.join(CSRC, "pair_bias_sm100.cuh"),
     os.path.join(CSRC, "grid_sm100.cuh"),
     os.path.join(CSRC, "ptx_sm100.cuh"),
+    os.path.join(CSRC, "token_sm100.cuh"),
     os.path.join(_HERE, "..", "include", "af3k.h"),
 ]
 NVCC_FLAGS = [

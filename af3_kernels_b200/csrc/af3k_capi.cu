@@ -15,6 +15,7 @@
 #include "attn_sm100.cuh"
 #include "grid_sm100.cuh"
 #include "pair_bias_sm100.cuh"
+#include "token_sm100.cuh"
 
 namespace {
 
@@ -105,16 +106,17 @@ int device_info(DeviceInfo** out) {
       return cuda_fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize, pair_bias)", e);
     if ((e = cudaFuncSetAttribute(pair_bias_mma_kernel, attr, kPbmSmemBytes)) != cudaSuccess)
       return cuda_fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize, pair_bias_mma)", e);
-    const std::pair<const void*, uint32_t> grid_kernels[] = {
+    const std::pair<const void*, uint32_t> gemm_kernels[] = {
         {(const void*)grid_front_kernel<128, __nv_bfloat16, true>, FrontTile<128>::kSmem}, {(const void*)grid_front_kernel<128, float, true>, FrontTile<128>::kSmem},
         {(const void*)grid_front_kernel<128, __nv_bfloat16, false>, FrontTile<128>::kSmem}, {(const void*)grid_front_kernel<64, __nv_bfloat16, true>, FrontTile<64>::kSmem},
         {(const void*)grid_front_kernel<64, float, true>, FrontTile<64>::kSmem}, {(const void*)grid_front_kernel<64, __nv_bfloat16, false>, FrontTile<64>::kSmem},
         {(const void*)grid_out_kernel<128, __nv_bfloat16>, OutTile<128>::kSmem}, {(const void*)grid_out_kernel<128, float>, OutTile<128>::kSmem},
         {(const void*)grid_out_kernel<64, __nv_bfloat16>, OutTile<64>::kSmem}, {(const void*)grid_out_kernel<64, float>, OutTile<64>::kSmem},
+        {(const void*)token_proj_kernel<64>, TokTile<64>::kSmem}, {(const void*)token_proj_kernel<128>, TokTile<128>::kSmem},
     };
-    for (const auto& k : grid_kernels)
+    for (const auto& k : gemm_kernels)
       if ((e = cudaFuncSetAttribute(k.first, attr, (int)k.second)) != cudaSuccess)
-        return cuda_fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize, grid)", e);
+        return cuda_fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize, projections)", e);
     d.attr_set = true;
   }
   *out = &d;
@@ -150,6 +152,11 @@ int validate(const af3k_attention_desc& d) {
   if (d.bias_prescaled != 0 && (d.bias_prescaled != 1 || d.qk_dtype != AF3K_FP8_E4M3 || d.bias_dtype != AF3K_BF16))
     return AF3K_ERR_BAD_DTYPE;
   if (d.max_ctas < 0) return AF3K_ERR_BAD_SHAPE;
+  if (d.gate != nullptr) {
+    if (!aligned16(d.gate)) return AF3K_ERR_BAD_ALIGNMENT;
+    for (int i = 0; i < 3; ++i)
+      if (d.gate_stride[i] < 0 || (d.gate_stride[i] * 2) % 16) return AF3K_ERR_BAD_STRIDE;
+  }
   const int64_t es = d.qk_dtype == AF3K_FP8_E4M3 ? 1 : 2;
   for (int i = 0; i < 3; ++i) {
     if (d.q_stride[i] < 0 || d.k_stride[i] < 0 || d.v_stride[i] < 0 || d.out_stride[i] < 0)
@@ -501,6 +508,10 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
   p.out_stride_b1 = d.out_stride[0];
   p.out_stride_b2 = d.out_stride[1];
   p.out_stride_s = d.out_stride[2];
+  p.gate = static_cast<const __nv_bfloat16*>(d.gate);
+  p.gate_stride_b1 = d.gate_stride[0];
+  p.gate_stride_b2 = d.gate_stride[1];
+  p.gate_stride_s = d.gate_stride[2];
   p.status = status_dev;
   p.wait_limit = wait_limit_cycles();
 
@@ -762,11 +773,12 @@ int af3k_grid_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void*
                    int64_t C, int64_t Hb, void* w4, void* wo, float* vec, void* stream_v) {
   t_last_launches = 0;
   if (C < 1 || C > 1024 || Hb < 0 || Hb > 1024 || (Hb > 0 && bias_w == nullptr)) return AF3K_ERR_BAD_SHAPE;
-  if (!w5 || !w4 || !wo || !vec) return AF3K_ERR_NULL_POINTER;
+  if (!w5 || !w4 || (w5[4].data && !wo) || ((gamma || beta || Hb > 0) && !vec)) return AF3K_ERR_NULL_POINTER;
   PackParams p;
   std::memset(&p, 0, sizeof(p));
   auto matrix = [](const af3k_matrix& m) { return PackMatrix{m.data, m.stride_out, m.stride_in, m.dtype == AF3K_F32 ? 1 : 0}; };
   for (int i = 0; i < 5; ++i) {
+    if (!w5[i].data && i == 4) continue;           // a block without an output projection
     if (!w5[i].data) return AF3K_ERR_NULL_POINTER;
     if (w5[i].dtype != AF3K_F32 && w5[i].dtype != AF3K_BF16) return AF3K_ERR_BAD_DTYPE;
     p.w[i] = matrix(w5[i]);
@@ -782,6 +794,49 @@ int af3k_grid_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void*
   grid_pack_kernel<<<(n + 255) / 256, 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail("launch grid_pack_kernel", e);
+  t_last_launches = 1;
+  return AF3K_OK;
+}
+
+int af3k_token_projection(const void* x, const void* w4, const void* q_bias, int32_t q_bias_dtype, int64_t M, int64_t C, float q_scale,
+                          void* out, int* status_dev, void* stream_v) {
+  t_last_launches = 0;
+  if (q_bias && q_bias_dtype != AF3K_BF16 && q_bias_dtype != AF3K_F32) return AF3K_ERR_BAD_DTYPE;
+  if (M < 0 || C < 8 || C % 8 != 0 || C > (1 << 20) || M > 0x7fffff00LL) return AF3K_ERR_BAD_SHAPE;
+  if (M == 0) return AF3K_OK;
+  if (!x || !w4 || !out) return AF3K_ERR_NULL_POINTER;
+  if (!aligned16(x) || !aligned16(w4) || !aligned16(out)) return AF3K_ERR_BAD_ALIGNMENT;
+  DeviceInfo* dev = nullptr;
+  int rc = device_info(&dev);
+  if (rc != AF3K_OK) return rc;
+  const int64_t m_tiles = (M + 127) / 128;
+  const int kn = m_tiles * ((4 * C + 127) / 128) >= dev->sm_count * 3 / 4 ? 128 : 64;   // enough tiles of 128 columns to fill the SMs?
+  const int64_t n_tiles = (4 * C + kn - 1) / kn;
+  if (n_tiles > 65535) return AF3K_ERR_BAD_SHAPE;
+  auto enc = tensor_map_encoder();
+  if (!enc) return driver_fail("cuTensorMapEncodeTiled entry point", -1);
+  CUtensorMap tm_x, tm_w;
+  auto map = [&](CUtensorMap* tm, const void* base, int64_t rows, int box_rows) {
+    cuuint64_t dims[2] = {(cuuint64_t)C, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)C * 2};
+    cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    return enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = map(&tm_x, x, M, 128);
+  if (r == CUDA_SUCCESS) r = map(&tm_w, w4, 4 * C, kn);
+  if (r != CUDA_SUCCESS) return driver_fail("cuTensorMapEncodeTiled(token projection)", (int)r);
+  TokParams p;
+  std::memset(&p, 0, sizeof(p));
+  p.M = (int)M; p.C = (int)C; p.q_bias = q_bias; p.q_bias_f32 = q_bias_dtype == AF3K_F32 ? 1 : 0; p.q_scale = q_scale;
+  p.out = static_cast<__nv_bfloat16*>(out); p.status = status_dev; p.wait_limit = wait_limit_cycles();
+  const dim3 grid((unsigned)m_tiles, (unsigned)n_tiles);
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
+  if (kn == 128) token_proj_kernel<128><<<grid, kTokThreads, TokTile<128>::kSmem, stream>>>(p, tm_x, tm_w);
+  else           token_proj_kernel<64><<<grid, kTokThreads, TokTile<64>::kSmem, stream>>>(p, tm_x, tm_w);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail("launch token_proj_kernel", e);
   t_last_launches = 1;
   return AF3K_OK;
 }

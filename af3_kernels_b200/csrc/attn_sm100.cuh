@@ -106,6 +106,8 @@ struct AttnParams {
   long long mask_row_stride;
   __nv_bfloat16* out;
   long long out_stride_b1, out_stride_b2, out_stride_s;
+  const __nv_bfloat16* gate;   // null, or [B1, B2, Sq, D]: the result is multiplied by sigmoid(gate) before it is rounded
+  long long gate_stride_b1, gate_stride_b2, gate_stride_s;
   int* status;           // int[4]: {status bits, 1 + first barrier slot that timed out, block, warp}
   long long wait_limit;  // SM clocks a single wait may take before the kernel gives up
   float* debug;          // diagnostic dump of block 0's first logits tile (debug build of the kernel)
@@ -887,6 +889,8 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
       const uint32_t o_taddr = c.tmem + lane_sel + kOCol + s * p.nv;
       __nv_bfloat16* orow = p.out + (long long)stream_row(p, it, s) * p.out_stride_b1 +
                             (long long)it.h * p.out_stride_b2 + (long long)qrow * p.out_stride_s;
+      const __nv_bfloat16* grow = p.gate == nullptr ? nullptr : p.gate + (long long)stream_row(p, it, s) * p.gate_stride_b1 +
+                                  (long long)it.h * p.gate_stride_b2 + (long long)qrow * p.gate_stride_s;
       for (int c0 = 0; c0 < p.nv; c0 += 16) {
         uint32_t o[16];
         tmem_ld_x16(o_taddr + c0, o);
@@ -902,6 +906,15 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
 #pragma unroll
           for (int hseg = 0; hseg < 2; ++hseg) {
             if (c0 + hseg * 8 + 8 <= p.D) {
+              if (grow != nullptr) {
+                const uint4 gv = __ldg(reinterpret_cast<const uint4*>(grow + c0 + hseg * 8));
+                const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                  const float g = __uint_as_float((e & 1) ? gw[e >> 1] & 0xffff0000u : gw[e >> 1] << 16);
+                  o[hseg * 8 + e] = __float_as_uint(__uint_as_float(o[hseg * 8 + e]) * sigmoid_fast(g));
+                }
+              }
               uint4 v;
               v.x = pack_bf16x2(__uint_as_float(o[hseg * 8 + 0]) * inv, __uint_as_float(o[hseg * 8 + 1]) * inv);
               v.y = pack_bf16x2(__uint_as_float(o[hseg * 8 + 2]) * inv, __uint_as_float(o[hseg * 8 + 3]) * inv);

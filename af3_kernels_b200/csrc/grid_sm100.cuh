@@ -591,7 +591,7 @@ done:
 // carry any strides (nn.Linear.weight or its transpose).
 struct PackMatrix { const void* src; long long so, si; int f32; };   // element (out, in) at so * out + si * in
 struct PackParams {
-  PackMatrix w[5];         // q, k, v, gate, output projection
+  PackMatrix w[5];         // q, k, v, gate, output projection (src == nullptr: absent)
   PackMatrix bias_w;       // [Hb, C]; src == nullptr: absent
   const void* gamma; const void* beta; int gamma_f32, beta_f32;
   int C, Hb;
@@ -605,6 +605,7 @@ __global__ void grid_pack_kernel(const __grid_constant__ PackParams p) {
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
     if (e < n_mat) {
       const int m = e / (C * C), r = e % (C * C) / C, c = e % C;
+      if (p.w[m].src == nullptr) continue;
       const __nv_bfloat16 v = __float2bfloat16_rn(pack_at(p.w[m].src, p.w[m].so * r + p.w[m].si * c, p.w[m].f32));
       if (m < 4) p.w4[(m * C + r) * C + c] = v; else p.wo[r * C + c] = v;
     } else {

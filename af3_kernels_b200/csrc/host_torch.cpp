@@ -34,6 +34,7 @@ struct Library {
   decltype(&af3k_grid_front) grid_front = nullptr;
   decltype(&af3k_grid_out) grid_out = nullptr;
   decltype(&af3k_grid_pack) grid_pack = nullptr;
+  decltype(&af3k_token_projection) token_projection = nullptr;
 };
 Library g_lib;
 
@@ -52,6 +53,7 @@ void bind_library(const std::string& path) {
   AF3K_BIND(grid_front, af3k_grid_front);
   AF3K_BIND(grid_out, af3k_grid_out);
   AF3K_BIND(grid_pack, af3k_grid_pack);
+  AF3K_BIND(token_projection, af3k_token_projection);
 #undef AF3K_BIND
 }
 
@@ -303,8 +305,8 @@ std::mutex g_packed_mu;
 std::list<Packed>* g_packed = new std::list<Packed>();
 constexpr size_t kPackedMost = 16;
 
-// params: q, k, v, gate, output projection [C, C] as (out, in) matrices, then (all or none) LayerNorm weight and
-// bias [C], bias projection [Hb, C]
+// params: q, k, v, gate and perhaps output projection [C, C] as (out, in) matrices, then (all or none) LayerNorm
+// weight and bias [C], bias projection [Hb, C]
 Packed packed_weights(const std::vector<Tensor>& params, int64_t C) {
   const at::Device dev = params[0].device();
   const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
@@ -344,12 +346,12 @@ Packed packed_weights(const std::vector<Tensor>& params, int64_t C) {
   auto dtype_of = [](const Tensor& t) { return t.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16; };
   auto matrix = [&](const Tensor& t) { return af3k_matrix{t.data_ptr(), t.stride(0), t.stride(1), dtype_of(t)}; };
   af3k_matrix w5[5], bw{};
-  for (int i = 0; i < 5; ++i) w5[i] = matrix(src[i]);
+  for (int i = 0; i < 5; ++i) w5[i] = i < (int)src.size() ? matrix(src[i]) : af3k_matrix{};
   if (with_ln) bw = matrix(src[7]);
   Packed e;
   const auto options = at::TensorOptions().device(dev);
   e.w4 = at::empty({4 * C, C}, options.dtype(at::kBFloat16));
-  e.wo = at::empty({C, C}, options.dtype(at::kBFloat16));
+  e.wo = at::empty({params.size() > 4 ? C : 0, C}, options.dtype(at::kBFloat16));
   e.vec = at::empty({(2 + Hb) * C}, options.dtype(at::kFloat));
   check(g_lib.grid_pack(w5, with_ln ? &bw : nullptr, with_ln ? src[5].data_ptr() : nullptr, with_ln ? src[6].data_ptr() : nullptr,
                         with_ln ? dtype_of(src[5]) : AF3K_F32, C, Hb, e.w4.data_ptr(), e.wo.data_ptr(), e.vec.data_ptr<float>(), stream));
@@ -451,6 +453,52 @@ Tensor grid_block(const Tensor& pair, const OptTensor& mask, const Tensor& bias,
   check(g_lib.grid_out(weighted.data_ptr(), gate.data_ptr(), w.wo.data_ptr(), out.data_ptr(), pair.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16,
                        M, C, status, stream));
   return out;
+}
+
+// ------------------------------------------------------------------ the single / diffusion attention block
+// x [N, C] -> the four projections in one GEMM (query bias and softmax scale folded in) -> attention, gated as it
+// leaves the kernel: two launches.  weights: q, k, v, gate as [out, in].
+Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, const std::vector<Tensor>& weights, Tensor q_bias, int64_t head) {
+  const at::Device dev = x_in.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  const int64_t N = x_in.size(0), C = x_in.size(1), D = C / head;
+  matrices(weights, C);
+  if (q_bias.numel() != C) value_error("q_bias must have one entry per channel");
+  if (bias.numel() != head * N * N) value_error("bias must have B2*Sq*Sk = " + std::to_string(head * N * N) + " elements, got " + std::to_string(bias.numel()));
+  if (bias.device() != dev) value_error("q, k, v, bias must live on the same device");
+  Tensor x = x_in.to(at::kBFloat16).contiguous();
+  if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0) x = x.clone();
+  if (N == 0) return at::empty({N, C}, x_in.options());
+  if (q_bias.device() != dev || (q_bias.scalar_type() != at::kBFloat16 && q_bias.scalar_type() != at::kFloat)) q_bias = q_bias.to(dev, at::kFloat);
+  q_bias = q_bias.contiguous();
+  const Packed w = packed_weights(weights, C);
+  const float scale = 1.0f / std::sqrt((float)D);
+  const bool in_place = bias.scalar_type() == at::kBFloat16 && bias.dim() == 3 && bias.stride(2) == 1 && (bias.stride(1) * 2) % 16 == 0 &&
+                        (bias.stride(0) * 2) % 16 == 0 && (bias.stride(0) != 0 || head == 1) && (bias.stride(1) != 0 || N == 1) &&
+                        reinterpret_cast<uintptr_t>(bias.data_ptr()) % 16 == 0;
+  if (!in_place) bias = staged_bias(bias, head, N, N, D, std::nullopt, std::nullopt, nullptr, nullptr, scale);
+  Tensor mask;
+  if (mask_in) {
+    if (mask_in->numel() != N) value_error("mask of shape " + shape_text(*mask_in) + " does not match B1=1, Sk=" + std::to_string(N));
+    mask = mask_in->device() == dev ? mask_in->contiguous() : mask_in->to(dev).contiguous();
+  }
+  Tensor qkvg = at::empty({4, N, C}, x.options()), out = at::empty({N, C}, x.options());
+  char* b = static_cast<char*>(qkvg.data_ptr());
+  const size_t part = (size_t)N * C * 2;
+  int* status = status_buffer(dev.index()).data_ptr<int>();
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  check(g_lib.token_projection(x.data_ptr(), w.w4.data_ptr(), q_bias.data_ptr(), q_bias.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16, N, C,
+                               scale, b, status, stream));
+  af3k_attention_desc d{};
+  d.B1 = 1; d.B2 = head; d.Sq = N; d.Sk = N; d.D = D;
+  for (int64_t* st : {d.q_stride, d.k_stride, d.v_stride, d.out_stride, d.gate_stride}) { st[0] = N * C; st[1] = D; st[2] = C; }
+  d.bias_stride[0] = bias.stride(0); d.bias_stride[1] = bias.stride(1);
+  d.qk_dtype = AF3K_BF16; d.bias_dtype = AF3K_BF16;
+  d.softmax_scale = 1.0f;                            // q left the projection scaled
+  d.gate = b + 3 * part;
+  check(g_lib.attention(&d, b, b + part, b + 2 * part, bias.data_ptr(), mask.defined() ? static_cast<const uint8_t*>(mask.data_ptr()) : nullptr,
+                        out.data_ptr(), nullptr, nullptr, nullptr, 0, status, stream));
+  return x_in.scalar_type() == at::kBFloat16 ? out : out.to(x_in.scalar_type());
 }
 
 // ------------------------------------------------------------------ the operator on host tensors
@@ -594,6 +642,7 @@ PYBIND11_MODULE(_host, m) {
   m.def("grid_fused", &grid_fused);
   m.def("grid_module", &grid_module, py::call_guard<py::gil_scoped_release>());
   m.def("grid_block", &grid_block, py::call_guard<py::gil_scoped_release>());
+  m.def("self_block", &self_block, py::call_guard<py::gil_scoped_release>());
   m.def("host_attention", &host_attention, py::call_guard<py::gil_scoped_release>());
   m.def("bind_library", &bind_library);
   m.def("status_buffer", &status_buffer);

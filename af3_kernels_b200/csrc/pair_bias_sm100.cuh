@@ -555,14 +555,6 @@ __global__ void __launch_bounds__(kPbmRows, 5) pair_bias_mma_kernel(const PairBi
 }
 
 // ---------------------------------------------------------------- sigmoid gate
-// sigmoid(x) = 1 / (1 + 2^(-x log2 e)), by the two approximate instructions (a few fp32 ulps; every use rounds
-// the product to bf16)
-__device__ __forceinline__ float sigmoid_fast(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + ex2_approx(-1.4426950408889634f * x)));
-  return r;
-}
-
 // out = weighted * sigmoid(gate), elementwise over bf16 tensors of n elements (n a multiple of 8,
 // pointers 16-byte aligned).  Stands in for the SigmoidFwdTPP + MulTPP pair behind the core in the
 // reference's fused blocks (src/csrc/dot_product_attention.cpp:339-345 and :522-528).  The

@@ -321,6 +321,13 @@ __device__ __forceinline__ float ex2_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// sigmoid(x) = 1 / (1 + 2^(-x log2 e)), by the two approximate instructions (a few fp32 ulps; every use rounds
+// the product to bf16)
+__device__ __forceinline__ float sigmoid_fast(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + ex2_approx(-1.4426950408889634f * x)));
+  return r;
+}
 // packs {lo, hi} -> bf16x2 with lo in bits [0,16)
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   uint32_t r;

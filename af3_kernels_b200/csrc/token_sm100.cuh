@@ -1,0 +1,177 @@
+// The four projections of the single / diffusion attention block in one GEMM, for sm_100a:
+//
+//     [q | k | v | gate] = x [M, C] * W4^T,   q <- (q + q_bias) * q_scale,     W4 = [Wq; Wk; Wv; Wg] ([4 C, C])
+//
+// Stands in for the projection BRGEMMs of the reference's fused block
+// (src/csrc/dot_product_attention.cpp:425-480).  M is a token count (tens to a few thousand), C 384 or 768
+// in practice: a few GFLOP, so what bounds it is latency - one tile of 128 rows x kN columns per CTA, the
+// K blocks of 64 channels streamed through six stages that hold all of K at C = 384, one warp each for the
+// TMA and the MMAs, four for the epilogue.  kN is 64 where tiles of 128 columns would leave SMs idle.
+#pragma once
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <cstdint>
+
+#include "ptx_sm100.cuh"
+
+namespace af3k {
+
+constexpr int kTokThreads = 192, kTokStages = 6;
+template <int kN> struct TokTile {
+  static constexpr uint32_t kA = 128 * 128, kB = kN * 128, kStage = kA + kB;
+  static constexpr uint32_t off_bar = kTokStages * kStage, kSmem = off_bar + 128;
+};
+
+struct TokParams {
+  int M, C;
+  const void* q_bias;        // [C] bf16 or fp32, may be null
+  int q_bias_f32;
+  float q_scale;
+  __nv_bfloat16* out;        // [4, M, C]
+  int* status;
+  long long wait_limit;
+};
+
+template <int kN>
+__global__ void __launch_bounds__(kTokThreads, 1)
+token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ CUtensorMap tm_x,
+                  const __grid_constant__ CUtensorMap tm_w) {
+  using Tile = TokTile<kN>;
+  extern __shared__ __align__(1024) uint8_t tok_smem[];
+  const uint32_t smem = smem_u32(tok_smem), bars = smem + Tile::off_bar;   // full [6], empty [6], acc
+  volatile uint32_t* slot = reinterpret_cast<volatile uint32_t*>(tok_smem + Tile::off_bar + 112);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tok_smem + Tile::off_bar + 116);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = blockIdx.x * 128, n0 = blockIdx.y * kN, kblocks = (p.C + 63) / 64;
+  auto timeout = [&](int bar) {
+    *abort_flag = 1;
+    if (p.status != nullptr) {
+      atomicOr(p.status, 1 /* wait timeout */);
+      if (atomicCAS(p.status + 1, 0, 3000 + bar + 1) == 0) { p.status[2] = blockIdx.x; p.status[3] = warp; }
+    }
+  };
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    prefetch_tensormap(&tm_x);
+    prefetch_tensormap(&tm_w);
+    for (int i = 0; i < 2 * kTokStages + 1; ++i) mbar_init(bars + 8u * i, 1);
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(slot)), kN);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int kb = 0; kb < kblocks; ++kb) {
+        const int st = kb % kTokStages;
+        if (kb >= kTokStages && !mbar_wait_bounded(bars + 8u * (kTokStages + st), ((kb / kTokStages) - 1) & 1, p.wait_limit, const_cast<volatile int*>(abort_flag))) {
+          timeout(kTokStages + st);
+          break;
+        }
+        const uint32_t full = bars + 8u * st, dst = smem + st * Tile::kStage;
+        mbar_arrive_expect_tx(full, Tile::kStage);
+        tma_load_2d(dst, &tm_x, full, kb * 64, m0);
+        tma_load_2d(dst + Tile::kA, &tm_w, full, kb * 64, n0);
+      }
+    }
+  } else if (warp == 1) {
+    const bool leader = elect_one();
+    const uint32_t idesc = make_idesc(1u, 1u, 0u, 0u, kN);
+    const uint64_t d0 = make_smem_desc(smem, 16, 8 * 128, 2);
+    const uint32_t lo = (uint32_t)d0, hi = (uint32_t)(d0 >> 32);
+    bool ok = true;
+    for (int kb = 0; kb < kblocks && ok; ++kb) {
+      const int st = kb % kTokStages;
+      ok = mbar_wait_bounded(bars + 8u * st, (kb / kTokStages) & 1, p.wait_limit, const_cast<volatile int*>(abort_flag));
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) { timeout(st); break; }
+      tc_fence_after();
+      if (leader) {
+        const uint32_t a = lo + ((st * Tile::kStage) >> 4), b = a + (Tile::kA >> 4);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) mma_ss_f16(tmem, a + 2 * ks, hi, b + 2 * ks, hi, idesc, kb + ks > 0 ? 1u : 0u);
+        tc_commit(bars + 8u * (kTokStages + st));
+        if (kb == kblocks - 1) tc_commit(bars + 8u * (2 * kTokStages));
+      }
+      __syncwarp();
+    }
+  } else {
+    // ---- epilogue: TMEM lane quarter; the stages are free when the accumulator is complete
+    const int quarter = warp & 3;
+    const bool ok = mbar_wait_bounded(bars + 8u * (2 * kTokStages), 0, p.wait_limit, const_cast<volatile int*>(abort_flag));
+    if (__all_sync(0xffffffffu, ok)) {
+      tc_fence_after();
+      const uint32_t t_base = tmem + ((uint32_t)(quarter * 32) << 16);
+      const uint32_t patch = smem + quarter * (32 * 128);
+#pragma unroll 1
+      for (int c0 = 0; c0 < kN; c0 += 64) {
+#pragma unroll
+        for (int hc = 0; hc < 2; ++hc) {
+          uint32_t acc[32];
+          tmem_ld_x32(t_base + c0 + 32 * hc, acc);
+          tc_wait_ld();
+          const int col = n0 + c0 + 32 * hc;
+          if (col < p.C) {             // (some) q columns
+#pragma unroll
+            for (int e = 0; e < 32; ++e) {
+              if (col + e < p.C) {
+                float bq = 0.f;
+                if (p.q_bias != nullptr)
+                  bq = p.q_bias_f32 ? __ldg(static_cast<const float*>(p.q_bias) + col + e)
+                                    : __bfloat162float(__ldg(static_cast<const __nv_bfloat16*>(p.q_bias) + col + e));
+                acc[e] = __float_as_uint((__uint_as_float(acc[e]) + bq) * p.q_scale);
+              }
+            }
+          }
+          // own row -> shared, piece at position piece ^ (row & 7): conflict-free both ways
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(patch + lane * 128 + (((4 * hc + j) ^ (lane & 7)) << 4)),
+                         "r"(pack_bf16x2(__uint_as_float(acc[8 * j]), __uint_as_float(acc[8 * j + 1]))),
+                         "r"(pack_bf16x2(__uint_as_float(acc[8 * j + 2]), __uint_as_float(acc[8 * j + 3]))),
+                         "r"(pack_bf16x2(__uint_as_float(acc[8 * j + 4]), __uint_as_float(acc[8 * j + 5]))),
+                         "r"(pack_bf16x2(__uint_as_float(acc[8 * j + 6]), __uint_as_float(acc[8 * j + 7]))) : "memory");
+        }
+        __syncwarp();
+        // shared -> global: lane l takes piece l & 7 of rows (l >> 3) + 4 it; eight columns never straddle outputs
+        const int col = n0 + c0 + 8 * (lane & 7);
+        if (col < 4 * p.C) {
+          const int which = col / p.C;
+          __nv_bfloat16* dst = p.out + ((long long)which * p.M) * p.C + (col - which * p.C);
+#pragma unroll
+          for (int it = 0; it < 8; ++it) {
+            const int row = it * 4 + (lane >> 3), m = m0 + quarter * 32 + row;
+            uint4 o;
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
+                         : "r"(patch + row * 128 + (((lane & 7) ^ (row & 7)) << 4)));
+            if (m < p.M) *reinterpret_cast<uint4*>(dst + (long long)m * p.C) = o;
+          }
+        }
+        __syncwarp();      // the patch is rewritten by the next 64 columns
+      }
+    } else {
+      timeout(2 * kTokStages);
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag != 0) {
+    for (int i = 0; i < 200; ++i) __nanosleep(10000);
+    __syncthreads();
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, kN);
+  }
+}
+
+}  // namespace af3k

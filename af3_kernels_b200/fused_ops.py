@@ -157,12 +157,15 @@ def self_attention_block(
     N, C = x.shape
     if C % head != 0:
         raise ValueError("channels must be divisible by the number of heads")
+    m = None if mask is None else bool_mask(mask.reshape(-1), 1, N)
+    if (C // head) % 8 == 0 and C // head <= 64 and C <= 1024:
+        # one GEMM for the four projections, one kernel for attention and gate
+        return _capi.host().self_block(x, m, bias, [w.t() for w in (q_proj, k_proj, v_proj, gating_query)], q_bias, head)
     D = C // head
     xb = _as_bf16(x)
     q = (torch.matmul(xb, _as_bf16(q_proj)) + _as_bf16(q_bias).reshape(C)).view(1, N, head, D).permute(0, 2, 1, 3)
     k = torch.matmul(xb, _as_bf16(k_proj)).view(1, N, head, D).permute(0, 2, 1, 3)
     v = torch.matmul(xb, _as_bf16(v_proj)).view(1, N, head, D).permute(0, 2, 1, 3)
     weighted = torch.empty((1, N, head, D), dtype=torch.bfloat16, device=x.device)
-    m = None if mask is None else mask.reshape(-1)
     dot_product_attention(q, k, v, m, bias, out=weighted.permute(0, 2, 1, 3))
     return sigmoid_gate(weighted.view(N, C), torch.matmul(xb, _as_bf16(gating_query))).to(x.dtype)

@@ -67,6 +67,10 @@ typedef struct af3k_attention_desc {
   int32_t max_ctas;       /* 0 = one CTA per SM; > 0: at most this many CTAs, leaving the other SMs to
                              kernels that run beside this one (the collective that gathers a
                              row-sharded output while the next piece is computed) */
+  const void* gate;       /* NULL, or bf16 [B1, B2, Sq, D], 16-byte aligned: the result is multiplied by
+                             sigmoid(gate) before it is rounded (what the reference's fused single attention
+                             block does behind its core, src/csrc/dot_product_attention.cpp:522-528) */
+  int64_t gate_stride[3]; /* b1, b2, s; innermost stride 1, 16-byte multiples */
 } af3k_attention_desc;
 
 /* Library / ABI version (major * 1000 + minor). */
@@ -254,6 +258,15 @@ int af3k_grid_front(const void* pair, int32_t pair_dtype, const float* gamma, co
 int af3k_grid_out(const void* weighted, const void* gate, const void* wo, void* out, int32_t out_dtype, int64_t M,
                   int64_t C, int* status_dev, void* stream);
 
+/* The four projections of the single / diffusion attention block:  out = [q | k | v | gate], each [M, C],
+ *     q = (x Wq^T + q_bias) * q_scale,  k = x Wk^T,  v = x Wv^T,  gate = x Wg^T
+ * Stands in for the projection BRGEMMs of the reference's fused block
+ * (src/csrc/dot_product_attention.cpp:425-480).
+ *   x [M, C] bf16;  w4 [4 C, C] bf16, rows = output channels of q, k, v, gate;  q_bias [C] bf16 or fp32, may be
+ *   NULL;  out [4, M, C] bf16.  C a multiple of 8.  All contiguous, pointers 16-byte aligned (q_bias: any). */
+int af3k_token_projection(const void* x, const void* w4, const void* q_bias, int32_t q_bias_dtype, int64_t M,
+                          int64_t C, float q_scale, void* out, int* status_dev, void* stream);
+
 /* A weight matrix of the block: element (out, in) at data[out * stride_out + in * stride_in], bf16 or fp32. */
 typedef struct af3k_matrix {
   const void* data;
@@ -262,7 +275,7 @@ typedef struct af3k_matrix {
 } af3k_matrix;
 
 /* Lays a block's parameters out for af3k_grid_front / af3k_grid_out in one launch: w5 = q, k, v, gate, output
- * projection -> w4 [4 C, C] and wo [C, C] bf16;  gamma, beta (both of ln_dtype, may be NULL) and bias_w [Hb, C]
+ * projection (data NULL: there is none, wo is not written) -> w4 [4 C, C] and wo [C, C] bf16;  gamma, beta (both of ln_dtype, may be NULL) and bias_w [Hb, C]
  * (NULL with Hb 0) -> vec: fp32 gamma [C], beta [C], bias_w [Hb, C].  No counterpart in the reference (which
  * repacks its weights for its CPU GEMM, src/csrc/tools.cpp:151-176). */
 int af3k_grid_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void* gamma, const void* beta,

@@ -240,3 +240,22 @@ def test_fused_grid_module_against_oracle(cuda_device, N, C, H, dtype, transpose
     _close(out, ref, (N, C, H, dtype, transpose))
     assert torch.equal(flipped, -out)
     assert read_status(cuda_device)[0] == 0
+
+
+@pytest.mark.parametrize("N,C,H,dtype", [(1, 64, 4, torch.bfloat16), (77, 384, 16, torch.bfloat16), (128, 200, 5, torch.float32),
+                                         (129, 768, 16, torch.bfloat16), (700, 384, 16, torch.float32), (1100, 512, 8, torch.bfloat16)])
+def test_self_block_against_oracle(cuda_device, N, C, H, dtype):
+    """Single block over what its projection kernel branches on: rows short of a tile and one past it, K blocks
+    short of 64 channels, fewer and more K blocks than stages, both tile widths; odd N stages the bias."""
+    g = torch.Generator().manual_seed(N)
+    x = torch.randn(N, C, generator=g).to(dtype)
+    ws = [(torch.randn(C, C, generator=g) * C ** -0.5).to(dtype) for _ in range(4)]        # [in, out]
+    qb = (torch.randn(C, generator=g) * 0.3).to(dtype)
+    bias = torch.randn(H, N, N, generator=g).to(dtype)
+    mask = torch.arange(N) < N - N // 9
+    ref = O.self_block_fp32(x, mask, bias, ws[0].T, qb, ws[1].T, ws[2].T, ws[3].T, H)
+    dev = cuda_device
+    out = A.self_attention_cpp(x.to(dev), mask.to(dev), bias.to(dev), ws[0].to(dev), qb.to(dev), *(w.to(dev) for w in ws[1:]), H)
+    assert out.dtype == dtype and out.shape == (N, C)
+    _close(out, ref, (N, C, H, dtype))
+    assert read_status(dev)[0] == 0
