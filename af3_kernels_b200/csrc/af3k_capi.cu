@@ -92,8 +92,9 @@ int device_info(DeviceInfo** out) {
     const int dyn = d.max_smem_optin - kStaticSmemReserve;
     const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     const void* kernels[] = {
-        (const void*)attention_kernel<false, false>, (const void*)attention_kernel<true, false>,
-        (const void*)attention_kernel<false, true>,  (const void*)attention_kernel<true, true>,
+        (const void*)attention_kernel<false, false, false>, (const void*)attention_kernel<true, false, false>,
+        (const void*)attention_kernel<false, true, false>,  (const void*)attention_kernel<true, true, false>,
+        (const void*)attention_kernel<false, false, true>,  (const void*)attention_kernel<false, true, true>,
     };
     e = cudaSuccess;
     for (const void* kfn : kernels)
@@ -522,10 +523,12 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
   p.scale_q = (fp8 || d.softmax_scale == 1.0f) ? 0 : 1;   // a scale of exactly 1 (q already scaled by its producer) needs no pass over Q
   const bool dbg = p.debug != nullptr;
 #define AF3K_LAUNCH(...) attention_kernel<__VA_ARGS__><<<plan.grid, kThreads, plan.smem_bytes, stream>>>(p, tm_q, tm_k, tm_v, tm_b)
-  if (!tc_bias) {
-    if (dbg) AF3K_LAUNCH(true, false); else AF3K_LAUNCH(false, false);
+  if (p.gate != nullptr) {
+    if (tc_bias) AF3K_LAUNCH(false, true, true); else AF3K_LAUNCH(false, false, true);
+  } else if (!tc_bias) {
+    if (dbg) AF3K_LAUNCH(true, false, false); else AF3K_LAUNCH(false, false, false);
   } else {
-    if (dbg) AF3K_LAUNCH(true, true); else AF3K_LAUNCH(false, true);
+    if (dbg) AF3K_LAUNCH(true, true, false); else AF3K_LAUNCH(false, true, false);
   }
 #undef AF3K_LAUNCH
   cudaError_t e = cudaGetLastError();
