@@ -181,6 +181,24 @@ int validate(const af3k_attention_desc& d) {
   return AF3K_OK;
 }
 
+// Launches a kernel whose blocks may become resident under the tail of the kernel before it on the stream; the
+// kernel itself waits for that one (grid_wait_previous) before it touches global memory.  Not with a block limit
+// (max_ctas): the SMs it leaves free are another stream's, and blocks that wait there would take them.
+template <typename... KArgs, typename... Args>
+void launch_overlapped(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t stream, bool overlap, const Args&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  (void)cudaLaunchKernelEx(&cfg, kernel, args...);   // the caller reads cudaGetLastError
+}
+
 struct Plan {
   AttnParams p;
   size_t smem_bytes;
@@ -522,7 +540,7 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
   const bool tc_bias = !fp8 || fp8_tc;
   p.scale_q = (fp8 || d.softmax_scale == 1.0f) ? 0 : 1;   // a scale of exactly 1 (q already scaled by its producer) needs no pass over Q
   const bool dbg = p.debug != nullptr;
-#define AF3K_LAUNCH(...) attention_kernel<__VA_ARGS__><<<plan.grid, kThreads, plan.smem_bytes, stream>>>(p, tm_q, tm_k, tm_v, tm_b)
+#define AF3K_LAUNCH(...) launch_overlapped(attention_kernel<__VA_ARGS__>, dim3(plan.grid), kThreads, plan.smem_bytes, stream, d.max_ctas <= 0, p, tm_q, tm_k, tm_v, tm_b)
   if (p.gate != nullptr) {
     if (tc_bias) AF3K_LAUNCH(false, true, true); else AF3K_LAUNCH(false, false, true);
   } else if (!tc_bias) {
@@ -686,9 +704,9 @@ int encode_weight_map(CUtensorMap* tm, const void* w, int64_t C, int64_t rows) {
 template <int C>
 void launch_front(const GridParams& p, const CUtensorMap& tm, unsigned grid, bool f32, bool ln, cudaStream_t stream) {
   constexpr uint32_t smem = FrontTile<C>::kSmem;
-  if (!ln)      grid_front_kernel<C, __nv_bfloat16, false><<<grid, kGridThreads, smem, stream>>>(p, tm);
-  else if (f32) grid_front_kernel<C, float, true><<<grid, kGridThreads, smem, stream>>>(p, tm);
-  else          grid_front_kernel<C, __nv_bfloat16, true><<<grid, kGridThreads, smem, stream>>>(p, tm);
+  if (!ln)      launch_overlapped(grid_front_kernel<C, __nv_bfloat16, false>, dim3(grid), kGridThreads, smem, stream, true, p, tm);
+  else if (f32) launch_overlapped(grid_front_kernel<C, float, true>, dim3(grid), kGridThreads, smem, stream, true, p, tm);
+  else          launch_overlapped(grid_front_kernel<C, __nv_bfloat16, true>, dim3(grid), kGridThreads, smem, stream, true, p, tm);
 }
 }  // namespace
 
@@ -760,11 +778,11 @@ int af3k_grid_out(const void* weighted, const void* gate, const void* wo, void* 
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   const bool f32 = out_dtype == AF3K_F32;
   if (C == 128) {
-    if (f32) grid_out_kernel<128, float><<<grid, kGridThreads, OutTile<128>::kSmem, stream>>>(p, tm);
-    else     grid_out_kernel<128, __nv_bfloat16><<<grid, kGridThreads, OutTile<128>::kSmem, stream>>>(p, tm);
+    if (f32) launch_overlapped(grid_out_kernel<128, float>, dim3(grid), kGridThreads, OutTile<128>::kSmem, stream, true, p, tm);
+    else     launch_overlapped(grid_out_kernel<128, __nv_bfloat16>, dim3(grid), kGridThreads, OutTile<128>::kSmem, stream, true, p, tm);
   } else {
-    if (f32) grid_out_kernel<64, float><<<grid, kGridThreads, OutTile<64>::kSmem, stream>>>(p, tm);
-    else     grid_out_kernel<64, __nv_bfloat16><<<grid, kGridThreads, OutTile<64>::kSmem, stream>>>(p, tm);
+    if (f32) launch_overlapped(grid_out_kernel<64, float>, dim3(grid), kGridThreads, OutTile<64>::kSmem, stream, true, p, tm);
+    else     launch_overlapped(grid_out_kernel<64, __nv_bfloat16>, dim3(grid), kGridThreads, OutTile<64>::kSmem, stream, true, p, tm);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail("launch grid_out_kernel", e);
@@ -836,8 +854,8 @@ int af3k_token_projection(const void* x, const void* w4, const void* q_bias, int
   p.out = static_cast<__nv_bfloat16*>(out); p.status = status_dev; p.wait_limit = wait_limit_cycles();
   const dim3 grid((unsigned)m_tiles, (unsigned)n_tiles);
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
-  if (kn == 128) token_proj_kernel<128><<<grid, kTokThreads, TokTile<128>::kSmem, stream>>>(p, tm_x, tm_w);
-  else           token_proj_kernel<64><<<grid, kTokThreads, TokTile<64>::kSmem, stream>>>(p, tm_x, tm_w);
+  if (kn == 128) launch_overlapped(token_proj_kernel<128>, grid, kTokThreads, TokTile<128>::kSmem, stream, true, p, tm_x, tm_w);
+  else           launch_overlapped(token_proj_kernel<64>, grid, kTokThreads, TokTile<64>::kSmem, stream, true, p, tm_x, tm_w);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail("launch token_proj_kernel", e);
   t_last_launches = 1;

@@ -908,7 +908,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
           for (int hseg = 0; hseg < 2; ++hseg) {
             if (c0 + hseg * 8 + 8 <= p.D) {
               if constexpr (kGate) {
-                const uint4 gv = __ldg(reinterpret_cast<const uint4*>(grow + c0 + hseg * 8));
+                const uint4 gv = *reinterpret_cast<const uint4*>(grow + c0 + hseg * 8);
                 const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
@@ -1004,6 +1004,8 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
                    "h"((uint16_t)0x3F80) : "memory");
     fence_proxy_async_smem();
   }
+  grid_wait_previous();
+  grid_release_next();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

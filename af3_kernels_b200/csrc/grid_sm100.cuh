@@ -119,7 +119,7 @@ __device__ __forceinline__ Raw8<T> load_raw8(const T* src, bool live) {
   Raw8<T> r;
 #pragma unroll
   for (int i = 0; i < (int)sizeof(T) / 2; ++i)
-    r.v[i] = live ? __ldg(reinterpret_cast<const uint4*>(src) + i) : make_uint4(0u, 0u, 0u, 0u);
+    r.v[i] = live ? reinterpret_cast<const uint4*>(src)[i] : make_uint4(0u, 0u, 0u, 0u);
   return r;
 }
 template <typename T>
@@ -157,6 +157,7 @@ __device__ __forceinline__ uint32_t grid_prologue(uint32_t smem, uint32_t bars, 
       mbar_init(bars + 8u * (GridBar::acc_empty + i), 4);
     }
     fence_barrier_init();
+    grid_wait_previous();
     mbar_arrive_expect_tx(bars + 8u * GridBar::w_full, (uint32_t)chunks * C * C * 2);
     for (int c = 0; c < chunks; ++c)
       for (int kb = 0; kb < C / 64; ++kb)
@@ -169,6 +170,9 @@ __device__ __forceinline__ uint32_t grid_prologue(uint32_t smem, uint32_t bars, 
     tmem_alloc(smem_u32(const_cast<uint32_t*>(slot)), tmem_cols);
     tmem_relinquish();
   }
+  // No grid_release_next here: the next kernel's blocks come in as this one's end.  Letting them in earlier was slower
+  // (389 rows 255 -> 257 us a module call, 768 rows 923 -> 926).
+  grid_wait_previous();
   fence_proxy_async_smem();      // whatever the caller stored for the tensor core
   tc_fence_before();
   __syncthreads();
@@ -209,6 +213,7 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
   const long long n_tiles = (p.M + 127) / 128;
   if (with_bias && threadIdx.x >= 128) {
     // bias projection rows, 16 bytes (8 channels) per thread
+    grid_wait_previous();
     for (int k = threadIdx.x - 128; k < kBiasRows * (C / 8); k += kGridThreads - 128) {
       const int r = k / (C / 8), c8 = k % (C / 8), h = r & 3;
       uint32_t w[4] = {0u, 0u, 0u, 0u};

@@ -62,6 +62,8 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
     tmem_alloc(smem_u32(const_cast<uint32_t*>(slot)), kN);
     tmem_relinquish();
   }
+  grid_wait_previous();
+  grid_release_next();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -124,8 +126,8 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
               if (col + e < p.C) {
                 float bq = 0.f;
                 if (p.q_bias != nullptr)
-                  bq = p.q_bias_f32 ? __ldg(static_cast<const float*>(p.q_bias) + col + e)
-                                    : __bfloat162float(__ldg(static_cast<const __nv_bfloat16*>(p.q_bias) + col + e));
+                  bq = p.q_bias_f32 ? static_cast<const float*>(p.q_bias)[col + e]
+                                    : __bfloat162float(static_cast<const __nv_bfloat16*>(p.q_bias)[col + e]);
                 acc[e] = __float_as_uint((__uint_as_float(acc[e]) + bq) * p.q_scale);
               }
             }

@@ -259,3 +259,56 @@ def test_self_block_against_oracle(cuda_device, N, C, H, dtype):
     assert out.dtype == dtype and out.shape == (N, C)
     _close(out, ref, (N, C, H, dtype))
     assert read_status(dev)[0] == 0
+
+
+@pytest.mark.parametrize("N,C,dtype", [(24, 128, torch.bfloat16), (129, 64, torch.float32), (200, 128, torch.float32)])
+def test_kernels_that_start_under_the_previous_ones_wait_for_them(cuda_device, N, C, dtype):
+    """Every kernel of a chain reads what the one before wrote (and overwrites buffers that it read): modules in both
+    orientations, a plain call and the single block, back to back, on two streams and from a graph, give the bits of
+    the same chain with a synchronisation behind every call."""
+    g = torch.Generator().manual_seed(21)
+    H, D = 4, C // 4
+    mods = []
+    for t in (False, True):
+        m = A.GridSelfAttentionCpp(C, H, t)
+        with torch.no_grad():
+            for p in m.parameters():
+                p.copy_(torch.randn(p.shape, generator=g) * (C ** -0.5 if p.dim() == 2 else 0.1))
+            m.act_norm.weight.add_(1.0)
+        mods.append(m.to(cuda_device, dtype).eval())
+    pair0 = torch.randn(N, N, C, generator=g).to(cuda_device, dtype)
+    mask = (torch.rand(N, N, generator=g) >= 0.1).to(cuda_device)
+    w = [(torch.randn(C, C, generator=g) * C ** -0.5).to(cuda_device, dtype) for _ in range(4)]
+    qb = torch.zeros(C, device=cuda_device, dtype=dtype)
+
+    def chain(pair, between):
+        for i in range(6):
+            pair = mods[i % 2](pair, mask)
+            between()
+            x = pair.reshape(N, N, H, D).permute(0, 2, 1, 3).to(torch.bfloat16)
+            pair = A.dot_product_attention_cpp(x, x, x, mask, x[:H, 0, :, :1].expand(H, N, N)).permute(0, 2, 1, 3).reshape(N, N, C).to(dtype)
+            between()
+            row = A.self_attention_cpp(pair[0], mask[0], pair.permute(2, 0, 1)[:H].contiguous(), *w[:1], qb, *w[1:], H)
+            between()
+            pair = pair + row
+        return pair
+
+    with torch.no_grad():
+        want = chain(pair0, torch.cuda.synchronize)
+        got = [chain(pair0, lambda: None) for _ in range(5)]
+        streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+        for s in streams * 2:
+            s.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(s):
+                got.append(chain(pair0, lambda: None))
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = chain(pair0, lambda: None)
+        for _ in range(3):
+            graph.replay()
+        torch.cuda.synchronize()
+        got.append(out)
+    for i, r in enumerate(got):
+        assert torch.equal(r, want), i
+    assert read_status(cuda_device)[0] == 0
