@@ -205,6 +205,12 @@ struct Plan {
   int grid;
 };
 
+// A logits tile of an item with one stream against one of an item with two: the warpgroup has the XU, the MMA
+// issuers and the instruction fetch to itself.  So where twice the CTAs are free, two query tiles take two of them:
+// 16 heads, us a call, two tiles per CTA -> one: 300 tokens 10.2 -> 8.5, 512 11.7 -> 9.6, 700 15.1 -> 13.0, 1152 (144
+// CTAs) 21.4 -> 16.8; 2 x 512 tokens 15.1 -> 11.9.  From there on the CTAs would take two rounds.
+constexpr double kLoneTile = 0.75;
+
 // Picks rows-per-item G and the K/V ring depth from a cost model of one CTA's time (below).
 // allow_q_split: the kernel variant that will run supports query-tile streams (every variant in
 // which the tensor core adds the bias).
@@ -236,14 +242,17 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   if (g_max > p.B1) g_max = p.B1 > 0 ? p.B1 : 1;
 
   int best_g = 0, best_stages = 0, best_qbuf = 0;
+  bool best_split = false;
   double best_cost = 0;
   // rows_per_item is a request: it is honoured up to what TMEM and the batch allow
   const int g_req = d.rows_per_item > g_max ? g_max : d.rows_per_item;
   for (int g = 1; g <= g_max; ++g) {
     if (g_req != 0 && g != g_req) continue;
-    for (int qbuf = 2; qbuf >= 1; --qbuf) {
-      // one pair row per item: the two softmax warpgroups take two neighbouring query tiles
-      const bool split = g == 1 && allow_q_split && p.n_qt >= 2;
+    // one pair row per item: the two softmax warpgroups take two neighbouring query tiles, or one of them idles
+    const bool may_split = g == 1 && allow_q_split && p.n_qt >= 2;
+    for (int form = may_split ? 0 : 2; form < 4; ++form) {
+      const bool split = form < 2;
+      const int qbuf = 2 - (form & 1);
       const int streams = split ? 2 : g;
       int stages = (budget - fixed - qbuf * streams * (int)p.q_tile_bytes) / kv_stage;
       if (stages > kMaxKvStages) stages = kMaxKvStages;
@@ -258,18 +267,18 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
       // a single Q buffer the next item's Q tiles are loaded and scaled at the hand-over (about 0.5:
       // each stream's tile is replaced as soon as its last Q K^T has finished).
       const int slots = split ? 2 : ((g & 1) ? g + 1 : g);
-      double cost = (double)rounds * (p.n_kt * (slots / 2) + 0.8 + (qbuf == 1 ? 0.5 : 0.0));
+      double cost = (double)rounds * (p.n_kt * (slots / 2) * (streams == 1 ? kLoneTile : 1.0) + 0.8 + (qbuf == 1 ? 0.5 : 0.0));
       // a K/V tile takes about two thousand cycles to arrive, most of a logits tile's time: with a
       // short ring the MMAs wait for their operands (measured: 4 stages cost about 3 %)
       static const double kRingPenalty[7] = {0, 0, 1.4, 1.15, 1.03, 1.0, 1.0};
       cost *= kRingPenalty[stages];
       if (split) cost *= 1.02;   // query-tile streams share no bias tile: pair rows win a tie
-      if (best_g == 0 || cost < best_cost) { best_g = g; best_cost = cost; best_stages = stages; best_qbuf = qbuf; }
+      if (best_g == 0 || cost < best_cost) { best_g = g; best_cost = cost; best_stages = stages; best_qbuf = qbuf; best_split = split; }
     }
   }
   if (best_g == 0) return AF3K_ERR_BAD_SHAPE;
   p.G = best_g;
-  p.q_split = (best_g == 1 && allow_q_split && p.n_qt >= 2) ? 1 : 0;
+  p.q_split = best_split ? 1 : 0;
   p.n_streams = p.q_split ? 2 : p.G;
   p.kv_stages = best_stages;
   p.q_buffers = best_qbuf;
@@ -578,7 +587,8 @@ int af3k_describe_plan(const af3k_attention_desc* desc, int32_t* out6) {
   if (rc != AF3K_OK) return rc;
   out6[0] = plan.p.G;
   out6[1] = plan.p.kv_stages;
-  out6[2] = plan.p.n_items;
+  // with one pair row per item always the number of query-tile pairs, also where each tile is an item of its own
+  out6[2] = plan.p.G == 1 && plan.p.n_qt >= 2 && !plan.p.q_split ? plan.p.B1 * plan.p.B2 * ((plan.p.n_qt + 1) / 2) : plan.p.n_items;
   out6[3] = plan.grid;
   out6[4] = (int32_t)plan.smem_bytes;
   out6[5] = (int32_t)kOCol + plan.p.n_streams * plan.p.nv;

@@ -401,3 +401,18 @@ def test_debug_dump_shows_the_tensor_core_stages(cuda_device):
     ref = O.oracle_fp32(q.cpu(), k.cpu(), v.cpu(), mask, bias.cpu())
     _check_bf16(out.cpu(), ref, "debug build")
 
+
+
+@pytest.mark.parametrize("B1,B2,S,D", [(1, 16, 129, 24), (1, 16, 257, 48), (1, 16, 1152, 32), (1, 3, 640, 64), (2, 16, 512, 48), (3, 16, 200, 32),
+                                       (1, 16, 1153, 16)])
+def test_query_tiles_on_ctas_of_their_own(cuda_device, B1, B2, S, D):
+    """Up to one CTA per SM every (row, head, query tile) gets a CTA of its own; a cap on the CTAs makes two query tiles
+    (or rows) share one.  Same bits, and the oracle's result."""
+    g = torch.Generator().manual_seed(B1 * S + D)
+    q, k, v = (torch.randn(B1, B2, S, D, generator=g).to(torch.bfloat16) for _ in range(3))
+    bias = torch.randn(B2, S, S, generator=g).to(torch.bfloat16)
+    mask = torch.rand(B1, S, generator=g) >= 0.1
+    own = _run(cuda_device, q, k, v, mask, bias)
+    tiles = B1 * B2 * ((S + 127) // 128)
+    assert torch.equal(_run(cuda_device, q, k, v, mask, bias, max_ctas=max(1, tiles // 2)), own)
+    _check_bf16(own, O.oracle_fp32(q, k, v, mask, bias), (B1, B2, S, D))
