@@ -392,7 +392,7 @@ int static_scratch_address(void** out) {
 
 extern "C" {
 
-int af3k_version(void) { return 1003; }
+int af3k_version(void) { return 1004; }
 
 const char* af3k_strerror(int code) {
   switch (code) {
@@ -712,7 +712,7 @@ int encode_weight_map(CUtensorMap* tm, const void* w, int64_t C, int64_t rows) {
 }
 
 template <int C>
-void launch_front(const GridParams& p, const CUtensorMap& tm, unsigned grid, bool f32, bool ln, cudaStream_t stream) {
+void launch_front(const GridParams& p, const FrontMaps& tm, unsigned grid, bool f32, bool ln, cudaStream_t stream) {
   constexpr uint32_t smem = FrontTile<C>::kSmem;
   if (!ln)      launch_overlapped(grid_front_kernel<C, __nv_bfloat16, false>, dim3(grid), kGridThreads, smem, stream, true, p, tm);
   else if (f32) launch_overlapped(grid_front_kernel<C, float, true>, dim3(grid), kGridThreads, smem, stream, true, p, tm);
@@ -722,30 +722,38 @@ void launch_front(const GridParams& p, const CUtensorMap& tm, unsigned grid, boo
 
 extern "C" {
 
-int af3k_grid_front(const void* pair, int32_t pair_dtype, const float* gamma, const float* beta, float eps, const float* bias_w,
-                    int64_t Hb, const void* w4, int64_t R, int64_t N, int64_t C, int64_t H, float q_scale, int32_t transpose,
-                    void* bias, int64_t bias_pitch, void* q, void* k, void* v, void* gate, int* status_dev, void* stream_v) {
+int af3k_grid_front_weights(const void* pair, int32_t pair_dtype, const af3k_front_weights* weights, float eps, int64_t Hb, int64_t R,
+                            int64_t N, int64_t C, int64_t H, float q_scale, int32_t transpose, void* bias, int64_t bias_pitch, void* q,
+                            void* k, void* v, void* gate, int* status_dev, void* stream_v) {
   t_last_launches = 0;
-  const bool ln = gamma != nullptr;
+  if (weights == nullptr) return AF3K_ERR_NULL_POINTER;
+  const af3k_front_weights& w = *weights;
+  const bool ln = w.gamma != nullptr;
   if (pair_dtype != AF3K_BF16 && !(pair_dtype == AF3K_F32 && ln)) return AF3K_ERR_BAD_DTYPE;
+  for (int32_t t : {w.ln_dtype, w.bias_w_dtype})
+    if (t != AF3K_BF16 && t != AF3K_F32) return AF3K_ERR_BAD_DTYPE;
   if (C != 64 && C != 128) return AF3K_ERR_BAD_SHAPE;
   if (R < 0 || N < 0 || H < 1 || C % H != 0 || (C / H) % 8 != 0 || Hb < 0 || Hb > 4 || (Hb > 0 && !ln)) return AF3K_ERR_BAD_SHAPE;
   if (R > 0x7fffffff || N > 0x7fffffff || R * N * C > 0x7fffffffLL) return AF3K_ERR_BAD_SHAPE;    // 32-bit element offsets
   if (Hb > 0 && (bias_pitch < N || (bias_pitch & 7) != 0)) return AF3K_ERR_BAD_STRIDE;
   if (R == 0 || N == 0) return AF3K_OK;
-  if (!pair || !w4 || !q || !k || !v || !gate || (ln && !beta) || (Hb > 0 && (!bias_w || !bias))) return AF3K_ERR_NULL_POINTER;
-  for (const void* ptr : {pair, w4, (const void*)q, (const void*)k, (const void*)v, (const void*)gate})
+  if (!pair || !q || !k || !v || !gate || (ln && !w.beta) || (Hb > 0 && (!w.bias_w || !bias))) return AF3K_ERR_NULL_POINTER;
+  for (const void* m : w.w)
+    if (!m) return AF3K_ERR_NULL_POINTER;
+  for (const void* ptr : {pair, w.w[0], w.w[1], w.w[2], w.w[3], (const void*)q, (const void*)k, (const void*)v, (const void*)gate})
     if (!aligned16(ptr)) return AF3K_ERR_BAD_ALIGNMENT;
-  if (Hb > 0 && (!aligned16(bias_w) || !aligned16(bias))) return AF3K_ERR_BAD_ALIGNMENT;
+  if (Hb > 0 && !aligned16(bias)) return AF3K_ERR_BAD_ALIGNMENT;
   DeviceInfo* dev = nullptr;
   int rc = device_info(&dev);
   if (rc != AF3K_OK) return rc;
-  CUtensorMap tm;
-  if ((rc = encode_weight_map(&tm, w4, C, 4 * C)) != AF3K_OK) return rc;
+  FrontMaps tm;
+  for (int i = 0; i < 4; ++i)
+    if ((rc = encode_weight_map(&tm.w[i], w.w[i], C, C)) != AF3K_OK) return rc;
   GridParams p;
   std::memset(&p, 0, sizeof(p));
   p.M = R * N; p.R = (int)R; p.N = (int)N; p.H = (int)H; p.D = (int)(C / H); p.transpose = transpose ? 1 : 0;
-  p.q_scale = q_scale; p.pair = pair; p.gamma = gamma; p.beta = beta; p.bias_w = bias_w; p.eps = eps; p.Hb = (int)Hb;
+  p.q_scale = q_scale; p.pair = pair; p.gamma = w.gamma; p.beta = w.beta; p.ln_f32 = w.ln_dtype == AF3K_F32 ? 1 : 0;
+  p.bias_w = w.bias_w; p.bias_w_f32 = w.bias_w_dtype == AF3K_F32 ? 1 : 0; p.eps = eps; p.Hb = (int)Hb;
   p.bias = static_cast<__nv_bfloat16*>(bias); p.bias_pitch = bias_pitch;
   p.q = static_cast<__nv_bfloat16*>(q); p.k = static_cast<__nv_bfloat16*>(k);
   p.v = static_cast<__nv_bfloat16*>(v); p.g = static_cast<__nv_bfloat16*>(gate);
@@ -764,6 +772,18 @@ int af3k_grid_front(const void* pair, int32_t pair_dtype, const float* gamma, co
   if (e != cudaSuccess) return cuda_fail("launch grid_front_kernel", e);
   t_last_launches = 1;
   return AF3K_OK;
+}
+
+int af3k_grid_front(const void* pair, int32_t pair_dtype, const float* gamma, const float* beta, float eps, const float* bias_w,
+                    int64_t Hb, const void* w4, int64_t R, int64_t N, int64_t C, int64_t H, float q_scale, int32_t transpose,
+                    void* bias, int64_t bias_pitch, void* q, void* k, void* v, void* gate, int* status_dev, void* stream_v) {
+  if (Hb > 0 && bias_w && !aligned16(bias_w)) { t_last_launches = 0; return AF3K_ERR_BAD_ALIGNMENT; }
+  af3k_front_weights w{};
+  for (int i = 0; i < 4; ++i) w.w[i] = w4 ? static_cast<const char*>(w4) + (size_t)i * C * C * 2 : nullptr;
+  w.gamma = gamma; w.beta = beta; w.bias_w = bias_w;
+  w.ln_dtype = w.bias_w_dtype = AF3K_F32;
+  return af3k_grid_front_weights(pair, pair_dtype, &w, eps, Hb, R, N, C, H, q_scale, transpose, bias, bias_pitch, q, k, v, gate,
+                                 status_dev, stream_v);
 }
 
 int af3k_grid_out(const void* weighted, const void* gate, const void* wo, void* out, int32_t out_dtype, int64_t M, int64_t C,
@@ -818,11 +838,12 @@ int af3k_grid_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void*
     if (bias_w->dtype != AF3K_F32 && bias_w->dtype != AF3K_BF16) return AF3K_ERR_BAD_DTYPE;
     p.bias_w = matrix(*bias_w);
   }
-  p.gamma = gamma; p.beta = beta; p.gamma_f32 = p.beta_f32 = ln_dtype == AF3K_F32 ? 1 : 0;
+  p.gamma = gamma; p.beta = beta; p.ln_f32 = ln_dtype == AF3K_F32 ? 1 : 0;
   p.C = (int)C; p.Hb = (int)Hb;
   p.w4 = static_cast<__nv_bfloat16*>(w4); p.wo = static_cast<__nv_bfloat16*>(wo); p.vec = vec;
-  const int n = (int)(5 * C * C + (2 + Hb) * C);
-  grid_pack_kernel<<<(n + 255) / 256, 256, 0, reinterpret_cast<cudaStream_t>(stream_v)>>>(p);
+  const unsigned tiles = (unsigned)((C + kPackTile - 1) / kPackTile);
+  const unsigned slices = vec != nullptr ? 6 : (w5[4].data ? 5 : 4);
+  launch_overlapped(grid_pack_kernel, dim3(tiles, tiles, slices), kPackThreads, 0, reinterpret_cast<cudaStream_t>(stream_v), true, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail("launch grid_pack_kernel", e);
   t_last_launches = 1;

@@ -32,6 +32,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <type_traits>
 
 #include "pair_bias_sm100.cuh"
 #include "ptx_sm100.cuh"
@@ -77,9 +78,10 @@ struct GridParams {
   int split;               // front: CTAs that share a tile's four outputs (small problems): 1, 2 or 4
   float q_scale;
   const void* pair;        // front: input rows
-  const float* gamma;      // front with LayerNorm
-  const float* beta;
-  const float* bias_w;     // [Hb, C]
+  const void* gamma;       // front with LayerNorm: [C], bf16 or fp32
+  const void* beta;
+  const void* bias_w;      // [Hb, C], bf16 or fp32
+  int ln_f32, bias_w_f32;
   float eps;
   int Hb;
   __nv_bfloat16* bias;     // [Hb, R, bias_pitch]
@@ -137,16 +139,33 @@ __device__ __forceinline__ uint32_t grid_piece(uint32_t tile, int row, int c8) {
   return tile + (uint32_t)((c8 >> 3) * (128 * 128) + row * 128 + (((c8 & 7) ^ (row & 7)) << 4));
 }
 
+// The front's four weight matrices [C, C] (output rows), each where its owner keeps it: a call reads the parameters
+// as they are then, and there is no copy that could be out of date.
+struct FrontMaps { CUtensorMap w[4]; };
+
+// elements i .. i + n - 1 of a parameter in the type it is kept in, all loads in flight at once (with the type looked at
+// per element they wait for one another)
+template <int n>
+__device__ __forceinline__ void params_at(const void* src, long long i, int f32, float (&x)[n]) {
+  if (f32) {
+#pragma unroll
+    for (int e = 0; e < n; ++e) x[e] = static_cast<const float*>(src)[i + e];
+  } else {
+#pragma unroll
+    for (int e = 0; e < n; ++e) x[e] = __bfloat162float(static_cast<const __nv_bfloat16*>(src)[i + e]);
+  }
+}
+
 // Barrier set-up, TMEM allocation and weight loads shared by both kernels (all threads; ends with a block
-// barrier).  The weights are `chunks` blocks of C rows from row w_row0 of the packed matrix on; `gap` rows are left
-// free behind the first one.
+// barrier).  The weights are `chunks` matrices of C rows, one tensor map each; `gap` rows are left free behind the
+// first one.
 template <class Tile, int C>
 __device__ __forceinline__ uint32_t grid_prologue(uint32_t smem, uint32_t bars, volatile uint32_t* slot, volatile int* abort_flag,
-                                                  uint32_t tmem_cols, const CUtensorMap* tm_w, int w_row0, int chunks, int gap) {
+                                                  uint32_t tmem_cols, const CUtensorMap* tm_w, int chunks, int gap) {
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    prefetch_tensormap(tm_w);
+    for (int c = 0; c < chunks; ++c) prefetch_tensormap(tm_w + c);
     mbar_init(bars + 8u * GridBar::w_full, 1);
     for (int i = 0; i < Tile::kStages; ++i) {
       mbar_init(bars + 8u * (GridBar::x_ready + i), kGridProducerWarps);
@@ -162,8 +181,8 @@ __device__ __forceinline__ uint32_t grid_prologue(uint32_t smem, uint32_t bars, 
     for (int c = 0; c < chunks; ++c)
       for (int kb = 0; kb < C / 64; ++kb)
         for (int r = 0; r < C; r += 64)
-          tma_load_2d(smem + kb * (Tile::kRows * 128) + (c * C + (c > 0 ? gap : 0) + r) * 128, tm_w, bars + 8u * GridBar::w_full,
-                      kb * 64, w_row0 + c * C + r);
+          tma_load_2d(smem + kb * (Tile::kRows * 128) + (c * C + (c > 0 ? gap : 0) + r) * 128, tm_w + c, bars + 8u * GridBar::w_full,
+                      kb * 64, r);
   }
   if (warp == 0) {
     __syncwarp();
@@ -196,7 +215,7 @@ __device__ __forceinline__ void grid_epilogue_common(volatile int* abort_flag, u
 
 template <int C, typename T, bool kLn>
 __global__ void __launch_bounds__(kGridThreads, 1)
-grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CUtensorMap tm_w) {
+grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ FrontMaps maps) {
   using Tile = FrontTile<C>;
   extern __shared__ __align__(1024) uint8_t grid_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -204,7 +223,7 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
   const uint32_t bars = smem + Tile::off_bar;
   volatile uint32_t* slot = reinterpret_cast<volatile uint32_t*>(grid_smem + Tile::off_slot);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(grid_smem + Tile::off_slot + 4);
-  constexpr uint32_t kAccCols = C + 32, kTmem = C == 128 ? 512 : 512;
+  constexpr uint32_t kAccCols = C + 32, kTmem = 512;
   static_assert(kFrontAcc * kAccCols <= kTmem, "accumulators exceed TMEM");
   // this CTA's outputs out of {q + bias, k, v, gate}: all of them unless split
   const int part = blockIdx.x % p.split, first = blockIdx.x / p.split, step = gridDim.x / p.split;
@@ -218,10 +237,11 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
       const int r = k / (C / 8), c8 = k % (C / 8), h = r & 3;
       uint32_t w[4] = {0u, 0u, 0u, 0u};
       if (h < p.Hb) {
-        const float* src = p.bias_w + h * C + c8 * 8;
+        float v[8];
+        params_at(p.bias_w, h * C + c8 * 8, p.bias_w_f32, v);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          float x = src[2 * e], y = src[2 * e + 1];
+          float x = v[2 * e], y = v[2 * e + 1];
           if (r >= 4) {   // what the bf16 high part leaves over
             x -= __bfloat162float(__float2bfloat16_rn(x));
             y -= __bfloat162float(__float2bfloat16_rn(y));
@@ -232,7 +252,7 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
       sts128(smem + (c8 >> 3) * (Tile::kRows * 128) + (C + r) * 128 + (((c8 & 7) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
     }
   }
-  const uint32_t tmem = grid_prologue<Tile, C>(smem, bars, slot, abort_flag, kTmem, &tm_w, chunk0 * C, chunks, kBiasRows);
+  const uint32_t tmem = grid_prologue<Tile, C>(smem, bars, slot, abort_flag, kTmem, maps.w + chunk0, chunks, kBiasRows);
 
   if (warp < 4) {
     setmaxnreg_dec<kGridRegsMisc>();
@@ -370,8 +390,8 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
     const int c8 = lane % kLanes, sub = lane / kLanes;  // channels 8 c8 .., row within the step
     float g[8], b[8];
     if (kLn) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) { g[e] = p.gamma[8 * c8 + e]; b[e] = p.beta[8 * c8 + e]; }
+      params_at(p.gamma, 8 * c8, p.ln_f32, g);
+      params_at(p.beta, 8 * c8, p.ln_f32, b);
     }
     const T* src = static_cast<const T*>(p.pair) + 8 * c8;
     Raw8<T> next[kBatch];
@@ -457,7 +477,7 @@ grid_out_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CU
   volatile int* abort_flag = reinterpret_cast<volatile int*>(grid_smem + Tile::off_slot + 4);
   constexpr uint32_t kTmem = 2 * C;               // two accumulators, taken in turn
   const long long n_tiles = (p.M + 127) / 128;
-  const uint32_t tmem = grid_prologue<Tile, C>(smem, bars, slot, abort_flag, kTmem, &tm_w, 0, 1, 0);
+  const uint32_t tmem = grid_prologue<Tile, C>(smem, bars, slot, abort_flag, kTmem, &tm_w, 1, 0);
 
   if (warp < 4) {
     setmaxnreg_dec<kGridRegsMisc>();
@@ -591,34 +611,65 @@ done:
 }
 
 // ------------------------------------------------------------------ packed weights
-// One launch that lays a block's parameters out for the two kernels: W4 [4 C, C] = q, k, v, gate rows, Wo [C, C]
-// (rows = output channels, bf16), gamma, beta, bias projection (fp32).  Sources may be bf16 or fp32 and
-// carry any strides (nn.Linear.weight or its transpose).
+// Parameters the kernels cannot read where they are (fp32, [in, out], any other strides), laid out for one call:
+// W4 [4 C, C] = q, k, v, gate rows, Wo [C, C] (rows = output channels, bf16), gamma, beta, bias projection (fp32).
+// Latency-bound (C = 384: 1.2 MB in and out), so one tile of 64 x 64 per block, read along the source's unit stride
+// and turned in shared memory: `[in, out]` weights read along `in` would touch a sector per element.
 struct PackMatrix { const void* src; long long so, si; int f32; };   // element (out, in) at so * out + si * in
 struct PackParams {
   PackMatrix w[5];         // q, k, v, gate, output projection (src == nullptr: absent)
   PackMatrix bias_w;       // [Hb, C]; src == nullptr: absent
-  const void* gamma; const void* beta; int gamma_f32, beta_f32;
+  const void* gamma; const void* beta; int ln_f32;
   int C, Hb;
-  __nv_bfloat16* w4; __nv_bfloat16* wo; float* vec;    // vec: gamma [C], beta [C], bias_w [Hb, C]
+  __nv_bfloat16* w4; __nv_bfloat16* wo; float* vec;    // vec: gamma [C], beta [C], bias_w [Hb, C]; null: none
 };
-__device__ __forceinline__ float pack_at(const void* src, long long i, int f32) {
-  return f32 ? static_cast<const float*>(src)[i] : __bfloat162float(static_cast<const __nv_bfloat16*>(src)[i]);
-}
-__global__ void grid_pack_kernel(const __grid_constant__ PackParams p) {
-  const int C = p.C, n_mat = 5 * C * C, n = n_mat + (2 + p.Hb) * C;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-    if (e < n_mat) {
-      const int m = e / (C * C), r = e % (C * C) / C, c = e % C;
-      if (p.w[m].src == nullptr) continue;
-      const __nv_bfloat16 v = __float2bfloat16_rn(pack_at(p.w[m].src, p.w[m].so * r + p.w[m].si * c, p.w[m].f32));
-      if (m < 4) p.w4[(m * C + r) * C + c] = v; else p.wo[r * C + c] = v;
-    } else {
-      const int v = (e - n_mat) / C, c = e % C;
-      if (v == 0) { if (p.gamma) p.vec[c] = pack_at(p.gamma, c, p.gamma_f32); }
-      else if (v == 1) { if (p.beta) p.vec[C + c] = pack_at(p.beta, c, p.beta_f32); }
-      else p.vec[v * C + c] = pack_at(p.bias_w.src, p.bias_w.so * (v - 2) + p.bias_w.si * c, p.bias_w.f32);
+constexpr int kPackTile = 64, kPackThreads = 256;
+// blockIdx = (tile along in, tile along out, matrix); blockIdx.z == 5: the vectors
+__global__ void __launch_bounds__(kPackThreads) grid_pack_kernel(const __grid_constant__ PackParams p) {
+  __shared__ __nv_bfloat16 tile[kPackTile][kPackTile + 2];
+  const int C = p.C, m = blockIdx.z;
+  grid_wait_previous();
+  grid_release_next();
+  if (m == 5) {
+    if (blockIdx.x != 0 || blockIdx.y != 0) return;
+    for (int e = threadIdx.x; e < (2 + p.Hb) * C; e += kPackThreads) {
+      const int v = e / C, c = e % C;
+      const void* src = v == 0 ? p.gamma : (v == 1 ? p.beta : p.bias_w.src);
+      if (src == nullptr) continue;
+      float x[1];
+      params_at(src, v < 2 ? c : p.bias_w.so * (v - 2) + p.bias_w.si * c, v < 2 ? p.ln_f32 : p.bias_w.f32, x);
+      p.vec[e] = x[0];
     }
+    return;
+  }
+  const PackMatrix w = p.w[m];
+  if (w.src == nullptr) return;
+  const int r0 = blockIdx.y * kPackTile, c0 = blockIdx.x * kPackTile;
+  const bool along_out = w.so == 1 && w.si != 1;
+  const int fast = threadIdx.x % kPackTile, slow = threadIdx.x / kPackTile;
+  constexpr int kStep = kPackThreads / kPackTile, kEach = kPackTile / kStep;
+  // all of a thread's loads in flight at once: the type is looked at outside the loop
+  auto load = [&](const auto* src) {
+    std::remove_const_t<std::remove_reference_t<decltype(*src)>> v[kEach];
+#pragma unroll
+    for (int i = 0; i < kEach; ++i) {
+      const int r = r0 + (along_out ? fast : slow + i * kStep), c = c0 + (along_out ? slow + i * kStep : fast);
+      if (r < C && c < C) v[i] = src[w.so * r + w.si * c];
+    }
+#pragma unroll
+    for (int i = 0; i < kEach; ++i) {
+      const int r = along_out ? fast : slow + i * kStep, c = along_out ? slow + i * kStep : fast;
+      tile[r][c] = (__nv_bfloat16)v[i];     // rounded to nearest
+    }
+  };
+  if (w.f32) load(static_cast<const float*>(w.src));
+  else       load(static_cast<const __nv_bfloat16*>(w.src));
+  __syncthreads();
+  __nv_bfloat16* dst = m < 4 ? p.w4 + (long long)m * C * C : p.wo;
+#pragma unroll
+  for (int i = 0; i < kPackTile; i += kStep) {
+    const int r = slow + i;
+    if (r0 + r < C && c0 + fast < C) dst[(long long)(r0 + r) * C + c0 + fast] = tile[r][fast];
   }
 }
 

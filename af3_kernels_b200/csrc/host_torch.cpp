@@ -31,7 +31,7 @@ struct Library {
   decltype(&af3k_dot_product_attention) attention = nullptr;
   decltype(&af3k_dot_product_attention_workspace) workspace = nullptr;
   decltype(&af3k_stage_bias) stage_bias = nullptr;
-  decltype(&af3k_grid_front) grid_front = nullptr;
+  decltype(&af3k_grid_front_weights) grid_front = nullptr;
   decltype(&af3k_grid_out) grid_out = nullptr;
   decltype(&af3k_grid_pack) grid_pack = nullptr;
   decltype(&af3k_token_projection) token_projection = nullptr;
@@ -50,7 +50,7 @@ void bind_library(const std::string& path) {
   AF3K_BIND(attention, af3k_dot_product_attention);
   AF3K_BIND(workspace, af3k_dot_product_attention_workspace);
   AF3K_BIND(stage_bias, af3k_stage_bias);
-  AF3K_BIND(grid_front, af3k_grid_front);
+  AF3K_BIND(grid_front, af3k_grid_front_weights);
   AF3K_BIND(grid_out, af3k_grid_out);
   AF3K_BIND(grid_pack, af3k_grid_pack);
   AF3K_BIND(token_projection, af3k_token_projection);
@@ -277,96 +277,67 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
   return f32_result ? out.to(at::kFloat) : out;
 }
 
-// ------------------------------------------------------------------ packed block weights
-// A block's parameters laid out for its kernels (bf16 matrices with output rows, fp32 vectors): made in one
-// launch, used again while the same storages are alive and unmodified.  Sixteen blocks' worth is kept
-// (C = 128: 164 KB each), the least recently used one goes first, those of dead parameters with the next
-// one made.
-struct ParamId {
-  c10::weak_intrusive_ptr<c10::StorageImpl> storage;
-  int64_t version, offset;
-  std::vector<int64_t> strides;
-  at::ScalarType dtype;
-  explicit ParamId(const Tensor& t)
-      : storage(t.storage().getWeakStorageImpl()), version(t._version()), offset(t.storage_offset()), strides(t.strides().vec()), dtype(t.scalar_type()) {}
-  bool is(const Tensor& t) const {
-    return !storage.expired() && storage._unsafe_get_target() == t.storage().unsafeGetStorageImpl() && version == (int64_t)t._version() &&
-           offset == t.storage_offset() && t.strides() == at::IntArrayRef(strides) && dtype == t.scalar_type();
-  }
-};
+// ------------------------------------------------------------------ block parameters
+// Every call reads the parameters as they are then.  Nothing made from them is kept between calls: a copy found again
+// by storage and version misses writes that bump no counter (p.data.copy_(), a collective or a kernel on the raw
+// pointer), and a captured graph would replay it after it was given up or had become old.
+int32_t dtype_code(const Tensor& t) { return t.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16; }
 
-struct Packed {
-  std::vector<ParamId> of;
-  Tensor w4, wo, vec;
-  at::cuda::CUDAEvent made;
-  std::vector<c10::StreamId> ordered;
-};
-std::mutex g_packed_mu;
-std::list<Packed>* g_packed = new std::list<Packed>();
-constexpr size_t kPackedMost = 16;
+Tensor kernel_dtype(const Tensor& t) {      // bf16 or fp32, without a gradient
+  const Tensor x = t.detach();
+  return x.scalar_type() == at::kFloat || x.scalar_type() == at::kBFloat16 ? x : x.to(at::kFloat);
+}
 
-// params: q, k, v, gate and perhaps output projection [C, C] as (out, in) matrices, then (all or none) LayerNorm
-// weight and bias [C], bias projection [Hb, C]
-Packed packed_weights(const std::vector<Tensor>& params, int64_t C) {
-  const at::Device dev = params[0].device();
-  const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
-  const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
-  bool cacheable = true;
-  for (const Tensor& t : params) cacheable = cacheable && !t.is_inference();
-  std::lock_guard<std::mutex> lock(g_packed_mu);
-  if (cacheable) {
-    for (auto it = g_packed->begin(); it != g_packed->end(); ++it) {
-      bool same = it->of.size() == params.size();
-      for (size_t i = 0; same && i < params.size(); ++i) same = it->of[i].is(params[i]);
-      if (!same) continue;
-      if (std::find(it->ordered.begin(), it->ordered.end(), stream.id()) == it->ordered.end()) {
-        if (capturing) break;
-        it->made.block(stream);
-        for (const Tensor* t : {&it->w4, &it->wo, &it->vec}) c10::cuda::CUDACachingAllocator::recordStream(t->storage().data_ptr(), stream);
-        it->ordered.push_back(stream.id());
-      }
-      if (it != g_packed->begin()) g_packed->splice(g_packed->begin(), *g_packed, it);
-      Packed r;
-      r.w4 = it->w4; r.wo = it->wo; r.vec = it->vec;
-      return r;
-    }
-  }
-  const bool with_ln = params.size() > 5;
-  const int64_t Hb = with_ln ? params[7].size(0) : 0;
+void matrices(const std::vector<Tensor>& w, int64_t C) {
+  for (const Tensor& t : w)
+    if (t.dim() != 2 || t.size(0) != C || t.size(1) != C) value_error("projection weights must be [C, C]");
+}
+
+// q, k, v, gate and perhaps output projection [C, C] as (out, in) matrices, in the kernels' layout: one launch
+// -> [4 C or 5 C, C] bf16
+Tensor packed_matrices(const std::vector<Tensor>& w, int64_t C, cudaStream_t stream) {
   std::vector<Tensor> src;
-  for (const Tensor& t : params) {
-    Tensor x = t.detach();
-    if (x.device() != dev || (x.scalar_type() != at::kFloat && x.scalar_type() != at::kBFloat16)) x = x.to(dev, at::kFloat);
-    src.push_back(x);
+  af3k_matrix w5[5] = {};
+  for (size_t i = 0; i < w.size(); ++i) {
+    src.push_back(kernel_dtype(w[i]));
+    w5[i] = af3k_matrix{src[i].data_ptr(), src[i].stride(0), src[i].stride(1), dtype_code(src[i])};
   }
-  if (with_ln) {
-    if (src[5].scalar_type() != src[6].scalar_type()) { src[5] = src[5].to(at::kFloat); src[6] = src[6].to(at::kFloat); }
-    src[5] = src[5].contiguous(); src[6] = src[6].contiguous();
+  Tensor packed = at::empty({(int64_t)w.size() * C, C}, src[0].options().dtype(at::kBFloat16));
+  char* p = static_cast<char*>(packed.data_ptr());
+  check(g_lib.grid_pack(w5, nullptr, nullptr, nullptr, AF3K_F32, C, 0, p, w.size() > 4 ? p + 4 * C * C * 2 : nullptr, nullptr, stream));
+  return packed;
+}
+
+// The grid block's parameters: matrices q, k, v, gate, output as [out, in], read where they are if the kernels can
+// (nn.Linear.weight in bf16), else packed for this call; then (all or none) LayerNorm weight and bias, bias projection.
+struct GridParameters {
+  af3k_front_weights front{};
+  const void* wo = nullptr;
+  std::vector<Tensor> keep;
+};
+GridParameters grid_parameters(const std::vector<Tensor>& params, int64_t C, cudaStream_t stream) {
+  GridParameters r;
+  r.front.ln_dtype = r.front.bias_w_dtype = AF3K_F32;
+  const void* m[5];
+  bool in_place = true;
+  for (int i = 0; i < 5; ++i) {
+    m[i] = params[i].data_ptr();
+    in_place = in_place && params[i].scalar_type() == at::kBFloat16 && params[i].is_contiguous() && reinterpret_cast<uintptr_t>(m[i]) % 16 == 0;
   }
-  auto dtype_of = [](const Tensor& t) { return t.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16; };
-  auto matrix = [&](const Tensor& t) { return af3k_matrix{t.data_ptr(), t.stride(0), t.stride(1), dtype_of(t)}; };
-  af3k_matrix w5[5], bw{};
-  for (int i = 0; i < 5; ++i) w5[i] = i < (int)src.size() ? matrix(src[i]) : af3k_matrix{};
-  if (with_ln) bw = matrix(src[7]);
-  Packed e;
-  const auto options = at::TensorOptions().device(dev);
-  e.w4 = at::empty({4 * C, C}, options.dtype(at::kBFloat16));
-  e.wo = at::empty({params.size() > 4 ? C : 0, C}, options.dtype(at::kBFloat16));
-  e.vec = at::empty({(2 + Hb) * C}, options.dtype(at::kFloat));
-  check(g_lib.grid_pack(w5, with_ln ? &bw : nullptr, with_ln ? src[5].data_ptr() : nullptr, with_ln ? src[6].data_ptr() : nullptr,
-                        with_ln ? dtype_of(src[5]) : AF3K_F32, C, Hb, e.w4.data_ptr(), e.wo.data_ptr(), e.vec.data_ptr<float>(), stream));
-  Packed r;
-  r.w4 = e.w4; r.wo = e.wo; r.vec = e.vec;
-  if (!cacheable || capturing) return r;
-  g_packed->remove_if([](const Packed& o) {
-    for (const ParamId& id : o.of) if (id.storage.expired()) return true;
-    return false;
-  });
-  while (g_packed->size() >= kPackedMost) g_packed->pop_back();
-  for (const Tensor& t : params) e.of.emplace_back(t);
-  e.made.record(stream);
-  e.ordered.push_back(stream.id());
-  g_packed->push_front(std::move(e));
+  if (!in_place) {
+    r.keep.push_back(packed_matrices({params.begin(), params.begin() + 5}, C, stream));
+    for (int i = 0; i < 5; ++i) m[i] = static_cast<char*>(r.keep[0].data_ptr()) + i * C * C * 2;
+  }
+  for (int i = 0; i < 4; ++i) r.front.w[i] = m[i];
+  r.wo = m[4];
+  if (params.size() > 5) {
+    Tensor gamma = kernel_dtype(params[5]), beta = kernel_dtype(params[6]), bw = kernel_dtype(params[7]).contiguous();
+    if (gamma.scalar_type() != beta.scalar_type()) { gamma = gamma.to(at::kFloat); beta = beta.to(at::kFloat); }
+    gamma = gamma.contiguous(); beta = beta.contiguous();
+    r.front.gamma = gamma.data_ptr(); r.front.beta = beta.data_ptr(); r.front.bias_w = bw.data_ptr();
+    r.front.ln_dtype = dtype_code(gamma); r.front.bias_w_dtype = dtype_code(bw);
+    r.keep.insert(r.keep.end(), {gamma, beta, bw});
+  }
   return r;
 }
 
@@ -376,12 +347,6 @@ bool grid_fused(const Tensor& pair, int64_t head, int64_t bias_heads) {
   const int64_t C = pair.size(2);
   return (C == 64 || C == 128) && head > 0 && C % head == 0 && (C / head) % 8 == 0 && bias_heads <= 4 &&
          (pair.scalar_type() == at::kBFloat16 || pair.scalar_type() == at::kFloat);
-}
-
-std::vector<Tensor> matrices(const std::vector<Tensor>& w, int64_t C) {
-  for (const Tensor& t : w)
-    if (t.dim() != 2 || t.size(0) != C || t.size(1) != C) value_error("projection weights must be [C, C]");
-  return w;
 }
 
 // The whole module: raw pair [N, N, C] -> front (LayerNorm, bias, q / k / v / gate) -> attention -> gate and output
@@ -401,8 +366,8 @@ Tensor grid_module(Tensor pair, const Tensor& mask_in, const std::vector<Tensor>
   Tensor mask = mask_in.device() == dev ? mask_in.contiguous() : mask_in.to(dev).contiguous();
   if (mask.size(-1) != N || (mask.dim() == 2 && mask.size(0) != 1 && mask.size(0) != N))
     value_error("mask of shape " + shape_text(mask) + " does not match B1=" + std::to_string(N) + ", Sk=" + std::to_string(N));
-  const Packed w = packed_weights(params, C);
-  const float* vec = w.vec.data_ptr<float>();
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  const GridParameters w = grid_parameters(params, C, stream);
   const auto bf16 = pair.options().dtype(at::kBFloat16);
   const int64_t pitch = (N + 7) / 8 * 8;
   Tensor bias = at::empty({head, N, pitch}, bf16);
@@ -413,9 +378,8 @@ Tensor grid_module(Tensor pair, const Tensor& mask_in, const std::vector<Tensor>
   void *q = b, *k = b + part, *v = b + 2 * part, *gate = b + 3 * part, *weighted = b + 4 * part;
   const bool f32 = pair.scalar_type() == at::kFloat;
   int* status = status_buffer(dev.index()).data_ptr<int>();
-  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
-  check(g_lib.grid_front(pair.data_ptr(), f32 ? AF3K_F32 : AF3K_BF16, vec, vec + C, (float)eps, vec + 2 * C, head, w.w4.data_ptr(), R, N,
-                         C, head, 1.0f / std::sqrt((float)D), transpose, bias.data_ptr(), pitch, q, k, v, gate, status, stream));
+  check(g_lib.grid_front(pair.data_ptr(), f32 ? AF3K_F32 : AF3K_BF16, &w.front, (float)eps, head, R, N, C, head,
+                         1.0f / std::sqrt((float)D), transpose, bias.data_ptr(), pitch, q, k, v, gate, status, stream));
   af3k_attention_desc d{};
   d.B1 = N; d.B2 = head; d.Sq = N; d.Sk = N; d.D = D;
   for (int64_t* st : {d.q_stride, d.k_stride, d.v_stride}) { st[0] = head * N * D; st[1] = N * D; st[2] = D; }
@@ -426,7 +390,7 @@ Tensor grid_module(Tensor pair, const Tensor& mask_in, const std::vector<Tensor>
   d.softmax_scale = 1.0f;                            // q left the projection scaled
   check(g_lib.attention(&d, q, k, v, bias.data_ptr(), static_cast<const uint8_t*>(mask.data_ptr()), weighted, nullptr, nullptr, nullptr, 0,
                         status, stream));
-  check(g_lib.grid_out(weighted, gate, w.wo.data_ptr(), out.data_ptr(), f32 ? AF3K_F32 : AF3K_BF16, M, C, status, stream));
+  check(g_lib.grid_out(weighted, gate, w.wo, out.data_ptr(), f32 ? AF3K_F32 : AF3K_BF16, M, C, status, stream));
   return out;
 }
 
@@ -439,18 +403,18 @@ Tensor grid_block(const Tensor& pair, const OptTensor& mask, const Tensor& bias,
   matrices(weights, C);
   Tensor x = pair.to(at::kBFloat16).contiguous();
   if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0) x = x.clone();
-  const Packed w = packed_weights(weights, C);
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  const GridParameters w = grid_parameters(weights, C, stream);
   Tensor buf = at::empty({5, M, C}, x.options());
   auto at_part = [&](int i, at::IntArrayRef sizes) { return buf.select(0, i).view(sizes); };
   Tensor q = at_part(0, {R, head, N, D}), k = at_part(1, {R, head, N, D}), v = at_part(2, {R, head, N, D});
   Tensor gate = at_part(3, {M, C}), weighted = at_part(4, {R, N, head, D});
   Tensor out = at::empty({R, N, C}, x.options().dtype(pair.scalar_type()));
   int* status = status_buffer(dev.index()).data_ptr<int>();
-  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
-  check(g_lib.grid_front(x.data_ptr(), AF3K_BF16, nullptr, nullptr, 0.f, nullptr, 0, w.w4.data_ptr(), R, N, C, head, 1.0f / std::sqrt((float)D), 0,
-                         nullptr, 0, q.data_ptr(), k.data_ptr(), v.data_ptr(), gate.data_ptr(), status, stream));
+  check(g_lib.grid_front(x.data_ptr(), AF3K_BF16, &w.front, 0.f, 0, R, N, C, head, 1.0f / std::sqrt((float)D), 0, nullptr, 0, q.data_ptr(),
+                         k.data_ptr(), v.data_ptr(), gate.data_ptr(), status, stream));
   attention(q, k, v, mask, bias, std::nullopt, std::nullopt, 1.0, 0, weighted.permute({0, 2, 1, 3}), true, true, 0, 0);
-  check(g_lib.grid_out(weighted.data_ptr(), gate.data_ptr(), w.wo.data_ptr(), out.data_ptr(), pair.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16,
+  check(g_lib.grid_out(weighted.data_ptr(), gate.data_ptr(), w.wo, out.data_ptr(), pair.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16,
                        M, C, status, stream));
   return out;
 }
@@ -471,7 +435,8 @@ Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, con
   if (N == 0) return at::empty({N, C}, x_in.options());
   if (q_bias.device() != dev || (q_bias.scalar_type() != at::kBFloat16 && q_bias.scalar_type() != at::kFloat)) q_bias = q_bias.to(dev, at::kFloat);
   q_bias = q_bias.contiguous();
-  const Packed w = packed_weights(weights, C);
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  const Tensor w4 = packed_matrices(weights, C, stream);
   const float scale = 1.0f / std::sqrt((float)D);
   const bool in_place = bias.scalar_type() == at::kBFloat16 && bias.dim() == 3 && bias.stride(2) == 1 && (bias.stride(1) * 2) % 16 == 0 &&
                         (bias.stride(0) * 2) % 16 == 0 && (bias.stride(0) != 0 || head == 1) && (bias.stride(1) != 0 || N == 1) &&
@@ -486,8 +451,7 @@ Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, con
   char* b = static_cast<char*>(qkvg.data_ptr());
   const size_t part = (size_t)N * C * 2;
   int* status = status_buffer(dev.index()).data_ptr<int>();
-  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
-  check(g_lib.token_projection(x.data_ptr(), w.w4.data_ptr(), q_bias.data_ptr(), q_bias.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16, N, C,
+  check(g_lib.token_projection(x.data_ptr(), w4.data_ptr(), q_bias.data_ptr(), q_bias.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16, N, C,
                                scale, b, status, stream));
   af3k_attention_desc d{};
   d.B1 = 1; d.B2 = head; d.Sq = N; d.Sk = N; d.D = D;

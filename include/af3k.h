@@ -250,6 +250,21 @@ int af3k_grid_front(const void* pair, int32_t pair_dtype, const float* gamma, co
                     float q_scale, int32_t transpose, void* bias, int64_t bias_pitch, void* q, void* k, void* v,
                     void* gate, int* status_dev, void* stream);
 
+/* The same front with the parameters where their owner keeps them (a module's nn.Linear / nn.LayerNorm tensors):
+ * nothing is laid out first, and the call sees the values they hold when it runs.  gamma NULL: no LayerNorm (beta
+ * ignored, Hb 0).  The four matrices are [C, C] bf16, output rows, contiguous, 16-byte aligned; the vectors and
+ * bias_w [Hb, C] are contiguous, bf16 or fp32. */
+typedef struct af3k_front_weights {
+  const void* w[4];                 /* q, k, v, gate */
+  const void *gamma, *beta;         /* [C], both of ln_dtype */
+  const void* bias_w;
+  int32_t ln_dtype, bias_w_dtype;
+} af3k_front_weights;
+int af3k_grid_front_weights(const void* pair, int32_t pair_dtype, const af3k_front_weights* weights, float eps,
+                            int64_t Hb, int64_t R, int64_t N, int64_t C, int64_t H, float q_scale, int32_t transpose,
+                            void* bias, int64_t bias_pitch, void* q, void* k, void* v, void* gate, int* status_dev,
+                            void* stream);
+
 /* The end of the block in one pass:  out = (weighted * sigmoid(gate)) Wo^T.
  * Stands in for the SigmoidFwdTPP + MulTPP pair and the output projection BRGEMM of the reference's fused
  * block (src/csrc/dot_product_attention.cpp:339-372).
@@ -275,9 +290,10 @@ typedef struct af3k_matrix {
   int32_t dtype;
 } af3k_matrix;
 
-/* Lays a block's parameters out for af3k_grid_front / af3k_grid_out in one launch: w5 = q, k, v, gate, output
- * projection (data NULL: there is none, wo is not written) -> w4 [4 C, C] and wo [C, C] bf16;  gamma, beta (both of ln_dtype, may be NULL) and bias_w [Hb, C]
- * (NULL with Hb 0) -> vec: fp32 gamma [C], beta [C], bias_w [Hb, C].  No counterpart in the reference (which
+/* Lays a block's parameters out for af3k_grid_front / af3k_grid_out / af3k_token_projection in one launch: w5 = q, k,
+ * v, gate, output projection (data NULL: there is none, wo is not written) -> w4 [4 C, C] and wo [C, C] bf16;  gamma,
+ * beta (both of ln_dtype, may be NULL) and bias_w [Hb, C] (NULL with Hb 0) -> vec: fp32 gamma [C], beta [C],
+ * bias_w [Hb, C] (NULL if there is none of the three).  No counterpart in the reference (which
  * repacks its weights for its CPU GEMM, src/csrc/tools.cpp:151-176). */
 int af3k_grid_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void* gamma, const void* beta,
                    int32_t ln_dtype, int64_t C, int64_t Hb, void* w4, void* wo, float* vec, void* stream);

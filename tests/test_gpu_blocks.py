@@ -312,3 +312,85 @@ def test_kernels_that_start_under_the_previous_ones_wait_for_them(cuda_device, N
     for i, r in enumerate(got):
         assert torch.equal(r, want), i
     assert read_status(cuda_device)[0] == 0
+
+
+def _block_calls(kind, C, dtype, device, seed):
+    """-> (parameters, call): one block of the given kind and a call of it on fixed inputs."""
+    g = torch.Generator().manual_seed(seed)
+    H, N = 4, 72
+    normal = lambda *s, std=1.0: (torch.randn(*s, generator=g) * std).to(device, dtype)
+    mask = (torch.rand(N, N, generator=g) >= 0.1).to(device)
+    if kind == "module":
+        m = A.GridSelfAttentionCpp(C, H, bool(seed % 2)).to(device, dtype).eval()
+        pair = normal(N, N, C)
+        params = list(m.parameters())
+        with torch.no_grad():
+            for p in params:
+                p.copy_(normal(*p.shape, std=C ** -0.5 if p.dim() == 2 else 0.3))
+        return params, lambda: m(pair, mask)
+    ws = [normal(C, C, std=C ** -0.5) for _ in range(5)]
+    bias = normal(H, N, N).to(torch.bfloat16)        # read in place: the staged copy of another bias is not the subject
+    if kind == "grid":
+        pair = normal(3, N, C)
+        return ws, lambda: A._attention_cpp(pair, mask[:3], bias, *ws, H)
+    x, qb = normal(N, C), normal(C, std=0.1)
+    return ws[:4] + [qb], lambda: A.self_attention_cpp(x, mask[0], bias, ws[0], qb, *ws[1:4], H)
+
+
+@pytest.mark.parametrize("kind,C,dtype", [("module", 128, torch.bfloat16), ("module", 64, torch.float32), ("grid", 128, torch.float32),
+                                          ("grid", 64, torch.bfloat16), ("self", 64, torch.bfloat16), ("self", 224, torch.float32)])
+def test_blocks_compute_with_the_parameters_as_they_are(cuda_device, kind, C, dtype):
+    """New values are seen by the next call and by the next replay of a graph captured on the stream that was warmed
+    up, however they were written (``.data`` bumps no version counter), and however many other blocks ran since."""
+    with torch.no_grad():
+        params, call = _block_calls(kind, C, dtype, cuda_device, 1)
+        values, want = [], []
+        for seed in (1, 2, 3):
+            p, c = _block_calls(kind, C, dtype, cuda_device, 1)
+            for i, t in enumerate(p):
+                t.copy_(torch.randn(t.shape, generator=torch.Generator().manual_seed(10 * seed + i)) * C ** -0.5)
+            values.append([t.clone() for t in p])
+            want.append(c())
+
+        def load(i):
+            for t, v in zip(params, values[i]):
+                t.data.copy_(v)
+
+        load(0)
+        assert torch.equal(call(), want[0])
+        load(1)
+        assert torch.equal(call(), want[1])
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            call()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=side):
+                out = call()
+        torch.cuda.current_stream().wait_stream(side)
+        keep = []
+        for seed in range(20):
+            keep.append(_block_calls(kind, C, dtype, cuda_device, 100 + seed))
+            keep[-1][1]()
+        for i in (1, 2, 0):
+            for t, v in zip(params, values[i]):
+                t.copy_(v)
+            graph.replay()
+            assert torch.equal(out, want[i]), i
+        torch.cuda.synchronize()
+    assert read_status(cuda_device)[0] == 0
+
+
+def test_a_part_of_the_weights_is_not_taken_for_the_whole(cuda_device):
+    """Views that differ in their extent only: a block on the corner of a larger block's weights."""
+    g = torch.Generator().manual_seed(8)
+    H, N = 4, 40
+    ws = [(torch.randn(256, 256, generator=g) * 0.1).to(cuda_device, torch.bfloat16) for _ in range(4)]
+    for C in (256, 128):
+        x = torch.randn(N, C, generator=g).to(torch.bfloat16)
+        bias = torch.randn(H, N, N, generator=g).to(torch.bfloat16)
+        part = [w[:C, :C] for w in ws]
+        qb = torch.zeros(C, dtype=torch.bfloat16)
+        out = A.self_attention_cpp(x.to(cuda_device), None, bias.to(cuda_device), part[0], qb.to(cuda_device), *part[1:], H)
+        cpu = [w.cpu() for w in part]
+        _close(out, O.self_block_fp32(x, torch.ones(N, dtype=torch.bool), bias, cpu[0].T, qb, *(w.T for w in cpu[1:]), H), C)
