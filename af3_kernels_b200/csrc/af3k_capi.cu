@@ -850,47 +850,69 @@ int af3k_grid_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void*
   return AF3K_OK;
 }
 
-int af3k_token_projection(const void* x, const void* w4, const void* q_bias, int32_t q_bias_dtype, int64_t M, int64_t C, float q_scale,
-                          void* out, int* status_dev, void* stream_v) {
+int af3k_token_projection_weights(const void* x, const af3k_matrix* w4, const void* q_bias, int32_t q_bias_dtype, int64_t M, int64_t C,
+                                  float q_scale, void* out, int* status_dev, void* stream_v) {
   t_last_launches = 0;
   if (q_bias && q_bias_dtype != AF3K_BF16 && q_bias_dtype != AF3K_F32) return AF3K_ERR_BAD_DTYPE;
   if (M < 0 || C < 8 || C % 8 != 0 || C > (1 << 20) || M > 0x7fffff00LL) return AF3K_ERR_BAD_SHAPE;
   if (M == 0) return AF3K_OK;
   if (!x || !w4 || !out) return AF3K_ERR_NULL_POINTER;
-  if (!aligned16(x) || !aligned16(w4) || !aligned16(out)) return AF3K_ERR_BAD_ALIGNMENT;
+  if (!aligned16(x) || !aligned16(out)) return AF3K_ERR_BAD_ALIGNMENT;
+  int mn_mask = 0;
+  for (int i = 0; i < 4; ++i) {
+    if (!w4[i].data) return AF3K_ERR_NULL_POINTER;
+    if (w4[i].dtype != AF3K_BF16) return AF3K_ERR_BAD_DTYPE;
+    if (!aligned16(w4[i].data)) return AF3K_ERR_BAD_ALIGNMENT;
+    const bool mn = w4[i].stride_in != 1;
+    const int64_t pitch = mn ? w4[i].stride_in : w4[i].stride_out;
+    if ((mn && w4[i].stride_out != 1) || pitch < C || pitch % 8 != 0 || pitch >= (1LL << 38)) return AF3K_ERR_BAD_STRIDE;
+    mn_mask |= mn << i;
+  }
   DeviceInfo* dev = nullptr;
   int rc = device_info(&dev);
   if (rc != AF3K_OK) return rc;
   const int64_t m_tiles = (M + 127) / 128;
-  const int kn = m_tiles * ((4 * C + 127) / 128) >= dev->sm_count * 3 / 4 ? 128 : 64;   // enough tiles of 128 columns to fill the SMs?
-  const int64_t n_tiles = (4 * C + kn - 1) / kn;
-  if (n_tiles > 65535) return AF3K_ERR_BAD_SHAPE;
+  const int kn = m_tiles * 4 * ((C + 127) / 128) >= dev->sm_count * 3 / 4 ? 128 : 64;   // enough tiles of 128 columns to fill the SMs?
+  const int64_t tiles_n = (C + kn - 1) / kn;
+  if (4 * tiles_n > 65535) return AF3K_ERR_BAD_SHAPE;
   auto enc = tensor_map_encoder();
   if (!enc) return driver_fail("cuTensorMapEncodeTiled entry point", -1);
-  CUtensorMap tm_x, tm_w;
-  auto map = [&](CUtensorMap* tm, const void* base, int64_t rows, int box_rows) {
+  CUtensorMap tm_x;
+  TokMaps maps;
+  auto map = [&](CUtensorMap* tm, const void* base, int64_t rows, int64_t pitch, int box_rows) {
     cuuint64_t dims[2] = {(cuuint64_t)C, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)C * 2};
+    cuuint64_t strides[1] = {(cuuint64_t)pitch * 2};
     cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     return enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   };
-  CUresult r = map(&tm_x, x, M, 128);
-  if (r == CUDA_SUCCESS) r = map(&tm_w, w4, 4 * C, kn);
+  CUresult r = map(&tm_x, x, M, C, 128);
+  for (int i = 0; i < 4 && r == CUDA_SUCCESS; ++i) {
+    const bool mn = (mn_mask >> i) & 1;
+    r = map(&maps.w[i], w4[i].data, C, mn ? w4[i].stride_in : w4[i].stride_out, mn ? 64 : kn);
+  }
   if (r != CUDA_SUCCESS) return driver_fail("cuTensorMapEncodeTiled(token projection)", (int)r);
   TokParams p;
   std::memset(&p, 0, sizeof(p));
-  p.M = (int)M; p.C = (int)C; p.q_bias = q_bias; p.q_bias_f32 = q_bias_dtype == AF3K_F32 ? 1 : 0; p.q_scale = q_scale;
+  p.M = (int)M; p.C = (int)C; p.tiles_n = (int)tiles_n; p.mn_mask = mn_mask;
+  p.q_bias = q_bias; p.q_bias_f32 = q_bias_dtype == AF3K_F32 ? 1 : 0; p.q_scale = q_scale;
   p.out = static_cast<__nv_bfloat16*>(out); p.status = status_dev; p.wait_limit = wait_limit_cycles();
-  const dim3 grid((unsigned)m_tiles, (unsigned)n_tiles);
+  const dim3 grid((unsigned)m_tiles, (unsigned)(4 * tiles_n));
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
-  if (kn == 128) launch_overlapped(token_proj_kernel<128>, grid, kTokThreads, TokTile<128>::kSmem, stream, true, p, tm_x, tm_w);
-  else           launch_overlapped(token_proj_kernel<64>, grid, kTokThreads, TokTile<64>::kSmem, stream, true, p, tm_x, tm_w);
+  if (kn == 128) launch_overlapped(token_proj_kernel<128>, grid, kTokThreads, TokTile<128>::kSmem, stream, true, p, tm_x, maps);
+  else           launch_overlapped(token_proj_kernel<64>, grid, kTokThreads, TokTile<64>::kSmem, stream, true, p, tm_x, maps);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail("launch token_proj_kernel", e);
   t_last_launches = 1;
   return AF3K_OK;
+}
+
+int af3k_token_projection(const void* x, const void* w4, const void* q_bias, int32_t q_bias_dtype, int64_t M, int64_t C, float q_scale,
+                          void* out, int* status_dev, void* stream_v) {
+  af3k_matrix w[4];
+  for (int i = 0; i < 4; ++i) w[i] = af3k_matrix{w4 ? static_cast<const char*>(w4) + (size_t)i * C * C * 2 : nullptr, C, 1, AF3K_BF16};
+  return af3k_token_projection_weights(x, w, q_bias, q_bias_dtype, M, C, q_scale, out, status_dev, stream_v);
 }
 
 int af3k_qkvg_projection(const void* x, const void* w4, int64_t R, int64_t N, int64_t H, float q_scale,

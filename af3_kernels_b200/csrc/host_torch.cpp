@@ -34,7 +34,7 @@ struct Library {
   decltype(&af3k_grid_front_weights) grid_front = nullptr;
   decltype(&af3k_grid_out) grid_out = nullptr;
   decltype(&af3k_grid_pack) grid_pack = nullptr;
-  decltype(&af3k_token_projection) token_projection = nullptr;
+  decltype(&af3k_token_projection_weights) token_projection = nullptr;
 };
 Library g_lib;
 
@@ -53,7 +53,7 @@ void bind_library(const std::string& path) {
   AF3K_BIND(grid_front, af3k_grid_front_weights);
   AF3K_BIND(grid_out, af3k_grid_out);
   AF3K_BIND(grid_pack, af3k_grid_pack);
-  AF3K_BIND(token_projection, af3k_token_projection);
+  AF3K_BIND(token_projection, af3k_token_projection_weights);
 #undef AF3K_BIND
 }
 
@@ -436,7 +436,20 @@ Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, con
   if (q_bias.device() != dev || (q_bias.scalar_type() != at::kBFloat16 && q_bias.scalar_type() != at::kFloat)) q_bias = q_bias.to(dev, at::kFloat);
   q_bias = q_bias.contiguous();
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
-  const Tensor w4 = packed_matrices(weights, C, stream);
+  // weights the kernel can read where they are: bf16, [out, in] or [in, out], rows of 16-byte multiples
+  af3k_matrix w4[4];
+  bool in_place_w = true;
+  for (int i = 0; i < 4; ++i) {
+    const int64_t so = weights[i].stride(0), si = weights[i].stride(1);
+    w4[i] = af3k_matrix{weights[i].data_ptr(), so, si, AF3K_BF16};
+    in_place_w = in_place_w && weights[i].scalar_type() == at::kBFloat16 && reinterpret_cast<uintptr_t>(w4[i].data) % 16 == 0 &&
+                 (so == 1 || si == 1) && std::max(so, si) >= C && std::max(so, si) % 8 == 0;
+  }
+  Tensor packed;
+  if (!in_place_w) {
+    packed = packed_matrices(weights, C, stream);
+    for (int i = 0; i < 4; ++i) w4[i] = af3k_matrix{static_cast<char*>(packed.data_ptr()) + i * C * C * 2, C, 1, AF3K_BF16};
+  }
   const float scale = 1.0f / std::sqrt((float)D);
   const bool in_place = bias.scalar_type() == at::kBFloat16 && bias.dim() == 3 && bias.stride(2) == 1 && (bias.stride(1) * 2) % 16 == 0 &&
                         (bias.stride(0) * 2) % 16 == 0 && (bias.stride(0) != 0 || head == 1) && (bias.stride(1) != 0 || N == 1) &&
@@ -451,7 +464,7 @@ Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, con
   char* b = static_cast<char*>(qkvg.data_ptr());
   const size_t part = (size_t)N * C * 2;
   int* status = status_buffer(dev.index()).data_ptr<int>();
-  check(g_lib.token_projection(x.data_ptr(), w4.data_ptr(), q_bias.data_ptr(), q_bias.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16, N, C,
+  check(g_lib.token_projection(x.data_ptr(), w4, q_bias.data_ptr(), q_bias.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16, N, C,
                                scale, b, status, stream));
   af3k_attention_desc d{};
   d.B1 = 1; d.B2 = head; d.Sq = N; d.Sk = N; d.D = D;

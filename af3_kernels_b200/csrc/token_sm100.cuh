@@ -1,6 +1,10 @@
 // The four projections of the single / diffusion attention block in one GEMM, for sm_100a:
 //
-//     [q | k | v | gate] = x [M, C] * W4^T,   q <- (q + q_bias) * q_scale,     W4 = [Wq; Wk; Wv; Wg] ([4 C, C])
+//     [q | k | v | gate] = x [M, C] * [Wq; Wk; Wv; Wg]^T,   q <- (q + q_bias) * q_scale
+//
+// The weights are read where their owner keeps them, `[out, in]` as a K-major B operand or `[in, out]` as an MN-major
+// one (64-column blocks of 64 K rows, so that either fills a stage): laying them out in a pass of its own took 4.5 us of
+// the 49 of a call at 1536 tokens and C = 384, and a copy kept between calls could be out of date.
 //
 // Stands in for the projection BRGEMMs of the reference's fused block
 // (src/csrc/dot_product_attention.cpp:425-480).  M is a token count (tens to a few thousand), C 384 or 768
@@ -23,8 +27,11 @@ template <int kN> struct TokTile {
   static constexpr uint32_t off_bar = kTokStages * kStage, kSmem = off_bar + 128;
 };
 
+struct TokMaps { CUtensorMap w[4]; };
 struct TokParams {
   int M, C;
+  int tiles_n;               // column tiles of one matrix; a tile never straddles two
+  int mn_mask;               // bit i: matrix i is kept [in, out]
   const void* q_bias;        // [C] bf16 or fp32, may be null
   int q_bias_f32;
   float q_scale;
@@ -36,14 +43,17 @@ struct TokParams {
 template <int kN>
 __global__ void __launch_bounds__(kTokThreads, 1)
 token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ CUtensorMap tm_x,
-                  const __grid_constant__ CUtensorMap tm_w) {
+                  const __grid_constant__ TokMaps maps) {
   using Tile = TokTile<kN>;
   extern __shared__ __align__(1024) uint8_t tok_smem[];
   const uint32_t smem = smem_u32(tok_smem), bars = smem + Tile::off_bar;   // full [6], empty [6], acc
   volatile uint32_t* slot = reinterpret_cast<volatile uint32_t*>(tok_smem + Tile::off_bar + 112);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tok_smem + Tile::off_bar + 116);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * 128, n0 = blockIdx.y * kN, kblocks = (p.C + 63) / 64;
+  const int which = blockIdx.y / p.tiles_n;                    // 0 q, 1 k, 2 v, 3 gate
+  const int m0 = blockIdx.x * 128, n0 = (blockIdx.y - which * p.tiles_n) * kN, kblocks = (p.C + 63) / 64;
+  const bool mn = (p.mn_mask >> which) & 1;
+  const CUtensorMap* tm_w = maps.w + which;
   auto timeout = [&](int bar) {
     *abort_flag = 1;
     if (p.status != nullptr) {
@@ -54,7 +64,7 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     prefetch_tensormap(&tm_x);
-    prefetch_tensormap(&tm_w);
+    prefetch_tensormap(tm_w);
     for (int i = 0; i < 2 * kTokStages + 1; ++i) mbar_init(bars + 8u * i, 1);
     fence_barrier_init();
   }
@@ -80,14 +90,21 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
         const uint32_t full = bars + 8u * st, dst = smem + st * Tile::kStage;
         mbar_arrive_expect_tx(full, Tile::kStage);
         tma_load_2d(dst, &tm_x, full, kb * 64, m0);
-        tma_load_2d(dst + Tile::kA, &tm_w, full, kb * 64, n0);
+        if (!mn) {
+          tma_load_2d(dst + Tile::kA, tm_w, full, kb * 64, n0);
+        } else {
+          for (int j = 0; j < kN; j += 64) tma_load_2d(dst + Tile::kA + j * 128, tm_w, full, n0 + j, kb * 64);
+        }
       }
     }
   } else if (warp == 1) {
     const bool leader = elect_one();
-    const uint32_t idesc = make_idesc(1u, 1u, 0u, 0u, kN);
-    const uint64_t d0 = make_smem_desc(smem, 16, 8 * 128, 2);
-    const uint32_t lo = (uint32_t)d0, hi = (uint32_t)(d0 >> 32);
+    const uint32_t idesc = make_idesc(1u, 1u, 0u, mn ? 1u : 0u, kN);
+    // B: K-major, 16 channels = 32 bytes along the 128-byte rows; MN-major, 16 rows of 128 bytes (64 columns), the next
+    // 64 columns 64 rows on
+    const uint64_t d0 = make_smem_desc(smem, 16, 8 * 128, 2), b0 = make_smem_desc(smem, mn ? 64 * 128 : 16, 8 * 128, 2);
+    const uint32_t lo = (uint32_t)d0, hi = (uint32_t)(d0 >> 32), b_lo = (uint32_t)b0, b_hi = (uint32_t)(b0 >> 32);
+    const uint32_t b_step = mn ? (16 * 128) >> 4 : 2;
     bool ok = true;
     for (int kb = 0; kb < kblocks && ok; ++kb) {
       const int st = kb % kTokStages;
@@ -96,9 +113,9 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
       if (!ok) { timeout(st); break; }
       tc_fence_after();
       if (leader) {
-        const uint32_t a = lo + ((st * Tile::kStage) >> 4), b = a + (Tile::kA >> 4);
+        const uint32_t a = lo + ((st * Tile::kStage) >> 4), b = b_lo + ((st * Tile::kStage + Tile::kA) >> 4);
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) mma_ss_f16(tmem, a + 2 * ks, hi, b + 2 * ks, hi, idesc, kb + ks > 0 ? 1u : 0u);
+        for (int ks = 0; ks < 4; ++ks) mma_ss_f16(tmem, a + 2 * ks, hi, b + b_step * ks, b_hi, idesc, kb + ks > 0 ? 1u : 0u);
         tc_commit(bars + 8u * (kTokStages + st));
         if (kb == kblocks - 1) tc_commit(bars + 8u * (2 * kTokStages));
       }
@@ -120,7 +137,7 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
           tmem_ld_x32(t_base + c0 + 32 * hc, acc);
           tc_wait_ld();
           const int col = n0 + c0 + 32 * hc;
-          if (col < p.C) {             // (some) q columns
+          if (which == 0) {
 #pragma unroll
             for (int e = 0; e < 32; ++e) {
               if (col + e < p.C) {
@@ -142,11 +159,10 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
                          "r"(pack_bf16x2(__uint_as_float(acc[8 * j + 6]), __uint_as_float(acc[8 * j + 7]))) : "memory");
         }
         __syncwarp();
-        // shared -> global: lane l takes piece l & 7 of rows (l >> 3) + 4 it; eight columns never straddle outputs
+        // shared -> global: lane l takes piece l & 7 of rows (l >> 3) + 4 it; C is a multiple of eight
         const int col = n0 + c0 + 8 * (lane & 7);
-        if (col < 4 * p.C) {
-          const int which = col / p.C;
-          __nv_bfloat16* dst = p.out + ((long long)which * p.M) * p.C + (col - which * p.C);
+        if (col < p.C) {
+          __nv_bfloat16* dst = p.out + ((long long)which * p.M) * p.C + col;
 #pragma unroll
           for (int it = 0; it < 8; ++it) {
             const int row = it * 4 + (lane >> 3), m = m0 + quarter * 32 + row;

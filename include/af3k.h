@@ -290,6 +290,12 @@ typedef struct af3k_matrix {
   int32_t dtype;
 } af3k_matrix;
 
+/* af3k_token_projection with the four weights where their owner keeps them: bf16, 16-byte aligned, one stride 1 ([out, in]
+ * or [in, out], each matrix on its own) and the other a multiple of 8 and at least C.  The call sees the values they hold
+ * when it runs. */
+int af3k_token_projection_weights(const void* x, const af3k_matrix* w4, const void* q_bias, int32_t q_bias_dtype, int64_t M,
+                                  int64_t C, float q_scale, void* out, int* status_dev, void* stream);
+
 /* Lays a block's parameters out for af3k_grid_front / af3k_grid_out / af3k_token_projection in one launch: w5 = q, k,
  * v, gate, output projection (data NULL: there is none, wo is not written) -> w4 [4 C, C] and wo [C, C] bf16;  gamma,
  * beta (both of ln_dtype, may be NULL) and bias_w [Hb, C] (NULL with Hb 0) -> vec: fp32 gamma [C], beta [C],

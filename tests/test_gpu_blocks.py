@@ -394,3 +394,41 @@ def test_a_part_of_the_weights_is_not_taken_for_the_whole(cuda_device):
         out = A.self_attention_cpp(x.to(cuda_device), None, bias.to(cuda_device), part[0], qb.to(cuda_device), *part[1:], H)
         cpu = [w.cpu() for w in part]
         _close(out, O.self_block_fp32(x, torch.ones(N, dtype=torch.bool), bias, cpu[0].T, qb, *(w.T for w in cpu[1:]), H), C)
+
+
+@pytest.mark.parametrize("N,C,H", [(1, 64, 4), (77, 72, 3), (130, 200, 5), (300, 384, 16), (1100, 512, 8), (129, 1024, 16)])
+def test_self_block_reads_weights_of_any_layout(cuda_device, N, C, H):
+    """Weights kept `[in, out]`, `[out, in]`, as parts of larger matrices, mixed, and in forms that are packed first
+    (odd pitch, odd offset, fp32 with the same values) give the same bits, on channel counts short of and past whole
+    64-column blocks."""
+    g = torch.Generator().manual_seed(C)
+    dev = cuda_device
+    x = torch.randn(N, C, generator=g).to(torch.bfloat16)
+    ws = [(torch.randn(C, C, generator=g) * C ** -0.5).to(torch.bfloat16) for _ in range(4)]        # [in, out]
+    qb = (torch.randn(C, generator=g) * 0.3).to(torch.bfloat16)
+    bias = torch.randn(H, N, N, generator=g).to(torch.bfloat16)
+
+    def part(w, rows, cols, r0, c0):
+        big = torch.full((rows, cols), float("nan"), dtype=w.dtype, device=dev)
+        big[r0:r0 + C, c0:c0 + C] = w.to(dev)
+        return big[r0:r0 + C, c0:c0 + C]
+
+    forms = {
+        "in_out": lambda w: w.to(dev).contiguous(),
+        "out_in": lambda w: w.T.contiguous().to(dev).T,
+        "part": lambda w: part(w, C + 3, C + 16, 2, 8),
+        "part_t": lambda w: part(w.T, C + 3, C + 16, 2, 8).T,
+        "odd_pitch": lambda w: part(w, C, C + 1, 0, 0),
+        "odd_offset": lambda w: part(w, C, C + 8, 0, 1),
+        "f32": lambda w: w.float().to(dev),
+        "f32_t": lambda w: w.float().T.contiguous().to(dev).T,
+    }
+    ref = O.self_block_fp32(x, torch.ones(N, dtype=torch.bool), bias, ws[0].T, qb, *(w.T for w in ws[1:]), H)
+    call = lambda w: A.self_attention_cpp(x.to(dev), None, bias.to(dev), w[0], qb.to(dev), *w[1:], H)
+    want = call([forms["out_in"](w) for w in ws])
+    _close(want, ref, (N, C, H))
+    for name, form in forms.items():
+        assert torch.equal(call([form(w) for w in ws]), want), name
+    mixed = [forms[n](w) for n, w in zip(("in_out", "out_in", "part", "part_t"), ws)]
+    assert torch.equal(call(mixed), want)
+    assert read_status(dev)[0] == 0
