@@ -83,6 +83,8 @@ Tensor status_buffer(int64_t device) {
 // not before it was divided by each head's logit scale, is converted once; the copy is used again
 // while the very same tensor object is alive and unmodified (its version counter) and, for fp8, the
 // scales are the same.  Four copies are kept; copies of dead tensors are dropped when another is made.
+// A stream that is being captured never gets one of them: the graph would go on reading the copy after the
+// list gave it up, and would not see a later write to the bias.  It converts inside the graph.
 struct TensorId {
   c10::weak_intrusive_ptr<c10::TensorImpl> impl;
   int64_t version = -1;
@@ -129,7 +131,7 @@ Tensor staged_bias(const Tensor& bias, int64_t B2, int64_t Sq, int64_t Sk, int64
                    const OptTensor& ks_id, const float* q_scale, const float* k_scale, float scale) {
   const auto stream = c10::cuda::getCurrentCUDAStream(bias.device().index());
   const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
-  const bool cacheable = !bias.is_inference() && !(qs_id && (qs_id->is_inference() || ks_id->is_inference()));
+  const bool cacheable = !capturing && !bias.is_inference() && !(qs_id && (qs_id->is_inference() || ks_id->is_inference()));
   std::lock_guard<std::mutex> lock(g_staged_mu);
   if (cacheable) {
     for (auto it = g_staged->begin(); it != g_staged->end(); ++it) {
@@ -139,7 +141,6 @@ Tensor staged_bias(const Tensor& bias, int64_t B2, int64_t Sq, int64_t Sk, int64
         continue;
       if (qs_id && (!e.q_scale->is(*qs_id) || !e.k_scale->is(*ks_id) || e.scale != scale)) continue;
       if (std::find(e.ordered.begin(), e.ordered.end(), stream.id()) == e.ordered.end()) {
-        if (capturing) break;              // a captured stream cannot wait for work outside the graph: convert inside it
         e.made.block(stream);
         c10::cuda::CUDACachingAllocator::recordStream(e.copy.storage().data_ptr(), stream);
         e.ordered.push_back(stream.id());
@@ -149,7 +150,7 @@ Tensor staged_bias(const Tensor& bias, int64_t B2, int64_t Sq, int64_t Sk, int64
     }
   }
   Tensor copy = make_staged(bias, B2, Sq, Sk, D, q_scale, k_scale, scale, stream);
-  if (!cacheable || capturing) return copy;     // a copy made inside a graph exists only while the graph replays
+  if (!cacheable) return copy;
   g_staged->remove_if([&](const Staged& e) { return e.bias.impl.expired() || e.bias.impl._unsafe_get_target() == bias.unsafeGetTensorImpl(); });
   while (g_staged->size() >= kStagedMost) g_staged->pop_back();
   Staged e{TensorId(bias), bias.sizes().vec(), bias.strides().vec(), bias.data_ptr(), B2, Sq, Sk, std::nullopt, std::nullopt, scale, copy,

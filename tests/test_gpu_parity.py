@@ -416,3 +416,35 @@ def test_query_tiles_on_ctas_of_their_own(cuda_device, B1, B2, S, D):
     tiles = B1 * B2 * ((S + 127) // 128)
     assert torch.equal(_run(cuda_device, q, k, v, mask, bias, max_ctas=max(1, tiles // 2)), own)
     _check_bf16(own, O.oracle_fp32(q, k, v, mask, bias), (B1, B2, S, D))
+
+
+@pytest.mark.parametrize("fp8,S", [(False, 200), (False, 77), (True, 128)])
+def test_a_graph_converts_the_bias_it_is_given(cuda_device, fp8, S):
+    """A bias that is staged first (fp32, ragged rows, fp8 scales), captured on the stream that was warmed up: a replay
+    sees the values the bias holds then, whatever other biases were staged since."""
+    g = torch.Generator().manual_seed(S)
+    B1, B2, D = 3, 4, 32
+    q, k, v = (torch.randn(B1, B2, S, D, generator=g).to(cuda_device, torch.bfloat16) for _ in range(3))
+    scales = {}
+    if fp8:
+        q, k = q.to(torch.float8_e4m3fn), k.to(torch.float8_e4m3fn)
+        scales = {n: torch.rand(B2, generator=g).to(cuda_device) + 0.5 for n in ("q_scale", "k_scale")}
+    biases = [torch.randn(B2, S, S, generator=g).to(cuda_device) for _ in range(8)]
+    bias = biases[0].clone()
+    call = lambda b: A.dot_product_attention_cpp(q, k, v, None, b, **scales)
+    want = [call(b) for b in biases]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        call(bias)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            out = call(bias)
+    torch.cuda.current_stream().wait_stream(side)
+    again = [call(b) for b in biases]
+    assert all(torch.equal(a, b) for a, b in zip(again, want))
+    for i in (0, 3, 5):
+        bias.copy_(biases[i])
+        graph.replay()
+        assert torch.equal(out, want[i]), i
+    torch.cuda.synchronize()
