@@ -251,6 +251,7 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
       value_error("out must be a bf16 [B1, B2, Sq, D] tensor with unit inner stride");
   }
   if (out.numel() == 0) return f32_result ? out.to(at::kFloat) : out;
+  if (out_in && !out.is_inference()) out.unsafeGetTensorImpl()->bump_version();   // written in place, as by any torch operator
 
   af3k_attention_desc d{};
   d.B1 = B1; d.B2 = B2; d.Sq = Sq; d.Sk = Sk; d.D = D;

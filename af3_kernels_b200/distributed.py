@@ -85,6 +85,9 @@ class RowShardedAttention:
         if mask is not None:
             m = mask.view(torch.uint8) if mask.dtype == torch.bool else mask
             dist.broadcast(m, src=src, group=self.group)
+        # a collective bumps no version counter, and the operator finds its staged copy of a bias by it
+        if not bias.is_inference():
+            torch.autograd.graph.increment_version(bias)
         return bias, mask
 
     def shard(self, full: torch.Tensor, rows: int) -> torch.Tensor:

@@ -139,6 +139,10 @@ def dot_product_attention(
     softmax threads add the bias themselves.  ``bias`` may be a ``StagedBias``; a plain tensor
     that needs the staging pass is staged once and the copy is reused while the same, unmodified
     tensor object keeps being passed (``cache_bias=False`` stages inside every call instead).
+    Unmodified means by its version counter: after a write that bumps none (``bias.data``, a
+    collective, a graph replay or a kernel on the raw pointer) pass ``cache_bias=False`` or call
+    ``torch.autograd.graph.increment_version(bias)``.  Under stream capture it is always staged
+    inside the graph.
     ``max_ctas`` > 0 caps the kernel's grid, leaving the other SMs to a kernel that runs beside it.
     """
     if mask is not None and q.dim() == 4 and k.dim() == 4:

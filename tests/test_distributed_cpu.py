@@ -137,3 +137,25 @@ def test_lost_rank_ends_the_gather_with_an_error():
     ret = mp.Manager().dict()
     mp.spawn(_lost_rank_worker, args=(ws, port, ret), nprocs=ws, join=True)
     assert ret[1] == "left" and ret[0] == "error", dict(ret)
+
+
+def _broadcast_worker(rank, ws, port, ret):
+    sys.path.insert(0, ROOT)
+    import datetime
+    dist.init_process_group("gloo", init_method=f"tcp://127.0.0.1:{port}", rank=rank, world_size=ws,
+                            timeout=datetime.timedelta(seconds=60))
+    try:
+        from af3_kernels_b200.distributed import RowShardedAttention
+        bias = torch.full((2, 8, 8), float(rank))
+        before = bias._version
+        RowShardedAttention(attention_fn=_oracle_fn).broadcast_shared(bias, None)
+        ret[rank] = bool((bias == 0).all()) and bias._version > before
+    finally:
+        dist.destroy_process_group()
+
+
+def test_broadcast_bias_counts_as_written():
+    """The operator finds its staged copy of a bias by the version counter, which a collective leaves alone."""
+    ret = mp.get_context("spawn").Manager().dict()
+    mp.spawn(_broadcast_worker, args=(2, _free_port(), ret), nprocs=2, join=True)
+    assert dict(ret) == {0: True, 1: True}

@@ -448,3 +448,13 @@ def test_a_graph_converts_the_bias_it_is_given(cuda_device, fp8, S):
         graph.replay()
         assert torch.equal(out, want[i]), i
     torch.cuda.synchronize()
+
+
+def test_out_counts_as_written(cuda_device):
+    """A result written into a caller's tensor bumps its version, as any in-place operator does: a staged copy made of
+    that tensor as a bias is not used again."""
+    q = torch.ones(1, 2, 40, 32, dtype=torch.bfloat16, device=cuda_device)
+    out = torch.empty_like(q)
+    before = out._version
+    A.dot_product_attention(q, q, q, None, torch.zeros(2, 40, 40, device=cuda_device), out=out)
+    assert out._version > before
