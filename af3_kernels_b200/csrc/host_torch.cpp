@@ -249,6 +249,7 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
     if (out.dim() != 4 || out.size(0) != B1 || out.size(1) != B2 || out.size(2) != Sq || out.size(3) != D ||
         out.scalar_type() != at::kBFloat16 || out.stride(3) != 1)
       value_error("out must be a bf16 [B1, B2, Sq, D] tensor with unit inner stride");
+    if (out.device() != dev) value_error("out must live on the device of q, k, v, bias");
   }
   if (out.numel() == 0) return f32_result ? out.to(at::kFloat) : out;
   if (out_in && !out.is_inference()) out.unsafeGetTensorImpl()->bump_version();   // written in place, as by any torch operator
@@ -290,9 +291,14 @@ Tensor kernel_dtype(const Tensor& t) {      // bf16 or fp32, without a gradient
   return x.scalar_type() == at::kFloat || x.scalar_type() == at::kBFloat16 ? x : x.to(at::kFloat);
 }
 
-void matrices(const std::vector<Tensor>& w, int64_t C) {
-  for (const Tensor& t : w)
-    if (t.dim() != 2 || t.size(0) != C || t.size(1) != C) value_error("projection weights must be [C, C]");
+// The first n parameters are [C, C]; all are where the activations are (a kernel handed the address of a module that was
+// left on the host would fault).
+void check_parameters(const std::vector<Tensor>& params, size_t n, int64_t C, const at::Device& dev) {
+  for (size_t i = 0; i < params.size(); ++i) {
+    const Tensor& t = params[i];
+    if (t.device() != dev) value_error("parameters must live on the device of the activations, " + dev.str() + ", got " + t.device().str());
+    if (i < n && (t.dim() != 2 || t.size(0) != C || t.size(1) != C)) value_error("projection weights must be [C, C]");
+  }
 }
 
 // q, k, v, gate and perhaps output projection [C, C] as (out, in) matrices, in the kernels' layout: one launch
@@ -360,7 +366,7 @@ Tensor grid_module(Tensor pair, const Tensor& mask_in, const std::vector<Tensor>
   const c10::cuda::CUDAGuard guard(dev);
   const int64_t R = pair.size(0), N = pair.size(1), C = pair.size(2), D = C / head, M = R * N;
   if (R != N) value_error("pair must be [N, N, c_pair]");
-  matrices({params.begin(), params.begin() + 5}, C);
+  check_parameters(params, 5, C, dev);
   if (params[7].dim() != 2 || params[7].size(0) != head || params[7].size(1) != C || params[5].numel() != C || params[6].numel() != C)
     value_error("LayerNorm and bias projection do not match the pair");
   pair = pair.contiguous();
@@ -402,7 +408,7 @@ Tensor grid_block(const Tensor& pair, const OptTensor& mask, const Tensor& bias,
   const at::Device dev = pair.device();
   const c10::cuda::CUDAGuard guard(dev);
   const int64_t R = pair.size(0), N = pair.size(1), C = pair.size(2), D = C / head, M = R * N;
-  matrices(weights, C);
+  check_parameters(weights, 5, C, dev);
   Tensor x = pair.to(at::kBFloat16).contiguous();
   if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0) x = x.clone();
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
@@ -428,15 +434,15 @@ Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, con
   const at::Device dev = x_in.device();
   const c10::cuda::CUDAGuard guard(dev);
   const int64_t N = x_in.size(0), C = x_in.size(1), D = C / head;
-  matrices(weights, C);
+  check_parameters(weights, 4, C, dev);
+  check_parameters({q_bias}, 0, C, dev);
   if (q_bias.numel() != C) value_error("q_bias must have one entry per channel");
   if (bias.numel() != head * N * N) value_error("bias must have B2*Sq*Sk = " + std::to_string(head * N * N) + " elements, got " + std::to_string(bias.numel()));
   if (bias.device() != dev) value_error("q, k, v, bias must live on the same device");
   Tensor x = x_in.to(at::kBFloat16).contiguous();
   if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0) x = x.clone();
   if (N == 0) return at::empty({N, C}, x_in.options());
-  if (q_bias.device() != dev || (q_bias.scalar_type() != at::kBFloat16 && q_bias.scalar_type() != at::kFloat)) q_bias = q_bias.to(dev, at::kFloat);
-  q_bias = q_bias.contiguous();
+  q_bias = kernel_dtype(q_bias).contiguous();
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
   // weights the kernel can read where they are: bf16, [out, in] or [in, out], rows of 16-byte multiples
   af3k_matrix w4[4];

@@ -41,6 +41,7 @@ def sigmoid_gate(weighted: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
     not a multiple of 8, non-contiguous) go through torch."""
     n = weighted.numel()
     if (weighted.dtype != torch.bfloat16 or gate.dtype != torch.bfloat16 or n % 8 != 0 or n == 0
+            or gate.shape != weighted.shape or gate.device != weighted.device
             or not weighted.is_contiguous() or not gate.is_contiguous()
             or weighted.data_ptr() % 16 != 0 or gate.data_ptr() % 16 != 0):
         return weighted * torch.sigmoid(gate)

@@ -432,3 +432,35 @@ def test_self_block_reads_weights_of_any_layout(cuda_device, N, C, H):
     mixed = [forms[n](w) for n, w in zip(("in_out", "out_in", "part", "part_t"), ws)]
     assert torch.equal(call(mixed), want)
     assert read_status(dev)[0] == 0
+
+
+@pytest.mark.parametrize("C", [64, 128])
+def test_parameters_on_another_device_are_refused(cuda_device, C):
+    """A module or weights left on the host: an exception before anything is launched."""
+    H, N = 4, 24
+    dev, bf16 = cuda_device, torch.bfloat16
+    pair, mask = torch.zeros(N, N, C, device=dev, dtype=bf16), torch.ones(N, N, dtype=torch.bool, device=dev)
+    bias = torch.zeros(H, N, N, device=dev, dtype=bf16)
+    w = [torch.zeros(C, C, dtype=bf16) for _ in range(5)]
+    on = [t.to(dev) for t in w]
+    m = A.GridSelfAttentionCpp(C, H).to(bf16)
+    with torch.no_grad():
+        with pytest.raises(ValueError, match="device"):
+            m(pair, mask)
+        m.to(dev).output_projection.cpu()
+        with pytest.raises(ValueError, match="device"):
+            m(pair, mask)
+        for i in range(5):
+            mixed = [w[j] if j == i else on[j] for j in range(5)]
+            with pytest.raises(ValueError, match="device"):
+                A._attention_cpp(pair, mask, bias, *mixed, H)
+            if i < 4:
+                with pytest.raises(ValueError, match="device"):
+                    A.self_attention_cpp(pair[0], mask[0], bias, mixed[0], torch.zeros(C, device=dev), *mixed[1:4], H)
+        with pytest.raises(ValueError, match="device"):
+            A.self_attention_cpp(pair[0], mask[0], bias, on[0], torch.zeros(C), *on[1:4], H)
+        q = torch.zeros(1, 2, 16, 32, device=dev, dtype=bf16)
+        with pytest.raises(ValueError, match="device"):
+            A.dot_product_attention(q, q, q, None, torch.zeros(2, 16, 16, device=dev), out=q.cpu())
+    torch.cuda.synchronize()
+    assert read_status(dev)[0] == 0
