@@ -108,11 +108,17 @@ std::mutex g_staged_mu;
 std::list<Staged>* g_staged = new std::list<Staged>();
 constexpr size_t kStagedMost = 4;
 
+// The bias as [B2, Sq, Sk]; another shape with as many elements (four dimensions, or three others) is reshaped.
+Tensor bias_3d(const Tensor& bias, int64_t B2, int64_t Sq, int64_t Sk) {
+  const int64_t sizes[3] = {B2, Sq, Sk};
+  return bias.sizes() == at::IntArrayRef(sizes, 3) ? bias : bias.reshape(sizes);
+}
+
 Tensor make_staged(const Tensor& bias_in, int64_t B2, int64_t Sq, int64_t Sk, int64_t D, const float* q_scale,
                    const float* k_scale, float scale, cudaStream_t stream) {
   Tensor bias = bias_in;
   if (bias.scalar_type() != at::kBFloat16 && bias.scalar_type() != at::kFloat) bias = bias.to(at::kFloat);
-  if (bias.dim() != 3) bias = bias.reshape({B2, Sq, Sk});
+  bias = bias_3d(bias, B2, Sq, Sk);
   if ((Sk > 1 && bias.stride(2) != 1) || (B2 > 1 && bias.stride(0) == 0) || (Sq > 1 && bias.stride(1) == 0)) bias = bias.contiguous();
   af3k_attention_desc d{};
   d.B1 = 1; d.B2 = B2; d.Sq = Sq; d.Sk = Sk; d.D = (D + 15) / 16 * 16;
@@ -215,8 +221,8 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
     if (bias.numel() != B2 * Sq * Sk) {
       value_error("bias must have B2*Sq*Sk = " + std::to_string(B2 * Sq * Sk) + " elements, got " + std::to_string(bias.numel()));
     }
-    const bool needs_copy = bias.scalar_type() != at::kBFloat16 || bias.dim() != 3 || bias.stride(2) != 1 ||
-                            (bias.stride(1) * 2) % 16 != 0 || (bias.stride(0) * 2) % 16 != 0 ||
+    const bool as_is = bias.dim() == 3 && bias.size(0) == B2 && bias.size(1) == Sq && bias.size(2) == Sk;
+    const bool needs_copy = bias.scalar_type() != at::kBFloat16 || !as_is || bias.stride(2) != 1 || (bias.stride(1) * 2) % 16 != 0 || (bias.stride(0) * 2) % 16 != 0 ||
                             reinterpret_cast<uintptr_t>(bias.data_ptr()) % 16 != 0;
     if (use_workspace && cache_bias && (needs_copy || fp8) && bias.numel() != 0) {
       bias = staged_bias(bias, B2, Sq, Sk, D, fp8 ? q_scale_in : std::nullopt, fp8 ? k_scale_in : std::nullopt,
@@ -224,7 +230,7 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
       prescaled = fp8;
     } else {
       if (bias.scalar_type() != at::kBFloat16 && bias.scalar_type() != at::kFloat) bias = bias.to(at::kFloat);
-      if (bias.dim() != 3) bias = bias.reshape({B2, Sq, Sk});
+      bias = bias_3d(bias, B2, Sq, Sk);
       if ((Sk > 1 && bias.stride(2) != 1) || (B2 > 1 && bias.stride(0) == 0) || (Sq > 1 && bias.stride(1) == 0)) bias = bias.contiguous();
     }
   }
@@ -459,7 +465,7 @@ Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, con
     for (int i = 0; i < 4; ++i) w4[i] = af3k_matrix{static_cast<char*>(packed.data_ptr()) + i * C * C * 2, C, 1, AF3K_BF16};
   }
   const float scale = 1.0f / std::sqrt((float)D);
-  const bool in_place = bias.scalar_type() == at::kBFloat16 && bias.dim() == 3 && bias.stride(2) == 1 && (bias.stride(1) * 2) % 16 == 0 &&
+  const bool in_place = bias.scalar_type() == at::kBFloat16 && bias.dim() == 3 && bias.size(0) == head && bias.size(1) == N && bias.stride(2) == 1 && (bias.stride(1) * 2) % 16 == 0 &&
                         (bias.stride(0) * 2) % 16 == 0 && (bias.stride(0) != 0 || head == 1) && (bias.stride(1) != 0 || N == 1) &&
                         reinterpret_cast<uintptr_t>(bias.data_ptr()) % 16 == 0;
   if (!in_place) bias = staged_bias(bias, head, N, N, D, std::nullopt, std::nullopt, nullptr, nullptr, scale);

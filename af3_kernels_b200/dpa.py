@@ -55,7 +55,7 @@ def stage_bias(bias: torch.Tensor, B2: int, Sq: int, Sk: int, *, q_scale=None, k
         raise ValueError(f"bias must have B2*Sq*Sk = {B2 * Sq * Sk} elements, got {bias.numel()}")
     if bias.dtype not in (torch.bfloat16, torch.float32):
         bias = bias.to(torch.float32)
-    bias = bias.reshape(B2, Sq, Sk) if bias.dim() != 3 else bias
+    bias = bias.reshape(B2, Sq, Sk) if bias.shape != (B2, Sq, Sk) else bias
     if (Sk > 1 and bias.stride(2) != 1) or (B2 > 1 and bias.stride(0) == 0) or (Sq > 1 and bias.stride(1) == 0):
         bias = bias.contiguous()
     fp8 = q_scale is not None

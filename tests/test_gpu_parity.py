@@ -458,3 +458,26 @@ def test_out_counts_as_written(cuda_device):
     before = out._version
     A.dot_product_attention(q, q, q, None, torch.zeros(2, 40, 40, device=cuda_device), out=out)
     assert out._version > before
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_bias_of_another_shape_is_reshaped(cuda_device, dtype):
+    """As many elements in another three (or four) dimensions: read as the [B2, Sq, Sk] tensor it reshapes to, on every
+    route a bias takes (in place, staged, staged by the caller, single block, host tensors)."""
+    from af3_kernels_b200.dpa import stage_bias
+    g = torch.Generator().manual_seed(2)
+    B2, S, D = 4, 64, 16
+    q, k, v = (torch.randn(2, B2, S, D, generator=g).to(cuda_device, torch.bfloat16) for _ in range(3))
+    bias = torch.randn(B2, S, S, generator=g).to(cuda_device, dtype)
+    want = A.dot_product_attention(q, k, v, None, bias)
+    w = [torch.randn(S, S, generator=g).to(cuda_device, torch.bfloat16) * 0.1 for _ in range(4)]
+    x, qb = q[0, 0].repeat(1, B2), torch.zeros(S, device=cuda_device)
+    block = lambda b: A.self_attention_cpp(x, None, b, w[0], qb, *w[1:], B2)
+    want_block = block(bias)
+    for shape in ((1, B2 * S, S), (B2 * S, 1, S), (S, B2, S), (1, B2, S, S), (B2 * S * S,)):
+        b = bias.reshape(shape)
+        assert torch.equal(A.dot_product_attention(q, k, v, None, b), want), shape
+        assert torch.equal(A.dot_product_attention(q, k, v, None, b, cache_bias=False), want), shape
+        assert torch.equal(A.dot_product_attention(q, k, v, None, stage_bias(b, B2, S, S)), want), shape
+        assert torch.equal(block(b), want_block), shape
+        assert torch.equal(A.dot_product_attention_host(q.cpu(), k.cpu(), v.cpu(), None, b.cpu()), want.cpu()), shape
