@@ -181,6 +181,12 @@ std::string shape_text(const Tensor& t) {
   return s.str();
 }
 
+// mask: bool, [Sk] or [1 | B1, Sk] (the Python side brings other forms to this one)
+void check_mask(const Tensor& mask, int64_t B1, int64_t Sk) {
+  if (mask.dim() < 1 || mask.dim() > 2 || mask.size(-1) != Sk || (mask.dim() == 2 && mask.size(0) != 1 && mask.size(0) != B1))
+    value_error("mask of shape " + shape_text(mask) + " does not match B1=" + std::to_string(B1) + ", Sk=" + std::to_string(Sk));
+}
+
 // bias_form: 0 an ordinary bias tensor, 1 the copy of a StagedBias, 2 the same divided by fp8 scales
 Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor bias, const OptTensor& q_scale_in,
                  const OptTensor& k_scale_in, std::optional<double> softmax_scale, int64_t rows_per_item, const OptTensor& out_in,
@@ -238,10 +244,9 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
 
   Tensor mask;
   int64_t mask_stride = 0;
-  if (mask_in) {      // bool, [Sk] or [1 | B1, Sk] (the Python side brings other forms to this one)
+  if (mask_in) {
     mask = *mask_in;
-    if (mask.size(-1) != Sk || (mask.dim() == 2 && mask.size(0) != 1 && mask.size(0) != B1) || mask.dim() > 2)
-      value_error("mask of shape " + shape_text(mask) + " does not match B1=" + std::to_string(B1) + ", Sk=" + std::to_string(Sk));
+    check_mask(mask, B1, Sk);
     mask = mask.contiguous();
     if (mask.device() != dev) mask = mask.to(dev);
     mask_stride = mask.dim() == 2 && !(mask.size(0) == 1 && B1 != 1) ? Sk : 0;
@@ -378,8 +383,7 @@ Tensor grid_module(Tensor pair, const Tensor& mask_in, const std::vector<Tensor>
   pair = pair.contiguous();
   if (reinterpret_cast<uintptr_t>(pair.data_ptr()) % 16 != 0) pair = pair.clone();
   Tensor mask = mask_in.device() == dev ? mask_in.contiguous() : mask_in.to(dev).contiguous();
-  if (mask.size(-1) != N || (mask.dim() == 2 && mask.size(0) != 1 && mask.size(0) != N))
-    value_error("mask of shape " + shape_text(mask) + " does not match B1=" + std::to_string(N) + ", Sk=" + std::to_string(N));
+  check_mask(mask, N, N);
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
   const GridParameters w = grid_parameters(params, C, stream);
   const auto bf16 = pair.options().dtype(at::kBFloat16);
@@ -522,6 +526,7 @@ void host_attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tens
       value_error("k and v must be [B1, B2, Sk, D] matching q");
   if (bias.numel() != B2 * Sq * Sk)
     value_error("bias must have B2*Sq*Sk = " + std::to_string(B2 * Sq * Sk) + " elements, got " + std::to_string(bias.numel()));
+  if (mask_in) check_mask(*mask_in, B1, Sk);
   const at::Device dev(at::kCUDA, (c10::DeviceIndex)device);
   const c10::cuda::CUDAGuard guard(dev);
   q = q.contiguous(); k = k.contiguous(); v = v.contiguous();

@@ -52,3 +52,11 @@ def test_host_row_blocks_give_the_device_result(cuda_device, B1, chunks):
     out = A.dot_product_attention_host(q, k, v, mask, bias, chunks=chunks)
     ref = A.dot_product_attention_cpp(*(t.to(cuda_device) for t in (q, k, v, mask, bias)))
     assert torch.equal(out, ref.cpu())
+
+
+def test_host_call_refuses_a_mask_of_one_block(cuda_device):
+    """A mask with as many rows as a row block has, not as the call has, is refused as it is for CUDA tensors."""
+    q = torch.zeros(40, 4, 331, 32, dtype=torch.bfloat16)
+    bias = torch.zeros(4, 331, 331, dtype=torch.bfloat16)
+    with pytest.raises(ValueError):
+        A.dot_product_attention_host(q, q, q, torch.ones(20, 331, dtype=torch.bool), bias, chunks=2)
