@@ -17,6 +17,7 @@
 #include <cmath>
 #include <cstring>
 #include <list>
+#include <map>
 #include <mutex>
 
 #include "../../include/af3k.h"
@@ -518,6 +519,17 @@ constexpr int64_t kHostBlockBytes = 2 << 20;
     }                                                                                          \
   } while (0)
 
+// The two copy streams of a thread on a device, the same in every call: streams taken anew from torch's pool would be
+// other ones each time.
+struct CopyStreams { c10::cuda::CUDAStream in, out; };
+const CopyStreams& copy_streams(c10::DeviceIndex device) {
+  static thread_local std::map<int, CopyStreams> kept;
+  auto it = kept.find(device);
+  if (it == kept.end())
+    it = kept.emplace(device, CopyStreams{c10::cuda::getStreamFromPool(false, device), c10::cuda::getStreamFromPool(false, device)}).first;
+  return it->second;
+}
+
 void host_attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor bias, const OptTensor& q_scale,
                     const OptTensor& k_scale, std::optional<double> softmax_scale, Tensor out, int64_t device, int64_t chunks) {
   const int64_t B1 = q.size(0), B2 = q.size(1), Sq = q.size(2), D = q.size(3), Sk = k.dim() == 4 ? k.size(2) : 0;
@@ -537,18 +549,18 @@ void host_attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tens
   bounds.push_back(B1);
   const int64_t blocks = (int64_t)bounds.size() - 1;
   const auto main = c10::cuda::getCurrentCUDAStream(dev.index());
-  const auto s_in = blocks > 1 ? c10::cuda::getStreamFromPool(false, dev.index()) : main;
-  const auto s_out = blocks > 1 ? c10::cuda::getStreamFromPool(false, dev.index()) : main;
+  const auto s_in = blocks > 1 ? copy_streams(dev.index()).in : main;
+  const auto s_out = blocks > 1 ? copy_streams(dev.index()).out : main;
 
   auto on_device = [&](const Tensor& t) { return at::empty(t.sizes(), t.options().device(dev).pinned_memory(false)); };
   auto copy = [&](void* dst, const void* src, size_t bytes, cudaMemcpyKind kind, cudaStream_t s) {
     if (bytes != 0) AF3K_CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, kind, s));
   };
-  auto send = [&](const Tensor& host) {
-    if (host.is_cuda()) return host.to(dev);
-    Tensor t = on_device(host);
-    copy(t.data_ptr(), host.data_ptr(), host.nbytes(), cudaMemcpyHostToDevice, s_in);
-    return t;
+  // a small operand, sent whole: its host form, and where it goes
+  struct Sent { Tensor host, device; };
+  auto place = [&](const Tensor& t) {
+    const Tensor c = t.contiguous();
+    return t.is_cuda() ? Sent{Tensor(), c.to(dev)} : Sent{c, on_device(c)};
   };
   // the call may only return (or throw) once nothing on the device touches the host tensors or the
   // buffers below any more
@@ -560,15 +572,22 @@ void host_attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tens
         for (cudaStream_t t : s) (void)cudaStreamSynchronize(t);
     }
   };
-  // buffers come from the caller's stream: what used their memory before is ordered ahead of that stream
+  // all buffers come from the caller's stream: what used their memory before is ordered ahead of that stream, and the
+  // copy streams wait for a point on it behind the last allocation
   Tensor dq = on_device(q), dk = on_device(k), dv = on_device(v), dout = on_device(out);
-  Tensor bias_sent, bias_d, mask_d;
+  Sent bias_s = place(bias), mask_s, qs_s, ks_s;
+  if (mask_in) mask_s = place(*mask_in);
+  if (q_scale) qs_s = place(q_scale->to(at::kFloat));
+  if (k_scale) ks_s = place(k_scale->to(at::kFloat));
+  Tensor bias_d = bias_s.device, mask_d = mask_s.device;
   // the kernels' status words live in pinned host memory here: only a wait that ran out writes them, and
   // reading them after the call's own synchronisation costs no copy
   Tensor status = at::empty({4}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
   int* st = status.data_ptr<int>();
   std::memset(st, 0, 16);
   OptTensor qs, ks;
+  if (q_scale) qs = qs_s.device;
+  if (k_scale) ks = ks_s.device;
   const bool fp8 = q.scalar_type() == at::kFloat8_e4m3fn;
   {
     Drain drain{{s_in, main, s_out}};
@@ -579,14 +598,8 @@ void host_attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tens
       ev[2 * blocks].block(s_out);
     }
     int64_t form = 0;
-    {
-      const c10::cuda::CUDAStreamGuard on_in(s_in);
-      if (q_scale) qs = send(q_scale->to(at::kFloat).contiguous());
-      if (k_scale) ks = send(k_scale->to(at::kFloat).contiguous());
-      bias_d = send(bias.contiguous());
-      if (mask_in) mask_d = send(mask_in->contiguous());
-    }
-    bias_sent = bias_d;
+    for (const Sent* t : {&qs_s, &ks_s, &bias_s, &mask_s})
+      if (t->host.defined()) copy(t->device.data_ptr(), t->host.data_ptr(), t->host.nbytes(), cudaMemcpyHostToDevice, s_in);
     const bool aligned = bias_d.scalar_type() == at::kBFloat16 && Sk % 8 == 0;
     if (fp8 ? (qs && ks && qs->numel() == B2 && ks->numel() == B2) : !aligned) {
       // converted on the caller's stream, under the copies of the first block

@@ -60,3 +60,17 @@ def test_host_call_refuses_a_mask_of_one_block(cuda_device):
     bias = torch.zeros(4, 331, 331, dtype=torch.bfloat16)
     with pytest.raises(ValueError):
         A.dot_product_attention_host(q, q, q, torch.ones(20, 331, dtype=torch.bool), bias, chunks=2)
+
+
+def test_host_calls_hold_no_more_memory_the_more_there_are(cuda_device):
+    """Forty pipelined calls reserve what two do."""
+    g = torch.Generator().manual_seed(3)
+    q = torch.randn(40, 4, 331, 32, generator=g).to(torch.bfloat16).pin_memory()
+    bias = torch.randn(4, 331, 331, generator=g).pin_memory()
+    mask = (torch.rand(40, 331, generator=g) >= 0.1).pin_memory()
+    first = A.dot_product_attention_host(q, q, q, mask, bias).clone()
+    A.dot_product_attention_host(q, q, q, mask, bias)
+    held = torch.cuda.memory_reserved()
+    for _ in range(40):
+        assert torch.equal(A.dot_product_attention_host(q, q, q, mask, bias), first)
+    assert torch.cuda.memory_reserved() == held
