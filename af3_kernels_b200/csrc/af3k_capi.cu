@@ -734,7 +734,7 @@ int af3k_grid_front_weights(const void* pair, int32_t pair_dtype, const af3k_fro
     if (t != AF3K_BF16 && t != AF3K_F32) return AF3K_ERR_BAD_DTYPE;
   if (C != 64 && C != 128) return AF3K_ERR_BAD_SHAPE;
   if (R < 0 || N < 0 || H < 1 || C % H != 0 || (C / H) % 8 != 0 || Hb < 0 || Hb > 4 || (Hb > 0 && !ln)) return AF3K_ERR_BAD_SHAPE;
-  if (R > 0x7fffffff || N > 0x7fffffff || R * N * C > 0x7fffffffLL) return AF3K_ERR_BAD_SHAPE;    // 32-bit element offsets
+  if (R > 0x7fffffff || N > 0x7fffffff || (R > 0 && N > 0x7fffffffLL / C / R)) return AF3K_ERR_BAD_SHAPE;   // 32-bit element offsets
   if (Hb > 0 && (bias_pitch < N || (bias_pitch & 7) != 0)) return AF3K_ERR_BAD_STRIDE;
   if (R == 0 || N == 0) return AF3K_OK;
   if (!pair || !q || !k || !v || !gate || (ln && !w.beta) || (Hb > 0 && (!w.bias_w || !bias))) return AF3K_ERR_NULL_POINTER;

@@ -362,10 +362,16 @@ GridParameters grid_parameters(const std::vector<Tensor>& params, int64_t C, cud
 }
 
 // ------------------------------------------------------------------ the grid attention block
+// The sizes all three kernels take: widths 64 and 128, heads of 8 to 64 channels (the attention kernel's), up to four
+// bias heads and 32-bit element offsets (the front's).  Others go through torch's projections.
+bool grid_sizes_fused(int64_t R, int64_t N, int64_t C, int64_t head, int64_t bias_heads) {
+  if ((C != 64 && C != 128) || head < 1 || C % head != 0 || bias_heads > 4) return false;
+  const int64_t D = C / head, most = 0x7fffffffLL / C;
+  return D % 8 == 0 && D <= 64 && R > 0 && N > 0 && R <= most && N <= most / R;
+}
+
 bool grid_fused(const Tensor& pair, int64_t head, int64_t bias_heads) {
-  if (!pair.is_cuda() || pair.dim() != 3 || pair.numel() == 0) return false;
-  const int64_t C = pair.size(2);
-  return (C == 64 || C == 128) && head > 0 && C % head == 0 && (C / head) % 8 == 0 && bias_heads <= 4 &&
+  return pair.is_cuda() && pair.dim() == 3 && grid_sizes_fused(pair.size(0), pair.size(1), pair.size(2), head, bias_heads) &&
          (pair.scalar_type() == at::kBFloat16 || pair.scalar_type() == at::kFloat);
 }
 
@@ -649,6 +655,7 @@ void host_attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tens
 
 PYBIND11_MODULE(_host, m) {
   m.def("grid_fused", &grid_fused);
+  m.def("grid_sizes_fused", &grid_sizes_fused);
   m.def("grid_module", &grid_module, py::call_guard<py::gil_scoped_release>());
   m.def("grid_block", &grid_block, py::call_guard<py::gil_scoped_release>());
   m.def("self_block", &self_block, py::call_guard<py::gil_scoped_release>());

@@ -229,3 +229,27 @@ def test_sigmoid_gate_argument_validation_codes():
     assert lib.af3k_sigmoid_gate(one, one, one, 0, None) == 0           # empty
     assert lib.af3k_sigmoid_gate(None, one, one, 8, None) == 6
     assert lib.af3k_sigmoid_gate(ctypes.c_void_p(8), one, one, 8, None) == 4
+
+
+@pytest.mark.parametrize("R,N,C,head,bias_heads,fused", [
+    (1, 1, 64, 1, 1, True), (768, 768, 128, 4, 4, True), (768, 768, 128, 2, 4, True), (768, 768, 64, 8, 0, True),
+    (768, 768, 128, 1, 1, False),                # heads of 128 channels: the attention kernel takes 64
+    (768, 768, 64, 16, 4, False), (768, 768, 128, 3, 3, False), (768, 768, 128, 0, 0, False),
+    (768, 768, 128, 8, 8, False), (768, 768, 96, 4, 4, False), (0, 768, 128, 4, 4, False),
+    (4095, 4096, 128, 4, 4, True), (4096, 4096, 128, 4, 4, False),      # 2^31 elements
+    (5792, 5792, 64, 4, 4, True), (5793, 5793, 64, 4, 4, False), (2 ** 40, 2 ** 40, 64, 4, 4, False)])
+def test_grid_dispatch_takes_what_its_kernels_take(R, N, C, head, bias_heads, fused):
+    """The fused route is chosen for exactly the sizes that the front and the attention kernel accept; the front's entry
+    point refuses the oversize ones by itself, without overflow."""
+    assert _capi.host().grid_sizes_fused(R, N, C, head, bias_heads) is fused
+    if C in (64, 128) and head and C % head == 0 and C // head % 8 == 0 and bias_heads <= 4 and R * N * C > 2 ** 31 - 1:
+        front = _capi.load().af3k_grid_front
+        front.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_float, ctypes.c_void_p] + \
+            [ctypes.c_longlong, ctypes.c_void_p] + [ctypes.c_longlong] * 4 + [ctypes.c_float, ctypes.c_int32, ctypes.c_void_p,
+                                                                             ctypes.c_longlong] + [ctypes.c_void_p] * 6
+        one = 16
+        assert front(one, _capi.AF3K_BF16, one, one, 1e-5, one, bias_heads, one, R, N, C, head, 1.0, 0, one, (N + 7) // 8 * 8, one, one,
+                     one, one, None, None) == 2
+    d = _desc(1, head, 128, C // head) if head and C % head == 0 else None
+    if fused:
+        assert _capi.load().af3k_describe_plan(ctypes.byref(d), (ctypes.c_int32 * 6)()) == 0
