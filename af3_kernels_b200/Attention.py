@@ -12,7 +12,7 @@ import torch.nn as nn
 
 from . import _capi, pair_bias
 from .dpa import bool_mask
-from .fused_ops import attention_block
+from .fused_ops import attention_block, differentiates
 from .tools import profile
 
 
@@ -54,9 +54,11 @@ class GridSelfAttentionCpp(nn.Module):
         if host.grid_fused(pair, self.num_head, self.num_head) and mask is not None:
             # c_pair 64 or 128, up to four heads: three launches, LayerNorm to output projection
             lin = (self.q_projection, self.k_projection, self.v_projection, self.gating_query, self.output_projection)
-            return host.grid_module(pair, bool_mask(mask, *pair.shape[:2]),
-                                    [m.weight for m in lin] + [self.act_norm.weight, self.act_norm.bias, self.pair_bias_projection.weight],
-                                    self.act_norm.eps, self.num_head, self.transpose)
+            by_torch = differentiates(self.output_projection.weight)
+            out = host.grid_module(pair, bool_mask(mask, *pair.shape[:2]),
+                                   [m.weight for m in lin] + [self.act_norm.weight, self.act_norm.bias, self.pair_bias_projection.weight],
+                                   self.act_norm.eps, self.num_head, self.transpose, not by_torch)
+            return torch.matmul(out, self.output_projection.weight.T.to(out.dtype)).to(pair.dtype) if by_torch else out
         dtype = pair.dtype
         pair, bias = self._norm_and_bias(pair)
         if self.transpose:

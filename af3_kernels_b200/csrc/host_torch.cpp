@@ -34,6 +34,7 @@ struct Library {
   decltype(&af3k_stage_bias) stage_bias = nullptr;
   decltype(&af3k_grid_front_weights) grid_front = nullptr;
   decltype(&af3k_grid_out) grid_out = nullptr;
+  decltype(&af3k_sigmoid_gate) sigmoid_gate = nullptr;
   decltype(&af3k_grid_pack) grid_pack = nullptr;
   decltype(&af3k_token_projection_weights) token_projection = nullptr;
 };
@@ -53,6 +54,7 @@ void bind_library(const std::string& path) {
   AF3K_BIND(stage_bias, af3k_stage_bias);
   AF3K_BIND(grid_front, af3k_grid_front_weights);
   AF3K_BIND(grid_out, af3k_grid_out);
+  AF3K_BIND(sigmoid_gate, af3k_sigmoid_gate);
   AF3K_BIND(grid_pack, af3k_grid_pack);
   AF3K_BIND(token_projection, af3k_token_projection_weights);
 #undef AF3K_BIND
@@ -378,8 +380,9 @@ bool grid_fused(const Tensor& pair, int64_t head, int64_t bias_heads) {
 // The whole module: raw pair [N, N, C] -> front (LayerNorm, bias, q / k / v / gate) -> attention -> gate and output
 // projection, three launches.  weights: nn.Linear.weight of q, k, v, gate, output; then LayerNorm weight and bias,
 // bias projection.  transpose: attention along the columns of the pair; q, k, v are written, and the result is
-// read back, in the exchanged order, so nothing is permuted in memory.
-Tensor grid_module(Tensor pair, const Tensor& mask_in, const std::vector<Tensor>& params, double eps, int64_t head, bool transpose) {
+// read back, in the exchanged order, so nothing is permuted in memory.  project false: up to the gated result (bf16),
+// for an output projection that torch differentiates.
+Tensor grid_module(Tensor pair, const Tensor& mask_in, const std::vector<Tensor>& params, double eps, int64_t head, bool transpose, bool project) {
   const at::Device dev = pair.device();
   const c10::cuda::CUDAGuard guard(dev);
   const int64_t R = pair.size(0), N = pair.size(1), C = pair.size(2), D = C / head, M = R * N;
@@ -397,7 +400,7 @@ Tensor grid_module(Tensor pair, const Tensor& mask_in, const std::vector<Tensor>
   const int64_t pitch = (N + 7) / 8 * 8;
   Tensor bias = at::empty({head, N, pitch}, bf16);
   Tensor buf = at::empty({5, M, C}, bf16);           // q, k, v, gate, attention result
-  Tensor out = at::empty({R, N, C}, pair.options());
+  Tensor out = at::empty({R, N, C}, project ? pair.options() : bf16);
   char* b = static_cast<char*>(buf.data_ptr());
   const size_t part = (size_t)M * C * 2;
   void *q = b, *k = b + part, *v = b + 2 * part, *gate = b + 3 * part, *weighted = b + 4 * part;
@@ -415,13 +418,14 @@ Tensor grid_module(Tensor pair, const Tensor& mask_in, const std::vector<Tensor>
   d.softmax_scale = 1.0f;                            // q left the projection scaled
   check(g_lib.attention(&d, q, k, v, bias.data_ptr(), static_cast<const uint8_t*>(mask.data_ptr()), weighted, nullptr, nullptr, nullptr, 0,
                         status, stream));
-  check(g_lib.grid_out(weighted, gate, w.wo, out.data_ptr(), f32 ? AF3K_F32 : AF3K_BF16, M, C, status, stream));
+  if (!project) check(g_lib.sigmoid_gate(weighted, gate, out.data_ptr(), M * C, stream));
+  else check(g_lib.grid_out(weighted, gate, w.wo, out.data_ptr(), f32 ? AF3K_F32 : AF3K_BF16, M, C, status, stream));
   return out;
 }
 
 // The block on an already normalised pair [R, N, C] with a bias of the caller's.  weights: q, k, v, gate, output as
 // [out, in].
-Tensor grid_block(const Tensor& pair, const OptTensor& mask, const Tensor& bias, const std::vector<Tensor>& weights, int64_t head) {
+Tensor grid_block(const Tensor& pair, const OptTensor& mask, const Tensor& bias, const std::vector<Tensor>& weights, int64_t head, bool project) {
   const at::Device dev = pair.device();
   const c10::cuda::CUDAGuard guard(dev);
   const int64_t R = pair.size(0), N = pair.size(1), C = pair.size(2), D = C / head, M = R * N;
@@ -434,12 +438,13 @@ Tensor grid_block(const Tensor& pair, const OptTensor& mask, const Tensor& bias,
   auto at_part = [&](int i, at::IntArrayRef sizes) { return buf.select(0, i).view(sizes); };
   Tensor q = at_part(0, {R, head, N, D}), k = at_part(1, {R, head, N, D}), v = at_part(2, {R, head, N, D});
   Tensor gate = at_part(3, {M, C}), weighted = at_part(4, {R, N, head, D});
-  Tensor out = at::empty({R, N, C}, x.options().dtype(pair.scalar_type()));
+  Tensor out = at::empty({R, N, C}, project ? x.options().dtype(pair.scalar_type()) : x.options());
   int* status = status_buffer(dev.index()).data_ptr<int>();
   check(g_lib.grid_front(x.data_ptr(), AF3K_BF16, &w.front, 0.f, 0, R, N, C, head, 1.0f / std::sqrt((float)D), 0, nullptr, 0, q.data_ptr(),
                          k.data_ptr(), v.data_ptr(), gate.data_ptr(), status, stream));
   attention(q, k, v, mask, bias, std::nullopt, std::nullopt, 1.0, 0, weighted.permute({0, 2, 1, 3}), true, true, 0, 0);
-  check(g_lib.grid_out(weighted.data_ptr(), gate.data_ptr(), w.wo, out.data_ptr(), pair.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16,
+  if (!project) check(g_lib.sigmoid_gate(weighted.data_ptr(), gate.data_ptr(), out.data_ptr(), M * C, stream));
+  else check(g_lib.grid_out(weighted.data_ptr(), gate.data_ptr(), w.wo, out.data_ptr(), pair.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16,
                        M, C, status, stream));
   return out;
 }

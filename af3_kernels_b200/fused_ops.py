@@ -101,6 +101,12 @@ def pair_front(pair: torch.Tensor, ln_weight: torch.Tensor, ln_bias: torch.Tenso
     return bias[:, :, :N], q, k, v, g
 
 
+def differentiates(out_proj: torch.Tensor) -> bool:
+    """Whether the output projection has to be torch's own: the blocks' kernels have no backward pass, but behind them
+    a gradient of the output projection is exact, and a program may train just that."""
+    return torch.is_grad_enabled() and out_proj.requires_grad
+
+
 def attention_block(
     pair: torch.Tensor,
     mask: torch.Tensor,
@@ -126,8 +132,10 @@ def attention_block(
     if host.grid_fused(pair, head, 0):
         # c_pair 64 or 128: one pass over x for all four projections (q, k, v leave head-major with q already
         # scaled), the attention core, and one pass for the gate and the output projection
-        return host.grid_block(pair, bool_mask(mask, R, N), bias,
-                               [w.t() for w in (q_proj, k_proj, v_proj, gating_query, out_proj)], head)
+        by_torch = differentiates(out_proj)
+        out = host.grid_block(pair, bool_mask(mask, R, N), bias,
+                              [w.t() for w in (q_proj, k_proj, v_proj, gating_query, out_proj)], head, not by_torch)
+        return torch.matmul(out, _as_bf16(out_proj)).to(pair.dtype) if by_torch else out
     x = _as_bf16(pair)
     q = torch.matmul(x, _as_bf16(q_proj)).view(R, N, head, D).permute(0, 2, 1, 3)
     k = torch.matmul(x, _as_bf16(k_proj)).view(R, N, head, D).permute(0, 2, 1, 3)

@@ -462,3 +462,28 @@ def test_parameters_on_another_device_are_refused(cuda_device, C):
             A.dot_product_attention(q, q, q, None, torch.zeros(2, 16, 16, device=dev), out=q.cpu())
     torch.cuda.synchronize()
     assert read_status(dev)[0] == 0
+
+
+@pytest.mark.parametrize("C,dtype,transpose", [(64, torch.bfloat16, False), (128, torch.float32, True), (128, torch.bfloat16, False)])
+def test_output_projection_has_a_gradient(cuda_device, C, dtype, transpose):
+    """Outside no_grad the result carries the gradient of the output projection (out = gated Wo^T is linear in it), and is
+    the result under no_grad up to bf16 rounding; module and functional block."""
+    g = torch.Generator().manual_seed(C)
+    H, N = 4, 40
+    m = A.GridSelfAttentionCpp(C, H, transpose).to(cuda_device, dtype)
+    pair = torch.randn(N, N, C, generator=g).to(cuda_device, dtype)
+    mask = torch.ones(N, N, dtype=torch.bool, device=cuda_device)
+    bias = torch.randn(H, N, N, generator=g).to(cuda_device, torch.bfloat16)
+    wo = m.output_projection.weight
+    for call in (lambda: m(pair, mask), lambda: A._attention_cpp(pair, mask, bias, *m._weights(), H)):
+        with torch.no_grad():
+            want = call()
+        out = call()
+        assert out.dtype == dtype and out.requires_grad and not want.requires_grad
+        scale = want.float().abs().max().item()
+        assert (out.detach().float() - want.float()).abs().max().item() <= 2.0 ** -7 * scale
+        wo.grad = None
+        (out.float() * want.float()).sum().backward()
+        # sum(out * c) is linear in Wo: its derivative along Wo itself is its value
+        along, value = (wo.grad.float() * wo.detach().float()).sum().item(), (out.detach().float() * want.float()).sum().item()
+        assert abs(along - value) <= 2e-2 * abs(value)
