@@ -48,10 +48,20 @@ class GridSelfAttentionCpp(nn.Module):
         bias = self.pair_bias_projection(pair).permute(2, 0, 1)     # [H, N, N]
         return pair, bias
 
+    def _norm_and_bias_as_built(self, pair: torch.Tensor) -> bool:
+        """Whether LayerNorm and bias projection may be computed from their parameters.  At c_pair = 128 they always are;
+        other widths call the two modules, so one that was replaced or carries hooks has to run."""
+        if pair_bias.supported(pair, self.num_head):
+            return True
+        norm, proj = self.act_norm, self.pair_bias_projection
+        return (type(norm) is nn.LayerNorm and norm.weight is not None and norm.bias is not None
+                and type(proj) is nn.Linear and proj.bias is None
+                and not any(m._forward_hooks or m._forward_pre_hooks for m in (norm, proj)))
+
     @profile("B200 GridSelfAttention")
     def forward(self, pair: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
         host = _capi.host()
-        if host.grid_fused(pair, self.num_head, self.num_head) and mask is not None:
+        if host.grid_fused(pair, self.num_head, self.num_head) and mask is not None and self._norm_and_bias_as_built(pair):
             # c_pair 64 or 128, up to four heads: three launches, LayerNorm to output projection
             lin = (self.q_projection, self.k_projection, self.v_projection, self.gating_query, self.output_projection)
             by_torch = differentiates(self.output_projection.weight)

@@ -487,3 +487,24 @@ def test_output_projection_has_a_gradient(cuda_device, C, dtype, transpose):
         # sum(out * c) is linear in Wo: its derivative along Wo itself is its value
         along, value = (wo.grad.float() * wo.detach().float()).sum().item(), (out.detach().float() * want.float()).sum().item()
         assert abs(along - value) <= 2e-2 * abs(value)
+
+
+def test_norm_and_bias_modules_that_were_hooked_or_replaced_run(cuda_device):
+    """At 64 channels LayerNorm and bias projection are the module's own: hooks on them fire, and one put in their place
+    is used."""
+    C, H, N = 64, 4, 24
+    m = A.GridSelfAttentionCpp(C, H).to(cuda_device).eval()
+    pair = torch.randn(N, N, C, generator=torch.Generator().manual_seed(1)).to(cuda_device)
+    mask = torch.ones(N, N, dtype=torch.bool, device=cuda_device)
+    with torch.no_grad():
+        plain = m(pair, mask)
+        seen = []
+        hooks = [x.register_forward_hook(lambda mod, a, out: seen.append(type(mod))) for x in (m.act_norm, m.pair_bias_projection)]
+        hooked = m(pair, mask)
+        assert seen == [torch.nn.LayerNorm, torch.nn.Linear]
+        _close(hooked, plain.cpu(), "hooked")
+        for h in hooks:
+            h.remove()
+        assert torch.equal(m(pair, mask), plain)
+        m.act_norm = torch.nn.LayerNorm(C, elementwise_affine=False, device=cuda_device)
+        _close(m(pair, mask), plain.cpu(), "without affine parameters (they were one and zero)")
