@@ -913,7 +913,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                   const float g = __uint_as_float((e & 1) ? gw[e >> 1] & 0xffff0000u : gw[e >> 1] << 16);
-                  o[hseg * 8 + e] = __float_as_uint(__uint_as_float(o[hseg * 8 + e]) * sigmoid_fast(g));
+                  o[hseg * 8 + e] = __float_as_uint(__uint_as_float(o[hseg * 8 + e]) * sigmoid_f32(g));
                 }
               }
               uint4 v;

@@ -594,8 +594,8 @@ grid_out_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CU
           uint32_t r[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e)
-            r[e] = pack_bf16x2(__uint_as_float(aw[e] << 16) * sigmoid_fast(__uint_as_float(gw[e] << 16)),
-                               __uint_as_float(aw[e] & 0xffff0000u) * sigmoid_fast(__uint_as_float(gw[e] & 0xffff0000u)));
+            r[e] = pack_bf16x2(__uint_as_float(aw[e] << 16) * sigmoid_f32(__uint_as_float(gw[e] << 16)),
+                               __uint_as_float(aw[e] & 0xffff0000u) * sigmoid_f32(__uint_as_float(gw[e] & 0xffff0000u)));
           const int row = w * kGridRowsPerWarp + (it0 + u) * kRowsIt + sub;
           sts128(grid_piece(x_tile, row, c8), r[0], r[1], r[2], r[3]);
         }

@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(256) sigmoid_gate_kernel(const uint4* __restri
     for (int e = 0; e < 4; ++e) {
       const float a0 = __uint_as_float(aw[e] << 16), a1 = __uint_as_float(aw[e] & 0xffff0000u);
       const float g0 = __uint_as_float(gw[e] << 16), g1 = __uint_as_float(gw[e] & 0xffff0000u);
-      r[e] = pb_pack_bf16x2(a0 * sigmoid_fast(g0), a1 * sigmoid_fast(g1));
+      r[e] = pb_pack_bf16x2(a0 * sigmoid_f32(g0), a1 * sigmoid_f32(g1));
     }
     out[i] = make_uint4(r[0], r[1], r[2], r[3]);
   }

@@ -508,3 +508,39 @@ def test_norm_and_bias_modules_that_were_hooked_or_replaced_run(cuda_device):
         assert torch.equal(m(pair, mask), plain)
         m.act_norm = torch.nn.LayerNorm(C, elementwise_affine=False, device=cuda_device)
         _close(m(pair, mask), plain.cpu(), "without affine parameters (they were one and zero)")
+
+
+def _gate_values(device):
+    """Every bf16 gate from -88.5 to 88.5, on 128 channels (below -128 ln 2 = -88.7 the exponential is past fp32 and the
+    sigmoid, under 2^-128, is zero)."""
+    bits = torch.arange(2 ** 16, dtype=torch.int32).to(torch.uint16).view(torch.bfloat16)
+    g = bits[bits.float().abs() <= 88.5]
+    return torch.nn.functional.pad(g, (0, -g.numel() % 128)).view(-1, 128).to(device)
+
+
+def _gated(weighted, gate):
+    """weighted * sigmoid(gate) in 64 bits, and the tolerance of its bf16 rounding: half an ulp (relative 2^-8), the
+    rounding of the exponent (up to 128, so 2^-18 ln 2) with a few fp32 ulps, and the smallest bf16 step below the normal
+    range."""
+    want = weighted.double() * torch.sigmoid(gate.double())
+    return want, want.abs() * (2.0 ** -8 + 2.0 ** -17) + 2.0 ** -133
+
+
+@pytest.mark.parametrize("factor", [1.0, 2.0 ** 100])
+def test_sigmoid_gate_over_every_gate(cuda_device, factor):
+    """The gate kernel and the gated output pass (identity weights), down to where the sigmoid is denormal."""
+    from af3_kernels_b200 import _capi
+    from af3_kernels_b200.fused_ops import sigmoid_gate
+    gate = _gate_values(cuda_device)
+    w = torch.full_like(gate, factor)
+    want, tol = _gated(w, gate)
+    got = sigmoid_gate(w, gate)
+    assert ((got.double() - want).abs() <= tol).all()
+    import ctypes
+    out = torch.empty(gate.shape, device=cuda_device)
+    eye = torch.eye(128, device=cuda_device, dtype=torch.bfloat16)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    i64 = ctypes.c_longlong
+    _capi.check(_capi.load().af3k_grid_out(p(w), p(gate), p(eye), p(out), _capi.AF3K_F32, i64(gate.shape[0]), i64(128), None,
+                                           ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    assert ((out.double() - want).abs() <= tol).all()
