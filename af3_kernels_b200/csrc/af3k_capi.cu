@@ -108,9 +108,9 @@ int device_info(DeviceInfo** out) {
     if ((e = cudaFuncSetAttribute(pair_bias_mma_kernel, attr, kPbmSmemBytes)) != cudaSuccess)
       return cuda_fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize, pair_bias_mma)", e);
     const std::pair<const void*, uint32_t> gemm_kernels[] = {
-        {(const void*)grid_front_kernel<128, __nv_bfloat16, true>, FrontTile<128>::kSmem}, {(const void*)grid_front_kernel<128, float, true>, FrontTile<128>::kSmem},
-        {(const void*)grid_front_kernel<128, __nv_bfloat16, false>, FrontTile<128>::kSmem}, {(const void*)grid_front_kernel<64, __nv_bfloat16, true>, FrontTile<64>::kSmem},
-        {(const void*)grid_front_kernel<64, float, true>, FrontTile<64>::kSmem}, {(const void*)grid_front_kernel<64, __nv_bfloat16, false>, FrontTile<64>::kSmem},
+        {(const void*)grid_front_kernel<128, __nv_bfloat16, true>, FrontTile<128, __nv_bfloat16>::kSmem}, {(const void*)grid_front_kernel<128, float, true>, FrontTile<128, float>::kSmem},
+        {(const void*)grid_front_kernel<128, __nv_bfloat16, false>, FrontTile<128, __nv_bfloat16>::kSmem}, {(const void*)grid_front_kernel<64, __nv_bfloat16, true>, FrontTile<64, __nv_bfloat16>::kSmem},
+        {(const void*)grid_front_kernel<64, float, true>, FrontTile<64, float>::kSmem}, {(const void*)grid_front_kernel<64, __nv_bfloat16, false>, FrontTile<64, __nv_bfloat16>::kSmem},
         {(const void*)grid_out_kernel<128, __nv_bfloat16>, OutTile<128>::kSmem}, {(const void*)grid_out_kernel<128, float>, OutTile<128>::kSmem},
         {(const void*)grid_out_kernel<64, __nv_bfloat16>, OutTile<64>::kSmem}, {(const void*)grid_out_kernel<64, float>, OutTile<64>::kSmem},
         {(const void*)token_proj_kernel<64>, TokTile<64>::kSmem}, {(const void*)token_proj_kernel<128>, TokTile<128>::kSmem},
@@ -713,7 +713,7 @@ int encode_weight_map(CUtensorMap* tm, const void* w, int64_t C, int64_t rows) {
 
 template <int C>
 void launch_front(const GridParams& p, const FrontMaps& tm, unsigned grid, bool f32, bool ln, cudaStream_t stream) {
-  constexpr uint32_t smem = FrontTile<C>::kSmem;
+  const uint32_t smem = f32 ? FrontTile<C, float>::kSmem : FrontTile<C, __nv_bfloat16>::kSmem;
   if (!ln)      launch_overlapped(grid_front_kernel<C, __nv_bfloat16, false>, dim3(grid), kGridThreads, smem, stream, true, p, tm);
   else if (f32) launch_overlapped(grid_front_kernel<C, float, true>, dim3(grid), kGridThreads, smem, stream, true, p, tm);
   else          launch_overlapped(grid_front_kernel<C, __nv_bfloat16, true>, dim3(grid), kGridThreads, smem, stream, true, p, tm);

@@ -48,13 +48,15 @@ static_assert(128 * kGridRegsMisc + 256 * kGridRegsEpi + 256 * kGridRegsRows <= 
               "setmaxnreg totals exceed the launch allocation");
 
 // Shared memory: kRows weight rows per panel of 64 channels, the A tiles, the epilogue patches, barriers.
-template <int C, int kRowsT, int kStagesT>
+template <int C, int kRowsT, int kStagesT, bool kLowT = false>
 struct GridTile {
   static constexpr int kStages = kStagesT, kRows = kRowsT;
+  static constexpr bool kLow = kLowT;                      // a second A tile per stage for what bf16 leaves over of x
   static constexpr uint32_t kX = 128 * C * 2;              // one A tile: C / 64 panels of 128 rows x 128 bytes
   static constexpr uint32_t kW = kRows * C * 2;            // weights: C / 64 panels of kRows rows x 128 bytes
   static constexpr uint32_t kPatch = 8 * 32 * 128;         // per epilogue warp: 32 rows x 128 bytes
-  static constexpr uint32_t off_x = kW, off_patch = off_x + kStages * kX, off_bar = off_patch + kPatch;
+  static constexpr uint32_t off_x = kW, off_low = off_x + kStages * kX, off_patch = off_low + (kLow ? kStages * kX : 0);
+  static constexpr uint32_t off_bar = off_patch + kPatch;
   static constexpr uint32_t off_slot = off_bar + 120;      // TMEM address, abort flag
   static constexpr uint32_t kSmem = off_bar + 128;
 };
@@ -62,7 +64,10 @@ struct GridTile {
 // 0-3, plus a bf16 low part, rows 4-7, so that it is not rounded to bf16), then the k, v and gate rows: the
 // bias comes out of the q rows' MMAs as 16 more columns (the upper eight read k rows and are not used).
 constexpr int kBiasRows = 8;
-template <int C> using FrontTile = GridTile<C, 4 * C + kBiasRows, C == 128 ? 2 : 4>;
+// fp32 pairs of 64 channels: x goes to the bias rows' MMAs in two parts as well, so that the bias is that of the fp32
+// normalised pair, as torch's LayerNorm and Linear compute it for other widths (at 128 channels af3k_pair_bias rounds x
+// first, and so does this).
+template <int C, typename T> using FrontTile = GridTile<C, 4 * C + kBiasRows, C == 128 ? 2 : 4, C == 64 && sizeof(T) == 4>;
 template <int C> using OutTile = GridTile<C, C, 4>;
 constexpr int kFrontAcc = 3;     // accumulators of C + 16 (rounded up to C + 32) TMEM columns, taken in turn
 
@@ -216,7 +221,7 @@ __device__ __forceinline__ void grid_epilogue_common(volatile int* abort_flag, u
 template <int C, typename T, bool kLn>
 __global__ void __launch_bounds__(kGridThreads, 1)
 grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ FrontMaps maps) {
-  using Tile = FrontTile<C>;
+  using Tile = FrontTile<C, T>;
   extern __shared__ __align__(1024) uint8_t grid_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t smem = smem_u32(grid_smem);
@@ -279,6 +284,16 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
               const uint32_t a = ad_lo + ((st * Tile::kX + (ks >> 2) * (128 * 128)) >> 4) + 2 * (ks & 3);
               const uint32_t b = bd_lo + (((ks >> 2) * (Tile::kRows * 128) + row * 128) >> 4) + 2 * (ks & 3);
               mma_ss_f16(tmem + buf * kAccCols, a, ad_hi, b, bd_hi, id, ks > 0 ? 1u : 0u);
+            }
+            if (Tile::kLow && c == 0 && with_bias) {
+              // onto the bias columns alone (N = 16: the eight bias rows and eight that are not used)
+              constexpr uint32_t idesc_low = make_idesc(1u, 1u, 0u, 0u, 16);
+#pragma unroll
+              for (int ks = 0; ks < C / 16; ++ks) {
+                const uint32_t a = ad_lo + ((Tile::off_low - Tile::off_x + st * Tile::kX + (ks >> 2) * (128 * 128)) >> 4) + 2 * (ks & 3);
+                const uint32_t b = bd_lo + (((ks >> 2) * (Tile::kRows * 128) + C * 128) >> 4) + 2 * (ks & 3);
+                mma_ss_f16(tmem + buf * kAccCols + C, a, ad_hi, b, bd_hi, idesc_low, 1u);
+              }
             }
             tc_commit(bars + 8u * (GridBar::acc_full + buf));
             if (c == chunks - 1) tc_commit(bars + 8u * (GridBar::x_empty + st));
@@ -453,6 +468,13 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
           for (int e = 0; e < 4; ++e) yw[u][e] = pack_bf16x2(y[u][2 * e], y[u][2 * e + 1]);
           const int row = w * kGridRowsPerWarp + (it0 + u) * kRowsIt + sub;
           sts128(grid_piece(x_tile, row, c8), yw[u][0], yw[u][1], yw[u][2], yw[u][3]);
+          if (Tile::kLow && with_bias) {
+            uint32_t lw[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              lw[e] = pack_bf16x2(y[u][2 * e] - __uint_as_float(yw[u][e] << 16), y[u][2 * e + 1] - __uint_as_float(yw[u][e] & 0xffff0000u));
+            sts128(grid_piece(x_tile + Tile::off_low - Tile::off_x, row, c8), lw[0], lw[1], lw[2], lw[3]);
+          }
         }
       }
       fence_proxy_async_smem();     // the tile was written through the generic proxy; the tensor core reads it

@@ -544,3 +544,30 @@ def test_sigmoid_gate_over_every_gate(cuda_device, factor):
     _capi.check(_capi.load().af3k_grid_out(p(w), p(gate), p(eye), p(out), _capi.AF3K_F32, i64(gate.shape[0]), i64(128), None,
                                            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
     assert ((out.double() - want).abs() <= tol).all()
+
+
+@pytest.mark.parametrize("R,N", [(3, 50), (40, 129), (160, 160)])
+def test_bias_of_a_narrow_fp32_pair_is_that_of_the_fp32_normalised_pair(cuda_device, R, N):
+    """64 channels, fp32: LayerNorm and bias projection against 64 bits.  x and the weights enter as two bf16 parts
+    (2^-16 relative each) and the sums are fp32, so the bound is half a bf16 ulp of the result (2^-8 relative) plus 2^-14
+    of the sum of absolute products; a bias of the rounded x is off by up to 2^-8 of it.  Tiles split over CTAs and not."""
+    import ctypes
+    from af3_kernels_b200 import _capi
+    g = torch.Generator().manual_seed(R)
+    C, H, Hb, dev = 64, 4, 3, cuda_device
+    pair = (torch.randn(R, N, C, generator=g) * 2 + 0.3).to(dev)
+    gamma, beta = (1 + 0.2 * torch.randn(C, generator=g)).to(dev), (0.1 * torch.randn(C, generator=g)).to(dev)
+    bw = (torch.randn(Hb, C, generator=g) * 0.3).to(dev)
+    w4 = torch.zeros(4 * C, C, dtype=torch.bfloat16, device=dev)
+    pitch = (N + 7) // 8 * 8
+    bias = torch.empty(Hb, R, pitch, dtype=torch.bfloat16, device=dev)
+    q, k, v, gate = (torch.empty(R * N * C, dtype=torch.bfloat16, device=dev) for _ in range(4))
+    p, i64, f = (lambda t: ctypes.c_void_p(t.data_ptr())), ctypes.c_longlong, ctypes.c_float
+    _capi.check(_capi.load().af3k_grid_front(
+        p(pair), ctypes.c_int32(_capi.AF3K_F32), p(gamma), p(beta), f(1e-5), p(bw), i64(Hb), p(w4), i64(R), i64(N), i64(C), i64(H), f(1.0),
+        ctypes.c_int32(0), p(bias), i64(pitch), p(q), p(k), p(v), p(gate), None, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    x = torch.nn.functional.layer_norm(pair.double(), (C,), gamma.double(), beta.double(), 1e-5)
+    want = torch.einsum("rnc,hc->hrn", x, bw.double())
+    size = torch.einsum("rnc,hc->hrn", x.abs(), bw.double().abs())
+    err = (bias[:, :, :N].double() - want).abs()
+    assert (err <= want.abs() * 2.0 ** -8 + size * 2.0 ** -14).all(), (err / size).max()
