@@ -587,8 +587,7 @@ int af3k_describe_plan(const af3k_attention_desc* desc, int32_t* out6) {
   if (rc != AF3K_OK) return rc;
   out6[0] = plan.p.G;
   out6[1] = plan.p.kv_stages;
-  // with one pair row per item always the number of query-tile pairs, also where each tile is an item of its own
-  out6[2] = plan.p.G == 1 && plan.p.n_qt >= 2 && !plan.p.q_split ? plan.p.B1 * plan.p.B2 * ((plan.p.n_qt + 1) / 2) : plan.p.n_items;
+  out6[2] = plan.p.n_items;
   out6[3] = plan.grid;
   out6[4] = (int32_t)plan.smem_bytes;
   out6[5] = (int32_t)kOCol + plan.p.n_streams * plan.p.nv;

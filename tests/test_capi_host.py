@@ -54,7 +54,7 @@ def _desc(B1, B2, S, D, bias_dtype=_capi.AF3K_F32, qk=_capi.AF3K_BF16):
 
 
 @pytest.mark.parametrize("shape", [(1, 16, 512, 32), (768, 4, 768, 32), (1, 16, 1536, 24),
-                                   (5, 16, 1536, 48), (2048, 4, 2048, 32)])
+                                   (5, 16, 1536, 48), (2048, 4, 2048, 32), (1, 16, 1152, 32), (1, 16, 1153, 32)])
 def test_launch_plan_fits_b200(shape):
     plan = _capi.describe_plan(_desc(*shape))
     assert 1 <= plan["rows_per_item"] <= 8
@@ -65,9 +65,10 @@ def test_launch_plan_fits_b200(shape):
     B1, B2, S, _ = shape
     groups = -(-B1 // plan["rows_per_item"])
     n_qt = -(-S // 128)
-    if plan["rows_per_item"] == 1 and n_qt >= 2:    # one pair row per item: two query tiles per item
+    if plan["rows_per_item"] == 1 and B1 * B2 * n_qt > 148:    # not an SM for every query tile: two per item
         n_qt = -(-n_qt // 2)
     assert plan["items"] == groups * B2 * n_qt
+    assert plan["grid"] <= plan["items"]
 
 
 def test_max_ctas_caps_the_grid():
