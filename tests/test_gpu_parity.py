@@ -481,3 +481,45 @@ def test_bias_of_another_shape_is_reshaped(cuda_device, dtype):
         assert torch.equal(A.dot_product_attention(q, k, v, None, stage_bias(b, B2, S, S)), want), shape
         assert torch.equal(block(b), want_block), shape
         assert torch.equal(A.dot_product_attention_host(q.cpu(), k.cpu(), v.cpu(), None, b.cpu()), want.cpu()), shape
+
+
+@pytest.mark.parametrize("fp8,workspace", [(False, False), (True, True), (True, False)])
+@pytest.mark.parametrize("B1,B2,S,D", [(1, 3, 77, 24), (2, 4, 200, 32), (3, 2, 129, 64)])
+def test_gated_result_of_every_kernel_variant(cuda_device, fp8, workspace, B1, B2, S, D):
+    """The descriptor's gate through the C ABI, rows with a pitch of their own: bf16 q and k, and fp8 on both of its
+    kernels (with a workspace the tensor core adds the bias, without one the softmax threads do)."""
+    g = torch.Generator().manual_seed(S)
+    dev = cuda_device
+    q, k, v = (torch.randn(B1, B2, S, D, generator=g).to(torch.bfloat16) for _ in range(3))
+    scales = {}
+    if fp8:
+        if D % 16:
+            pytest.skip("fp8 rows are 16-byte multiples")
+        q, k = q.to(torch.float8_e4m3fn), k.to(torch.float8_e4m3fn)
+        scales = {n: torch.rand(B2, generator=g) * 0.5 + 0.5 for n in ("q_scale", "k_scale")}
+    pitch = (S + 7) // 8 * 8
+    bias = torch.randn(B2, S, pitch, generator=g).to(torch.bfloat16)
+    gate = (torch.randn(B1, S, B2 + 1, D, generator=g) * 3).to(torch.bfloat16)      # [B1, S, H, D]: one head more than used
+    mask = torch.rand(B1, S, generator=g) >= 0.1
+    gated = gate[:, :, :B2].permute(0, 2, 1, 3)
+    ref = O.oracle_fp32(q, k, v, mask, bias[:, :, :S], **scales) * torch.sigmoid(gated.float())
+    qd, kd, vd, bd, gd, md = (t.to(dev) for t in (q, k, v, bias, gate, mask))
+    sd = {n: t.to(dev) for n, t in scales.items()}
+    out = torch.empty(B1, B2, S, D, dtype=torch.bfloat16, device=dev)
+    d = _capi.AttentionDesc()
+    d.B1, d.B2, d.Sq, d.Sk, d.D = B1, B2, S, S, D
+    for name, t in (("q_stride", qd), ("k_stride", kd), ("v_stride", vd), ("out_stride", out), ("gate_stride", gd[:, :, :B2].permute(0, 2, 1, 3))):
+        getattr(d, name)[:] = list(t.stride()[:3])
+    d.bias_stride[:] = [S * pitch, pitch]
+    d.mask_row_stride, d.softmax_scale = S, D ** -0.5
+    d.qk_dtype, d.bias_dtype, d.gate = (_capi.AF3K_FP8_E4M3 if fp8 else _capi.AF3K_BF16), _capi.AF3K_BF16, gd.data_ptr()
+    lib, p = _capi.load(), lambda t: None if t is None else t.data_ptr()
+    n = lib.af3k_dot_product_attention_workspace(ctypes.byref(d), p(bd)) if workspace else 0
+    ws = torch.empty(n, dtype=torch.uint8, device=dev) if n else None
+    _capi.check(lib.af3k_dot_product_attention(
+        ctypes.byref(d), p(qd), p(kd), p(vd), p(bd), p(md.view(torch.uint8)), p(out), p(sd.get("q_scale")), p(sd.get("k_scale")), p(ws), n,
+        None, torch.cuda.current_stream().cuda_stream))
+    if fp8:
+        assert O.error_stats(out.cpu(), ref)["max_abs"] <= FP8_MAX_ABS
+    else:
+        _check_bf16(out.cpu(), ref, (B1, B2, S, D))
