@@ -664,6 +664,12 @@ PYBIND11_MODULE(_host, m) {
   m.def("grid_module", &grid_module, py::call_guard<py::gil_scoped_release>());
   m.def("grid_block", &grid_block, py::call_guard<py::gil_scoped_release>());
   m.def("self_block", &self_block, py::call_guard<py::gil_scoped_release>());
+  m.def("stage_bias", [](const Tensor& bias, int64_t B2, int64_t Sq, int64_t Sk, int64_t D, const OptTensor& q_scale, const OptTensor& k_scale,
+                         double scale) {
+    const c10::cuda::CUDAGuard guard(bias.device());
+    return make_staged(bias, B2, Sq, Sk, D, q_scale ? q_scale->data_ptr<float>() : nullptr, k_scale ? k_scale->data_ptr<float>() : nullptr,
+                       (float)scale, c10::cuda::getCurrentCUDAStream(bias.device().index()));
+  }, py::call_guard<py::gil_scoped_release>());
   m.def("host_attention", &host_attention, py::call_guard<py::gil_scoped_release>());
   m.def("bind_library", &bind_library);
   m.def("status_buffer", &status_buffer);

@@ -9,7 +9,6 @@ call on host tensors.  There is no CPU path.
 """
 from __future__ import annotations
 
-import ctypes
 import math
 import os
 from typing import Optional
@@ -53,30 +52,14 @@ def stage_bias(bias: torch.Tensor, B2: int, Sq: int, Sk: int, *, q_scale=None, k
         raise RuntimeError("af3_kernels_b200 runs on CUDA tensors only (no CPU fallback)")
     if bias.numel() != B2 * Sq * Sk:
         raise ValueError(f"bias must have B2*Sq*Sk = {B2 * Sq * Sk} elements, got {bias.numel()}")
-    if bias.dtype not in (torch.bfloat16, torch.float32):
-        bias = bias.to(torch.float32)
-    bias = bias.reshape(B2, Sq, Sk) if bias.shape != (B2, Sq, Sk) else bias
-    if (Sk > 1 and bias.stride(2) != 1) or (B2 > 1 and bias.stride(0) == 0) or (Sq > 1 and bias.stride(1) == 0):
-        bias = bias.contiguous()
     fp8 = q_scale is not None
-    desc = _capi.AttentionDesc()
-    desc.B1, desc.B2, desc.Sq, desc.Sk, desc.D = 1, B2, Sq, Sk, 16 * ((head_dim + 15) // 16)
-    for name in ("q_stride", "k_stride", "v_stride", "out_stride"):
-        getattr(desc, name)[:] = [B2 * max(Sq, Sk) * 64, max(Sq, Sk) * 64, 64]
-    desc.bias_stride[:] = [bias.stride(0), bias.stride(1)]
-    desc.qk_dtype = _capi.AF3K_FP8_E4M3 if fp8 else _capi.AF3K_BF16
-    desc.bias_dtype = _capi.AF3K_BF16 if bias.dtype == torch.bfloat16 else _capi.AF3K_F32
-    desc.softmax_scale = float(softmax_scale) if softmax_scale is not None else 1.0 / math.sqrt(head_dim)
-    pitch = (Sk + 7) // 8 * 8
-    staged = torch.empty((B2, Sq, pitch), dtype=torch.bfloat16, device=bias.device)
     if fp8:
         q_scale = q_scale.to(device=bias.device, dtype=torch.float32).contiguous()
         k_scale = k_scale.to(device=bias.device, dtype=torch.float32).contiguous()
-    with torch.cuda.device(bias.device):
-        _capi.check(_capi.load().af3k_stage_bias(
-            ctypes.byref(desc), bias.data_ptr(), q_scale.data_ptr() if fp8 else None,
-            k_scale.data_ptr() if fp8 else None, staged.data_ptr(), staged.numel() * 2,
-            torch.cuda.current_stream().cuda_stream))
+        if q_scale.numel() != B2 or k_scale.numel() != B2:
+            raise ValueError("q_scale / k_scale must have one entry per head")
+    staged = _capi.host().stage_bias(bias, B2, Sq, Sk, head_dim, q_scale, k_scale if fp8 else None,
+                                     float(softmax_scale) if softmax_scale is not None else 1.0 / math.sqrt(head_dim))
     return StagedBias(staged, B2, Sq, Sk, fp8)
 
 
