@@ -51,7 +51,7 @@ class GridSelfAttentionCpp(nn.Module):
     def _norm_and_bias_as_built(self, pair: torch.Tensor) -> bool:
         """Whether LayerNorm and bias projection may be computed from their parameters.  At c_pair = 128 they always are;
         other widths call the two modules, so one that was replaced or carries hooks has to run."""
-        if pair_bias.supported(pair, self.num_head):
+        if pair.shape[-1] == pair_bias.CHANNELS:
             return True
         norm, proj = self.act_norm, self.pair_bias_projection
         return (type(norm) is nn.LayerNorm and norm.weight is not None and norm.bias is not None

@@ -729,7 +729,7 @@ int af3k_grid_front_weights(const void* pair, int32_t pair_dtype, const af3k_fro
   const af3k_front_weights& w = *weights;
   const bool ln = w.gamma != nullptr;
   if (pair_dtype != AF3K_BF16 && !(pair_dtype == AF3K_F32 && ln)) return AF3K_ERR_BAD_DTYPE;
-  for (int32_t t : {w.ln_dtype, w.bias_w_dtype})
+  for (int32_t t : {w.w_dtype, w.ln_dtype, w.bias_w_dtype})
     if (t != AF3K_BF16 && t != AF3K_F32) return AF3K_ERR_BAD_DTYPE;
   if (C != 64 && C != 128) return AF3K_ERR_BAD_SHAPE;
   if (R < 0 || N < 0 || H < 1 || C % H != 0 || (C / H) % 8 != 0 || Hb < 0 || Hb > 4 || (Hb > 0 && !ln)) return AF3K_ERR_BAD_SHAPE;
@@ -745,12 +745,14 @@ int af3k_grid_front_weights(const void* pair, int32_t pair_dtype, const af3k_fro
   DeviceInfo* dev = nullptr;
   int rc = device_info(&dev);
   if (rc != AF3K_OK) return rc;
-  FrontMaps tm;
-  for (int i = 0; i < 4; ++i)
+  FrontMaps tm{};
+  for (int i = 0; i < 4 && w.w_dtype == AF3K_BF16; ++i)
     if ((rc = encode_weight_map(&tm.w[i], w.w[i], C, C)) != AF3K_OK) return rc;
   GridParams p;
   std::memset(&p, 0, sizeof(p));
   p.M = R * N; p.R = (int)R; p.N = (int)N; p.H = (int)H; p.D = (int)(C / H); p.transpose = transpose ? 1 : 0;
+  for (int i = 0; i < 4; ++i) p.w[i] = w.w[i];
+  p.w_f32 = w.w_dtype == AF3K_F32 ? 1 : 0;
   p.q_scale = q_scale; p.pair = pair; p.gamma = w.gamma; p.beta = w.beta; p.ln_f32 = w.ln_dtype == AF3K_F32 ? 1 : 0;
   p.bias_w = w.bias_w; p.bias_w_f32 = w.bias_w_dtype == AF3K_F32 ? 1 : 0; p.eps = eps; p.Hb = (int)Hb;
   p.bias = static_cast<__nv_bfloat16*>(bias); p.bias_pitch = bias_pitch;
@@ -780,15 +782,17 @@ int af3k_grid_front(const void* pair, int32_t pair_dtype, const float* gamma, co
   af3k_front_weights w{};
   for (int i = 0; i < 4; ++i) w.w[i] = w4 ? static_cast<const char*>(w4) + (size_t)i * C * C * 2 : nullptr;
   w.gamma = gamma; w.beta = beta; w.bias_w = bias_w;
+  w.w_dtype = AF3K_BF16;
   w.ln_dtype = w.bias_w_dtype = AF3K_F32;
   return af3k_grid_front_weights(pair, pair_dtype, &w, eps, Hb, R, N, C, H, q_scale, transpose, bias, bias_pitch, q, k, v, gate,
                                  status_dev, stream_v);
 }
 
-int af3k_grid_out(const void* weighted, const void* gate, const void* wo, void* out, int32_t out_dtype, int64_t M, int64_t C,
-                  int* status_dev, void* stream_v) {
+int af3k_grid_out_weights(const void* weighted, const void* gate, const void* wo, int32_t wo_dtype, void* out, int32_t out_dtype, int64_t M,
+                          int64_t C, int* status_dev, void* stream_v) {
   t_last_launches = 0;
-  if (out_dtype != AF3K_BF16 && out_dtype != AF3K_F32) return AF3K_ERR_BAD_DTYPE;
+  for (int32_t t : {wo_dtype, out_dtype})
+    if (t != AF3K_BF16 && t != AF3K_F32) return AF3K_ERR_BAD_DTYPE;
   if ((C != 64 && C != 128) || M < 0 || M > 0x7fffffff) return AF3K_ERR_BAD_SHAPE;
   if (M == 0) return AF3K_OK;
   if (!weighted || !gate || !wo || !out) return AF3K_ERR_NULL_POINTER;
@@ -796,10 +800,11 @@ int af3k_grid_out(const void* weighted, const void* gate, const void* wo, void* 
   DeviceInfo* dev = nullptr;
   int rc = device_info(&dev);
   if (rc != AF3K_OK) return rc;
-  CUtensorMap tm;
-  if ((rc = encode_weight_map(&tm, wo, C, C)) != AF3K_OK) return rc;
+  CUtensorMap tm{};
+  if (wo_dtype == AF3K_BF16 && (rc = encode_weight_map(&tm, wo, C, C)) != AF3K_OK) return rc;
   GridParams p;
   std::memset(&p, 0, sizeof(p));
+  p.w[0] = wo; p.w_f32 = wo_dtype == AF3K_F32 ? 1 : 0;
   p.M = M; p.weighted = static_cast<const __nv_bfloat16*>(weighted); p.gate = static_cast<const __nv_bfloat16*>(gate);
   p.out = out; p.status = status_dev; p.wait_limit = wait_limit_cycles();
   const long long n_tiles = (M + 127) / 128;
@@ -817,6 +822,11 @@ int af3k_grid_out(const void* weighted, const void* gate, const void* wo, void* 
   if (e != cudaSuccess) return cuda_fail("launch grid_out_kernel", e);
   t_last_launches = 1;
   return AF3K_OK;
+}
+
+int af3k_grid_out(const void* weighted, const void* gate, const void* wo, void* out, int32_t out_dtype, int64_t M, int64_t C,
+                  int* status_dev, void* stream_v) {
+  return af3k_grid_out_weights(weighted, gate, wo, AF3K_BF16, out, out_dtype, M, C, status_dev, stream_v);
 }
 
 int af3k_grid_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void* gamma, const void* beta, int32_t ln_dtype,

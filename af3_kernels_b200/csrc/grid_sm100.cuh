@@ -82,6 +82,8 @@ struct GridParams {
   int transpose;           // 1: q, k, v are those of the pair with its two positions exchanged: [N, H, R, D]
   int split;               // front: CTAs that share a tile's four outputs (small problems): 1, 2 or 4
   float q_scale;
+  const void* w[4];        // fp32 weight matrices [C, C] (front: q, k, v, gate; out: output projection), if w_f32
+  int w_f32;               // 0: bf16, read through the tensor maps
   const void* pair;        // front: input rows
   const void* gamma;       // front with LayerNorm: [C], bf16 or fp32
   const void* beta;
@@ -161,16 +163,44 @@ __device__ __forceinline__ void params_at(const void* src, long long i, int f32,
   }
 }
 
-// Barrier set-up, TMEM allocation and weight loads shared by both kernels (all threads; ends with a block
-// barrier).  The weights are `chunks` matrices of C rows, one tensor map each; `gap` rows are left free behind the
-// first one.
+// One fp32 weight matrix [C, C] as rows row0 .. of the B operand, rounded to bf16 on the way (the 512 threads behind the
+// first four warps).  A packing pass in front of the block took 5 us: 389 fp32 rows 264 us a call, with this 261.
 template <class Tile, int C>
-__device__ __forceinline__ uint32_t grid_prologue(uint32_t smem, uint32_t bars, volatile uint32_t* slot, volatile int* abort_flag,
-                                                  uint32_t tmem_cols, const CUtensorMap* tm_w, int chunks, int gap) {
+__device__ __forceinline__ void grid_convert_weights(uint32_t smem, const void* src, int row0) {
+  constexpr int kItems = C * C / 8 / (kGridThreads - 128);      // 8 channels of a row each, all in flight at once
+  static_assert(kItems * 8 * (kGridThreads - 128) == C * C, "whole items per thread");
+  uint4 v[kItems][2];
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const uint4* s = static_cast<const uint4*>(src) + 2 * (i * (kGridThreads - 128) + threadIdx.x - 128);
+    v[i][0] = s[0];
+    v[i][1] = s[1];
+  }
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const int k = i * (kGridThreads - 128) + threadIdx.x - 128, r = row0 + k / (C / 8), c8 = k % (C / 8);
+    sts128(smem + (c8 >> 3) * (Tile::kRows * 128) + r * 128 + (((c8 & 7) ^ (r & 7)) << 4),
+           pack_bf16x2(__uint_as_float(v[i][0].x), __uint_as_float(v[i][0].y)), pack_bf16x2(__uint_as_float(v[i][0].z), __uint_as_float(v[i][0].w)),
+           pack_bf16x2(__uint_as_float(v[i][1].x), __uint_as_float(v[i][1].y)), pack_bf16x2(__uint_as_float(v[i][1].z), __uint_as_float(v[i][1].w)));
+  }
+}
+
+// Barrier set-up, TMEM allocation and weight loads shared by both kernels (all threads; ends with a block
+// barrier).  The weights are `chunks` matrices of C rows from p.w[chunk0] on, one tensor map each; `gap` rows are left
+// free behind the first one.
+template <class Tile, int C>
+__device__ __forceinline__ uint32_t grid_prologue(const GridParams& p, uint32_t smem, uint32_t bars, volatile uint32_t* slot,
+                                                  volatile int* abort_flag, uint32_t tmem_cols, const CUtensorMap* tm_w, int chunk0, int chunks,
+                                                  int gap) {
   const int warp = threadIdx.x >> 5;
+  if (p.w_f32 && threadIdx.x >= 128) {
+    grid_wait_previous();
+    for (int c = 0; c < chunks; ++c) grid_convert_weights<Tile, C>(smem, p.w[chunk0 + c], c * C + (c > 0 ? gap : 0));
+  }
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    for (int c = 0; c < chunks; ++c) prefetch_tensormap(tm_w + c);
+    if (!p.w_f32)
+      for (int c = 0; c < chunks; ++c) prefetch_tensormap(tm_w + chunk0 + c);
     mbar_init(bars + 8u * GridBar::w_full, 1);
     for (int i = 0; i < Tile::kStages; ++i) {
       mbar_init(bars + 8u * (GridBar::x_ready + i), kGridProducerWarps);
@@ -182,12 +212,16 @@ __device__ __forceinline__ uint32_t grid_prologue(uint32_t smem, uint32_t bars, 
     }
     fence_barrier_init();
     grid_wait_previous();
-    mbar_arrive_expect_tx(bars + 8u * GridBar::w_full, (uint32_t)chunks * C * C * 2);
-    for (int c = 0; c < chunks; ++c)
-      for (int kb = 0; kb < C / 64; ++kb)
-        for (int r = 0; r < C; r += 64)
-          tma_load_2d(smem + kb * (Tile::kRows * 128) + (c * C + (c > 0 ? gap : 0) + r) * 128, tm_w + c, bars + 8u * GridBar::w_full,
-                      kb * 64, r);
+    if (p.w_f32) {
+      mbar_arrive(bars + 8u * GridBar::w_full);
+    } else {
+      mbar_arrive_expect_tx(bars + 8u * GridBar::w_full, (uint32_t)chunks * C * C * 2);
+      for (int c = 0; c < chunks; ++c)
+        for (int kb = 0; kb < C / 64; ++kb)
+          for (int r = 0; r < C; r += 64)
+            tma_load_2d(smem + kb * (Tile::kRows * 128) + (c * C + (c > 0 ? gap : 0) + r) * 128, tm_w + chunk0 + c, bars + 8u * GridBar::w_full,
+                        kb * 64, r);
+    }
   }
   if (warp == 0) {
     __syncwarp();
@@ -257,7 +291,7 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
       sts128(smem + (c8 >> 3) * (Tile::kRows * 128) + (C + r) * 128 + (((c8 & 7) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
     }
   }
-  const uint32_t tmem = grid_prologue<Tile, C>(smem, bars, slot, abort_flag, kTmem, maps.w + chunk0, chunks, kBiasRows);
+  const uint32_t tmem = grid_prologue<Tile, C>(p, smem, bars, slot, abort_flag, kTmem, maps.w, chunk0, chunks, kBiasRows);
 
   if (warp < 4) {
     setmaxnreg_dec<kGridRegsMisc>();
@@ -499,7 +533,7 @@ grid_out_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CU
   volatile int* abort_flag = reinterpret_cast<volatile int*>(grid_smem + Tile::off_slot + 4);
   constexpr uint32_t kTmem = 2 * C;               // two accumulators, taken in turn
   const long long n_tiles = (p.M + 127) / 128;
-  const uint32_t tmem = grid_prologue<Tile, C>(smem, bars, slot, abort_flag, kTmem, &tm_w, 1, 0);
+  const uint32_t tmem = grid_prologue<Tile, C>(p, smem, bars, slot, abort_flag, kTmem, &tm_w, 0, 1, 0);
 
   if (warp < 4) {
     setmaxnreg_dec<kGridRegsMisc>();
@@ -633,7 +667,8 @@ done:
 }
 
 // ------------------------------------------------------------------ packed weights
-// Parameters the kernels cannot read where they are (fp32, [in, out], any other strides), laid out for one call:
+// Parameters the kernels cannot read where they are ([in, out] in the grid block, fp32 in the single block, any other
+// strides), laid out for one call:
 // W4 [4 C, C] = q, k, v, gate rows, Wo [C, C] (rows = output channels, bf16), gamma, beta, bias projection (fp32).
 // Latency-bound (C = 384: 1.2 MB in and out), so one tile of 64 x 64 per block, read along the source's unit stride
 // and turned in shared memory: `[in, out]` weights read along `in` would touch a sector per element.

@@ -33,7 +33,7 @@ struct Library {
   decltype(&af3k_dot_product_attention_workspace) workspace = nullptr;
   decltype(&af3k_stage_bias) stage_bias = nullptr;
   decltype(&af3k_grid_front_weights) grid_front = nullptr;
-  decltype(&af3k_grid_out) grid_out = nullptr;
+  decltype(&af3k_grid_out_weights) grid_out = nullptr;
   decltype(&af3k_sigmoid_gate) sigmoid_gate = nullptr;
   decltype(&af3k_grid_pack) grid_pack = nullptr;
   decltype(&af3k_token_projection_weights) token_projection = nullptr;
@@ -53,7 +53,7 @@ void bind_library(const std::string& path) {
   AF3K_BIND(workspace, af3k_dot_product_attention_workspace);
   AF3K_BIND(stage_bias, af3k_stage_bias);
   AF3K_BIND(grid_front, af3k_grid_front_weights);
-  AF3K_BIND(grid_out, af3k_grid_out);
+  AF3K_BIND(grid_out, af3k_grid_out_weights);
   AF3K_BIND(sigmoid_gate, af3k_sigmoid_gate);
   AF3K_BIND(grid_pack, af3k_grid_pack);
   AF3K_BIND(token_projection, af3k_token_projection_weights);
@@ -300,9 +300,8 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
 // pointer), and a captured graph would replay it after it was given up or had become old.
 int32_t dtype_code(const Tensor& t) { return t.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16; }
 
-Tensor kernel_dtype(const Tensor& t) {      // bf16 or fp32, without a gradient
-  const Tensor x = t.detach();
-  return x.scalar_type() == at::kFloat || x.scalar_type() == at::kBFloat16 ? x : x.to(at::kFloat);
+Tensor kernel_dtype(const Tensor& t) {      // bf16 or fp32
+  return t.scalar_type() == at::kFloat || t.scalar_type() == at::kBFloat16 ? t : t.detach().to(at::kFloat);
 }
 
 // The first n parameters are [C, C]; all are where the activations are (a kernel handed the address of a module that was
@@ -331,7 +330,7 @@ Tensor packed_matrices(const std::vector<Tensor>& w, int64_t C, cudaStream_t str
 }
 
 // The grid block's parameters: matrices q, k, v, gate, output as [out, in], read where they are if the kernels can
-// (nn.Linear.weight in bf16), else packed for this call; then (all or none) LayerNorm weight and bias, bias projection.
+// (nn.Linear.weight, bf16 or fp32), else packed for this call; then (all or none) LayerNorm weight and bias, bias projection.
 struct GridParameters {
   af3k_front_weights front{};
   const void* wo = nullptr;
@@ -341,11 +340,13 @@ GridParameters grid_parameters(const std::vector<Tensor>& params, int64_t C, cud
   GridParameters r;
   r.front.ln_dtype = r.front.bias_w_dtype = AF3K_F32;
   const void* m[5];
-  bool in_place = true;
+  const at::ScalarType type = params[0].scalar_type();
+  bool in_place = type == at::kBFloat16 || type == at::kFloat;
   for (int i = 0; i < 5; ++i) {
     m[i] = params[i].data_ptr();
-    in_place = in_place && params[i].scalar_type() == at::kBFloat16 && params[i].is_contiguous() && reinterpret_cast<uintptr_t>(m[i]) % 16 == 0;
+    in_place = in_place && params[i].scalar_type() == type && params[i].is_contiguous() && reinterpret_cast<uintptr_t>(m[i]) % 16 == 0;
   }
+  r.front.w_dtype = in_place ? dtype_code(params[0]) : AF3K_BF16;
   if (!in_place) {
     r.keep.push_back(packed_matrices({params.begin(), params.begin() + 5}, C, stream));
     for (int i = 0; i < 5; ++i) m[i] = static_cast<char*>(r.keep[0].data_ptr()) + i * C * C * 2;
@@ -353,8 +354,9 @@ GridParameters grid_parameters(const std::vector<Tensor>& params, int64_t C, cud
   for (int i = 0; i < 4; ++i) r.front.w[i] = m[i];
   r.wo = m[4];
   if (params.size() > 5) {
-    Tensor gamma = kernel_dtype(params[5]), beta = kernel_dtype(params[6]), bw = kernel_dtype(params[7]).contiguous();
-    if (gamma.scalar_type() != beta.scalar_type()) { gamma = gamma.to(at::kFloat); beta = beta.to(at::kFloat); }
+    Tensor gamma = kernel_dtype(params[5]), beta = kernel_dtype(params[6]);
+    const Tensor bw = kernel_dtype(params[7]).contiguous();
+    if (gamma.scalar_type() != beta.scalar_type()) { gamma = gamma.detach().to(at::kFloat); beta = beta.detach().to(at::kFloat); }
     gamma = gamma.contiguous(); beta = beta.contiguous();
     r.front.gamma = gamma.data_ptr(); r.front.beta = beta.data_ptr(); r.front.bias_w = bw.data_ptr();
     r.front.ln_dtype = dtype_code(gamma); r.front.bias_w_dtype = dtype_code(bw);
@@ -419,7 +421,7 @@ Tensor grid_module(Tensor pair, const Tensor& mask_in, const std::vector<Tensor>
   check(g_lib.attention(&d, q, k, v, bias.data_ptr(), static_cast<const uint8_t*>(mask.data_ptr()), weighted, nullptr, nullptr, nullptr, 0,
                         status, stream));
   if (!project) check(g_lib.sigmoid_gate(weighted, gate, out.data_ptr(), M * C, stream));
-  else check(g_lib.grid_out(weighted, gate, w.wo, out.data_ptr(), f32 ? AF3K_F32 : AF3K_BF16, M, C, status, stream));
+  else check(g_lib.grid_out(weighted, gate, w.wo, w.front.w_dtype, out.data_ptr(), f32 ? AF3K_F32 : AF3K_BF16, M, C, status, stream));
   return out;
 }
 
@@ -444,7 +446,7 @@ Tensor grid_block(const Tensor& pair, const OptTensor& mask, const Tensor& bias,
                          k.data_ptr(), v.data_ptr(), gate.data_ptr(), status, stream));
   attention(q, k, v, mask, bias, std::nullopt, std::nullopt, 1.0, 0, weighted.permute({0, 2, 1, 3}), true, true, 0, 0);
   if (!project) check(g_lib.sigmoid_gate(weighted.data_ptr(), gate.data_ptr(), out.data_ptr(), M * C, stream));
-  else check(g_lib.grid_out(weighted.data_ptr(), gate.data_ptr(), w.wo, out.data_ptr(), pair.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16,
+  else check(g_lib.grid_out(weighted.data_ptr(), gate.data_ptr(), w.wo, w.front.w_dtype, out.data_ptr(), pair.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16,
                        M, C, status, stream));
   return out;
 }

@@ -252,13 +252,13 @@ int af3k_grid_front(const void* pair, int32_t pair_dtype, const float* gamma, co
 
 /* The same front with the parameters where their owner keeps them (a module's nn.Linear / nn.LayerNorm tensors):
  * nothing is laid out first, and the call sees the values they hold when it runs.  gamma NULL: no LayerNorm (beta
- * ignored, Hb 0).  The four matrices are [C, C] bf16, output rows, contiguous, 16-byte aligned; the vectors and
- * bias_w [Hb, C] are contiguous, bf16 or fp32. */
+ * ignored, Hb 0).  The four matrices are [C, C], output rows, contiguous, 16-byte aligned, all of w_dtype (fp32 is rounded
+ * to bf16 on the way in); the vectors and bias_w [Hb, C] are contiguous, bf16 or fp32. */
 typedef struct af3k_front_weights {
   const void* w[4];                 /* q, k, v, gate */
   const void *gamma, *beta;         /* [C], both of ln_dtype */
   const void* bias_w;
-  int32_t ln_dtype, bias_w_dtype;
+  int32_t w_dtype, ln_dtype, bias_w_dtype;
 } af3k_front_weights;
 int af3k_grid_front_weights(const void* pair, int32_t pair_dtype, const af3k_front_weights* weights, float eps,
                             int64_t Hb, int64_t R, int64_t N, int64_t C, int64_t H, float q_scale, int32_t transpose,
@@ -273,6 +273,10 @@ int af3k_grid_front_weights(const void* pair, int32_t pair_dtype, const af3k_fro
  * All pointers 16-byte aligned. */
 int af3k_grid_out(const void* weighted, const void* gate, const void* wo, void* out, int32_t out_dtype, int64_t M,
                   int64_t C, int* status_dev, void* stream);
+
+/* af3k_grid_out with wo in wo_dtype: bf16, or fp32 that is rounded to bf16 on the way in. */
+int af3k_grid_out_weights(const void* weighted, const void* gate, const void* wo, int32_t wo_dtype, void* out,
+                          int32_t out_dtype, int64_t M, int64_t C, int* status_dev, void* stream);
 
 /* The four projections of the single / diffusion attention block:  out = [q | k | v | gate], each [M, C],
  *     q = (x Wq^T + q_bias) * q_scale,  k = x Wk^T,  v = x Wv^T,  gate = x Wg^T

@@ -571,3 +571,26 @@ def test_bias_of_a_narrow_fp32_pair_is_that_of_the_fp32_normalised_pair(cuda_dev
     size = torch.einsum("rnc,hc->hrn", x.abs(), bw.double().abs())
     err = (bias[:, :, :N].double() - want).abs()
     assert (err <= want.abs() * 2.0 ** -8 + size * 2.0 ** -14).all(), (err / size).max()
+
+
+@pytest.mark.parametrize("C", [64, 128])
+@pytest.mark.parametrize("R,N", [(2, 30), (70, 90), (200, 200)])
+def test_grid_block_reads_weights_of_any_layout(cuda_device, R, N, C):
+    """`[out, in]` weights are read where they are (bf16 by TMA, fp32 converted on the way in), others are packed first:
+    the same bits for the same values, with a tile's outputs on four, two and one CTAs."""
+    g = torch.Generator().manual_seed(C + N)
+    H, dev = 4, cuda_device
+    pair = torch.randn(R, N, C, generator=g).to(dev, torch.bfloat16)
+    mask = (torch.rand(R, N, generator=g) >= 0.1).to(dev)
+    bias = torch.randn(H, N, N, generator=g).to(dev, torch.bfloat16)
+    ws = [(torch.randn(C, C, generator=g) * C ** -0.5).to(dev, torch.bfloat16) for _ in range(5)]      # [in, out]
+    out_in = lambda w: w.T.contiguous().T
+    forms = {"out_in": out_in, "in_out": lambda w: w, "f32": lambda w: out_in(w.float()), "f32_in_out": lambda w: w.float(),
+             "odd_offset": lambda w: torch.nn.functional.pad(w.T.reshape(-1), (1, 0))[1:].view(C, C).T}
+    with torch.no_grad():
+        res = {n: A._attention_cpp(pair, mask, bias, *map(f, ws), H) for n, f in forms.items()}
+        mixed = A._attention_cpp(pair, mask, bias, *[f(w) for f, w in zip(forms.values(), ws)], H)
+    for n, r in res.items():
+        assert torch.equal(r, res["out_in"]), n
+    assert torch.equal(mixed, res["out_in"])
+    assert read_status(dev)[0] == 0
