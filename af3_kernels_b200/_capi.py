@@ -42,6 +42,7 @@ EXPORTED_SYMBOLS = (
     "af3k_grid_out",
     "af3k_grid_out_weights",
     "af3k_grid_pack",
+    "af3k_token_pack",
     "af3k_token_projection",
     "af3k_token_projection_weights",
 )

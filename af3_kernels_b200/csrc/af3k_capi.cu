@@ -829,8 +829,9 @@ int af3k_grid_out(const void* weighted, const void* gate, const void* wo, void* 
   return af3k_grid_out_weights(weighted, gate, wo, AF3K_BF16, out, out_dtype, M, C, status_dev, stream_v);
 }
 
-int af3k_grid_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void* gamma, const void* beta, int32_t ln_dtype,
-                   int64_t C, int64_t Hb, void* w4, void* wo, float* vec, void* stream_v) {
+namespace {
+int launch_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void* gamma, const void* beta, int32_t ln_dtype, int64_t C,
+                int64_t Hb, void* w4, void* wo, float* vec, const float* x, void* x_bf16, int64_t x_n, void* stream_v) {
   t_last_launches = 0;
   if (C < 1 || C > 1024 || Hb < 0 || Hb > 1024 || (Hb > 0 && bias_w == nullptr)) return AF3K_ERR_BAD_SHAPE;
   if (!w5 || !w4 || (w5[4].data && !wo) || ((gamma || beta || Hb > 0) && !vec)) return AF3K_ERR_NULL_POINTER;
@@ -851,12 +852,34 @@ int af3k_grid_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void*
   p.C = (int)C; p.Hb = (int)Hb;
   p.w4 = static_cast<__nv_bfloat16*>(w4); p.wo = static_cast<__nv_bfloat16*>(wo); p.vec = vec;
   const unsigned tiles = (unsigned)((C + kPackTile - 1) / kPackTile);
-  const unsigned slices = vec != nullptr ? 6 : (w5[4].data ? 5 : 4);
+  unsigned slices = vec != nullptr ? 6 : (w5[4].data ? 5 : 4);
+  if (x_n > 0) {
+    p.x = reinterpret_cast<const float4*>(x); p.x_bf16 = static_cast<uint2*>(x_bf16); p.x_n4 = x_n / 4;
+    const long long per_slice = (long long)tiles * tiles * kPackThreads * kPackXEach, more = (p.x_n4 + per_slice - 1) / per_slice;
+    if (more > 65535 - kPackSlices) return AF3K_ERR_BAD_SHAPE;
+    slices = kPackSlices + (unsigned)more;
+  }
   launch_overlapped(grid_pack_kernel, dim3(tiles, tiles, slices), kPackThreads, 0, reinterpret_cast<cudaStream_t>(stream_v), true, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail("launch grid_pack_kernel", e);
   t_last_launches = 1;
   return AF3K_OK;
+}
+}  // namespace
+
+int af3k_grid_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void* gamma, const void* beta, int32_t ln_dtype,
+                   int64_t C, int64_t Hb, void* w4, void* wo, float* vec, void* stream_v) {
+  return launch_pack(w5, bias_w, gamma, beta, ln_dtype, C, Hb, w4, wo, vec, nullptr, nullptr, 0, stream_v);
+}
+
+int af3k_token_pack(const af3k_matrix* w4, int64_t C, void* w4_bf16, const float* x, int64_t M, void* x_bf16, void* stream_v) {
+  t_last_launches = 0;
+  if (!w4) return AF3K_ERR_NULL_POINTER;
+  if (C < 4 || C % 4 != 0 || M < 0 || M > 0x7fffff00LL) return AF3K_ERR_BAD_SHAPE;
+  if (M > 0 && (!x || !x_bf16)) return AF3K_ERR_NULL_POINTER;
+  if (!aligned16(x) || !aligned16(x_bf16)) return AF3K_ERR_BAD_ALIGNMENT;
+  af3k_matrix w5[5] = {w4[0], w4[1], w4[2], w4[3], {}};
+  return launch_pack(w5, nullptr, nullptr, nullptr, AF3K_F32, C, 0, w4_bf16, nullptr, nullptr, x, x_bf16, M * C, stream_v);
 }
 
 int af3k_token_projection_weights(const void* x, const af3k_matrix* w4, const void* q_bias, int32_t q_bias_dtype, int64_t M, int64_t C,

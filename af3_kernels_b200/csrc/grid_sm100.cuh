@@ -679,15 +679,28 @@ struct PackParams {
   const void* gamma; const void* beta; int ln_f32;
   int C, Hb;
   __nv_bfloat16* w4; __nv_bfloat16* wo; float* vec;    // vec: gamma [C], beta [C], bias_w [Hb, C]; null: none
+  const float4* x; uint2* x_bf16; long long x_n4;      // activations to round in the same launch, in pieces of four; null: none
 };
-constexpr int kPackTile = 64, kPackThreads = 256;
-// blockIdx = (tile along in, tile along out, matrix); blockIdx.z == 5: the vectors
+constexpr int kPackTile = 64, kPackThreads = 256, kPackSlices = 6, kPackXEach = 4;
+// blockIdx = (tile along in, tile along out, matrix); blockIdx.z == 5: the vectors, from kPackSlices on: the activations
 __global__ void __launch_bounds__(kPackThreads) grid_pack_kernel(const __grid_constant__ PackParams p) {
   __shared__ __nv_bfloat16 tile[kPackTile][kPackTile + 2];
   const int C = p.C, m = blockIdx.z;
   grid_wait_previous();
   grid_release_next();
+  if (m >= kPackSlices) {
+    const long long first = (((long long)(m - kPackSlices) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * (kPackThreads * kPackXEach) + threadIdx.x;
+    float4 v[kPackXEach];
+#pragma unroll
+    for (int i = 0; i < kPackXEach; ++i)
+      if (first + i * kPackThreads < p.x_n4) v[i] = p.x[first + i * kPackThreads];
+#pragma unroll
+    for (int i = 0; i < kPackXEach; ++i)
+      if (first + i * kPackThreads < p.x_n4) p.x_bf16[first + i * kPackThreads] = make_uint2(pack_bf16x2(v[i].x, v[i].y), pack_bf16x2(v[i].z, v[i].w));
+    return;
+  }
   if (m == 5) {
+    if (p.vec == nullptr) return;
     if (blockIdx.x != 0 || blockIdx.y != 0) return;
     for (int e = threadIdx.x; e < (2 + p.Hb) * C; e += kPackThreads) {
       const int v = e / C, c = e % C;

@@ -36,6 +36,7 @@ struct Library {
   decltype(&af3k_grid_out_weights) grid_out = nullptr;
   decltype(&af3k_sigmoid_gate) sigmoid_gate = nullptr;
   decltype(&af3k_grid_pack) grid_pack = nullptr;
+  decltype(&af3k_token_pack) token_pack = nullptr;
   decltype(&af3k_token_projection_weights) token_projection = nullptr;
 };
 Library g_lib;
@@ -56,6 +57,7 @@ void bind_library(const std::string& path) {
   AF3K_BIND(grid_out, af3k_grid_out_weights);
   AF3K_BIND(sigmoid_gate, af3k_sigmoid_gate);
   AF3K_BIND(grid_pack, af3k_grid_pack);
+  AF3K_BIND(token_pack, af3k_token_pack);
   AF3K_BIND(token_projection, af3k_token_projection_weights);
 #undef AF3K_BIND
 }
@@ -315,8 +317,9 @@ void check_parameters(const std::vector<Tensor>& params, size_t n, int64_t C, co
 }
 
 // q, k, v, gate and perhaps output projection [C, C] as (out, in) matrices, in the kernels' layout: one launch
-// -> [4 C or 5 C, C] bf16
-Tensor packed_matrices(const std::vector<Tensor>& w, int64_t C, cudaStream_t stream) {
+// -> [4 C or 5 C, C] bf16.  tokens: fp32 activations of the single block that the same launch rounds to bf16, in place of
+// which their bf16 form is left.
+Tensor packed_matrices(const std::vector<Tensor>& w, int64_t C, cudaStream_t stream, Tensor* tokens = nullptr) {
   std::vector<Tensor> src;
   af3k_matrix w5[5] = {};
   for (size_t i = 0; i < w.size(); ++i) {
@@ -325,6 +328,12 @@ Tensor packed_matrices(const std::vector<Tensor>& w, int64_t C, cudaStream_t str
   }
   Tensor packed = at::empty({(int64_t)w.size() * C, C}, src[0].options().dtype(at::kBFloat16));
   char* p = static_cast<char*>(packed.data_ptr());
+  if (tokens != nullptr) {
+    const Tensor x = *tokens;
+    *tokens = at::empty(x.sizes(), x.options().dtype(at::kBFloat16));
+    check(g_lib.token_pack(w5, C, p, x.data_ptr<float>(), x.size(0), tokens->data_ptr(), stream));
+    return packed;
+  }
   check(g_lib.grid_pack(w5, nullptr, nullptr, nullptr, AF3K_F32, C, 0, p, w.size() > 4 ? p + 4 * C * C * 2 : nullptr, nullptr, stream));
   return packed;
 }
@@ -463,8 +472,6 @@ Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, con
   if (q_bias.numel() != C) value_error("q_bias must have one entry per channel");
   if (bias.numel() != head * N * N) value_error("bias must have B2*Sq*Sk = " + std::to_string(head * N * N) + " elements, got " + std::to_string(bias.numel()));
   if (bias.device() != dev) value_error("q, k, v, bias must live on the same device");
-  Tensor x = x_in.to(at::kBFloat16).contiguous();
-  if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0) x = x.clone();
   if (N == 0) return at::empty({N, C}, x_in.options());
   q_bias = kernel_dtype(q_bias).contiguous();
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
@@ -477,9 +484,15 @@ Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, con
     in_place_w = in_place_w && weights[i].scalar_type() == at::kBFloat16 && reinterpret_cast<uintptr_t>(w4[i].data) % 16 == 0 &&
                  (so == 1 || si == 1) && std::max(so, si) >= C && std::max(so, si) % 8 == 0;
   }
-  Tensor packed;
+  // fp32 tokens are rounded in the same launch as weights that are packed
+  const bool with_tokens = !in_place_w && x_in.scalar_type() == at::kFloat && x_in.is_contiguous() && reinterpret_cast<uintptr_t>(x_in.data_ptr()) % 16 == 0;
+  Tensor packed, x = x_in;
+  if (!with_tokens) {
+    x = x_in.to(at::kBFloat16).contiguous();
+    if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0) x = x.clone();
+  }
   if (!in_place_w) {
-    packed = packed_matrices(weights, C, stream);
+    packed = packed_matrices(weights, C, stream, with_tokens ? &x : nullptr);
     for (int i = 0; i < 4; ++i) w4[i] = af3k_matrix{static_cast<char*>(packed.data_ptr()) + i * C * C * 2, C, 1, AF3K_BF16};
   }
   const float scale = 1.0f / std::sqrt((float)D);

@@ -308,6 +308,11 @@ int af3k_token_projection_weights(const void* x, const af3k_matrix* w4, const vo
 int af3k_grid_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void* gamma, const void* beta,
                    int32_t ln_dtype, int64_t C, int64_t Hb, void* w4, void* wo, float* vec, void* stream);
 
+/* What af3k_token_projection needs of fp32 tokens and of weights it cannot read where they are, in one launch:
+ * w4 (any strides, bf16 or fp32) -> w4_bf16 [4 C, C], x [M, C] fp32 contiguous -> x_bf16 [M, C].  C a multiple of 4;
+ * x, x_bf16 16-byte aligned; M 0: no tokens. */
+int af3k_token_pack(const af3k_matrix* w4, int64_t C, void* w4_bf16, const float* x, int64_t M, void* x_bf16, void* stream);
+
 /* out = weighted * sigmoid(gate), elementwise over n bf16 elements (n a multiple of 8; all three
  * pointers 16-byte aligned; out may be weighted).  Stands in for the SigmoidFwdTPP + MulTPP pair
  * behind the attention core in the reference's fused blocks
