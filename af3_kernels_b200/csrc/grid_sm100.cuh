@@ -16,7 +16,8 @@
 //                reads are full 16-byte pieces of consecutive lanes, the LayerNorm reductions are four
 //                (C = 64: three) shuffles and its parameters stay in registers.  The next rows are
 //                requested before the current ones are worked on.
-//   warp 0       TMEM allocation, the weights' TMA loads, the MMAs (fp32 accumulators in TMEM)
+//   warp 0       TMEM allocation, the weights' TMA loads (fp32 weights: converted by warps 4-19), the MMAs (fp32
+//                accumulators in TMEM)
 //   warps 4-11   epilogue, one TMEM lane quarter each, the two warpgroups taking the accumulators in turn: TMEM ->
 //                registers -> bf16 or fp32 -> a private XOR-swizzled patch of shared memory -> 16-byte stores
 //                in runs of 128 bytes
@@ -26,7 +27,7 @@
 // (+ 2 Hb), the output pass reads 512 and writes 256.  The normalised pair and the gated product never
 // reach HBM.  The pair bias is part of the GEMM: as arithmetic of the row producers (32 FMAs and five
 // shuffles per row piece) it made their chain the limit, 185 us against 148 (768 x 768 x 128 bf16; 116 us at
-// the copy rate).  The output pass takes 82 us there (69 at the copy rate).
+// the copy rate).  The output pass takes 89 us there (69 at the copy rate).
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -229,7 +230,7 @@ __device__ __forceinline__ uint32_t grid_prologue(const GridParams& p, uint32_t 
     tmem_relinquish();
   }
   // No grid_release_next here: the next kernel's blocks come in as this one's end.  Letting them in earlier was slower
-  // (389 rows 255 -> 257 us a module call, 768 rows 923 -> 926).
+  // (389 rows 255 -> 257 us a module call).
   grid_wait_previous();
   fence_proxy_async_smem();      // whatever the caller stored for the tensor core
   tc_fence_before();

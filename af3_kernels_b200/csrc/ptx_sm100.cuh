@@ -124,8 +124,8 @@ __device__ __forceinline__ bool mbar_wait_bounded_compact(uint32_t bar, uint32_t
 // and loads behind it must not be of the read-only kind (__ldg), which may be moved or served across it.
 // release: the next kernel's blocks may come in as SMs become free (without it: as this kernel's blocks end).
 // Measured, us a call, before -> after: 512 tokens 14.4 -> 11.7, 1536 tokens 30.8 -> 29.7, diffusion 5 x 1536
-// 114.8 -> 112.0, 768 rows 669 -> 666; grid module 64 rows 25.7 -> 22.2, 256 rows of 64 channels 63.0 -> 57.6, 389
-// fp32 rows 260 -> 255, 768 rows 924 -> 923; single block of 1536 tokens 48.0 -> 43.3.
+// 114.8 -> 112.0; grid module 64 rows 25.7 -> 22.2, 256 rows of 64 channels 63.0 -> 57.6, 389 fp32 rows 260 -> 255;
+// single block of 1536 tokens 48.0 -> 43.3.  Calls of 0.6 ms and more: no difference beyond the runs' own.
 __device__ __forceinline__ void grid_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

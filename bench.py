@@ -646,7 +646,7 @@ def main():
 
 def grid_block_line(args, dev):
     """Extra workload (not the headline line): the whole grid self-attention module at N = 768,
-    c_pair = 128, 4 heads - LayerNorm, bias and q/k/v/gate projections (cuBLAS), the attention
+    c_pair = 128, 4 heads - LayerNorm, bias and q/k/v/gate projections, the attention
     kernel, gating and output projection - on a device-resident pair representation."""
     import af3_kernels_b200 as A
     N, C, H = (args.rows or 768), 128, 4
@@ -678,8 +678,8 @@ def grid_block_line(args, dev):
 def self_block_line(args, dev):
     """Extra workload (not the headline line): the single attention block with pair bias
     (self_attention_cpp) at the pairformer size, N = 1536 tokens, c = 384, 16 heads of 24, bias
-    [16, N, N] bf16 - four projections (cuBLAS), the attention kernel, the sigmoid gate.  The block
-    is a handful of short launches, so it is timed both launch by launch and replayed from a CUDA
+    [16, N, N] bf16 - the four projections in one GEMM, the attention kernel with the gate.  The block
+    is two short launches, so it is timed both launch by launch and replayed from a CUDA
     graph."""
     import af3_kernels_b200 as A
     N, C, H = (args.rows or 1536), 384, 16

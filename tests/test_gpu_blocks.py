@@ -1,5 +1,5 @@
-"""GPU parity of the two attention blocks and the grid modules (projections through cuBLAS, core
-through libaf3k.so) against golden outputs of the reference's PyTorch models and the fp32 block
+"""GPU parity of the two attention blocks and the grid modules (fused passes, and projections through
+torch for the sizes those do not take) against golden outputs of the reference's PyTorch models and the fp32 block
 oracles.  The blocks compute in bf16, so errors are judged against the size of the outputs:
 max-abs <= 4 % of the largest reference magnitude, mean-abs <= 2 % of the mean magnitude (four
 bf16 roundings in a row: projections, P, gated product, output projection)."""
@@ -144,7 +144,7 @@ def test_fused_projection_kernel_matches_plain_gemms(cuda_device):
 
 
 def test_self_block_replays_from_a_cuda_graph(cuda_device):
-    """The block is a handful of short launches (four GEMMs, the attention kernel, the gate); its
+    """The block is two short launches (the projections, the attention kernel with the gate); its
     calls into the library allocate nothing the graph allocator cannot serve and never synchronise,
     so the whole block can be captured once and replayed - with results identical to the eager call."""
     dev = cuda_device
@@ -231,7 +231,7 @@ def test_fused_grid_module_against_oracle(cuda_device, N, C, H, dtype, transpose
     m = m.to(cuda_device)
     with torch.no_grad():
         out = m(pair.to(cuda_device), mask.to(cuda_device))
-        # new values in the same parameters are seen (the packed copy follows the version counter)
+        # new values in the same parameters are seen
         m.output_projection.weight.neg_()
         flipped = m(pair.to(cuda_device), mask.to(cuda_device))
     assert out.dtype == dtype and out.shape == (N, N, C)
