@@ -180,6 +180,7 @@ class RowShardedAttention:
         self.last_exchange = exchange
         if exchange == "copy":
             full, hdl, peer_full = symm
+            full = full.detach()        # a result that carries a gradient must not tie its history to the kept buffer
             # nobody may still be writing into (or, two calls back, reading from) this buffer
             hdl.barrier(channel=0)
             n_cs = self.copy_streams if self.copy_streams > 0 else max(1, ws - 1)
@@ -218,7 +219,7 @@ class RowShardedAttention:
                         r = (rank + kk) % ws
                         cs = self._copy_streams[(kk - 1) % len(self._copy_streams)]
                         cs.wait_event(ev)
-                        with torch.cuda.stream(cs):
+                        with torch.cuda.stream(cs), torch.no_grad():
                             peer_full[r][rank, p0:p1].copy_(full[rank, p0:p1], non_blocking=True)
             elif use_streams:
                 ev = torch.cuda.Event()

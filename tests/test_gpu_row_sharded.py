@@ -141,3 +141,32 @@ def test_distributed_grid_module_equals_plain_module(cuda_device, n):
             p.terminate()
     assert all(p.exitcode == 0 for p in procs), [p.exitcode for p in procs]
     assert all(ret.get(r) for r in range(ws)), dict(ret)
+
+
+def test_kept_buffers_carry_no_gradient_history(cuda_device):
+    """With gradients enabled the pieces may carry one (the block's output projection): the result of a call has it, the
+    buffers that are kept for the next call do not, its own and the peers'.  One process in place of rank 0 of two, the
+    peer's buffer an ordinary tensor."""
+    from af3_kernels_b200 import RowShardedAttention
+
+    class NoBarrier:
+        def barrier(self, channel):
+            pass
+
+    class RankZeroOfTwo(RowShardedAttention):
+        world_size, rank = 2, 0
+
+        def _symmetric_result(self, shape, dtype, device):
+            return kept
+
+    kept = (torch.zeros(2, 4, 3, device=cuda_device), NoBarrier(), [None, torch.zeros(2, 4, 3, device=cuda_device)])
+    w = torch.tensor(2.0, device=cuda_device, requires_grad=True)
+    op = RankZeroOfTwo(attention_fn=lambda *a: None)
+    for call in range(2):
+        out = op.gather_rows(8, (3,), torch.float32, cuda_device, lambda lo, hi, slot, kw: slot.copy_(w * (torch.ones_like(slot) + call)))
+        w.grad = None
+        out.sum().backward()
+        assert w.grad.item() == 12.0 * (1 + call)
+        assert not kept[0].requires_grad and not kept[2][1].requires_grad
+        torch.cuda.synchronize()
+        assert torch.equal(kept[2][1][0], torch.full((4, 3), 2.0 * (1 + call), device=cuda_device))
