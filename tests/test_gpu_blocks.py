@@ -394,7 +394,7 @@ def test_a_part_of_the_weights_is_not_taken_for_the_whole(cuda_device):
         _close(out, O.self_block_fp32(x, torch.ones(N, dtype=torch.bool), bias, cpu[0].T, qb, *(w.T for w in cpu[1:]), H), C)
 
 
-@pytest.mark.parametrize("N,C,H", [(1, 64, 4), (77, 72, 3), (130, 200, 5), (300, 384, 16), (1100, 512, 8), (129, 1024, 16)])
+@pytest.mark.parametrize("N,C,H", [(1, 64, 4), (77, 72, 3), (130, 200, 5), (300, 384, 16), (1100, 512, 8), (129, 1024, 16), (3600, 72, 3)])
 def test_self_block_reads_weights_of_any_layout(cuda_device, N, C, H):
     """Weights kept `[in, out]`, `[out, in]`, as parts of larger matrices, mixed, and in forms that are packed first
     (odd pitch, odd offset, fp32 with the same values) give the same bits, on channel counts short of and past whole
