@@ -135,7 +135,8 @@ struct BarIdx {
   static constexpr int q_full = 12 + 2 * kMaxKvStages;       // [2 * kMaxStreams]  Q tile landed
   static constexpr int q_empty = q_full + 2 * kMaxStreams;   // [2 * kMaxStreams]  last Q K^T of the stream finished
   static constexpr int q_scaled = q_empty + 2 * kMaxStreams; // [2 * kMaxStreams]  the P V warp has scaled the Q tile
-  static constexpr int count = q_scaled + 2 * kMaxStreams;
+  static constexpr int o_done = q_scaled + 2 * kMaxStreams;  // [2]  the item's last P V of the warpgroup finished
+  static constexpr int count = o_done + 2;
 };
 static_assert(BarIdx::count * 8 <= (int)kBarrierBlockBytes, "barrier block too small");
 
@@ -237,25 +238,35 @@ __device__ __forceinline__ Item decode_item(const AttnParams& p, int item) {
 __device__ __forceinline__ int stream_row(const AttnParams& p, const Item& it, int s) { return p.q_split ? it.r0 : it.r0 + s; }
 __device__ __forceinline__ int stream_qt(const AttnParams& p, const Item& it, int s) { return p.q_split ? it.qt + s : it.qt; }
 
-// Q buffer of the CTA's j-th item and how often that buffer was used before.
+// Q buffer of the CTA's j-th item.
 __device__ __forceinline__ uint32_t q_buf(const AttnParams& p, uint32_t j) { return p.q_buffers == 2 ? (j & 1u) : 0u; }
-__device__ __forceinline__ uint32_t q_use(const AttnParams& p, uint32_t j) { return p.q_buffers == 2 ? (j >> 1) : j; }
+
+// Uses of every Q slot (buffer x stream) so far, modulo two.  Counted by slot: items differ in their streams, so a slot
+// is not used each time its buffer is.
+struct QUses {
+  uint32_t odd = 0;
+  __device__ __forceinline__ uint32_t parity(int slot) const { return (odd >> slot) & 1u; }   // of the next use's phase
+  __device__ __forceinline__ void used(int slot) { odd ^= 1u << slot; }
+};
 
 // ------------------------------------------------------------------ producer (one thread)
 __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUtensorMap* tm_k,
                               const CUtensorMap* tm_v, const CUtensorMap* tm_bias) {
   const AttnParams& p = *c.p;
-  uint32_t ucount = 0, bcount = 0, icount = 0;
+  uint32_t ucount = 0, bcount = 0, icount = 0, q_before = 0;
+  QUses q_uses;
   const uint32_t nkv = p.kv_stages;
   // With two Q buffers the tiles of the next item are requested while the current item runs, so
   // that they are in place (and scaled) when it ends; with one (tiles too large for two), as
   // soon as the current item's K/V loads are all issued.
   auto load_q = [&](const Item& it, uint32_t j) {
-    const uint32_t buf = q_buf(p, j), use = q_use(p, j);
+    const uint32_t buf = q_buf(p, j);
     for (int s = 0; s < it.gv; ++s) {
       const int slot = (int)buf * kMaxStreams + s;
       // the buffer's previous user must have finished its last Q K^T of this stream
-      if (use >= 1) AF3K_WAIT_NORET(c, BarIdx::q_empty + slot, (use - 1) & 1);
+      if ((q_before >> slot) & 1u) AF3K_WAIT_NORET(c, BarIdx::q_empty + slot, q_uses.parity(slot) ^ 1u);
+      q_before |= 1u << slot;
+      q_uses.used(slot);
       mbar_arrive_expect_tx(bar_addr(c, BarIdx::q_full + slot), p.q_tile_bytes);
       tma_load_4d(c.smem + p.off_q + (buf * p.n_streams + s) * p.q_tile_bytes, tm_q, bar_addr(c, BarIdx::q_full + slot),
                   0, stream_qt(p, it, s) * kTile, it.h, stream_row(p, it, s));
@@ -342,6 +353,7 @@ __device__ __forceinline__ uint16_t masked_value_bits(const AttnParams& p, int h
 struct QScaler {
   uint32_t item = 0, chunk = 0;   // item index (per CTA) of the tiles being scaled, next piece
   int gv = 0, tile = 0;           // tiles that item has, next tile
+  QUses uses;
   __device__ __forceinline__ void start(uint32_t j, int n) { item = j; gv = n; tile = 0; chunk = 0; }
   __device__ __forceinline__ bool pending() const { return tile < gv; }
   // One piece.  block: wait (bounded) for the tile to land, else give up if it has not.
@@ -352,7 +364,7 @@ struct QScaler {
     const uint32_t buf = q_buf(p, item);
     const int slot = (int)buf * kMaxStreams + tile;
     if (chunk == 0) {
-      const uint32_t par = q_use(p, item) & 1;
+      const uint32_t par = uses.parity(slot);
       bool ok = mbar_test_wait(bar_addr(c, BarIdx::q_full + slot), par);
       if (!__all_sync(0xffffffffu, ok)) {
         if (!block) return 0;
@@ -368,6 +380,7 @@ struct QScaler {
       fence_proxy_async_smem();    // make the generic-proxy stores visible to the tensor core
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::q_scaled + slot));
+      uses.used(slot);
       chunk = 0;
       ++tile;
     }
@@ -478,6 +491,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
   // ring positions / barrier parities are carried incrementally: no division on this warp
   uint32_t st = 0, kv_par = 0, icount = 0, bst = 0, b_par = 0;
   uint32_t sfree_par[2] = {0, 0}, first[2] = {1, 1};
+  QUses q_uses;
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
     const Item it = decode_item(p, item);
     const int gv = it.gv;
@@ -493,14 +507,15 @@ __device__ void qk_issuer_role(const Ctx& c) {
           bool ok = mbar_test_wait(bar_addr(c, BarIdx::kv_full + st), kv_par);
           if (need_sfree) ok = mbar_test_wait(bar_addr(c, BarIdx::s_free + b), sfree_par[b]) && ok;
           if (need_bias) ok = mbar_test_wait(bar_addr(c, BarIdx::bias_full + bst), b_par) && ok;
-          if (kt == 0) ok = mbar_test_wait(bar_addr(c, q_bar), q_use(p, icount) & 1) && ok;
+          if (kt == 0) ok = mbar_test_wait(bar_addr(c, q_bar), q_uses.parity(qslot)) && ok;
           if (!__all_sync(0xffffffffu, ok)) {
             if (need_bias) AF3K_WAIT_WARP_C(c, BarIdx::bias_full + bst, b_par);
             // the softmax warpgroup of this buffer must have read the previous logits tile
             if (need_sfree) AF3K_WAIT_WARP_C(c, BarIdx::s_free + b, sfree_par[b]);
-            if (kt == 0) AF3K_WAIT_WARP_C(c, q_bar, q_use(p, icount) & 1);
+            if (kt == 0) AF3K_WAIT_WARP_C(c, q_bar, q_uses.parity(qslot));
             AF3K_WAIT_WARP_C(c, BarIdx::kv_full + st, kv_par);
           }
+          if (kt == 0) q_uses.used(qslot);
         }
         if (need_sfree) sfree_par[b] ^= 1;
         first[b] = 0;
@@ -597,6 +612,7 @@ __device__ void pv_issuer_role(const Ctx& c, int lane) {
             mma_ts_f16(o_tmem, p_tmem + k * 8, b_lo + k * v_kstep, vd_hi, idesc_pv, 1u);
           // one completion signal: the K/V stage is free, and so are this tile's P buffer and O
           tc_commit(bar_addr(c, BarIdx::kv_empty + st));
+          if (kt == p.n_kt - 1 && s + 2 >= gv) tc_commit(bar_addr(c, BarIdx::o_done + b));
           if (tl != nullptr && tl_n + 2 <= 2 * kDbgTimelineTiles) { tl[tl_n++] = t0; tl[tl_n++] = clock64(); }
         }
         __syncwarp();
@@ -723,7 +739,7 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, float* dbg, int wg, i
   // passes, when both read logits, search the maximum and hand P over and the XU idles.
   const uint64_t l2e2 = pack_f32x2(ef, ef);
   const uint64_t nm2 = pack_f32x2(-m_use, -m_use);
-  const float nml = -m_use * ef;
+  const float nml = fminf(-m_use * ef, 3.0e38f);   // finite for bias entries of the type's lowest value: such keys weigh nothing
   const uint64_t nml2 = pack_f32x2(nml, nml);
   uint64_t suma = pack_f32x2(0.f, 0.f), sumb = suma;
   // The first kHeld column groups are computed before anything is written: the P buffer and the
@@ -812,6 +828,8 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
   // position of tiles in the CTA-wide order (all streams): gives the K/V stage a tile used
   uint32_t kt_stage = 0, kt_round = 0;                // ring stage / lap of stream 0's tile at the current key tile
   uint32_t prev_stage = 0, prev_round = 0;            // the same for this warpgroup's last tile
+  uint32_t kt_tile = 0, prev_tile = 0;                // and the positions themselves
+  uint32_t own_items = 0;                             // items in which this warpgroup had a stream
   const uint32_t nkv = p.kv_stages;
 
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
@@ -848,8 +866,12 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
         float* dbg = nullptr;
         if (kDebug && p.debug != nullptr && blockIdx.x == 0 && icount == 0 && s == 0 && kt == 0)
           dbg = p.debug + (size_t)row * kTile;
+        // a warpgroup that had no stream for a while: its previous P V has finished when a later tile took the K/V stage,
+        // and the stage's barrier, laps on, no longer tells
+        const uint32_t tile = kt_tile + (uint32_t)s;
+        const bool prev_pending = ucnt > 0 && tile - prev_tile < nkv;
         if (!softmax_tile<kTcBias>(c, dbg, wg, lane, s_taddr, p_taddr, o_taddr, p.nv, bias_row, row & 7, scale,
-                                   kt == 0, ucnt > 0, BarIdx::kv_empty + (int)prev_stage, prev_round & 1, m_run,
+                                   kt == 0, prev_pending, BarIdx::kv_empty + (int)prev_stage, prev_round & 1, m_run,
                                    l_run, BarIdx::s_full + wg, (ucnt + 1) & 1, s_ready, ts))
           return;
         ++ucnt;
@@ -857,6 +879,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
           // tiles are numbered in the producer's order; the numbers are carried without a division
           prev_stage = kt_stage + (uint32_t)s;
           prev_round = kt_round;
+          prev_tile = tile;
           while (prev_stage >= nkv) { prev_stage -= nkv; ++prev_round; }
         }
         tc_fence_before();
@@ -869,6 +892,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
         if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::bias_empty + bst));
       }
       ++bcount;
+      kt_tile += (uint32_t)it.gv;
       kt_stage += (uint32_t)it.gv;
       while (kt_stage >= nkv) { kt_stage -= nkv; ++kt_round; }
     }
@@ -877,10 +901,9 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
     // ---- epilogue: O / l -> bf16 -> global, once this warpgroup's last P V has finished (the
     // other warpgroup may still be working on its own streams)
     if (kDebug && last_ts != nullptr) last_ts[5] = clock64();
-    // only a warpgroup that had a stream in this item has a P V of this item to wait for (with an
-    // odd row count the last item leaves warpgroup 1 without one: its record of a previous tile
-    // may be a whole number of ring laps old, and the parity test would then wait for ever)
-    if (wg < it.gv) AF3K_WAIT_WARP(c, BarIdx::kv_empty + (int)prev_stage, prev_round & 1);
+    // (a barrier of its own, once per item with a stream: the K/V stage of its last tile may be taken again, by tiles of
+    // the other warpgroup alone, before this one looks)
+    if (wg < it.gv) { AF3K_WAIT_WARP(c, BarIdx::o_done + wg, own_items & 1); ++own_items; }
     tc_fence_after();
     if (kDebug && last_ts != nullptr) last_ts[6] = clock64();
     for (int s = wg; s < it.gv; s += 2) {
@@ -968,6 +991,7 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar_addr(c, BarIdx::epi_done + i), 4);
+      mbar_init(bar_addr(c, BarIdx::o_done + i), 1);
       mbar_init(bar_addr(c, BarIdx::s_full + i), 1);
       mbar_init(bar_addr(c, BarIdx::s_free + i), 4);
       mbar_init(bar_addr(c, BarIdx::p_ready + i), 4);
