@@ -92,9 +92,11 @@ int device_info(DeviceInfo** out) {
     const int dyn = d.max_smem_optin - kStaticSmemReserve;
     const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     const void* kernels[] = {
-        (const void*)attention_kernel<false, false, false>, (const void*)attention_kernel<true, false, false>,
-        (const void*)attention_kernel<false, true, false>,  (const void*)attention_kernel<true, true, false>,
-        (const void*)attention_kernel<false, false, true>,  (const void*)attention_kernel<false, true, true>,
+        (const void*)attention_kernel<false, true, false, false>, (const void*)attention_kernel<false, true, false, true>,
+        (const void*)attention_kernel<false, true, true, false>,  (const void*)attention_kernel<false, true, true, true>,
+        (const void*)attention_kernel<false, false, true, false>, (const void*)attention_kernel<false, false, true, true>,
+        (const void*)attention_kernel<true, true, false, false>,  (const void*)attention_kernel<true, true, true, false>,
+        (const void*)attention_kernel<true, false, true, false>,
     };
     e = cudaSuccess;
     for (const void* kfn : kernels)
@@ -221,7 +223,6 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   p.B1 = (int)d.B1; p.B2 = (int)d.B2; p.Sq = (int)d.Sq; p.Sk = (int)d.Sk; p.D = (int)d.D;
   p.n_qt = (p.Sq + kTile - 1) / kTile;
   p.n_kt = (p.Sk + kTile - 1) / kTile;
-  p.qk_is_fp8 = es == 1;
   p.qk_row_bytes = row_bytes_for(d.D * es);
   p.v_row_bytes = row_bytes_for(d.D * 2);
   p.qk_ksteps = (int)((d.D * es + 31) / 32);
@@ -286,6 +287,8 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   const long long items = groups * p.B2 * (p.q_split ? (p.n_qt + 1) / 2 : p.n_qt);
   if (items > 0x7fffffff) return AF3K_ERR_BAD_SHAPE;
   p.n_items = (int)items;
+  p.div_q = make_divisor((uint32_t)(p.q_split ? (p.n_qt + 1) / 2 : p.n_qt));
+  p.div_h = make_divisor((uint32_t)p.B2);
 
   uint32_t off = 0;
   p.off_q = off;      off += p.q_buffers * p.n_streams * p.q_tile_bytes;
@@ -551,11 +554,17 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
   const bool dbg = p.debug != nullptr;
 #define AF3K_LAUNCH(...) launch_overlapped(attention_kernel<__VA_ARGS__>, dim3(plan.grid), kThreads, plan.smem_bytes, stream, d.max_ctas <= 0, p, tm_q, tm_k, tm_v, tm_b)
   if (p.gate != nullptr) {
-    if (tc_bias) AF3K_LAUNCH(false, true, true); else AF3K_LAUNCH(false, false, true);
-  } else if (!tc_bias) {
-    if (dbg) AF3K_LAUNCH(true, false, false); else AF3K_LAUNCH(false, false, false);
+    if (!fp8)         AF3K_LAUNCH(false, true, false, true);
+    else if (tc_bias) AF3K_LAUNCH(false, true, true, true);
+    else              AF3K_LAUNCH(false, false, true, true);
+  } else if (dbg) {
+    if (!fp8)         AF3K_LAUNCH(true, true, false, false);
+    else if (tc_bias) AF3K_LAUNCH(true, true, true, false);
+    else              AF3K_LAUNCH(true, false, true, false);
   } else {
-    if (dbg) AF3K_LAUNCH(true, true, false); else AF3K_LAUNCH(false, true, false);
+    if (!fp8)         AF3K_LAUNCH(false, true, false, false);
+    else if (tc_bias) AF3K_LAUNCH(false, true, true, false);
+    else              AF3K_LAUNCH(false, false, true, false);
   }
 #undef AF3K_LAUNCH
   cudaError_t e = cudaGetLastError();

@@ -84,6 +84,23 @@ enum StatusBits : int {
   kStatusWaitTimeout = 1,   // a bounded mbarrier wait ran out
 };
 
+// x / d for 0 <= x < 2^31 by a multiplication (d == 1: mul == 0).  Every role decodes every item, and a division is some
+// forty instructions, several times over in each role's loop.
+struct Divisor {
+  uint32_t d, mul, shift;
+};
+inline Divisor make_divisor(uint32_t d) {
+  Divisor r{d, 0, 0};
+  if (d > 1) {
+    uint32_t l = 1;
+    while ((1ull << l) < d) ++l;
+    r.mul = (uint32_t)(((1ull << (31 + l)) + d - 1) / d);
+    r.shift = l - 1;
+  }
+  return r;
+}
+__device__ __forceinline__ uint32_t divide(uint32_t x, const Divisor& v) { return v.mul != 0 ? __umulhi(x, v.mul) >> v.shift : x; }
+
 struct AttnParams {
   int B1, B2, Sq, Sk, D;
   int n_qt, n_kt;
@@ -91,13 +108,13 @@ struct AttnParams {
   int q_split;           // 1: the streams of an item are two neighbouring query tiles of ONE pair row (G == 1)
   int n_streams;         // streams per work item: G, or 2 with q_split
   int n_items;
+  Divisor div_q, div_h;  // query tiles (or pairs of them) per row and head, heads
   int qk_row_bytes;      // smem bytes per Q / K tile row: 32, 64 or 128 (= swizzle span)
   int v_row_bytes;       // same for V
   int qk_ksteps;         // number of 32-byte K steps of the first GEMM
   int nv;                // N of the second GEMM: D rounded up to 16
   int kv_stages;
   int q_buffers;         // 2: Q tiles double-buffered by item (the next item's land while this one runs); 1: single
-  int qk_is_fp8;
   int scale_q;           // 1: bf16 q/k, the Q tiles are multiplied by `scale` in shared memory
   float scale;           // softmax scale; multiplied by q_scale[h] * k_scale[h] when those are set
   const float* q_scale;
@@ -156,58 +173,70 @@ struct Ctx {
 
 __device__ __forceinline__ uint32_t bar_addr(const Ctx& c, int idx) { return c.bars + 8u * idx; }
 
-__device__ __noinline__ void report_timeout(const Ctx& c, int bar_idx) {
-  *c.abort_flag = 1;
-  if (c.p->status != nullptr) {
-    atomicOr(c.p->status, kStatusWaitTimeout);
-    if (atomicCAS(c.p->status + 1, 0, bar_idx + 1) == 0) {
-      c.p->status[2] = blockIdx.x;
-      c.p->status[3] = threadIdx.x >> 5;
+// Arguments by value: a reference to the context would keep it in memory.
+__device__ __noinline__ void report_timeout_at(const AttnParams* p, volatile int* abort_flag, int bar_idx) {
+  *abort_flag = 1;
+  if (p->status != nullptr) {
+    atomicOr(p->status, kStatusWaitTimeout);
+    if (atomicCAS(p->status + 1, 0, bar_idx + 1) == 0) {
+      p->status[2] = blockIdx.x;
+      p->status[3] = threadIdx.x >> 5;
     }
   }
+}
+__device__ __forceinline__ void report_timeout(const Ctx& c, int bar_idx) { report_timeout_at(c.p, c.abort_flag, bar_idx); }
+
+// A complete phase, or one parked attempt: most real waits end inside it.
+__device__ __forceinline__ bool mbar_test_or_park(uint32_t bar, uint32_t parity) {
+  return mbar_test_wait(bar, parity) || mbar_try_wait_park(bar, parity, 2000u);
+}
+
+// The waiting loops of the single-warp roles, out of line, with the report of a wait that ran out: a whole warp (the same
+// result in every lane), and one thread (the producer).
+__device__ __noinline__ bool wait_warp_slow_at(const AttnParams* p, volatile int* abort_flag, uint32_t bars, int idx, uint32_t parity) {
+  if (__all_sync(0xffffffffu, mbar_wait_bounded(bars + 8u * idx, parity, p->wait_limit, abort_flag))) return true;
+  report_timeout_at(p, abort_flag, idx);
+  return false;
+}
+__device__ __forceinline__ bool wait_warp_slow(const Ctx& c, int idx, uint32_t parity) {
+  return wait_warp_slow_at(c.p, c.abort_flag, c.bars, idx, parity);
+}
+__device__ __noinline__ bool wait_thread_slow_at(const AttnParams* p, volatile int* abort_flag, uint32_t bars, int idx, uint32_t parity) {
+  if (mbar_wait_bounded(bars + 8u * idx, parity, p->wait_limit, abort_flag)) return true;
+  report_timeout_at(p, abort_flag, idx);
+  return false;
+}
+__device__ __forceinline__ bool wait_thread(const Ctx& c, int idx, uint32_t parity) {
+  return mbar_test_or_park(bar_addr(c, idx), parity) || wait_thread_slow_at(c.p, c.abort_flag, c.bars, idx, parity);
 }
 
 #define AF3K_WAIT(ctx, idx, parity)                                                          \
   do {                                                                                       \
-    if (!mbar_wait_bounded(bar_addr(ctx, idx), (parity), (ctx).p->wait_limit,                \
-                           (ctx).abort_flag)) {                                              \
-      report_timeout(ctx, idx);                                                              \
-      return;                                                                                \
-    }                                                                                        \
+    if (!wait_thread(ctx, idx, parity)) return;                                              \
   } while (0)
 
 // Form for helpers that report failure through their return value.
 #define AF3K_WAIT_NORET(ctx, idx, parity)                                                    \
   do {                                                                                       \
-    if (!mbar_wait_bounded(bar_addr(ctx, idx), (parity), (ctx).p->wait_limit,                \
-                           (ctx).abort_flag)) {                                              \
-      report_timeout(ctx, idx);                                                              \
-      return false;                                                                          \
-    }                                                                                        \
+    if (!wait_thread(ctx, idx, parity)) return false;                                        \
   } while (0)
 
-// Warp-collective form: every lane leaves together, so no .sync.aligned instruction is ever
-// executed by part of a warp after a timeout.
-// The same for the single-warp roles, with the waiting loop out of line: these warps run their
-// per-tile loops rarely, next to warps that stream through long unrolled loops, and one pass of
-// such a loop costs 700 - 1 500 cycles whatever it does, so the path taken when nothing has to be
-// waited for is kept short.
+// Warp-collective forms: every lane leaves together, so no .sync.aligned instruction is ever executed by part of a warp
+// after a timeout.  _C is that of the single-warp roles, with the waiting loop out of line: one pass of their per-tile
+// loops costs 700 - 1 500 cycles whatever it does, next to warps that stream through long unrolled loops, so the path taken
+// when nothing has to be waited for is kept short.
 #define AF3K_WAIT_WARP_C(ctx, idx, parity)                                                   \
   do {                                                                                       \
-    const bool ok_ = mbar_wait_bounded_compact(bar_addr(ctx, idx), (parity), (ctx).p->wait_limit, \
-                                               (ctx).abort_flag);                            \
-    if (!__all_sync(0xffffffffu, ok_)) {                                                     \
-      report_timeout(ctx, idx);                                                              \
-      return;                                                                                \
-    }                                                                                        \
+    if (!__all_sync(0xffffffffu, mbar_test_or_park(bar_addr(ctx, idx), (parity))))           \
+      if (!wait_warp_slow(ctx, idx, parity)) return;                                         \
   } while (0)
-
+// The softmax warps keep the waiting loop inline: a call would have to save their registers.
 #define AF3K_WAIT_WARP(ctx, idx, parity)                                                     \
   do {                                                                                       \
     const bool ok_ = mbar_wait_bounded(bar_addr(ctx, idx), (parity), (ctx).p->wait_limit,    \
                                        (ctx).abort_flag);                                    \
     if (!__all_sync(0xffffffffu, ok_)) {                                                     \
-      report_timeout(ctx, idx);                                                                \
+      report_timeout(ctx, idx);                                                              \
       return;                                                                                \
     }                                                                                        \
   } while (0)
@@ -226,12 +255,10 @@ struct Item {
 };
 __device__ __forceinline__ Item decode_item(const AttnParams& p, int item) {
   Item it;
-  const int nq = p.q_split ? (p.n_qt + 1) >> 1 : p.n_qt;
-  it.qt = (item % nq) << p.q_split;
-  int t = item / nq;
-  it.h = t % p.B2;
-  int rg = t / p.B2;
-  it.r0 = rg * p.G;
+  const uint32_t t = divide((uint32_t)item, p.div_q), rg = divide(t, p.div_h);
+  it.qt = (int)((uint32_t)item - t * p.div_q.d) << p.q_split;
+  it.h = (int)(t - rg * p.div_h.d);
+  it.r0 = (int)rg * p.G;
   it.gv = p.q_split ? min(2, p.n_qt - it.qt) : min(p.G, p.B1 - it.r0);
   return it;
 }
@@ -261,6 +288,7 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
   // soon as the current item's K/V loads are all issued.
   auto load_q = [&](const Item& it, uint32_t j) {
     const uint32_t buf = q_buf(p, j);
+#pragma unroll 1
     for (int s = 0; s < it.gv; ++s) {
       const int slot = (int)buf * kMaxStreams + s;
       // the buffer's previous user must have finished its last Q K^T of this stream
@@ -276,9 +304,12 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
   if ((int)blockIdx.x < p.n_items) {
     if (!load_q(decode_item(p, blockIdx.x), 0)) return;
   }
+#pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
     const Item it = decode_item(p, item);
+#pragma unroll 1
     for (int kt = 0; kt < p.n_kt; ++kt) {
+#pragma unroll 1
       for (int s = 0; s < it.gv; ++s) {
         if (s == 0 || p.q_split) {   // one bias tile per key tile, or per stream when the streams are query tiles
           const uint32_t bst = bcount % kBiasStages;
@@ -365,14 +396,9 @@ struct QScaler {
     const int slot = (int)buf * kMaxStreams + tile;
     if (chunk == 0) {
       const uint32_t par = uses.parity(slot);
-      bool ok = mbar_test_wait(bar_addr(c, BarIdx::q_full + slot), par);
-      if (!__all_sync(0xffffffffu, ok)) {
+      if (!__all_sync(0xffffffffu, mbar_test_wait(bar_addr(c, BarIdx::q_full + slot), par))) {
         if (!block) return 0;
-        ok = mbar_wait_bounded(bar_addr(c, BarIdx::q_full + slot), par, p.wait_limit, c.abort_flag);
-        if (!__all_sync(0xffffffffu, ok)) {
-          report_timeout(c, BarIdx::q_full + slot);
-          return -1;
-        }
+        if (!wait_warp_slow(c, BarIdx::q_full + slot, par)) return -1;
       }
     }
     scale_q_chunk(c.smem + p.off_q + (buf * p.n_streams + tile) * p.q_tile_bytes + (chunk << 10), p.scale, lane);
@@ -412,19 +438,22 @@ __device__ void mask_writer_role(const Ctx& c, int lane) {
   const AttnParams& p = *c.p;
   const uint32_t nkv = p.kv_stages;
   uint32_t st = 0, round = 0;      // ring slot, how many times the ring wrapped
+#pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
     const Item it = decode_item(p, item);
-    uint16_t val[4];
+    uint16_t val[4] = {};
     const uint16_t masked = masked_value_bits(p, it.h);
-    mask_values(p, it, 0, 0, lane, masked, val);
-    for (int kt = 0; kt < p.n_kt; ++kt) {
-      for (int s = 0; s < it.gv; ++s) {
-        const uint16_t cur[4] = {val[0], val[1], val[2], val[3]};
-        {
-          const int ns = s + 1 < it.gv ? s + 1 : 0;
-          const int nkt = s + 1 < it.gv ? kt : kt + 1;
-          if (nkt < p.n_kt) mask_values(p, it, nkt, ns, lane, masked, val);
-        }
+    // step i writes the values of tile i (key tiles outermost, then streams) and requests those of tile i + 1
+    const int tiles = p.n_kt * it.gv;
+    int nkt = 0, ns = 0;           // the tile requested next
+#pragma unroll 1
+    for (int i = -1; i < tiles; ++i) {
+      const uint16_t cur[4] = {val[0], val[1], val[2], val[3]};
+      if (i + 1 < tiles) {
+        mask_values(p, it, nkt, ns, lane, masked, val);
+        if (++ns == it.gv) { ns = 0; ++nkt; }
+      }
+      if (i >= 0) {
         if (round > 0) AF3K_WAIT_WARP_C(c, BarIdx::kv_empty + st, (round - 1) & 1);
         const uint32_t slot = c.smem + p.off_mcol + st * kMaskPanelBytes;
 #pragma unroll
@@ -452,7 +481,7 @@ __device__ void mask_writer_role(const Ctx& c, int lane) {
 // Logits of every tile, in order: Q K^T, then the mask column, then (bf16 q/k) the bias slices.
 // (The MMA loops are real loops and the fp8 / bf16 choice is a template argument: the warp pays an
 // instruction-cache miss for most lines of this loop on every pass, so the loop is kept small.)
-template <bool kTcBias, bool kFp8>
+template <bool kDebug, bool kTcBias, bool kFp8>
 __device__ void qk_issuer_role(const Ctx& c) {
   const AttnParams& p = *c.p;
   const bool leader = elect_one();
@@ -484,41 +513,45 @@ __device__ void qk_issuer_role(const Ctx& c) {
   const uint32_t bd_lo = (uint32_t)bd0, bd_hi = (uint32_t)(bd0 >> 32);
   const uint32_t id_lo = (uint32_t)id0, id_hi = (uint32_t)(id0 >> 32);
   const uint32_t idesc_bias = make_idesc(1u, 1u, 0u, 0u, 16);
-  long long* tl = (p.debug != nullptr && blockIdx.x == 0)
+  long long* tl = (kDebug && p.debug != nullptr && blockIdx.x == 0)
                       ? reinterpret_cast<long long*>(p.debug + kDbgFloats) + 2 * kDbgTimelineTiles * 8
                       : nullptr;
   uint32_t tl_n = 0;
   // ring positions / barrier parities are carried incrementally: no division on this warp
   uint32_t st = 0, kv_par = 0, icount = 0, bst = 0, b_par = 0;
-  uint32_t sfree_par[2] = {0, 0}, first[2] = {1, 1};
+  uint32_t sfree_par = 0, used = 0;   // bit b: parity of buffer b's next release; buffer b has held a tile
   QUses q_uses;
+#pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
     const Item it = decode_item(p, item);
     const int gv = it.gv;
+#pragma unroll 1
     for (int kt = 0; kt < p.n_kt; ++kt) {
+#pragma unroll 1
       for (int s = 0; s < gv; ++s) {
         const int b = s & 1;
         const int qslot = (int)q_buf(p, icount) * kMaxStreams + s;
         const int q_bar = (p.scale_q ? BarIdx::q_scaled : BarIdx::q_full) + qslot;
         const bool need_bias = kTcBias && (s == 0 || p.q_split);
-        const bool need_sfree = !first[b];
+        const bool need_sfree = (used >> b) & 1u;
+        const uint32_t sf_par = (sfree_par >> b) & 1u;
         {
           // everything the tile needs is normally there already: test all its barriers, vote once
           bool ok = mbar_test_wait(bar_addr(c, BarIdx::kv_full + st), kv_par);
-          if (need_sfree) ok = mbar_test_wait(bar_addr(c, BarIdx::s_free + b), sfree_par[b]) && ok;
+          if (need_sfree) ok = mbar_test_wait(bar_addr(c, BarIdx::s_free + b), sf_par) && ok;
           if (need_bias) ok = mbar_test_wait(bar_addr(c, BarIdx::bias_full + bst), b_par) && ok;
           if (kt == 0) ok = mbar_test_wait(bar_addr(c, q_bar), q_uses.parity(qslot)) && ok;
           if (!__all_sync(0xffffffffu, ok)) {
             if (need_bias) AF3K_WAIT_WARP_C(c, BarIdx::bias_full + bst, b_par);
             // the softmax warpgroup of this buffer must have read the previous logits tile
-            if (need_sfree) AF3K_WAIT_WARP_C(c, BarIdx::s_free + b, sfree_par[b]);
+            if (need_sfree) AF3K_WAIT_WARP_C(c, BarIdx::s_free + b, sf_par);
             if (kt == 0) AF3K_WAIT_WARP_C(c, q_bar, q_uses.parity(qslot));
             AF3K_WAIT_WARP_C(c, BarIdx::kv_full + st, kv_par);
           }
           if (kt == 0) q_uses.used(qslot);
         }
-        if (need_sfree) sfree_par[b] ^= 1;
-        first[b] = 0;
+        if (need_sfree) sfree_par ^= 1u << b;
+        used |= 1u << b;
         tc_fence_after();
         const uint32_t a_lo = qd_lo + (q_buf(p, icount) * p.n_streams + s) * q_step;
         const uint32_t b_lo = kd_lo + st * stage_step;
@@ -526,7 +559,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
         const uint32_t slot16 = st * (kMaskPanelBytes >> 4);
         const uint32_t bias_lo = bd_lo + bst * (kBiasTileBytes >> 4);
         if (leader) {
-          const long long t0 = tl != nullptr ? clock64() : 0;
+          const long long t0 = kDebug && tl != nullptr ? clock64() : 0;
 #pragma unroll 1
           for (int k = 0; k < ksteps; ++k) {     // one K step = 32 bytes of a tile row
             if (fp8) mma_ss_f8(s_tmem, a_lo + 2 * k, qd_hi, b_lo + 2 * k, kd_hi, idesc_qk, k > 0 ? 1u : 0u);
@@ -544,7 +577,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
           }
           tc_commit(bar_addr(c, BarIdx::s_full + b));
           if (kt == p.n_kt - 1) tc_commit(bar_addr(c, BarIdx::q_empty + qslot));
-          if (tl != nullptr && tl_n + 2 <= 2 * kDbgTimelineTiles) { tl[tl_n++] = t0; tl[tl_n++] = clock64(); }
+          if (kDebug && tl != nullptr && tl_n + 2 <= 2 * kDbgTimelineTiles) { tl[tl_n++] = t0; tl[tl_n++] = clock64(); }
         }
         __syncwarp();
         if (++st == nkv) { st = 0; kv_par ^= 1; }
@@ -562,7 +595,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
 // O += P V for every tile, in order.  This warp mostly waits for the softmax warpgroups, so (bf16
 // q/k) it also scales the Q tiles: the first item's up front, the next item's in 1 KB pieces
 // while it waits, what is left when the item's last P V has been issued.
-template <bool kTcBias>
+template <bool kDebug, bool kTcBias>
 __device__ void pv_issuer_role(const Ctx& c, int lane) {
   const AttnParams& p = *c.p;
   const bool leader = elect_one();
@@ -581,22 +614,25 @@ __device__ void pv_issuer_role(const Ctx& c, int lane) {
   const uint32_t vd_lo = (uint32_t)vd0, vd_hi = (uint32_t)(vd0 >> 32);
   const uint32_t stage_step = kv_stage_bytes >> 4;
   const uint32_t v_kstep = (16u * p.v_row_bytes) >> 4;
-  long long* tl = (p.debug != nullptr && blockIdx.x == 0)
+  long long* tl = (kDebug && p.debug != nullptr && blockIdx.x == 0)
                       ? reinterpret_cast<long long*>(p.debug + kDbgFloats) + 2 * kDbgTimelineTiles * 8 +
                             2 * kDbgTimelineTiles
                       : nullptr;
   uint32_t tl_n = 0;
   uint32_t st = 0, icount = 0;
-  uint32_t pready_par[2] = {0, 0};
+  uint32_t pready_par = 0;         // bit b: of warpgroup b's next P
+#pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
     const Item it = decode_item(p, item);
     const int gv = it.gv;
     scaler.start(icount + 1, (kTcBias && p.scale_q && item + (int)gridDim.x < p.n_items) ? decode_item(p, item + gridDim.x).gv : 0);
+#pragma unroll 1
     for (int kt = 0; kt < p.n_kt; ++kt) {
+#pragma unroll 1
       for (int s = 0; s < gv; ++s) {
         const int b = s & 1;
-        if (b) { AF3K_WAIT_WARP_OR_SCALE(c, BarIdx::p_ready + 1, pready_par[1], scaler, lane); pready_par[1] ^= 1; }
-        else   { AF3K_WAIT_WARP_OR_SCALE(c, BarIdx::p_ready + 0, pready_par[0], scaler, lane); pready_par[0] ^= 1; }
+        AF3K_WAIT_WARP_OR_SCALE(c, BarIdx::p_ready + b, (pready_par >> b) & 1u, scaler, lane);
+        pready_par ^= 1u << b;
         // the warpgroup's epilogue of the previous item must have read its O accumulators before
         // its first P V of this item overwrites one
         if (kt == 0 && s < 2 && icount > 0) AF3K_WAIT_WARP_C(c, BarIdx::epi_done + b, (icount - 1) & 1);
@@ -605,7 +641,7 @@ __device__ void pv_issuer_role(const Ctx& c, int lane) {
         const uint32_t o_tmem = c.tmem + kOCol + s * p.nv;
         const uint32_t p_tmem = c.tmem + kPCol + b * 64;
         if (leader) {
-          const long long t0 = tl != nullptr ? clock64() : 0;
+          const long long t0 = kDebug && tl != nullptr ? clock64() : 0;
           mma_ts_f16(o_tmem, p_tmem, b_lo, vd_hi, idesc_pv, kt > 0 ? 1u : 0u);
 #pragma unroll 1
           for (int k = 1; k < kTile / 16; ++k)   // 16 keys per step: 8 TMEM columns of P
@@ -613,7 +649,7 @@ __device__ void pv_issuer_role(const Ctx& c, int lane) {
           // one completion signal: the K/V stage is free, and so are this tile's P buffer and O
           tc_commit(bar_addr(c, BarIdx::kv_empty + st));
           if (kt == p.n_kt - 1 && s + 2 >= gv) tc_commit(bar_addr(c, BarIdx::o_done + b));
-          if (tl != nullptr && tl_n + 2 <= 2 * kDbgTimelineTiles) { tl[tl_n++] = t0; tl[tl_n++] = clock64(); }
+          if (kDebug && tl != nullptr && tl_n + 2 <= 2 * kDbgTimelineTiles) { tl[tl_n++] = t0; tl[tl_n++] = clock64(); }
         }
         __syncwarp();
         if (++st == nkv) st = 0;
@@ -778,6 +814,7 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, float* dbg, int wg, i
         tc_fence_after();
       }
       if (__any_sync(0xffffffffu, need)) {
+#pragma unroll 1
         for (int c0 = 0; c0 < nv; c0 += 16) {
           uint32_t o[16];
           tmem_ld_x16(o_taddr + c0, o);
@@ -832,6 +869,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
   uint32_t own_items = 0;                             // items in which this warpgroup had a stream
   const uint32_t nkv = p.kv_stages;
 
+#pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
     const Item it = decode_item(p, item);
     // fp32 path: the logit scale the softmax threads apply themselves.  Tensor-core path: the
@@ -841,12 +879,14 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
     if (kTcBias) scale = (p.scale_q ? 1.0f : scale) * kLog2e;
 
     long long* last_ts = nullptr;     // debug build: timeline slot of the warpgroup's last tile
+#pragma unroll 1
     for (int kt = 0; kt < p.n_kt; ++kt) {
       // fp8 q/k: this thread adds the bias itself, from its row of the staged tile
       const uint32_t bst = bcount % kBiasStages;
       if (!kTcBias) AF3K_WAIT_WARP(c, BarIdx::bias_full + bst, (bcount / kBiasStages) & 1);
       const uint32_t bias_row = c.smem + p.off_bias + bst * kBiasTileBytes + row * 128;
 
+#pragma unroll 1
       for (int s = wg; s < it.gv; s += 2) {
         float m_run = -INFINITY, l_run = 0.f;
         const int si = (s - wg) >> 1;
@@ -906,6 +946,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
     if (wg < it.gv) { AF3K_WAIT_WARP(c, BarIdx::o_done + wg, own_items & 1); ++own_items; }
     tc_fence_after();
     if (kDebug && last_ts != nullptr) last_ts[6] = clock64();
+#pragma unroll 1
     for (int s = wg; s < it.gv; s += 2) {
       const int qrow = stream_qt(p, it, s) * kTile + row;
       const float inv = __frcp_rn(s == wg ? l_st[0] : l_st[1]);
@@ -915,6 +956,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
       const __nv_bfloat16* grow = nullptr;
       if constexpr (kGate)
         grow = p.gate + (long long)stream_row(p, it, s) * p.gate_stride_b1 + (long long)it.h * p.gate_stride_b2 + (long long)qrow * p.gate_stride_s;
+#pragma unroll 1
       for (int c0 = 0; c0 < p.nv; c0 += 16) {
         uint32_t o[16];
         tmem_ld_x16(o_taddr + c0, o);
@@ -960,7 +1002,12 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
 // ------------------------------------------------------------------ kernel
 // kGate: the result is multiplied by sigmoid(gate).  A template argument, because a run-time test of the pointer
 // cost calls without a gate 0.9 % (768 rows of 768 keys: 671 -> 677 us).
-template <bool kDebug, bool kTcBias, bool kGate>
+// kFp8 likewise, and for the same reason no debug stamps, divisions, second copies of a waiting loop or of a loop body
+// are left in the production kernel: nearly every line of instructions is fetched from the SM's instruction cache (432
+// requests a logits tile), which the hot loops of the roles just overflow (10 misses a tile; code added beside
+// them, with the same work done, took 43 misses and 665 -> 792 us).  83 KB of code -> 55 KB: 389 rows 261 -> 253.5 us
+// a module call, 256 rows of 64 channels 58.2 -> 57.5; 768 rows 672.6 -> 671.0, 1536 tokens 30.5 -> 30.7.
+template <bool kDebug, bool kTcBias, bool kFp8, bool kGate>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -1041,10 +1088,9 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     if (warp == 0) {
       if (lane == 0) producer_role(c, &tm_q, &tm_k, &tm_v, &tm_bias);
     } else if (warp == 1) {
-      if (p.qk_is_fp8) qk_issuer_role<kTcBias, true>(c);
-      else             qk_issuer_role<kTcBias, false>(c);
+      qk_issuer_role<kDebug, kTcBias, kFp8>(c);
     } else if (warp == 2) {
-      pv_issuer_role<kTcBias>(c, lane);
+      pv_issuer_role<kDebug, kTcBias>(c, lane);
     } else if (warp == 3) {
       if (p.mask_col) mask_writer_role(c, lane);
     }
