@@ -205,13 +205,30 @@ struct Plan {
   AttnParams p;
   size_t smem_bytes;
   int grid;
+  long long whole_items;   // work items if all were of the main size
 };
+
+// The longest CTA's time when n_main items of cost c_main and then n_tail of cost c_tail are dealt out round-robin.
+double dealt_cost(long long n_main, double c_main, long long n_tail, double c_tail, long long ctas) {
+  const long long n = n_main + n_tail, cuts[] = {0, n_main % ctas - 1, n_main % ctas, n % ctas - 1, n % ctas, ctas - 1};
+  double most = 0;
+  for (long long b : cuts) {
+    if (b < 0 || b >= ctas) continue;
+    const long long m = n_main / ctas + (b < n_main % ctas), all = n / ctas + (b < n % ctas);
+    const double cost = m * c_main + (all - m) * c_tail;
+    if (cost > most) most = cost;
+  }
+  return most;
+}
 
 // A logits tile of an item with one stream against one of an item with two: the warpgroup has the XU, the MMA
 // issuers and the instruction fetch to itself.  So where twice the CTAs are free, two query tiles take two of them:
 // 16 heads, us a call, two tiles per CTA -> one: 300 tokens 10.2 -> 8.5, 512 11.7 -> 9.6, 700 15.1 -> 13.0, 1152 (144
 // CTAs) 21.4 -> 16.8; 2 x 512 tokens 15.1 -> 11.9.  From there on the CTAs would take two rounds.
 constexpr double kLoneTile = 0.75;
+
+// Smaller items behind the last full round have to promise this much: the model is no better than that.
+constexpr double kTailGain = 0.98;
 
 // Picks rows-per-item G and the K/V ring depth from a cost model of one CTA's time (below).
 // allow_q_split: the kernel variant that will run supports query-tile streams (every variant in
@@ -242,11 +259,22 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   int g_max = kMaxStreams < g_tmem ? kMaxStreams : g_tmem;
   if (g_max > p.B1) g_max = p.B1 > 0 ? p.B1 : 1;
 
-  int best_g = 0, best_stages = 0, best_qbuf = 0;
-  bool best_split = false;
+  int best_g = 0, best_stages = 0, best_qbuf = 0, best_tail_g = 0;
+  bool best_split = false, best_tail_split = false;
+  long long best_rows = 0;     // pair rows taken by the main items
   double best_cost = 0;
+  const int ctas = (d.max_ctas > 0 && d.max_ctas < dev.sm_count) ? d.max_ctas : dev.sm_count;
   // rows_per_item is a request: it is honoured up to what TMEM and the batch allow
   const int g_req = d.rows_per_item > g_max ? g_max : d.rows_per_item;
+  auto tiles_of = [&](bool split) { return (long long)(split ? (p.n_qt + 1) / 2 : p.n_qt); };
+  // An item's time, in logits-tile times of one warpgroup: streams alternate between the two softmax warpgroups (an odd
+  // count leaves one idle slot), n_kt tiles for each of a warpgroup's slots, plus about 0.8 for the epilogue and the
+  // hand-over to the next item; with a single Q buffer the next item's Q tiles are loaded and scaled at the hand-over
+  // (about 0.5: each stream's tile is replaced as soon as its last Q K^T has finished).
+  auto item_cost = [&](int g, bool split, int qbuf) {
+    const int streams = split ? 2 : g;
+    return p.n_kt * ((streams + 1) / 2) * (streams == 1 ? kLoneTile : 1.0) + 0.8 + (qbuf == 1 ? 0.5 : 0.0);
+  };
   for (int g = 1; g <= g_max; ++g) {
     if (g_req != 0 && g != g_req) continue;
     // one pair row per item: the two softmax warpgroups take two neighbouring query tiles, or one of them idles
@@ -258,23 +286,35 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
       int stages = (budget - fixed - qbuf * streams * (int)p.q_tile_bytes) / kv_stage;
       if (stages > kMaxKvStages) stages = kMaxKvStages;
       if (stages < 2) continue;
-      const long long groups = (p.B1 + g - 1) / g;
-      const long long items = groups * p.B2 * (split ? (p.n_qt + 1) / 2 : p.n_qt);
-      const int ctas_avail = (d.max_ctas > 0 && d.max_ctas < dev.sm_count) ? d.max_ctas : dev.sm_count;
-      const long long rounds = (items + ctas_avail - 1) / ctas_avail;
-      // streams alternate between the two softmax warpgroups: an odd count leaves one idle slot.
-      // A CTA's time, in logits-tile times of one warpgroup: per item n_kt tiles for each of its
-      // slots / 2 streams plus about 0.8 for the epilogue and the hand-over to the next item; with
-      // a single Q buffer the next item's Q tiles are loaded and scaled at the hand-over (about 0.5:
-      // each stream's tile is replaced as soon as its last Q K^T has finished).
-      const int slots = split ? 2 : ((g & 1) ? g + 1 : g);
-      double cost = (double)rounds * (p.n_kt * (slots / 2) * (streams == 1 ? kLoneTile : 1.0) + 0.8 + (qbuf == 1 ? 0.5 : 0.0));
       // a K/V tile takes about two thousand cycles to arrive, most of a logits tile's time: with a
       // short ring the MMAs wait for their operands (measured: 4 stages cost about 3 %)
       static const double kRingPenalty[7] = {0, 0, 1.4, 1.15, 1.03, 1.0, 1.0};
-      cost *= kRingPenalty[stages];
-      if (split) cost *= 1.02;   // query-tile streams share no bias tile: pair rows win a tie
-      if (best_g == 0 || cost < best_cost) { best_g = g; best_cost = cost; best_stages = stages; best_qbuf = qbuf; best_split = split; }
+      double weight = kRingPenalty[stages];
+      if (split) weight *= 1.02;   // query-tile streams share no bias tile: pair rows win a tie
+      const double main_cost = item_cost(g, split, qbuf);
+      const long long per_group = (long long)p.B2 * tiles_of(split), groups = (p.B1 + g - 1) / g;
+      auto offer = [&](double cost, long long rows, int tail_g, bool tail_split) {
+        cost *= weight;
+        if (best_g != 0 && cost >= (tail_g != 0 ? kTailGain : 1.0) * best_cost) return;
+        best_g = g; best_cost = cost; best_stages = stages; best_qbuf = qbuf; best_split = split;
+        best_rows = rows; best_tail_g = tail_g; best_tail_split = tail_split;
+      };
+      offer(dealt_cost(groups * per_group, main_cost, 0, 0.0, ctas), p.B1, 0, false);
+      // A last round that is not full: the rows from some row on go to smaller items (256 rows of 64 channels, 512 items of
+      // four rows in four rounds -> 440 and 144 of two: 57.9 -> 54.5 us a module call).
+      const long long rounds = groups * per_group / ctas;
+      for (long long r = rounds; r >= 1 && r >= rounds - 1 && g_req == 0; --r) {
+        const long long main_groups = r * ctas / per_group, rows = main_groups * g;
+        if (main_groups < 1 || rows >= p.B1) continue;
+        for (int tg = 1; tg <= g; ++tg)
+          for (int ts = 0; ts <= (tg == 1 && may_split ? 1 : 0); ++ts) {
+            // two streams at least, so that both warpgroups have work, and no more than the Q buffers hold
+            const int tail_streams = ts != 0 ? 2 : tg;
+            if ((tg == g && (ts != 0) == split) || tail_streams < 2 || tail_streams > streams) continue;
+            const long long tail = (p.B1 - rows + tg - 1) / tg * p.B2 * tiles_of(ts != 0);
+            offer(dealt_cost(main_groups * per_group, main_cost, tail, item_cost(tg, ts != 0, qbuf), ctas), rows, tg, ts != 0);
+          }
+      }
     }
   }
   if (best_g == 0) return AF3K_ERR_BAD_SHAPE;
@@ -283,12 +323,18 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   p.n_streams = p.q_split ? 2 : p.G;
   p.kv_stages = best_stages;
   p.q_buffers = best_qbuf;
-  const long long groups = (p.B1 + p.G - 1) / p.G;
-  const long long items = groups * p.B2 * (p.q_split ? (p.n_qt + 1) / 2 : p.n_qt);
-  if (items > 0x7fffffff) return AF3K_ERR_BAD_SHAPE;
-  p.n_items = (int)items;
-  p.div_q = make_divisor((uint32_t)(p.q_split ? (p.n_qt + 1) / 2 : p.n_qt));
+  p.tail_g = best_tail_g;
+  p.tail_split = best_tail_split ? 1 : 0;
+  p.tail_row = (int)best_rows;
+  const long long n_main = (best_rows + p.G - 1) / p.G * p.B2 * tiles_of(best_split);
+  const long long n_tail = best_tail_g == 0 ? 0 : (p.B1 - best_rows + best_tail_g - 1) / best_tail_g * p.B2 * tiles_of(best_tail_split);
+  if (n_main + n_tail > 0x7fffffff) return AF3K_ERR_BAD_SHAPE;
+  p.n_main = (int)n_main;
+  p.n_items = (int)(n_main + n_tail);
+  p.div_q = make_divisor((uint32_t)tiles_of(best_split));
+  p.tail_div_q = make_divisor((uint32_t)tiles_of(best_tail_split));
   p.div_h = make_divisor((uint32_t)p.B2);
+  plan->whole_items = (p.B1 + p.G - 1) / p.G * (long long)p.B2 * tiles_of(best_split);
 
   uint32_t off = 0;
   p.off_q = off;      off += p.q_buffers * p.n_streams * p.q_tile_bytes;
@@ -304,7 +350,6 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   // shared memory even when the tiles need less.
   if (smem < 120 * 1024) smem = 120 * 1024;
   plan->smem_bytes = smem;
-  const int ctas = (d.max_ctas > 0 && d.max_ctas < dev.sm_count) ? d.max_ctas : dev.sm_count;
   plan->grid = p.n_items < ctas ? p.n_items : ctas;
   return AF3K_OK;
 }
@@ -596,7 +641,7 @@ int af3k_describe_plan(const af3k_attention_desc* desc, int32_t* out6) {
   if (rc != AF3K_OK) return rc;
   out6[0] = plan.p.G;
   out6[1] = plan.p.kv_stages;
-  out6[2] = plan.p.n_items;
+  out6[2] = (int32_t)plan.whole_items;
   out6[3] = plan.grid;
   out6[4] = (int32_t)plan.smem_bytes;
   out6[5] = (int32_t)kOCol + plan.p.n_streams * plan.p.nv;

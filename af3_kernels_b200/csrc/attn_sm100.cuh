@@ -55,8 +55,8 @@ namespace af3k {
 
 constexpr int kTile = 128;         // query rows per tile == keys per tile
 constexpr int kThreads = 384;      // 12 warps
-// 65536 registers per SM: launched at 168 per thread, then 128 x 56 + 256 x 224 = 64512
-constexpr int kRegsMisc = 56, kRegsSoftmax = 224;
+// 65536 registers per SM: launched at 168 per thread, then 128 x 72 + 256 x 216 = 64512
+constexpr int kRegsMisc = 72, kRegsSoftmax = 216;
 constexpr int kMaxStreams = 4;     // pair rows per work item (two per softmax warpgroup; TMEM: kOCol + G * nv <= 512 columns)
 // TMEM columns: two fp32 logits buffers, two bf16 P buffers (two keys per column), then O.
 constexpr uint32_t kSCol = 0, kPCol = 2 * 128, kOCol = 2 * 128 + 2 * 64;
@@ -108,6 +108,9 @@ struct AttnParams {
   int q_split;           // 1: the streams of an item are two neighbouring query tiles of ONE pair row (G == 1)
   int n_streams;         // streams per work item: G, or 2 with q_split
   int n_items;
+  // the items behind the first n_main are smaller: tail_g rows (or two query tiles) each, of the rows from tail_row on
+  int n_main, tail_g, tail_split, tail_row;
+  Divisor tail_div_q;
   Divisor div_q, div_h;  // query tiles (or pairs of them) per row and head, heads
   int qk_row_bytes;      // smem bytes per Q / K tile row: 32, 64 or 128 (= swizzle span)
   int v_row_bytes;       // same for V
@@ -251,53 +254,54 @@ __device__ __forceinline__ uint32_t swizzle_layout_code(int row_bytes) {
 // is not left idle) they are gv neighbouring query tiles of pair row r0, each with its own bias
 // tiles.
 struct Item {
-  int qt, h, r0, gv;
+  int qt, h, r0, gv, split;
 };
 __device__ __forceinline__ Item decode_item(const AttnParams& p, int item) {
   Item it;
-  const uint32_t t = divide((uint32_t)item, p.div_q), rg = divide(t, p.div_h);
-  it.qt = (int)((uint32_t)item - t * p.div_q.d) << p.q_split;
+  const bool tail = item >= p.n_main;
+  const uint32_t i = (uint32_t)(tail ? item - p.n_main : item);
+  const Divisor div_q = tail ? p.tail_div_q : p.div_q;
+  const int g = tail ? p.tail_g : p.G, row = tail ? p.tail_row : 0, end = tail ? p.B1 : p.tail_row;
+  it.split = tail ? p.tail_split : p.q_split;
+  const uint32_t t = divide(i, div_q), rg = divide(t, p.div_h);
+  it.qt = (int)(i - t * div_q.d) << it.split;
   it.h = (int)(t - rg * p.div_h.d);
-  it.r0 = (int)rg * p.G;
-  it.gv = p.q_split ? min(2, p.n_qt - it.qt) : min(p.G, p.B1 - it.r0);
+  it.r0 = row + (int)rg * g;
+  it.gv = it.split ? min(2, p.n_qt - it.qt) : min(g, end - it.r0);
   return it;
 }
-__device__ __forceinline__ int stream_row(const AttnParams& p, const Item& it, int s) { return p.q_split ? it.r0 : it.r0 + s; }
-__device__ __forceinline__ int stream_qt(const AttnParams& p, const Item& it, int s) { return p.q_split ? it.qt + s : it.qt; }
+__device__ __forceinline__ int stream_row(const Item& it, int s) { return it.split ? it.r0 : it.r0 + s; }
+__device__ __forceinline__ int stream_qt(const Item& it, int s) { return it.split ? it.qt + s : it.qt; }
 
-// Q buffer of the CTA's j-th item.
+// Q buffer of the CTA's j-th item and how often that buffer was used before.  An item with fewer streams than the Q
+// buffers hold takes the slots of the others through their phases all the same (an arrival on each of their barriers), so
+// that one count serves all slots: counting every slot's own uses in the issuer's loop cost 2 - 5 %.
 __device__ __forceinline__ uint32_t q_buf(const AttnParams& p, uint32_t j) { return p.q_buffers == 2 ? (j & 1u) : 0u; }
-
-// Uses of every Q slot (buffer x stream) so far, modulo two.  Counted by slot: items differ in their streams, so a slot
-// is not used each time its buffer is.
-struct QUses {
-  uint32_t odd = 0;
-  __device__ __forceinline__ uint32_t parity(int slot) const { return (odd >> slot) & 1u; }   // of the next use's phase
-  __device__ __forceinline__ void used(int slot) { odd ^= 1u << slot; }
-};
+__device__ __forceinline__ uint32_t q_use(const AttnParams& p, uint32_t j) { return p.q_buffers == 2 ? (j >> 1) : j; }
 
 // ------------------------------------------------------------------ producer (one thread)
 __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUtensorMap* tm_k,
                               const CUtensorMap* tm_v, const CUtensorMap* tm_bias) {
   const AttnParams& p = *c.p;
-  uint32_t ucount = 0, bcount = 0, icount = 0, q_before = 0;
-  QUses q_uses;
+  uint32_t ucount = 0, bcount = 0, icount = 0;
   const uint32_t nkv = p.kv_stages;
   // With two Q buffers the tiles of the next item are requested while the current item runs, so
   // that they are in place (and scaled) when it ends; with one (tiles too large for two), as
   // soon as the current item's K/V loads are all issued.
   auto load_q = [&](const Item& it, uint32_t j) {
-    const uint32_t buf = q_buf(p, j);
+    const uint32_t buf = q_buf(p, j), use = q_use(p, j);
 #pragma unroll 1
-    for (int s = 0; s < it.gv; ++s) {
+    for (int s = 0; s < p.n_streams; ++s) {
       const int slot = (int)buf * kMaxStreams + s;
       // the buffer's previous user must have finished its last Q K^T of this stream
-      if ((q_before >> slot) & 1u) AF3K_WAIT_NORET(c, BarIdx::q_empty + slot, q_uses.parity(slot) ^ 1u);
-      q_before |= 1u << slot;
-      q_uses.used(slot);
+      if (use >= 1) AF3K_WAIT_NORET(c, BarIdx::q_empty + slot, (use - 1) & 1);
+      if (s >= it.gv) {
+        mbar_arrive(bar_addr(c, BarIdx::q_full + slot));
+        continue;
+      }
       mbar_arrive_expect_tx(bar_addr(c, BarIdx::q_full + slot), p.q_tile_bytes);
       tma_load_4d(c.smem + p.off_q + (buf * p.n_streams + s) * p.q_tile_bytes, tm_q, bar_addr(c, BarIdx::q_full + slot),
-                  0, stream_qt(p, it, s) * kTile, it.h, stream_row(p, it, s));
+                  0, stream_qt(it, s) * kTile, it.h, stream_row(it, s));
     }
     return true;
   };
@@ -311,15 +315,15 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
     for (int kt = 0; kt < p.n_kt; ++kt) {
 #pragma unroll 1
       for (int s = 0; s < it.gv; ++s) {
-        if (s == 0 || p.q_split) {   // one bias tile per key tile, or per stream when the streams are query tiles
+        if (s == 0 || it.split) {   // one bias tile per key tile, or per stream when the streams are query tiles
           const uint32_t bst = bcount % kBiasStages;
           if (bcount >= kBiasStages)
             AF3K_WAIT(c, BarIdx::bias_empty + bst, ((bcount / kBiasStages) - 1) & 1);
           const uint32_t bfull = bar_addr(c, BarIdx::bias_full + bst);
           const uint32_t bdst = c.smem + p.off_bias + bst * kBiasTileBytes;
           mbar_arrive_expect_tx(bfull, kBiasTileBytes);
-          tma_load_3d(bdst, tm_bias, bfull, kt * kTile, stream_qt(p, it, s) * kTile, it.h);
-          tma_load_3d(bdst + kBiasTileBytes / 2, tm_bias, bfull, kt * kTile + 64, stream_qt(p, it, s) * kTile, it.h);
+          tma_load_3d(bdst, tm_bias, bfull, kt * kTile, stream_qt(it, s) * kTile, it.h);
+          tma_load_3d(bdst + kBiasTileBytes / 2, tm_bias, bfull, kt * kTile + 64, stream_qt(it, s) * kTile, it.h);
           ++bcount;
         }
         const uint32_t st = ucount % nkv;
@@ -327,8 +331,8 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
         const uint32_t full = bar_addr(c, BarIdx::kv_full + st);
         const uint32_t kdst = c.smem + p.off_kv + st * (p.k_tile_bytes + p.v_tile_bytes);
         mbar_arrive_expect_tx(full, p.k_tile_bytes + p.v_tile_bytes);
-        tma_load_4d(kdst, tm_k, full, 0, kt * kTile, it.h, stream_row(p, it, s));
-        tma_load_4d(kdst + p.k_tile_bytes, tm_v, full, 0, kt * kTile, it.h, stream_row(p, it, s));
+        tma_load_4d(kdst, tm_k, full, 0, kt * kTile, it.h, stream_row(it, s));
+        tma_load_4d(kdst + p.k_tile_bytes, tm_v, full, 0, kt * kTile, it.h, stream_row(it, s));
         ++ucount;
       }
       if (kt == (p.q_buffers == 2 ? 0 : p.n_kt - 1) && item + (int)gridDim.x < p.n_items) {
@@ -360,7 +364,7 @@ __device__ __forceinline__ void scale_q_chunk(uint32_t addr, float scale, int la
 // The 128 mask-column values (bf16) of one logits tile, four per lane.
 __device__ __forceinline__ void mask_values(const AttnParams& p, const Item& it, int kt, int s, int lane,
                                             uint16_t masked, uint16_t (&val)[4]) {
-  const uint8_t* mrow = p.mask != nullptr ? p.mask + (long long)stream_row(p, it, s) * p.mask_row_stride : nullptr;
+  const uint8_t* mrow = p.mask != nullptr ? p.mask + (long long)stream_row(it, s) * p.mask_row_stride : nullptr;
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     const int key = kt * kTile + 32 * g + lane;
@@ -384,7 +388,6 @@ __device__ __forceinline__ uint16_t masked_value_bits(const AttnParams& p, int h
 struct QScaler {
   uint32_t item = 0, chunk = 0;   // item index (per CTA) of the tiles being scaled, next piece
   int gv = 0, tile = 0;           // tiles that item has, next tile
-  QUses uses;
   __device__ __forceinline__ void start(uint32_t j, int n) { item = j; gv = n; tile = 0; chunk = 0; }
   __device__ __forceinline__ bool pending() const { return tile < gv; }
   // One piece.  block: wait (bounded) for the tile to land, else give up if it has not.
@@ -395,7 +398,7 @@ struct QScaler {
     const uint32_t buf = q_buf(p, item);
     const int slot = (int)buf * kMaxStreams + tile;
     if (chunk == 0) {
-      const uint32_t par = uses.parity(slot);
+      const uint32_t par = q_use(p, item) & 1;
       if (!__all_sync(0xffffffffu, mbar_test_wait(bar_addr(c, BarIdx::q_full + slot), par))) {
         if (!block) return 0;
         if (!wait_warp_slow(c, BarIdx::q_full + slot, par)) return -1;
@@ -406,7 +409,6 @@ struct QScaler {
       fence_proxy_async_smem();    // make the generic-proxy stores visible to the tensor core
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::q_scaled + slot));
-      uses.used(slot);
       chunk = 0;
       ++tile;
     }
@@ -520,7 +522,6 @@ __device__ void qk_issuer_role(const Ctx& c) {
   // ring positions / barrier parities are carried incrementally: no division on this warp
   uint32_t st = 0, kv_par = 0, icount = 0, bst = 0, b_par = 0;
   uint32_t sfree_par = 0, used = 0;   // bit b: parity of buffer b's next release; buffer b has held a tile
-  QUses q_uses;
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
     const Item it = decode_item(p, item);
@@ -532,7 +533,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
         const int b = s & 1;
         const int qslot = (int)q_buf(p, icount) * kMaxStreams + s;
         const int q_bar = (p.scale_q ? BarIdx::q_scaled : BarIdx::q_full) + qslot;
-        const bool need_bias = kTcBias && (s == 0 || p.q_split);
+        const bool need_bias = kTcBias && (s == 0 || it.split);
         const bool need_sfree = (used >> b) & 1u;
         const uint32_t sf_par = (sfree_par >> b) & 1u;
         {
@@ -540,15 +541,14 @@ __device__ void qk_issuer_role(const Ctx& c) {
           bool ok = mbar_test_wait(bar_addr(c, BarIdx::kv_full + st), kv_par);
           if (need_sfree) ok = mbar_test_wait(bar_addr(c, BarIdx::s_free + b), sf_par) && ok;
           if (need_bias) ok = mbar_test_wait(bar_addr(c, BarIdx::bias_full + bst), b_par) && ok;
-          if (kt == 0) ok = mbar_test_wait(bar_addr(c, q_bar), q_uses.parity(qslot)) && ok;
+          if (kt == 0) ok = mbar_test_wait(bar_addr(c, q_bar), q_use(p, icount) & 1) && ok;
           if (!__all_sync(0xffffffffu, ok)) {
             if (need_bias) AF3K_WAIT_WARP_C(c, BarIdx::bias_full + bst, b_par);
             // the softmax warpgroup of this buffer must have read the previous logits tile
             if (need_sfree) AF3K_WAIT_WARP_C(c, BarIdx::s_free + b, sf_par);
-            if (kt == 0) AF3K_WAIT_WARP_C(c, q_bar, q_uses.parity(qslot));
+            if (kt == 0) AF3K_WAIT_WARP_C(c, q_bar, q_use(p, icount) & 1);
             AF3K_WAIT_WARP_C(c, BarIdx::kv_full + st, kv_par);
           }
-          if (kt == 0) q_uses.used(qslot);
         }
         if (need_sfree) sfree_par ^= 1u << b;
         used |= 1u << b;
@@ -581,7 +581,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
         }
         __syncwarp();
         if (++st == nkv) { st = 0; kv_par ^= 1; }
-        if (kTcBias && (s == gv - 1 || p.q_split)) {
+        if (kTcBias && (s == gv - 1 || it.split)) {
           // every bias MMA that reads this stage is issued: the stage is free when they finish
           if (leader) tc_commit(bar_addr(c, BarIdx::bias_empty + bst));
           __syncwarp();
@@ -589,6 +589,14 @@ __device__ void qk_issuer_role(const Ctx& c) {
         }
       }
     }
+    // the slots that this item does not use: their scaling and their release (this warp is the one that waits for the
+    // former and, through the producer, for the latter, so neither can run ahead of it)
+    if (leader)
+      for (int s = gv; s < p.n_streams; ++s) {
+        mbar_arrive(bar_addr(c, BarIdx::q_scaled + (int)q_buf(p, icount) * kMaxStreams + s));
+        mbar_arrive(bar_addr(c, BarIdx::q_empty + (int)q_buf(p, icount) * kMaxStreams + s));
+      }
+    __syncwarp();
   }
 }
 
@@ -865,7 +873,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
   // position of tiles in the CTA-wide order (all streams): gives the K/V stage a tile used
   uint32_t kt_stage = 0, kt_round = 0;                // ring stage / lap of stream 0's tile at the current key tile
   uint32_t prev_stage = 0, prev_round = 0;            // the same for this warpgroup's last tile
-  uint32_t kt_tile = 0, prev_tile = 0;                // and the positions themselves
+  bool prev_pending = false;                          // its P V may not have finished
   uint32_t own_items = 0;                             // items in which this warpgroup had a stream
   const uint32_t nkv = p.kv_stages;
 
@@ -906,10 +914,6 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
         float* dbg = nullptr;
         if (kDebug && p.debug != nullptr && blockIdx.x == 0 && icount == 0 && s == 0 && kt == 0)
           dbg = p.debug + (size_t)row * kTile;
-        // a warpgroup that had no stream for a while: its previous P V has finished when a later tile took the K/V stage,
-        // and the stage's barrier, laps on, no longer tells
-        const uint32_t tile = kt_tile + (uint32_t)s;
-        const bool prev_pending = ucnt > 0 && tile - prev_tile < nkv;
         if (!softmax_tile<kTcBias>(c, dbg, wg, lane, s_taddr, p_taddr, o_taddr, p.nv, bias_row, row & 7, scale,
                                    kt == 0, prev_pending, BarIdx::kv_empty + (int)prev_stage, prev_round & 1, m_run,
                                    l_run, BarIdx::s_full + wg, (ucnt + 1) & 1, s_ready, ts))
@@ -919,7 +923,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
           // tiles are numbered in the producer's order; the numbers are carried without a division
           prev_stage = kt_stage + (uint32_t)s;
           prev_round = kt_round;
-          prev_tile = tile;
+          prev_pending = true;
           while (prev_stage >= nkv) { prev_stage -= nkv; ++prev_round; }
         }
         tc_fence_before();
@@ -932,7 +936,6 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
         if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::bias_empty + bst));
       }
       ++bcount;
-      kt_tile += (uint32_t)it.gv;
       kt_stage += (uint32_t)it.gv;
       while (kt_stage >= nkv) { kt_stage -= nkv; ++kt_round; }
     }
@@ -944,18 +947,21 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
     // (a barrier of its own, once per item with a stream: the K/V stage of its last tile may be taken again, by tiles of
     // the other warpgroup alone, before this one looks)
     if (wg < it.gv) { AF3K_WAIT_WARP(c, BarIdx::o_done + wg, own_items & 1); ++own_items; }
+    // Its last P V has finished: nothing is left to wait for in front of the next tile.  (The K/V stage's barrier could not
+    // tell a warpgroup that has no stream for a while: it moves on by laps.)
+    prev_pending = false;
     tc_fence_after();
     if (kDebug && last_ts != nullptr) last_ts[6] = clock64();
 #pragma unroll 1
     for (int s = wg; s < it.gv; s += 2) {
-      const int qrow = stream_qt(p, it, s) * kTile + row;
+      const int qrow = stream_qt(it, s) * kTile + row;
       const float inv = __frcp_rn(s == wg ? l_st[0] : l_st[1]);
       const uint32_t o_taddr = c.tmem + lane_sel + kOCol + s * p.nv;
-      __nv_bfloat16* orow = p.out + (long long)stream_row(p, it, s) * p.out_stride_b1 +
+      __nv_bfloat16* orow = p.out + (long long)stream_row(it, s) * p.out_stride_b1 +
                             (long long)it.h * p.out_stride_b2 + (long long)qrow * p.out_stride_s;
       const __nv_bfloat16* grow = nullptr;
       if constexpr (kGate)
-        grow = p.gate + (long long)stream_row(p, it, s) * p.gate_stride_b1 + (long long)it.h * p.gate_stride_b2 + (long long)qrow * p.gate_stride_s;
+        grow = p.gate + (long long)stream_row(it, s) * p.gate_stride_b1 + (long long)it.h * p.gate_stride_b2 + (long long)qrow * p.gate_stride_s;
 #pragma unroll 1
       for (int c0 = 0; c0 < p.nv; c0 += 16) {
         uint32_t o[16];

@@ -1,5 +1,5 @@
 """The attention kernel's forms at the sizes where they can go wrong: ragged last key tiles, references that rise late,
-items of different widths on one CTA.  Against the fp32 oracle with the
+smaller items behind the last full round, items of different widths on one CTA.  Against the fp32 oracle with the
 tolerances of the bf16 path; forms that only deal the same work out differently give the same bits."""
 import pytest
 import torch
@@ -72,6 +72,15 @@ def test_leading_keys_out_of_play(cuda_device, gone, how):
         bias[:, :, :gone] = torch.finfo(torch.bfloat16).min
     mask[1:, -1] = True
     _check(_call(cuda_device, q, k, v, mask, bias), O.oracle_fp32(q, k, v, mask, bias), (how, gone))
+
+
+@pytest.mark.parametrize("B1,B2,S,D", [(78, 8, 256, 16), (77, 8, 250, 32), (41, 4, 640, 32), (5, 16, 700, 48), (7, 16, 900, 64), (150, 1, 130, 8)])
+def test_smaller_items_behind_the_last_full_round(cuda_device, B1, B2, S, D):
+    q, k, v, mask, bias = _inputs(B1, B2, S, D, S + D)
+    out = _call(cuda_device, q, k, v, mask, bias)
+    assert torch.equal(_call(cuda_device, q, k, v, mask, bias, rows_per_item=1), out)
+    rows = [0, B1 // 2, B1 - 1]
+    _check(out[rows], O.oracle_fp32(q[rows], k[rows], v[rows], mask[rows], bias), (B1, B2, S, D))
 
 
 def test_items_of_one_and_two_query_tiles_on_one_cta(cuda_device):
