@@ -245,7 +245,12 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   p.qk_ksteps = (int)((d.D * es + 31) / 32);
   p.nv = (int)((d.D + 15) / 16 * 16);
   p.q_tile_bytes = kTile * p.qk_row_bytes;
-  p.k_tile_bytes = kTile * p.qk_row_bytes;
+  if (es == 2 && d.D > 32 && d.D <= 48) {
+    p.qk_narrow = 1;
+    p.qk_row_bytes = 64;
+    p.q_tile_bytes = kTile * (64 + 32);
+  }
+  p.k_tile_bytes = p.q_tile_bytes;
   p.v_tile_bytes = kTile * p.v_row_bytes;
   p.scale = d.softmax_scale;
 
@@ -355,7 +360,7 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
 }
 
 int encode_qkv_map(CUtensorMap* tm, const void* base, bool fp8, int64_t D, int64_t S, int64_t B2,
-                   int64_t B1, const int64_t* stride, int row_bytes) {
+                   int64_t B1, const int64_t* stride, int row_bytes) {   // row_bytes: of the box
   auto enc = tensor_map_encoder();
   if (!enc) return driver_fail("cuTensorMapEncodeTiled entry point", -1);
   const uint64_t es = fp8 ? 1 : 2;
@@ -573,6 +578,10 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
   if ((rc = encode_qkv_map(&tm_q, q, fp8, d.D, d.Sq, d.B2, d.B1, d.q_stride, p.qk_row_bytes))) return rc;
   if ((rc = encode_qkv_map(&tm_k, k, fp8, d.D, d.Sk, d.B2, d.B1, d.k_stride, p.qk_row_bytes))) return rc;
   if ((rc = encode_qkv_map(&tm_v, v, false, d.D, d.Sk, d.B2, d.B1, d.v_stride, p.v_row_bytes))) return rc;
+  CUtensorMap tm_q2{}, tm_k2{};
+  if (p.qk_narrow && ((rc = encode_qkv_map(&tm_q2, q, fp8, d.D, d.Sq, d.B2, d.B1, d.q_stride, 32)) ||
+                      (rc = encode_qkv_map(&tm_k2, k, fp8, d.D, d.Sk, d.B2, d.B1, d.k_stride, 32))))
+    return rc;
   if ((rc = encode_bias_map(&tm_b, bias_base, d.Sk, d.Sq, d.B2, bias_sh, bias_sr))) return rc;
 
   p.q_scale = q_scale;
@@ -597,7 +606,7 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
   const bool tc_bias = !fp8 || fp8_tc;
   p.scale_q = (fp8 || d.softmax_scale == 1.0f) ? 0 : 1;   // a scale of exactly 1 (q already scaled by its producer) needs no pass over Q
   const bool dbg = p.debug != nullptr;
-#define AF3K_LAUNCH(...) launch_overlapped(attention_kernel<__VA_ARGS__>, dim3(plan.grid), kThreads, plan.smem_bytes, stream, d.max_ctas <= 0, p, tm_q, tm_k, tm_v, tm_b)
+#define AF3K_LAUNCH(...) launch_overlapped(attention_kernel<__VA_ARGS__>, dim3(plan.grid), kThreads, plan.smem_bytes, stream, d.max_ctas <= 0, p, tm_q, tm_k, tm_v, tm_b, tm_q2, tm_k2)
   if (p.gate != nullptr) {
     if (!fp8)         AF3K_LAUNCH(false, true, false, true);
     else if (tc_bias) AF3K_LAUNCH(false, true, true, true);

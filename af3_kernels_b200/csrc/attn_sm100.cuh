@@ -64,6 +64,7 @@ constexpr float kLazyRescaleLog2 = 8.0f;   // keep a stale row max while exp2 ar
 constexpr int kBiasStages = 2;
 constexpr int kBiasTileBytes = kTile * kTile * 2;  // bf16, two 128B-swizzled boxes of 64 columns
 constexpr int kMaxKvStages = 6;
+constexpr uint32_t kNarrowOff = kTile * 64;        // qk_narrow: channels 32 .. 47 behind the first 32
 constexpr uint32_t kTmemCols = 512;
 // bf16 bit patterns of the mask column.  -2^47 stands in for the reference's "-1e9" fill: added
 // in fp32 to any logit below 2^23 in magnitude it gives exactly -2^47, so all masked keys of a
@@ -113,6 +114,11 @@ struct AttnParams {
   Divisor tail_div_q;
   Divisor div_q, div_h;  // query tiles (or pairs of them) per row and head, heads
   int qk_row_bytes;      // smem bytes per Q / K tile row: 32, 64 or 128 (= swizzle span)
+  // 1: bf16 heads of 33 to 48 channels.  A Q / K tile is 32 channels in rows of 64 bytes, then 16 in rows of 32 bytes: 12 KB
+  // instead of the 16 KB of 128-byte rows, which makes room for a fourth K/V stage beside two streams' Q tiles (three stages
+  // do not cover the loads' latency; 5 x 16 heads x 1536 tokens x 48 channels: 111.1 -> 99.6 us a call).  V keeps its
+  // 128-byte rows: it is an MN-major operand, whose columns one MMA reads in one swizzle.
+  int qk_narrow;
   int v_row_bytes;       // same for V
   int qk_ksteps;         // number of 32-byte K steps of the first GEMM
   int nv;                // N of the second GEMM: D rounded up to 16
@@ -281,7 +287,7 @@ __device__ __forceinline__ uint32_t q_use(const AttnParams& p, uint32_t j) { ret
 
 // ------------------------------------------------------------------ producer (one thread)
 __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUtensorMap* tm_k,
-                              const CUtensorMap* tm_v, const CUtensorMap* tm_bias) {
+                              const CUtensorMap* tm_v, const CUtensorMap* tm_bias, const CUtensorMap* tm_q2, const CUtensorMap* tm_k2) {
   const AttnParams& p = *c.p;
   uint32_t ucount = 0, bcount = 0, icount = 0;
   const uint32_t nkv = p.kv_stages;
@@ -300,8 +306,10 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
         continue;
       }
       mbar_arrive_expect_tx(bar_addr(c, BarIdx::q_full + slot), p.q_tile_bytes);
-      tma_load_4d(c.smem + p.off_q + (buf * p.n_streams + s) * p.q_tile_bytes, tm_q, bar_addr(c, BarIdx::q_full + slot),
-                  0, stream_qt(it, s) * kTile, it.h, stream_row(it, s));
+      const uint32_t qdst = c.smem + p.off_q + (buf * p.n_streams + s) * p.q_tile_bytes;
+      tma_load_4d(qdst, tm_q, bar_addr(c, BarIdx::q_full + slot), 0, stream_qt(it, s) * kTile, it.h, stream_row(it, s));
+      if (p.qk_narrow)
+        tma_load_4d(qdst + kNarrowOff, tm_q2, bar_addr(c, BarIdx::q_full + slot), 32, stream_qt(it, s) * kTile, it.h, stream_row(it, s));
     }
     return true;
   };
@@ -332,6 +340,7 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
         const uint32_t kdst = c.smem + p.off_kv + st * (p.k_tile_bytes + p.v_tile_bytes);
         mbar_arrive_expect_tx(full, p.k_tile_bytes + p.v_tile_bytes);
         tma_load_4d(kdst, tm_k, full, 0, kt * kTile, it.h, stream_row(it, s));
+        if (p.qk_narrow) tma_load_4d(kdst + kNarrowOff, tm_k2, full, 32, kt * kTile, it.h, stream_row(it, s));
         tma_load_4d(kdst + p.k_tile_bytes, tm_v, full, 0, kt * kTile, it.h, stream_row(it, s));
         ++ucount;
       }
@@ -496,7 +505,9 @@ __device__ void qk_issuer_role(const Ctx& c) {
   const uint64_t qd0 = make_smem_desc(c.smem + p.off_q, 16, 8 * p.qk_row_bytes, qk_layout);
   const uint64_t kd0 = make_smem_desc(c.smem + p.off_kv, 16, 8 * p.qk_row_bytes, qk_layout);
   const uint32_t qd_lo = (uint32_t)qd0, qd_hi = (uint32_t)(qd0 >> 32);
-  const uint32_t kd_lo = (uint32_t)kd0, kd_hi = (uint32_t)(kd0 >> 32);
+  const uint32_t kd_lo = (uint32_t)kd0;
+  const uint32_t narrow_hi = (uint32_t)(make_smem_desc(0, 16, 8 * 32, swizzle_layout_code(32)) >> 32);
+  const int wide_ksteps = p.qk_narrow ? 2 : p.qk_ksteps;
   const uint32_t q_step = p.q_tile_bytes >> 4, stage_step = kv_stage_bytes >> 4;
   const int ksteps = p.qk_ksteps;
   // extra K step: ones column x mask column, both K-major without swizzle (8-row groups 128 bytes
@@ -562,8 +573,11 @@ __device__ void qk_issuer_role(const Ctx& c) {
           const long long t0 = kDebug && tl != nullptr ? clock64() : 0;
 #pragma unroll 1
           for (int k = 0; k < ksteps; ++k) {     // one K step = 32 bytes of a tile row
-            if (fp8) mma_ss_f8(s_tmem, a_lo + 2 * k, qd_hi, b_lo + 2 * k, kd_hi, idesc_qk, k > 0 ? 1u : 0u);
-            else     mma_ss_f16(s_tmem, a_lo + 2 * k, qd_hi, b_lo + 2 * k, kd_hi, idesc_qk, k > 0 ? 1u : 0u);
+            // (Q and K tiles have one layout, so one high descriptor word)
+            const bool last16 = !fp8 && k >= wide_ksteps;
+            const uint32_t off = last16 ? kNarrowOff >> 4 : 2 * k, hi = last16 ? narrow_hi : qd_hi;
+            if (fp8) mma_ss_f8(s_tmem, a_lo + off, hi, b_lo + off, hi, idesc_qk, k > 0 ? 1u : 0u);
+            else     mma_ss_f16(s_tmem, a_lo + off, hi, b_lo + off, hi, idesc_qk, k > 0 ? 1u : 0u);
           }
           // mask column: start address and leading offset both move with the ring slot (the
           // zero block stays put)
@@ -1017,7 +1031,8 @@ template <bool kDebug, bool kTcBias, bool kFp8, bool kGate>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                 const __grid_constant__ CUtensorMap tm_bias) {
+                 const __grid_constant__ CUtensorMap tm_bias, const __grid_constant__ CUtensorMap tm_q2,
+                 const __grid_constant__ CUtensorMap tm_k2) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
@@ -1092,7 +1107,7 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     // warps 0-3 need few registers; the two softmax warpgroups take what they give up
     setmaxnreg_dec<kRegsMisc>();
     if (warp == 0) {
-      if (lane == 0) producer_role(c, &tm_q, &tm_k, &tm_v, &tm_bias);
+      if (lane == 0) producer_role(c, &tm_q, &tm_k, &tm_v, &tm_bias, &tm_q2, &tm_k2);
     } else if (warp == 1) {
       qk_issuer_role<kDebug, kTcBias, kFp8>(c);
     } else if (warp == 2) {

@@ -90,3 +90,12 @@ def test_items_of_one_and_two_query_tiles_on_one_cta(cuda_device):
     ref = O.oracle_fp32(q, k, v, mask, bias)
     for ctas in (9, 11, 13):
         _check(_call(cuda_device, q, k, v, mask, bias, max_ctas=ctas), ref, ctas)
+
+
+@pytest.mark.parametrize("D", [32, 40, 48, 56])
+@pytest.mark.parametrize("B1,B2,S", [(1, 2, 77), (5, 3, 300), (2, 16, 1100)])
+def test_heads_of_33_to_48_channels(cuda_device, B1, B2, S, D):
+    """Q and K tiles in two parts (40 and 48 channels) beside the widths around them, channels strided as in [B1, S, B2, D]."""
+    q, k, v, mask, bias = _inputs(B1, B2, S, D, S + D)
+    q, k = (t.transpose(1, 2).contiguous().transpose(1, 2) for t in (q, k))
+    _check(_call(cuda_device, q, k, v, mask, bias), O.oracle_fp32(q, k, v, mask, bias), (B1, B2, S, D))
