@@ -161,8 +161,7 @@ struct BarIdx {
   static constexpr int q_full = 12 + 2 * kMaxKvStages;       // [2 * kMaxStreams]  Q tile landed
   static constexpr int q_empty = q_full + 2 * kMaxStreams;   // [2 * kMaxStreams]  last Q K^T of the stream finished
   static constexpr int q_scaled = q_empty + 2 * kMaxStreams; // [2 * kMaxStreams]  the P V warp has scaled the Q tile
-  static constexpr int o_done = q_scaled + 2 * kMaxStreams;  // [2]  the item's last P V of the warpgroup finished
-  static constexpr int count = o_done + 2;
+  static constexpr int count = q_scaled + 2 * kMaxStreams;
 };
 static_assert(BarIdx::count * 8 <= (int)kBarrierBlockBytes, "barrier block too small");
 
@@ -617,12 +616,12 @@ __device__ void qk_issuer_role(const Ctx& c) {
 // O += P V for every tile, in order.  This warp mostly waits for the softmax warpgroups, so (bf16
 // q/k) it also scales the Q tiles: the first item's up front, the next item's in 1 KB pieces
 // while it waits, what is left when the item's last P V has been issued.
-template <bool kDebug, bool kTcBias>
+template <bool kDebug, bool kScalesQ>
 __device__ void pv_issuer_role(const Ctx& c, int lane) {
   const AttnParams& p = *c.p;
   const bool leader = elect_one();
   QScaler scaler;
-  if (kTcBias && p.scale_q && (int)blockIdx.x < p.n_items) {
+  if (kScalesQ && p.scale_q && (int)blockIdx.x < p.n_items) {
     scaler.start(0, decode_item(p, blockIdx.x).gv);
     while (scaler.pending())
       if (scaler.step(c, lane, true) < 0) return;
@@ -642,22 +641,33 @@ __device__ void pv_issuer_role(const Ctx& c, int lane) {
                       : nullptr;
   uint32_t tl_n = 0;
   uint32_t st = 0, icount = 0;
+  uint32_t epi_seen = 0, epi_par = 0;   // bit b: warpgroup b has had an item; parity of its last one's epilogue
   uint32_t pready_par = 0;         // bit b: of warpgroup b's next P
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
     const Item it = decode_item(p, item);
     const int gv = it.gv;
-    scaler.start(icount + 1, (kTcBias && p.scale_q && item + (int)gridDim.x < p.n_items) ? decode_item(p, item + gridDim.x).gv : 0);
+    scaler.start(icount + 1, (kScalesQ && p.scale_q && item + (int)gridDim.x < p.n_items) ? decode_item(p, item + gridDim.x).gv : 0);
 #pragma unroll 1
     for (int kt = 0; kt < p.n_kt; ++kt) {
 #pragma unroll 1
       for (int s = 0; s < gv; ++s) {
         const int b = s & 1;
-        AF3K_WAIT_WARP_OR_SCALE(c, BarIdx::p_ready + b, (pready_par >> b) & 1u, scaler, lane);
+        if (kScalesQ) AF3K_WAIT_WARP_OR_SCALE(c, BarIdx::p_ready + b, (pready_par >> b) & 1u, scaler, lane);
+        else          AF3K_WAIT_WARP_C(c, BarIdx::p_ready + b, (pready_par >> b) & 1u);
         pready_par ^= 1u << b;
         // the warpgroup's epilogue of the previous item must have read its O accumulators before
         // its first P V of this item overwrites one
-        if (kt == 0 && s < 2 && icount > 0) AF3K_WAIT_WARP_C(c, BarIdx::epi_done + b, (icount - 1) & 1);
+        if (kt == 0 && s < 2) {
+          if ((epi_seen >> b) & 1u) {
+            AF3K_WAIT_WARP_C(c, BarIdx::epi_done + b, (epi_par >> b) & 1u);
+            epi_par ^= 1u << b;
+          }
+          epi_seen |= 1u << b;
+          // an item of one stream: the other warpgroup must have finished its item before (it looks at the barrier of a K/V
+          // stage for that, which must not go through another lap meanwhile)
+          if (gv == 1 && epi_seen == 3u) AF3K_WAIT_WARP_C(c, BarIdx::epi_done + 1, epi_par >> 1);
+        }
         tc_fence_after();
         const uint32_t b_lo = vd_lo + st * stage_step;
         const uint32_t o_tmem = c.tmem + kOCol + s * p.nv;
@@ -670,14 +680,13 @@ __device__ void pv_issuer_role(const Ctx& c, int lane) {
             mma_ts_f16(o_tmem, p_tmem + k * 8, b_lo + k * v_kstep, vd_hi, idesc_pv, 1u);
           // one completion signal: the K/V stage is free, and so are this tile's P buffer and O
           tc_commit(bar_addr(c, BarIdx::kv_empty + st));
-          if (kt == p.n_kt - 1 && s + 2 >= gv) tc_commit(bar_addr(c, BarIdx::o_done + b));
           if (kDebug && tl != nullptr && tl_n + 2 <= 2 * kDbgTimelineTiles) { tl[tl_n++] = t0; tl[tl_n++] = clock64(); }
         }
         __syncwarp();
         if (++st == nkv) st = 0;
       }
     }
-    while (scaler.pending())
+    while (kScalesQ && scaler.pending())
       if (scaler.step(c, lane, true) < 0) return;
   }
 }
@@ -888,7 +897,6 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
   uint32_t kt_stage = 0, kt_round = 0;                // ring stage / lap of stream 0's tile at the current key tile
   uint32_t prev_stage = 0, prev_round = 0;            // the same for this warpgroup's last tile
   bool prev_pending = false;                          // its P V may not have finished
-  uint32_t own_items = 0;                             // items in which this warpgroup had a stream
   const uint32_t nkv = p.kv_stages;
 
 #pragma unroll 1
@@ -958,9 +966,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
     // ---- epilogue: O / l -> bf16 -> global, once this warpgroup's last P V has finished (the
     // other warpgroup may still be working on its own streams)
     if (kDebug && last_ts != nullptr) last_ts[5] = clock64();
-    // (a barrier of its own, once per item with a stream: the K/V stage of its last tile may be taken again, by tiles of
-    // the other warpgroup alone, before this one looks)
-    if (wg < it.gv) { AF3K_WAIT_WARP(c, BarIdx::o_done + wg, own_items & 1); ++own_items; }
+    if (wg < it.gv) AF3K_WAIT_WARP(c, BarIdx::kv_empty + (int)prev_stage, prev_round & 1);
     // Its last P V has finished: nothing is left to wait for in front of the next tile.  (The K/V stage's barrier could not
     // tell a warpgroup that has no stream for a while: it moves on by laps.)
     prev_pending = false;
@@ -1014,7 +1020,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
     }
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::epi_done + wg));
+    if (lane == 0 && wg < it.gv) mbar_arrive(bar_addr(c, BarIdx::epi_done + wg));   // (once per item with a stream of its own)
     if (kDebug && last_ts != nullptr) last_ts[7] = clock64();
   }
 }
@@ -1059,7 +1065,6 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar_addr(c, BarIdx::epi_done + i), 4);
-      mbar_init(bar_addr(c, BarIdx::o_done + i), 1);
       mbar_init(bar_addr(c, BarIdx::s_full + i), 1);
       mbar_init(bar_addr(c, BarIdx::s_free + i), 4);
       mbar_init(bar_addr(c, BarIdx::p_ready + i), 4);
@@ -1111,7 +1116,7 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     } else if (warp == 1) {
       qk_issuer_role<kDebug, kTcBias, kFp8>(c);
     } else if (warp == 2) {
-      pv_issuer_role<kDebug, kTcBias>(c, lane);
+      pv_issuer_role<kDebug, !kFp8>(c, lane);
     } else if (warp == 3) {
       if (p.mask_col) mask_writer_role(c, lane);
     }
