@@ -738,6 +738,17 @@ __device__ __forceinline__ void max_half(const uint32_t (&xr)[kTile], float& mxa
   }
 }
 
+// Weights are exp2(x * f + c), one fused multiply-add, with constants that go with the row's reference m: f = ef, the factor
+// from logits to exponents of 2, and c = -m * ef rounded.  The rounding leaves up to 2^-24 |m * ef| in every exponent of the
+// row, a factor that the division by their sum takes out again - as long as it is a number.  From |m * ef| = 2^31 on (biases
+// of -1e10, masked rows) it need not be: there f is a power of two, so that x * f + c is (x - m) * f exactly, 0 for x == m.
+// Other logits of that size are at least 2^31 / 2^24 of the exponent's units away and weigh nothing with either factor; half
+// of ef's power of two keeps m * f finite for any finite m.
+__device__ __forceinline__ void exponent_terms(float m, float ef, float& f, float& c) {
+  f = fabsf(m * ef) < 2147483648.0f ? ef : 0.5f * __uint_as_float(__float_as_uint(ef) & 0x7f800000u);
+  c = -m * f;
+}
+
 // One 128 x 128 logits tile of one stream; the thread owns row `row` (TMEM lane).
 // m_run is the reference maximum the running sums are scaled by (it may lag the true maximum by
 // up to kLazyRescaleLog2 bits), l_run the running sum of the fp32 weights.
@@ -789,24 +800,21 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, float* dbg, int wg, i
     m_use = mt;
   } else {
     need = (mt - m_run) * ef > kLazyRescaleLog2;
-    if (need) {
-      m_use = mt;
-      alpha = ex2_approx((m_run - mt) * ef);
-    }
+    if (need) m_use = mt;
   }
+  float f = ef, nml = 0.f;
+  if (kTcBias) exponent_terms(m_use, ef, f, nml);
   if (ts != nullptr) ts[3] = clock64();   // exponential pass starts
   // p = exp2((x - m) * log2e).  fp8 path: the subtraction comes first so that x == m gives
   // exactly 0 even for the huge negative values of masked keys (a row with no attended key: all
-  // weights 1).  bf16 path: one fused multiply-add, x * log2e - m * log2e; for such a row x and
-  // m are the same power of two, both products are exact and the result is 0 as well.
+  // weights 1).  bf16 path: one fused multiply-add (exponent_terms).
   // The pass is one ex2 per logit on the XU (a warp-wide ex2 every 8 cycles per scheduler, shared
   // by the scheduler's two softmax warps) with one packed FMA, one packed add and one bf16 pack per
   // pair of logits around it.  The two warpgroups run their passes in step (2 000 - 2 500 cycles per
   // pass against 2 048 for the XU alone); what keeps the kernel above that is the time between
   // passes, when both read logits, search the maximum and hand P over and the XU idles.
-  const uint64_t l2e2 = pack_f32x2(ef, ef);
+  const uint64_t l2e2 = pack_f32x2(f, f);
   const uint64_t nm2 = pack_f32x2(-m_use, -m_use);
-  const float nml = fminf(-m_use * ef, 3.0e38f);   // finite for bias entries of the type's lowest value: such keys weigh nothing
   const uint64_t nml2 = pack_f32x2(nml, nml);
   uint64_t suma = pack_f32x2(0.f, 0.f), sumb = suma;
   // The first kHeld column groups are computed before anything is written: the P buffer and the
@@ -845,6 +853,16 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, float* dbg, int wg, i
         tc_fence_after();
       }
       if (__any_sync(0xffffffffu, need)) {
+        if (need) {
+          if (kTcBias) {
+            // what a key at the old reference weighs under the new one, over what it was counted with
+            float f_run, nml_run;
+            exponent_terms(m_run, ef, f_run, nml_run);
+            alpha = ex2_approx(__fmaf_rn(m_run, f, nml) - __fmaf_rn(m_run, f_run, nml_run));
+          } else {
+            alpha = ex2_approx((m_run - mt) * ef);
+          }
+        }
 #pragma unroll 1
         for (int c0 = 0; c0 < nv; c0 += 16) {
           uint32_t o[16];

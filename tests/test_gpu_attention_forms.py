@@ -21,7 +21,7 @@ def _inputs(B1, B2, S, D, seed, Sk=None):
 
 
 def _call(dev, q, k, v, mask, bias, **kw):
-    return dot_product_attention(*(t.to(dev) for t in (q, k, v, mask, bias)), check_status=True, **kw).cpu()
+    return dot_product_attention(*(None if t is None else t.to(dev) for t in (q, k, v, mask, bias)), check_status=True, **kw).cpu()
 
 
 def _check(out, ref, what):
@@ -72,6 +72,71 @@ def test_leading_keys_out_of_play(cuda_device, gone, how):
         bias[:, :, :gone] = torch.finfo(torch.bfloat16).min
     mask[1:, -1] = True
     _check(_call(cuda_device, q, k, v, mask, bias), O.oracle_fp32(q, k, v, mask, bias), (how, gone))
+
+
+_LOWEST = torch.finfo(torch.bfloat16).min
+
+
+@pytest.mark.parametrize("route", ["scaled_q", "unscaled_q", "f32_bias", "fp8", "fp8_no_workspace"])
+@pytest.mark.parametrize("value", [-1e7, -1e9, -2e9, -1e10, -1e12, -1e15, -1e30, -2.2e38, _LOWEST])
+def test_keys_far_below_all_others(cuda_device, value, route):
+    """A bias far below every logit, down to the type's lowest value: on the first 1 to 300 keys it takes them out, on a
+    whole query row it leaves the softmax uniform.  (No mask: whether a masked key lies above such a bias is the caller's
+    choice of fill.)"""
+    B1, B2, S, D = 3, 2, 392, 32
+    if route == "fp8" and value < -1e38:
+        pytest.skip("divided by the logit scale such a bias leaves the type's range")
+    q, k, v, _, bias = _inputs(B1, B2, S, D, 7)
+    bias = bias.float()
+    for first, row in [(1, 3), (40, 10), (128, 11), (160, 150), (300, 260)]:
+        bias[:, row::23, :first] = value
+    bias[:, 5::7] = value                       # whole rows
+    scales, kw, scale = {}, {}, None
+    if route == "unscaled_q":
+        q, scale = q * D ** -0.5, 1.0           # the producer has applied the softmax scale
+    if route.startswith("fp8"):
+        (q, qs), (k, ks) = O.quantize_e4m3_per_head(q.float()), O.quantize_e4m3_per_head(k.float())
+        scales = {"q_scale": qs, "k_scale": ks}
+        kw = {"use_workspace": route == "fp8"}
+    if route != "f32_bias":
+        bias = bias.to(torch.bfloat16)
+    qf = (q.float() * qs.view(1, -1, 1, 1) if scales else q.float()).double() * (D ** -0.5 if scale is None else scale)
+    kf = (k.float() * ks.view(1, -1, 1, 1) if scales else k.float()).double()
+    # the logits as fp32 holds them: next to 1e9 products of q and k are below half of the last bit
+    logits = (qf @ kf.transpose(-1, -2) + bias.double()).float().double()
+    ref = torch.softmax(logits, -1) @ v.double()
+    out = _call(cuda_device, q, k, v, None, bias, softmax_scale=scale, **{n: t.to(cuda_device) for n, t in scales.items()}, **kw)
+    assert torch.isfinite(out.float()).all(), (route, value, torch.isfinite(out.float()).all(-1).sum())
+    # rows that keep an ordinary key, and rows that have none above the value.  At 1e7 fp32's last bit is 1, so a row's logits there
+    # are rounded to whole numbers, by the oracle in one step and by the kernel in several: such rows are compared from 1e9 on.
+    whole = torch.arange(S) % 7 == 5
+    limit = (6e-2, 6e-3) if scales else (2e-2, 2e-3)
+    for rows in [~whole] + ([whole] if abs(value) >= 1e9 else []):
+        st = O.error_stats(out[:, :, rows], ref[:, :, rows].float())
+        assert st["max_abs"] <= limit[0] and st["mean_abs"] <= limit[1], (route, value, st)
+
+
+@pytest.mark.parametrize("value", [0, -38 * 2 ** 12, -152 * 2 ** 14, -152 * 2 ** 16, 152 * 2 ** 16])
+def test_reference_rises_under_a_large_bias(cuda_device, value):
+    """Logits of 1e7 that differ by a few units, all whole numbers that fp32 holds exactly: what earlier key tiles summed
+    up is brought to the later reference without the rounding of the one or the other (half a unit of the exponent here)."""
+    B1, B2, S, D = 2, 3, 500, 32
+    g = torch.Generator().manual_seed(11)
+    k = torch.zeros(B1, B2, S, D)
+    k[..., 0] = torch.randint(-60, -40, (B1, B2, S), generator=g).float()
+    k[:, :, :128, 0] = 0                                  # 128 keys of weight e^-6 .. e^-9, then one of weight 1
+    for n, step in enumerate((6, 7, 9)):
+        k[:, n, 200 + 100 * n, 0] = step
+    q = torch.zeros(B1, B2, S, D)
+    q[..., 0] = 1
+    v = torch.randn(B1, B2, S, D, generator=g).to(torch.bfloat16)
+    v[:, :, :128] += 2
+    bias = torch.full((B2, S, S), float(value)) - torch.randint(0, 2, (B2, S, 1), generator=g) * 2.0 ** 16
+    q, k, bias = (t.to(torch.bfloat16) for t in (q, k, bias))
+    logits = q.double() @ k.double().transpose(-1, -2) + bias.double()
+    assert torch.equal(logits.float().double(), logits)
+    ref = torch.softmax(logits, -1) @ v.double()
+    _check(_call(cuda_device, q, k, v, None, bias, softmax_scale=1.0), ref.float(), value)
 
 
 @pytest.mark.parametrize("B1,B2,S,D", [(78, 8, 256, 16), (77, 8, 250, 32), (41, 4, 640, 32), (5, 16, 700, 48), (7, 16, 900, 64), (150, 1, 130, 8)])
