@@ -1161,6 +1161,14 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
 // With fp8 q/k (q_scale / k_scale given) every value is divided by the head's logit scale
 // softmax_scale * q_scale[h] * k_scale[h]: the tensor core then adds it to the raw fp8 products
 // and the softmax threads apply that scale to the sum.
+// What bf16 cannot hold (fp32's lowest value, a quotient, -inf) becomes bf16's largest value of its sign: the tensor core
+// adds a slice of the bias by products with 1 and 0, and an infinity times 0 would make NaN of the 15 keys beside it.
+// +inf and NaN stay, as the softmax of such a row is not a number either.
+__device__ __forceinline__ float staged_value(float b, float mul) {
+  const float x = b * mul;
+  return b < INFINITY ? fminf(fmaxf(x, -3.38953139e38f), 3.38953139e38f) : x;
+}
+
 template <typename T>
 __global__ void bias_to_bf16_kernel(const T* __restrict__ src, __nv_bfloat16* __restrict__ dst,
                                     int B2, int Sq, int Sk, long long src_stride_h,
@@ -1176,8 +1184,8 @@ __global__ void bias_to_bf16_kernel(const T* __restrict__ src, __nv_bfloat16* __
     const T* s = src + h * src_stride_h + r * src_stride_r;
     const float mul = q_scale != nullptr ? 1.0f / (softmax_scale * q_scale[h] * k_scale[h]) : 1.0f;
     const int col = cp * 2;
-    const float a = col < Sk ? (float)s[col] * mul : 0.f;
-    const float b = col + 1 < Sk ? (float)s[col + 1] * mul : 0.f;
+    const float a = col < Sk ? staged_value((float)s[col], mul) : 0.f;
+    const float b = col + 1 < Sk ? staged_value((float)s[col + 1], mul) : 0.f;
     reinterpret_cast<uint32_t*>(dst)[i] = pack_bf16x2(a, b);
   }
 }

@@ -78,14 +78,14 @@ _LOWEST = torch.finfo(torch.bfloat16).min
 
 
 @pytest.mark.parametrize("route", ["scaled_q", "unscaled_q", "f32_bias", "fp8", "fp8_no_workspace"])
-@pytest.mark.parametrize("value", [-1e7, -1e9, -2e9, -1e10, -1e12, -1e15, -1e30, -2.2e38, _LOWEST])
+@pytest.mark.parametrize("value", [-1e7, -1e9, -2e9, -1e10, -1e12, -1e15, -1e30, -2.2e38, _LOWEST, torch.finfo(torch.float32).min])
 def test_keys_far_below_all_others(cuda_device, value, route):
     """A bias far below every logit, down to the type's lowest value: on the first 1 to 300 keys it takes them out, on a
     whole query row it leaves the softmax uniform.  (No mask: whether a masked key lies above such a bias is the caller's
     choice of fill.)"""
     B1, B2, S, D = 3, 2, 392, 32
-    if route == "fp8" and value < -1e38:
-        pytest.skip("divided by the logit scale such a bias leaves the type's range")
+    if route != "f32_bias":
+        value = max(value, _LOWEST)
     q, k, v, _, bias = _inputs(B1, B2, S, D, 7)
     bias = bias.float()
     for first, row in [(1, 3), (40, 10), (128, 11), (160, 150), (300, 260)]:
@@ -114,6 +114,24 @@ def test_keys_far_below_all_others(cuda_device, value, route):
     for rows in [~whole] + ([whole] if abs(value) >= 1e9 else []):
         st = O.error_stats(out[:, :, rows], ref[:, :, rows].float())
         assert st["max_abs"] <= limit[0] and st["mean_abs"] <= limit[1], (route, value, st)
+
+
+@pytest.mark.parametrize("dtype,Sk", [(torch.float32, 392), (torch.bfloat16, 389)])
+def test_minus_infinity_in_a_bias_that_is_converted(cuda_device, dtype, Sk):
+    """fp32 or ragged rows: keys with a bias of -inf have no weight, the keys beside them keep theirs; +inf and NaN still
+    make their row NaN and no other."""
+    q, k, v, mask, bias = _inputs(3, 2, 200, 32, 8, Sk)
+    bias = bias.to(dtype)
+    g = torch.Generator().manual_seed(3)
+    bias[torch.rand(bias.shape, generator=g) < 0.2] = -float("inf")
+    bias[:, 7, :140] = -float("inf")
+    mask[:, -1], bias[..., -1] = True, 0
+    ref = O.oracle_fp32(q, k, v, mask, bias)
+    _check(_call(cuda_device, q, k, v, mask, bias), ref, "-inf")
+    for n, value in enumerate((float("inf"), float("nan"))):
+        bias[:, 20 + n, Sk - 1] = value
+    nan = torch.isnan(_call(cuda_device, q, k, v, mask, bias)).all(-1).all(0).all(0)
+    assert nan.nonzero().flatten().tolist() == [20, 21]
 
 
 @pytest.mark.parametrize("value", [0, -38 * 2 ** 12, -152 * 2 ** 14, -152 * 2 ** 16, 152 * 2 ** 16])
