@@ -11,7 +11,7 @@ import torch.distributed as dist
 import torch.nn as nn
 
 from . import _capi, pair_bias
-from .dpa import bool_mask
+from .dpa import bool_mask, readable_bias
 from .fused_ops import attention_block, differentiates
 from .tools import profile
 
@@ -102,7 +102,7 @@ class DistributedGridSelfAttentionCpp(GridSelfAttentionCpp):
         local_mask = mask[rows]
 
         pair, bias = self._norm_and_bias(pair)
-        bias = bias.contiguous()
+        bias = readable_bias(bias, self.num_head, seq_len, seq_len)        # once for all pieces
         if self.transpose:
             pair = pair.permute(1, 0, 2)
         chunk = pair[rows]

@@ -63,21 +63,22 @@ def dot_product_attention_cpp(
     ``use_flash_attention``, ``BLK_SZ`` and ``FLASH_SZ`` are accepted and checked but do not
     select code: the CUDA kernel always runs an online softmax over 128-key tiles.  Unlike the
     reference the call never writes to ``q`` and a 1-D mask broadcasts over the batch.
-    ``q_scale`` / ``k_scale`` (keyword-only) enable float8_e4m3fn q and k.  CUDA tensors are
+    ``q_scale`` / ``k_scale`` (keyword-only) enable float8_e4m3fn q and k.  Nothing is kept between calls: a bias that is
+    converted (fp32, rows that are not 16-byte multiples, fp8 q and k) is converted in each; ``stage_bias`` and
+    ``dot_product_attention`` are for a bias applied many times.  CUDA tensors are
     computed in place on their device; host tensors (what the reference takes) go through
     ``dot_product_attention_host`` and come back as a host tensor.
     """
     if int(BLK_SZ) <= 0 or int(FLASH_SZ) <= 0:
         raise ValueError("BLK_SZ and FLASH_SZ must be positive")
     if q.is_cuda and (mask is None or (mask.dtype is torch.bool and 0 < mask.dim() < 3)) and isinstance(bias, torch.Tensor) and not _DEBUG:
-        # the ordinary call, straight to the native path: what dot_product_attention would hand it with its defaults
-        # (77 tokens: 7.7 us a call through it)
-        return _capi.host().attention(q, k, v, mask, bias, q_scale, k_scale, None, 0, None, True, True, 0, 0)
+        # the ordinary call, straight to the native path, as below
+        return _capi.host().attention(q, k, v, mask, bias, q_scale, k_scale, None, 0, None, True, False, 0, 0)
     if not q.is_cuda:
         # host tensors, as the reference takes them: pipelined over PCIe, computed on the GPU,
         # result in host memory
         return dot_product_attention_host(q, k, v, mask, bias, q_scale=q_scale, k_scale=k_scale)
-    return dot_product_attention(q, k, v, mask, bias, q_scale=q_scale, k_scale=k_scale)
+    return dot_product_attention(q, k, v, mask, bias, q_scale=q_scale, k_scale=k_scale, cache_bias=False)
 
 
 def _not_built(name: str):

@@ -88,6 +88,8 @@ Tensor status_buffer(int64_t device) {
 // not before it was divided by each head's logit scale, is converted once; the copy is used again
 // while the very same tensor object is alive and unmodified (its version counter) and, for fp8, the
 // scales are the same.  Four copies are kept; copies of dead tensors are dropped when another is made.
+// Only for dot_product_attention(cache_bias=True): a write that bumps no counter (.data, a collective) is missed, so the
+// entry points with the reference's signatures and the blocks convert in every call.
 // A stream that is being captured never gets one of them: the graph would go on reading the copy after the
 // list gave it up, and would not see a later write to the bias.  It converts inside the graph.
 struct TensorId {
@@ -453,7 +455,7 @@ Tensor grid_block(const Tensor& pair, const OptTensor& mask, const Tensor& bias,
   int* status = status_buffer(dev.index()).data_ptr<int>();
   check(g_lib.grid_front(x.data_ptr(), AF3K_BF16, &w.front, 0.f, 0, R, N, C, head, 1.0f / std::sqrt((float)D), 0, nullptr, 0, q.data_ptr(),
                          k.data_ptr(), v.data_ptr(), gate.data_ptr(), status, stream));
-  attention(q, k, v, mask, bias, std::nullopt, std::nullopt, 1.0, 0, weighted.permute({0, 2, 1, 3}), true, true, 0, 0);
+  attention(q, k, v, mask, bias, std::nullopt, std::nullopt, 1.0, 0, weighted.permute({0, 2, 1, 3}), true, false, 0, 0);
   if (!project) check(g_lib.sigmoid_gate(weighted.data_ptr(), gate.data_ptr(), out.data_ptr(), M * C, stream));
   else check(g_lib.grid_out(weighted.data_ptr(), gate.data_ptr(), w.wo, w.front.w_dtype, out.data_ptr(), pair.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16,
                        M, C, status, stream));
@@ -499,7 +501,7 @@ Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, con
   const bool in_place = bias.scalar_type() == at::kBFloat16 && bias.dim() == 3 && bias.size(0) == head && bias.size(1) == N && bias.stride(2) == 1 && (bias.stride(1) * 2) % 16 == 0 &&
                         (bias.stride(0) * 2) % 16 == 0 && (bias.stride(0) != 0 || head == 1) && (bias.stride(1) != 0 || N == 1) &&
                         reinterpret_cast<uintptr_t>(bias.data_ptr()) % 16 == 0;
-  if (!in_place) bias = staged_bias(bias, head, N, N, D, std::nullopt, std::nullopt, nullptr, nullptr, scale);
+  if (!in_place) bias = make_staged(bias, head, N, N, D, nullptr, nullptr, scale, stream);
   Tensor mask;
   if (mask_in) {
     if (mask_in->numel() != N) value_error("mask of shape " + shape_text(*mask_in) + " does not match B1=1, Sk=" + std::to_string(N));

@@ -11,6 +11,7 @@ queue around ``dist.all_gather``, Attention.py:162-195).
 """
 from __future__ import annotations
 
+import functools
 import time
 from typing import Callable, Optional, Tuple
 
@@ -65,7 +66,8 @@ class RowShardedAttention:
         # the CUDA operator writes into a caller-provided ``out``; a stand-in (CPU tests) returns its result
         self.writes_in_place = attention_fn is None
         if attention_fn is None:
-            from .dpa import dot_product_attention as attention_fn
+            from .dpa import dot_product_attention
+            attention_fn = functools.partial(dot_product_attention, cache_bias=False)
         self.attention_fn = attention_fn
         self._comm_stream = None
 
@@ -85,7 +87,7 @@ class RowShardedAttention:
         if mask is not None:
             m = mask.view(torch.uint8) if mask.dtype == torch.bool else mask
             dist.broadcast(m, src=src, group=self.group)
-        # a collective bumps no version counter, and the operator finds its staged copy of a bias by it
+        # a collective bumps no version counter, and dot_product_attention finds its staged copy of a bias by it
         if not bias.is_inference():
             torch.autograd.graph.increment_version(bias)
         return bias, mask
@@ -140,6 +142,9 @@ class RowShardedAttention:
             raise ValueError(f"rank {rank} expected {local_rows} local rows, got {q.shape[0]}")
         _, H, N, D = q.shape
         out_dtype = torch.bfloat16 if q.is_cuda else q.dtype
+        if self.writes_in_place:
+            from .dpa import readable_bias
+            bias = readable_bias(bias, H, N, k.shape[2] if k.dim() == 4 else N)        # once for all pieces
 
         def compute(lo, hi, slot, kw):
             m = None

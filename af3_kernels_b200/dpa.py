@@ -63,6 +63,15 @@ def stage_bias(bias: torch.Tensor, B2: int, Sq: int, Sk: int, *, q_scale=None, k
     return StagedBias(staged, B2, Sq, Sk, fp8)
 
 
+def readable_bias(bias: torch.Tensor, B2: int, Sq: int, Sk: int) -> torch.Tensor:
+    """``bias`` itself where the kernel reads it in place with bf16 q/k, else a bf16 copy ``[B2, Sq, Sk]`` made now that it
+    can read: for several calls of one step on the same bias."""
+    if (bias.dtype == torch.bfloat16 and bias.shape == (B2, Sq, Sk) and bias.stride(2) == 1 and bias.stride(1) % 8 == 0
+            and bias.stride(0) % 8 == 0 and 0 not in bias.stride() and bias.data_ptr() % 16 == 0):
+        return bias
+    return bias if bias.numel() == 0 or not bias.is_cuda else stage_bias(bias, B2, Sq, Sk).data[:, :, :Sk]
+
+
 def _mask_rows(mask: Optional[torch.Tensor], B1: int, Sk: int):
     """-> (uint8 tensor [rows, Sk] with unit inner stride, row stride in bytes) or (None, 0).
 

@@ -141,7 +141,7 @@ def attention_block(
     k = torch.matmul(x, _as_bf16(k_proj)).view(R, N, head, D).permute(0, 2, 1, 3)
     v = torch.matmul(x, _as_bf16(v_proj)).view(R, N, head, D).permute(0, 2, 1, 3)
     weighted = torch.empty((R, N, head, D), dtype=torch.bfloat16, device=pair.device)
-    dot_product_attention(q, k, v, mask, bias, out=weighted.permute(0, 2, 1, 3))
+    dot_product_attention(q, k, v, mask, bias, out=weighted.permute(0, 2, 1, 3), cache_bias=False)
     gated = sigmoid_gate(weighted.view(R, N, C), torch.matmul(x, _as_bf16(gating_query)))
     return torch.matmul(gated, _as_bf16(out_proj)).to(pair.dtype)
 
@@ -176,5 +176,5 @@ def self_attention_block(
     k = torch.matmul(xb, _as_bf16(k_proj)).view(1, N, head, D).permute(0, 2, 1, 3)
     v = torch.matmul(xb, _as_bf16(v_proj)).view(1, N, head, D).permute(0, 2, 1, 3)
     weighted = torch.empty((1, N, head, D), dtype=torch.bfloat16, device=x.device)
-    dot_product_attention(q, k, v, m, bias, out=weighted.permute(0, 2, 1, 3))
+    dot_product_attention(q, k, v, m, bias, out=weighted.permute(0, 2, 1, 3), cache_bias=False)
     return sigmoid_gate(weighted.view(N, C), torch.matmul(xb, _as_bf16(gating_query))).to(x.dtype)

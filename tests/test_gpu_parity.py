@@ -356,6 +356,44 @@ def test_staged_bias_is_reused_and_follows_in_place_updates(cuda_device):
     assert lib.af3k_last_launch_count() == 1
 
 
+def test_ordinary_calls_see_every_write_to_the_bias(cuda_device):
+    """The reference's signatures keep no copy of a bias or of fp8 scales: a write that bumps no version counter
+    (``.data``, as a collective or a kernel on the raw pointer) shows in the next call of the operator and of the blocks."""
+    g = torch.Generator().manual_seed(9)
+    dev = cuda_device
+    B1, B2, S, D = 3, 4, 200, 32
+    C = B2 * D
+    q, k, v = (torch.randn(B1, B2, S, D, generator=g).to(torch.bfloat16).to(dev) for _ in range(3))
+    mask = (torch.rand(B1, S, generator=g) >= 0.1).to(dev)
+    w = [(torch.randn(C, C, generator=g) * C ** -0.5).to(torch.bfloat16).to(dev) for _ in range(5)]
+    wide = [(torch.randn(96, 96, generator=g) * 0.1).to(torch.bfloat16).to(dev) for _ in range(5)]     # not a fused size
+    x, pair, other = (torch.randn(*s, generator=g).to(torch.bfloat16).to(dev) for s in ((S, C), (B1, S, C), (B1, S, 96)))
+    q8, qs = O.quantize_e4m3_per_head(q.float().cpu())
+    k8, ks = O.quantize_e4m3_per_head(k.float().cpu())
+    q8, k8, qs, ks = q8.to(dev), k8.to(dev), qs.to(dev), ks.to(dev)
+    calls = {
+        "operator": lambda b: A.dot_product_attention_cpp(q, k, v, mask, b),
+        "operator, byte mask": lambda b: A.dot_product_attention_cpp(q, k, v, mask.to(torch.uint8), b),
+        "operator, fp8": lambda b: A.dot_product_attention_cpp(q8, k8, v, mask, b, q_scale=qs, k_scale=ks),
+        "grid block": lambda b: A._attention_cpp(pair, mask, b, *w, B2),
+        "grid block, torch projections": lambda b: A._attention_cpp(other, mask, b, *wide, B2),
+        "single block": lambda b: A.self_attention_cpp(x, mask[0], b, w[0], torch.zeros(C, device=dev), *w[1:4], B2),
+        "single block, torch projections": lambda b: A.self_attention_cpp(x[:, :96], mask[0], b, wide[0], torch.zeros(96, device=dev), *wide[1:4], B2),
+    }
+    for name, call in calls.items():
+        bias, new = (torch.randn(B2, S, S, generator=g).to(dev) for _ in range(2))
+        first = call(bias)
+        assert torch.equal(call(bias), first), name
+        bias.data.copy_(new)
+        assert torch.equal(call(bias), call(new.clone())), name
+        assert not torch.equal(call(bias), first), name
+    bias = torch.randn(B2, S, S, generator=g).to(dev)
+    first = calls["operator, fp8"](bias)
+    qs.data.mul_(0.5)
+    assert torch.equal(calls["operator, fp8"](bias), calls["operator, fp8"](bias.clone()))
+    assert not torch.equal(calls["operator, fp8"](bias), first)
+
+
 def test_debug_dump_shows_the_tensor_core_stages(cuda_device):
     """The diagnostic build dumps the first logits tile: the logits as the tensor core delivers them
     (scaled Q K^T + bias + mask column), P as written to TMEM, the un-normalised accumulator and
