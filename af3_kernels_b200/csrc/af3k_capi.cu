@@ -480,17 +480,15 @@ namespace {
 int launch_bias_staging(const af3k_attention_desc& d, const DeviceInfo& dev, const void* bias, const float* sq,
                         const float* sk, void* staged, cudaStream_t stream) {
   const int64_t pitch = staged_bias_pitch(d.Sk);
-  const long long total = (long long)d.B2 * d.Sq * (pitch / 2);
-  int blocks = (int)((total + 255) / 256);
-  if (blocks > dev.sm_count * 16) blocks = dev.sm_count * 16;
-  if (d.bias_dtype == AF3K_F32)
-    bias_to_bf16_kernel<float><<<blocks, 256, 0, stream>>>(
-        static_cast<const float*>(bias), static_cast<__nv_bfloat16*>(staged), (int)d.B2, (int)d.Sq,
-        (int)d.Sk, d.bias_stride[0], d.bias_stride[1], (int)pitch, sq, sk, d.softmax_scale);
-  else
-    bias_to_bf16_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(bias), static_cast<__nv_bfloat16*>(staged), (int)d.B2,
-        (int)d.Sq, (int)d.Sk, d.bias_stride[0], d.bias_stride[1], (int)pitch, sq, sk, d.softmax_scale);
+  const long long total = (long long)d.B2 * d.Sq * (pitch / 8);
+  long long blocks = (total + kBiasThreads - 1) / kBiasThreads;
+  if (blocks > dev.sm_count * 8) blocks = dev.sm_count * 8;
+  const auto launch = [&](auto kernel, auto* src) {
+    launch_overlapped(kernel, dim3((unsigned)blocks), kBiasThreads, 0, stream, d.max_ctas <= 0, src, static_cast<__nv_bfloat16*>(staged), (int)d.B2,
+                      (int)d.Sq, (int)d.Sk, (long long)d.bias_stride[0], (long long)d.bias_stride[1], (int)pitch, sq, sk, d.softmax_scale);
+  };
+  if (d.bias_dtype == AF3K_F32) launch(bias_to_bf16_kernel<float>, static_cast<const float*>(bias));
+  else                          launch(bias_to_bf16_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(bias));
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? AF3K_OK : cuda_fail("launch bias_to_bf16_kernel", e);
 }

@@ -1169,24 +1169,49 @@ __device__ __forceinline__ float staged_value(float b, float mul) {
   return b < INFINITY ? fminf(fmaxf(x, -3.38953139e38f), 3.38953139e38f) : x;
 }
 
+// One thread converts eight columns, two 16-byte loads where every row starts on a 16-byte boundary (else one by one) and one
+// 16-byte store, as many blocks as stay resident: it is bound by memory, and a call that converts pays it in full.
+// Two columns a thread, with two 64-bit divisions for each pair, against this, us: 16 heads of 512 x 512 fp32 11.3 -> 4.9 (5.2
+// TB/s), of 1536 x 1536 76.2 -> 35.2 (6.4 TB/s), 4 heads of 768 x 768 6.9 -> 3.0, of 2048 x 2048 bf16 with scales 40.9 -> 14.0.
+constexpr int kBiasThreads = 256;
 template <typename T>
-__global__ void bias_to_bf16_kernel(const T* __restrict__ src, __nv_bfloat16* __restrict__ dst,
-                                    int B2, int Sq, int Sk, long long src_stride_h,
-                                    long long src_stride_r, int pitch, const float* __restrict__ q_scale,
-                                    const float* __restrict__ k_scale, float softmax_scale) {
-  const long long total = (long long)B2 * Sq * (pitch / 2);
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int cp = (int)(i % (pitch / 2));
-    const long long t = i / (pitch / 2);
-    const int r = (int)(t % Sq);
-    const int h = (int)(t / Sq);
-    const T* s = src + h * src_stride_h + r * src_stride_r;
+__global__ void __launch_bounds__(kBiasThreads, 8)
+bias_to_bf16_kernel(const T* __restrict__ src, __nv_bfloat16* __restrict__ dst, int B2, int Sq, int Sk, long long src_stride_h,
+                    long long src_stride_r, int pitch, const float* __restrict__ q_scale, const float* __restrict__ k_scale,
+                    float softmax_scale) {
+  grid_wait_previous();
+  grid_release_next();
+  const uint32_t chunks = (uint32_t)pitch / 8;
+  const long long total = (long long)B2 * Sq * chunks;
+  const bool wide = ((reinterpret_cast<uintptr_t>(src) | (uintptr_t)(src_stride_h * sizeof(T)) | (uintptr_t)(src_stride_r * sizeof(T))) & 15u) == 0;
+  for (long long i = (long long)blockIdx.x * kBiasThreads + threadIdx.x; i < total; i += (long long)gridDim.x * kBiasThreads) {
+    long long t;             // row among all heads'
+    if (total <= 0x7fffffff) t = (uint32_t)i / chunks; else t = i / chunks;
+    const int col = (int)(i - t * chunks) * 8;
+    int h, r;
+    if (t <= 0x7fffffff) { h = (int)((uint32_t)t / (uint32_t)Sq); r = (int)((uint32_t)t % (uint32_t)Sq); }
+    else                 { h = (int)(t / Sq); r = (int)(t % Sq); }
+    const T* s = src + h * src_stride_h + r * src_stride_r + col;
+    float x[8];
+    if (wide && col + 8 <= Sk) {
+      if constexpr (sizeof(T) == 4) {
+        const float4 a = *reinterpret_cast<const float4*>(s), b = *reinterpret_cast<const float4*>(s + 4);
+        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+      } else {
+        const uint4 a = *reinterpret_cast<const uint4*>(s);
+        const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = __uint_as_float((e & 1) ? w[e >> 1] & 0xffff0000u : w[e >> 1] << 16);
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = col + e < Sk ? (float)s[e] : 0.f;
+    }
     const float mul = q_scale != nullptr ? 1.0f / (softmax_scale * q_scale[h] * k_scale[h]) : 1.0f;
-    const int col = cp * 2;
-    const float a = col < Sk ? staged_value((float)s[col], mul) : 0.f;
-    const float b = col + 1 < Sk ? staged_value((float)s[col + 1], mul) : 0.f;
-    reinterpret_cast<uint32_t*>(dst)[i] = pack_bf16x2(a, b);
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[e] = pack_bf16x2(staged_value(x[2 * e], mul), staged_value(x[2 * e + 1], mul));
+    reinterpret_cast<uint4*>(dst)[i] = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 

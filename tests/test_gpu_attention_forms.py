@@ -4,7 +4,7 @@ tolerances of the bf16 path; forms that only deal the same work out differently 
 import pytest
 import torch
 
-from af3_kernels_b200.dpa import dot_product_attention
+from af3_kernels_b200.dpa import dot_product_attention, stage_bias
 from oracle import attention_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -114,6 +114,22 @@ def test_keys_far_below_all_others(cuda_device, value, route):
     for rows in [~whole] + ([whole] if abs(value) >= 1e9 else []):
         st = O.error_stats(out[:, :, rows], ref[:, :, rows].float())
         assert st["max_abs"] <= limit[0] and st["mean_abs"] <= limit[1], (route, value, st)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("Sk,pitch,offset", [(1, 1, 0), (7, 8, 0), (8, 8, 0), (9, 16, 0), (9, 9, 0), (64, 72, 3), (77, 80, 0), (77, 84, 4), (129, 136, 8)])
+def test_conversion_of_the_bias(cuda_device, Sk, pitch, offset, dtype):
+    """Eight columns a thread: rows that do and do not start on 16-byte boundaries, last columns of every remainder.  The
+    same bits as torch's conversion, zeros in the padding; with fp8 scales the quotient is taken first."""
+    B2, Sq = 3, 37
+    g = torch.Generator().manual_seed(Sk)
+    buf = torch.randn(B2 * Sq * pitch + 16, generator=g).to(cuda_device, dtype)
+    bias = buf[offset:offset + B2 * Sq * pitch].view(B2, Sq, pitch)[:, :, :Sk]
+    scales = (torch.rand(2, B2, generator=g) + 0.5).to(cuda_device)
+    plain, scaled = stage_bias(bias, B2, Sq, Sk).data, stage_bias(bias, B2, Sq, Sk, q_scale=scales[0], k_scale=scales[1], softmax_scale=0.25).data
+    factor = (1.0 / (0.25 * scales[0] * scales[1])).view(B2, 1, 1)
+    for got, want in [(plain, bias.float()), (scaled, bias.float() * factor)]:
+        assert torch.equal(got[:, :, :Sk], want.to(torch.bfloat16)) and not got[:, :, Sk:].any()
 
 
 @pytest.mark.parametrize("dtype,Sk", [(torch.float32, 392), (torch.bfloat16, 389)])
