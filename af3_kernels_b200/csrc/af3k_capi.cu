@@ -205,7 +205,6 @@ struct Plan {
   AttnParams p;
   size_t smem_bytes;
   int grid;
-  long long whole_items;   // work items if all were of the main size
 };
 
 // The longest CTA's time when n_main items of cost c_main and then n_tail of cost c_tail are dealt out round-robin.
@@ -339,7 +338,6 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   p.div_q = make_divisor((uint32_t)tiles_of(best_split));
   p.tail_div_q = make_divisor((uint32_t)tiles_of(best_tail_split));
   p.div_h = make_divisor((uint32_t)p.B2);
-  plan->whole_items = (p.B1 + p.G - 1) / p.G * (long long)p.B2 * tiles_of(best_split);
 
   uint32_t off = 0;
   p.off_q = off;      off += p.q_buffers * p.n_streams * p.q_tile_bytes;
@@ -648,7 +646,7 @@ int af3k_describe_plan(const af3k_attention_desc* desc, int32_t* out6) {
   if (rc != AF3K_OK) return rc;
   out6[0] = plan.p.G;
   out6[1] = plan.p.kv_stages;
-  out6[2] = (int32_t)plan.whole_items;
+  out6[2] = plan.p.n_items;
   out6[3] = plan.grid;
   out6[4] = (int32_t)plan.smem_bytes;
   out6[5] = (int32_t)kOCol + plan.p.n_streams * plan.p.nv;

@@ -166,9 +166,9 @@ void af3k_set_wait_limit_cycles(long long cycles);
  * 227 KB of shared memory per block is assumed when no such device is present, so this also
  * works on a CPU-only host): out6 = {pair rows per work item, K/V ring stages, work items,
  * grid size, dynamic shared memory bytes, TMEM columns used}.  With one pair row per item an item is
- * one query tile while there is an SM for each, else two.  The work items are counted as if all had that size; those behind
- * the last full round may be launched as more, smaller ones.  Diagnostic; no counterpart in the
- * reference. */
+ * one query tile while there is an SM for each, else two.  Where the pair rows behind the last full round go to smaller
+ * items, there are more of them than rows, heads and query tiles make of the first size.  Diagnostic; no counterpart in
+ * the reference. */
 int af3k_describe_plan(const af3k_attention_desc* desc, int32_t* out6);
 
 /* Diagnostic: when dump_dev is non-NULL, later attention calls run a debug build of the kernel

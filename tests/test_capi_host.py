@@ -71,6 +71,18 @@ def test_launch_plan_fits_b200(shape):
     assert plan["grid"] <= plan["items"]
 
 
+@pytest.mark.parametrize("shape,qk,main,rest", [((256, 4, 256, 32), _capi.AF3K_BF16, 440, 144), ((256, 4, 256, 32), _capi.AF3K_FP8_E4M3, 440, 144),
+                                                ((99, 3, 130, 24), _capi.AF3K_BF16, 144, 84), ((77, 8, 250, 32), _capi.AF3K_BF16, 288, 48)])
+def test_plan_reports_smaller_items(shape, qk, main, rest):
+    """Rows behind the last full round in items of two: both kinds are counted."""
+    plan = _capi.describe_plan(_desc(*shape, qk=qk))
+    B1, B2, S, _ = shape
+    tiles = B2 * -(-S // 128)
+    assert main % tiles == 0 and rest == -(-(B1 - main // tiles * plan["rows_per_item"]) // 2) * tiles
+    if not torch.cuda.is_available() or plan["grid"] == 148:
+        assert plan["items"] == main + rest and plan["grid"] == 148
+
+
 def test_max_ctas_caps_the_grid():
     d = _desc(768, 4, 768, 32)
     full = _capi.describe_plan(d)
