@@ -4,6 +4,7 @@ tolerances of the bf16 path; forms that only deal the same work out differently 
 import pytest
 import torch
 
+from af3_kernels_b200 import _capi
 from af3_kernels_b200.dpa import dot_product_attention, stage_bias
 from oracle import attention_oracle as O
 
@@ -173,22 +174,71 @@ def test_reference_rises_under_a_large_bias(cuda_device, value):
     _check(_call(cuda_device, q, k, v, None, bias, softmax_scale=1.0), ref.float(), value)
 
 
-@pytest.mark.parametrize("B1,B2,S,D", [(78, 8, 256, 16), (77, 8, 250, 32), (41, 4, 640, 32), (5, 16, 700, 48), (7, 16, 900, 64), (150, 1, 130, 8)])
-def test_smaller_items_behind_the_last_full_round(cuda_device, B1, B2, S, D):
+def _quantised(q, k):
+    (q, qs), (k, ks) = O.quantize_e4m3_per_head(q.float()), O.quantize_e4m3_per_head(k.float())
+    return q, k, {"q_scale": qs, "k_scale": ks}
+
+
+def _plan(B1, B2, S, D, fp8):
+    d = _capi.AttentionDesc()
+    d.B1, d.B2, d.Sq, d.Sk, d.D = B1, B2, S, S, D
+    for n in ("q_stride", "k_stride", "v_stride", "out_stride"):
+        getattr(d, n)[:] = [B2 * S * D, S * D, D]
+    d.bias_stride[:], d.mask_row_stride, d.softmax_scale = [S * S, S], S, D ** -0.5
+    d.qk_dtype, d.bias_dtype = _capi.AF3K_FP8_E4M3 if fp8 else _capi.AF3K_BF16, _capi.AF3K_BF16
+    return _capi.describe_plan(d)
+
+
+def _check_form(dev, B1, B2, S, D, qk, **other):
+    """One row of items against the oracle, and the same bits as with another split of the work."""
     q, k, v, mask, bias = _inputs(B1, B2, S, D, S + D)
-    out = _call(cuda_device, q, k, v, mask, bias)
-    assert torch.equal(_call(cuda_device, q, k, v, mask, bias, rows_per_item=1), out)
-    rows = [0, B1 // 2, B1 - 1]
-    _check(out[rows], O.oracle_fp32(q[rows], k[rows], v[rows], mask[rows], bias), (B1, B2, S, D))
+    scales, kw, on_dev = {}, {}, {}
+    if qk != "bf16":
+        q, k, scales = _quantised(q, k)
+        kw = {"use_workspace": qk == "fp8"}
+        on_dev = {n: t.to(dev) for n, t in scales.items()}
+    out = _call(dev, q, k, v, mask, bias, **kw, **on_dev)
+    assert torch.equal(_call(dev, q, k, v, mask, bias, **other, **kw, **on_dev), out)
+    rows = [0, B1 // 2, B1 - 2, B1 - 1]
+    st = O.error_stats(out[rows], O.oracle_fp32(q[rows], k[rows], v[rows], mask[rows], bias, **scales))
+    limit = (2e-2, 2e-3) if qk == "bf16" else (6e-2, 6e-3)
+    assert st["nan"] == 0 and st["max_abs"] <= limit[0] and st["mean_abs"] <= limit[1], st
 
 
-def test_items_of_one_and_two_query_tiles_on_one_cta(cuda_device):
+@pytest.mark.parametrize("B1,B2,S,D,qk", [
+    (99, 3, 130, 8, "bf16"), (99, 3, 130, 24, "bf16"), (46, 8, 136, 16, "bf16"), (78, 8, 256, 16, "bf16"), (77, 8, 250, 32, "bf16"), (41, 4, 640, 32, "bf16"),
+    (46, 8, 136, 16, "fp8"), (99, 3, 136, 32, "fp8"), (41, 4, 640, 32, "fp8"), (46, 8, 136, 16, "fp8_no_workspace"), (99, 3, 136, 32, "fp8_no_workspace"),
+    (41, 4, 640, 32, "fp8_no_workspace")])
+def test_smaller_items_behind_the_last_full_round(cuda_device, B1, B2, S, D, qk):
+    """Items of three or four rows, then items of two."""
+    plan = _plan(B1, B2, S, D, qk != "bf16")
+    tiles = B2 * ((S + 127) // 128)
+    assert plan["rows_per_item"] > 2 and plan["items"] > -(-B1 // plan["rows_per_item"]) * tiles, plan
+    _check_form(cuda_device, B1, B2, S, D, qk, rows_per_item=1)
+
+
+@pytest.mark.parametrize("B1,B2,S,D,qk", [(5, 16, 700, 48, "bf16"), (7, 16, 900, 64, "bf16"), (150, 1, 130, 8, "bf16"), (7, 16, 904, 64, "fp8"),
+                                          (7, 16, 904, 64, "fp8_no_workspace"), (149, 2, 264, 16, "fp8"), (149, 2, 264, 16, "fp8_no_workspace")])
+def test_rows_that_do_not_fill_the_last_item(cuda_device, B1, B2, S, D, qk):
+    """Items of one width, the last of them of fewer rows; a cap on the CTAs gives each CTA several of both."""
+    _check_form(cuda_device, B1, B2, S, D, qk, max_ctas=B2 * 3)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+def test_items_of_one_and_two_query_tiles_on_one_cta(cuda_device, fp8):
     """Nine query tiles in pairs leave items of one; with five items to a CTA a slot of the Q buffers is skipped and used
     again."""
     q, k, v, mask, bias = _inputs(1, 10, 1100, 32, 3)
-    ref = O.oracle_fp32(q, k, v, mask, bias)
+    scales = {}
+    if fp8:
+        q, k, scales = _quantised(q, k)
+    ref = O.oracle_fp32(q, k, v, mask, bias, **scales)
     for ctas in (9, 11, 13):
-        _check(_call(cuda_device, q, k, v, mask, bias, max_ctas=ctas), ref, ctas)
+        out = _call(cuda_device, q, k, v, mask, bias, max_ctas=ctas, **{n: t.to(cuda_device) for n, t in scales.items()})
+        if fp8:
+            assert O.error_stats(out, ref)["max_abs"] <= 6e-2, ctas
+        else:
+            _check(out, ref, ctas)
 
 
 @pytest.mark.parametrize("D", [32, 40, 48, 56])
