@@ -817,10 +817,11 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, float* dbg, int wg, i
   const uint64_t nm2 = pack_f32x2(-m_use, -m_use);
   const uint64_t nml2 = pack_f32x2(nml, nml);
   uint64_t suma = pack_f32x2(0.f, 0.f), sumb = suma;
-  // The first kHeld column groups are computed before anything is written: the P buffer and the
-  // O accumulator only become free when the previous P V of this warpgroup has finished, and that
-  // wait is taken as late as the registers allow.
-  constexpr int kHeld = 3;
+  // The first kHeld column groups are computed before anything is written: the P buffer and the O accumulator only become free
+  // when the previous P V of this warpgroup has finished.  Held groups cost eight registers each, and two cover that wait:
+  // 2048 fp8 rows 11 340 us with three, 10 920 with two, 768 bf16 rows 659 and 646; one is as fast there and
+  // slower at 389 rows (168 -> 174).
+  constexpr int kHeld = 2;
   uint32_t pk[8][8];
 #pragma unroll
   for (int cidx = 0; cidx < 8; ++cidx) {
