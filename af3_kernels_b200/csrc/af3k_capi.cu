@@ -263,8 +263,8 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   int g_max = kMaxStreams < g_tmem ? kMaxStreams : g_tmem;
   if (g_max > p.B1) g_max = p.B1 > 0 ? p.B1 : 1;
 
-  int best_g = 0, best_stages = 0, best_qbuf = 0, best_tail_g = 0;
-  bool best_split = false, best_tail_split = false;
+  int best_g = 0, best_stages = 0, best_qbuf = 0;
+  bool best_split = false;
   long long best_rows = 0;     // pair rows taken by the main items
   double best_cost = 0;
   const int ctas = (d.max_ctas > 0 && d.max_ctas < dev.sm_count) ? d.max_ctas : dev.sm_count;
@@ -297,27 +297,22 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
       if (split) weight *= 1.02;   // query-tile streams share no bias tile: pair rows win a tie
       const double main_cost = item_cost(g, split, qbuf);
       const long long per_group = (long long)p.B2 * tiles_of(split), groups = (p.B1 + g - 1) / g;
-      auto offer = [&](double cost, long long rows, int tail_g, bool tail_split) {
+      auto offer = [&](double cost, long long rows) {
         cost *= weight;
-        if (best_g != 0 && cost >= (tail_g != 0 ? kTailGain : 1.0) * best_cost) return;
+        if (best_g != 0 && cost >= (rows < p.B1 ? kTailGain : 1.0) * best_cost) return;
         best_g = g; best_cost = cost; best_stages = stages; best_qbuf = qbuf; best_split = split;
-        best_rows = rows; best_tail_g = tail_g; best_tail_split = tail_split;
+        best_rows = rows;
       };
-      offer(dealt_cost(groups * per_group, main_cost, 0, 0.0, ctas), p.B1, 0, false);
-      // A last round that is not full: the rows from some row on go to smaller items (256 rows of 64 channels, 512 items of
-      // four rows in four rounds -> 440 and 144 of two: 57.9 -> 54.5 us a module call).
+      offer(dealt_cost(groups * per_group, main_cost, 0, 0.0, ctas), p.B1);
+      // A last round that is not full: the rows from some row on go to items of two rows (256 rows of 64 channels, 512 items
+      // of four rows in four rounds -> 440 and 144 of two: 57.9 -> 54.5 us a module call).  One row would leave a warpgroup
+      // without work, three take as long as four.
       const long long rounds = groups * per_group / ctas;
-      for (long long r = rounds; r >= 1 && r >= rounds - 1 && g_req == 0; --r) {
+      for (long long r = rounds; r >= 1 && r >= rounds - 1 && g_req == 0 && g > kTailRows; --r) {
         const long long main_groups = r * ctas / per_group, rows = main_groups * g;
         if (main_groups < 1 || rows >= p.B1) continue;
-        for (int tg = 1; tg <= g; ++tg)
-          for (int ts = 0; ts <= (tg == 1 && may_split ? 1 : 0); ++ts) {
-            // two streams at least, so that both warpgroups have work, and no more than the Q buffers hold
-            const int tail_streams = ts != 0 ? 2 : tg;
-            if ((tg == g && (ts != 0) == split) || tail_streams < 2 || tail_streams > streams) continue;
-            const long long tail = (p.B1 - rows + tg - 1) / tg * p.B2 * tiles_of(ts != 0);
-            offer(dealt_cost(main_groups * per_group, main_cost, tail, item_cost(tg, ts != 0, qbuf), ctas), rows, tg, ts != 0);
-          }
+        const long long tail = (p.B1 - rows + kTailRows - 1) / kTailRows * per_group;
+        offer(dealt_cost(main_groups * per_group, main_cost, tail, item_cost(kTailRows, false, qbuf), ctas), rows);
       }
     }
   }
@@ -327,16 +322,13 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   p.n_streams = p.q_split ? 2 : p.G;
   p.kv_stages = best_stages;
   p.q_buffers = best_qbuf;
-  p.tail_g = best_tail_g;
-  p.tail_split = best_tail_split ? 1 : 0;
   p.tail_row = (int)best_rows;
-  const long long n_main = (best_rows + p.G - 1) / p.G * p.B2 * tiles_of(best_split);
-  const long long n_tail = best_tail_g == 0 ? 0 : (p.B1 - best_rows + best_tail_g - 1) / best_tail_g * p.B2 * tiles_of(best_tail_split);
+  const long long per_group = (long long)p.B2 * tiles_of(best_split);
+  const long long n_main = (best_rows + p.G - 1) / p.G * per_group, n_tail = (p.B1 - best_rows + kTailRows - 1) / kTailRows * per_group;
   if (n_main + n_tail > 0x7fffffff) return AF3K_ERR_BAD_SHAPE;
   p.n_main = (int)n_main;
   p.n_items = (int)(n_main + n_tail);
   p.div_q = make_divisor((uint32_t)tiles_of(best_split));
-  p.tail_div_q = make_divisor((uint32_t)tiles_of(best_tail_split));
   p.div_h = make_divisor((uint32_t)p.B2);
 
   uint32_t off = 0;

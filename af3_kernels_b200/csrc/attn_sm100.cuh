@@ -61,6 +61,7 @@ constexpr int kMaxStreams = 4;     // pair rows per work item (two per softmax w
 // TMEM columns: two fp32 logits buffers, two bf16 P buffers (two keys per column), then O.
 constexpr uint32_t kSCol = 0, kPCol = 2 * 128, kOCol = 2 * 128 + 2 * 64;
 constexpr float kLazyRescaleLog2 = 8.0f;   // keep a stale row max while exp2 arguments stay <= 8
+constexpr int kTailRows = 2;       // pair rows of an item behind the last full round: both softmax warpgroups have work
 constexpr int kBiasStages = 2;
 constexpr int kBiasTileBytes = kTile * kTile * 2;  // bf16, two 128B-swizzled boxes of 64 columns
 constexpr int kMaxKvStages = 6;
@@ -109,9 +110,7 @@ struct AttnParams {
   int q_split;           // 1: the streams of an item are two neighbouring query tiles of ONE pair row (G == 1)
   int n_streams;         // streams per work item: G, or 2 with q_split
   int n_items;
-  // the items behind the first n_main are smaller: tail_g rows (or two query tiles) each, of the rows from tail_row on
-  int n_main, tail_g, tail_split, tail_row;
-  Divisor tail_div_q;
+  int n_main, tail_row;  // the items behind the first n_main are smaller: kTailRows rows each, of the rows from tail_row on
   Divisor div_q, div_h;  // query tiles (or pairs of them) per row and head, heads
   int qk_row_bytes;      // smem bytes per Q / K tile row: 32, 64 or 128 (= swizzle span)
   // 1: bf16 heads of 33 to 48 channels.  A Q / K tile is 32 channels in rows of 64 bytes, then 16 in rows of 32 bytes: 12 KB
@@ -259,24 +258,22 @@ __device__ __forceinline__ uint32_t swizzle_layout_code(int row_bytes) {
 // is not left idle) they are gv neighbouring query tiles of pair row r0, each with its own bias
 // tiles.
 struct Item {
-  int qt, h, r0, gv, split;
+  int qt, h, r0, gv;
 };
 __device__ __forceinline__ Item decode_item(const AttnParams& p, int item) {
   Item it;
   const bool tail = item >= p.n_main;
   const uint32_t i = (uint32_t)(tail ? item - p.n_main : item);
-  const Divisor div_q = tail ? p.tail_div_q : p.div_q;
-  const int g = tail ? p.tail_g : p.G, row = tail ? p.tail_row : 0, end = tail ? p.B1 : p.tail_row;
-  it.split = tail ? p.tail_split : p.q_split;
-  const uint32_t t = divide(i, div_q), rg = divide(t, p.div_h);
-  it.qt = (int)(i - t * div_q.d) << it.split;
+  const int g = tail ? kTailRows : p.G, row = tail ? p.tail_row : 0, end = tail ? p.B1 : p.tail_row;
+  const uint32_t t = divide(i, p.div_q), rg = divide(t, p.div_h);
+  it.qt = (int)(i - t * p.div_q.d) << p.q_split;
   it.h = (int)(t - rg * p.div_h.d);
   it.r0 = row + (int)rg * g;
-  it.gv = it.split ? min(2, p.n_qt - it.qt) : min(g, end - it.r0);
+  it.gv = p.q_split ? min(2, p.n_qt - it.qt) : min(g, end - it.r0);
   return it;
 }
-__device__ __forceinline__ int stream_row(const Item& it, int s) { return it.split ? it.r0 : it.r0 + s; }
-__device__ __forceinline__ int stream_qt(const Item& it, int s) { return it.split ? it.qt + s : it.qt; }
+__device__ __forceinline__ int stream_row(const AttnParams& p, const Item& it, int s) { return p.q_split ? it.r0 : it.r0 + s; }
+__device__ __forceinline__ int stream_qt(const AttnParams& p, const Item& it, int s) { return p.q_split ? it.qt + s : it.qt; }
 
 // Q buffer of the CTA's j-th item and how often that buffer was used before.  An item with fewer streams than the Q
 // buffers hold takes the slots of the others through their phases all the same (an arrival on each of their barriers), so
@@ -306,9 +303,9 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
       }
       mbar_arrive_expect_tx(bar_addr(c, BarIdx::q_full + slot), p.q_tile_bytes);
       const uint32_t qdst = c.smem + p.off_q + (buf * p.n_streams + s) * p.q_tile_bytes;
-      tma_load_4d(qdst, tm_q, bar_addr(c, BarIdx::q_full + slot), 0, stream_qt(it, s) * kTile, it.h, stream_row(it, s));
+      tma_load_4d(qdst, tm_q, bar_addr(c, BarIdx::q_full + slot), 0, stream_qt(p, it, s) * kTile, it.h, stream_row(p, it, s));
       if (p.qk_narrow)
-        tma_load_4d(qdst + kNarrowOff, tm_q2, bar_addr(c, BarIdx::q_full + slot), 32, stream_qt(it, s) * kTile, it.h, stream_row(it, s));
+        tma_load_4d(qdst + kNarrowOff, tm_q2, bar_addr(c, BarIdx::q_full + slot), 32, stream_qt(p, it, s) * kTile, it.h, stream_row(p, it, s));
     }
     return true;
   };
@@ -322,15 +319,15 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
     for (int kt = 0; kt < p.n_kt; ++kt) {
 #pragma unroll 1
       for (int s = 0; s < it.gv; ++s) {
-        if (s == 0 || it.split) {   // one bias tile per key tile, or per stream when the streams are query tiles
+        if (s == 0 || p.q_split) {   // one bias tile per key tile, or per stream when the streams are query tiles
           const uint32_t bst = bcount % kBiasStages;
           if (bcount >= kBiasStages)
             AF3K_WAIT(c, BarIdx::bias_empty + bst, ((bcount / kBiasStages) - 1) & 1);
           const uint32_t bfull = bar_addr(c, BarIdx::bias_full + bst);
           const uint32_t bdst = c.smem + p.off_bias + bst * kBiasTileBytes;
           mbar_arrive_expect_tx(bfull, kBiasTileBytes);
-          tma_load_3d(bdst, tm_bias, bfull, kt * kTile, stream_qt(it, s) * kTile, it.h);
-          tma_load_3d(bdst + kBiasTileBytes / 2, tm_bias, bfull, kt * kTile + 64, stream_qt(it, s) * kTile, it.h);
+          tma_load_3d(bdst, tm_bias, bfull, kt * kTile, stream_qt(p, it, s) * kTile, it.h);
+          tma_load_3d(bdst + kBiasTileBytes / 2, tm_bias, bfull, kt * kTile + 64, stream_qt(p, it, s) * kTile, it.h);
           ++bcount;
         }
         const uint32_t st = ucount % nkv;
@@ -338,9 +335,9 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
         const uint32_t full = bar_addr(c, BarIdx::kv_full + st);
         const uint32_t kdst = c.smem + p.off_kv + st * (p.k_tile_bytes + p.v_tile_bytes);
         mbar_arrive_expect_tx(full, p.k_tile_bytes + p.v_tile_bytes);
-        tma_load_4d(kdst, tm_k, full, 0, kt * kTile, it.h, stream_row(it, s));
-        if (p.qk_narrow) tma_load_4d(kdst + kNarrowOff, tm_k2, full, 32, kt * kTile, it.h, stream_row(it, s));
-        tma_load_4d(kdst + p.k_tile_bytes, tm_v, full, 0, kt * kTile, it.h, stream_row(it, s));
+        tma_load_4d(kdst, tm_k, full, 0, kt * kTile, it.h, stream_row(p, it, s));
+        if (p.qk_narrow) tma_load_4d(kdst + kNarrowOff, tm_k2, full, 32, kt * kTile, it.h, stream_row(p, it, s));
+        tma_load_4d(kdst + p.k_tile_bytes, tm_v, full, 0, kt * kTile, it.h, stream_row(p, it, s));
         ++ucount;
       }
       if (kt == (p.q_buffers == 2 ? 0 : p.n_kt - 1) && item + (int)gridDim.x < p.n_items) {
@@ -372,7 +369,7 @@ __device__ __forceinline__ void scale_q_chunk(uint32_t addr, float scale, int la
 // The 128 mask-column values (bf16) of one logits tile, four per lane.
 __device__ __forceinline__ void mask_values(const AttnParams& p, const Item& it, int kt, int s, int lane,
                                             uint16_t masked, uint16_t (&val)[4]) {
-  const uint8_t* mrow = p.mask != nullptr ? p.mask + (long long)stream_row(it, s) * p.mask_row_stride : nullptr;
+  const uint8_t* mrow = p.mask != nullptr ? p.mask + (long long)stream_row(p, it, s) * p.mask_row_stride : nullptr;
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     const int key = kt * kTile + 32 * g + lane;
@@ -543,7 +540,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
         const int b = s & 1;
         const int qslot = (int)q_buf(p, icount) * kMaxStreams + s;
         const int q_bar = (p.scale_q ? BarIdx::q_scaled : BarIdx::q_full) + qslot;
-        const bool need_bias = kTcBias && (s == 0 || it.split);
+        const bool need_bias = kTcBias && (s == 0 || p.q_split);
         const bool need_sfree = (used >> b) & 1u;
         const uint32_t sf_par = (sfree_par >> b) & 1u;
         {
@@ -594,7 +591,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
         }
         __syncwarp();
         if (++st == nkv) { st = 0; kv_par ^= 1; }
-        if (kTcBias && (s == gv - 1 || it.split)) {
+        if (kTcBias && (s == gv - 1 || p.q_split)) {
           // every bias MMA that reads this stage is issued: the stage is free when they finish
           if (leader) tc_commit(bar_addr(c, BarIdx::bias_empty + bst));
           __syncwarp();
@@ -993,14 +990,14 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
     if (kDebug && last_ts != nullptr) last_ts[6] = clock64();
 #pragma unroll 1
     for (int s = wg; s < it.gv; s += 2) {
-      const int qrow = stream_qt(it, s) * kTile + row;
+      const int qrow = stream_qt(p, it, s) * kTile + row;
       const float inv = __frcp_rn(s == wg ? l_st[0] : l_st[1]);
       const uint32_t o_taddr = c.tmem + lane_sel + kOCol + s * p.nv;
-      __nv_bfloat16* orow = p.out + (long long)stream_row(it, s) * p.out_stride_b1 +
+      __nv_bfloat16* orow = p.out + (long long)stream_row(p, it, s) * p.out_stride_b1 +
                             (long long)it.h * p.out_stride_b2 + (long long)qrow * p.out_stride_s;
       const __nv_bfloat16* grow = nullptr;
       if constexpr (kGate)
-        grow = p.gate + (long long)stream_row(it, s) * p.gate_stride_b1 + (long long)it.h * p.gate_stride_b2 + (long long)qrow * p.gate_stride_s;
+        grow = p.gate + (long long)stream_row(p, it, s) * p.gate_stride_b1 + (long long)it.h * p.gate_stride_b2 + (long long)qrow * p.gate_stride_s;
 #pragma unroll 1
       for (int c0 = 0; c0 < p.nv; c0 += 16) {
         uint32_t o[16];
