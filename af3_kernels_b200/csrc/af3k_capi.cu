@@ -92,11 +92,14 @@ int device_info(DeviceInfo** out) {
     const int dyn = d.max_smem_optin - kStaticSmemReserve;
     const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     const void* kernels[] = {
-        (const void*)attention_kernel<false, true, false, false>, (const void*)attention_kernel<false, true, false, true>,
-        (const void*)attention_kernel<false, true, true, false>,  (const void*)attention_kernel<false, true, true, true>,
-        (const void*)attention_kernel<false, false, true, false>, (const void*)attention_kernel<false, false, true, true>,
-        (const void*)attention_kernel<true, true, false, false>,  (const void*)attention_kernel<true, true, true, false>,
-        (const void*)attention_kernel<true, false, true, false>,
+        (const void*)attention_kernel<false, true, false, false, false>, (const void*)attention_kernel<false, true, false, true, false>,
+        (const void*)attention_kernel<false, true, true, false, false>,  (const void*)attention_kernel<false, true, true, true, false>,
+        (const void*)attention_kernel<false, false, true, false, false>, (const void*)attention_kernel<false, false, true, true, false>,
+        (const void*)attention_kernel<false, true, false, false, true>,  (const void*)attention_kernel<false, true, false, true, true>,
+        (const void*)attention_kernel<false, true, true, false, true>,   (const void*)attention_kernel<false, true, true, true, true>,
+        (const void*)attention_kernel<false, false, true, false, true>,  (const void*)attention_kernel<false, false, true, true, true>,
+        (const void*)attention_kernel<true, true, false, false, true>,   (const void*)attention_kernel<true, true, true, false, true>,
+        (const void*)attention_kernel<true, false, true, false, true>,
     };
     e = cudaSuccess;
     for (const void* kfn : kernels)
@@ -327,6 +330,7 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   const long long n_main = (best_rows + p.G - 1) / p.G * per_group, n_tail = (p.B1 - best_rows + kTailRows - 1) / kTailRows * per_group;
   if (n_main + n_tail > 0x7fffffff) return AF3K_ERR_BAD_SHAPE;
   p.n_main = (int)n_main;
+  p.mixed = (n_tail != 0 || (p.q_split ? p.n_qt % 2 : p.B1 % p.G) != 0) ? 1 : 0;
   p.n_items = (int)(n_main + n_tail);
   p.div_q = make_divisor((uint32_t)tiles_of(best_split));
   p.div_h = make_divisor((uint32_t)p.B2);
@@ -594,21 +598,23 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
   const bool tc_bias = !fp8 || fp8_tc;
   p.scale_q = (fp8 || d.softmax_scale == 1.0f) ? 0 : 1;   // a scale of exactly 1 (q already scaled by its producer) needs no pass over Q
   const bool dbg = p.debug != nullptr;
-#define AF3K_LAUNCH(...) launch_overlapped(attention_kernel<__VA_ARGS__>, dim3(plan.grid), kThreads, plan.smem_bytes, stream, d.max_ctas <= 0, p, tm_q, tm_k, tm_v, tm_b, tm_q2, tm_k2)
+#define AF3K_LAUNCH_AS(...) launch_overlapped(attention_kernel<__VA_ARGS__>, dim3(plan.grid), kThreads, plan.smem_bytes, stream, d.max_ctas <= 0, p, tm_q, tm_k, tm_v, tm_b, tm_q2, tm_k2)
+#define AF3K_LAUNCH(...) (p.mixed ? AF3K_LAUNCH_AS(__VA_ARGS__, true) : AF3K_LAUNCH_AS(__VA_ARGS__, false))
   if (p.gate != nullptr) {
     if (!fp8)         AF3K_LAUNCH(false, true, false, true);
     else if (tc_bias) AF3K_LAUNCH(false, true, true, true);
     else              AF3K_LAUNCH(false, false, true, true);
   } else if (dbg) {
-    if (!fp8)         AF3K_LAUNCH(true, true, false, false);
-    else if (tc_bias) AF3K_LAUNCH(true, true, true, false);
-    else              AF3K_LAUNCH(true, false, true, false);
+    if (!fp8)         AF3K_LAUNCH_AS(true, true, false, false, true);
+    else if (tc_bias) AF3K_LAUNCH_AS(true, true, true, false, true);
+    else              AF3K_LAUNCH_AS(true, false, true, false, true);
   } else {
     if (!fp8)         AF3K_LAUNCH(false, true, false, false);
     else if (tc_bias) AF3K_LAUNCH(false, true, true, false);
     else              AF3K_LAUNCH(false, false, true, false);
   }
 #undef AF3K_LAUNCH
+#undef AF3K_LAUNCH_AS
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail("launch attention_kernel", e);
   ++launches;

@@ -110,6 +110,7 @@ struct AttnParams {
   int q_split;           // 1: the streams of an item are two neighbouring query tiles of ONE pair row (G == 1)
   int n_streams;         // streams per work item: G, or 2 with q_split
   int n_items;
+  int mixed;             // 1: the kernel's kMixed
   int n_main, tail_row;  // the items behind the first n_main are smaller: kTailRows rows each, of the rows from tail_row on
   Divisor div_q, div_h;  // query tiles (or pairs of them) per row and head, heads
   int qk_row_bytes;      // smem bytes per Q / K tile row: 32, 64 or 128 (= swizzle span)
@@ -260,8 +261,17 @@ __device__ __forceinline__ uint32_t swizzle_layout_code(int row_bytes) {
 struct Item {
   int qt, h, r0, gv;
 };
+template <bool kMixed>
 __device__ __forceinline__ Item decode_item(const AttnParams& p, int item) {
   Item it;
+  if (!kMixed) {
+    const uint32_t t = divide((uint32_t)item, p.div_q), rg = divide(t, p.div_h);
+    it.qt = (int)((uint32_t)item - t * p.div_q.d) << p.q_split;
+    it.h = (int)(t - rg * p.div_h.d);
+    it.r0 = (int)rg * p.G;
+    it.gv = p.n_streams;
+    return it;
+  }
   const bool tail = item >= p.n_main;
   const uint32_t i = (uint32_t)(tail ? item - p.n_main : item);
   const int g = tail ? kTailRows : p.G, row = tail ? p.tail_row : 0, end = tail ? p.B1 : p.tail_row;
@@ -275,13 +285,14 @@ __device__ __forceinline__ Item decode_item(const AttnParams& p, int item) {
 __device__ __forceinline__ int stream_row(const AttnParams& p, const Item& it, int s) { return p.q_split ? it.r0 : it.r0 + s; }
 __device__ __forceinline__ int stream_qt(const AttnParams& p, const Item& it, int s) { return p.q_split ? it.qt + s : it.qt; }
 
-// Q buffer of the CTA's j-th item and how often that buffer was used before.  An item with fewer streams than the Q
+// Q buffer of the CTA's j-th item and how often that buffer was used before.  (kMixed) An item with fewer streams than the Q
 // buffers hold takes the slots of the others through their phases all the same (an arrival on each of their barriers), so
 // that one count serves all slots: counting every slot's own uses in the issuer's loop cost 2 - 5 %.
 __device__ __forceinline__ uint32_t q_buf(const AttnParams& p, uint32_t j) { return p.q_buffers == 2 ? (j & 1u) : 0u; }
 __device__ __forceinline__ uint32_t q_use(const AttnParams& p, uint32_t j) { return p.q_buffers == 2 ? (j >> 1) : j; }
 
 // ------------------------------------------------------------------ producer (one thread)
+template <bool kMixed>
 __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUtensorMap* tm_k,
                               const CUtensorMap* tm_v, const CUtensorMap* tm_bias, const CUtensorMap* tm_q2, const CUtensorMap* tm_k2) {
   const AttnParams& p = *c.p;
@@ -297,7 +308,7 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
       const int slot = (int)buf * kMaxStreams + s;
       // the buffer's previous user must have finished its last Q K^T of this stream
       if (use >= 1) AF3K_WAIT_NORET(c, BarIdx::q_empty + slot, (use - 1) & 1);
-      if (s >= it.gv) {
+      if (kMixed && s >= it.gv) {
         mbar_arrive(bar_addr(c, BarIdx::q_full + slot));
         continue;
       }
@@ -310,11 +321,11 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
     return true;
   };
   if ((int)blockIdx.x < p.n_items) {
-    if (!load_q(decode_item(p, blockIdx.x), 0)) return;
+    if (!load_q(decode_item<kMixed>(p, blockIdx.x), 0)) return;
   }
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
-    const Item it = decode_item(p, item);
+    const Item it = decode_item<kMixed>(p, item);
 #pragma unroll 1
     for (int kt = 0; kt < p.n_kt; ++kt) {
 #pragma unroll 1
@@ -341,7 +352,7 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
         ++ucount;
       }
       if (kt == (p.q_buffers == 2 ? 0 : p.n_kt - 1) && item + (int)gridDim.x < p.n_items) {
-        if (!load_q(decode_item(p, item + gridDim.x), icount + 1)) return;
+        if (!load_q(decode_item<kMixed>(p, item + gridDim.x), icount + 1)) return;
       }
     }
   }
@@ -441,13 +452,14 @@ struct QScaler {
 // K step; only element 0 of each key's 16-byte row changes, the rest stays zero.  Arrives on the
 // tile's kv_full barrier (which then counts two arrivals: this one and the producer's).  The mask
 // bytes of a tile are requested one tile ahead, so their latency is not on the path.
+template <bool kMixed>
 __device__ void mask_writer_role(const Ctx& c, int lane) {
   const AttnParams& p = *c.p;
   const uint32_t nkv = p.kv_stages;
   uint32_t st = 0, round = 0;      // ring slot, how many times the ring wrapped
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
-    const Item it = decode_item(p, item);
+    const Item it = decode_item<kMixed>(p, item);
     uint16_t val[4] = {};
     const uint16_t masked = masked_value_bits(p, it.h);
     // step i writes the values of tile i (key tiles outermost, then streams) and requests those of tile i + 1
@@ -488,7 +500,7 @@ __device__ void mask_writer_role(const Ctx& c, int lane) {
 // Logits of every tile, in order: Q K^T, then the mask column, then (bf16 q/k) the bias slices.
 // (The MMA loops are real loops and the fp8 / bf16 choice is a template argument: the warp pays an
 // instruction-cache miss for most lines of this loop on every pass, so the loop is kept small.)
-template <bool kDebug, bool kTcBias, bool kFp8>
+template <bool kDebug, bool kTcBias, bool kFp8, bool kMixed>
 __device__ void qk_issuer_role(const Ctx& c) {
   const AttnParams& p = *c.p;
   const bool leader = elect_one();
@@ -531,7 +543,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
   uint32_t sfree_par = 0, used = 0;   // bit b: parity of buffer b's next release; buffer b has held a tile
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
-    const Item it = decode_item(p, item);
+    const Item it = decode_item<kMixed>(p, item);
     const int gv = it.gv;
 #pragma unroll 1
     for (int kt = 0; kt < p.n_kt; ++kt) {
@@ -601,25 +613,27 @@ __device__ void qk_issuer_role(const Ctx& c) {
     }
     // the slots that this item does not use: their scaling and their release (this warp is the one that waits for the
     // former and, through the producer, for the latter, so neither can run ahead of it)
-    if (leader)
-      for (int s = gv; s < p.n_streams; ++s) {
-        mbar_arrive(bar_addr(c, BarIdx::q_scaled + (int)q_buf(p, icount) * kMaxStreams + s));
-        mbar_arrive(bar_addr(c, BarIdx::q_empty + (int)q_buf(p, icount) * kMaxStreams + s));
-      }
-    __syncwarp();
+    if (kMixed) {
+      if (leader)
+        for (int s = gv; s < p.n_streams; ++s) {
+          mbar_arrive(bar_addr(c, BarIdx::q_scaled + (int)q_buf(p, icount) * kMaxStreams + s));
+          mbar_arrive(bar_addr(c, BarIdx::q_empty + (int)q_buf(p, icount) * kMaxStreams + s));
+        }
+      __syncwarp();
+    }
   }
 }
 
 // O += P V for every tile, in order.  This warp mostly waits for the softmax warpgroups, so (bf16
 // q/k) it also scales the Q tiles: the first item's up front, the next item's in 1 KB pieces
 // while it waits, what is left when the item's last P V has been issued.
-template <bool kDebug, bool kScalesQ>
+template <bool kDebug, bool kScalesQ, bool kMixed>
 __device__ void pv_issuer_role(const Ctx& c, int lane) {
   const AttnParams& p = *c.p;
   const bool leader = elect_one();
   QScaler scaler;
   if (kScalesQ && p.scale_q && (int)blockIdx.x < p.n_items) {
-    scaler.start(0, decode_item(p, blockIdx.x).gv);
+    scaler.start(0, decode_item<kMixed>(p, blockIdx.x).gv);
     while (scaler.pending())
       if (scaler.step(c, lane, true) < 0) return;
   }
@@ -642,9 +656,9 @@ __device__ void pv_issuer_role(const Ctx& c, int lane) {
   uint32_t pready_par = 0;         // bit b: of warpgroup b's next P
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
-    const Item it = decode_item(p, item);
+    const Item it = decode_item<kMixed>(p, item);
     const int gv = it.gv;
-    scaler.start(icount + 1, (kScalesQ && p.scale_q && item + (int)gridDim.x < p.n_items) ? decode_item(p, item + gridDim.x).gv : 0);
+    scaler.start(icount + 1, (kScalesQ && p.scale_q && item + (int)gridDim.x < p.n_items) ? decode_item<kMixed>(p, item + gridDim.x).gv : 0);
 #pragma unroll 1
     for (int kt = 0; kt < p.n_kt; ++kt) {
 #pragma unroll 1
@@ -655,7 +669,9 @@ __device__ void pv_issuer_role(const Ctx& c, int lane) {
         pready_par ^= 1u << b;
         // the warpgroup's epilogue of the previous item must have read its O accumulators before
         // its first P V of this item overwrites one
-        if (kt == 0 && s < 2) {
+        if (!kMixed) {
+          if (kt == 0 && s < 2 && icount > 0) AF3K_WAIT_WARP_C(c, BarIdx::epi_done + b, (icount - 1) & 1);
+        } else if (kt == 0 && s < 2) {
           if ((epi_seen >> b) & 1u) {
             AF3K_WAIT_WARP_C(c, BarIdx::epi_done + b, (epi_par >> b) & 1u);
             epi_par ^= 1u << b;
@@ -898,7 +914,7 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, float* dbg, int wg, i
   return true;
 }
 
-template <bool kDebug, bool kTcBias, bool kGate>
+template <bool kDebug, bool kTcBias, bool kGate, bool kMixed>
 __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
   const AttnParams& p = *c.p;
   const int row = wq * 32 + lane;                    // row of the 128-query tile == TMEM lane
@@ -917,7 +933,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
 
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
-    const Item it = decode_item(p, item);
+    const Item it = decode_item<kMixed>(p, item);
     // fp32 path: the logit scale the softmax threads apply themselves.  Tensor-core path: the
     // factor from logit differences to exponents of 2 (the scale is in Q already for bf16 q/k)
     float scale = p.scale;
@@ -1049,7 +1065,10 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
 // requests a logits tile), which the hot loops of the roles just overflow (10 misses a tile; code added beside
 // them, with the same work done, took 43 misses and 665 -> 792 us).  83 KB of code -> 55 KB: 389 rows 261 -> 253.5 us
 // a module call, 256 rows of 64 channels 58.2 -> 57.5; 768 rows 672.6 -> 671.0, 1536 tokens 30.5 -> 30.7.
-template <bool kDebug, bool kTcBias, bool kFp8, bool kGate>
+// kMixed: some items have fewer streams than the others (smaller ones behind the last full round, rows or pairs of query
+// tiles that leave a remainder), which takes slots and barriers that an item does not use through their phases and two sets
+// of constants to decode an item.  A plan of equal items runs without: 768 rows 645 -> 636 us.
+template <bool kDebug, bool kTcBias, bool kFp8, bool kGate, bool kMixed>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -1128,17 +1147,17 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     // warps 0-3 need few registers; the two softmax warpgroups take what they give up
     setmaxnreg_dec<kRegsMisc>();
     if (warp == 0) {
-      if (lane == 0) producer_role(c, &tm_q, &tm_k, &tm_v, &tm_bias, &tm_q2, &tm_k2);
+      if (lane == 0) producer_role<kMixed>(c, &tm_q, &tm_k, &tm_v, &tm_bias, &tm_q2, &tm_k2);
     } else if (warp == 1) {
-      qk_issuer_role<kDebug, kTcBias, kFp8>(c);
+      qk_issuer_role<kDebug, kTcBias, kFp8, kMixed>(c);
     } else if (warp == 2) {
-      pv_issuer_role<kDebug, !kFp8>(c, lane);
+      pv_issuer_role<kDebug, !kFp8, kMixed>(c, lane);
     } else if (warp == 3) {
-      if (p.mask_col) mask_writer_role(c, lane);
+      if (p.mask_col) mask_writer_role<kMixed>(c, lane);
     }
   } else {
     setmaxnreg_inc<kRegsSoftmax>();
-    softmax_role<kDebug, kTcBias, kGate>(c, (warp - 4) >> 2, warp & 3, lane);
+    softmax_role<kDebug, kTcBias, kGate, kMixed>(c, (warp - 4) >> 2, warp & 3, lane);
   }
 
   tc_fence_before();
