@@ -1193,9 +1193,9 @@ __device__ __forceinline__ float staged_value(float b, float mul) {
 constexpr int kBiasThreads = 256;
 template <typename T>
 __global__ void __launch_bounds__(kBiasThreads, 8)
-bias_to_bf16_kernel(const T* __restrict__ src, __nv_bfloat16* __restrict__ dst, int B2, int Sq, int Sk, long long src_stride_h,
-                    long long src_stride_r, int pitch, const float* __restrict__ q_scale, const float* __restrict__ k_scale,
-                    float softmax_scale) {
+bias_to_bf16_kernel(const T* src, __nv_bfloat16* dst, int B2, int Sq, int Sk, long long src_stride_h, long long src_stride_r, int pitch,
+                    const float* q_scale, const float* k_scale, float softmax_scale) {
+  // (no __restrict__: it would allow loads of the read-only kind, which need not stay behind the wait)
   grid_wait_previous();
   grid_release_next();
   const uint32_t chunks = (uint32_t)pitch / 8;
