@@ -73,7 +73,7 @@ def dot_product_attention_cpp(
         raise ValueError("BLK_SZ and FLASH_SZ must be positive")
     if q.is_cuda and (mask is None or (mask.dtype is torch.bool and 0 < mask.dim() < 3)) and isinstance(bias, torch.Tensor) and not _DEBUG:
         # the ordinary call, straight to the native path, as below
-        return _capi.host().attention(q, k, v, mask, bias, q_scale, k_scale, None, 0, None, True, False, 0, 0)
+        return _capi.host().attention(q, k, v, mask, bias, q_scale, k_scale, None, 0, None, True, False, 0, 3)
     if not q.is_cuda:
         # host tensors, as the reference takes them: pipelined over PCIe, computed on the GPU,
         # result in host memory

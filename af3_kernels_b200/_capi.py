@@ -30,6 +30,7 @@ EXPORTED_SYMBOLS = (
     "af3k_last_launch_count",
     "af3k_set_wait_limit_cycles",
     "af3k_describe_plan",
+    "af3k_dot_product_attention_convert",
     "af3k_pair_bias_status",
     "af3k_pair_front",
     "af3k_debug_set_dump",
@@ -124,6 +125,8 @@ def load() -> ctypes.CDLL:
     lib.af3k_stage_bias.argtypes = [dp, vp, vp, vp, vp, sz, vp]
     lib.af3k_dot_product_attention.restype = ctypes.c_int
     lib.af3k_dot_product_attention.argtypes = [dp, vp, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp, vp]
+    lib.af3k_dot_product_attention_convert.restype = ctypes.c_int
+    lib.af3k_dot_product_attention_convert.argtypes = [dp, vp, vp, vp, vp, vp, vp, vp, vp]
     lib.af3k_dot_product_attention_noalloc.restype = ctypes.c_int
     lib.af3k_dot_product_attention_noalloc.argtypes = [dp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]
     lib.af3k_static_scratch_bytes.restype = sz

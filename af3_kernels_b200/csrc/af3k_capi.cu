@@ -100,6 +100,7 @@ int device_info(DeviceInfo** out) {
         (const void*)attention_kernel<false, false, true, false, true>,  (const void*)attention_kernel<false, false, true, true, true>,
         (const void*)attention_kernel<true, true, false, false, true>,   (const void*)attention_kernel<true, true, true, false, true>,
         (const void*)attention_kernel<true, false, true, false, true>,
+        (const void*)attention_kernel<false, true, false, false, false, true>, (const void*)attention_kernel<false, true, false, true, false, true>,
     };
     e = cudaSuccess;
     for (const void* kfn : kernels)
@@ -509,10 +510,10 @@ int af3k_stage_bias(const af3k_attention_desc* desc, const void* bias, const flo
   return rc;
 }
 
-int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, const void* k,
-                               const void* v, const void* bias, const uint8_t* mask, void* out,
-                               const float* q_scale, const float* k_scale, void* workspace,
-                               size_t workspace_bytes, int* status_dev, void* stream_v) {
+namespace {
+// convert: the kernel itself may convert the bias
+int attention_call(const af3k_attention_desc* desc, const void* q, const void* k, const void* v, const void* bias, const uint8_t* mask, void* out,
+                   const float* q_scale, const float* k_scale, void* workspace, size_t workspace_bytes, int* status_dev, void* stream_v, bool convert) {
   t_last_launches = 0;
   if (desc == nullptr) return AF3K_ERR_NULL_POINTER;
   const af3k_attention_desc& d = *desc;
@@ -553,7 +554,12 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
   const bool stage_fp8 = fp8 && !d.bias_prescaled && workspace != nullptr && workspace_bytes >= stage_bytes &&
                          aligned16(workspace);
   const bool fp8_tc = fp8 && (d.bias_prescaled || stage_fp8);
-  if (must_stage || stage_fp8) {
+  p.debug = g_debug_dump.load();
+  // the kernel converts the bias itself: items of one query tile, rows that start on vectors or a single key tile
+  const uintptr_t bias_es = d.bias_dtype == AF3K_F32 ? 4 : 2;
+  p.bias_wide = d.Sk % 4 == 0 && (reinterpret_cast<uintptr_t>(bias) | (uintptr_t)bias_sh * bias_es | (uintptr_t)bias_sr * bias_es) % (4 * bias_es) == 0 ? 1 : 0;
+  const bool in_kernel = convert && must_stage && !fp8 && p.n_streams == 1 && !p.mixed && (p.bias_wide || p.n_kt == 1) && p.debug == nullptr;
+  if ((must_stage && !in_kernel) || stage_fp8) {
     if (workspace == nullptr || workspace_bytes < stage_bytes) return AF3K_ERR_WORKSPACE;
     if (!aligned16(workspace)) return AF3K_ERR_BAD_ALIGNMENT;
     const int64_t pitch = staged_bias_pitch(d.Sk);
@@ -566,7 +572,7 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
     bias_sh = pitch * d.Sq;
   }
 
-  CUtensorMap tm_q, tm_k, tm_v, tm_b;
+  CUtensorMap tm_q, tm_k, tm_v, tm_b{};
   if ((rc = encode_qkv_map(&tm_q, q, fp8, d.D, d.Sq, d.B2, d.B1, d.q_stride, p.qk_row_bytes))) return rc;
   if ((rc = encode_qkv_map(&tm_k, k, fp8, d.D, d.Sk, d.B2, d.B1, d.k_stride, p.qk_row_bytes))) return rc;
   if ((rc = encode_qkv_map(&tm_v, v, false, d.D, d.Sk, d.B2, d.B1, d.v_stride, p.v_row_bytes))) return rc;
@@ -574,7 +580,12 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
   if (p.qk_narrow && ((rc = encode_qkv_map(&tm_q2, q, fp8, d.D, d.Sq, d.B2, d.B1, d.q_stride, 32)) ||
                       (rc = encode_qkv_map(&tm_k2, k, fp8, d.D, d.Sk, d.B2, d.B1, d.k_stride, 32))))
     return rc;
-  if ((rc = encode_bias_map(&tm_b, bias_base, d.Sk, d.Sq, d.B2, bias_sh, bias_sr))) return rc;
+  if (in_kernel) {
+    p.bias_src = bias;
+    p.bias_stride_h = bias_sh;
+    p.bias_stride_r = bias_sr;
+    p.bias_f32 = bias_es == 4 ? 1 : 0;
+  } else if ((rc = encode_bias_map(&tm_b, bias_base, d.Sk, d.Sq, d.B2, bias_sh, bias_sr))) return rc;
 
   p.q_scale = q_scale;
   p.k_scale = k_scale;
@@ -592,7 +603,6 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
   p.status = status_dev;
   p.wait_limit = wait_limit_cycles();
 
-  p.debug = g_debug_dump.load();
   // scale, bias and mask all come out of the tensor core, except for fp8 q/k without a staging
   // copy of the bias: there the softmax threads apply scale and bias in fp32
   const bool tc_bias = !fp8 || fp8_tc;
@@ -600,7 +610,10 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
   const bool dbg = p.debug != nullptr;
 #define AF3K_LAUNCH_AS(...) launch_overlapped(attention_kernel<__VA_ARGS__>, dim3(plan.grid), kThreads, plan.smem_bytes, stream, d.max_ctas <= 0, p, tm_q, tm_k, tm_v, tm_b, tm_q2, tm_k2)
 #define AF3K_LAUNCH(...) (p.mixed ? AF3K_LAUNCH_AS(__VA_ARGS__, true) : AF3K_LAUNCH_AS(__VA_ARGS__, false))
-  if (p.gate != nullptr) {
+  if (in_kernel) {
+    if (p.gate != nullptr) AF3K_LAUNCH_AS(false, true, false, true, false, true);
+    else                   AF3K_LAUNCH_AS(false, true, false, false, false, true);
+  } else if (p.gate != nullptr) {
     if (!fp8)         AF3K_LAUNCH(false, true, false, true);
     else if (tc_bias) AF3K_LAUNCH(false, true, true, true);
     else              AF3K_LAUNCH(false, false, true, true);
@@ -620,6 +633,20 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
   ++launches;
   t_last_launches = launches;
   return AF3K_OK;
+}
+
+}  // namespace
+
+int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, const void* k,
+                               const void* v, const void* bias, const uint8_t* mask, void* out,
+                               const float* q_scale, const float* k_scale, void* workspace,
+                               size_t workspace_bytes, int* status_dev, void* stream) {
+  return attention_call(desc, q, k, v, bias, mask, out, q_scale, k_scale, workspace, workspace_bytes, status_dev, stream, false);
+}
+
+int af3k_dot_product_attention_convert(const af3k_attention_desc* desc, const void* q, const void* k, const void* v, const void* bias,
+                                       const uint8_t* mask, void* out, int* status_dev, void* stream) {
+  return attention_call(desc, q, k, v, bias, mask, out, nullptr, nullptr, nullptr, 0, status_dev, stream, true);
 }
 
 void af3k_debug_set_dump(float* dump_dev) { g_debug_dump.store(dump_dev); }

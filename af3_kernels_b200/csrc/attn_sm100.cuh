@@ -48,6 +48,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <type_traits>
 
 #include "ptx_sm100.cuh"
 
@@ -144,6 +145,10 @@ struct AttnParams {
   //   (key, 0) = mask value;  off_zero: the all-zero second half of K shared by both.
   uint32_t off_ones, off_mcol, off_zero;
   uint32_t off_ident;    // 16 x 16 identity (B operand of the bias MMAs)
+  // kConvert: the bias as the caller holds it
+  const void* bias_src;
+  long long bias_stride_h, bias_stride_r;
+  int bias_f32, bias_wide;   // bias_wide: rows start on boundaries of four keys and end there
   int mask_col;          // 1: the extra K step runs (a mask was given or Sk is not a tile multiple)
 };
 
@@ -292,7 +297,7 @@ __device__ __forceinline__ uint32_t q_buf(const AttnParams& p, uint32_t j) { ret
 __device__ __forceinline__ uint32_t q_use(const AttnParams& p, uint32_t j) { return p.q_buffers == 2 ? (j >> 1) : j; }
 
 // ------------------------------------------------------------------ producer (one thread)
-template <bool kMixed>
+template <bool kMixed, bool kConvert>
 __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUtensorMap* tm_k,
                               const CUtensorMap* tm_v, const CUtensorMap* tm_bias, const CUtensorMap* tm_q2, const CUtensorMap* tm_k2) {
   const AttnParams& p = *c.p;
@@ -330,7 +335,7 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
     for (int kt = 0; kt < p.n_kt; ++kt) {
 #pragma unroll 1
       for (int s = 0; s < it.gv; ++s) {
-        if (s == 0 || p.q_split) {   // one bias tile per key tile, or per stream when the streams are query tiles
+        if (!kConvert && (s == 0 || p.q_split)) {   // one bias tile per key tile, or per stream when the streams are query tiles
           const uint32_t bst = bcount % kBiasStages;
           if (bcount >= kBiasStages)
             AF3K_WAIT(c, BarIdx::bias_empty + bst, ((bcount / kBiasStages) - 1) & 1);
@@ -1057,6 +1062,136 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
   }
 }
 
+// ------------------------------------------------------------------ bias converted in the kernel
+// Two keys' bias in bf16.  What bf16 cannot hold (fp32's lowest value, a quotient, an infinity) becomes its largest value of
+// that sign: the tensor core adds a slice of the bias by products with 1 and 0, and an infinity times 0 would make NaN of the 15
+// keys beside it.  NaN stays.
+__device__ __forceinline__ uint32_t staged_pair(float a, float b) {
+  uint32_t w = pack_bf16x2(a, b);
+  asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(w) : "r"(0xff7fff7fu));
+  asm("min.NaN.bf16x2 %0, %0, %1;" : "+r"(w) : "r"(0x7f7f7f7fu));
+  return w;
+}
+
+constexpr int kConvertRows = 16;   // rows of a tile in one round of loads
+
+// A load with a predicate and without a branch, so that many are out at once.
+__device__ __forceinline__ float load_if(const float* a, uint32_t there) {
+  float x = 0.f;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.f32 %0, [%1];\n\t}" : "+f"(x) : "l"(a), "r"(there));
+  return x;
+}
+__device__ __forceinline__ float load_if(const uint16_t* a, uint32_t there) {
+  uint16_t x = 0;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.u16 %0, [%1];\n\t}" : "+h"(x) : "l"(a), "r"(there));
+  return __uint_as_float((uint32_t)x << 16);
+}
+
+// One row's keys 4 lane .. 4 lane + 3 into a staged tile: two boxes of 64 keys, rows of 128 bytes, 128-byte swizzle.
+__device__ __forceinline__ void store_bias4(uint32_t tile, int row, int lane, uint32_t w0, uint32_t w1) {
+  const uint32_t at = tile + row * 128 + (lane >> 4) * (kBiasTileBytes / 2) + (lane & 1) * 8 + ((((lane >> 1) & 7) ^ (row & 7)) << 4);
+  asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at), "r"(w0), "r"(w1) : "memory");
+}
+
+// kConvert: the softmax warpgroup that has no stream in items of one makes the bias tiles of the other, from fp32 or from
+// bf16 rows that TMA cannot address, in place of the producer's loads.  Otherwise such a call takes a launch more, and for a
+// short call that is a good part of it.  us, bias in place / converted here / in a pass before, 16 heads, fp32: 77 tokens 5.4 / 5.7
+// / 6.8, 512 9.0 / 10.1 / 13.5, 1000 14.4 / 17.3 / 26.6.  A warp takes 32 rows of a tile, a lane four keys of each.  What does
+// not exist takes the bias of a row or key that does, or anything: of such rows nothing is stored, such keys are at -inf.
+//
+// Rows that start on vectors (bias_wide): 16 rows' loads for the next tile follow directly on their store for this one, so that
+// 32 rows' are out nearly all the time.  The warp is alone on its scheduler beside a softmax warp that streams through its code, so the
+// loop is kept short: with a test for infinities and a second pass behind it 512 tokens took 11.4 us.
+template <bool kF32>
+__device__ void bias_convert_role(const Ctx& c, int wq, int lane) {
+  const AttnParams& p = *c.p;
+  constexpr int es = kF32 ? 4 : 2;
+  using Vec = typename std::conditional<kF32, float4, uint2>::type;
+  const int row0 = wq * 32;
+  const long long step = p.bias_stride_r * es;
+  Vec x[2][kConvertRows];
+  auto load = [&](const Item& it, int kt, int half) {
+    const int first = it.qt * kTile + row0, last = min(31, p.Sq - 1 - first);
+    if (last < 0) return;
+    const char* src = static_cast<const char*>(p.bias_src) + (it.h * p.bias_stride_h + first * p.bias_stride_r + min(kt * kTile + 4 * lane, p.Sk - 4)) * es;
+#pragma unroll
+    for (int r = 0; r < kConvertRows; ++r) x[half][r] = *reinterpret_cast<const Vec*>(src + min(half * kConvertRows + r, last) * step);
+  };
+  auto store = [&](uint32_t tile, int half) {
+#pragma unroll
+    for (int r = 0; r < kConvertRows; ++r) {
+      uint32_t w0, w1;
+      if constexpr (kF32) {
+        w0 = staged_pair(x[half][r].x, x[half][r].y);
+        w1 = staged_pair(x[half][r].z, x[half][r].w);
+      } else {
+        w0 = staged_pair(__uint_as_float(x[half][r].x << 16), __uint_as_float(x[half][r].x & 0xffff0000u));
+        w1 = staged_pair(__uint_as_float(x[half][r].y << 16), __uint_as_float(x[half][r].y & 0xffff0000u));
+      }
+      store_bias4(tile, row0 + half * kConvertRows + r, lane, w0, w1);
+    }
+  };
+  int item = blockIdx.x, kt = 0;
+  Item it = decode_item<false>(p, item);     // (the grid has no more blocks than items)
+#pragma unroll
+  for (int half = 0; half < 2; ++half) load(it, 0, half);
+#pragma unroll 1
+  for (uint32_t n = 0; item < p.n_items; ++n) {
+    const uint32_t bst = n % kBiasStages;
+    const uint32_t tile = c.smem + p.off_bias + bst * kBiasTileBytes;
+    // the bias MMAs of the stage's tile before must have finished
+    if (n >= kBiasStages) AF3K_WAIT_WARP(c, BarIdx::bias_empty + bst, ((n / kBiasStages) - 1) & 1);
+    if (++kt == p.n_kt) {                    // the tile after this one
+      kt = 0;
+      item += gridDim.x;
+      if (item < p.n_items) it = decode_item<false>(p, item);
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      store(tile, half);
+      if (item < p.n_items) load(it, kt, half);
+    }
+    fence_proxy_async_smem();    // make the generic-proxy stores visible to the tensor core
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::bias_full + bst));
+  }
+}
+
+// Rows that start anywhere, for items of one key tile: with more of them a pass of its own over the bias is faster (389 tokens
+// of ragged rows 12.7 us with it, 13.9 so).
+template <typename T>
+__device__ void bias_convert_ragged_role(const Ctx& c, int wq, int lane) {
+  const AttnParams& p = *c.p;
+  const int row0 = wq * 32;
+  uint32_t n = 0;
+#pragma unroll 1
+  for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
+    const Item it = decode_item<false>(p, item);
+#pragma unroll 1
+    for (int kt = 0; kt < p.n_kt; ++kt, ++n) {
+      const uint32_t bst = n % kBiasStages;
+      const uint32_t tile = c.smem + p.off_bias + bst * kBiasTileBytes;
+      const int first = it.qt * kTile + row0, last = min(31, p.Sq - 1 - first), key = kt * kTile + 4 * lane;
+      const T* src = static_cast<const T*>(p.bias_src) + it.h * p.bias_stride_h + first * p.bias_stride_r + key;
+#pragma unroll 1
+      for (int r0 = 0; r0 < 32; r0 += kConvertRows) {
+        float x[kConvertRows][4];
+#pragma unroll
+        for (int r = 0; r < kConvertRows; ++r)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[r][e] = load_if(src + min(r0 + r, last) * p.bias_stride_r + e, last >= 0 && key + e < p.Sk ? 1u : 0u);
+        if (r0 == 0 && n >= kBiasStages) AF3K_WAIT_WARP(c, BarIdx::bias_empty + bst, ((n / kBiasStages) - 1) & 1);
+#pragma unroll
+        for (int r = 0; r < kConvertRows; ++r)
+          store_bias4(tile, row0 + r0 + r, lane, staged_pair(x[r][0], x[r][1]), staged_pair(x[r][2], x[r][3]));
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::bias_full + bst));
+    }
+  }
+}
+
 // ------------------------------------------------------------------ kernel
 // kGate: the result is multiplied by sigmoid(gate).  A template argument, because a run-time test of the pointer
 // cost calls without a gate 0.9 % (768 rows of 768 keys: 671 -> 677 us).
@@ -1068,12 +1203,14 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
 // kMixed: some items have fewer streams than the others (smaller ones behind the last full round, rows or pairs of query
 // tiles that leave a remainder), which takes slots and barriers that an item does not use through their phases and two sets
 // of constants to decode an item.  A plan of equal items runs without: 768 rows 645 -> 636 us.
-template <bool kDebug, bool kTcBias, bool kFp8, bool kGate, bool kMixed>
+// kConvert: plans of one stream per item, bf16 q and k; see bias_convert_role.
+template <bool kDebug, bool kTcBias, bool kFp8, bool kGate, bool kMixed, bool kConvert = false>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                  const __grid_constant__ CUtensorMap tm_bias, const __grid_constant__ CUtensorMap tm_q2,
                  const __grid_constant__ CUtensorMap tm_k2) {
+  static_assert(!kConvert || (kTcBias && !kFp8 && !kMixed), "the bias is converted for bf16 q and k and equal items only");
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
@@ -1092,7 +1229,7 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     prefetch_tensormap(&tm_q);
     prefetch_tensormap(&tm_k);
     prefetch_tensormap(&tm_v);
-    prefetch_tensormap(&tm_bias);
+    if (!kConvert) prefetch_tensormap(&tm_bias);
     for (int i = 0; i < 2 * kMaxStreams; ++i) {
       mbar_init(bar_addr(c, BarIdx::q_full + i), 1);
       mbar_init(bar_addr(c, BarIdx::q_empty + i), 1);
@@ -1105,7 +1242,7 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
       mbar_init(bar_addr(c, BarIdx::p_ready + i), 4);
     }
     for (int i = 0; i < kBiasStages; ++i) {
-      mbar_init(bar_addr(c, BarIdx::bias_full + i), 1);
+      mbar_init(bar_addr(c, BarIdx::bias_full + i), kConvert ? 4 : 1);
       // freed by the bias MMAs' completion (bf16 q/k) or by the eight softmax warps (fp8 q/k)
       mbar_init(bar_addr(c, BarIdx::bias_empty + i), kTcBias ? 1 : 8);
     }
@@ -1147,7 +1284,7 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     // warps 0-3 need few registers; the two softmax warpgroups take what they give up
     setmaxnreg_dec<kRegsMisc>();
     if (warp == 0) {
-      if (lane == 0) producer_role<kMixed>(c, &tm_q, &tm_k, &tm_v, &tm_bias, &tm_q2, &tm_k2);
+      if (lane == 0) producer_role<kMixed, kConvert>(c, &tm_q, &tm_k, &tm_v, &tm_bias, &tm_q2, &tm_k2);
     } else if (warp == 1) {
       qk_issuer_role<kDebug, kTcBias, kFp8, kMixed>(c);
     } else if (warp == 2) {
@@ -1157,7 +1294,17 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     }
   } else {
     setmaxnreg_inc<kRegsSoftmax>();
-    softmax_role<kDebug, kTcBias, kGate, kMixed>(c, (warp - 4) >> 2, warp & 3, lane);
+    if (kConvert && warp >= 8) {
+      if (p.bias_wide) {
+        if (p.bias_f32) bias_convert_role<true>(c, warp & 3, lane);
+        else            bias_convert_role<false>(c, warp & 3, lane);
+      } else {
+        if (p.bias_f32) bias_convert_ragged_role<float>(c, warp & 3, lane);
+        else            bias_convert_ragged_role<uint16_t>(c, warp & 3, lane);
+      }
+    } else {
+      softmax_role<kDebug, kTcBias, kGate, kMixed>(c, (warp - 4) >> 2, warp & 3, lane);
+    }
   }
 
   tc_fence_before();
@@ -1178,14 +1325,7 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
 // With fp8 q/k (q_scale / k_scale given) every value is divided by the head's logit scale
 // softmax_scale * q_scale[h] * k_scale[h]: the tensor core then adds it to the raw fp8 products
 // and the softmax threads apply that scale to the sum.
-// What bf16 cannot hold (fp32's lowest value, a quotient, -inf) becomes bf16's largest value of its sign: the tensor core
-// adds a slice of the bias by products with 1 and 0, and an infinity times 0 would make NaN of the 15 keys beside it.
-// +inf and NaN stay, as the softmax of such a row is not a number either.
-__device__ __forceinline__ float staged_value(float b, float mul) {
-  const float x = b * mul;
-  return b < INFINITY ? fminf(fmaxf(x, -3.38953139e38f), 3.38953139e38f) : x;
-}
-
+// (staged_pair says what becomes of values that bf16 cannot hold.)
 // One thread converts eight columns, two 16-byte loads where every row starts on a 16-byte boundary (else one by one) and one
 // 16-byte store, as many blocks as stay resident: it is bound by memory, and a call that converts pays it in full.
 // Two columns a thread, with two 64-bit divisions for each pair, against this, us: 16 heads of 512 x 512 fp32 11.3 -> 4.9 (5.2
@@ -1227,7 +1367,7 @@ bias_to_bf16_kernel(const T* src, __nv_bfloat16* dst, int B2, int Sq, int Sk, lo
     const float mul = q_scale != nullptr ? 1.0f / (softmax_scale * q_scale[h] * k_scale[h]) : 1.0f;
     uint32_t o[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) o[e] = pack_bf16x2(staged_value(x[2 * e], mul), staged_value(x[2 * e + 1], mul));
+    for (int e = 0; e < 4; ++e) o[e] = staged_pair(x[2 * e] * mul, x[2 * e + 1] * mul);
     reinterpret_cast<uint4*>(dst)[i] = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }

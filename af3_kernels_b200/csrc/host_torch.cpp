@@ -30,6 +30,7 @@ using OptTensor = std::optional<Tensor>;
 // ------------------------------------------------------------------ library and errors
 struct Library {
   decltype(&af3k_dot_product_attention) attention = nullptr;
+  decltype(&af3k_dot_product_attention_convert) attention_convert = nullptr;
   decltype(&af3k_dot_product_attention_workspace) workspace = nullptr;
   decltype(&af3k_stage_bias) stage_bias = nullptr;
   decltype(&af3k_grid_front_weights) grid_front = nullptr;
@@ -51,6 +52,7 @@ void bind_library(const std::string& path) {
   };
 #define AF3K_BIND(field, name) g_lib.field = reinterpret_cast<decltype(g_lib.field)>(find(#name))
   AF3K_BIND(attention, af3k_dot_product_attention);
+  AF3K_BIND(attention_convert, af3k_dot_product_attention_convert);
   AF3K_BIND(workspace, af3k_dot_product_attention_workspace);
   AF3K_BIND(stage_bias, af3k_stage_bias);
   AF3K_BIND(grid_front, af3k_grid_front_weights);
@@ -121,12 +123,16 @@ Tensor bias_3d(const Tensor& bias, int64_t B2, int64_t Sq, int64_t Sk) {
   return bias.sizes() == at::IntArrayRef(sizes, 3) ? bias : bias.reshape(sizes);
 }
 
-Tensor make_staged(const Tensor& bias_in, int64_t B2, int64_t Sq, int64_t Sk, int64_t D, const float* q_scale,
-                   const float* k_scale, float scale, cudaStream_t stream) {
-  Tensor bias = bias_in;
+// The bias as the library takes it: bf16 or fp32, [B2, Sq, Sk], rows of any pitch.
+Tensor plain_bias(Tensor bias, int64_t B2, int64_t Sq, int64_t Sk) {
   if (bias.scalar_type() != at::kBFloat16 && bias.scalar_type() != at::kFloat) bias = bias.to(at::kFloat);
   bias = bias_3d(bias, B2, Sq, Sk);
-  if ((Sk > 1 && bias.stride(2) != 1) || (B2 > 1 && bias.stride(0) == 0) || (Sq > 1 && bias.stride(1) == 0)) bias = bias.contiguous();
+  return (Sk > 1 && bias.stride(2) != 1) || (B2 > 1 && bias.stride(0) == 0) || (Sq > 1 && bias.stride(1) == 0) ? bias.contiguous() : bias;
+}
+
+Tensor make_staged(const Tensor& bias_in, int64_t B2, int64_t Sq, int64_t Sk, int64_t D, const float* q_scale,
+                   const float* k_scale, float scale, cudaStream_t stream) {
+  const Tensor bias = plain_bias(bias_in, B2, Sq, Sk);
   af3k_attention_desc d{};
   d.B1 = 1; d.B2 = B2; d.Sq = Sq; d.Sk = Sk; d.D = (D + 15) / 16 * 16;
   const int64_t most = std::max(Sq, Sk) * 64;
@@ -194,7 +200,8 @@ void check_mask(const Tensor& mask, int64_t B1, int64_t Sk) {
     value_error("mask of shape " + shape_text(mask) + " does not match B1=" + std::to_string(B1) + ", Sk=" + std::to_string(Sk));
 }
 
-// bias_form: 0 an ordinary bias tensor, 1 the copy of a StagedBias, 2 the same divided by fp8 scales
+// bias_form: 0 an ordinary bias tensor, 1 the copy of a StagedBias, 2 the same divided by fp8 scales, 3 an ordinary one that
+// the kernel may convert itself
 Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor bias, const OptTensor& q_scale_in,
                  const OptTensor& k_scale_in, std::optional<double> softmax_scale, int64_t rows_per_item, const OptTensor& out_in,
                  bool use_workspace, bool cache_bias, int64_t max_ctas, int64_t bias_form, int* status = nullptr) {
@@ -230,7 +237,7 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
   const float scale = softmax_scale ? (float)*softmax_scale : (float)(1.0 / std::sqrt((double)D));
 
   bool prescaled = bias_form == 2;
-  if (bias_form == 0) {
+  if (bias_form == 0 || bias_form == 3) {
     if (bias.numel() != B2 * Sq * Sk) {
       value_error("bias must have B2*Sq*Sk = " + std::to_string(B2 * Sq * Sk) + " elements, got " + std::to_string(bias.numel()));
     }
@@ -242,9 +249,7 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
                          fp8 ? q_scale.data_ptr<float>() : nullptr, fp8 ? k_scale.data_ptr<float>() : nullptr, scale);
       prescaled = fp8;
     } else {
-      if (bias.scalar_type() != at::kBFloat16 && bias.scalar_type() != at::kFloat) bias = bias.to(at::kFloat);
-      bias = bias_3d(bias, B2, Sq, Sk);
-      if ((Sk > 1 && bias.stride(2) != 1) || (B2 > 1 && bias.stride(0) == 0) || (Sq > 1 && bias.stride(1) == 0)) bias = bias.contiguous();
+      bias = plain_bias(bias, B2, Sq, Sk);
     }
   }
   q = inner_contiguous(q); k = inner_contiguous(k); v = inner_contiguous(v);
@@ -285,16 +290,24 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
   d.rows_per_item = (int32_t)rows_per_item;
   d.bias_prescaled = prescaled ? 1 : 0;
   d.max_ctas = (int32_t)max_ctas;
+  const uint8_t* mask_data = mask.defined() ? static_cast<const uint8_t*>(mask.data_ptr()) : nullptr;
+  int* const status_data = status != nullptr ? status : status_buffer(dev.index()).data_ptr<int>();
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  if (bias_form == 3 && !fp8) {
+    const int rc = g_lib.attention_convert(&d, q.data_ptr(), k.data_ptr(), v.data_ptr(), bias.data_ptr(), mask_data, out.data_ptr(), status_data, stream);
+    if (rc != AF3K_ERR_WORKSPACE) {
+      check(rc);
+      return f32_result ? out.to(at::kFloat) : out;
+    }
+  }
   Tensor ws;
   if (use_workspace) {
     const size_t bytes = g_lib.workspace(&d, bias.data_ptr());
     if (bytes != 0) ws = at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(dev));
   }
-  check(g_lib.attention(&d, q.data_ptr(), k.data_ptr(), v.data_ptr(), bias.data_ptr(),
-                        mask.defined() ? static_cast<const uint8_t*>(mask.data_ptr()) : nullptr, out.data_ptr(),
-                        fp8 ? q_scale.data_ptr<float>() : nullptr, fp8 ? k_scale.data_ptr<float>() : nullptr,
+  check(g_lib.attention(&d, q.data_ptr(), k.data_ptr(), v.data_ptr(), bias.data_ptr(), mask_data, out.data_ptr(), fp8 ? q_scale.data_ptr<float>() : nullptr, fp8 ? k_scale.data_ptr<float>() : nullptr,
                         ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? (size_t)ws.numel() : 0,
-                        status != nullptr ? status : status_buffer(dev.index()).data_ptr<int>(), c10::cuda::getCurrentCUDAStream(dev.index())));
+                        status_data, stream));
   return f32_result ? out.to(at::kFloat) : out;
 }
 
@@ -455,7 +468,7 @@ Tensor grid_block(const Tensor& pair, const OptTensor& mask, const Tensor& bias,
   int* status = status_buffer(dev.index()).data_ptr<int>();
   check(g_lib.grid_front(x.data_ptr(), AF3K_BF16, &w.front, 0.f, 0, R, N, C, head, 1.0f / std::sqrt((float)D), 0, nullptr, 0, q.data_ptr(),
                          k.data_ptr(), v.data_ptr(), gate.data_ptr(), status, stream));
-  attention(q, k, v, mask, bias, std::nullopt, std::nullopt, 1.0, 0, weighted.permute({0, 2, 1, 3}), true, false, 0, 0);
+  attention(q, k, v, mask, bias, std::nullopt, std::nullopt, 1.0, 0, weighted.permute({0, 2, 1, 3}), true, false, 0, 3);
   if (!project) check(g_lib.sigmoid_gate(weighted.data_ptr(), gate.data_ptr(), out.data_ptr(), M * C, stream));
   else check(g_lib.grid_out(weighted.data_ptr(), gate.data_ptr(), w.wo, w.front.w_dtype, out.data_ptr(), pair.scalar_type() == at::kFloat ? AF3K_F32 : AF3K_BF16,
                        M, C, status, stream));
@@ -501,7 +514,7 @@ Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, con
   const bool in_place = bias.scalar_type() == at::kBFloat16 && bias.dim() == 3 && bias.size(0) == head && bias.size(1) == N && bias.stride(2) == 1 && (bias.stride(1) * 2) % 16 == 0 &&
                         (bias.stride(0) * 2) % 16 == 0 && (bias.stride(0) != 0 || head == 1) && (bias.stride(1) != 0 || N == 1) &&
                         reinterpret_cast<uintptr_t>(bias.data_ptr()) % 16 == 0;
-  if (!in_place) bias = make_staged(bias, head, N, N, D, nullptr, nullptr, scale, stream);
+  if (!in_place) bias = plain_bias(bias, head, N, N);
   Tensor mask;
   if (mask_in) {
     if (mask_in->numel() != N) value_error("mask of shape " + shape_text(*mask_in) + " does not match B1=1, Sk=" + std::to_string(N));
@@ -516,12 +529,21 @@ Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, con
   af3k_attention_desc d{};
   d.B1 = 1; d.B2 = head; d.Sq = N; d.Sk = N; d.D = D;
   for (int64_t* st : {d.q_stride, d.k_stride, d.v_stride, d.out_stride, d.gate_stride}) { st[0] = N * C; st[1] = D; st[2] = C; }
-  d.bias_stride[0] = bias.stride(0); d.bias_stride[1] = bias.stride(1);
-  d.qk_dtype = AF3K_BF16; d.bias_dtype = AF3K_BF16;
+  d.qk_dtype = AF3K_BF16;
   d.softmax_scale = 1.0f;                            // q left the projection scaled
   d.gate = b + 3 * part;
-  check(g_lib.attention(&d, b, b + part, b + 2 * part, bias.data_ptr(), mask.defined() ? static_cast<const uint8_t*>(mask.data_ptr()) : nullptr,
-                        out.data_ptr(), nullptr, nullptr, nullptr, 0, status, stream));
+  const auto call = [&] {
+    d.bias_stride[0] = bias.stride(0); d.bias_stride[1] = bias.stride(1);
+    d.bias_dtype = dtype_code(bias);
+    return g_lib.attention_convert(&d, b, b + part, b + 2 * part, bias.data_ptr(), mask.defined() ? static_cast<const uint8_t*>(mask.data_ptr()) : nullptr,
+                                   out.data_ptr(), status, stream);
+  };
+  int rc = call();
+  if (rc == AF3K_ERR_WORKSPACE) {
+    bias = make_staged(bias, head, N, N, D, nullptr, nullptr, scale, stream);
+    rc = call();
+  }
+  check(rc);
   return x_in.scalar_type() == at::kBFloat16 ? out : out.to(x_in.scalar_type());
 }
 

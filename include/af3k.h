@@ -125,6 +125,14 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
                                const float* q_scale, const float* k_scale, void* workspace,
                                size_t workspace_bytes, int* status_dev, void* stream);
 
+/* The same operation with bf16 q/k in one launch, without a workspace: where every work item has one query tile (small
+ * calls), and Sk is at most 128 or the bias rows start and end on groups of four keys, the kernel converts an fp32 or
+ * ragged bias itself, from where it is.  AF3K_ERR_WORKSPACE, and nothing is launched, where the bias needs converting and
+ * that does not hold: then use af3k_dot_product_attention.  The results are the same bits.  No counterpart in the
+ * reference. */
+int af3k_dot_product_attention_convert(const af3k_attention_desc* desc, const void* q, const void* k, const void* v,
+                                       const void* bias, const uint8_t* mask, void* out, int* status_dev, void* stream);
+
 /* The same operation for callers that cannot supply a workspace and cannot allocate one: a
  * host that handed all device memory to its own arena at start-up, a plug-in boundary that only
  * carries inputs and outputs, or a serving loop where cudaMalloc (which synchronises the whole

@@ -4,6 +4,7 @@ tolerances of the bf16 path; forms that only deal the same work out differently 
 import pytest
 import torch
 
+import af3_kernels_b200 as A
 from af3_kernels_b200 import _capi
 from af3_kernels_b200.dpa import dot_product_attention, stage_bias
 from oracle import attention_oracle as O
@@ -133,10 +134,51 @@ def test_conversion_of_the_bias(cuda_device, Sk, pitch, offset, dtype):
         assert torch.equal(got[:, :, :Sk], want.to(torch.bfloat16)) and not got[:, :, Sk:].any()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B1,B2,Sq,Sk,D,pitch,offset", [
+    (1, 16, 77, 77, 24, 77, 0), (1, 16, 512, 512, 32, 516, 4), (1, 3, 129, 131, 64, 131, 0), (2, 16, 300, 300, 48, 300, 0), (1, 2, 1, 1, 8, 1, 0),
+    (1, 5, 130, 385, 32, 388, 8), (1, 5, 130, 388, 32, 388, 8), (1, 4, 127, 640, 40, 644, 3), (1, 4, 127, 640, 40, 644, 4), (1, 4, 250, 100, 32, 100, 0),
+    (1, 300, 100, 260, 16, 260, 0), (1, 300, 100, 99, 16, 99, 0), (1, 16, 1100, 1100, 24, 1100, 0)])
+def test_bias_converted_by_the_attention_kernel(cuda_device, B1, B2, Sq, Sk, D, pitch, offset, dtype):
+    """Items of one query tile (several to a CTA with 300 heads), rows that start on four keys or a single key tile: one
+    launch, the same bits as with a pass of its own over the bias; -inf and the lowest value included.  Otherwise that pass."""
+    q, k, v, mask, _ = _inputs(B1, B2, Sq, D, Sk, Sk)
+    g = torch.Generator().manual_seed(Sk)
+    mask[:, -1] = True
+    flat = torch.randn(B2 * Sq * pitch + 16, generator=g)
+    bias = flat[offset:offset + B2 * Sq * pitch].view(B2, Sq, pitch)[:, :, :Sk]
+    bias[torch.rand(bias.shape, generator=g) < 0.05] = -float("inf")
+    bias[:, Sq // 2] = torch.finfo(dtype).min
+    bias[..., -1] = 0
+    on_dev = flat.to(cuda_device, dtype)
+    bias = on_dev[offset:offset + B2 * Sq * pitch].view(B2, Sq, pitch)[:, :, :Sk]
+    args = [t.to(cuda_device) for t in (q, k, v, mask)]
+    lib = _capi.load()
+    out = A.dot_product_attention_cpp(*args, bias)
+    in_kernel = Sk <= 128 or (Sk % 4 == 0 and pitch % 4 == 0 and offset % 4 == 0)
+    assert lib.af3k_last_launch_count() == (1 if in_kernel else 2)
+    staged = dot_product_attention(*args, bias, cache_bias=False, check_status=True)
+    assert lib.af3k_last_launch_count() == 2
+    assert torch.equal(out, staged)
+    _check(out.cpu(), O.oracle_fp32(q, k, v, mask, bias.cpu()), (B1, B2, Sq, Sk, D))
+
+
+@pytest.mark.parametrize("N", [77, 500, 1300])
+def test_single_block_converts_its_bias(cuda_device, N):
+    """With the gate: the same bits as with the bf16 bias in rows of 16 bytes, within the kernel's own conversion and beyond."""
+    g = torch.Generator().manual_seed(N)
+    H, C = 4, 96
+    x, w = torch.randn(N, C, generator=g).to(cuda_device, torch.bfloat16), [(torch.randn(C, C, generator=g) * 0.1).to(cuda_device, torch.bfloat16) for _ in range(4)]
+    bias = torch.randn(H, N, N, generator=g).to(cuda_device)
+    mask = (torch.rand(N, generator=g) >= 0.1).to(cuda_device)
+    block = lambda b: A.self_attention_cpp(x, mask, b, w[0], torch.zeros(C, device=cuda_device), *w[1:], H)
+    assert torch.equal(block(bias), block(stage_bias(bias, H, N, N).data[:, :, :N]))
+
+
 @pytest.mark.parametrize("dtype,Sk", [(torch.float32, 392), (torch.bfloat16, 389)])
 def test_minus_infinity_in_a_bias_that_is_converted(cuda_device, dtype, Sk):
-    """fp32 or ragged rows: keys with a bias of -inf have no weight, the keys beside them keep theirs; +inf and NaN still
-    make their row NaN and no other."""
+    """fp32 or ragged rows: keys with a bias of -inf have no weight, a key with +inf has all of it, the keys beside them keep
+    theirs; NaN still makes its row NaN and no other."""
     q, k, v, mask, bias = _inputs(3, 2, 200, 32, 8, Sk)
     bias = bias.to(dtype)
     g = torch.Generator().manual_seed(3)
@@ -145,10 +187,10 @@ def test_minus_infinity_in_a_bias_that_is_converted(cuda_device, dtype, Sk):
     mask[:, -1], bias[..., -1] = True, 0
     ref = O.oracle_fp32(q, k, v, mask, bias)
     _check(_call(cuda_device, q, k, v, mask, bias), ref, "-inf")
-    for n, value in enumerate((float("inf"), float("nan"))):
-        bias[:, 20 + n, Sk - 1] = value
-    nan = torch.isnan(_call(cuda_device, q, k, v, mask, bias)).all(-1).all(0).all(0)
-    assert nan.nonzero().flatten().tolist() == [20, 21]
+    bias[:, 20, Sk - 1], bias[:, 21, Sk - 1] = float("inf"), float("nan")
+    out = _call(cuda_device, q, k, v, mask, bias)
+    assert torch.isnan(out).any(-1).any(0).any(0).nonzero().flatten().tolist() == [21]
+    assert torch.equal(out[:, :, 20], v[:, :, Sk - 1])
 
 
 @pytest.mark.parametrize("value", [0, -38 * 2 ** 12, -152 * 2 ** 14, -152 * 2 ** 16, 152 * 2 ** 16])
