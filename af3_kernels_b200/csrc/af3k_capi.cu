@@ -440,7 +440,7 @@ int static_scratch_address(void** out) {
 
 extern "C" {
 
-int af3k_version(void) { return 1004; }
+int af3k_version(void) { return 1005; }
 
 const char* af3k_strerror(int code) {
   switch (code) {

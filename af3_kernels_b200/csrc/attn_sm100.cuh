@@ -117,7 +117,7 @@ struct AttnParams {
   int qk_row_bytes;      // smem bytes per Q / K tile row: 32, 64 or 128 (= swizzle span)
   // 1: bf16 heads of 33 to 48 channels.  A Q / K tile is 32 channels in rows of 64 bytes, then 16 in rows of 32 bytes: 12 KB
   // instead of the 16 KB of 128-byte rows, which makes room for a fourth K/V stage beside two streams' Q tiles (three stages
-  // do not cover the loads' latency; 5 x 16 heads x 1536 tokens x 48 channels: 111.1 -> 99.6 us a call).  V keeps its
+  // do not cover the loads' latency; 5 x 16 heads x 1536 tokens x 48 channels: 112 -> 99 us a call).  V keeps its
   // 128-byte rows: it is an MN-major operand, whose columns one MMA reads in one swizzle.
   int qk_narrow;
   int v_row_bytes;       // same for V
@@ -1196,10 +1196,10 @@ __device__ void bias_convert_ragged_role(const Ctx& c, int wq, int lane) {
 // kGate: the result is multiplied by sigmoid(gate).  A template argument, because a run-time test of the pointer
 // cost calls without a gate 0.9 % (768 rows of 768 keys: 671 -> 677 us).
 // kFp8 likewise, and for the same reason no debug stamps, divisions, second copies of a waiting loop or of a loop body
-// are left in the production kernel: nearly every line of instructions is fetched from the SM's instruction cache (432
-// requests a logits tile), which the hot loops of the roles just overflow (10 misses a tile; code added beside
-// them, with the same work done, took 43 misses and 665 -> 792 us).  83 KB of code -> 55 KB: 389 rows 261 -> 253.5 us
-// a module call, 256 rows of 64 channels 58.2 -> 57.5; 768 rows 672.6 -> 671.0, 1536 tokens 30.5 -> 30.7.
+// are left in the production kernel (389 rows 261 -> 253.5 us a module call, 256 rows of 64 channels 58.2 -> 57.5; 768 rows
+// and 1536 tokens unchanged).  The roles' loops come from the SM's instruction cache, 440 requests and 10 misses a logits
+// tile, which is what it was with more code as well; four copies of the softmax tile beside them took 43 misses and 192 -> 222 us
+// on 192 rows of 768.
 // kMixed: some items have fewer streams than the others (smaller ones behind the last full round, rows or pairs of query
 // tiles that leave a remainder), which takes slots and barriers that an item does not use through their phases and two sets
 // of constants to decode an item.  A plan of equal items runs without: 768 rows 645 -> 636 us.
