@@ -6,7 +6,7 @@
 //
 //   warp 0      TMA producer: Q tiles, K/V ring, bias ring (cp.async.bulk.tensor, each CTA loads its own tiles)
 //   warp 1      tcgen05.mma issuer for the logits (smem x smem -> TMEM)
-//   warp 2      TMEM allocator, then tcgen05.mma issuer for O += P V (TMEM x smem -> TMEM); Q scaler
+//   warp 2      TMEM allocator, then tcgen05.mma issuer for O += P V (TMEM x smem -> TMEM)
 //   warp 3      key-mask writer (see below)
 //   warps 4-7   softmax warpgroup 0 (owns S / P buffer 0 and the even streams of a work item)
 //   warps 8-11  softmax warpgroup 1 (owns S / P buffer 1 and the odd streams)
@@ -20,7 +20,7 @@
 // 16-lane XU, every other instruction competing for the same issue slots), so everything that
 // can be an MMA is one.  With bf16 q/k the whole logit comes out of the tensor core:
 //
-//   * scale: warp 2 multiplies each Q tile by the softmax scale in shared memory and rounds it
+//   * scale: the softmax warps multiply each Q tile by the softmax scale in shared memory, an item ahead, and round it
 //     back to bf16 - the reference's own first step (q = q * scaling, in bf16);
 //   * bias: eight small MMAs per tile (M = 128, N = 16, K = 16) whose A operand is a 16-key
 //     slice of the staged bf16 bias tile and whose B operand is a 16 x 16 identity, each adding
@@ -157,7 +157,7 @@ struct BarIdx {
   static constexpr int s_full = 0;      // [2]  logits of a tile finished
   static constexpr int s_free = 2;      // [2]  softmax warpgroup has the logits in registers
   static constexpr int p_ready = 4;     // [2]  P written (and O rescaled if needed)
-  static constexpr int epi_done = 6;    // [2]  warpgroup has read its O accumulators of the item
+  static constexpr int pv_done = 6;     // [2]  the warpgroup's last P V has finished: its P buffer and that O are free
   static constexpr int bias_full = 8;   // [kBiasStages]
   static constexpr int bias_empty = 10; // [kBiasStages]
   static constexpr int kv_full = 12;    // [kMaxKvStages]
@@ -165,13 +165,14 @@ struct BarIdx {
   // Q tiles: slot = (Q buffer) * kMaxStreams + stream
   static constexpr int q_full = 12 + 2 * kMaxKvStages;       // [2 * kMaxStreams]  Q tile landed
   static constexpr int q_empty = q_full + 2 * kMaxStreams;   // [2 * kMaxStreams]  last Q K^T of the stream finished
-  static constexpr int q_scaled = q_empty + 2 * kMaxStreams; // [2 * kMaxStreams]  the P V warp has scaled the Q tile
+  static constexpr int q_scaled = q_empty + 2 * kMaxStreams; // [2 * kMaxStreams]  the softmax warpgroup's warps have scaled the Q tile
   static constexpr int count = q_scaled + 2 * kMaxStreams;
 };
-static_assert(BarIdx::count * 8 <= (int)kBarrierBlockBytes, "barrier block too small");
+constexpr uint32_t kWaitBlockOff = kBarrierBlockBytes - 32;
+static_assert(BarIdx::count * 8 <= (int)kWaitBlockOff, "barrier block too small");
 
 // Diagnostic dump: four [128][128] float sections, row = query row of block 0's first tile:
-// raw logits, packed P words (64 used), un-normalised O (nv used), {running max, running sum}.
+// raw logits, packed P words (64 used), un-normalised O (nv used), {unused, running sum}.
 constexpr int kDbgTimelineTiles = 256;   // per warpgroup; 8 clock values each, after kDbgFloats floats
 constexpr int kDbgS = 0, kDbgP = kTile * kTile, kDbgO = 2 * kTile * kTile, kDbgML = 3 * kTile * kTile,
               kDbgFloats = 4 * kTile * kTile;
@@ -186,62 +187,51 @@ struct Ctx {
 
 __device__ __forceinline__ uint32_t bar_addr(const Ctx& c, int idx) { return c.bars + 8u * idx; }
 
-// Arguments by value: a reference to the context would keep it in memory.
-__device__ __noinline__ void report_timeout_at(const AttnParams* p, volatile int* abort_flag, int bar_idx) {
+// Behind the barriers, for waits that take long: what the waiting loop needs, so that a call of it carries three words.
+struct WaitBlock {
+  long long limit;     // AttnParams::wait_limit
+  int* status;         // AttnParams::status
+  int* abort_flag;
+};
+
+__device__ __forceinline__ const WaitBlock* wait_block_of(uint32_t bars) {
+  return reinterpret_cast<const WaitBlock*>(__cvta_shared_to_generic(bars + kWaitBlockOff));
+}
+
+__device__ __noinline__ void report_timeout_at(int* status, volatile int* abort_flag, int bar_idx) {
   *abort_flag = 1;
-  if (p->status != nullptr) {
-    atomicOr(p->status, kStatusWaitTimeout);
-    if (atomicCAS(p->status + 1, 0, bar_idx + 1) == 0) {
-      p->status[2] = blockIdx.x;
-      p->status[3] = threadIdx.x >> 5;
+  if (status != nullptr) {
+    atomicOr(status, kStatusWaitTimeout);
+    if (atomicCAS(status + 1, 0, bar_idx + 1) == 0) {
+      status[2] = blockIdx.x;
+      status[3] = threadIdx.x >> 5;
     }
   }
 }
-__device__ __forceinline__ void report_timeout(const Ctx& c, int bar_idx) { report_timeout_at(c.p, c.abort_flag, bar_idx); }
+__device__ __forceinline__ void report_timeout(const Ctx& c, int bar_idx) { report_timeout_at(c.p->status, c.abort_flag, bar_idx); }
 
-// A complete phase, or one parked attempt: most real waits end inside it.
-__device__ __forceinline__ bool mbar_test_or_park(uint32_t bar, uint32_t parity) {
-  return mbar_test_wait(bar, parity) || mbar_try_wait_park(bar, parity, 2000u);
-}
-
-// The waiting loops of the single-warp roles, out of line, with the report of a wait that ran out: a whole warp (the same
-// result in every lane), and one thread (the producer).
-__device__ __noinline__ bool wait_warp_slow_at(const AttnParams* p, volatile int* abort_flag, uint32_t bars, int idx, uint32_t parity) {
-  if (__all_sync(0xffffffffu, mbar_wait_bounded(bars + 8u * idx, parity, p->wait_limit, abort_flag))) return true;
-  report_timeout_at(p, abort_flag, idx);
+// The waiting loop of the single-warp roles, out of line, with the report of a wait that ran out.
+__device__ __noinline__ bool wait_slow(uint32_t bar, uint32_t parity, const WaitBlock* w) {
+  if (mbar_wait_bounded(bar, parity, w->limit, w->abort_flag)) return true;
+  report_timeout_at(w->status, w->abort_flag, (int)((bar - smem_u32(w) + kWaitBlockOff) >> 3));
   return false;
 }
-__device__ __forceinline__ bool wait_warp_slow(const Ctx& c, int idx, uint32_t parity) {
-  return wait_warp_slow_at(c.p, c.abort_flag, c.bars, idx, parity);
-}
-__device__ __noinline__ bool wait_thread_slow_at(const AttnParams* p, volatile int* abort_flag, uint32_t bars, int idx, uint32_t parity) {
-  if (mbar_wait_bounded(bars + 8u * idx, parity, p->wait_limit, abort_flag)) return true;
-  report_timeout_at(p, abort_flag, idx);
-  return false;
-}
-__device__ __forceinline__ bool wait_thread(const Ctx& c, int idx, uint32_t parity) {
-  return mbar_test_or_park(bar_addr(c, idx), parity) || wait_thread_slow_at(c.p, c.abort_flag, c.bars, idx, parity);
-}
 
-#define AF3K_WAIT(ctx, idx, parity)                                                          \
-  do {                                                                                       \
-    if (!wait_thread(ctx, idx, parity)) return;                                              \
+// One thread (the producer).
+#define AF3K_WAIT(ctx, idx, parity)                                                                     \
+  do {                                                                                                  \
+    const uint32_t bar_ = bar_addr(ctx, idx), par_ = (parity);                                          \
+    if (!mbar_try_wait_park(bar_, par_, 2000u) && !wait_slow(bar_, par_, wait_block)) return;           \
   } while (0)
 
-// Form for helpers that report failure through their return value.
-#define AF3K_WAIT_NORET(ctx, idx, parity)                                                    \
-  do {                                                                                       \
-    if (!wait_thread(ctx, idx, parity)) return false;                                        \
-  } while (0)
-
-// Warp-collective forms: every lane leaves together, so no .sync.aligned instruction is ever executed by part of a warp
-// after a timeout.  _C is that of the single-warp roles, with the waiting loop out of line: one pass of their per-tile
-// loops costs 700 - 1 500 cycles whatever it does, next to warps that stream through long unrolled loops, so the path taken
-// when nothing has to be waited for is kept short.
-#define AF3K_WAIT_WARP_C(ctx, idx, parity)                                                   \
-  do {                                                                                       \
-    if (!__all_sync(0xffffffffu, mbar_test_or_park(bar_addr(ctx, idx), (parity))))           \
-      if (!wait_warp_slow(ctx, idx, parity)) return;                                         \
+// A whole warp: every lane leaves together, so no .sync.aligned instruction is ever executed by part of a warp after a
+// timeout.  One parked attempt, in which most real waits end; the rest is out of line, because the single-warp roles' loops are
+// fetched again for every tile, beside warps that stream through long unrolled code.
+#define AF3K_WAIT_WARP_C(ctx, idx, parity)                                                              \
+  do {                                                                                                  \
+    const uint32_t bar_ = bar_addr(ctx, idx), par_ = (parity);                                          \
+    if (!__all_sync(0xffffffffu, mbar_try_wait_park(bar_, par_, 2000u)))                                \
+      if (!__all_sync(0xffffffffu, wait_slow(bar_, par_, wait_block))) return;                          \
   } while (0)
 // The softmax warps keep the waiting loop inline: a call would have to save their registers.
 #define AF3K_WAIT_WARP(ctx, idx, parity)                                                     \
@@ -301,85 +291,92 @@ template <bool kMixed, bool kConvert>
 __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUtensorMap* tm_k,
                               const CUtensorMap* tm_v, const CUtensorMap* tm_bias, const CUtensorMap* tm_q2, const CUtensorMap* tm_k2) {
   const AttnParams& p = *c.p;
-  uint32_t ucount = 0, bcount = 0, icount = 0;
+  const WaitBlock* wait_block = wait_block_of(c.bars);
+  uint32_t icount = 0;
+  uint32_t st = 0, lap = 0, bst = 0, blap = 0;     // K/V and bias ring: stage, laps before
   const uint32_t nkv = p.kv_stages;
   // With two Q buffers the tiles of the next item are requested while the current item runs, so
   // that they are in place (and scaled) when it ends; with one (tiles too large for two), as
-  // soon as the current item's K/V loads are all issued.
-  auto load_q = [&](const Item& it, uint32_t j) {
-    const uint32_t buf = q_buf(p, j), use = q_use(p, j);
-#pragma unroll 1
-    for (int s = 0; s < p.n_streams; ++s) {
-      const int slot = (int)buf * kMaxStreams + s;
-      // the buffer's previous user must have finished its last Q K^T of this stream
-      if (use >= 1) AF3K_WAIT_NORET(c, BarIdx::q_empty + slot, (use - 1) & 1);
-      if (kMixed && s >= it.gv) {
-        mbar_arrive(bar_addr(c, BarIdx::q_full + slot));
-        continue;
-      }
-      mbar_arrive_expect_tx(bar_addr(c, BarIdx::q_full + slot), p.q_tile_bytes);
-      const uint32_t qdst = c.smem + p.off_q + (buf * p.n_streams + s) * p.q_tile_bytes;
-      tma_load_4d(qdst, tm_q, bar_addr(c, BarIdx::q_full + slot), 0, stream_qt(p, it, s) * kTile, it.h, stream_row(p, it, s));
-      if (p.qk_narrow)
-        tma_load_4d(qdst + kNarrowOff, tm_q2, bar_addr(c, BarIdx::q_full + slot), 32, stream_qt(p, it, s) * kTile, it.h, stream_row(p, it, s));
-    }
-    return true;
-  };
-  if ((int)blockIdx.x < p.n_items) {
-    if (!load_q(decode_item<kMixed>(p, blockIdx.x), 0)) return;
-  }
+  // soon as the current item's K/V loads are all issued.  (Not before a K/V stage of this item has come free: the loads wait
+  // for the last Q K^T of the item before, and the K/V ring would run empty meanwhile.)
+  const int q_at = p.q_buffers == 2 ? min((int)(nkv / (uint32_t)p.n_streams) + 1, p.n_kt) : p.n_kt;
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
     const Item it = decode_item<kMixed>(p, item);
 #pragma unroll 1
-    for (int kt = 0; kt < p.n_kt; ++kt) {
+    for (int kt = 0; kt <= p.n_kt; ++kt) {
+      const bool own = kt == 0 && icount == 0;
+      const int q_item = own ? item : item + (int)gridDim.x;
+      if ((own || kt == q_at) && q_item < p.n_items) {
+        const uint32_t j = own ? 0 : icount + 1, buf = q_buf(p, j), use = q_use(p, j);
+        const Item qi = decode_item<kMixed>(p, q_item);
+#pragma unroll 1
+        for (int s = 0; s < p.n_streams; ++s) {
+          const int slot = (int)buf * kMaxStreams + s;
+          // the buffer's previous user must have finished its last Q K^T of this stream
+          if (use >= 1) AF3K_WAIT(c, BarIdx::q_empty + slot, (use - 1) & 1);
+          const uint32_t full = bar_addr(c, BarIdx::q_full + slot);
+          if (kMixed && s >= qi.gv) {
+            mbar_arrive(full);
+            continue;
+          }
+          mbar_arrive_expect_tx(full, p.q_tile_bytes);
+          const uint32_t qdst = c.smem + p.off_q + (buf * p.n_streams + s) * p.q_tile_bytes;
+          tma_load_4d(qdst, tm_q, full, 0, stream_qt(p, qi, s) * kTile, qi.h, stream_row(p, qi, s));
+          if (p.qk_narrow) tma_load_4d(qdst + kNarrowOff, tm_q2, full, 32, stream_qt(p, qi, s) * kTile, qi.h, stream_row(p, qi, s));
+        }
+      }
+      if (kt == p.n_kt) break;
 #pragma unroll 1
       for (int s = 0; s < it.gv; ++s) {
         if (!kConvert && (s == 0 || p.q_split)) {   // one bias tile per key tile, or per stream when the streams are query tiles
-          const uint32_t bst = bcount % kBiasStages;
-          if (bcount >= kBiasStages)
-            AF3K_WAIT(c, BarIdx::bias_empty + bst, ((bcount / kBiasStages) - 1) & 1);
+          if (blap != 0) AF3K_WAIT(c, BarIdx::bias_empty + bst, (blap - 1) & 1);
           const uint32_t bfull = bar_addr(c, BarIdx::bias_full + bst);
           const uint32_t bdst = c.smem + p.off_bias + bst * kBiasTileBytes;
           mbar_arrive_expect_tx(bfull, kBiasTileBytes);
           tma_load_3d(bdst, tm_bias, bfull, kt * kTile, stream_qt(p, it, s) * kTile, it.h);
           tma_load_3d(bdst + kBiasTileBytes / 2, tm_bias, bfull, kt * kTile + 64, stream_qt(p, it, s) * kTile, it.h);
-          ++bcount;
+          if (++bst == kBiasStages) { bst = 0; ++blap; }
         }
-        const uint32_t st = ucount % nkv;
-        if (ucount >= nkv) AF3K_WAIT(c, BarIdx::kv_empty + st, ((ucount / nkv) - 1) & 1);
+        if (lap != 0) AF3K_WAIT(c, BarIdx::kv_empty + st, (lap - 1) & 1);
         const uint32_t full = bar_addr(c, BarIdx::kv_full + st);
         const uint32_t kdst = c.smem + p.off_kv + st * (p.k_tile_bytes + p.v_tile_bytes);
         mbar_arrive_expect_tx(full, p.k_tile_bytes + p.v_tile_bytes);
         tma_load_4d(kdst, tm_k, full, 0, kt * kTile, it.h, stream_row(p, it, s));
         if (p.qk_narrow) tma_load_4d(kdst + kNarrowOff, tm_k2, full, 32, kt * kTile, it.h, stream_row(p, it, s));
         tma_load_4d(kdst + p.k_tile_bytes, tm_v, full, 0, kt * kTile, it.h, stream_row(p, it, s));
-        ++ucount;
-      }
-      if (kt == (p.q_buffers == 2 ? 0 : p.n_kt - 1) && item + (int)gridDim.x < p.n_items) {
-        if (!load_q(decode_item<kMixed>(p, item + gridDim.x), icount + 1)) return;
+        if (++st == nkv) { st = 0; ++lap; }
       }
     }
   }
 }
 
 // ------------------------------------------------------------------ Q scaling and key-mask column
-// q <- bf16(q * scale) for 1 KB of a Q tile in shared memory, 32 bytes per lane (any swizzle: the
-// operation is elementwise).
-__device__ __forceinline__ void scale_q_chunk(uint32_t addr, float scale, int lane) {
-  uint32_t w[8];
-  const uint32_t a = addr + lane * 16;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(a));
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(a + 512));
+// q <- bf16(q * scale) for some KB of a Q tile in shared memory, 32 bytes per lane and KB (any swizzle: the operation is
+// elementwise), then one arrival per warp.  (Out of line: two callers, once per item each.)
+__device__ __noinline__ void scale_q(uint32_t addr, uint32_t bytes, float scale, int lane, uint32_t bar) {
+  const uint64_t scale2 = pack_f32x2(scale, scale);
+#pragma unroll 1
+  for (uint32_t a = addr + lane * 16, end = a + bytes; a < end; a += 1024) {
+    uint32_t w[8];
 #pragma unroll
-  for (int e = 0; e < 8; ++e)
-    w[e] = pack_bf16x2(__uint_as_float(w[e] << 16) * scale, __uint_as_float(w[e] & 0xffff0000u) * scale);
-  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(w[0]), "r"(w[1]), "r"(w[2]),
-               "r"(w[3]) : "memory");
-  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a + 512), "r"(w[4]), "r"(w[5]),
-               "r"(w[6]), "r"(w[7]) : "memory");
+    for (int i = 0; i < 2; ++i)
+      asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(w[4 * i]), "=r"(w[4 * i + 1]), "=r"(w[4 * i + 2]), "=r"(w[4 * i + 3]) : "r"(a + 512 * i));
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float q0, q1;
+      unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(w[e] << 16), __uint_as_float(w[e] & 0xffff0000u)), scale2), q0, q1);
+      w[e] = pack_bf16x2(q0, q1);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a + 512 * i), "r"(w[4 * i]), "r"(w[4 * i + 1]), "r"(w[4 * i + 2]),
+                   "r"(w[4 * i + 3]) : "memory");
+  }
+  fence_proxy_async_smem();    // make the generic-proxy stores visible to the tensor core
+  __syncwarp();
+  if (lane == 0) mbar_arrive(bar);
 }
 
 // The 128 mask-column values (bf16) of one logits tile, four per lane.
@@ -404,54 +401,6 @@ __device__ __forceinline__ uint16_t masked_value_bits(const AttnParams& p, int h
   return (uint16_t)(0x8000u | ((uint32_t)(e + 127) << 7));
 }
 
-// Scaling of Q tiles, cut into 1 KB pieces so that the warp doing it (the P V issuer, which
-// mostly waits) can fit the pieces into its waiting time.
-struct QScaler {
-  uint32_t item = 0, chunk = 0;   // item index (per CTA) of the tiles being scaled, next piece
-  int gv = 0, tile = 0;           // tiles that item has, next tile
-  __device__ __forceinline__ void start(uint32_t j, int n) { item = j; gv = n; tile = 0; chunk = 0; }
-  __device__ __forceinline__ bool pending() const { return tile < gv; }
-  // One piece.  block: wait (bounded) for the tile to land, else give up if it has not.
-  // Returns 1 = did a piece, 0 = nothing to do (now), -1 = a wait ran out.
-  __device__ __forceinline__ int step(const Ctx& c, int lane, bool block) {
-    const AttnParams& p = *c.p;
-    if (tile >= gv) return 0;
-    const uint32_t buf = q_buf(p, item);
-    const int slot = (int)buf * kMaxStreams + tile;
-    if (chunk == 0) {
-      const uint32_t par = q_use(p, item) & 1;
-      if (!__all_sync(0xffffffffu, mbar_test_wait(bar_addr(c, BarIdx::q_full + slot), par))) {
-        if (!block) return 0;
-        if (!wait_warp_slow(c, BarIdx::q_full + slot, par)) return -1;
-      }
-    }
-    scale_q_chunk(c.smem + p.off_q + (buf * p.n_streams + tile) * p.q_tile_bytes + (chunk << 10), p.scale, lane);
-    if (++chunk == (p.q_tile_bytes >> 10)) {
-      fence_proxy_async_smem();    // make the generic-proxy stores visible to the tensor core
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::q_scaled + slot));
-      chunk = 0;
-      ++tile;
-    }
-    return 1;
-  }
-};
-
-// Waits for a barrier phase; while it is pending, does Q scaling pieces (if any are left).
-#define AF3K_WAIT_WARP_OR_SCALE(ctx, idx, parity, scaler, lane)                              \
-  do {                                                                                       \
-    while (true) {                                                                           \
-      const bool done_ = mbar_test_wait(bar_addr(ctx, idx), (parity));                       \
-      if (__all_sync(0xffffffffu, done_)) break;                                             \
-      const int r_ = (scaler).step(ctx, lane, false);                                        \
-      if (r_ < 0) return;                                                                    \
-      if (r_ == 0) {                                                                         \
-        AF3K_WAIT_WARP_C(ctx, idx, parity);                                                  \
-        break;                                                                               \
-      }                                                                                      \
-    }                                                                                        \
-  } while (0)
-
 // Key-mask writer (one warp).  For every logits tile, in the producer's order: write the tile's
 // 128 mask values into its slot of the mask-column ring.  The slot is the B operand of the extra
 // K step; only element 0 of each key's 16-byte row changes, the rest stays zero.  Arrives on the
@@ -460,6 +409,7 @@ struct QScaler {
 template <bool kMixed>
 __device__ void mask_writer_role(const Ctx& c, int lane) {
   const AttnParams& p = *c.p;
+  const WaitBlock* wait_block = wait_block_of(c.bars);
   const uint32_t nkv = p.kv_stages;
   uint32_t st = 0, round = 0;      // ring slot, how many times the ring wrapped
 #pragma unroll 1
@@ -508,6 +458,7 @@ __device__ void mask_writer_role(const Ctx& c, int lane) {
 template <bool kDebug, bool kTcBias, bool kFp8, bool kMixed>
 __device__ void qk_issuer_role(const Ctx& c) {
   const AttnParams& p = *c.p;
+  const WaitBlock* wait_block = wait_block_of(c.bars);
   const bool leader = elect_one();
   const uint32_t nkv = p.kv_stages;
   const uint32_t qk_layout = swizzle_layout_code(p.qk_row_bytes);
@@ -567,9 +518,9 @@ __device__ void qk_issuer_role(const Ctx& c) {
           if (need_bias) ok = mbar_test_wait(bar_addr(c, BarIdx::bias_full + bst), b_par) && ok;
           if (kt == 0) ok = mbar_test_wait(bar_addr(c, q_bar), q_use(p, icount) & 1) && ok;
           if (!__all_sync(0xffffffffu, ok)) {
-            if (need_bias) AF3K_WAIT_WARP_C(c, BarIdx::bias_full + bst, b_par);
-            // the softmax warpgroup of this buffer must have read the previous logits tile
+            // (the softmax warpgroup of this buffer must have read the previous logits tile)
             if (need_sfree) AF3K_WAIT_WARP_C(c, BarIdx::s_free + b, sf_par);
+            if (need_bias) AF3K_WAIT_WARP_C(c, BarIdx::bias_full + bst, b_par);
             if (kt == 0) AF3K_WAIT_WARP_C(c, q_bar, q_use(p, icount) & 1);
             AF3K_WAIT_WARP_C(c, BarIdx::kv_full + st, kv_par);
           }
@@ -621,7 +572,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
     if (kMixed) {
       if (leader)
         for (int s = gv; s < p.n_streams; ++s) {
-          mbar_arrive(bar_addr(c, BarIdx::q_scaled + (int)q_buf(p, icount) * kMaxStreams + s));
+          for (int w = 0; w < 4; ++w) mbar_arrive(bar_addr(c, BarIdx::q_scaled + (int)q_buf(p, icount) * kMaxStreams + s));
           mbar_arrive(bar_addr(c, BarIdx::q_empty + (int)q_buf(p, icount) * kMaxStreams + s));
         }
       __syncwarp();
@@ -629,19 +580,12 @@ __device__ void qk_issuer_role(const Ctx& c) {
   }
 }
 
-// O += P V for every tile, in order.  This warp mostly waits for the softmax warpgroups, so (bf16
-// q/k) it also scales the Q tiles: the first item's up front, the next item's in 1 KB pieces
-// while it waits, what is left when the item's last P V has been issued.
-template <bool kDebug, bool kScalesQ, bool kMixed>
-__device__ void pv_issuer_role(const Ctx& c, int lane) {
+// O += P V for every tile, in order.
+template <bool kDebug, bool kMixed>
+__device__ void pv_issuer_role(const Ctx& c) {
   const AttnParams& p = *c.p;
+  const WaitBlock* wait_block = wait_block_of(c.bars);
   const bool leader = elect_one();
-  QScaler scaler;
-  if (kScalesQ && p.scale_q && (int)blockIdx.x < p.n_items) {
-    scaler.start(0, decode_item<kMixed>(p, blockIdx.x).gv);
-    while (scaler.pending())
-      if (scaler.step(c, lane, true) < 0) return;
-  }
   const uint32_t nkv = p.kv_stages;
   const uint32_t v_layout = swizzle_layout_code(p.v_row_bytes);
   const uint32_t idesc_pv = make_idesc(1u, 1u, 0u, 1u, (uint32_t)p.nv);   // A = P and B = V, both bf16 (kind::f16 takes no mixed pair)
@@ -656,36 +600,19 @@ __device__ void pv_issuer_role(const Ctx& c, int lane) {
                             2 * kDbgTimelineTiles
                       : nullptr;
   uint32_t tl_n = 0;
-  uint32_t st = 0, icount = 0;
-  uint32_t epi_seen = 0, epi_par = 0;   // bit b: warpgroup b has had an item; parity of its last one's epilogue
+  uint32_t st = 0;
   uint32_t pready_par = 0;         // bit b: of warpgroup b's next P
 #pragma unroll 1
-  for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
+  for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
     const Item it = decode_item<kMixed>(p, item);
     const int gv = it.gv;
-    scaler.start(icount + 1, (kScalesQ && p.scale_q && item + (int)gridDim.x < p.n_items) ? decode_item<kMixed>(p, item + gridDim.x).gv : 0);
 #pragma unroll 1
     for (int kt = 0; kt < p.n_kt; ++kt) {
 #pragma unroll 1
       for (int s = 0; s < gv; ++s) {
         const int b = s & 1;
-        if (kScalesQ) AF3K_WAIT_WARP_OR_SCALE(c, BarIdx::p_ready + b, (pready_par >> b) & 1u, scaler, lane);
-        else          AF3K_WAIT_WARP_C(c, BarIdx::p_ready + b, (pready_par >> b) & 1u);
+        AF3K_WAIT_WARP_C(c, BarIdx::p_ready + b, (pready_par >> b) & 1u);
         pready_par ^= 1u << b;
-        // the warpgroup's epilogue of the previous item must have read its O accumulators before
-        // its first P V of this item overwrites one
-        if (!kMixed) {
-          if (kt == 0 && s < 2 && icount > 0) AF3K_WAIT_WARP_C(c, BarIdx::epi_done + b, (icount - 1) & 1);
-        } else if (kt == 0 && s < 2) {
-          if ((epi_seen >> b) & 1u) {
-            AF3K_WAIT_WARP_C(c, BarIdx::epi_done + b, (epi_par >> b) & 1u);
-            epi_par ^= 1u << b;
-          }
-          epi_seen |= 1u << b;
-          // an item of one stream: the other warpgroup must have finished its item before (it looks at the barrier of a K/V
-          // stage for that, which must not go through another lap meanwhile)
-          if (gv == 1 && epi_seen == 3u) AF3K_WAIT_WARP_C(c, BarIdx::epi_done + 1, epi_par >> 1);
-        }
         tc_fence_after();
         const uint32_t b_lo = vd_lo + st * stage_step;
         const uint32_t o_tmem = c.tmem + kOCol + s * p.nv;
@@ -696,7 +623,7 @@ __device__ void pv_issuer_role(const Ctx& c, int lane) {
 #pragma unroll 1
           for (int k = 1; k < kTile / 16; ++k)   // 16 keys per step: 8 TMEM columns of P
             mma_ts_f16(o_tmem, p_tmem + k * 8, b_lo + k * v_kstep, vd_hi, idesc_pv, 1u);
-          // one completion signal: the K/V stage is free, and so are this tile's P buffer and O
+          tc_commit(bar_addr(c, BarIdx::pv_done + b));
           tc_commit(bar_addr(c, BarIdx::kv_empty + st));
           if (kDebug && tl != nullptr && tl_n + 2 <= 2 * kDbgTimelineTiles) { tl[tl_n++] = t0; tl[tl_n++] = clock64(); }
         }
@@ -704,8 +631,6 @@ __device__ void pv_issuer_role(const Ctx& c, int lane) {
         if (++st == nkv) st = 0;
       }
     }
-    while (kScalesQ && scaler.pending())
-      if (scaler.step(c, lane, true) < 0) return;
   }
 }
 
@@ -767,29 +692,121 @@ __device__ __forceinline__ void exponent_terms(float m, float ef, float& f, floa
   c = -m * f;
 }
 
+// O accumulator of this thread's row times alpha.
+__device__ __forceinline__ void rescale_output(uint32_t o_taddr, int nv, float alpha) {
+#pragma unroll 1
+  for (int c0 = 0; c0 < nv; c0 += 16) {
+    uint32_t o[16];
+    tmem_ld_x16(o_taddr + c0, o);
+    tc_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+    tmem_st_x16(o_taddr + c0, o);
+  }
+}
+
+// A softmax warp's wait, after a test that came too early (the loop is inline: a call would have to save the registers).
+__device__ __forceinline__ bool softmax_wait(const Ctx& c, int idx, uint32_t parity) {
+  const bool ok = mbar_wait_bounded(bar_addr(c, idx), parity, c.p->wait_limit, c.abort_flag);
+  if (__all_sync(0xffffffffu, ok)) return true;
+  report_timeout(c, idx);
+  return false;
+}
+
+// What a softmax thread carries from tile to tile.
+struct SoftmaxState {
+  float m[2], l[2];          // reference maximum and sum of its streams: [0] the stream whose turn it is, [1] the other one
+  uint64_t sum_a, sum_b;     // the last tile's weights, not yet in its stream's sum
+  uint32_t s_par, pv_par;    // parities of the next logits tile and of the last P V
+  bool s_ready;              // the next logits tile was seen complete already
+  bool started;              // there is a last P V
+  bool swap;                 // the last tile's stream has another one beside it, whose turn it is now
+  // A stream that has had its last key tile: its result is still in TMEM (0: none).
+  uint32_t done_o;
+  float done_l;
+  __nv_bfloat16* done_row;   // where this thread's row goes (null: beyond the matrix)
+  const __nv_bfloat16* done_gate;
+};
+
+// The last tile's weights enter its stream's sum and the turn passes to the other stream.
+__device__ __forceinline__ void close_tile(SoftmaxState& st) {
+  float s0, s1, s2, s3;
+  unpack_f32x2(st.sum_a, s0, s1);
+  unpack_f32x2(st.sum_b, s2, s3);
+  st.l[0] += (s0 + s1) + (s2 + s3);
+  st.done_l = st.l[0];
+  if (st.swap) {
+    const float m = st.m[0], l = st.l[0];
+    st.m[0] = st.m[1]; st.l[0] = st.l[1];
+    st.m[1] = m; st.l[1] = l;
+  }
+}
+
+// O / l -> bf16 -> global for the stream that is done.
+template <bool kDebug, bool kGate>
+__device__ __forceinline__ void store_result(const Ctx& c, const SoftmaxState& st, float* dbg) {
+  const AttnParams& p = *c.p;
+  const float inv = __frcp_rn(st.done_l);
+#pragma unroll 1
+  for (int c0 = 0; c0 < p.nv; c0 += 16) {
+    uint32_t o[16];
+    tmem_ld_x16(st.done_o + c0, o);
+    tc_wait_ld();
+    if (kDebug && dbg != nullptr) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) dbg[kDbgO + c0 + i] = __uint_as_float(o[i]);
+      dbg[kDbgML + 1] = st.done_l;
+    }
+    if (st.done_row != nullptr) {
+#pragma unroll
+      for (int hseg = 0; hseg < 2; ++hseg) {
+        if (c0 + hseg * 8 + 8 <= p.D) {
+          if constexpr (kGate) {
+            const uint4 gv = *reinterpret_cast<const uint4*>(st.done_gate + c0 + hseg * 8);
+            const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float g = __uint_as_float((e & 1) ? gw[e >> 1] & 0xffff0000u : gw[e >> 1] << 16);
+              o[hseg * 8 + e] = __float_as_uint(__uint_as_float(o[hseg * 8 + e]) * sigmoid_f32(g));
+            }
+          }
+          uint4 v;
+          v.x = pack_bf16x2(__uint_as_float(o[hseg * 8 + 0]) * inv, __uint_as_float(o[hseg * 8 + 1]) * inv);
+          v.y = pack_bf16x2(__uint_as_float(o[hseg * 8 + 2]) * inv, __uint_as_float(o[hseg * 8 + 3]) * inv);
+          v.z = pack_bf16x2(__uint_as_float(o[hseg * 8 + 4]) * inv, __uint_as_float(o[hseg * 8 + 5]) * inv);
+          v.w = pack_bf16x2(__uint_as_float(o[hseg * 8 + 6]) * inv, __uint_as_float(o[hseg * 8 + 7]) * inv);
+          *reinterpret_cast<uint4*>(st.done_row + c0 + hseg * 8) = v;
+        }
+      }
+    }
+  }
+}
+
 // One 128 x 128 logits tile of one stream; the thread owns row `row` (TMEM lane).
-// m_run is the reference maximum the running sums are scaled by (it may lag the true maximum by
-// up to kLazyRescaleLog2 bits), l_run the running sum of the fp32 weights.
-template <bool kTcBias>
-__device__ __forceinline__ bool softmax_tile(const Ctx& c, float* dbg, int wg, int lane,
+// st.m[0] is the reference maximum the running sums are scaled by (it may lag the true maximum by
+// up to kLazyRescaleLog2 bits), st.l[0] the running sum of the fp32 weights.
+template <bool kDebug, bool kTcBias, bool kGate>
+__device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, float* dbg, float* dbg_o, int wg, int lane,
                                              uint32_t s_taddr, uint32_t p_taddr, uint32_t o_taddr,
-                                             int nv, uint32_t bias_row, uint32_t row7, float scale,
-                                             bool first_kt, bool wait_prev_pv, int prev_pv_bar,
-                                             uint32_t prev_pv_parity, float& m_run, float& l_run,
-                                             int next_s_bar, uint32_t next_s_parity, bool& next_ready,
-                                             long long* ts = nullptr) {
+                                             uint32_t bias_row, uint32_t row7, float scale, bool first_kt, long long* ts) {
+  if (kDebug && ts != nullptr) ts[0] = clock64();
+  if (!st.s_ready && !softmax_wait(c, BarIdx::s_full + wg, st.s_par)) return false;
+  st.s_par ^= 1;
+  tc_fence_after();
+  if (kDebug && ts != nullptr) ts[1] = clock64();
   uint32_t xr[kTile];
+  tmem_ld_x32(s_taddr + 0, &xr[0]);
+  tmem_ld_x32(s_taddr + 32, &xr[32]);
+  // Under the loads: what is left of the tile before, and a look whether its P V has finished.
+  close_tile(st);
+  if (first_kt) { st.m[0] = -INFINITY; st.l[0] = 0.f; }
+  const bool pv_ok = mbar_test_wait(bar_addr(c, BarIdx::pv_done + wg), st.pv_par) || !st.started;
+  const float m_run = st.m[0];
   float mt;
   {
-    tmem_ld_x32(s_taddr + 0, &xr[0]);
-    tmem_ld_x32(s_taddr + 32, &xr[32]);
     tc_wait_ld();
     tmem_ld_x32(s_taddr + 64, &xr[64]);
     tmem_ld_x32(s_taddr + 96, &xr[96]);
-    if (dbg != nullptr) {
-#pragma unroll
-      for (int i = 0; i < 64; ++i) dbg[kDbgS + i] = __uint_as_float(xr[i]);
-    }
     const uint64_t scale2 = pack_f32x2(scale, scale);
     float mxa = -INFINITY, mxb = -INFINITY;
     if (kTcBias) max_half<0>(xr, mxa, mxb);
@@ -799,50 +816,44 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, float* dbg, int wg, i
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::s_free + wg));
-    if (dbg != nullptr) {
+    if (kDebug && dbg != nullptr) {
 #pragma unroll
-      for (int i = 64; i < kTile; ++i) dbg[kDbgS + i] = __uint_as_float(xr[i]);
+      for (int i = 0; i < kTile; ++i) dbg[kDbgS + i] = __uint_as_float(xr[i]);
     }
     if (kTcBias) max_half<64>(xr, mxa, mxb);
     else         logits_half<64>(xr, bias_row, row7, scale2, mxa, mxb);
     mt = fmaxf(mxa, mxb);
   }
-  if (ts != nullptr) ts[2] = clock64() + (long long)(mt == 123.456f);   // logits and row maximum in registers
+  if (kDebug && ts != nullptr) ts[2] = clock64() + (long long)(mt == 123.456f);   // logits and row maximum in registers
   // factor between a logit difference and the exponent of 2: log2(e), times the logit scale when
   // the tensor core's logits still lack it (fp8 q/k with tensor-core bias: `scale` carries it)
   const float ef = kTcBias ? scale : kLog2e;
-  float m_use = m_run;
-  float alpha = 1.0f;
-  bool need = false;
-  if (first_kt) {
-    m_use = mt;
-  } else {
-    need = (mt - m_run) * ef > kLazyRescaleLog2;
-    if (need) m_use = mt;
-  }
+  // (m_run is -inf in front of the first key tile)
+  const bool grown = (mt - m_run) * ef > kLazyRescaleLog2;
+  const float m_use = first_kt || grown ? mt : m_run;
+  const bool need = grown && !first_kt;
   float f = ef, nml = 0.f;
   if (kTcBias) exponent_terms(m_use, ef, f, nml);
-  if (ts != nullptr) ts[3] = clock64();   // exponential pass starts
+  // The P buffer and the O accumulators are this warpgroup's again when its last P V has finished.  Waited for in front of
+  // the pass, because a branch within it drains the exponentials in flight.
+  if (!__all_sync(0xffffffffu, pv_ok) && !softmax_wait(c, BarIdx::pv_done + wg, st.pv_par)) return false;
+  st.pv_par ^= st.started ? 1u : 0u;
+  st.started = true;
+  tc_fence_after();
+  if (kDebug && ts != nullptr) ts[3] = clock64();   // last P V awaited, exponential pass starts
   // p = exp2((x - m) * log2e).  fp8 path: the subtraction comes first so that x == m gives
   // exactly 0 even for the huge negative values of masked keys (a row with no attended key: all
   // weights 1).  bf16 path: one fused multiply-add (exponent_terms).
   // The pass is one ex2 per logit on the XU (a warp-wide ex2 every 8 cycles per scheduler, shared
   // by the scheduler's two softmax warps) with one packed FMA, one packed add and one bf16 pack per
-  // pair of logits around it.  The two warpgroups run their passes in step (2 000 - 2 500 cycles per
-  // pass against 2 048 for the XU alone); what keeps the kernel above that is the time between
-  // passes, when both read logits, search the maximum and hand P over and the XU idles.
+  // pair of logits around it.
   const uint64_t l2e2 = pack_f32x2(f, f);
   const uint64_t nm2 = pack_f32x2(-m_use, -m_use);
   const uint64_t nml2 = pack_f32x2(nml, nml);
   uint64_t suma = pack_f32x2(0.f, 0.f), sumb = suma;
-  // The first kHeld column groups are computed before anything is written: the P buffer and the O accumulator only become free
-  // when the previous P V of this warpgroup has finished.  Held groups cost eight registers each, and two cover that wait:
-  // 2048 fp8 rows 11 340 us with three, 10 920 with two, 768 bf16 rows 659 and 646; one is as fast there and
-  // slower at 389 rows (168 -> 174).
-  constexpr int kHeld = 2;
-  uint32_t pk[8][8];
 #pragma unroll
   for (int cidx = 0; cidx < 8; ++cidx) {
+    uint32_t pk[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int col = cidx * 16 + 2 * i;
@@ -854,87 +865,91 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, float* dbg, int wg, i
       const float p1 = ex2_approx(y1);
       if (i & 1) sumb = add_f32x2(sumb, pack_f32x2(p0, p1));
       else       suma = add_f32x2(suma, pack_f32x2(p0, p1));
-      pk[cidx][i] = pack_bf16x2(p0, p1);
+      pk[i] = pack_bf16x2(p0, p1);
     }
-    if (dbg != nullptr) {
+    if (kDebug && dbg != nullptr) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) dbg[kDbgP + cidx * 8 + i] = __uint_as_float(pk[cidx][i]);
+      for (int i = 0; i < 8; ++i) dbg[kDbgP + cidx * 8 + i] = __uint_as_float(pk[i]);
     }
-    if (cidx == kHeld - 1) {
-      // the completion that frees P and O is the one that also frees the previous tile's K/V stage
-      if (wait_prev_pv) {
-        const bool ok = mbar_wait_bounded(bar_addr(c, prev_pv_bar), prev_pv_parity, c.p->wait_limit,
-                                          c.abort_flag);
-        if (!__all_sync(0xffffffffu, ok)) {
-          report_timeout(c, prev_pv_bar);
-          return false;
-        }
-        tc_fence_after();
-      }
-      if (__any_sync(0xffffffffu, need)) {
-        if (need) {
-          if (kTcBias) {
-            // what a key at the old reference weighs under the new one, over what it was counted with
-            float f_run, nml_run;
-            exponent_terms(m_run, ef, f_run, nml_run);
-            alpha = ex2_approx(__fmaf_rn(m_run, f, nml) - __fmaf_rn(m_run, f_run, nml_run));
-          } else {
-            alpha = ex2_approx((m_run - mt) * ef);
-          }
-        }
-#pragma unroll 1
-        for (int c0 = 0; c0 < nv; c0 += 16) {
-          uint32_t o[16];
-          tmem_ld_x16(o_taddr + c0, o);
-          tc_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tmem_st_x16(o_taddr + c0, o);
-        }
-      }
-      if (ts != nullptr) ts[5] = clock64();   // previous P V awaited
-    }
-    if (cidx >= kHeld - 1) {
-      // P as bf16, two keys per 32-bit TMEM column: the A operand of the second GEMM
-#pragma unroll
-      for (int cc = (cidx == kHeld - 1 ? 0 : cidx); cc <= cidx; ++cc)
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
-                     ::"r"(pk[cc][0]), "r"(pk[cc][1]), "r"(pk[cc][2]), "r"(pk[cc][3]), "r"(pk[cc][4]),
-                     "r"(pk[cc][5]), "r"(pk[cc][6]), "r"(pk[cc][7]), "r"(p_taddr + cc * 8)
-                     : "memory");
-    }
+    // P as bf16, two keys per 32-bit TMEM column: the A operand of the second GEMM
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                 ::"r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]),
+                 "r"(p_taddr + cidx * 8)
+                 : "memory");
   }
-  if (ts != nullptr) ts[6] = clock64();     // last exponential issued
+  if (kDebug && ts != nullptr) ts[6] = clock64();     // last exponential issued
+  // What else has to be done with the accumulators before the next P V may write one.
+  if (__any_sync(0xffffffffu, need)) {
+    float alpha = 1.0f;
+    if (need) {
+      if (kTcBias) {
+        // what a key at the old reference weighs under the new one, over what it was counted with
+        float f_run, nml_run;
+        exponent_terms(m_run, ef, f_run, nml_run);
+        alpha = ex2_approx(__fmaf_rn(m_run, f, nml) - __fmaf_rn(m_run, f_run, nml_run));
+      } else {
+        alpha = ex2_approx((m_run - mt) * ef);
+      }
+    }
+    st.l[0] *= alpha;
+    rescale_output(o_taddr, c.p->nv, alpha);
+  }
+  if (st.done_o != 0) {
+    store_result<kDebug, kGate>(c, st, dbg_o);
+    st.done_o = 0;
+  }
+  st.m[0] = m_use;
+  st.sum_a = suma;
+  st.sum_b = sumb;
   // The next tile's logits are normally finished by now: ask while the P stores drain, so that the
-  // barrier's round trip (about two hundred cycles even when the phase is complete) is not paid
-  // between two tiles.
-  next_ready = __all_sync(0xffffffffu, mbar_test_wait(bar_addr(c, next_s_bar), next_s_parity));
+  // barrier's round trip is not paid between two tiles.
+  st.s_ready = __all_sync(0xffffffffu, mbar_test_wait(bar_addr(c, BarIdx::s_full + wg), st.s_par));
   tc_wait_st();
-  if (ts != nullptr) ts[4] = clock64();   // P stored
-  float s0, s1, s2, s3;
-  unpack_f32x2(suma, s0, s1);
-  unpack_f32x2(sumb, s2, s3);
-  m_run = m_use;
-  l_run = l_run * alpha + ((s0 + s1) + (s2 + s3));
+  tc_fence_before();
+  __syncwarp();
+  if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::p_ready + wg));
+  if (kDebug && ts != nullptr) ts[4] = clock64();   // P handed over
   return true;
 }
 
-template <bool kDebug, bool kTcBias, bool kGate, bool kMixed>
+// (bf16 q/k) A softmax warp scales its quarter of its warpgroup's Q tiles of the CTA's j-th item.  Eight warps do in 300 cycles
+// what took a single-warp role several thousand, and 12 instructions a tile are little beside the softmax's own 450.
+template <bool kMixed>
+__device__ __forceinline__ bool scale_own_q(const Ctx& c, int item, uint32_t j, int wg, int wq, int lane) {
+  const AttnParams& p = *c.p;
+  const Item it = decode_item<kMixed>(p, item);
+  const uint32_t buf = q_buf(p, j), par = q_use(p, j) & 1, bytes = p.q_tile_bytes >> 2;
+#pragma unroll 1
+  for (int s = wg; s < it.gv; s += 2) {
+    const int slot = (int)buf * kMaxStreams + s;
+    if (!softmax_wait(c, BarIdx::q_full + slot, par)) return false;
+    scale_q(c.smem + p.off_q + (buf * p.n_streams + s) * p.q_tile_bytes + wq * bytes, bytes, p.scale, lane, bar_addr(c, BarIdx::q_scaled + slot));
+  }
+  return true;
+}
+
+template <bool kDebug, bool kTcBias, bool kGate, bool kMixed, bool kScalesQ>
 __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
   const AttnParams& p = *c.p;
   const int row = wq * 32 + lane;                    // row of the 128-query tile == TMEM lane
   const uint32_t lane_sel = (uint32_t)(wq * 32) << 16;
   const uint32_t s_taddr = c.tmem + lane_sel + kSCol + wg * kTile;
   const uint32_t p_taddr = c.tmem + lane_sel + kPCol + wg * 64;
-  // running statistics of the warpgroup's (at most two) streams, kept in registers
-  float m_st[2] = {-INFINITY, -INFINITY}, l_st[2] = {0.f, 0.f};
-  uint32_t ucnt = 0, bcount = 0, icount = 0;         // tiles done by this warpgroup, bias tiles, items
-  bool s_ready = false;                              // the next tile's s_full phase was seen complete already
-  // position of tiles in the CTA-wide order (all streams): gives the K/V stage a tile used
-  uint32_t kt_stage = 0, kt_round = 0;                // ring stage / lap of stream 0's tile at the current key tile
-  uint32_t prev_stage = 0, prev_round = 0;            // the same for this warpgroup's last tile
-  bool prev_pending = false;                          // its P V may not have finished
-  const uint32_t nkv = p.kv_stages;
+  SoftmaxState st;
+  st.m[0] = st.m[1] = -INFINITY;
+  st.l[0] = st.l[1] = 0.f;
+  st.sum_a = st.sum_b = 0;
+  st.s_par = st.pv_par = 0;
+  st.s_ready = st.started = st.swap = false;
+  st.done_o = 0;
+  st.done_gate = nullptr;
+  uint32_t bst = 0, b_par = 0;                       // (fp8 without tensor-core bias) bias ring
+  uint32_t n_tiles = 0;                              // (debug build)
+  // The next item's Q tiles are scaled behind the last key tile but one (with a single Q buffer they come later), the first item's here.
+  const bool scales = kScalesQ && p.scale_q;
+  const int scale_kt = !scales ? -1 : (p.q_buffers == 2 ? max(p.n_kt - 2, 0) : p.n_kt - 1);
+  uint32_t icount = 0;
+  if (scales && (int)blockIdx.x < p.n_items && !scale_own_q<kMixed>(c, blockIdx.x, 0, wg, wq, lane)) return;
 
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
@@ -945,120 +960,57 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
     if (p.q_scale != nullptr) scale *= p.q_scale[it.h] * p.k_scale[it.h];
     if (kTcBias) scale = (p.scale_q ? 1.0f : scale) * kLog2e;
 
-    long long* last_ts = nullptr;     // debug build: timeline slot of the warpgroup's last tile
 #pragma unroll 1
     for (int kt = 0; kt < p.n_kt; ++kt) {
       // fp8 q/k: this thread adds the bias itself, from its row of the staged tile
-      const uint32_t bst = bcount % kBiasStages;
-      if (!kTcBias) AF3K_WAIT_WARP(c, BarIdx::bias_full + bst, (bcount / kBiasStages) & 1);
+      if (!kTcBias) AF3K_WAIT_WARP(c, BarIdx::bias_full + bst, b_par);
       const uint32_t bias_row = c.smem + p.off_bias + bst * kBiasTileBytes + row * 128;
 
 #pragma unroll 1
       for (int s = wg; s < it.gv; s += 2) {
-        float m_run = -INFINITY, l_run = 0.f;
-        const int si = (s - wg) >> 1;
-        if (kt > 0) { m_run = si ? m_st[1] : m_st[0]; l_run = si ? l_st[1] : l_st[0]; }
-
         // diagnostic timeline (debug build only): SM clock at the phase boundaries of every tile
         // this warp processes, 8 slots per tile, behind the tile dump
         long long* ts = nullptr;
-        if (kDebug && p.debug != nullptr && blockIdx.x == 0 && wq == 0 && lane == 0 && ucnt < kDbgTimelineTiles)
-          ts = reinterpret_cast<long long*>(p.debug + kDbgFloats) + ((size_t)wg * kDbgTimelineTiles + ucnt) * 8;
-        if (ts != nullptr) ts[0] = clock64();
-        if (kDebug) last_ts = ts;
-        if (!s_ready) AF3K_WAIT_WARP(c, BarIdx::s_full + wg, ucnt & 1);
-        tc_fence_after();
-        if (ts != nullptr) ts[1] = clock64();
-        const uint32_t o_taddr = c.tmem + lane_sel + kOCol + s * p.nv;
-        float* dbg = nullptr;
-        if (kDebug && p.debug != nullptr && blockIdx.x == 0 && icount == 0 && s == 0 && kt == 0)
-          dbg = p.debug + (size_t)row * kTile;
-        if (!softmax_tile<kTcBias>(c, dbg, wg, lane, s_taddr, p_taddr, o_taddr, p.nv, bias_row, row & 7, scale,
-                                   kt == 0, prev_pending, BarIdx::kv_empty + (int)prev_stage, prev_round & 1, m_run,
-                                   l_run, BarIdx::s_full + wg, (ucnt + 1) & 1, s_ready, ts))
-          return;
-        ++ucnt;
-        {
-          // tiles are numbered in the producer's order; the numbers are carried without a division
-          prev_stage = kt_stage + (uint32_t)s;
-          prev_round = kt_round;
-          prev_pending = true;
-          while (prev_stage >= nkv) { prev_stage -= nkv; ++prev_round; }
+        float *dbg = nullptr, *dbg_o = nullptr;
+        if (kDebug && p.debug != nullptr && blockIdx.x == 0) {
+          if (wq == 0 && lane == 0 && n_tiles < kDbgTimelineTiles)
+            ts = reinterpret_cast<long long*>(p.debug + kDbgFloats) + ((size_t)wg * kDbgTimelineTiles + n_tiles) * 8;
+          if (item == 0 && s == 0 && kt == 0) dbg = p.debug + (size_t)row * kTile;
+          if (item == 0 && s == 2 && kt == p.n_kt - 1) dbg_o = p.debug + (size_t)row * kTile;
+          ++n_tiles;
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::p_ready + wg));
-        if (si) { m_st[1] = m_run; l_st[1] = l_run; } else { m_st[0] = m_run; l_st[0] = l_run; }
+        if (!softmax_tile<kDebug, kTcBias, kGate>(c, st, dbg, dbg_o, wg, lane, s_taddr, p_taddr, c.tmem + lane_sel + kOCol + s * p.nv, bias_row,
+                                                  row & 7, scale, kt == 0, ts))
+          return;
+        st.swap = it.gv > wg + 2;
+        if (kt == p.n_kt - 1) {
+          const int qrow = stream_qt(p, it, s) * kTile + row;
+          st.done_o = c.tmem + lane_sel + kOCol + s * p.nv;
+          st.done_row = qrow < p.Sq ? p.out + (long long)stream_row(p, it, s) * p.out_stride_b1 + (long long)it.h * p.out_stride_b2 +
+                                          (long long)qrow * p.out_stride_s
+                                    : nullptr;
+          if constexpr (kGate)
+            st.done_gate = p.gate + (long long)stream_row(p, it, s) * p.gate_stride_b1 + (long long)it.h * p.gate_stride_b2 +
+                           (long long)qrow * p.gate_stride_s;
+        }
       }
       if (!kTcBias) {
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::bias_empty + bst));
+        if (++bst == kBiasStages) { bst = 0; b_par ^= 1; }
       }
-      ++bcount;
-      kt_stage += (uint32_t)it.gv;
-      while (kt_stage >= nkv) { kt_stage -= nkv; ++kt_round; }
+      if (kScalesQ && kt == scale_kt && item + (int)gridDim.x < p.n_items &&
+          !scale_own_q<kMixed>(c, item + gridDim.x, icount + 1, wg, wq, lane))
+        return;
     }
-
-
-    // ---- epilogue: O / l -> bf16 -> global, once this warpgroup's last P V has finished (the
-    // other warpgroup may still be working on its own streams)
-    if (kDebug && last_ts != nullptr) last_ts[5] = clock64();
-    if (wg < it.gv) AF3K_WAIT_WARP(c, BarIdx::kv_empty + (int)prev_stage, prev_round & 1);
-    // Its last P V has finished: nothing is left to wait for in front of the next tile.  (The K/V stage's barrier could not
-    // tell a warpgroup that has no stream for a while: it moves on by laps.)
-    prev_pending = false;
+  }
+  // the last stream's result
+  if (st.done_o != 0) {
+    close_tile(st);
+    AF3K_WAIT_WARP(c, BarIdx::pv_done + wg, st.pv_par);
     tc_fence_after();
-    if (kDebug && last_ts != nullptr) last_ts[6] = clock64();
-#pragma unroll 1
-    for (int s = wg; s < it.gv; s += 2) {
-      const int qrow = stream_qt(p, it, s) * kTile + row;
-      const float inv = __frcp_rn(s == wg ? l_st[0] : l_st[1]);
-      const uint32_t o_taddr = c.tmem + lane_sel + kOCol + s * p.nv;
-      __nv_bfloat16* orow = p.out + (long long)stream_row(p, it, s) * p.out_stride_b1 +
-                            (long long)it.h * p.out_stride_b2 + (long long)qrow * p.out_stride_s;
-      const __nv_bfloat16* grow = nullptr;
-      if constexpr (kGate)
-        grow = p.gate + (long long)stream_row(p, it, s) * p.gate_stride_b1 + (long long)it.h * p.gate_stride_b2 + (long long)qrow * p.gate_stride_s;
-#pragma unroll 1
-      for (int c0 = 0; c0 < p.nv; c0 += 16) {
-        uint32_t o[16];
-        tmem_ld_x16(o_taddr + c0, o);
-        tc_wait_ld();
-        if (kDebug && p.debug != nullptr && blockIdx.x == 0 && icount == 0 && s == 0) {
-          float* dbg = p.debug + (size_t)row * kTile;
-#pragma unroll
-          for (int i = 0; i < 16; ++i) dbg[kDbgO + c0 + i] = __uint_as_float(o[i]);
-          dbg[kDbgML + 0] = m_st[0];
-          dbg[kDbgML + 1] = l_st[0];
-        }
-        if (qrow < p.Sq) {
-#pragma unroll
-          for (int hseg = 0; hseg < 2; ++hseg) {
-            if (c0 + hseg * 8 + 8 <= p.D) {
-              if constexpr (kGate) {
-                const uint4 gv = *reinterpret_cast<const uint4*>(grow + c0 + hseg * 8);
-                const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                  const float g = __uint_as_float((e & 1) ? gw[e >> 1] & 0xffff0000u : gw[e >> 1] << 16);
-                  o[hseg * 8 + e] = __float_as_uint(__uint_as_float(o[hseg * 8 + e]) * sigmoid_f32(g));
-                }
-              }
-              uint4 v;
-              v.x = pack_bf16x2(__uint_as_float(o[hseg * 8 + 0]) * inv, __uint_as_float(o[hseg * 8 + 1]) * inv);
-              v.y = pack_bf16x2(__uint_as_float(o[hseg * 8 + 2]) * inv, __uint_as_float(o[hseg * 8 + 3]) * inv);
-              v.z = pack_bf16x2(__uint_as_float(o[hseg * 8 + 4]) * inv, __uint_as_float(o[hseg * 8 + 5]) * inv);
-              v.w = pack_bf16x2(__uint_as_float(o[hseg * 8 + 6]) * inv, __uint_as_float(o[hseg * 8 + 7]) * inv);
-              *reinterpret_cast<uint4*>(orow + c0 + hseg * 8) = v;
-            }
-          }
-        }
-      }
-    }
-    tc_fence_before();
-    __syncwarp();
-    if (lane == 0 && wg < it.gv) mbar_arrive(bar_addr(c, BarIdx::epi_done + wg));   // (once per item with a stream of its own)
-    if (kDebug && last_ts != nullptr) last_ts[7] = clock64();
+    float* dbg_o = kDebug && p.debug != nullptr && blockIdx.x == 0 && wg == 0 && p.n_items == 1 && p.n_streams == 1 ? p.debug + (size_t)row * kTile : nullptr;
+    store_result<kDebug, kGate>(c, st, dbg_o);
   }
 }
 
@@ -1226,6 +1178,7 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
+    *const_cast<WaitBlock*>(wait_block_of(c.bars)) = WaitBlock{p.wait_limit, p.status, &abort_flag};
     prefetch_tensormap(&tm_q);
     prefetch_tensormap(&tm_k);
     prefetch_tensormap(&tm_v);
@@ -1233,10 +1186,10 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     for (int i = 0; i < 2 * kMaxStreams; ++i) {
       mbar_init(bar_addr(c, BarIdx::q_full + i), 1);
       mbar_init(bar_addr(c, BarIdx::q_empty + i), 1);
-      mbar_init(bar_addr(c, BarIdx::q_scaled + i), 1);
+      mbar_init(bar_addr(c, BarIdx::q_scaled + i), 4);
     }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(bar_addr(c, BarIdx::epi_done + i), 4);
+      mbar_init(bar_addr(c, BarIdx::pv_done + i), 1);
       mbar_init(bar_addr(c, BarIdx::s_full + i), 1);
       mbar_init(bar_addr(c, BarIdx::s_free + i), 4);
       mbar_init(bar_addr(c, BarIdx::p_ready + i), 4);
@@ -1288,7 +1241,7 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     } else if (warp == 1) {
       qk_issuer_role<kDebug, kTcBias, kFp8, kMixed>(c);
     } else if (warp == 2) {
-      pv_issuer_role<kDebug, !kFp8, kMixed>(c, lane);
+      pv_issuer_role<kDebug, kMixed>(c);
     } else if (warp == 3) {
       if (p.mask_col) mask_writer_role<kMixed>(c, lane);
     }
@@ -1303,7 +1256,7 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
         else            bias_convert_ragged_role<uint16_t>(c, warp & 3, lane);
       }
     } else {
-      softmax_role<kDebug, kTcBias, kGate, kMixed>(c, (warp - 4) >> 2, warp & 3, lane);
+      softmax_role<kDebug, kTcBias, kGate, kMixed, !kFp8>(c, (warp - 4) >> 2, warp & 3, lane);
     }
   }
 
