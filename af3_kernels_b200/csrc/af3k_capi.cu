@@ -259,7 +259,8 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
 
   const int budget = dev.max_smem_optin - kStaticSmemReserve;
   p.mask_col = 1;   // set for real in the launch path once the mask pointer is known
-  const int fixed = kBiasStages * kBiasTileBytes + (int)kBarrierBlockBytes +
+  constexpr int kSharedBiasStages = 2;
+  const int fixed = kSharedBiasStages * kBiasTileBytes + (int)kBarrierBlockBytes +
                     (kMaxKvStages + 2) * (int)kMaskPanelBytes /*ones column, mask ring, zero block*/ +
                     (int)kIdentBytes;
   const int kv_stage = (int)(p.k_tile_bytes + p.v_tile_bytes);
@@ -336,10 +337,28 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   p.div_q = make_divisor((uint32_t)tiles_of(best_split));
   p.div_h = make_divisor((uint32_t)p.B2);
 
+  // Streams that are query tiles bring a bias tile for each of their logits tiles (32 KB beside 16 KB of K and V), and with
+  // two stages a load's latency was the time between two tiles: a third stage where K and V keep one more than that.  (Nothing
+  // is gained where a lone query tile uses them, and the warps that convert an fp32 bias get slower: 512 tokens 10.7 -> 12.7 us.)
+  // The Q tiles of a CTA's only item need no second buffer.  16 heads, bf16 bias, us, two stages -> three -> four: 1536 tokens
+  // 29.1 -> 24.5 -> 26.0, 2048 tokens 35.0 -> 30.5 -> 31.4.
+  p.bias_stages = kSharedBiasStages;
+  if (p.q_split) {
+    if (p.n_items <= ctas) p.q_buffers = 1;
+    int lead = 0;
+    for (int nb = kSharedBiasStages; nb <= kMaxBiasStages; ++nb) {
+      int stages = (budget - fixed - (nb - kSharedBiasStages) * kBiasTileBytes - p.q_buffers * p.n_streams * (int)p.q_tile_bytes) / kv_stage;
+      if (stages > kMaxKvStages) stages = kMaxKvStages;
+      if (stages < 2) break;
+      const int l = nb < stages - 1 ? nb : stages - 1;     // logits tiles whose operands can be under way
+      if (l > lead) { lead = l; p.bias_stages = nb; p.kv_stages = stages; }
+    }
+  }
+
   uint32_t off = 0;
   p.off_q = off;      off += p.q_buffers * p.n_streams * p.q_tile_bytes;
   p.off_kv = off;     off += p.kv_stages * kv_stage;
-  p.off_bias = off;   off += kBiasStages * kBiasTileBytes;
+  p.off_bias = off;   off += p.bias_stages * kBiasTileBytes;
   p.off_bar = off;    off += kBarrierBlockBytes;
   p.off_ones = off;   off += kMaskPanelBytes;
   p.off_mcol = off;   off += kMaxKvStages * kMaskPanelBytes;

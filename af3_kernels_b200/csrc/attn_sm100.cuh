@@ -63,7 +63,7 @@ constexpr int kMaxStreams = 4;     // pair rows per work item (two per softmax w
 constexpr uint32_t kSCol = 0, kPCol = 2 * 128, kOCol = 2 * 128 + 2 * 64;
 constexpr float kLazyRescaleLog2 = 8.0f;   // keep a stale row max while exp2 arguments stay <= 8
 constexpr int kTailRows = 2;       // pair rows of an item behind the last full round: both softmax warpgroups have work
-constexpr int kBiasStages = 2;
+constexpr int kMaxBiasStages = 3;
 constexpr int kBiasTileBytes = kTile * kTile * 2;  // bf16, two 128B-swizzled boxes of 64 columns
 constexpr int kMaxKvStages = 6;
 constexpr uint32_t kNarrowOff = kTile * 64;        // qk_narrow: channels 32 .. 47 behind the first 32
@@ -124,6 +124,7 @@ struct AttnParams {
   int qk_ksteps;         // number of 32-byte K steps of the first GEMM
   int nv;                // N of the second GEMM: D rounded up to 16
   int kv_stages;
+  int bias_stages;
   int q_buffers;         // 2: Q tiles double-buffered by item (the next item's land while this one runs); 1: single
   int scale_q;           // 1: bf16 q/k, the Q tiles are multiplied by `scale` in shared memory
   float scale;           // softmax scale; multiplied by q_scale[h] * k_scale[h] when those are set
@@ -158,12 +159,12 @@ struct BarIdx {
   static constexpr int s_free = 2;      // [2]  softmax warpgroup has the logits in registers
   static constexpr int p_ready = 4;     // [2]  P written (and O rescaled if needed)
   static constexpr int pv_done = 6;     // [2]  the warpgroup's last P V has finished: its P buffer and that O are free
-  static constexpr int bias_full = 8;   // [kBiasStages]
-  static constexpr int bias_empty = 10; // [kBiasStages]
-  static constexpr int kv_full = 12;    // [kMaxKvStages]
-  static constexpr int kv_empty = 12 + kMaxKvStages;       // P V of the stage's tile finished
+  static constexpr int bias_full = 8;   // [kMaxBiasStages]
+  static constexpr int bias_empty = bias_full + kMaxBiasStages;
+  static constexpr int kv_full = bias_empty + kMaxBiasStages;   // [kMaxKvStages]
+  static constexpr int kv_empty = kv_full + kMaxKvStages;       // P V of the stage's tile finished
   // Q tiles: slot = (Q buffer) * kMaxStreams + stream
-  static constexpr int q_full = 12 + 2 * kMaxKvStages;       // [2 * kMaxStreams]  Q tile landed
+  static constexpr int q_full = kv_empty + kMaxKvStages;       // [2 * kMaxStreams]  Q tile landed
   static constexpr int q_empty = q_full + 2 * kMaxStreams;   // [2 * kMaxStreams]  last Q K^T of the stream finished
   static constexpr int q_scaled = q_empty + 2 * kMaxStreams; // [2 * kMaxStreams]  the softmax warpgroup's warps have scaled the Q tile
   static constexpr int count = q_scaled + 2 * kMaxStreams;
@@ -294,7 +295,7 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
   const WaitBlock* wait_block = wait_block_of(c.bars);
   uint32_t icount = 0;
   uint32_t st = 0, lap = 0, bst = 0, blap = 0;     // K/V and bias ring: stage, laps before
-  const uint32_t nkv = p.kv_stages;
+  const uint32_t nkv = p.kv_stages, n_bias = p.bias_stages;
   // With two Q buffers the tiles of the next item are requested while the current item runs, so
   // that they are in place (and scaled) when it ends; with one (tiles too large for two), as
   // soon as the current item's K/V loads are all issued.  (Not before a K/V stage of this item has come free: the loads wait
@@ -336,7 +337,7 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
           mbar_arrive_expect_tx(bfull, kBiasTileBytes);
           tma_load_3d(bdst, tm_bias, bfull, kt * kTile, stream_qt(p, it, s) * kTile, it.h);
           tma_load_3d(bdst + kBiasTileBytes / 2, tm_bias, bfull, kt * kTile + 64, stream_qt(p, it, s) * kTile, it.h);
-          if (++bst == kBiasStages) { bst = 0; ++blap; }
+          if (++bst == n_bias) { bst = 0; ++blap; }
         }
         if (lap != 0) AF3K_WAIT(c, BarIdx::kv_empty + st, (lap - 1) & 1);
         const uint32_t full = bar_addr(c, BarIdx::kv_full + st);
@@ -563,7 +564,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
           // every bias MMA that reads this stage is issued: the stage is free when they finish
           if (leader) tc_commit(bar_addr(c, BarIdx::bias_empty + bst));
           __syncwarp();
-          if (++bst == kBiasStages) { bst = 0; b_par ^= 1; }
+          if (++bst == (uint32_t)p.bias_stages) { bst = 0; b_par ^= 1; }
         }
       }
     }
@@ -997,7 +998,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
       if (!kTcBias) {
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::bias_empty + bst));
-        if (++bst == kBiasStages) { bst = 0; b_par ^= 1; }
+        if (++bst == (uint32_t)p.bias_stages) { bst = 0; b_par ^= 1; }
       }
       if (kScalesQ && kt == scale_kt && item + (int)gridDim.x < p.n_items &&
           !scale_own_q<kMixed>(c, item + gridDim.x, icount + 1, wg, wq, lane))
@@ -1088,11 +1089,10 @@ __device__ void bias_convert_role(const Ctx& c, int wq, int lane) {
 #pragma unroll
   for (int half = 0; half < 2; ++half) load(it, 0, half);
 #pragma unroll 1
-  for (uint32_t n = 0; item < p.n_items; ++n) {
-    const uint32_t bst = n % kBiasStages;
+  for (uint32_t bst = 0, lap = 0; item < p.n_items;) {
     const uint32_t tile = c.smem + p.off_bias + bst * kBiasTileBytes;
     // the bias MMAs of the stage's tile before must have finished
-    if (n >= kBiasStages) AF3K_WAIT_WARP(c, BarIdx::bias_empty + bst, ((n / kBiasStages) - 1) & 1);
+    if (lap != 0) AF3K_WAIT_WARP(c, BarIdx::bias_empty + bst, (lap - 1) & 1);
     if (++kt == p.n_kt) {                    // the tile after this one
       kt = 0;
       item += gridDim.x;
@@ -1106,6 +1106,7 @@ __device__ void bias_convert_role(const Ctx& c, int wq, int lane) {
     fence_proxy_async_smem();    // make the generic-proxy stores visible to the tensor core
     __syncwarp();
     if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::bias_full + bst));
+    if (++bst == (uint32_t)p.bias_stages) { bst = 0; ++lap; }
   }
 }
 
@@ -1115,13 +1116,12 @@ template <typename T>
 __device__ void bias_convert_ragged_role(const Ctx& c, int wq, int lane) {
   const AttnParams& p = *c.p;
   const int row0 = wq * 32;
-  uint32_t n = 0;
+  uint32_t bst = 0, lap = 0;
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
     const Item it = decode_item<false>(p, item);
 #pragma unroll 1
-    for (int kt = 0; kt < p.n_kt; ++kt, ++n) {
-      const uint32_t bst = n % kBiasStages;
+    for (int kt = 0; kt < p.n_kt; ++kt) {
       const uint32_t tile = c.smem + p.off_bias + bst * kBiasTileBytes;
       const int first = it.qt * kTile + row0, last = min(31, p.Sq - 1 - first), key = kt * kTile + 4 * lane;
       const T* src = static_cast<const T*>(p.bias_src) + it.h * p.bias_stride_h + first * p.bias_stride_r + key;
@@ -1132,7 +1132,7 @@ __device__ void bias_convert_ragged_role(const Ctx& c, int wq, int lane) {
         for (int r = 0; r < kConvertRows; ++r)
 #pragma unroll
           for (int e = 0; e < 4; ++e) x[r][e] = load_if(src + min(r0 + r, last) * p.bias_stride_r + e, last >= 0 && key + e < p.Sk ? 1u : 0u);
-        if (r0 == 0 && n >= kBiasStages) AF3K_WAIT_WARP(c, BarIdx::bias_empty + bst, ((n / kBiasStages) - 1) & 1);
+        if (r0 == 0 && lap != 0) AF3K_WAIT_WARP(c, BarIdx::bias_empty + bst, (lap - 1) & 1);
 #pragma unroll
         for (int r = 0; r < kConvertRows; ++r)
           store_bias4(tile, row0 + r0 + r, lane, staged_pair(x[r][0], x[r][1]), staged_pair(x[r][2], x[r][3]));
@@ -1140,6 +1140,7 @@ __device__ void bias_convert_ragged_role(const Ctx& c, int wq, int lane) {
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::bias_full + bst));
+      if (++bst == (uint32_t)p.bias_stages) { bst = 0; ++lap; }
     }
   }
 }
@@ -1194,7 +1195,7 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
       mbar_init(bar_addr(c, BarIdx::s_free + i), 4);
       mbar_init(bar_addr(c, BarIdx::p_ready + i), 4);
     }
-    for (int i = 0; i < kBiasStages; ++i) {
+    for (int i = 0; i < kMaxBiasStages; ++i) {
       mbar_init(bar_addr(c, BarIdx::bias_full + i), kConvert ? 4 : 1);
       // freed by the bias MMAs' completion (bf16 q/k) or by the eight softmax warps (fp8 q/k)
       mbar_init(bar_addr(c, BarIdx::bias_empty + i), kTcBias ? 1 : 8);
