@@ -671,12 +671,11 @@ __device__ __forceinline__ void logits_half(uint32_t (&xr)[kTile], uint32_t bias
   }
 }
 
-// Row maximum over 64 finished logits (bf16 q/k: the tensor core has already applied scale, bias
-// and mask).
-template <int kCol0>
-__device__ __forceinline__ void max_half(const uint32_t (&xr)[kTile], float& mxa, float& mxb) {
+// Row maximum over finished logits (bf16 q/k: the tensor core has already applied scale, bias and mask).
+template <int kCol0, int kCol1>
+__device__ __forceinline__ void row_max(const uint32_t (&xr)[kTile], float& mxa, float& mxb) {
 #pragma unroll
-  for (int i = kCol0; i < kCol0 + 64; i += 4) {
+  for (int i = kCol0; i < kCol1; i += 4) {
     mxa = max3(mxa, __uint_as_float(xr[i]), __uint_as_float(xr[i + 1]));
     mxb = max3(mxb, __uint_as_float(xr[i + 2]), __uint_as_float(xr[i + 3]));
   }
@@ -796,9 +795,8 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, flo
   tc_fence_after();
   if (kDebug && ts != nullptr) ts[1] = clock64();
   uint32_t xr[kTile];
-  tmem_ld_x32(s_taddr + 0, &xr[0]);
-  tmem_ld_x32(s_taddr + 32, &xr[32]);
-  // Under the loads: what is left of the tile before, and a look whether its P V has finished.
+  tmem_ld_x32(s_taddr, &xr[0]);
+  // Under the load: what is left of the tile before, and a look whether its P V has finished.
   close_tile(st);
   if (first_kt) { st.m[0] = -INFINITY; st.l[0] = 0.f; }
   const bool pv_ok = mbar_test_wait(bar_addr(c, BarIdx::pv_done + wg), st.pv_par) || !st.started;
@@ -806,12 +804,11 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, flo
   float mt;
   {
     tc_wait_ld();
+    tmem_ld_x32(s_taddr + 32, &xr[32]);
     tmem_ld_x32(s_taddr + 64, &xr[64]);
     tmem_ld_x32(s_taddr + 96, &xr[96]);
-    const uint64_t scale2 = pack_f32x2(scale, scale);
     float mxa = -INFINITY, mxb = -INFINITY;
-    if (kTcBias) max_half<0>(xr, mxa, mxb);
-    else         logits_half<0>(xr, bias_row, row7, scale2, mxa, mxb);
+    if (kTcBias) row_max<0, 32>(xr, mxa, mxb);
     tc_wait_ld();
     // the logits are in registers: hand the S buffer back so that the next Q K^T can start
     tc_fence_before();
@@ -821,8 +818,13 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, flo
 #pragma unroll
       for (int i = 0; i < kTile; ++i) dbg[kDbgS + i] = __uint_as_float(xr[i]);
     }
-    if (kTcBias) max_half<64>(xr, mxa, mxb);
-    else         logits_half<64>(xr, bias_row, row7, scale2, mxa, mxb);
+    if (kTcBias) {
+      row_max<32, kTile>(xr, mxa, mxb);
+    } else {
+      const uint64_t scale2 = pack_f32x2(scale, scale);
+      logits_half<0>(xr, bias_row, row7, scale2, mxa, mxb);
+      logits_half<64>(xr, bias_row, row7, scale2, mxa, mxb);
+    }
     mt = fmaxf(mxa, mxb);
   }
   if (kDebug && ts != nullptr) ts[2] = clock64() + (long long)(mt == 123.456f);   // logits and row maximum in registers
@@ -852,31 +854,27 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, flo
   const uint64_t nm2 = pack_f32x2(-m_use, -m_use);
   const uint64_t nml2 = pack_f32x2(nml, nml);
   uint64_t suma = pack_f32x2(0.f, 0.f), sumb = suma;
+  uint32_t pk[kTile / 2];        // P as bf16, two keys per 32-bit TMEM column: the A operand of the second GEMM
 #pragma unroll
-  for (int cidx = 0; cidx < 8; ++cidx) {
-    uint32_t pk[8];
+  for (int i = 0; i < kTile / 2; ++i) {
+    float y0, y1;
+    const uint64_t x2 = pack_f32x2(__uint_as_float(xr[2 * i]), __uint_as_float(xr[2 * i + 1]));
+    if (kTcBias) unpack_f32x2(fma_f32x2(x2, l2e2, nml2), y0, y1);
+    else         unpack_f32x2(mul_f32x2(add_f32x2(x2, nm2), l2e2), y0, y1);
+    const float p0 = ex2_approx(y0);
+    const float p1 = ex2_approx(y1);
+    // (two chains: one takes 9 % longer, 2048 fp8 rows 9 970 -> 10 840 us, four 1 %)
+    if (i & 1) sumb = add_f32x2(sumb, pack_f32x2(p0, p1));
+    else       suma = add_f32x2(suma, pack_f32x2(p0, p1));
+    pk[i] = pack_bf16x2(p0, p1);
+    // Few and wide stores: 2048 fp8 rows, eight of 8 columns 10 370 us, four of 16 10 050, 32 and twice 16 9 900, two of 32 10 040.
+    if (i == 31) tmem_st_x32(p_taddr, pk);
+    if (i == 47) tmem_st_x16(p_taddr + 32, pk + 32);
+    if (i == 63) tmem_st_x16(p_taddr + 48, pk + 48);
+  }
+  if (kDebug && dbg != nullptr) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int col = cidx * 16 + 2 * i;
-      float y0, y1;
-      const uint64_t x2 = pack_f32x2(__uint_as_float(xr[col]), __uint_as_float(xr[col + 1]));
-      if (kTcBias) unpack_f32x2(fma_f32x2(x2, l2e2, nml2), y0, y1);
-      else         unpack_f32x2(mul_f32x2(add_f32x2(x2, nm2), l2e2), y0, y1);
-      const float p0 = ex2_approx(y0);
-      const float p1 = ex2_approx(y1);
-      if (i & 1) sumb = add_f32x2(sumb, pack_f32x2(p0, p1));
-      else       suma = add_f32x2(suma, pack_f32x2(p0, p1));
-      pk[i] = pack_bf16x2(p0, p1);
-    }
-    if (kDebug && dbg != nullptr) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) dbg[kDbgP + cidx * 8 + i] = __uint_as_float(pk[i]);
-    }
-    // P as bf16, two keys per 32-bit TMEM column: the A operand of the second GEMM
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
-                 ::"r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]),
-                 "r"(p_taddr + cidx * 8)
-                 : "memory");
+    for (int i = 0; i < kTile / 2; ++i) dbg[kDbgP + i] = __uint_as_float(pk[i]);
   }
   if (kDebug && ts != nullptr) ts[6] = clock64();     // last exponential issued
   // What else has to be done with the accumulators before the next P V may write one.
