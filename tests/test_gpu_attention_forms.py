@@ -290,3 +290,39 @@ def test_heads_of_33_to_48_channels(cuda_device, B1, B2, S, D):
     q, k, v, mask, bias = _inputs(B1, B2, S, D, S + D)
     q, k = (t.transpose(1, 2).contiguous().transpose(1, 2) for t in (q, k))
     _check(_call(cuda_device, q, k, v, mask, bias), O.oracle_fp32(q, k, v, mask, bias), (B1, B2, S, D))
+
+
+@pytest.mark.parametrize("B1,B2,S,D", [(12, 2, 100, 32), (12, 2, 100, 64), (14, 2, 128, 16), (6, 2, 200, 48), (9, 2, 300, 32), (8, 2, 260, 64), (1, 4, 100, 32),
+                                       (1, 6, 129, 64)])
+@pytest.mark.parametrize("scale", [None, 1.0])
+def test_several_items_on_one_cta(cuda_device, B1, B2, S, D, scale):
+    """One, two or four streams and one to three key tiles per item, many items per CTA: a stream's result is stored under the tile
+    that comes next, and the next item's Q tiles are scaled meanwhile (not at all with a scale of 1).  Logits that grow by more than the
+    lazy bound between key tiles have the accumulator next to it rescaled at the same time."""
+    q, k, v, mask, bias = _inputs(B1, B2, S, D, S + D + B1)
+    if scale:
+        q = (q * D ** -0.5).to(torch.bfloat16)
+    bias[..., 128:] += 12
+    bias[..., 256:] += 12
+    kw = {"softmax_scale": scale} if scale else {}
+    ref = O.oracle_fp32(q, k, v, mask, bias)
+    if scale:
+        logits = q.float() @ k.float().transpose(-1, -2) + bias.float()
+        ref = torch.softmax(logits.masked_fill(~mask[:, None, None, :], -1e9), -1) @ v.float()
+    out = _call(cuda_device, q, k, v, mask, bias, **kw)
+    _check(out, ref, (B1, B2, S, D))
+    for other in ({"max_ctas": 2}, {"max_ctas": 3}, {"max_ctas": 2, "rows_per_item": 2}, {"rows_per_item": 1}):
+        assert torch.equal(_call(cuda_device, q, k, v, mask, bias, **kw, **other), out), other
+
+
+@pytest.mark.parametrize("S", [300, 640, 1100, 1152])
+@pytest.mark.parametrize("D", [8, 24, 32, 48, 64])
+def test_bias_stages_of_query_tile_streams(cuda_device, S, D):
+    """Two query tiles per item bring three bias stages (two from 33 channels on), one per item and shared ones two: more key tiles than
+    stages, an odd number of query tiles, one item and several per CTA."""
+    q, k, v, mask, bias = _inputs(1, 2, S, D, S + D)
+    out = _call(cuda_device, q, k, v, mask, bias)
+    _check(out, O.oracle_fp32(q, k, v, mask, bias), (S, D))
+    tiles = (S + 127) // 128
+    for ctas in (1, 3, tiles + tiles % 2):
+        assert torch.equal(_call(cuda_device, q, k, v, mask, bias, max_ctas=ctas), out), ctas
