@@ -298,9 +298,10 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
   const uint32_t nkv = p.kv_stages, n_bias = p.bias_stages;
   // With two Q buffers the tiles of the next item are requested while the current item runs, so
   // that they are in place (and scaled) when it ends; with one (tiles too large for two), as
-  // soon as the current item's K/V loads are all issued.  (Not before a K/V stage of this item has come free: the loads wait
-  // for the last Q K^T of the item before, and the K/V ring would run empty meanwhile.)
-  const int q_at = p.q_buffers == 2 ? min((int)(nkv / (uint32_t)p.n_streams) + 1, p.n_kt) : p.n_kt;
+  // soon as the current item's K/V loads are all issued.  When a K/V stage of this item has come free, the last item's Q K^T have
+  // finished, which the loads wait for (5 x 1536 tokens of 48 channels 86.9 us, 87.5 behind the first key tile; others the same), but where they
+  // are scaled in front of the last key tile, so that this is not left over (256 rows of two key tiles, 16 channels: 29.5 us, 30.7 behind it).
+  const int q_at = p.q_buffers == 2 ? min((int)(nkv / (uint32_t)p.n_streams) + 1, max(p.n_kt - p.scale_q, 1)) : p.n_kt;
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
     const Item it = decode_item<kMixed>(p, item);
