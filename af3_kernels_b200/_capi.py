@@ -30,6 +30,7 @@ EXPORTED_SYMBOLS = (
     "af3k_last_launch_count",
     "af3k_set_wait_limit_cycles",
     "af3k_describe_plan",
+    "af3k_describe_plan_streams",
     "af3k_dot_product_attention_convert",
     "af3k_pair_bias_status",
     "af3k_pair_front",
@@ -137,6 +138,8 @@ def load() -> ctypes.CDLL:
     lib.af3k_set_wait_limit_cycles.argtypes = [i64]
     lib.af3k_describe_plan.restype = ctypes.c_int
     lib.af3k_describe_plan.argtypes = [dp, ctypes.POINTER(ctypes.c_int32)]
+    lib.af3k_describe_plan_streams.restype = ctypes.c_int
+    lib.af3k_describe_plan_streams.argtypes = [dp, ctypes.POINTER(ctypes.c_int32)]
     lib.af3k_debug_set_dump.restype = None
     lib.af3k_debug_set_dump.argtypes = [vp]
     lib.af3k_selftest_wait_timeout.restype = ctypes.c_int
@@ -166,7 +169,8 @@ def check(code: int) -> None:
 
 
 def describe_plan(desc: AttentionDesc) -> dict:
-    out = (ctypes.c_int32 * 6)()
+    out, streams = (ctypes.c_int32 * 6)(), (ctypes.c_int32 * 4)()
     check(load().af3k_describe_plan(ctypes.byref(desc), out))
-    keys = ("rows_per_item", "kv_stages", "items", "grid", "smem_bytes", "tmem_cols")
-    return dict(zip(keys, list(out)))
+    check(load().af3k_describe_plan_streams(ctypes.byref(desc), streams))
+    keys = ("rows_per_item", "kv_stages", "items", "grid", "smem_bytes", "tmem_cols", "streams", "query_tile_streams", "q_buffers", "bias_stages")
+    return dict(zip(keys, [*out, *streams]))

@@ -670,8 +670,8 @@ int af3k_dot_product_attention_convert(const af3k_attention_desc* desc, const vo
 
 void af3k_debug_set_dump(float* dump_dev) { g_debug_dump.store(dump_dev); }
 
-int af3k_describe_plan(const af3k_attention_desc* desc, int32_t* out6) {
-  if (desc == nullptr || out6 == nullptr) return AF3K_ERR_NULL_POINTER;
+static int describe(const af3k_attention_desc* desc, Plan* plan) {
+  if (desc == nullptr) return AF3K_ERR_NULL_POINTER;
   int rc = validate(*desc);
   if (rc != AF3K_OK) return rc;
   DeviceInfo dev;
@@ -685,8 +685,12 @@ int af3k_describe_plan(const af3k_attention_desc* desc, int32_t* out6) {
     dev.sm_count = prop.multiProcessorCount;
     dev.max_smem_optin = (int)prop.sharedMemPerBlockOptin;
   }
+  return make_plan(*desc, dev, plan);
+}
+
+int af3k_describe_plan(const af3k_attention_desc* desc, int32_t* out6) {
   Plan plan;
-  rc = make_plan(*desc, dev, &plan);
+  int rc = out6 == nullptr ? AF3K_ERR_NULL_POINTER : describe(desc, &plan);
   if (rc != AF3K_OK) return rc;
   out6[0] = plan.p.G;
   out6[1] = plan.p.kv_stages;
@@ -694,6 +698,17 @@ int af3k_describe_plan(const af3k_attention_desc* desc, int32_t* out6) {
   out6[3] = plan.grid;
   out6[4] = (int32_t)plan.smem_bytes;
   out6[5] = (int32_t)kOCol + plan.p.n_streams * plan.p.nv;
+  return AF3K_OK;
+}
+
+int af3k_describe_plan_streams(const af3k_attention_desc* desc, int32_t* out4) {
+  Plan plan;
+  int rc = out4 == nullptr ? AF3K_ERR_NULL_POINTER : describe(desc, &plan);
+  if (rc != AF3K_OK) return rc;
+  out4[0] = plan.p.n_streams;
+  out4[1] = plan.p.q_split;
+  out4[2] = plan.p.q_buffers;
+  out4[3] = plan.p.bias_stages;
   return AF3K_OK;
 }
 

@@ -282,8 +282,12 @@ __device__ __forceinline__ int stream_row(const AttnParams& p, const Item& it, i
 __device__ __forceinline__ int stream_qt(const AttnParams& p, const Item& it, int s) { return p.q_split ? it.qt + s : it.qt; }
 
 // Q buffer of the CTA's j-th item and how often that buffer was used before.  (kMixed) An item with fewer streams than the Q
-// buffers hold takes the slots of the others through their phases all the same (an arrival on each of their barriers), so
-// that one count serves all slots: counting every slot's own uses in the issuer's loop cost 2 - 5 %.
+// buffers hold takes the slots of the others through their phases all the same, so that one count serves all slots: counting
+// every slot's own uses in the issuer's loop cost 2 - 5 %.  Each role does there what it does for a slot in use, less the copy,
+// the scaling and the MMAs: a wait by parity cannot tell a phase from the one two before it, so whoever waits on a slot's barriers
+// at all must wait for every phase of theirs and must itself be waited for before the phase after the next can end.  The producer
+// arrives (q_full), the softmax warps wait for that and arrive (q_scaled; nobody does where Q is not scaled), the issuer waits for that and
+// arrives (q_empty), the producer waits for that.  A warpgroup without a stream in an item (a lone query tile) is held by nothing else.
 __device__ __forceinline__ uint32_t q_buf(const AttnParams& p, uint32_t j) { return p.q_buffers == 2 ? (j & 1u) : 0u; }
 __device__ __forceinline__ uint32_t q_use(const AttnParams& p, uint32_t j) { return p.q_buffers == 2 ? (j >> 1) : j; }
 
@@ -569,15 +573,16 @@ __device__ void qk_issuer_role(const Ctx& c) {
         }
       }
     }
-    // the slots that this item does not use: their scaling and their release (this warp is the one that waits for the
-    // former and, through the producer, for the latter, so neither can run ahead of it)
+    // the slots that this item does not use (where Q is not scaled, the producer's arrival on q_full came before the K/V loads that
+    // were waited for above)
     if (kMixed) {
-      if (leader)
-        for (int s = gv; s < p.n_streams; ++s) {
-          for (int w = 0; w < 4; ++w) mbar_arrive(bar_addr(c, BarIdx::q_scaled + (int)q_buf(p, icount) * kMaxStreams + s));
-          mbar_arrive(bar_addr(c, BarIdx::q_empty + (int)q_buf(p, icount) * kMaxStreams + s));
-        }
-      __syncwarp();
+#pragma unroll 1
+      for (int s = gv; s < p.n_streams; ++s) {
+        const int qslot = (int)q_buf(p, icount) * kMaxStreams + s;
+        if (p.scale_q) AF3K_WAIT_WARP_C(c, BarIdx::q_scaled + qslot, q_use(p, icount) & 1);
+        if (leader) mbar_arrive(bar_addr(c, BarIdx::q_empty + qslot));
+        __syncwarp();
+      }
     }
   }
 }
@@ -927,10 +932,12 @@ __device__ __forceinline__ bool scale_own_q(const Ctx& c, int item, uint32_t j, 
   const Item it = decode_item<kMixed>(p, item);
   const uint32_t buf = q_buf(p, j), par = q_use(p, j) & 1, bytes = p.q_tile_bytes >> 2;
 #pragma unroll 1
-  for (int s = wg; s < it.gv; s += 2) {
+  for (int s = wg; s < (kMixed ? p.n_streams : it.gv); s += 2) {
     const int slot = (int)buf * kMaxStreams + s;
     if (!softmax_wait(c, BarIdx::q_full + slot, par)) return false;
-    scale_q(c.smem + p.off_q + (buf * p.n_streams + s) * p.q_tile_bytes + wq * bytes, bytes, p.scale, lane, bar_addr(c, BarIdx::q_scaled + slot));
+    // (nothing is in a slot that the item does not use: an arrival only)
+    scale_q(c.smem + p.off_q + (buf * p.n_streams + s) * p.q_tile_bytes + wq * bytes, kMixed && s >= it.gv ? 0u : bytes, p.scale, lane,
+            bar_addr(c, BarIdx::q_scaled + slot));
   }
   return true;
 }

@@ -179,6 +179,10 @@ void af3k_set_wait_limit_cycles(long long cycles);
  * the reference. */
 int af3k_describe_plan(const af3k_attention_desc* desc, int32_t* out6);
 
+/* The same plan's streams: out4 = {streams per work item, 1 if they are neighbouring query tiles of one pair row (0: pair
+ * rows), Q buffers per stream, bias ring stages}.  Diagnostic; no counterpart in the reference. */
+int af3k_describe_plan_streams(const af3k_attention_desc* desc, int32_t* out4);
+
 /* Diagnostic: when dump_dev is non-NULL, later attention calls run a debug build of the kernel
  * that writes block 0's first logits tile to dump_dev (4 * 128 * 128 floats: logits as the
  * tensor core delivers them - with bf16 q/k that is scale * q k^T + bias + mask value -, packed

@@ -83,6 +83,15 @@ def test_plan_reports_smaller_items(shape, qk, main, rest):
         assert plan["items"] == main + rest and plan["grid"] == 148
 
 
+@pytest.mark.parametrize("shape,streams", [((1, 16, 512, 32), (1, 0, 2, 2)), ((1, 16, 1536, 24), (2, 1, 1, 3)), ((1, 16, 2400, 64), (2, 1, 1, 2)),
+                                           ((3, 16, 1400, 48), (2, 1, 1, 2)), ((5, 16, 1536, 48), (2, 0, 1, 2)), ((768, 4, 768, 32), (4, 0, 2, 2))])
+def test_plan_reports_its_streams(shape, streams):
+    """Streams per item, whether they are query tiles, Q buffers, bias stages."""
+    plan = _capi.describe_plan(_desc(*shape, bias_dtype=_capi.AF3K_BF16))
+    assert tuple(plan[n] for n in ("streams", "query_tile_streams", "q_buffers", "bias_stages")) == streams
+    assert _capi.load().af3k_describe_plan_streams(None, (ctypes.c_int32 * 4)()) == 6
+
+
 def test_max_ctas_caps_the_grid():
     d = _desc(768, 4, 768, 32)
     full = _capi.describe_plan(d)

@@ -221,12 +221,13 @@ def _quantised(q, k):
     return q, k, {"q_scale": qs, "k_scale": ks}
 
 
-def _plan(B1, B2, S, D, fp8):
+def _plan(B1, B2, S, D, fp8=False, Sk=None, max_ctas=0):
+    Sk = Sk or S
     d = _capi.AttentionDesc()
-    d.B1, d.B2, d.Sq, d.Sk, d.D = B1, B2, S, S, D
-    for n in ("q_stride", "k_stride", "v_stride", "out_stride"):
-        getattr(d, n)[:] = [B2 * S * D, S * D, D]
-    d.bias_stride[:], d.mask_row_stride, d.softmax_scale = [S * S, S], S, D ** -0.5
+    d.B1, d.B2, d.Sq, d.Sk, d.D = B1, B2, S, Sk, D
+    for n, keys in (("q_stride", S), ("k_stride", Sk), ("v_stride", Sk), ("out_stride", S)):
+        getattr(d, n)[:] = [B2 * keys * D, keys * D, D]
+    d.bias_stride[:], d.mask_row_stride, d.softmax_scale, d.max_ctas = [S * Sk, Sk], Sk, D ** -0.5, max_ctas
     d.qk_dtype, d.bias_dtype = _capi.AF3K_FP8_E4M3 if fp8 else _capi.AF3K_BF16, _capi.AF3K_BF16
     return _capi.describe_plan(d)
 
@@ -326,3 +327,23 @@ def test_bias_stages_of_query_tile_streams(cuda_device, S, D):
     tiles = (S + 127) // 128
     for ctas in (1, 3, tiles + tiles % 2):
         assert torch.equal(_call(cuda_device, q, k, v, mask, bias, max_ctas=ctas), out), ctas
+
+
+@pytest.mark.parametrize("B1,B2,S,Sk,D,max_ctas,q_buffers", [
+    (1, 3, 300, 300, 64, 3, 1), (1, 3, 300, 200, 64, 3, 1), (1, 3, 300, 100, 32, 3, 2), (1, 7, 300, 300, 48, 5, 2), (1, 16, 2400, 2400, 64, 0, 1),
+    (3, 16, 1400, 1400, 48, 0, 1), (5, 16, 1660, 1660, 48, 0, 1)])
+def test_pair_of_query_tiles_behind_a_lone_one(cuda_device, B1, B2, S, Sk, D, max_ctas, q_buffers):
+    """CTAs that begin with a lone query tile, on which one softmax warpgroup has no stream, and go on with a pair of them: that
+    warpgroup scales the pair's second Q tile, from a slot that the lone tile's item went through without using it."""
+    plan = _plan(B1, B2, S, D, Sk=Sk, max_ctas=max_ctas)
+    tiles = (S + 127) // 128
+    lone = lambda item: item % (tiles // 2 + 1) == tiles // 2
+    assert tiles % 2 and plan["query_tile_streams"] and plan["q_buffers"] == q_buffers, plan
+    assert any(lone(c) and not lone(c + plan["grid"]) for c in range(plan["items"] - plan["grid"])), plan
+    q, k, v, mask, bias = _inputs(B1, B2, S, D, S + D, Sk)
+    out = _call(cuda_device, q, k, v, mask, bias, max_ctas=max_ctas)
+    _check(out, O.oracle_fp32(q, k, v, mask, bias), plan)
+    on_dev = [t.to(cuda_device) for t in (q, k, v, mask, bias)]
+    out = out.to(cuda_device)
+    for _ in range(50):
+        assert torch.equal(dot_product_attention(*on_dev, max_ctas=max_ctas, check_status=True), out)
