@@ -172,8 +172,8 @@ struct BarIdx {
 constexpr uint32_t kWaitBlockOff = kBarrierBlockBytes - 32;
 static_assert(BarIdx::count * 8 <= (int)kWaitBlockOff, "barrier block too small");
 
-// Diagnostic dump: four [128][128] float sections, row = query row of block 0's first tile:
-// raw logits, packed P words (64 used), un-normalised O (nv used), {unused, running sum}.
+// Diagnostic dump: four [128][128] float sections, row = query row of block 0's first stream: raw logits and packed P words (64
+// used) of its first key tile, un-normalised O (nv used) and {unused, sum} behind its last.
 constexpr int kDbgTimelineTiles = 256;   // per warpgroup; 8 clock values each, after kDbgFloats floats
 constexpr int kDbgS = 0, kDbgP = kTile * kTile, kDbgO = 2 * kTile * kTile, kDbgML = 3 * kTile * kTile,
               kDbgFloats = 4 * kTile * kTile;
@@ -735,6 +735,7 @@ struct SoftmaxState {
   float done_l;
   __nv_bfloat16* done_row;   // where this thread's row goes (null: beyond the matrix)
   const __nv_bfloat16* done_gate;
+  float* done_dbg;           // (debug build) its row of the dump: block 0's first stream only
 };
 
 // The last tile's weights enter its stream's sum and the turn passes to the other stream.
@@ -753,7 +754,7 @@ __device__ __forceinline__ void close_tile(SoftmaxState& st) {
 
 // O / l -> bf16 -> global for the stream that is done.
 template <bool kDebug, bool kGate>
-__device__ __forceinline__ void store_result(const Ctx& c, const SoftmaxState& st, float* dbg) {
+__device__ __forceinline__ void store_result(const Ctx& c, const SoftmaxState& st) {
   const AttnParams& p = *c.p;
   const float inv = __frcp_rn(st.done_l);
 #pragma unroll 1
@@ -761,10 +762,10 @@ __device__ __forceinline__ void store_result(const Ctx& c, const SoftmaxState& s
     uint32_t o[16];
     tmem_ld_x16(st.done_o + c0, o);
     tc_wait_ld();
-    if (kDebug && dbg != nullptr) {
+    if (kDebug && st.done_dbg != nullptr) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) dbg[kDbgO + c0 + i] = __uint_as_float(o[i]);
-      dbg[kDbgML + 1] = st.done_l;
+      for (int i = 0; i < 16; ++i) st.done_dbg[kDbgO + c0 + i] = __uint_as_float(o[i]);
+      st.done_dbg[kDbgML + 1] = st.done_l;
     }
     if (st.done_row != nullptr) {
 #pragma unroll
@@ -795,7 +796,7 @@ __device__ __forceinline__ void store_result(const Ctx& c, const SoftmaxState& s
 // st.m[0] is the reference maximum the running sums are scaled by (it may lag the true maximum by
 // up to kLazyRescaleLog2 bits), st.l[0] the running sum of the fp32 weights.
 template <bool kDebug, bool kTcBias, bool kGate>
-__device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, float* dbg, float* dbg_o, int wg, int lane,
+__device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, float* dbg, int wg, int lane,
                                              uint32_t s_taddr, uint32_t p_taddr, uint32_t o_taddr,
                                              uint32_t bias_row, uint32_t row7, float scale, bool first_kt, long long* ts) {
   if (kDebug && ts != nullptr) ts[0] = clock64();
@@ -906,7 +907,7 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, flo
     rescale_output(o_taddr, c.p->nv, alpha);
   }
   if (st.done_o != 0) {
-    store_result<kDebug, kGate>(c, st, dbg_o);
+    store_result<kDebug, kGate>(c, st);
     st.done_o = 0;
   }
   st.m[0] = m_use;
@@ -957,6 +958,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
   st.s_ready = st.started = st.swap = false;
   st.done_o = 0;
   st.done_gate = nullptr;
+  st.done_dbg = nullptr;
   uint32_t bst = 0, b_par = 0;                       // (fp8 without tensor-core bias) bias ring
   uint32_t n_tiles = 0;                              // (debug build)
   // The next item's Q tiles are scaled behind the last key tile but one (with a single Q buffer they come later), the first item's here.
@@ -985,16 +987,15 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
         // diagnostic timeline (debug build only): SM clock at the phase boundaries of every tile
         // this warp processes, 8 slots per tile, behind the tile dump
         long long* ts = nullptr;
-        float *dbg = nullptr, *dbg_o = nullptr;
+        float* dbg = nullptr;
         if (kDebug && p.debug != nullptr && blockIdx.x == 0) {
           if (wq == 0 && lane == 0 && n_tiles < kDbgTimelineTiles)
             ts = reinterpret_cast<long long*>(p.debug + kDbgFloats) + ((size_t)wg * kDbgTimelineTiles + n_tiles) * 8;
           if (item == 0 && s == 0 && kt == 0) dbg = p.debug + (size_t)row * kTile;
-          if (item == 0 && s == 2 && kt == p.n_kt - 1) dbg_o = p.debug + (size_t)row * kTile;
           ++n_tiles;
         }
-        if (!softmax_tile<kDebug, kTcBias, kGate>(c, st, dbg, dbg_o, wg, lane, s_taddr, p_taddr, c.tmem + lane_sel + kOCol + s * p.nv, bias_row,
-                                                  row & 7, scale, kt == 0, ts))
+        if (!softmax_tile<kDebug, kTcBias, kGate>(c, st, dbg, wg, lane, s_taddr, p_taddr, c.tmem + lane_sel + kOCol + s * p.nv, bias_row, row & 7, scale,
+                                                  kt == 0, ts))
           return;
         st.swap = it.gv > wg + 2;
         if (kt == p.n_kt - 1) {
@@ -1003,6 +1004,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
           st.done_row = qrow < p.Sq ? p.out + (long long)stream_row(p, it, s) * p.out_stride_b1 + (long long)it.h * p.out_stride_b2 +
                                           (long long)qrow * p.out_stride_s
                                     : nullptr;
+          if (kDebug) st.done_dbg = p.debug != nullptr && item == 0 && s == 0 ? p.debug + (size_t)row * kTile : nullptr;
           if constexpr (kGate)
             st.done_gate = p.gate + (long long)stream_row(p, it, s) * p.gate_stride_b1 + (long long)it.h * p.gate_stride_b2 +
                            (long long)qrow * p.gate_stride_s;
@@ -1023,8 +1025,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
     close_tile(st);
     AF3K_WAIT_WARP(c, BarIdx::pv_done + wg, st.pv_par);
     tc_fence_after();
-    float* dbg_o = kDebug && p.debug != nullptr && blockIdx.x == 0 && wg == 0 && p.n_items == 1 && p.n_streams == 1 ? p.debug + (size_t)row * kTile : nullptr;
-    store_result<kDebug, kGate>(c, st, dbg_o);
+    store_result<kDebug, kGate>(c, st);
   }
 }
 

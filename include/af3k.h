@@ -186,7 +186,7 @@ int af3k_describe_plan_streams(const af3k_attention_desc* desc, int32_t* out4);
 /* Diagnostic: when dump_dev is non-NULL, later attention calls run a debug build of the kernel
  * that writes block 0's first logits tile to dump_dev (4 * 128 * 128 floats: logits as the
  * tensor core delivers them - with bf16 q/k that is scale * q k^T + bias + mask value -, packed
- * P words, un-normalised O, {unused, sum}), followed by 2 * (2 * 256 * 8 + 4 * 256) floats of
+ * P words, then that stream's un-normalised O and {unused, sum} behind its last key tile), followed by 2 * (2 * 256 * 8 + 4 * 256) floats of
  * SM-clock stamps.  Pass NULL to switch it off.  No counterpart in the reference. */
 void af3k_debug_set_dump(float* dump_dev);
 

@@ -221,13 +221,13 @@ def _quantised(q, k):
     return q, k, {"q_scale": qs, "k_scale": ks}
 
 
-def _plan(B1, B2, S, D, fp8=False, Sk=None, max_ctas=0):
+def _plan(B1, B2, S, D, fp8=False, Sk=None, max_ctas=0, rows_per_item=0):
     Sk = Sk or S
     d = _capi.AttentionDesc()
     d.B1, d.B2, d.Sq, d.Sk, d.D = B1, B2, S, Sk, D
     for n, keys in (("q_stride", S), ("k_stride", Sk), ("v_stride", Sk), ("out_stride", S)):
         getattr(d, n)[:] = [B2 * keys * D, keys * D, D]
-    d.bias_stride[:], d.mask_row_stride, d.softmax_scale, d.max_ctas = [S * Sk, Sk], Sk, D ** -0.5, max_ctas
+    d.bias_stride[:], d.mask_row_stride, d.softmax_scale, d.max_ctas, d.rows_per_item = [S * Sk, Sk], Sk, D ** -0.5, max_ctas, rows_per_item
     d.qk_dtype, d.bias_dtype = _capi.AF3K_FP8_E4M3 if fp8 else _capi.AF3K_BF16, _capi.AF3K_BF16
     return _capi.describe_plan(d)
 
@@ -347,3 +347,27 @@ def test_pair_of_query_tiles_behind_a_lone_one(cuda_device, B1, B2, S, Sk, D, ma
     out = out.to(cuda_device)
     for _ in range(50):
         assert torch.equal(dot_product_attention(*on_dev, max_ctas=max_ctas, check_status=True), out)
+
+
+@pytest.mark.parametrize("B1,B2,S,rows_per_item,max_ctas,streams", [(1, 3, 128, 0, 1, 1), (3, 2, 200, 2, 0, 2), (2, 1, 300, 2, 1, 2), (1, 1, 256, 0, 1, 2), (1, 2, 300, 0, 1, 2),
+                                                                    (4, 1, 130, 3, 1, 3), (8, 1, 100, 4, 1, 4)])
+def test_debug_dump_has_the_first_result(cuda_device, B1, B2, S, rows_per_item, max_ctas, streams):
+    """Pair rows or query tiles, one item on a CTA and several: accumulator and sum of block 0's first stream are in the dump, and their
+    quotient is the result but for its rounding to bf16."""
+    D = 32
+    other = {"rows_per_item": rows_per_item, "max_ctas": max_ctas}
+    plan = _plan(B1, B2, S, D, **other)
+    assert plan["streams"] == streams, plan
+    lib = _capi.load()
+    q, k, v, mask, bias = _inputs(B1, B2, S, D, S)
+    dump = torch.full((4 * 128 * 128 + 2 * (2 * 256 * 8 + 4 * 256),), float("nan"), device=cuda_device)
+    lib.af3k_debug_set_dump(dump.data_ptr())
+    try:
+        out = _call(cuda_device, q, k, v, mask, bias, **other)
+    finally:
+        lib.af3k_debug_set_dump(None)
+    _check(out, O.oracle_fp32(q, k, v, mask, bias), plan)
+    n = min(S, 128)
+    _, _, acc, sums = dump[:4 * 128 * 128].view(4, 128, 128)[:, :n].cpu()
+    want = acc[:, :D] / sums[:, 1:2]
+    assert ((out[0, 0, :n].float() - want).abs() <= 2 ** -8 * want.abs()).all()
