@@ -324,8 +324,12 @@ def test_bias_stages_of_query_tile_streams(cuda_device, S, D):
     q, k, v, mask, bias = _inputs(1, 2, S, D, S + D)
     out = _call(cuda_device, q, k, v, mask, bias)
     _check(out, O.oracle_fp32(q, k, v, mask, bias), (S, D))
+    assert _plan(1, 2, S, D)["streams"] == 1
     tiles = (S + 127) // 128
     for ctas in (1, 3, tiles + tiles % 2):
+        plan = _plan(1, 2, S, D, max_ctas=ctas)
+        pairs = ctas != 3 or tiles > 3
+        assert plan["query_tile_streams"] == pairs and plan["bias_stages"] == (3 if pairs and D <= 32 else 2), plan
         assert torch.equal(_call(cuda_device, q, k, v, mask, bias, max_ctas=ctas), out), ctas
 
 
