@@ -279,7 +279,8 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   // An item's time, in logits-tile times of one warpgroup: streams alternate between the two softmax warpgroups (an odd
   // count leaves one idle slot), n_kt tiles for each of a warpgroup's slots, plus about 0.8 for the epilogue and the
   // hand-over to the next item; with a single Q buffer the next item's Q tiles are loaded and scaled at the hand-over
-  // (about 0.5: each stream's tile is replaced as soon as its last Q K^T has finished).
+  // (about 0.5: each stream's tile is replaced as soon as its last Q K^T has finished).  These figures, kLoneTile and kRingPenalty are
+  // from when results were stored at the item's end and the P V issuer scaled Q; they were not measured again since.
   auto item_cost = [&](int g, bool split, int qbuf) {
     const int streams = split ? 2 : g;
     return p.n_kt * ((streams + 1) / 2) * (streams == 1 ? kLoneTile : 1.0) + 0.8 + (qbuf == 1 ? 0.5 : 0.0);
@@ -337,6 +338,7 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   p.div_q = make_divisor((uint32_t)tiles_of(best_split));
   p.div_h = make_divisor((uint32_t)p.B2);
 
+  // (After the choice: the cost model compares such plans with two bias stages and the Q buffers it asked for.)
   // Streams that are query tiles bring a bias tile for each of their logits tiles (32 KB beside 16 KB of K and V), and with
   // two stages a load's latency was the time between two tiles: a third stage where K and V keep one more than that.  (Nothing
   // is gained where a lone query tile uses them, and the warps that convert an fp32 bias get slower: 512 tokens 10.7 -> 12.7 us.)

@@ -721,8 +721,9 @@ __device__ __forceinline__ bool softmax_wait(const Ctx& c, int idx, uint32_t par
 
 // What a softmax thread carries from tile to tile.  A stream's result is stored at the end of its warpgroup's next tile, before
 // that tile's P is handed over (the next P V may write the same accumulator): its last P V has been waited for by then, which a
-// warpgroup that stored it at once spent 700 - 1 400 cycles on, and as much again on the way to its next tile.  With Q scaled by these warps
-// and the other changes of the hand-over, us: 768 rows 635 -> 617, 389 rows 169 -> 157, 1000 fp8 rows 1 389 -> 1 285.
+// warpgroup that stored it at once spent 700 - 1 400 cycles on, and as much again on the way to its next tile.  With Q scaled by these warps, the
+// wider stores of P and the other changes of the hand-over, us a call on changing inputs: 768 rows 649 -> 628, 389 rows (grid module)
+// 248 -> 236, 2048 fp8 rows 10 900 -> 9 845, 5 x 1536 tokens of 48 channels 97.9 -> 93.7.
 struct SoftmaxState {
   float m[2], l[2];          // reference maximum and sum of its streams: [0] the stream whose turn it is, [1] the other one
   uint64_t sum_a, sum_b;     // the last tile's weights, not yet in its stream's sum
@@ -860,7 +861,7 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, flo
   // The pass is one ex2 per logit on the XU (a warp-wide ex2 every 8 cycles per scheduler, shared
   // by the scheduler's two softmax warps) with one packed FMA, one packed add and one bf16 pack per
   // pair of logits around it.  Two warps alone on a scheduler take 2 230 cycles for a tile each, 2 048 of them the XU's; the kernel
-  // takes 2 600 - 2 900, for what a warp runs between two passes: some 110 instructions in one chain, six cycles each.  (Tried
+  // takes 2 590 with fp8 and 2 950 - 2 990 with bf16, for what a warp runs between two passes: some 110 instructions in one chain, six cycles each.  (Tried
   // and slower: the maximum searched along with the pass and the pass repeated where a row has grown, 768 rows 636 -> 690 us, for the
   // logits that stay live; the wait for P and O after one or two column groups, 2048 fp8 rows 10 300 -> 11 700.)
   const uint64_t l2e2 = pack_f32x2(f, f);
@@ -926,7 +927,7 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, flo
 
 // (bf16 q/k) A softmax warp scales its quarter of its warpgroup's Q tiles of the CTA's j-th item.  Eight warps do in 300 cycles
 // what took a single-warp role several thousand, and 12 instructions a tile are little beside the softmax's own 450: 768 rows
-// 617 us, with the P V issuer scaling 616 - 666, with the mask writer 641 - 676, with q scaled by its producer 596.
+// 617 us (kernel alone, as it then was), with the P V issuer scaling 616 - 666, with the mask writer 641 - 676, with q scaled by its producer 596.
 template <bool kMixed>
 __device__ __forceinline__ bool scale_own_q(const Ctx& c, int item, uint32_t j, int wg, int wq, int lane) {
   const AttnParams& p = *c.p;
