@@ -229,8 +229,6 @@ __device__ __forceinline__ uint32_t grid_prologue(const GridParams& p, uint32_t 
     tmem_alloc(smem_u32(const_cast<uint32_t*>(slot)), tmem_cols);
     tmem_relinquish();
   }
-  // No grid_release_next here: the next kernel's blocks come in as this one's end.  Letting them in earlier was slower
-  // (389 rows 255 -> 257 us a module call).
   grid_wait_previous();
   fence_proxy_async_smem();      // whatever the caller stored for the tensor core
   tc_fence_before();
@@ -306,6 +304,10 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
       uint32_t n = 0, buf = 0, lap = 0;
       for (long long tile = first; tile < n_tiles; tile += step, ++n) {
         const uint32_t st = n % Tile::kStages;
+        // The next kernel's blocks may come in from each CTA's last tile on: they set themselves up as SMs become free.  (From the
+        // prologue on they were in the way, 389 rows 255 -> 257 us a module call; as blocks end, 192 rows 48.5 us on the device,
+        // 256 rows of 64 channels 50.9, here 46.5 and 49.9.)
+        if (tile + step >= n_tiles) grid_release_next();
         AF3K_GRID_WAIT(GridBar::x_ready + st, (n / Tile::kStages) & 1);
         for (int c = 0; c < chunks; ++c) {
           // the epilogue warps must have read this accumulator's previous columns
@@ -547,6 +549,7 @@ grid_out_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CU
       uint32_t n = 0;
       for (long long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++n) {
         const uint32_t st = n % Tile::kStages, buf = n & 1;
+        if (tile + gridDim.x >= n_tiles) grid_release_next();
         AF3K_GRID_WAIT(GridBar::x_ready + st, (n / Tile::kStages) & 1);
         if (n >= 2) AF3K_GRID_WAIT(GridBar::acc_empty + buf, ((n >> 1) - 1) & 1);
         tc_fence_after();
