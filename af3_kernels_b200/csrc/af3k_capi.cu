@@ -7,6 +7,7 @@
 #include <cstring>
 #include <mutex>
 #include <utility>
+#include <vector>
 
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -63,6 +64,22 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 constexpr int kStaticSmemReserve = 1024;   // the kernels' few static bytes, padded to the dynamic part's alignment
 
+// Key tiles come in these widths; every width is a kernel of its own, whose softmax warps have that many logits in registers.
+constexpr int kKeyWidths[] = {32, 64, 80, 96, 112, 128};
+
+// f(kernel) for the kernel of key tiles of kw keys.
+template <bool kFp8, bool kGate, bool kMixed, bool kConvert, typename F>
+void with_width(int kw, F&& f) {
+  switch (kw) {
+    case 32: return f(attention_kernel<false, true, kFp8, kGate, kMixed, kConvert, 32>);
+    case 64: return f(attention_kernel<false, true, kFp8, kGate, kMixed, kConvert, 64>);
+    case 80: return f(attention_kernel<false, true, kFp8, kGate, kMixed, kConvert, 80>);
+    case 96: return f(attention_kernel<false, true, kFp8, kGate, kMixed, kConvert, 96>);
+    case 112: return f(attention_kernel<false, true, kFp8, kGate, kMixed, kConvert, 112>);
+    default: return f(attention_kernel<false, true, kFp8, kGate, kMixed, kConvert, 128>);
+  }
+}
+
 struct DeviceInfo {
   int sm_count = 0;
   int cc_major = 0;
@@ -91,17 +108,20 @@ int device_info(DeviceInfo** out) {
     // the opt-in limit covers static + dynamic shared memory; the kernel has a few static bytes
     const int dyn = d.max_smem_optin - kStaticSmemReserve;
     const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    const void* kernels[] = {
-        (const void*)attention_kernel<false, true, false, false, false>, (const void*)attention_kernel<false, true, false, true, false>,
-        (const void*)attention_kernel<false, true, true, false, false>,  (const void*)attention_kernel<false, true, true, true, false>,
+    std::vector<const void*> kernels = {
+        (const void*)attention_kernel<false, true, true, true, false>,   (const void*)attention_kernel<false, true, true, true, true>,
         (const void*)attention_kernel<false, false, true, false, false>, (const void*)attention_kernel<false, false, true, true, false>,
-        (const void*)attention_kernel<false, true, false, false, true>,  (const void*)attention_kernel<false, true, false, true, true>,
-        (const void*)attention_kernel<false, true, true, false, true>,   (const void*)attention_kernel<false, true, true, true, true>,
         (const void*)attention_kernel<false, false, true, false, true>,  (const void*)attention_kernel<false, false, true, true, true>,
         (const void*)attention_kernel<true, true, false, false, true>,   (const void*)attention_kernel<true, true, true, false, true>,
         (const void*)attention_kernel<true, false, true, false, true>,
-        (const void*)attention_kernel<false, true, false, false, false, true>, (const void*)attention_kernel<false, true, false, true, false, true>,
     };
+    const auto add = [&](auto kernel) { kernels.push_back((const void*)kernel); };
+    for (int kw : kKeyWidths) {
+      with_width<false, false, false, false>(kw, add); with_width<false, false, true, false>(kw, add);
+      with_width<false, true, false, false>(kw, add);  with_width<false, true, true, false>(kw, add);
+      with_width<false, false, false, true>(kw, add);  with_width<false, true, false, true>(kw, add);
+      with_width<true, false, false, false>(kw, add);  with_width<true, false, true, false>(kw, add);
+    }
     e = cudaSuccess;
     for (const void* kfn : kernels)
       if (e == cudaSuccess) e = cudaFuncSetAttribute(kfn, attr, dyn);
@@ -233,6 +253,21 @@ constexpr double kLoneTile = 0.75;
 // Smaller items behind the last full round have to promise this much: the model is no better than that.
 constexpr double kTailGain = 0.98;
 
+// Keys per key tile: as many tiles as 128 keys each make, and of those the narrowest that hold the call's keys, because a
+// tile's loads from TMEM, maximum, exponentials, stores and MMAs go with its width while its waits and hand-overs do not.
+// (Depends on nothing but the keys and the kind of kernel, so that all plans of a call add up the same tiles.)  Attention kernel in
+// the grid module, us, tiles of 128 -> as wide as needed: 192 rows (96) 27.1 -> 24.3, 389 rows (112) 151 -> 139, 30 rows (32)
+// 6.3 -> 4.8; the operator on 77 keys (80) 5.6 -> 5.3.  With the width as a run-time value in the issuers' loops 1536 tokens took
+// 25.2 instead of 24.5, so it is a template argument of every role.
+int key_width(const af3k_attention_desc& d, bool tc_bias, bool debug) {
+  const bool fp8 = d.qk_dtype == AF3K_FP8_E4M3;
+  if (!tc_bias || (fp8 && d.gate != nullptr) || debug) return kTile;   // kernels of one width
+  const int64_t tiles = (d.Sk + kTile - 1) / kTile, need = (d.Sk + tiles - 1) / tiles;
+  for (int kw : kKeyWidths)
+    if (kw >= need) return kw;
+  return kTile;
+}
+
 // Picks rows-per-item G and the K/V ring depth from a cost model of one CTA's time (below).
 // allow_q_split: the kernel variant that will run supports query-tile streams (every variant in
 // which the tensor core adds the bias).
@@ -242,7 +277,9 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   const int es = d.qk_dtype == AF3K_FP8_E4M3 ? 1 : 2;
   p.B1 = (int)d.B1; p.B2 = (int)d.B2; p.Sq = (int)d.Sq; p.Sk = (int)d.Sk; p.D = (int)d.D;
   p.n_qt = (p.Sq + kTile - 1) / kTile;
-  p.n_kt = (p.Sk + kTile - 1) / kTile;
+  p.debug = g_debug_dump.load();
+  p.kw = key_width(d, allow_q_split, p.debug != nullptr);
+  p.n_kt = (p.Sk + p.kw - 1) / p.kw;
   p.qk_row_bytes = row_bytes_for(d.D * es);
   p.v_row_bytes = row_bytes_for(d.D * 2);
   p.qk_ksteps = (int)((d.D * es + 31) / 32);
@@ -255,6 +292,7 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   }
   p.k_tile_bytes = p.q_tile_bytes;
   p.v_tile_bytes = kTile * p.v_row_bytes;
+  p.kv_load_bytes = p.kw * (p.k_tile_bytes / kTile + p.v_row_bytes);
   p.scale = d.softmax_scale;
 
   const int budget = dev.max_smem_optin - kStaticSmemReserve;
@@ -376,7 +414,7 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
 }
 
 int encode_qkv_map(CUtensorMap* tm, const void* base, bool fp8, int64_t D, int64_t S, int64_t B2,
-                   int64_t B1, const int64_t* stride, int row_bytes) {   // row_bytes: of the box
+                   int64_t B1, const int64_t* stride, int row_bytes, int rows) {   // row_bytes, rows: of the box
   auto enc = tensor_map_encoder();
   if (!enc) return driver_fail("cuTensorMapEncodeTiled entry point", -1);
   const uint64_t es = fp8 ? 1 : 2;
@@ -386,7 +424,7 @@ int encode_qkv_map(CUtensorMap* tm, const void* base, bool fp8, int64_t D, int64
   // a dimension of extent 1 may carry any stride; TMA still wants it non-zero and 16-aligned
   for (int i = 0; i < 3; ++i)
     if (strides[i] == 0) strides[i] = 16;
-  cuuint32_t box[4] = {(cuuint32_t)(row_bytes / es), (cuuint32_t)kTile, 1, 1};
+  cuuint32_t box[4] = {(cuuint32_t)(row_bytes / es), (cuuint32_t)rows, 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = enc(tm, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4,
                    const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -575,7 +613,6 @@ int attention_call(const af3k_attention_desc* desc, const void* q, const void* k
   const bool stage_fp8 = fp8 && !d.bias_prescaled && workspace != nullptr && workspace_bytes >= stage_bytes &&
                          aligned16(workspace);
   const bool fp8_tc = fp8 && (d.bias_prescaled || stage_fp8);
-  p.debug = g_debug_dump.load();
   // the kernel converts the bias itself: items of one query tile, rows that start on vectors or a single key tile
   const uintptr_t bias_es = d.bias_dtype == AF3K_F32 ? 4 : 2;
   p.bias_wide = d.Sk % 4 == 0 && (reinterpret_cast<uintptr_t>(bias) | (uintptr_t)bias_sh * bias_es | (uintptr_t)bias_sr * bias_es) % (4 * bias_es) == 0 ? 1 : 0;
@@ -594,12 +631,12 @@ int attention_call(const af3k_attention_desc* desc, const void* q, const void* k
   }
 
   CUtensorMap tm_q, tm_k, tm_v, tm_b{};
-  if ((rc = encode_qkv_map(&tm_q, q, fp8, d.D, d.Sq, d.B2, d.B1, d.q_stride, p.qk_row_bytes))) return rc;
-  if ((rc = encode_qkv_map(&tm_k, k, fp8, d.D, d.Sk, d.B2, d.B1, d.k_stride, p.qk_row_bytes))) return rc;
-  if ((rc = encode_qkv_map(&tm_v, v, false, d.D, d.Sk, d.B2, d.B1, d.v_stride, p.v_row_bytes))) return rc;
+  if ((rc = encode_qkv_map(&tm_q, q, fp8, d.D, d.Sq, d.B2, d.B1, d.q_stride, p.qk_row_bytes, kTile))) return rc;
+  if ((rc = encode_qkv_map(&tm_k, k, fp8, d.D, d.Sk, d.B2, d.B1, d.k_stride, p.qk_row_bytes, p.kw))) return rc;
+  if ((rc = encode_qkv_map(&tm_v, v, false, d.D, d.Sk, d.B2, d.B1, d.v_stride, p.v_row_bytes, p.kw))) return rc;
   CUtensorMap tm_q2{}, tm_k2{};
-  if (p.qk_narrow && ((rc = encode_qkv_map(&tm_q2, q, fp8, d.D, d.Sq, d.B2, d.B1, d.q_stride, 32)) ||
-                      (rc = encode_qkv_map(&tm_k2, k, fp8, d.D, d.Sk, d.B2, d.B1, d.k_stride, 32))))
+  if (p.qk_narrow && ((rc = encode_qkv_map(&tm_q2, q, fp8, d.D, d.Sq, d.B2, d.B1, d.q_stride, 32, kTile)) ||
+                      (rc = encode_qkv_map(&tm_k2, k, fp8, d.D, d.Sk, d.B2, d.B1, d.k_stride, 32, p.kw))))
     return rc;
   if (in_kernel) {
     p.bias_src = bias;
@@ -612,7 +649,7 @@ int attention_call(const af3k_attention_desc* desc, const void* q, const void* k
   p.k_scale = k_scale;
   p.mask = mask;
   p.mask_row_stride = d.mask_row_stride;
-  p.mask_col = (mask != nullptr || d.Sk % kTile != 0) ? 1 : 0;
+  p.mask_col = (mask != nullptr || d.Sk % p.kw != 0) ? 1 : 0;
   p.out = static_cast<__nv_bfloat16*>(out);
   p.out_stride_b1 = d.out_stride[0];
   p.out_stride_b2 = d.out_stride[1];
@@ -629,26 +666,27 @@ int attention_call(const af3k_attention_desc* desc, const void* q, const void* k
   const bool tc_bias = !fp8 || fp8_tc;
   p.scale_q = (fp8 || d.softmax_scale == 1.0f) ? 0 : 1;   // a scale of exactly 1 (q already scaled by its producer) needs no pass over Q
   const bool dbg = p.debug != nullptr;
-#define AF3K_LAUNCH_AS(...) launch_overlapped(attention_kernel<__VA_ARGS__>, dim3(plan.grid), kThreads, plan.smem_bytes, stream, d.max_ctas <= 0, p, tm_q, tm_k, tm_v, tm_b, tm_q2, tm_k2)
-#define AF3K_LAUNCH(...) (p.mixed ? AF3K_LAUNCH_AS(__VA_ARGS__, true) : AF3K_LAUNCH_AS(__VA_ARGS__, false))
+  const auto launch = [&](auto kernel) {
+    launch_overlapped(kernel, dim3(plan.grid), kThreads, plan.smem_bytes, stream, d.max_ctas <= 0, p, tm_q, tm_k, tm_v, tm_b, tm_q2, tm_k2);
+  };
   if (in_kernel) {
-    if (p.gate != nullptr) AF3K_LAUNCH_AS(false, true, false, true, false, true);
-    else                   AF3K_LAUNCH_AS(false, true, false, false, false, true);
+    if (p.gate != nullptr) with_width<false, true, false, true>(p.kw, launch);
+    else                   with_width<false, false, false, true>(p.kw, launch);
+  } else if (dbg && p.gate == nullptr) {
+    if (!fp8)         launch(attention_kernel<true, true, false, false, true>);
+    else if (tc_bias) launch(attention_kernel<true, true, true, false, true>);
+    else              launch(attention_kernel<true, false, true, false, true>);
+  } else if (!fp8) {
+    if (p.gate != nullptr) { if (p.mixed) with_width<false, true, true, false>(p.kw, launch);  else with_width<false, true, false, false>(p.kw, launch); }
+    else                   { if (p.mixed) with_width<false, false, true, false>(p.kw, launch); else with_width<false, false, false, false>(p.kw, launch); }
   } else if (p.gate != nullptr) {
-    if (!fp8)         AF3K_LAUNCH(false, true, false, true);
-    else if (tc_bias) AF3K_LAUNCH(false, true, true, true);
-    else              AF3K_LAUNCH(false, false, true, true);
-  } else if (dbg) {
-    if (!fp8)         AF3K_LAUNCH_AS(true, true, false, false, true);
-    else if (tc_bias) AF3K_LAUNCH_AS(true, true, true, false, true);
-    else              AF3K_LAUNCH_AS(true, false, true, false, true);
+    if (tc_bias) { if (p.mixed) launch(attention_kernel<false, true, true, true, true>);  else launch(attention_kernel<false, true, true, true, false>); }
+    else         { if (p.mixed) launch(attention_kernel<false, false, true, true, true>); else launch(attention_kernel<false, false, true, true, false>); }
+  } else if (tc_bias) {
+    if (p.mixed) with_width<true, false, true, false>(p.kw, launch); else with_width<true, false, false, false>(p.kw, launch);
   } else {
-    if (!fp8)         AF3K_LAUNCH(false, true, false, false);
-    else if (tc_bias) AF3K_LAUNCH(false, true, true, false);
-    else              AF3K_LAUNCH(false, false, true, false);
+    if (p.mixed) launch(attention_kernel<false, false, true, false, true>); else launch(attention_kernel<false, false, true, false, false>);
   }
-#undef AF3K_LAUNCH
-#undef AF3K_LAUNCH_AS
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail("launch attention_kernel", e);
   ++launches;

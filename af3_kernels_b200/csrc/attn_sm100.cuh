@@ -54,7 +54,7 @@
 
 namespace af3k {
 
-constexpr int kTile = 128;         // query rows per tile == keys per tile
+constexpr int kTile = 128;         // query rows per tile, and the most keys
 constexpr int kThreads = 384;      // 12 warps
 // 65536 registers per SM: launched at 168 per thread, then 128 x 72 + 256 x 216 = 64512
 constexpr int kRegsMisc = 72, kRegsSoftmax = 216;
@@ -107,6 +107,7 @@ __device__ __forceinline__ uint32_t divide(uint32_t x, const Divisor& v) { retur
 struct AttnParams {
   int B1, B2, Sq, Sk, D;
   int n_qt, n_kt;
+  int kw;                // keys per key tile (the kernel's kW)
   int G;                 // pair rows per work item
   int q_split;           // 1: the streams of an item are two neighbouring query tiles of ONE pair row (G == 1)
   int n_streams;         // streams per work item: G, or 2 with q_split
@@ -139,7 +140,8 @@ struct AttnParams {
   int* status;           // int[4]: {status bits, 1 + first barrier slot that timed out, block, warp}
   long long wait_limit;  // SM clocks a single wait may take before the kernel gives up
   float* debug;          // diagnostic dump of block 0's first logits tile (debug build of the kernel)
-  uint32_t q_tile_bytes, k_tile_bytes, v_tile_bytes;
+  uint32_t q_tile_bytes, k_tile_bytes, v_tile_bytes;   // in shared memory: 128 rows each
+  uint32_t kv_load_bytes;                              // what a K and V tile's loads bring
   uint32_t off_q, off_kv, off_bias, off_bar;   // from the 1024-aligned smem base
   // mask-column operands of the extra K step (all no-swizzle, K-major, 16-byte rows):
   //   off_ones: A operand, element (row, 0) = 1;  off_mcol: ring of per-tile B operands, element
@@ -292,7 +294,7 @@ __device__ __forceinline__ uint32_t q_buf(const AttnParams& p, uint32_t j) { ret
 __device__ __forceinline__ uint32_t q_use(const AttnParams& p, uint32_t j) { return p.q_buffers == 2 ? (j >> 1) : j; }
 
 // ------------------------------------------------------------------ producer (one thread)
-template <bool kMixed, bool kConvert>
+template <bool kMixed, bool kConvert, int kW>
 __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUtensorMap* tm_k,
                               const CUtensorMap* tm_v, const CUtensorMap* tm_bias, const CUtensorMap* tm_q2, const CUtensorMap* tm_k2) {
   const AttnParams& p = *c.p;
@@ -339,18 +341,18 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
           if (blap != 0) AF3K_WAIT(c, BarIdx::bias_empty + bst, (blap - 1) & 1);
           const uint32_t bfull = bar_addr(c, BarIdx::bias_full + bst);
           const uint32_t bdst = c.smem + p.off_bias + bst * kBiasTileBytes;
-          mbar_arrive_expect_tx(bfull, kBiasTileBytes);
-          tma_load_3d(bdst, tm_bias, bfull, kt * kTile, stream_qt(p, it, s) * kTile, it.h);
-          tma_load_3d(bdst + kBiasTileBytes / 2, tm_bias, bfull, kt * kTile + 64, stream_qt(p, it, s) * kTile, it.h);
+          mbar_arrive_expect_tx(bfull, kW > 64 ? kBiasTileBytes : kBiasTileBytes / 2);
+          tma_load_3d(bdst, tm_bias, bfull, kt * kW, stream_qt(p, it, s) * kTile, it.h);
+          if (kW > 64) tma_load_3d(bdst + kBiasTileBytes / 2, tm_bias, bfull, kt * kW + 64, stream_qt(p, it, s) * kTile, it.h);
           if (++bst == n_bias) { bst = 0; ++blap; }
         }
         if (lap != 0) AF3K_WAIT(c, BarIdx::kv_empty + st, (lap - 1) & 1);
         const uint32_t full = bar_addr(c, BarIdx::kv_full + st);
         const uint32_t kdst = c.smem + p.off_kv + st * (p.k_tile_bytes + p.v_tile_bytes);
-        mbar_arrive_expect_tx(full, p.k_tile_bytes + p.v_tile_bytes);
-        tma_load_4d(kdst, tm_k, full, 0, kt * kTile, it.h, stream_row(p, it, s));
-        if (p.qk_narrow) tma_load_4d(kdst + kNarrowOff, tm_k2, full, 32, kt * kTile, it.h, stream_row(p, it, s));
-        tma_load_4d(kdst + p.k_tile_bytes, tm_v, full, 0, kt * kTile, it.h, stream_row(p, it, s));
+        mbar_arrive_expect_tx(full, p.kv_load_bytes);
+        tma_load_4d(kdst, tm_k, full, 0, kt * kW, it.h, stream_row(p, it, s));
+        if (p.qk_narrow) tma_load_4d(kdst + kNarrowOff, tm_k2, full, 32, kt * kW, it.h, stream_row(p, it, s));
+        tma_load_4d(kdst + p.k_tile_bytes, tm_v, full, 0, kt * kW, it.h, stream_row(p, it, s));
         if (++st == nkv) { st = 0; ++lap; }
       }
     }
@@ -385,13 +387,14 @@ __device__ __noinline__ void scale_q(uint32_t addr, uint32_t bytes, float scale,
   if (lane == 0) mbar_arrive(bar);
 }
 
-// The 128 mask-column values (bf16) of one logits tile, four per lane.
+// The mask-column values (bf16) of one logits tile, four per lane (those behind its last key are not read).
+template <int kW>
 __device__ __forceinline__ void mask_values(const AttnParams& p, const Item& it, int kt, int s, int lane,
                                             uint16_t masked, uint16_t (&val)[4]) {
   const uint8_t* mrow = p.mask != nullptr ? p.mask + (long long)stream_row(p, it, s) * p.mask_row_stride : nullptr;
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
-    const int key = kt * kTile + 32 * g + lane;
+    const int key = kt * kW + 32 * g + lane;
     val[g] = key >= p.Sk ? kMaskColAbsent : ((mrow == nullptr || mrow[key] != 0) ? kMaskColKeep : masked);
   }
 }
@@ -408,11 +411,11 @@ __device__ __forceinline__ uint16_t masked_value_bits(const AttnParams& p, int h
 }
 
 // Key-mask writer (one warp).  For every logits tile, in the producer's order: write the tile's
-// 128 mask values into its slot of the mask-column ring.  The slot is the B operand of the extra
+// mask values into its slot of the mask-column ring.  The slot is the B operand of the extra
 // K step; only element 0 of each key's 16-byte row changes, the rest stays zero.  Arrives on the
 // tile's kv_full barrier (which then counts two arrivals: this one and the producer's).  The mask
 // bytes of a tile are requested one tile ahead, so their latency is not on the path.
-template <bool kMixed>
+template <bool kMixed, int kW>
 __device__ void mask_writer_role(const Ctx& c, int lane) {
   const AttnParams& p = *c.p;
   const WaitBlock* wait_block = wait_block_of(c.bars);
@@ -430,7 +433,7 @@ __device__ void mask_writer_role(const Ctx& c, int lane) {
     for (int i = -1; i < tiles; ++i) {
       const uint16_t cur[4] = {val[0], val[1], val[2], val[3]};
       if (i + 1 < tiles) {
-        mask_values(p, it, nkt, ns, lane, masked, val);
+        mask_values<kW>(p, it, nkt, ns, lane, masked, val);
         if (++ns == it.gv) { ns = 0; ++nkt; }
       }
       if (i >= 0) {
@@ -461,7 +464,7 @@ __device__ void mask_writer_role(const Ctx& c, int lane) {
 // Logits of every tile, in order: Q K^T, then the mask column, then (bf16 q/k) the bias slices.
 // (The MMA loops are real loops and the fp8 / bf16 choice is a template argument: the warp pays an
 // instruction-cache miss for most lines of this loop on every pass, so the loop is kept small.)
-template <bool kDebug, bool kTcBias, bool kFp8, bool kMixed>
+template <bool kDebug, bool kTcBias, bool kFp8, bool kMixed, int kW>
 __device__ void qk_issuer_role(const Ctx& c) {
   const AttnParams& p = *c.p;
   const WaitBlock* wait_block = wait_block_of(c.bars);
@@ -469,7 +472,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
   const uint32_t nkv = p.kv_stages;
   const uint32_t qk_layout = swizzle_layout_code(p.qk_row_bytes);
   constexpr bool fp8 = kFp8;
-  const uint32_t idesc_qk = make_idesc(fp8 ? 0u : 1u, fp8 ? 0u : 1u, 0u, 0u, kTile);
+  const uint32_t idesc_qk = make_idesc(fp8 ? 0u : 1u, fp8 ? 0u : 1u, 0u, 0u, kW);
   const uint32_t kv_stage_bytes = p.k_tile_bytes + p.v_tile_bytes;
   // descriptor words for tile 0 / stage 0; later tiles only move the start-address field
   const uint64_t qd0 = make_smem_desc(c.smem + p.off_q, 16, 8 * p.qk_row_bytes, qk_layout);
@@ -486,7 +489,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
   const uint64_t md0 = make_smem_desc(c.smem + p.off_mcol, p.off_zero - p.off_mcol, 128, 0);
   const uint32_t od_lo = (uint32_t)od0, od_hi = (uint32_t)(od0 >> 32);
   const uint32_t md_lo = (uint32_t)md0, md_hi = (uint32_t)(md0 >> 32);
-  const uint32_t idesc_mask = make_idesc(1u, 1u, 0u, 0u, kTile);
+  const uint32_t idesc_mask = make_idesc(1u, 1u, 0u, 0u, kW);
   const bool mask_col = p.mask_col != 0;
   // bias slices: A = 16 keys of the staged bias tile (K-major, 128-byte swizzled rows, two boxes
   // of 64 keys), B = the 16 x 16 identity (K-major, no swizzle: 8-key halves 256 bytes apart,
@@ -555,7 +558,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
             mma_ss_f16(s_tmem, od_lo, od_hi, md_lo + slot16 - (slot16 << 16), md_hi, idesc_mask, 1u);
           if (kTcBias) {
 #pragma unroll 1
-            for (int k = 0; k < kTile / 16; ++k)   // keys 16k .. 16k + 15: box k / 4, 32 bytes per step
+            for (int k = 0; k < kW / 16; ++k)   // keys 16k .. 16k + 15: box k / 4, 32 bytes per step
               mma_ss_f16(s_tmem + 16 * k, bias_lo + (k >> 2) * (kBiasTileBytes >> 5) + 2 * (k & 3), bd_hi,
                          id_lo, id_hi, idesc_bias, 1u);
           }
@@ -588,7 +591,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
 }
 
 // O += P V for every tile, in order.
-template <bool kDebug, bool kMixed>
+template <bool kDebug, bool kMixed, int kW>
 __device__ void pv_issuer_role(const Ctx& c) {
   const AttnParams& p = *c.p;
   const WaitBlock* wait_block = wait_block_of(c.bars);
@@ -628,7 +631,7 @@ __device__ void pv_issuer_role(const Ctx& c) {
           const long long t0 = kDebug && tl != nullptr ? clock64() : 0;
           mma_ts_f16(o_tmem, p_tmem, b_lo, vd_hi, idesc_pv, kt > 0 ? 1u : 0u);
 #pragma unroll 1
-          for (int k = 1; k < kTile / 16; ++k)   // 16 keys per step: 8 TMEM columns of P
+          for (int k = 1; k < kW / 16; ++k)   // 16 keys per step: 8 TMEM columns of P
             mma_ts_f16(o_tmem, p_tmem + k * 8, b_lo + k * v_kstep, vd_hi, idesc_pv, 1u);
           tc_commit(bar_addr(c, BarIdx::pv_done + b));
           tc_commit(bar_addr(c, BarIdx::kv_empty + st));
@@ -678,8 +681,8 @@ __device__ __forceinline__ void logits_half(uint32_t (&xr)[kTile], uint32_t bias
 }
 
 // Row maximum over finished logits (bf16 q/k: the tensor core has already applied scale, bias and mask).
-template <int kCol0, int kCol1>
-__device__ __forceinline__ void row_max(const uint32_t (&xr)[kTile], float& mxa, float& mxb) {
+template <int kCol0, int kCol1, int kW>
+__device__ __forceinline__ void row_max(const uint32_t (&xr)[kW], float& mxa, float& mxb) {
 #pragma unroll
   for (int i = kCol0; i < kCol1; i += 4) {
     mxa = max3(mxa, __uint_as_float(xr[i]), __uint_as_float(xr[i + 1]));
@@ -793,10 +796,10 @@ __device__ __forceinline__ void store_result(const Ctx& c, const SoftmaxState& s
   }
 }
 
-// One 128 x 128 logits tile of one stream; the thread owns row `row` (TMEM lane).
+// One logits tile of 128 rows and kW keys of one stream; the thread owns row `row` (TMEM lane).
 // st.m[0] is the reference maximum the running sums are scaled by (it may lag the true maximum by
 // up to kLazyRescaleLog2 bits), st.l[0] the running sum of the fp32 weights.
-template <bool kDebug, bool kTcBias, bool kGate>
+template <bool kDebug, bool kTcBias, bool kGate, int kW>
 __device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, float* dbg, int wg, int lane,
                                              uint32_t s_taddr, uint32_t p_taddr, uint32_t o_taddr,
                                              uint32_t bias_row, uint32_t row7, float scale, bool first_kt, long long* ts) {
@@ -805,7 +808,8 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, flo
   st.s_par ^= 1;
   tc_fence_after();
   if (kDebug && ts != nullptr) ts[1] = clock64();
-  uint32_t xr[kTile];
+  static_assert(kW % 16 == 0 && kW >= 32 && kW <= kTile && (kTcBias || kW == kTile), "key tiles of 32 to 128 keys");
+  uint32_t xr[kW];
   tmem_ld_x32(s_taddr, &xr[0]);
   // Under the load: what is left of the tile before, and a look whether its P V has finished.
   close_tile(st);
@@ -815,9 +819,9 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, flo
   float mt;
   {
     tc_wait_ld();
-    tmem_ld_x32(s_taddr + 32, &xr[32]);
-    tmem_ld_x32(s_taddr + 64, &xr[64]);
-    tmem_ld_x32(s_taddr + 96, &xr[96]);
+#pragma unroll
+    for (int i = 32; i + 32 <= kW; i += 32) tmem_ld_x32(s_taddr + i, &xr[i]);
+    if constexpr (kW % 32 != 0) tmem_ld_x16(s_taddr + kW - 16, &xr[kW - 16]);
     float mxa = -INFINITY, mxb = -INFINITY;
     if (kTcBias) row_max<0, 32>(xr, mxa, mxb);
     tc_wait_ld();
@@ -827,10 +831,10 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, flo
     if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::s_free + wg));
     if (kDebug && dbg != nullptr) {
 #pragma unroll
-      for (int i = 0; i < kTile; ++i) dbg[kDbgS + i] = __uint_as_float(xr[i]);
+      for (int i = 0; i < kW; ++i) dbg[kDbgS + i] = __uint_as_float(xr[i]);
     }
-    if (kTcBias) {
-      row_max<32, kTile>(xr, mxa, mxb);
+    if constexpr (kTcBias) {
+      row_max<32, kW>(xr, mxa, mxb);
     } else {
       const uint64_t scale2 = pack_f32x2(scale, scale);
       logits_half<0>(xr, bias_row, row7, scale2, mxa, mxb);
@@ -868,9 +872,9 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, flo
   const uint64_t nm2 = pack_f32x2(-m_use, -m_use);
   const uint64_t nml2 = pack_f32x2(nml, nml);
   uint64_t suma = pack_f32x2(0.f, 0.f), sumb = suma;
-  uint32_t pk[kTile / 2];        // P as bf16, two keys per 32-bit TMEM column: the A operand of the second GEMM
+  uint32_t pk[kW / 2];           // P as bf16, two keys per 32-bit TMEM column: the A operand of the second GEMM
 #pragma unroll
-  for (int i = 0; i < kTile / 2; ++i) {
+  for (int i = 0; i < kW / 2; ++i) {
     float y0, y1;
     const uint64_t x2 = pack_f32x2(__uint_as_float(xr[2 * i]), __uint_as_float(xr[2 * i + 1]));
     if (kTcBias) unpack_f32x2(fma_f32x2(x2, l2e2, nml2), y0, y1);
@@ -882,13 +886,18 @@ __device__ __forceinline__ bool softmax_tile(const Ctx& c, SoftmaxState& st, flo
     else       suma = add_f32x2(suma, pack_f32x2(p0, p1));
     pk[i] = pack_bf16x2(p0, p1);
     // Few and wide stores: 2048 fp8 rows, eight of 8 columns 10 370 us, four of 16 10 050, 32 and twice 16 9 900, two of 32 10 040.
-    if (i == 31) tmem_st_x32(p_taddr, pk);
-    if (i == 47) tmem_st_x16(p_taddr + 32, pk + 32);
-    if (i == 63) tmem_st_x16(p_taddr + 48, pk + 48);
+    constexpr int kWide = kW >= 80 ? 32 : 16;          // columns of the first store; 16 after that, 8 at the end of an odd multiple
+    if (i + 1 == kWide) {
+      if constexpr (kWide == 32) tmem_st_x32(p_taddr, pk); else tmem_st_x16(p_taddr, pk);
+    } else if (i + 1 > kWide && (i + 1 - kWide) % 16 == 0) {
+      tmem_st_x16(p_taddr + i - 15, pk + i - 15);
+    } else if (i + 1 == kW / 2) {
+      tmem_st_x8(p_taddr + i - 7, pk + i - 7);
+    }
   }
   if (kDebug && dbg != nullptr) {
 #pragma unroll
-    for (int i = 0; i < kTile / 2; ++i) dbg[kDbgP + i] = __uint_as_float(pk[i]);
+    for (int i = 0; i < kW / 2; ++i) dbg[kDbgP + i] = __uint_as_float(pk[i]);
   }
   if (kDebug && ts != nullptr) ts[6] = clock64();     // last exponential issued
   // What else has to be done with the accumulators before the next P V may write one.
@@ -944,7 +953,7 @@ __device__ __forceinline__ bool scale_own_q(const Ctx& c, int item, uint32_t j, 
   return true;
 }
 
-template <bool kDebug, bool kTcBias, bool kGate, bool kMixed, bool kScalesQ>
+template <bool kDebug, bool kTcBias, bool kGate, bool kMixed, bool kScalesQ, int kW>
 __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
   const AttnParams& p = *c.p;
   const int row = wq * 32 + lane;                    // row of the 128-query tile == TMEM lane
@@ -995,7 +1004,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
           if (item == 0 && s == 0 && kt == 0) dbg = p.debug + (size_t)row * kTile;
           ++n_tiles;
         }
-        if (!softmax_tile<kDebug, kTcBias, kGate>(c, st, dbg, wg, lane, s_taddr, p_taddr, c.tmem + lane_sel + kOCol + s * p.nv, bias_row, row & 7, scale,
+        if (!softmax_tile<kDebug, kTcBias, kGate, kW>(c, st, dbg, wg, lane, s_taddr, p_taddr, c.tmem + lane_sel + kOCol + s * p.nv, bias_row, row & 7, scale,
                                                   kt == 0, ts))
           return;
         st.swap = it.gv > wg + 2;
@@ -1070,7 +1079,7 @@ __device__ __forceinline__ void store_bias4(uint32_t tile, int row, int lane, ui
 // Rows that start on vectors (bias_wide): 16 rows' loads for the next tile follow directly on their store for this one, so that
 // 32 rows' are out nearly all the time.  The warp is alone on its scheduler beside a softmax warp that streams through its code, so the
 // loop is kept short: with a test for infinities and a second pass behind it 512 tokens took 11.4 us.
-template <bool kF32>
+template <bool kF32, int kW>
 __device__ void bias_convert_role(const Ctx& c, int wq, int lane) {
   const AttnParams& p = *c.p;
   constexpr int es = kF32 ? 4 : 2;
@@ -1081,7 +1090,7 @@ __device__ void bias_convert_role(const Ctx& c, int wq, int lane) {
   auto load = [&](const Item& it, int kt, int half) {
     const int first = it.qt * kTile + row0, last = min(31, p.Sq - 1 - first);
     if (last < 0) return;
-    const char* src = static_cast<const char*>(p.bias_src) + (it.h * p.bias_stride_h + first * p.bias_stride_r + min(kt * kTile + 4 * lane, p.Sk - 4)) * es;
+    const char* src = static_cast<const char*>(p.bias_src) + (it.h * p.bias_stride_h + first * p.bias_stride_r + min(kt * kW + 4 * lane, p.Sk - 4)) * es;
 #pragma unroll
     for (int r = 0; r < kConvertRows; ++r) x[half][r] = *reinterpret_cast<const Vec*>(src + min(half * kConvertRows + r, last) * step);
   };
@@ -1127,7 +1136,7 @@ __device__ void bias_convert_role(const Ctx& c, int wq, int lane) {
 
 // Rows that start anywhere, for items of one key tile: with more of them a pass of its own over the bias is faster (389 tokens
 // of ragged rows 12.7 us with it, 13.9 so).
-template <typename T>
+template <typename T, int kW>
 __device__ void bias_convert_ragged_role(const Ctx& c, int wq, int lane) {
   const AttnParams& p = *c.p;
   const int row0 = wq * 32;
@@ -1138,7 +1147,7 @@ __device__ void bias_convert_ragged_role(const Ctx& c, int wq, int lane) {
 #pragma unroll 1
     for (int kt = 0; kt < p.n_kt; ++kt) {
       const uint32_t tile = c.smem + p.off_bias + bst * kBiasTileBytes;
-      const int first = it.qt * kTile + row0, last = min(31, p.Sq - 1 - first), key = kt * kTile + 4 * lane;
+      const int first = it.qt * kTile + row0, last = min(31, p.Sq - 1 - first), key = kt * kW + 4 * lane;
       const T* src = static_cast<const T*>(p.bias_src) + it.h * p.bias_stride_h + first * p.bias_stride_r + key;
 #pragma unroll 1
       for (int r0 = 0; r0 < 32; r0 += kConvertRows) {
@@ -1172,7 +1181,8 @@ __device__ void bias_convert_ragged_role(const Ctx& c, int wq, int lane) {
 // tiles that leave a remainder), which takes slots and barriers that an item does not use through their phases and two sets
 // of constants to decode an item.  A plan of equal items runs without: 768 rows 645 -> 636 us.
 // kConvert: plans of one stream per item, bf16 q and k; see bias_convert_role.
-template <bool kDebug, bool kTcBias, bool kFp8, bool kGate, bool kMixed, bool kConvert = false>
+// kW: keys per key tile, 32 to 128 (chosen by key_width in the C API).
+template <bool kDebug, bool kTcBias, bool kFp8, bool kGate, bool kMixed, bool kConvert = false, int kW = kTile>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -1253,26 +1263,26 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     // warps 0-3 need few registers; the two softmax warpgroups take what they give up
     setmaxnreg_dec<kRegsMisc>();
     if (warp == 0) {
-      if (lane == 0) producer_role<kMixed, kConvert>(c, &tm_q, &tm_k, &tm_v, &tm_bias, &tm_q2, &tm_k2);
+      if (lane == 0) producer_role<kMixed, kConvert, kW>(c, &tm_q, &tm_k, &tm_v, &tm_bias, &tm_q2, &tm_k2);
     } else if (warp == 1) {
-      qk_issuer_role<kDebug, kTcBias, kFp8, kMixed>(c);
+      qk_issuer_role<kDebug, kTcBias, kFp8, kMixed, kW>(c);
     } else if (warp == 2) {
-      pv_issuer_role<kDebug, kMixed>(c);
+      pv_issuer_role<kDebug, kMixed, kW>(c);
     } else if (warp == 3) {
-      if (p.mask_col) mask_writer_role<kMixed>(c, lane);
+      if (p.mask_col) mask_writer_role<kMixed, kW>(c, lane);
     }
   } else {
     setmaxnreg_inc<kRegsSoftmax>();
     if (kConvert && warp >= 8) {
       if (p.bias_wide) {
-        if (p.bias_f32) bias_convert_role<true>(c, warp & 3, lane);
-        else            bias_convert_role<false>(c, warp & 3, lane);
+        if (p.bias_f32) bias_convert_role<true, kW>(c, warp & 3, lane);
+        else            bias_convert_role<false, kW>(c, warp & 3, lane);
       } else {
-        if (p.bias_f32) bias_convert_ragged_role<float>(c, warp & 3, lane);
-        else            bias_convert_ragged_role<uint16_t>(c, warp & 3, lane);
+        if (p.bias_f32) bias_convert_ragged_role<float, kW>(c, warp & 3, lane);
+        else            bias_convert_ragged_role<uint16_t, kW>(c, warp & 3, lane);
       }
     } else {
-      softmax_role<kDebug, kTcBias, kGate, kMixed, !kFp8>(c, (warp - 4) >> 2, warp & 3, lane);
+      softmax_role<kDebug, kTcBias, kGate, kMixed, !kFp8, kW>(c, (warp - 4) >> 2, warp & 3, lane);
     }
   }
 

@@ -375,3 +375,25 @@ def test_debug_dump_has_the_first_result(cuda_device, B1, B2, S, rows_per_item, 
     _, _, acc, sums = dump[:4 * 128 * 128].view(4, 128, 128)[:, :n].cpu()
     want = acc[:, :D] / sums[:, 1:2]
     assert ((out[0, 0, :n].float() - want).abs() <= 2 ** -8 * want.abs()).all()
+
+
+@pytest.mark.parametrize("Sk", [1, 16, 31, 32, 33, 64, 65, 80, 81, 96, 97, 112, 113, 128, 129, 160, 161, 192, 193, 224, 225, 256, 257, 288, 289, 336, 337, 385, 448,
+                                449, 560, 561])
+@pytest.mark.parametrize("qk,D", [("bf16", 24), ("bf16", 48), ("bf16", 64), ("fp8", 32)])
+def test_key_tiles_of_every_width(cuda_device, Sk, qk, D):
+    """Key tiles are as wide as the keys of a call need: first and last length of each width, with one to five tiles.  Several
+    pair rows per item with a remainder, two query tiles, and (fp32 bias, a single pair row) the bias converted on the way in."""
+    for B1, Sq in ((5, 140), (1, 70)):
+        q, k, v, mask, bias = _inputs(B1, 3, Sq, D, Sk + D, Sk)
+        mask[:, -1] = True
+        bias[..., -1] += 3            # the last key counts
+        scales = {}
+        if qk == "fp8":
+            q, k, scales = _quantised(q, k)
+        bias = bias.float() if B1 == 1 else bias.to(torch.bfloat16)
+        out = A.dot_product_attention_cpp(*(t.to(cuda_device) for t in (q, k, v, mask, bias)), **{n: t.to(cuda_device) for n, t in scales.items()}).cpu()
+        ref = O.oracle_fp32(q, k, v, mask, bias, **scales)
+        if qk == "fp8":
+            assert O.error_stats(out, ref)["max_abs"] <= 6e-2, (B1, Sk)
+        else:
+            _check(out, ref, (B1, Sk, D))
