@@ -871,9 +871,10 @@ int encode_weight_map(CUtensorMap* tm, const void* w, int64_t C, int64_t rows) {
 template <int C>
 void launch_front(const GridParams& p, const FrontMaps& tm, unsigned grid, bool f32, bool ln, cudaStream_t stream) {
   const uint32_t smem = f32 ? FrontTile<C, float>::kSmem : FrontTile<C, __nv_bfloat16>::kSmem;
-  if (!ln)      launch_overlapped(grid_front_kernel<C, __nv_bfloat16, false>, dim3(grid), kGridThreads, smem, stream, true, p, tm);
-  else if (f32) launch_overlapped(grid_front_kernel<C, float, true>, dim3(grid), kGridThreads, smem, stream, true, p, tm);
-  else          launch_overlapped(grid_front_kernel<C, __nv_bfloat16, true>, dim3(grid), kGridThreads, smem, stream, true, p, tm);
+  constexpr int kThreads = FrontTile<C, float>::kThreads;
+  if (!ln)      launch_overlapped(grid_front_kernel<C, __nv_bfloat16, false>, dim3(grid), kThreads, smem, stream, true, p, tm);
+  else if (f32) launch_overlapped(grid_front_kernel<C, float, true>, dim3(grid), kThreads, smem, stream, true, p, tm);
+  else          launch_overlapped(grid_front_kernel<C, __nv_bfloat16, true>, dim3(grid), kThreads, smem, stream, true, p, tm);
 }
 }  // namespace
 
@@ -970,11 +971,11 @@ int af3k_grid_out_weights(const void* weighted, const void* gate, const void* wo
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   const bool f32 = out_dtype == AF3K_F32;
   if (C == 128) {
-    if (f32) launch_overlapped(grid_out_kernel<128, float>, dim3(grid), kGridThreads, OutTile<128>::kSmem, stream, true, p, tm);
-    else     launch_overlapped(grid_out_kernel<128, __nv_bfloat16>, dim3(grid), kGridThreads, OutTile<128>::kSmem, stream, true, p, tm);
+    if (f32) launch_overlapped(grid_out_kernel<128, float>, dim3(grid), OutTile<128>::kThreads, OutTile<128>::kSmem, stream, true, p, tm);
+    else     launch_overlapped(grid_out_kernel<128, __nv_bfloat16>, dim3(grid), OutTile<128>::kThreads, OutTile<128>::kSmem, stream, true, p, tm);
   } else {
-    if (f32) launch_overlapped(grid_out_kernel<64, float>, dim3(grid), kGridThreads, OutTile<64>::kSmem, stream, true, p, tm);
-    else     launch_overlapped(grid_out_kernel<64, __nv_bfloat16>, dim3(grid), kGridThreads, OutTile<64>::kSmem, stream, true, p, tm);
+    if (f32) launch_overlapped(grid_out_kernel<64, float>, dim3(grid), OutTile<64>::kThreads, OutTile<64>::kSmem, stream, true, p, tm);
+    else     launch_overlapped(grid_out_kernel<64, __nv_bfloat16>, dim3(grid), OutTile<64>::kThreads, OutTile<64>::kSmem, stream, true, p, tm);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail("launch grid_out_kernel", e);

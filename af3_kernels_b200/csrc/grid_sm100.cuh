@@ -10,13 +10,13 @@
 //
 // Both are the same machine: persistent CTAs over tiles of 128 rows, the weights resident in shared memory,
 //
-//   warps 12-19  row producers: global -> registers -> (LayerNorm | gate product) -> bf16 ->
+//   warps 12-    row producers: global -> registers -> (LayerNorm | gate product) -> bf16 ->
 //                shared memory in the layout of a tcgen05.mma A operand (K-major, 128-byte swizzle,
 //                panels of 64 channels).  A row is spread over C / 8 lanes, 8 channels each, so global
 //                reads are full 16-byte pieces of consecutive lanes, the LayerNorm reductions are four
 //                (C = 64: three) shuffles and its parameters stay in registers.  The next rows are
 //                requested before the current ones are worked on.
-//   warp 0       TMEM allocation, the weights' TMA loads (fp32 weights: converted by warps 4-19), the MMAs (fp32
+//   warp 0       TMEM allocation, the weights' TMA loads (fp32 weights: converted by warps 4 on), the MMAs (fp32
 //                accumulators in TMEM)
 //   warps 4-11   epilogue, one TMEM lane quarter each, the two warpgroups taking the accumulators in turn: TMEM ->
 //                registers -> bf16 or fp32 -> a private XOR-swizzled patch of shared memory -> 16-byte stores
@@ -40,17 +40,23 @@
 
 namespace af3k {
 
-constexpr int kGridThreads = 640;
-constexpr int kGridProducerWarps = 8, kGridRowsPerWarp = 16;
-// Registers: launched with 96 per thread (61440, the pool setmaxnreg works in), then 128 x 32 (warps 0-3)
-// + 256 x 104 (epilogue) + 256 x 120 (row producers) = 61440.
-constexpr int kGridRegsMisc = 32, kGridRegsEpi = 104, kGridRegsRows = 120;
-static_assert(128 * kGridRegsMisc + 256 * kGridRegsEpi + 256 * kGridRegsRows <= 96 * kGridThreads,
-              "setmaxnreg totals exceed the launch allocation");
+// Twelve warps and the row producers, of which the front has 8 and the output pass 16: its rows carry two exponentials and
+// divisions per element in one chain, and two such warps per scheduler left it half idle (us, 8 -> 16 warps: 768 rows 90.5 -> 85.8,
+// 389 rows bf16 26.1 -> 24.1, fp32 29.8 -> 28.5, 256 rows of 64 channels 7.4 -> 7.1).  The front is bound by its writes: 768 rows
+// 149.7 -> 152.4 with 16, where reading 151 MB and writing 604 takes a bare kernel 144.
+// Registers: launched with kLaunch per thread (the pool setmaxnreg works in), then 128 x 32 (warps 0-3) + 256 x kEpi (epilogue)
+// + 32 kRowWarps x kRow (row producers).
+constexpr int kGridRegsMisc = 32;
+template <int kRowWarpsT> struct GridRoles {
+  static constexpr int kRowWarps = kRowWarpsT, kThreads = 32 * (12 + kRowWarps), kRowsPerWarp = 128 / kRowWarps;
+  static constexpr int kBatch = 32 / kRowWarps;      // steps of rows in flight (and worked on together) per warp
+  static constexpr int kLaunch = kRowWarps == 8 ? 96 : 72, kEpi = kRowWarps == 8 ? 104 : 88, kRow = kRowWarps == 8 ? 120 : 72;
+  static_assert(128 * kGridRegsMisc + 256 * kEpi + 32 * kRowWarps * kRow <= kLaunch * kThreads, "setmaxnreg totals exceed the launch allocation");
+};
 
 // Shared memory: kRows weight rows per panel of 64 channels, the A tiles, the epilogue patches, barriers.
-template <int C, int kRowsT, int kStagesT, bool kLowT = false>
-struct GridTile {
+template <int C, int kRowsT, int kStagesT, int kRowWarpsT, bool kLowT = false>
+struct GridTile : GridRoles<kRowWarpsT> {
   static constexpr int kStages = kStagesT, kRows = kRowsT;
   static constexpr bool kLow = kLowT;                      // a second A tile per stage for what bf16 leaves over of x
   static constexpr uint32_t kX = 128 * C * 2;              // one A tile: C / 64 panels of 128 rows x 128 bytes
@@ -68,8 +74,8 @@ constexpr int kBiasRows = 8;
 // fp32 pairs of 64 channels: x goes to the bias rows' MMAs in two parts as well, so that the bias is that of the fp32
 // normalised pair, as torch's LayerNorm and Linear compute it for other widths (at 128 channels af3k_pair_bias rounds x
 // first, and so does this).
-template <int C, typename T> using FrontTile = GridTile<C, 4 * C + kBiasRows, C == 128 ? 2 : 4, C == 64 && sizeof(T) == 4>;
-template <int C> using OutTile = GridTile<C, C, 4>;
+template <int C, typename T> using FrontTile = GridTile<C, 4 * C + kBiasRows, C == 128 ? 2 : 4, 8, C == 64 && sizeof(T) == 4>;
+template <int C> using OutTile = GridTile<C, C, 4, 16>;
 constexpr int kFrontAcc = 3;     // accumulators of C + 16 (rounded up to C + 32) TMEM columns, taken in turn
 
 struct GridBar {
@@ -164,22 +170,22 @@ __device__ __forceinline__ void params_at(const void* src, long long i, int f32,
   }
 }
 
-// One fp32 weight matrix [C, C] as rows row0 .. of the B operand, rounded to bf16 on the way (the 512 threads behind the
+// One fp32 weight matrix [C, C] as rows row0 .. of the B operand, rounded to bf16 on the way (the threads behind the
 // first four warps).  A packing pass in front of the block took 5 us: 389 fp32 rows 264 us a call, with this 261.
 template <class Tile, int C>
 __device__ __forceinline__ void grid_convert_weights(uint32_t smem, const void* src, int row0) {
-  constexpr int kItems = C * C / 8 / (kGridThreads - 128);      // 8 channels of a row each, all in flight at once
-  static_assert(kItems * 8 * (kGridThreads - 128) == C * C, "whole items per thread");
+  constexpr int kItems = (C * C / 8 + Tile::kThreads - 129) / (Tile::kThreads - 128);      // 8 channels of a row each, all in flight at once
   uint4 v[kItems][2];
 #pragma unroll
   for (int i = 0; i < kItems; ++i) {
-    const uint4* s = static_cast<const uint4*>(src) + 2 * (i * (kGridThreads - 128) + threadIdx.x - 128);
-    v[i][0] = s[0];
-    v[i][1] = s[1];
+    const int k = i * (Tile::kThreads - 128) + threadIdx.x - 128;
+    const uint4* s = static_cast<const uint4*>(src) + 2 * k;
+    if (k < C * C / 8) { v[i][0] = s[0]; v[i][1] = s[1]; }
   }
 #pragma unroll
   for (int i = 0; i < kItems; ++i) {
-    const int k = i * (kGridThreads - 128) + threadIdx.x - 128, r = row0 + k / (C / 8), c8 = k % (C / 8);
+    const int k = i * (Tile::kThreads - 128) + threadIdx.x - 128, r = row0 + k / (C / 8), c8 = k % (C / 8);
+    if (k >= C * C / 8) break;
     sts128(smem + (c8 >> 3) * (Tile::kRows * 128) + r * 128 + (((c8 & 7) ^ (r & 7)) << 4),
            pack_bf16x2(__uint_as_float(v[i][0].x), __uint_as_float(v[i][0].y)), pack_bf16x2(__uint_as_float(v[i][0].z), __uint_as_float(v[i][0].w)),
            pack_bf16x2(__uint_as_float(v[i][1].x), __uint_as_float(v[i][1].y)), pack_bf16x2(__uint_as_float(v[i][1].z), __uint_as_float(v[i][1].w)));
@@ -204,7 +210,7 @@ __device__ __forceinline__ uint32_t grid_prologue(const GridParams& p, uint32_t 
       for (int c = 0; c < chunks; ++c) prefetch_tensormap(tm_w + chunk0 + c);
     mbar_init(bars + 8u * GridBar::w_full, 1);
     for (int i = 0; i < Tile::kStages; ++i) {
-      mbar_init(bars + 8u * (GridBar::x_ready + i), kGridProducerWarps);
+      mbar_init(bars + 8u * (GridBar::x_ready + i), Tile::kRowWarps);
       mbar_init(bars + 8u * (GridBar::x_empty + i), 1);
     }
     for (int i = 0; i < 3; ++i) {
@@ -252,7 +258,7 @@ __device__ __forceinline__ void grid_epilogue_common(volatile int* abort_flag, u
 }
 
 template <int C, typename T, bool kLn>
-__global__ void __launch_bounds__(kGridThreads, 1)
+__global__ void __launch_bounds__(FrontTile<C, T>::kThreads, 1)
 grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ FrontMaps maps) {
   using Tile = FrontTile<C, T>;
   extern __shared__ __align__(1024) uint8_t grid_smem[];
@@ -271,7 +277,7 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
   if (with_bias && threadIdx.x >= 128) {
     // bias projection rows, 16 bytes (8 channels) per thread
     grid_wait_previous();
-    for (int k = threadIdx.x - 128; k < kBiasRows * (C / 8); k += kGridThreads - 128) {
+    for (int k = threadIdx.x - 128; k < kBiasRows * (C / 8); k += Tile::kThreads - 128) {
       const int r = k / (C / 8), c8 = k % (C / 8), h = r & 3;
       uint32_t w[4] = {0u, 0u, 0u, 0u};
       if (h < p.Hb) {
@@ -342,7 +348,7 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
     }
   } else if (warp < 12) {
     // ---- epilogue: TMEM lane quarter; warps 4-7 take the CTA's even outputs, 8-11 the odd ones
-    setmaxnreg_inc<kGridRegsEpi>();
+    setmaxnreg_inc<Tile::kEpi>();
     const int quarter = warp & 3, wg = (warp - 4) >> 2;
     const uint32_t t_lane = tmem + ((uint32_t)(quarter * 32) << 16);
     const uint32_t patch = smem + Tile::off_patch + (uint32_t)(warp - 4) * (32 * 128);
@@ -431,13 +437,13 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
       }
     }
   } else {
-    // ---- row producers: warp w normalises rows 16 w .. 16 w + 15 of every tile
-    setmaxnreg_inc<kGridRegsRows>();
+    // ---- row producers: warp w normalises its rows of every tile
+    setmaxnreg_inc<Tile::kRow>();
     const int w = warp - 12;
     constexpr int kLanes = C / 8;                       // lanes per row
     constexpr int kRowsIt = 32 / kLanes;                // rows per step of the warp
-    constexpr int kIts = kGridRowsPerWarp / kRowsIt;    // steps per tile
-    constexpr int kBatch = sizeof(T) == 2 ? 4 : 2;      // steps in flight (and worked on together)
+    constexpr int kIts = Tile::kRowsPerWarp / kRowsIt;    // steps per tile
+    constexpr int kBatch = sizeof(T) == 2 ? Tile::kBatch : Tile::kBatch / 2;
     static_assert(kIts % kBatch == 0, "whole batches per tile");
     const int c8 = lane % kLanes, sub = lane / kLanes;  // channels 8 c8 .., row within the step
     float g[8], b[8];
@@ -450,7 +456,7 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
     auto request = [&](long long tile, int it0) {
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {
-        const long long m = tile * 128 + w * kGridRowsPerWarp + (it0 + u) * kRowsIt + sub;
+        const long long m = tile * 128 + w * Tile::kRowsPerWarp + (it0 + u) * kRowsIt + sub;
         next[u] = load_raw8<T>(src + m * C, m < p.M);
       }
     };
@@ -503,7 +509,7 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
         for (int u = 0; u < kBatch; ++u) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) yw[u][e] = pack_bf16x2(y[u][2 * e], y[u][2 * e + 1]);
-          const int row = w * kGridRowsPerWarp + (it0 + u) * kRowsIt + sub;
+          const int row = w * Tile::kRowsPerWarp + (it0 + u) * kRowsIt + sub;
           sts128(grid_piece(x_tile, row, c8), yw[u][0], yw[u][1], yw[u][2], yw[u][3]);
           if (Tile::kLow && with_bias) {
             uint32_t lw[4];
@@ -525,7 +531,7 @@ done:
 }
 
 template <int C, typename TOut>
-__global__ void __launch_bounds__(kGridThreads, 1)
+__global__ void __launch_bounds__(OutTile<C>::kThreads, 1)
 grid_out_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CUtensorMap tm_w) {
   using Tile = OutTile<C>;
   extern __shared__ __align__(1024) uint8_t grid_smem[];
@@ -568,7 +574,7 @@ grid_out_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CU
     }
   } else if (warp < 12) {
     // ---- epilogue: warps 4-7 take the even tiles (accumulator 0), warps 8-11 the odd ones
-    setmaxnreg_inc<kGridRegsEpi>();
+    setmaxnreg_inc<Tile::kEpi>();
     const int quarter = warp & 3, buf = (warp - 4) >> 2;
     const uint32_t t_base = tmem + ((uint32_t)(quarter * 32) << 16) + buf * C;
     const uint32_t patch = smem + Tile::off_patch + (uint32_t)(warp - 4) * (32 * 128);
@@ -621,16 +627,15 @@ grid_out_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CU
     }
   } else {
     // ---- row producers: weighted * sigmoid(gate), sigmoid in fp32, rounded once
-    setmaxnreg_inc<kGridRegsRows>();
     const int w = warp - 12;
-    constexpr int kLanes = C / 8, kRowsIt = 32 / kLanes, kIts = kGridRowsPerWarp / kRowsIt, kBatch = 4;
+    constexpr int kLanes = C / 8, kRowsIt = 32 / kLanes, kIts = Tile::kRowsPerWarp / kRowsIt, kBatch = Tile::kBatch;
     static_assert(kIts % kBatch == 0, "whole batches per tile");
     const int c8 = lane % kLanes, sub = lane / kLanes;
     uint4 na[kBatch], ng[kBatch];
     auto request = [&](long long tile, int it0) {
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {
-        const long long m = tile * 128 + w * kGridRowsPerWarp + (it0 + u) * kRowsIt + sub;
+        const long long m = tile * 128 + w * Tile::kRowsPerWarp + (it0 + u) * kRowsIt + sub;
         na[u] = load_raw8<__nv_bfloat16>(p.weighted + m * C + 8 * c8, m < p.M).v[0];
         ng[u] = load_raw8<__nv_bfloat16>(p.gate + m * C + 8 * c8, m < p.M).v[0];
       }
@@ -656,7 +661,7 @@ grid_out_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CU
           for (int e = 0; e < 4; ++e)
             r[e] = pack_bf16x2(__uint_as_float(aw[e] << 16) * sigmoid_f32(__uint_as_float(gw[e] << 16)),
                                __uint_as_float(aw[e] & 0xffff0000u) * sigmoid_f32(__uint_as_float(gw[e] & 0xffff0000u)));
-          const int row = w * kGridRowsPerWarp + (it0 + u) * kRowsIt + sub;
+          const int row = w * Tile::kRowsPerWarp + (it0 + u) * kRowsIt + sub;
           sts128(grid_piece(x_tile, row, c8), r[0], r[1], r[2], r[3]);
         }
       }
