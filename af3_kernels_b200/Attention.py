@@ -61,6 +61,10 @@ class GridSelfAttentionCpp(nn.Module):
     @profile("B200 GridSelfAttention")
     def forward(self, pair: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
         host = _capi.host()
+        if type(self) is GridSelfAttentionCpp:
+            out = host.grid_forward(self, pair, mask, nn.Linear, nn.LayerNorm)        # the ordinary call
+            if out is not None:
+                return out
         if host.grid_fused(pair, self.num_head, self.num_head) and mask is not None and self._norm_and_bias_as_built(pair):
             # c_pair 64 or 128, up to four heads: three launches, LayerNorm to output projection
             lin = (self.q_projection, self.k_projection, self.v_projection, self.gating_query, self.output_projection)

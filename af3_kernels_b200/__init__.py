@@ -69,11 +69,12 @@ def dot_product_attention_cpp(
     computed in place on their device; host tensors (what the reference takes) go through
     ``dot_product_attention_host`` and come back as a host tensor.
     """
-    if int(BLK_SZ) <= 0 or int(FLASH_SZ) <= 0:
+    if (BLK_SZ != 128 or FLASH_SZ != 1024) and (int(BLK_SZ) <= 0 or int(FLASH_SZ) <= 0):
         raise ValueError("BLK_SZ and FLASH_SZ must be positive")
-    if q.is_cuda and (mask is None or (mask.dtype is torch.bool and 0 < mask.dim() < 3)) and isinstance(bias, torch.Tensor) and not _DEBUG:
-        # the ordinary call, straight to the native path, as below
-        return _capi.host().attention(q, k, v, mask, bias, q_scale, k_scale, None, 0, None, True, False, 0, 3)
+    if not _DEBUG:
+        out = _capi.host().operator_call(q, k, v, mask, bias, q_scale, k_scale)       # the ordinary call
+        if out is not None:
+            return out
     if not q.is_cuda:
         # host tensors, as the reference takes them: pipelined over PCIe, computed on the GPU,
         # result in host memory

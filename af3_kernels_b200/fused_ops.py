@@ -159,6 +159,9 @@ def self_attention_block(
 ) -> torch.Tensor:
     """x [N, C]; mask [N], True = attend; bias [head, N, N]; weights [C, C] as [in, out]; q_bias
     [C] (or [head, D]).  Returns [N, C] in ``x.dtype``."""
+    out = _capi.host().self_forward(x, mask, bias, q_proj, q_bias, k_proj, v_proj, gating_query, head)     # the ordinary call
+    if out is not None:
+        return out
     if x.dim() != 2:
         raise ValueError("x must be [num_tokens, channels]")
     if not x.is_cuda:
@@ -169,7 +172,7 @@ def self_attention_block(
     m = None if mask is None else bool_mask(mask.reshape(-1), 1, N)
     if (C // head) % 8 == 0 and C // head <= 64 and C <= 1024:
         # one GEMM for the four projections, one kernel for attention and gate
-        return _capi.host().self_block(x, m, bias, [w.t() for w in (q_proj, k_proj, v_proj, gating_query)], q_bias, head)
+        return _capi.host().self_block(x, m, bias, [q_proj, k_proj, v_proj, gating_query], q_bias, head)
     D = C // head
     xb = _as_bf16(x)
     q = (torch.matmul(xb, _as_bf16(q_proj)) + _as_bf16(q_bias).reshape(C)).view(1, N, head, D).permute(0, 2, 1, 3)

@@ -275,3 +275,16 @@ def test_grid_dispatch_takes_what_its_kernels_take(R, N, C, head, bias_heads, fu
     d = _desc(1, head, 128, C // head) if head and C % head == 0 else None
     if fused:
         assert _capi.load().af3k_describe_plan(ctypes.byref(d), (ctypes.c_int32 * 6)()) == 0
+
+
+def test_ordinary_calls_leave_host_tensors_to_the_general_way():
+    """The native short cuts answer None for what is not theirs."""
+    import af3_kernels_b200 as A
+    host = _capi.host()
+    q, bias = torch.zeros(1, 2, 16, 8, dtype=torch.bfloat16), torch.zeros(2, 16, 16)
+    assert host.operator_call(q, q, q, None, bias, None, None) is None
+    x, w = torch.zeros(16, 16), torch.zeros(16, 16)
+    assert host.self_forward(x, None, bias, w, w[0], w, w, w, 2) is None
+    m = A.GridSelfAttentionCpp(64, 4)
+    assert host.grid_forward(m, torch.zeros(8, 8, 64), torch.ones(8, 8, dtype=torch.bool), torch.nn.Linear, torch.nn.LayerNorm) is None
+    assert host.grid_forward(object(), torch.zeros(8, 8, 64), None, torch.nn.Linear, torch.nn.LayerNorm) is None

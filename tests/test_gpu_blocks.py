@@ -594,3 +594,84 @@ def test_grid_block_reads_weights_of_any_layout(cuda_device, R, N, C):
         assert torch.equal(r, res["out_in"]), n
     assert torch.equal(mixed, res["out_in"])
     assert read_status(dev)[0] == 0
+
+
+class _Subclass(A.GridSelfAttentionCpp):      # takes the module's general way
+    pass
+
+
+class _Scaled(torch.nn.Linear):
+    """A Linear whose weight is not what its parameters hold."""
+
+    def __getattr__(self, name):
+        value = super().__getattr__(name)
+        return value * 2 if name == "weight" else value
+
+
+@pytest.mark.parametrize("C", [64, 128])
+@pytest.mark.parametrize("form", ["plain", "mask_1d", "mask_uint8", "mask_3d", "float32", "hook", "replaced", "weight_in_dict", "functional", "half_norm", "trains_output"])
+def test_module_call_straight_from_python(cuda_device, C, form):
+    """Whatever parameters, layers, masks and modes a module is called with: the bits of the general way, and hooks run."""
+    g = torch.Generator().manual_seed(C)
+    N = 40
+    plain, general = A.GridSelfAttentionCpp(C, 4, True).to(cuda_device, torch.bfloat16), _Subclass(C, 4, True).to(cuda_device, torch.bfloat16)
+    calls = []
+    for m in (plain, general):
+        if form == "float32":
+            m.float()
+        if form == "half_norm":
+            m.act_norm.half()
+        if form == "replaced":
+            m.k_projection = _Scaled(C, C, bias=False).to(cuda_device, torch.bfloat16)
+        if form == "hook":
+            m.act_norm.register_forward_hook(lambda *a: calls.append(1))
+    params = [(torch.randn(p.shape, generator=g) * (C ** -0.5 if p.dim() == 2 else 0.2)).to(cuda_device) for p in plain.parameters()]
+    with torch.no_grad():
+        for m in (plain, general):
+            for p, value in zip(m.parameters(), params):
+                p.copy_(value)
+    if form == "weight_in_dict":
+        for m in (plain, general):
+            m.v_projection.__dict__["weight"] = m.v_projection.weight.detach() * 3
+    pair = torch.randn(N, N, C, generator=g).to(cuda_device, torch.float32 if form == "float32" else torch.bfloat16)
+    mask = (torch.rand(N, N, generator=g) >= 0.2).to(cuda_device)
+    mask = {"mask_1d": mask[0], "mask_uint8": mask.to(torch.uint8), "mask_3d": mask[:, None, None, :]}.get(form, mask)
+    call = lambda m: m(pair, mask)
+    if form == "functional":
+        new = {n: (p.detach() * 1.5) for n, p in plain.named_parameters()}
+        call = lambda m: torch.func.functional_call(m, new, (pair, mask))
+    with torch.enable_grad() if form == "trains_output" else torch.no_grad():
+        out, want = call(plain), call(general)
+    assert torch.equal(out, want) and out.dtype == pair.dtype
+    assert out.requires_grad == (form == "trains_output")
+    assert len(calls) == (2 if form == "hook" and C == 64 else 0)
+    assert read_status(cuda_device)[0] == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_single_block_and_operator_straight_from_python(cuda_device, dtype):
+    """Masks in other forms take the general way: the same bits; what is refused is refused on both."""
+    g = torch.Generator().manual_seed(5)
+    N, C, H = 70, 96, 4
+    x = torch.randn(N, C, generator=g).to(cuda_device, dtype)
+    ws = [(torch.randn(C, C, generator=g) * 0.1).to(cuda_device, dtype) for _ in range(4)]
+    qb, bias = torch.randn(C, generator=g).to(cuda_device), torch.randn(H, N, N, generator=g).to(cuda_device, dtype)
+    mask = (torch.rand(N, generator=g) >= 0.2).to(cuda_device)
+    for forms in ((None, torch.ones_like(mask)), (mask, mask.to(torch.uint8), mask[None], mask.float().reshape(1, 1, N))):
+        outs = [A.self_attention_cpp(x, m, bias, ws[0], qb, *ws[1:], H) for m in forms]
+        assert all(torch.equal(o, outs[0]) for o in outs) and outs[0].dtype == dtype
+    # [in, out] weights as views of [out, in] ones, and other strides
+    views = [w.t().contiguous().t() for w in ws]
+    assert torch.equal(A.self_attention_cpp(x, mask, bias, views[0], qb, *views[1:], H), outs[0])
+    strided = [torch.cat([w, w])[:, :].as_strided((C, C), (C, 1)) for w in ws]
+    assert torch.equal(A.self_attention_cpp(x, mask, bias, strided[0], qb, *strided[1:], H), outs[0])
+    q = x.reshape(1, N, H, C // H).permute(0, 2, 1, 3)
+    outs = [A.dot_product_attention_cpp(q, q, q, m, bias) for m in (mask, mask.to(torch.uint8), mask[None, None, None])]
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    for bad in (mask[:-1], torch.ones(3, N, dtype=torch.bool, device=cuda_device)):
+        with pytest.raises(ValueError):
+            A.dot_product_attention_cpp(q, q, q, bad, bias)
+        with pytest.raises(ValueError):
+            A.self_attention_cpp(x, bad, bias, ws[0], qb, *ws[1:], H)
+    with pytest.raises(ValueError):
+        A.dot_product_attention_cpp(q, q, q, mask, bias, False, 0)
