@@ -324,6 +324,10 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
           // the buffer's previous user must have finished its last Q K^T of this stream
           if (use >= 1) AF3K_WAIT(c, BarIdx::q_empty + slot, (use - 1) & 1);
           const uint32_t full = bar_addr(c, BarIdx::q_full + slot);
+          if (own && s == 0) {       // (a CTA's first item has a first stream)
+            grid_wait_previous();
+            grid_release_next();
+          }
           if (kMixed && s >= qi.gv) {
             mbar_arrive(full);
             continue;
@@ -421,6 +425,7 @@ __device__ void mask_writer_role(const Ctx& c, int lane) {
   const WaitBlock* wait_block = wait_block_of(c.bars);
   const uint32_t nkv = p.kv_stages;
   uint32_t st = 0, round = 0;      // ring slot, how many times the ring wrapped
+  grid_wait_previous();
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
     const Item it = decode_item<kMixed>(p, item);
@@ -976,6 +981,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
   const int scale_kt = !scales ? -1 : (p.q_buffers == 2 ? max(p.n_kt - 2, 0) : p.n_kt - 1);
   uint32_t icount = 0;
   if (scales && (int)blockIdx.x < p.n_items && !scale_own_q<kMixed>(c, blockIdx.x, 0, wg, wq, lane)) return;
+  grid_wait_previous();
 
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
@@ -1110,6 +1116,7 @@ __device__ void bias_convert_role(const Ctx& c, int wq, int lane) {
   };
   int item = blockIdx.x, kt = 0;
   Item it = decode_item<false>(p, item);     // (the grid has no more blocks than items)
+  grid_wait_previous();
 #pragma unroll
   for (int half = 0; half < 2; ++half) load(it, 0, half);
 #pragma unroll 1
@@ -1141,6 +1148,7 @@ __device__ void bias_convert_ragged_role(const Ctx& c, int wq, int lane) {
   const AttnParams& p = *c.p;
   const int row0 = wq * 32;
   uint32_t bst = 0, lap = 0;
+  grid_wait_previous();
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
     const Item it = decode_item<false>(p, item);
@@ -1252,8 +1260,6 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
                    "h"((uint16_t)0x3F80) : "memory");
     fence_proxy_async_smem();
   }
-  grid_wait_previous();
-  grid_release_next();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

@@ -16,7 +16,7 @@
 //                reads are full 16-byte pieces of consecutive lanes, the LayerNorm reductions are four
 //                (C = 64: three) shuffles and its parameters stay in registers.  The next rows are
 //                requested before the current ones are worked on.
-//   warp 0       TMEM allocation, the weights' TMA loads (fp32 weights: converted by warps 4 on), the MMAs (fp32
+//   warp 0       TMEM allocation, the weights' TMA loads (fp32 weights: converted by the epilogue warps), the MMAs (fp32
 //                accumulators in TMEM)
 //   warps 4-11   epilogue, one TMEM lane quarter each, the two warpgroups taking the accumulators in turn: TMEM ->
 //                registers -> bf16 or fp32 -> a private XOR-swizzled patch of shared memory -> 16-byte stores
@@ -44,14 +44,13 @@ namespace af3k {
 // divisions per element in one chain, and two such warps per scheduler left it half idle (us, 8 -> 16 warps: 768 rows 90.5 -> 85.8,
 // 389 rows bf16 26.1 -> 24.1, fp32 29.8 -> 28.5, 256 rows of 64 channels 7.4 -> 7.1).  The front is bound by its writes: 768 rows
 // 149.7 -> 152.4 with 16, where reading 151 MB and writing 604 takes a bare kernel 144.
-// Registers: launched with kLaunch per thread (the pool setmaxnreg works in), then 128 x 32 (warps 0-3) + 256 x kEpi (epilogue)
+// Registers: launched with kLaunch per thread (the pool setmaxnreg works in), then 128 x kMisc (warps 0-3) + 256 x kEpi (epilogue)
 // + 32 kRowWarps x kRow (row producers).
-constexpr int kGridRegsMisc = 32;
 template <int kRowWarpsT> struct GridRoles {
   static constexpr int kRowWarps = kRowWarpsT, kThreads = 32 * (12 + kRowWarps), kRowsPerWarp = 128 / kRowWarps;
   static constexpr int kBatch = 32 / kRowWarps;      // steps of rows in flight (and worked on together) per warp
-  static constexpr int kLaunch = kRowWarps == 8 ? 96 : 72, kEpi = kRowWarps == 8 ? 104 : 88, kRow = kRowWarps == 8 ? 120 : 72;
-  static_assert(128 * kGridRegsMisc + 256 * kEpi + 32 * kRowWarps * kRow <= kLaunch * kThreads, "setmaxnreg totals exceed the launch allocation");
+  static constexpr int kLaunch = kRowWarps == 8 ? 96 : 72, kMisc = kRowWarps == 8 ? 48 : 40, kEpi = kRowWarps == 8 ? 96 : 88, kRow = kRowWarps == 8 ? 120 : 72;
+  static_assert(128 * kMisc + 256 * kEpi + 32 * kRowWarps * kRow <= kLaunch * kThreads, "setmaxnreg totals exceed the launch allocation");
 };
 
 // Shared memory: kRows weight rows per panel of 64 channels, the A tiles, the epilogue patches, barriers.
@@ -170,45 +169,40 @@ __device__ __forceinline__ void params_at(const void* src, long long i, int f32,
   }
 }
 
-// One fp32 weight matrix [C, C] as rows row0 .. of the B operand, rounded to bf16 on the way (the threads behind the
-// first four warps).  A packing pass in front of the block took 5 us: 389 fp32 rows 264 us a call, with this 261.
-template <class Tile, int C>
-__device__ __forceinline__ void grid_convert_weights(uint32_t smem, const void* src, int row0) {
-  constexpr int kItems = (C * C / 8 + Tile::kThreads - 129) / (Tile::kThreads - 128);      // 8 channels of a row each, all in flight at once
+// One fp32 weight matrix [C, C] as rows row0 .. of the B operand, rounded to bf16 on the way (the 256 threads of the epilogue
+// warps).  A packing pass in front of the block took 5 us: 389 fp32 rows 264 us a call, with this 261.
+template <int C>
+__device__ __forceinline__ void grid_convert_weights(uint32_t smem, int rows, const void* src, int row0) {
+  constexpr int kItems = C * C / 8 / 256;      // 8 channels of a row each, all in flight at once
+  static_assert(kItems * 8 * 256 == C * C, "whole items per thread");
   uint4 v[kItems][2];
+  const int k0 = threadIdx.x - 128;
 #pragma unroll
   for (int i = 0; i < kItems; ++i) {
-    const int k = i * (Tile::kThreads - 128) + threadIdx.x - 128;
-    const uint4* s = static_cast<const uint4*>(src) + 2 * k;
-    if (k < C * C / 8) { v[i][0] = s[0]; v[i][1] = s[1]; }
+    const uint4* s = static_cast<const uint4*>(src) + 2 * (k0 + i * 256);
+    v[i][0] = s[0];
+    v[i][1] = s[1];
   }
 #pragma unroll
   for (int i = 0; i < kItems; ++i) {
-    const int k = i * (Tile::kThreads - 128) + threadIdx.x - 128, r = row0 + k / (C / 8), c8 = k % (C / 8);
-    if (k >= C * C / 8) break;
-    sts128(smem + (c8 >> 3) * (Tile::kRows * 128) + r * 128 + (((c8 & 7) ^ (r & 7)) << 4),
+    const int k = k0 + i * 256, r = row0 + k / (C / 8), c8 = k % (C / 8);
+    sts128(smem + (c8 >> 3) * (rows * 128) + r * 128 + (((c8 & 7) ^ (r & 7)) << 4),
            pack_bf16x2(__uint_as_float(v[i][0].x), __uint_as_float(v[i][0].y)), pack_bf16x2(__uint_as_float(v[i][0].z), __uint_as_float(v[i][0].w)),
            pack_bf16x2(__uint_as_float(v[i][1].x), __uint_as_float(v[i][1].y)), pack_bf16x2(__uint_as_float(v[i][1].z), __uint_as_float(v[i][1].w)));
   }
 }
 
-// Barrier set-up, TMEM allocation and weight loads shared by both kernels (all threads; ends with a block
-// barrier).  The weights are `chunks` matrices of C rows from p.w[chunk0] on, one tensor map each; `gap` rows are left
-// free behind the first one.
-template <class Tile, int C>
-__device__ __forceinline__ uint32_t grid_prologue(const GridParams& p, uint32_t smem, uint32_t bars, volatile uint32_t* slot,
-                                                  volatile int* abort_flag, uint32_t tmem_cols, const CUtensorMap* tm_w, int chunk0, int chunks,
-                                                  int gap) {
+// Barrier set-up and TMEM allocation shared by both kernels (all threads; ends with a block barrier).  Nothing here touches
+// global memory: each role waits for the kernel before (grid_wait_previous) where it first does, with its set-up behind it.
+template <class Tile>
+__device__ __forceinline__ uint32_t grid_prologue(const GridParams& p, uint32_t bars, volatile uint32_t* slot, volatile int* abort_flag, uint32_t tmem_cols,
+                                                  const CUtensorMap* tm_w, int chunks) {
   const int warp = threadIdx.x >> 5;
-  if (p.w_f32 && threadIdx.x >= 128) {
-    grid_wait_previous();
-    for (int c = 0; c < chunks; ++c) grid_convert_weights<Tile, C>(smem, p.w[chunk0 + c], c * C + (c > 0 ? gap : 0));
-  }
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     if (!p.w_f32)
-      for (int c = 0; c < chunks; ++c) prefetch_tensormap(tm_w + chunk0 + c);
-    mbar_init(bars + 8u * GridBar::w_full, 1);
+      for (int c = 0; c < chunks; ++c) prefetch_tensormap(tm_w + c);
+    mbar_init(bars + 8u * GridBar::w_full, 1 + 8);           // the loading thread, the epilogue warps
     for (int i = 0; i < Tile::kStages; ++i) {
       mbar_init(bars + 8u * (GridBar::x_ready + i), Tile::kRowWarps);
       mbar_init(bars + 8u * (GridBar::x_empty + i), 1);
@@ -218,29 +212,43 @@ __device__ __forceinline__ uint32_t grid_prologue(const GridParams& p, uint32_t 
       mbar_init(bars + 8u * (GridBar::acc_empty + i), 4);
     }
     fence_barrier_init();
-    grid_wait_previous();
-    if (p.w_f32) {
-      mbar_arrive(bars + 8u * GridBar::w_full);
-    } else {
-      mbar_arrive_expect_tx(bars + 8u * GridBar::w_full, (uint32_t)chunks * C * C * 2);
-      for (int c = 0; c < chunks; ++c)
-        for (int kb = 0; kb < C / 64; ++kb)
-          for (int r = 0; r < C; r += 64)
-            tma_load_2d(smem + kb * (Tile::kRows * 128) + (c * C + (c > 0 ? gap : 0) + r) * 128, tm_w + chunk0 + c, bars + 8u * GridBar::w_full,
-                        kb * 64, r);
-    }
   }
   if (warp == 0) {
     __syncwarp();
     tmem_alloc(smem_u32(const_cast<uint32_t*>(slot)), tmem_cols);
     tmem_relinquish();
   }
-  grid_wait_previous();
-  fence_proxy_async_smem();      // whatever the caller stored for the tensor core
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   return *slot;
+}
+
+// The weights, `chunks` matrices of C rows from p.w[chunk0] on, one tensor map each; `gap` rows are left free behind the first one.
+// One thread requests bf16 ones ...
+template <class Tile, int C>
+__device__ __forceinline__ void grid_load_weights(const GridParams& p, uint32_t smem, uint32_t bars, const CUtensorMap* tm_w, int chunk0, int chunks, int gap) {
+  grid_wait_previous();
+  if (p.w_f32) {
+    mbar_arrive(bars + 8u * GridBar::w_full);
+    return;
+  }
+  mbar_arrive_expect_tx(bars + 8u * GridBar::w_full, (uint32_t)chunks * C * C * 2);
+  for (int c = 0; c < chunks; ++c)
+    for (int kb = 0; kb < C / 64; ++kb)
+      for (int r = 0; r < C; r += 64)
+        tma_load_2d(smem + kb * (Tile::kRows * 128) + (c * C + (c > 0 ? gap : 0) + r) * 128, tm_w + chunk0 + c, bars + 8u * GridBar::w_full, kb * 64, r);
+}
+// ... the epilogue warps convert fp32 ones while there is nothing to store yet (and the front's write its bias rows), then arrive.
+template <class Tile, int C>
+__device__ __forceinline__ void grid_convert_all(const GridParams& p, uint32_t smem, int chunk0, int chunks, int gap) {
+  if (p.w_f32)
+    for (int c = 0; c < chunks; ++c) grid_convert_weights<C>(smem, Tile::kRows, p.w[chunk0 + c], c * C + (c > 0 ? gap : 0));
+}
+__device__ __forceinline__ void grid_weights_written(uint32_t bars, int lane) {
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) mbar_arrive(bars + 8u * GridBar::w_full);
 }
 
 // Block-wide end of both kernels.
@@ -274,38 +282,18 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
   const int chunks = 4 / p.split, chunk0 = part * chunks;
   const bool with_bias = kLn && p.Hb > 0 && part == 0;
   const long long n_tiles = (p.M + 127) / 128;
-  if (with_bias && threadIdx.x >= 128) {
-    // bias projection rows, 16 bytes (8 channels) per thread
-    grid_wait_previous();
-    for (int k = threadIdx.x - 128; k < kBiasRows * (C / 8); k += Tile::kThreads - 128) {
-      const int r = k / (C / 8), c8 = k % (C / 8), h = r & 3;
-      uint32_t w[4] = {0u, 0u, 0u, 0u};
-      if (h < p.Hb) {
-        float v[8];
-        params_at(p.bias_w, h * C + c8 * 8, p.bias_w_f32, v);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float x = v[2 * e], y = v[2 * e + 1];
-          if (r >= 4) {   // what the bf16 high part leaves over
-            x -= __bfloat162float(__float2bfloat16_rn(x));
-            y -= __bfloat162float(__float2bfloat16_rn(y));
-          }
-          w[e] = pack_bf16x2(x, y);
-        }
-      }
-      sts128(smem + (c8 >> 3) * (Tile::kRows * 128) + (C + r) * 128 + (((c8 & 7) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
-    }
-  }
-  const uint32_t tmem = grid_prologue<Tile, C>(p, smem, bars, slot, abort_flag, kTmem, maps.w, chunk0, chunks, kBiasRows);
+  const uint32_t tmem = grid_prologue<Tile>(p, bars, slot, abort_flag, kTmem, maps.w + chunk0, chunks);
 
   if (warp < 4) {
-    setmaxnreg_dec<kGridRegsMisc>();
+    setmaxnreg_dec<Tile::kMisc>();
     if (warp == 0) {
       // ---- MMA issuer: the tile's outputs one after the other, into the accumulators in turn
       const bool leader = elect_one();
       const uint32_t idesc = make_idesc(1u, 1u, 0u, 0u, C), idesc_q = make_idesc(1u, 1u, 0u, 0u, C + 16);
       const uint64_t ad0 = make_smem_desc(smem + Tile::off_x, 16, 8 * 128, 2), bd0 = make_smem_desc(smem, 16, 8 * 128, 2);
       const uint32_t ad_lo = (uint32_t)ad0, ad_hi = (uint32_t)(ad0 >> 32), bd_lo = (uint32_t)bd0, bd_hi = (uint32_t)(bd0 >> 32);
+      if (leader) grid_load_weights<Tile, C>(p, smem, bars, maps.w, chunk0, chunks, kBiasRows);
+      __syncwarp();
       AF3K_GRID_WAIT(GridBar::w_full, 0);
       uint32_t n = 0, buf = 0, lap = 0;
       for (long long tile = first; tile < n_tiles; tile += step, ++n) {
@@ -348,7 +336,30 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
     }
   } else if (warp < 12) {
     // ---- epilogue: TMEM lane quarter; warps 4-7 take the CTA's even outputs, 8-11 the odd ones
-    setmaxnreg_inc<Tile::kEpi>();
+    grid_wait_previous();
+    if (with_bias) {
+      // bias projection rows, 16 bytes (8 channels) per thread
+      for (int k = threadIdx.x - 128; k < kBiasRows * (C / 8); k += 256) {
+        const int r = k / (C / 8), c8 = k % (C / 8), h = r & 3;
+        uint32_t w[4] = {0u, 0u, 0u, 0u};
+        if (h < p.Hb) {
+          float v[8];
+          params_at(p.bias_w, h * C + c8 * 8, p.bias_w_f32, v);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            float x = v[2 * e], y = v[2 * e + 1];
+            if (r >= 4) {   // what the bf16 high part leaves over
+              x -= __bfloat162float(__float2bfloat16_rn(x));
+              y -= __bfloat162float(__float2bfloat16_rn(y));
+            }
+            w[e] = pack_bf16x2(x, y);
+          }
+        }
+        sts128(smem + (c8 >> 3) * (Tile::kRows * 128) + (C + r) * 128 + (((c8 & 7) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+      }
+    }
+    grid_convert_all<Tile, C>(p, smem, chunk0, chunks, kBiasRows);
+    grid_weights_written(bars, lane);
     const int quarter = warp & 3, wg = (warp - 4) >> 2;
     const uint32_t t_lane = tmem + ((uint32_t)(quarter * 32) << 16);
     const uint32_t patch = smem + Tile::off_patch + (uint32_t)(warp - 4) * (32 * 128);
@@ -446,11 +457,6 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
     constexpr int kBatch = sizeof(T) == 2 ? Tile::kBatch : Tile::kBatch / 2;
     static_assert(kIts % kBatch == 0, "whole batches per tile");
     const int c8 = lane % kLanes, sub = lane / kLanes;  // channels 8 c8 .., row within the step
-    float g[8], b[8];
-    if (kLn) {
-      params_at(p.gamma, 8 * c8, p.ln_f32, g);
-      params_at(p.beta, 8 * c8, p.ln_f32, b);
-    }
     const T* src = static_cast<const T*>(p.pair) + 8 * c8;
     Raw8<T> next[kBatch];
     auto request = [&](long long tile, int it0) {
@@ -460,7 +466,13 @@ grid_front_kernel(const __grid_constant__ GridParams p, const __grid_constant__ 
         next[u] = load_raw8<T>(src + m * C, m < p.M);
       }
     };
+    float g[8], b[8];
+    grid_wait_previous();
     if (first < n_tiles) request(first, 0);
+    if (kLn) {
+      params_at(p.gamma, 8 * c8, p.ln_f32, g);
+      params_at(p.beta, 8 * c8, p.ln_f32, b);
+    }
     uint32_t n = 0;
     for (long long tile = first; tile < n_tiles; tile += step, ++n) {
       const uint32_t st = n % Tile::kStages;
@@ -542,15 +554,17 @@ grid_out_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CU
   volatile int* abort_flag = reinterpret_cast<volatile int*>(grid_smem + Tile::off_slot + 4);
   constexpr uint32_t kTmem = 2 * C;               // two accumulators, taken in turn
   const long long n_tiles = (p.M + 127) / 128;
-  const uint32_t tmem = grid_prologue<Tile, C>(p, smem, bars, slot, abort_flag, kTmem, &tm_w, 0, 1, 0);
+  const uint32_t tmem = grid_prologue<Tile>(p, bars, slot, abort_flag, kTmem, &tm_w, 1);
 
   if (warp < 4) {
-    setmaxnreg_dec<kGridRegsMisc>();
+    setmaxnreg_dec<Tile::kMisc>();
     if (warp == 0) {
       const bool leader = elect_one();
       const uint32_t idesc = make_idesc(1u, 1u, 0u, 0u, (uint32_t)C);
       const uint64_t ad0 = make_smem_desc(smem + Tile::off_x, 16, 8 * 128, 2), bd0 = make_smem_desc(smem, 16, 8 * 128, 2);
       const uint32_t ad_lo = (uint32_t)ad0, ad_hi = (uint32_t)(ad0 >> 32), bd_lo = (uint32_t)bd0, bd_hi = (uint32_t)(bd0 >> 32);
+      if (leader) grid_load_weights<Tile, C>(p, smem, bars, &tm_w, 0, 1, 0);
+      __syncwarp();
       AF3K_GRID_WAIT(GridBar::w_full, 0);
       uint32_t n = 0;
       for (long long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++n) {
@@ -579,6 +593,9 @@ grid_out_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CU
     const uint32_t t_base = tmem + ((uint32_t)(quarter * 32) << 16) + buf * C;
     const uint32_t patch = smem + Tile::off_patch + (uint32_t)(warp - 4) * (32 * 128);
     constexpr int kCols = 128 / (int)sizeof(TOut);      // columns per 128-byte piece of a row
+    grid_wait_previous();
+    grid_convert_all<Tile, C>(p, smem, 0, 1, 0);
+    grid_weights_written(bars, lane);
     uint32_t n = (uint32_t)buf;
     for (long long tile = blockIdx.x + (long long)buf * gridDim.x; tile < n_tiles; tile += 2LL * gridDim.x, n += 2) {
       const long long m0 = tile * 128 + quarter * 32;
@@ -640,6 +657,7 @@ grid_out_kernel(const __grid_constant__ GridParams p, const __grid_constant__ CU
         ng[u] = load_raw8<__nv_bfloat16>(p.gate + m * C + 8 * c8, m < p.M).v[0];
       }
     };
+    grid_wait_previous();
     if ((long long)blockIdx.x < n_tiles) request(blockIdx.x, 0);
     uint32_t n = 0;
     for (long long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++n) {

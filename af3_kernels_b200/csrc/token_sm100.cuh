@@ -72,8 +72,6 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
     tmem_alloc(smem_u32(const_cast<uint32_t*>(slot)), kN);
     tmem_relinquish();
   }
-  grid_wait_previous();
-  grid_release_next();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -88,6 +86,10 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
           break;
         }
         const uint32_t full = bars + 8u * st, dst = smem + st * Tile::kStage;
+        if (kb == 0) {
+          grid_wait_previous();
+          grid_release_next();
+        }
         mbar_arrive_expect_tx(full, Tile::kStage);
         tma_load_2d(dst, &tm_x, full, kb * 64, m0);
         if (!mn) {
@@ -124,6 +126,7 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
   } else {
     // ---- epilogue: TMEM lane quarter; the stages are free when the accumulator is complete
     const int quarter = warp & 3;
+    grid_wait_previous();
     // The query bias lands in shared memory while the GEMM runs.  Read in the epilogue, element by element in the type it is kept in,
     // it was most of the kernel, each load behind the one before: 1536 tokens of 384 channels 13.7 -> 5.1 us, of 768 18.4 -> 12.5,
     // 128 tokens of 384 9.4 -> 4.0.
