@@ -229,6 +229,7 @@ struct Plan {
   AttnParams p;
   size_t smem_bytes;
   int grid;
+  double cost;     // of the longest CTA, in logits-tile times of one warpgroup
 };
 
 // The longest CTA's time when n_main items of cost c_main and then n_tail of cost c_tail are dealt out round-robin.
@@ -271,7 +272,8 @@ int key_width(const af3k_attention_desc& d, bool tc_bias, bool debug) {
 // Picks rows-per-item G and the K/V ring depth from a cost model of one CTA's time (below).
 // allow_q_split: the kernel variant that will run supports query-tile streams (every variant in
 // which the tensor core adds the bias).
-int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, bool allow_q_split = true) {
+// lone: one query tile of one pair row per item.
+int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, bool allow_q_split = true, bool lone = false) {
   AttnParams& p = plan->p;
   std::memset(&p, 0, sizeof(p));
   const int es = d.qk_dtype == AF3K_FP8_E4M3 ? 1 : 2;
@@ -305,6 +307,7 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   const int g_tmem = (int)((kTmemCols - kOCol) / p.nv);
   int g_max = kMaxStreams < g_tmem ? kMaxStreams : g_tmem;
   if (g_max > p.B1) g_max = p.B1 > 0 ? p.B1 : 1;
+  if (lone) g_max = 1;
 
   int best_g = 0, best_stages = 0, best_qbuf = 0;
   bool best_split = false;
@@ -326,7 +329,7 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   for (int g = 1; g <= g_max; ++g) {
     if (g_req != 0 && g != g_req) continue;
     // one pair row per item: the two softmax warpgroups take two neighbouring query tiles, or one of them idles
-    const bool may_split = g == 1 && allow_q_split && p.n_qt >= 2;
+    const bool may_split = g == 1 && allow_q_split && p.n_qt >= 2 && !lone;
     for (int form = may_split ? 0 : 2; form < 4; ++form) {
       const bool split = form < 2;
       const int qbuf = 2 - (form & 1);
@@ -361,6 +364,7 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
     }
   }
   if (best_g == 0) return AF3K_ERR_BAD_SHAPE;
+  plan->cost = best_cost;
   p.G = best_g;
   p.q_split = best_split ? 1 : 0;
   p.n_streams = p.q_split ? 2 : p.G;
@@ -411,6 +415,31 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   plan->smem_bytes = smem;
   plan->grid = p.n_items < ctas ? p.n_items : ctas;
   return AF3K_OK;
+}
+
+// Whether the attention kernel is to convert the bias itself (then *plan is one that can: one query tile of one pair row per item).
+// Estimates in us, for key tiles of 128: the pass 1.7 and 5 TB/s; a tile of a pair of streams 1.6; a lone tile whose bias is converted
+// 1.65 (rows on vectors; no slower than in place) or, where rows start anywhere, 2.2, which is 0.75 more than in place.
+// Measured, us, pass before -> here: 16 heads, rows anywhere: 129 tokens 7.1 -> 6.3, 389 bf16 12.0 -> 10.5, 1001 bf16 26.8 -> 19.5,
+// fp32 34.4 -> 19.5; 5 heads of 385 9.5 (here 10.4).  In place of pairs of query tiles: 1300 tokens bf16 43.7 -> 38.1, fp32 53.8 -> 43.7;
+// 1536 fp32 61 -> 46; 2047 bf16 89 -> 79, fp32 118 -> 79; 2048 fp32 96 -> 63; 1301 bf16 43.9 and 1537 bf16 57.4 keep the pass.
+// (Calls of a few items, bound by the host either way, keep it too.)
+constexpr int kFewItems = 16;
+bool convert_in_kernel(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, bool wide) {
+  const AttnParams& p = plan->p;
+  const double es = d.bias_dtype == AF3K_F32 ? 4 : 2, elements = (double)d.B2 * d.Sq * d.Sk, width = p.kw / (double)kTile;
+  const double pass = 1.7 + elements * (es + 2) / 5e6;
+  if (p.n_streams == 1 && !p.mixed) {
+    const int rounds = (p.n_items + plan->grid - 1) / plan->grid;
+    return wide || p.n_kt == 1 || (p.n_items >= kFewItems && rounds * p.n_kt * 0.75 * width < pass);
+  }
+  Plan lone;
+  if (d.rows_per_item > 1 || make_plan(d, dev, &lone, true, true) != AF3K_OK || lone.p.mixed) return false;
+  const int rounds = (lone.p.n_items + lone.grid - 1) / lone.grid;
+  const double here = rounds * (lone.p.n_kt * (wide ? 1.65 : 2.2) * width + 1.3), reads = d.B1 * elements * es / 5e6;   // each pair row reads the whole bias
+  if ((here > reads ? here : reads) >= 0.95 * (plan->cost * 1.6 * width + pass)) return false;
+  *plan = lone;
+  return true;
 }
 
 int encode_qkv_map(CUtensorMap* tm, const void* base, bool fp8, int64_t D, int64_t S, int64_t B2,
@@ -613,10 +642,11 @@ int attention_call(const af3k_attention_desc* desc, const void* q, const void* k
   const bool stage_fp8 = fp8 && !d.bias_prescaled && workspace != nullptr && workspace_bytes >= stage_bytes &&
                          aligned16(workspace);
   const bool fp8_tc = fp8 && (d.bias_prescaled || stage_fp8);
-  // the kernel converts the bias itself: items of one query tile, rows that start on vectors or a single key tile
+  // the kernel converts the bias itself: items of one query tile
   const uintptr_t bias_es = d.bias_dtype == AF3K_F32 ? 4 : 2;
-  p.bias_wide = d.Sk % 4 == 0 && (reinterpret_cast<uintptr_t>(bias) | (uintptr_t)bias_sh * bias_es | (uintptr_t)bias_sr * bias_es) % (4 * bias_es) == 0 ? 1 : 0;
-  const bool in_kernel = convert && must_stage && !fp8 && p.n_streams == 1 && !p.mixed && (p.bias_wide || p.n_kt == 1) && p.debug == nullptr;
+  const bool wide = d.Sk % 4 == 0 && (reinterpret_cast<uintptr_t>(bias) | (uintptr_t)bias_sh * bias_es | (uintptr_t)bias_sr * bias_es) % (4 * bias_es) == 0;
+  const bool in_kernel = convert && must_stage && !fp8 && p.debug == nullptr && convert_in_kernel(d, *dev, &plan, wide);
+  p.bias_wide = wide ? 1 : 0;
   if ((must_stage && !in_kernel) || stage_fp8) {
     if (workspace == nullptr || workspace_bytes < stage_bytes) return AF3K_ERR_WORKSPACE;
     if (!aligned16(workspace)) return AF3K_ERR_BAD_ALIGNMENT;
@@ -667,7 +697,7 @@ int attention_call(const af3k_attention_desc* desc, const void* q, const void* k
   p.scale_q = (fp8 || d.softmax_scale == 1.0f) ? 0 : 1;   // a scale of exactly 1 (q already scaled by its producer) needs no pass over Q
   const bool dbg = p.debug != nullptr;
   const auto launch = [&](auto kernel) {
-    launch_overlapped(kernel, dim3(plan.grid), kThreads, plan.smem_bytes, stream, d.max_ctas <= 0, p, tm_q, tm_k, tm_v, tm_b, tm_q2, tm_k2);
+    launch_overlapped(kernel, dim3(plan.grid), in_kernel ? kConvertThreads : kThreads, plan.smem_bytes, stream, d.max_ctas <= 0, p, tm_q, tm_k, tm_v, tm_b, tm_q2, tm_k2);
   };
   if (in_kernel) {
     if (p.gate != nullptr) with_width<false, true, false, true>(p.kw, launch);

@@ -56,8 +56,11 @@ namespace af3k {
 
 constexpr int kTile = 128;         // query rows per tile, and the most keys
 constexpr int kThreads = 384;      // 12 warps
+constexpr int kConvertThreads = 512;   // kConvert: one softmax warpgroup, eight warps that make bias tiles
 // 65536 registers per SM: launched at 168 per thread, then 128 x 72 + 256 x 216 = 64512
 constexpr int kRegsMisc = 72, kRegsSoftmax = 216;
+// kConvert: launched at 128 per thread, then 128 x 72 + 128 x 216 + 256 x 104 = 63488 of 65536
+constexpr int kRegsConvert = 104;
 constexpr int kMaxStreams = 4;     // pair rows per work item (two per softmax warpgroup; TMEM: kOCol + G * nv <= 512 columns)
 // TMEM columns: two fp32 logits buffers, two bf16 P buffers (two keys per column), then O.
 constexpr uint32_t kSCol = 0, kPCol = 2 * 128, kOCol = 2 * 128 + 2 * 64;
@@ -1056,19 +1059,14 @@ __device__ __forceinline__ uint32_t staged_pair(float a, float b) {
   return w;
 }
 
-constexpr int kConvertRows = 16;   // rows of a tile in one round of loads
+// The same for two that are bf16 already.
+__device__ __forceinline__ uint32_t clamped_pair(uint32_t w) {
+  asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(w) : "r"(0xff7fff7fu));
+  asm("min.NaN.bf16x2 %0, %0, %1;" : "+r"(w) : "r"(0x7f7f7f7fu));
+  return w;
+}
 
-// A load with a predicate and without a branch, so that many are out at once.
-__device__ __forceinline__ float load_if(const float* a, uint32_t there) {
-  float x = 0.f;
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.f32 %0, [%1];\n\t}" : "+f"(x) : "l"(a), "r"(there));
-  return x;
-}
-__device__ __forceinline__ float load_if(const uint16_t* a, uint32_t there) {
-  uint16_t x = 0;
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.u16 %0, [%1];\n\t}" : "+h"(x) : "l"(a), "r"(there));
-  return __uint_as_float((uint32_t)x << 16);
-}
+constexpr int kConvertWarps = 8, kConvertRows = 8;   // each warp makes 16 rows of a tile (two rounds of loads)
 
 // One row's keys 4 lane .. 4 lane + 3 into a staged tile: two boxes of 64 keys, rows of 128 bytes, 128-byte swizzle.
 __device__ __forceinline__ void store_bias4(uint32_t tile, int row, int lane, uint32_t w0, uint32_t w1) {
@@ -1076,25 +1074,25 @@ __device__ __forceinline__ void store_bias4(uint32_t tile, int row, int lane, ui
   asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at), "r"(w0), "r"(w1) : "memory");
 }
 
-// kConvert: the softmax warpgroup that has no stream in items of one makes the bias tiles of the other, from fp32 or from
-// bf16 rows that TMA cannot address, in place of the producer's loads.  Otherwise such a call takes a launch more, and for a
+// kConvert: eight warps in place of the second softmax warpgroup, which has no stream in items of one, make the bias tiles, from fp32 or
+// from bf16 rows that TMA cannot address, in place of the producer's loads.  Otherwise such a call takes a launch more, and for a
 // short call that is a good part of it.  us, bias in place / converted here / in a pass before, 16 heads, fp32: 77 tokens 5.4 / 5.7
-// / 6.8, 512 9.0 / 10.1 / 13.5, 1000 14.4 / 17.3 / 26.6.  A warp takes 32 rows of a tile, a lane four keys of each.  What does
+// / 6.8, 512 9.0 / 10.1 / 13.5, 1000 14.4 / 17.3 / 26.6.  A warp takes 16 rows of a tile, a lane four keys of each.  What does
 // not exist takes the bias of a row or key that does, or anything: of such rows nothing is stored, such keys are at -inf.
 //
-// Rows that start on vectors (bias_wide): 16 rows' loads for the next tile follow directly on their store for this one, so that
-// 32 rows' are out nearly all the time.  The warp is alone on its scheduler beside a softmax warp that streams through its code, so the
+// Rows that start on vectors (bias_wide): 8 rows' loads for the next tile follow directly on their store for this one, so that
+// 16 rows' are out nearly all the time.  The warp is alone on its scheduler beside a softmax warp that streams through its code, so the
 // loop is kept short: with a test for infinities and a second pass behind it 512 tokens took 11.4 us.
 template <bool kF32, int kW>
-__device__ void bias_convert_role(const Ctx& c, int wq, int lane) {
+__device__ void bias_convert_role(const Ctx& c, int cw, int lane) {
   const AttnParams& p = *c.p;
   constexpr int es = kF32 ? 4 : 2;
   using Vec = typename std::conditional<kF32, float4, uint2>::type;
-  const int row0 = wq * 32;
+  const int row0 = cw * 2 * kConvertRows;
   const long long step = p.bias_stride_r * es;
   Vec x[2][kConvertRows];
   auto load = [&](const Item& it, int kt, int half) {
-    const int first = it.qt * kTile + row0, last = min(31, p.Sq - 1 - first);
+    const int first = it.qt * kTile + row0, last = min(2 * kConvertRows - 1, p.Sq - 1 - first);
     if (last < 0) return;
     const char* src = static_cast<const char*>(p.bias_src) + (it.h * p.bias_stride_h + first * p.bias_stride_r + min(kt * kW + 4 * lane, p.Sk - 4)) * es;
 #pragma unroll
@@ -1141,39 +1139,69 @@ __device__ void bias_convert_role(const Ctx& c, int wq, int lane) {
   }
 }
 
-// Rows that start anywhere, for items of one key tile: with more of them a pass of its own over the bias is faster (389 tokens
-// of ragged rows 12.7 us with it, 13.9 so).
-template <typename T, int kW>
-__device__ void bias_convert_ragged_role(const Ctx& c, int wq, int lane) {
+// Rows that start anywhere: a lane takes keys 32 apart, element by element, so that a warp's loads are whole pieces of the row
+// wherever it starts; a row is requested again, for the next tile, as soon as it has been stored, so that a whole tile is under way.
+// Keys that do not exist get 0.  The fetch of instructions is what this kernel is short of, so the code is kept short.  Tried for 1001
+// tokens, us a tile (in place 1.4): aligned vectors of four elements stored in pieces that depend on where the row starts 8, put
+// together by shuffles 3.9, the same with eight warps 2.5, copied through shared memory in a rolled loop 3.3 - 3.9; this 2.2.
+// us, 16 heads, in place / here / pass before: 129 tokens 4.8 / 6.3 / 7.1, 389 bf16 7.7 / 10.5 / 12.0, 1001 fp32 13.5 / 19.5 / 34.4.
+template <bool kF32, int kW>
+__device__ void bias_convert_ragged_role(const Ctx& c, int cw, int lane) {
   const AttnParams& p = *c.p;
-  const int row0 = wq * 32;
-  uint32_t bst = 0, lap = 0;
-  grid_wait_previous();
-#pragma unroll 1
-  for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
-    const Item it = decode_item<false>(p, item);
-#pragma unroll 1
-    for (int kt = 0; kt < p.n_kt; ++kt) {
-      const uint32_t tile = c.smem + p.off_bias + bst * kBiasTileBytes;
-      const int first = it.qt * kTile + row0, last = min(31, p.Sq - 1 - first), key = kt * kW + 4 * lane;
-      const T* src = static_cast<const T*>(p.bias_src) + it.h * p.bias_stride_h + first * p.bias_stride_r + key;
-#pragma unroll 1
-      for (int r0 = 0; r0 < 32; r0 += kConvertRows) {
-        float x[kConvertRows][4];
+  using T = typename std::conditional<kF32, float, uint16_t>::type;
+  constexpr int kRows = 2 * kConvertRows;
+  const int row0 = cw * kRows;
+  T x[kRows][4];
+  struct Rows { const T* src; int last; };      // of this warp in an item, from this lane's first key on
+  auto rows_of = [&](const Item& it) {
+    const int first = it.qt * kTile + row0, last = min(kRows - 1, p.Sq - 1 - first);
+    return Rows{static_cast<const T*>(p.bias_src) + it.h * p.bias_stride_h + (last >= 0 ? first : p.Sq - 1) * p.bias_stride_r + lane, max(last, 0)};
+  };
+  auto load_row = [&](const Rows& w, int kt, int r) {
+    const T* src = w.src + min(r, w.last) * p.bias_stride_r + kt * kW;
+    const int n = p.Sk - kt * kW - lane;
 #pragma unroll
-        for (int r = 0; r < kConvertRows; ++r)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) x[r][e] = load_if(src + min(r0 + r, last) * p.bias_stride_r + e, last >= 0 && key + e < p.Sk ? 1u : 0u);
-        if (r0 == 0 && lap != 0) AF3K_WAIT_WARP(c, BarIdx::bias_empty + bst, (lap - 1) & 1);
-#pragma unroll
-        for (int r = 0; r < kConvertRows; ++r)
-          store_bias4(tile, row0 + r0 + r, lane, staged_pair(x[r][0], x[r][1]), staged_pair(x[r][2], x[r][3]));
-      }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::bias_full + bst));
-      if (++bst == (uint32_t)p.bias_stages) { bst = 0; ++lap; }
+    for (int j = 0; j < 4; ++j) {
+      x[r][j] = T(0);
+      if (32 * j < kW && n > 32 * j) x[r][j] = src[32 * j];
     }
+  };
+  auto clamped = [&](T a, T b) {
+    if constexpr (kF32) return staged_pair(a, b); else return clamped_pair((uint32_t)a | (uint32_t)b << 16);
+  };
+  auto write = [&](uint32_t addr, uint32_t w) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"((uint16_t)w) : "memory"); };
+  int item = blockIdx.x, kt = 0;
+  Rows w = rows_of(decode_item<false>(p, item));     // (the grid has no more blocks than items)
+  grid_wait_previous();
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) load_row(w, 0, r);
+#pragma unroll 1
+  for (uint32_t bst = 0, lap = 0; item < p.n_items;) {
+    const uint32_t tile = c.smem + p.off_bias + bst * kBiasTileBytes + row0 * 128 + (lane & 7) * 2;
+    // the bias MMAs of the stage's tile before must have finished
+    if (lap != 0) AF3K_WAIT_WARP(c, BarIdx::bias_empty + bst, (lap - 1) & 1);
+    if (++kt == p.n_kt) {                    // the tile after this one
+      kt = 0;
+      item += gridDim.x;
+      if (item < p.n_items) w = rows_of(decode_item<false>(p, item));
+    }
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      const uint32_t to = tile + r * 128 + (((lane >> 3) ^ (r & 7)) << 4);
+      const uint32_t w0 = clamped(x[r][0], x[r][1]);
+      write(to, w0);
+      write(to ^ 64u, w0 >> 16);
+      if (kW > 64) {
+        const uint32_t w1 = clamped(x[r][2], x[r][3]);
+        write(to + kBiasTileBytes / 2, w1);
+        if (kW > 96) write((to ^ 64u) + kBiasTileBytes / 2, w1 >> 16);
+      }
+      if (item < p.n_items) load_row(w, kt, r);
+    }
+    fence_proxy_async_smem();    // make the generic-proxy stores visible to the tensor core
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar_addr(c, BarIdx::bias_full + bst));
+    if (++bst == (uint32_t)p.bias_stages) { bst = 0; ++lap; }
   }
 }
 
@@ -1191,7 +1219,7 @@ __device__ void bias_convert_ragged_role(const Ctx& c, int wq, int lane) {
 // kConvert: plans of one stream per item, bf16 q and k; see bias_convert_role.
 // kW: keys per key tile, 32 to 128 (chosen by key_width in the C API).
 template <bool kDebug, bool kTcBias, bool kFp8, bool kGate, bool kMixed, bool kConvert = false, int kW = kTile>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kConvert ? kConvertThreads : kThreads, 1)
 attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                  const __grid_constant__ CUtensorMap tm_bias, const __grid_constant__ CUtensorMap tm_q2,
@@ -1229,7 +1257,7 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
       mbar_init(bar_addr(c, BarIdx::p_ready + i), 4);
     }
     for (int i = 0; i < kMaxBiasStages; ++i) {
-      mbar_init(bar_addr(c, BarIdx::bias_full + i), kConvert ? 4 : 1);
+      mbar_init(bar_addr(c, BarIdx::bias_full + i), kConvert ? kConvertWarps : 1);
       // freed by the bias MMAs' completion (bf16 q/k) or by the eight softmax warps (fp8 q/k)
       mbar_init(bar_addr(c, BarIdx::bias_empty + i), kTcBias ? 1 : 8);
     }
@@ -1277,19 +1305,20 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     } else if (warp == 3) {
       if (p.mask_col) mask_writer_role<kMixed, kW>(c, lane);
     }
+  } else if (kConvert && warp >= 8) {
+    if constexpr (kConvert) {
+      setmaxnreg_dec<kRegsConvert>();
+      if (p.bias_wide) {
+        if (p.bias_f32) bias_convert_role<true, kW>(c, warp - 8, lane);
+        else            bias_convert_role<false, kW>(c, warp - 8, lane);
+      } else {
+        if (p.bias_f32) bias_convert_ragged_role<true, kW>(c, warp - 8, lane);
+        else            bias_convert_ragged_role<false, kW>(c, warp - 8, lane);
+      }
+    }
   } else {
     setmaxnreg_inc<kRegsSoftmax>();
-    if (kConvert && warp >= 8) {
-      if (p.bias_wide) {
-        if (p.bias_f32) bias_convert_role<true, kW>(c, warp & 3, lane);
-        else            bias_convert_role<false, kW>(c, warp & 3, lane);
-      } else {
-        if (p.bias_f32) bias_convert_ragged_role<float, kW>(c, warp & 3, lane);
-        else            bias_convert_ragged_role<uint16_t, kW>(c, warp & 3, lane);
-      }
-    } else {
-      softmax_role<kDebug, kTcBias, kGate, kMixed, !kFp8, kW>(c, (warp - 4) >> 2, warp & 3, lane);
-    }
+    softmax_role<kDebug, kTcBias, kGate, kMixed, !kFp8, kW>(c, (warp - 4) >> 2, warp & 3, lane);
   }
 
   tc_fence_before();

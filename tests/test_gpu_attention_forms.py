@@ -397,3 +397,27 @@ def test_key_tiles_of_every_width(cuda_device, Sk, qk, D):
             assert O.error_stats(out, ref)["max_abs"] <= 6e-2, (B1, Sk)
         else:
             _check(out, ref, (B1, Sk, D))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B1,B2,Sq,Sk,D,pitch,offset,launches", [
+    (1, 16, 129, 129, 32, 129, 0, 1), (1, 16, 140, 161, 24, 161, 1, 1), (1, 16, 250, 225, 48, 231, 2, 1), (2, 16, 200, 257, 32, 257, 3, 1), (1, 6, 400, 389, 64, 389, 5, None),
+    (1, 5, 385, 385, 32, 385, 0, None), (1, 16, 1300, 1300, 24, 1300, 0, 1), (1, 16, 1290, 1301, 16, 1301, 1, None), (1, 20, 1100, 1030, 40, 1032, 4, None)])
+def test_ragged_rows_of_several_key_tiles_converted_by_the_attention_kernel(cuda_device, dtype, B1, B2, Sq, Sk, D, pitch, offset, launches):
+    """Rows that start anywhere, key tiles of 80 to 128 keys, more query tiles than SMs among them: the bits of the pass, whatever stands
+    in front of, between and behind the rows."""
+    g = torch.Generator().manual_seed(Sk)
+    q, k, v = (torch.randn(B1, B2, s, D, generator=g).to(cuda_device, torch.bfloat16) for s in (Sq, Sk, Sk))
+    mask = (torch.rand(B1, Sk, generator=g) >= 0.1).to(cuda_device)
+    mask[:, -1] = True
+    flat = torch.full((B2 * Sq * pitch + 16,), float("nan"), device=cuda_device, dtype=dtype)
+    bias = flat[offset:offset + B2 * Sq * pitch].view(B2, Sq, pitch)[:, :, :Sk]
+    bias.copy_(torch.randn(B2, Sq, Sk, generator=g))
+    bias[torch.rand(bias.shape, generator=g).to(cuda_device) < 0.02] = -float("inf")
+    bias[..., -1] = 1
+    lib = _capi.load()
+    out = A.dot_product_attention_cpp(q, k, v, mask, bias)
+    assert launches is None or lib.af3k_last_launch_count() == launches
+    staged = dot_product_attention(q, k, v, mask, bias, cache_bias=False, check_status=True)
+    assert lib.af3k_last_launch_count() == 2 and not out.isnan().any()
+    assert torch.equal(out, staged)
