@@ -37,6 +37,7 @@ EXPORTED_SYMBOLS = (
     "af3k_debug_set_dump",
     "af3k_selftest_wait_timeout",
     "af3k_pair_bias",
+    "af3k_cast",
     "af3k_sigmoid_gate",
     "af3k_qkvg_projection",
     "af3k_grid_front",
@@ -154,6 +155,8 @@ def load() -> ctypes.CDLL:
     lib.af3k_pair_front.restype = ctypes.c_int
     lib.af3k_pair_front.argtypes = [vp, vp, vp, ctypes.c_float, vp, i64, vp, i64, i64, i64, ctypes.c_float, vp, i64,
                                     vp, vp, vp, vp, vp, vp]
+    lib.af3k_cast.restype = ctypes.c_int
+    lib.af3k_cast.argtypes = [ctypes.POINTER(vp), ctypes.POINTER(vp), ctypes.POINTER(i64), ctypes.c_int32, ctypes.c_int32, vp]
     lib.af3k_sigmoid_gate.restype = ctypes.c_int
     lib.af3k_sigmoid_gate.argtypes = [vp, vp, vp, i64, vp]
     _lib = lib

@@ -1151,6 +1151,36 @@ int af3k_pair_front(const void* pair, const float* gamma, const float* beta, flo
                          status_dev, stream_v);
 }
 
+int af3k_cast(const void* const* src, void* const* dst, const int64_t* n, int32_t count, int32_t to_dtype, void* stream_v) {
+  t_last_launches = 0;
+  if (to_dtype != AF3K_BF16 && to_dtype != AF3K_F32) return AF3K_ERR_BAD_DTYPE;
+  if (count < 0 || count > kMaxCasts) return AF3K_ERR_BAD_SHAPE;
+  if (count > 0 && (!src || !dst || !n)) return AF3K_ERR_NULL_POINTER;
+  CastParams p{};
+  long long most = 0;
+  for (int i = 0; i < count; ++i) {
+    if (n[i] < 0) return AF3K_ERR_BAD_SHAPE;
+    if (n[i] > 0 && (!src[i] || !dst[i])) return AF3K_ERR_NULL_POINTER;
+    if (!aligned16(src[i]) || !aligned16(dst[i])) return AF3K_ERR_BAD_ALIGNMENT;
+    p.src[i] = src[i]; p.dst[i] = dst[i]; p.n[i] = n[i];
+    if (n[i] > most) most = n[i];
+  }
+  if (most == 0) return AF3K_OK;
+  DeviceInfo* dev = nullptr;
+  int rc = device_info(&dev);
+  if (rc != AF3K_OK) return rc;
+  long long blocks = (most / 8 + kCastThreads) / kCastThreads;
+  if (blocks > dev->sm_count * 8) blocks = dev->sm_count * 8;
+  const dim3 grid((unsigned)blocks, (unsigned)count);
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
+  if (to_dtype == AF3K_BF16) launch_overlapped(cast_kernel<true>, grid, kCastThreads, 0, stream, true, p);
+  else                       launch_overlapped(cast_kernel<false>, grid, kCastThreads, 0, stream, true, p);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail("launch cast_kernel", e);
+  t_last_launches = 1;
+  return AF3K_OK;
+}
+
 int af3k_sigmoid_gate(const void* weighted, const void* gate, void* out, int64_t n, void* stream_v) {
   t_last_launches = 0;
   if (n < 0 || (n & 7) != 0) return AF3K_ERR_BAD_SHAPE;

@@ -37,6 +37,7 @@ struct Library {
   decltype(&af3k_grid_front_weights) grid_front = nullptr;
   decltype(&af3k_grid_out_weights) grid_out = nullptr;
   decltype(&af3k_sigmoid_gate) sigmoid_gate = nullptr;
+  decltype(&af3k_cast) cast = nullptr;
   decltype(&af3k_grid_pack) grid_pack = nullptr;
   decltype(&af3k_token_pack) token_pack = nullptr;
   decltype(&af3k_token_projection_weights) token_projection = nullptr;
@@ -59,6 +60,7 @@ void bind_library(const std::string& path) {
   AF3K_BIND(grid_front, af3k_grid_front_weights);
   AF3K_BIND(grid_out, af3k_grid_out_weights);
   AF3K_BIND(sigmoid_gate, af3k_sigmoid_gate);
+  AF3K_BIND(cast, af3k_cast);
   AF3K_BIND(grid_pack, af3k_grid_pack);
   AF3K_BIND(token_pack, af3k_token_pack);
   AF3K_BIND(token_projection, af3k_token_projection_weights);
@@ -88,6 +90,38 @@ Tensor status_buffer(int64_t device) {
   Tensor& t = bufs->at(device);
   if (!t.defined()) t = at::zeros({4}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
   return t;
+}
+
+// ------------------------------------------------------------------ conversions
+// Each of up to three tensors as bf16: those that are fp32, contiguous and aligned in one launch of the library's, others by torch.
+void to_bf16(std::initializer_list<Tensor*> tensors, cudaStream_t stream) {
+  const void* src[3];
+  void* dst[3];
+  int64_t n[3];
+  int32_t count = 0;
+  std::vector<std::pair<Tensor*, Tensor>> made;
+  for (Tensor* t : tensors) {
+    if (t->scalar_type() == at::kBFloat16) continue;
+    if (t->scalar_type() != at::kFloat || !t->is_contiguous() || !t->is_cuda() || reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 != 0) {
+      *t = t->to(at::kBFloat16);
+      continue;
+    }
+    Tensor b = new_tensor(t->sizes(), at::kBFloat16, t->device());
+    src[count] = t->data_ptr(); dst[count] = b.data_ptr(); n[count++] = t->numel();
+    made.emplace_back(t, std::move(b));
+  }
+  if (count != 0) check(g_lib.cast(src, dst, n, count, AF3K_BF16, stream));
+  for (auto& [t, b] : made) *t = std::move(b);
+}
+
+// A contiguous bf16 result as fp32.
+Tensor to_float(const Tensor& t, cudaStream_t stream) {
+  Tensor f = new_tensor(t.sizes(), at::kFloat, t.device());
+  const void* src = t.data_ptr();
+  void* dst = f.data_ptr();
+  const int64_t n = t.numel();
+  check(g_lib.cast(&src, &dst, &n, 1, AF3K_F32, stream));
+  return f;
 }
 
 // ------------------------------------------------------------------ staged biases
@@ -231,12 +265,11 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
       // the reference has an fp32 instantiation (src/csrc/dot_product_attention.cpp:554-558); here fp32
       // callers get the bf16 kernel (operands rounded once) and an fp32 result
       if (out_in) value_error("`out` must be omitted with fp32 q (the result is converted from the kernel's bf16 output)");
-      q = q.to(at::kBFloat16);
       f32_result = true;
     }
-    if (q.scalar_type() != at::kBFloat16) type_error(std::string("q must be bfloat16, float32 or float8_e4m3fn, got ") + c10::toString(q.scalar_type()));
+    if (q.scalar_type() != at::kBFloat16 && !f32_result) type_error(std::string("q must be bfloat16, float32 or float8_e4m3fn, got ") + c10::toString(q.scalar_type()));
     if ((q_scale_in || k_scale_in) && !f32_result) type_error("q_scale / k_scale are only valid with fp8 q and k");
-    if (k.scalar_type() != at::kBFloat16) k = k.to(at::kBFloat16);
+    to_bf16({&q, &k, &v}, c10::cuda::getCurrentCUDAStream(dev.index()));
   }
   if (v.scalar_type() != at::kBFloat16) v = v.to(at::kBFloat16);
   const float scale = softmax_scale ? (float)*softmax_scale : (float)(1.0 / std::sqrt((double)D));
@@ -302,7 +335,7 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
     const int rc = g_lib.attention_convert(&d, q.data_ptr(), k.data_ptr(), v.data_ptr(), bias.data_ptr(), mask_data, out.data_ptr(), status_data, stream);
     if (rc != AF3K_ERR_WORKSPACE) {
       check(rc);
-      return f32_result ? out.to(at::kFloat) : out;
+      return f32_result ? to_float(out, stream) : out;
     }
   }
   Tensor ws;
@@ -313,7 +346,7 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
   check(g_lib.attention(&d, q.data_ptr(), k.data_ptr(), v.data_ptr(), bias.data_ptr(), mask_data, out.data_ptr(), fp8 ? q_scale.data_ptr<float>() : nullptr, fp8 ? k_scale.data_ptr<float>() : nullptr,
                         ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? (size_t)ws.numel() : 0,
                         status_data, stream));
-  return f32_result ? out.to(at::kFloat) : out;
+  return f32_result ? to_float(out, stream) : out;
 }
 
 // ------------------------------------------------------------------ block parameters
@@ -507,7 +540,8 @@ Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, con
   const bool with_tokens = !in_place_w && x_in.scalar_type() == at::kFloat && x_in.is_contiguous() && reinterpret_cast<uintptr_t>(x_in.data_ptr()) % 16 == 0;
   Tensor packed, x = x_in;
   if (!with_tokens) {
-    x = x_in.to(at::kBFloat16).contiguous();
+    to_bf16({&x}, stream);
+    x = x.contiguous();
     if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0) x = x.clone();
   }
   if (!in_place_w) {
@@ -548,6 +582,7 @@ Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, con
     rc = call();
   }
   check(rc);
+  if (x_in.scalar_type() == at::kFloat) return to_float(out, stream);
   return x_in.scalar_type() == at::kBFloat16 ? out : out.to(x_in.scalar_type());
 }
 

@@ -326,6 +326,11 @@ int af3k_grid_pack(const af3k_matrix* w5, const af3k_matrix* bias_w, const void*
  * x, x_bf16 16-byte aligned; M 0: no tokens. */
 int af3k_token_pack(const af3k_matrix* w4, int64_t C, void* w4_bf16, const float* x, int64_t M, void* x_bf16, void* stream);
 
+/* Up to three contiguous arrays of n[i] elements, 16-byte aligned, fp32 -> bf16 (to_dtype AF3K_BF16, rounded to nearest) or
+ * bf16 -> fp32 (AF3K_F32) in one launch: operands and results of fp32 callers (the reference's fp32 instantiation,
+ * src/csrc/dot_product_attention.cpp:554-558). */
+int af3k_cast(const void* const* src, void* const* dst, const int64_t* n, int32_t count, int32_t to_dtype, void* stream);
+
 /* out = weighted * sigmoid(gate), elementwise over n bf16 elements (n a multiple of 8; all three
  * pointers 16-byte aligned; out may be weighted).  Stands in for the SigmoidFwdTPP + MulTPP pair
  * behind the attention core in the reference's fused blocks

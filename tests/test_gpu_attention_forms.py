@@ -421,3 +421,42 @@ def test_ragged_rows_of_several_key_tiles_converted_by_the_attention_kernel(cuda
     staged = dot_product_attention(q, k, v, mask, bias, cache_bias=False, check_status=True)
     assert lib.af3k_last_launch_count() == 2 and not out.isnan().any()
     assert torch.equal(out, staged)
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 2047, 2048, 300001])
+def test_conversions_in_one_launch(cuda_device, n):
+    """Three arrays of different lengths to bf16, one back: torch's roundings, infinities and NaN, nothing written behind the ends."""
+    import ctypes
+    lib = _capi.load()
+    g = torch.Generator().manual_seed(n)
+    lengths = [n, max(n // 3, 1), 5]
+    src = [(torch.randn(m, generator=g) * 10.0 ** torch.randint(-45, 39, (m,), generator=g)).to(cuda_device) for m in lengths]
+    src[0][0] = float("nan")
+    src[2][:2] = torch.tensor([float("inf"), -3.4e38])
+    dst = [torch.full((m + 8,), 7.0, device=cuda_device, dtype=torch.bfloat16) for m in lengths]
+    stream = torch.cuda.current_stream().cuda_stream
+    pointers = lambda ts: (ctypes.c_void_p * len(ts))(*(t.data_ptr() for t in ts))
+    assert lib.af3k_cast(pointers(src), pointers(dst), (ctypes.c_int64 * 3)(*lengths), 3, _capi.AF3K_BF16, stream) == 0
+    assert lib.af3k_last_launch_count() == 1
+    for a, b, m in zip(src, dst, lengths):
+        assert torch.equal(b[:m].nan_to_num(5.0), a.to(torch.bfloat16).nan_to_num(5.0)) and torch.equal(b[:m].isnan(), a.isnan()) and (b[m:] == 7).all()
+    back = torch.full((n + 8,), 7.0, device=cuda_device)
+    assert lib.af3k_cast(pointers(dst[:1]), pointers([back]), (ctypes.c_int64 * 1)(n), 1, _capi.AF3K_F32, stream) == 0
+    assert torch.equal(back[:n].nan_to_num(5.0), dst[0][:n].float().nan_to_num(5.0)) and (back[n:] == 7).all()
+    assert lib.af3k_cast(pointers([src[0][1:]]) if n > 1 else pointers(src[:1]), pointers(dst[:1]), (ctypes.c_int64 * 1)(n - 1), 1, _capi.AF3K_BF16, stream) == (4 if n > 1 else 0)
+
+
+@pytest.mark.parametrize("form", ["contiguous", "permuted", "offset", "mixed"])
+def test_fp32_operands_give_the_bits_of_their_bf16_forms(cuda_device, form):
+    g = torch.Generator().manual_seed(4)
+    B1, B2, S, D = 2, 4, 150, 24
+    make = lambda: torch.randn(B1, S, B2, D, generator=g).to(cuda_device).permute(0, 2, 1, 3) if form == "permuted" else torch.randn(B1, B2, S, D, generator=g).to(cuda_device)
+    q, k, v = make(), make(), make()
+    if form == "offset":
+        q = torch.cat([q.flatten(), q.flatten()[:1]])[1:].view(B1, B2, S, D)
+    if form == "mixed":
+        k, v = k.to(torch.bfloat16), v.double()
+    bias = torch.randn(B2, S, S, generator=g).to(cuda_device)
+    out = A.dot_product_attention_cpp(q, k, v, None, bias)
+    assert out.dtype == torch.float32
+    assert torch.equal(out, A.dot_product_attention_cpp(*(t.to(torch.bfloat16) for t in (q, k, v)), None, bias).float())
