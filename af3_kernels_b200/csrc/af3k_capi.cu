@@ -139,7 +139,7 @@ int device_info(DeviceInfo** out) {
         {(const void*)grid_front_kernel<64, float, true>, FrontTile<64, float>::kSmem}, {(const void*)grid_front_kernel<64, __nv_bfloat16, false>, FrontTile<64, __nv_bfloat16>::kSmem},
         {(const void*)grid_out_kernel<128, __nv_bfloat16>, OutTile<128>::kSmem}, {(const void*)grid_out_kernel<128, float>, OutTile<128>::kSmem},
         {(const void*)grid_out_kernel<64, __nv_bfloat16>, OutTile<64>::kSmem}, {(const void*)grid_out_kernel<64, float>, OutTile<64>::kSmem},
-        {(const void*)token_proj_kernel<64>, TokTile<64>::kSmem}, {(const void*)token_proj_kernel<128>, TokTile<128>::kSmem},
+        {(const void*)token_proj_kernel<64>, TokTile<64>::kSmem}, {(const void*)token_proj_kernel<128>, TokTile<128>::kSmem}, {(const void*)token_proj_kernel<256>, TokTile<256>::kSmem},
     };
     for (const auto& k : gemm_kernels)
       if ((e = cudaFuncSetAttribute(k.first, attr, (int)k.second)) != cudaSuccess)
@@ -1093,7 +1093,12 @@ int af3k_token_projection_weights(const void* x, const af3k_matrix* w4, const vo
   int rc = device_info(&dev);
   if (rc != AF3K_OK) return rc;
   const int64_t m_tiles = (M + 127) / 128;
-  const int kn = m_tiles * 4 * ((C + 127) / 128) >= dev->sm_count * 3 / 4 ? 128 : 64;   // enough tiles of 128 columns to fill the SMs?
+  // Columns of a tile: the narrowest that takes fewest rounds of one CTA per SM (64 with some SMs to spare).  Single block, us on the
+  // device, 64 / 128 / 256: 384 channels 256 tokens 10.5 / 11.0 / 12.4, 1024 21.9 / 20.5 / 21.0, 2048 44.5 / 41.3 / 39.5; 768 channels
+  // 384 tokens 15.9 / 15.1 / 17.0, 512 20.1 / 17.2 / 18.4, 1536 49.4 / 41.8 / 38.3.
+  const auto tiles = [&](int64_t n) { return m_tiles * 4 * ((C + n - 1) / n); };
+  const auto rounds = [&](int64_t n) { return (tiles(n) + dev->sm_count - 1) / dev->sm_count; };
+  const int kn = tiles(64) <= dev->sm_count * 3 / 4 ? 64 : (rounds(128) <= rounds(256) ? 128 : 256);
   const int64_t tiles_n = (C + kn - 1) / kn;
   if (4 * tiles_n > 65535) return AF3K_ERR_BAD_SHAPE;
   auto enc = tensor_map_encoder();
@@ -1121,7 +1126,8 @@ int af3k_token_projection_weights(const void* x, const af3k_matrix* w4, const vo
   p.out = static_cast<__nv_bfloat16*>(out); p.status = status_dev; p.wait_limit = wait_limit_cycles();
   const dim3 grid((unsigned)m_tiles, (unsigned)(4 * tiles_n));
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
-  if (kn == 128) launch_overlapped(token_proj_kernel<128>, grid, kTokThreads, TokTile<128>::kSmem, stream, true, p, tm_x, maps);
+  if (kn == 256) launch_overlapped(token_proj_kernel<256>, grid, kTokThreads, TokTile<256>::kSmem, stream, true, p, tm_x, maps);
+  else if (kn == 128) launch_overlapped(token_proj_kernel<128>, grid, kTokThreads, TokTile<128>::kSmem, stream, true, p, tm_x, maps);
   else           launch_overlapped(token_proj_kernel<64>, grid, kTokThreads, TokTile<64>::kSmem, stream, true, p, tm_x, maps);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail("launch token_proj_kernel", e);

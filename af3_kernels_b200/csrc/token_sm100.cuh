@@ -10,7 +10,8 @@
 // (src/csrc/dot_product_attention.cpp:425-480).  M is a token count (tens to a few thousand), C 384 or 768
 // in practice: a few GFLOP, so what bounds it is latency - one tile of 128 rows x kN columns per CTA, the
 // K blocks of 64 channels streamed through six stages that hold all of K at C = 384, one warp each for the
-// TMA and the MMAs, four for the epilogue.  kN is 64 where tiles of 128 columns would leave SMs idle.
+// TMA and the MMAs, four for the epilogue.  kN is 64, 128 or 256, so that
+// few rounds of CTAs do and few SMs are idle.
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -21,10 +22,11 @@
 
 namespace af3k {
 
-constexpr int kTokThreads = 192, kTokStages = 6;
+constexpr int kTokThreads = 192;
 template <int kN> struct TokTile {
+  static constexpr int kStages = kN == 256 ? 4 : 6;
   static constexpr uint32_t kA = 128 * 128, kB = kN * 128, kStage = kA + kB;
-  static constexpr uint32_t off_bar = kTokStages * kStage, off_bias = off_bar + 128, kSmem = off_bias + kN * 4;   // off_bias: query bias, fp32
+  static constexpr uint32_t off_bar = kStages * kStage, off_bias = off_bar + 128, kSmem = off_bias + kN * 4;   // off_bias: query bias, fp32
 };
 
 struct TokMaps { CUtensorMap w[4]; };
@@ -46,7 +48,7 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
                   const __grid_constant__ TokMaps maps) {
   using Tile = TokTile<kN>;
   extern __shared__ __align__(1024) uint8_t tok_smem[];
-  const uint32_t smem = smem_u32(tok_smem), bars = smem + Tile::off_bar;   // full [6], empty [6], acc
+  const uint32_t smem = smem_u32(tok_smem), bars = smem + Tile::off_bar;   // full [kStages], empty [kStages], acc
   volatile uint32_t* slot = reinterpret_cast<volatile uint32_t*>(tok_smem + Tile::off_bar + 112);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tok_smem + Tile::off_bar + 116);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -65,7 +67,7 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
     *abort_flag = 0;
     prefetch_tensormap(&tm_x);
     prefetch_tensormap(tm_w);
-    for (int i = 0; i < 2 * kTokStages + 1; ++i) mbar_init(bars + 8u * i, 1);
+    for (int i = 0; i < 2 * Tile::kStages + 1; ++i) mbar_init(bars + 8u * i, 1);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -80,9 +82,9 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
   if (warp == 0) {
     if (lane == 0) {
       for (int kb = 0; kb < kblocks; ++kb) {
-        const int st = kb % kTokStages;
-        if (kb >= kTokStages && !mbar_wait_bounded(bars + 8u * (kTokStages + st), ((kb / kTokStages) - 1) & 1, p.wait_limit, const_cast<volatile int*>(abort_flag))) {
-          timeout(kTokStages + st);
+        const int st = kb % Tile::kStages;
+        if (kb >= Tile::kStages && !mbar_wait_bounded(bars + 8u * (Tile::kStages + st), ((kb / Tile::kStages) - 1) & 1, p.wait_limit, const_cast<volatile int*>(abort_flag))) {
+          timeout(Tile::kStages + st);
           break;
         }
         const uint32_t full = bars + 8u * st, dst = smem + st * Tile::kStage;
@@ -109,8 +111,8 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
     const uint32_t b_step = mn ? (16 * 128) >> 4 : 2;
     bool ok = true;
     for (int kb = 0; kb < kblocks && ok; ++kb) {
-      const int st = kb % kTokStages;
-      ok = mbar_wait_bounded(bars + 8u * st, (kb / kTokStages) & 1, p.wait_limit, const_cast<volatile int*>(abort_flag));
+      const int st = kb % Tile::kStages;
+      ok = mbar_wait_bounded(bars + 8u * st, (kb / Tile::kStages) & 1, p.wait_limit, const_cast<volatile int*>(abort_flag));
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) { timeout(st); break; }
       tc_fence_after();
@@ -118,8 +120,8 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
         const uint32_t a = lo + ((st * Tile::kStage) >> 4), b = b_lo + ((st * Tile::kStage + Tile::kA) >> 4);
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) mma_ss_f16(tmem, a + 2 * ks, hi, b + b_step * ks, b_hi, idesc, kb + ks > 0 ? 1u : 0u);
-        tc_commit(bars + 8u * (kTokStages + st));
-        if (kb == kblocks - 1) tc_commit(bars + 8u * (2 * kTokStages));
+        tc_commit(bars + 8u * (Tile::kStages + st));
+        if (kb == kblocks - 1) tc_commit(bars + 8u * (2 * Tile::kStages));
       }
       __syncwarp();
     }
@@ -139,7 +141,7 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");      // the four epilogue warps
     }
-    const bool ok = mbar_wait_bounded(bars + 8u * (2 * kTokStages), 0, p.wait_limit, const_cast<volatile int*>(abort_flag));
+    const bool ok = mbar_wait_bounded(bars + 8u * (2 * Tile::kStages), 0, p.wait_limit, const_cast<volatile int*>(abort_flag));
     if (__all_sync(0xffffffffu, ok)) {
       tc_fence_after();
       const uint32_t t_base = tmem + ((uint32_t)(quarter * 32) << 16);
@@ -188,7 +190,7 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
         __syncwarp();      // the patch is rewritten by the next 64 columns
       }
     } else {
-      timeout(2 * kTokStages);
+      timeout(2 * Tile::kStages);
     }
   }
 

@@ -675,3 +675,9 @@ def test_single_block_and_operator_straight_from_python(cuda_device, dtype):
             A.self_attention_cpp(x, bad, bias, ws[0], qb, *ws[1:], H)
     with pytest.raises(ValueError):
         A.dot_product_attention_cpp(q, q, q, mask, bias, False, 0)
+
+
+@pytest.mark.parametrize("N,C,H", [(900, 704, 11), (1030, 520, 13)])
+def test_projection_tiles_of_256_columns(cuda_device, N, C, H):
+    """Where tiles of 128 columns would take two rounds of CTAs; matrices that end inside such a tile."""
+    test_self_block_reads_weights_of_any_layout(cuda_device, N, C, H)
