@@ -61,7 +61,7 @@ def dot_product_attention_cpp(
     """Same positional signature as the reference (src/af3_kernels/__init__.py:31-40).
 
     ``use_flash_attention``, ``BLK_SZ`` and ``FLASH_SZ`` are accepted and checked but do not
-    select code: the CUDA kernel always runs an online softmax over 128-key tiles.  Unlike the
+    select code: the CUDA kernel always runs an online softmax over key tiles of up to 128.  Unlike the
     reference the call never writes to ``q`` and a 1-D mask broadcasts over the batch.
     ``q_scale`` / ``k_scale`` (keyword-only) enable float8_e4m3fn q and k.  Nothing is kept between calls: a bias that is
     converted (fp32, rows that are not 16-byte multiples, fp8 q and k) is converted in each; ``stage_bias`` and

@@ -9,7 +9,8 @@
 //   warp 2      TMEM allocator, then tcgen05.mma issuer for O += P V (TMEM x smem -> TMEM)
 //   warp 3      key-mask writer (see below)
 //   warps 4-7   softmax warpgroup 0 (owns S / P buffer 0 and the even streams of a work item)
-//   warps 8-11  softmax warpgroup 1 (owns S / P buffer 1 and the odd streams)
+//   warps 8-11  softmax warpgroup 1 (owns S / P buffer 1 and the odd streams); or, where items have one stream and the bias
+//               is converted here, warps 8-15 that make the bias tiles
 //
 // A work item is (head, 128-query tile, group of G pair rows).  The G "streams" of an item use
 // the same bias tiles, so one staged bias tile serves G logits tiles; each stream has its own

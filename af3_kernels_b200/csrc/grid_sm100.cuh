@@ -26,8 +26,8 @@
 // What bounds them is HBM: per row of a bf16 pair with C = 128 the front reads 256 bytes and writes 1 024
 // (+ 2 Hb), the output pass reads 512 and writes 256.  The normalised pair and the gated product never
 // reach HBM.  The pair bias is part of the GEMM: as arithmetic of the row producers (32 FMAs and five
-// shuffles per row piece) it made their chain the limit, 185 us against 148 (768 x 768 x 128 bf16; 116 us at
-// the copy rate).  The output pass takes 89 us there (69 at the copy rate).
+// shuffles per row piece) it made their chain the limit, 185 us against 148 (768 x 768 x 128 bf16; a bare kernel
+// that reads and writes as much takes 144).  The output pass takes 86 us there (69 at the copy rate).
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
