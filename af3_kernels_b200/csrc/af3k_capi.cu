@@ -2,6 +2,7 @@
 // TMA descriptor encoding and kernel launches.  No torch types cross this boundary.
 #include "../../include/af3k.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstring>
@@ -419,12 +420,14 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
 
 // Whether the attention kernel is to convert the bias itself (then *plan is one that can: one query tile of one pair row per item).
 // Estimates in us, for key tiles of 128: the pass 1.7 and 5 TB/s; a tile of a pair of streams 1.6; a lone tile whose bias is converted
-// 1.65 (rows on vectors; no slower than in place) or, where rows start anywhere, 2.2, which is 0.75 more than in place.
+// 1.65 (rows on vectors) or, where rows start anywhere, 2.2, which is 0.75 more than in place, and 1.2 for each such item.
 // Measured, us, pass before -> here: 16 heads, rows anywhere: 129 tokens 7.1 -> 6.3, 389 bf16 12.0 -> 10.5, 1001 bf16 26.8 -> 19.5,
 // fp32 34.4 -> 19.5; 5 heads of 385 9.5 (here 10.4).  In place of pairs of query tiles: 1300 tokens bf16 43.7 -> 38.1, fp32 53.8 -> 43.7;
-// 1536 fp32 61 -> 46; 2047 bf16 89 -> 79, fp32 118 -> 79; 2048 fp32 96 -> 63; 1301 bf16 43.9 and 1537 bf16 57.4 keep the pass.
+// 1536 fp32 61 -> 46; 2047 bf16 89 -> 79, fp32 118 -> 79; 2048 fp32 96 -> 63; 1301 bf16 43.9 and 1537 bf16 57.4 keep the pass.  In place of
+// several pair rows, us a call with its host: 45 rows, 4 heads 8.7 -> 7.1, 62 rows 8.7 -> 7.6; 75 rows 8.8 (here 9.5), 128 fp32 10.0 (13.2).
 // (Calls of a few items, bound by the host either way, keep it too.)
 constexpr int kFewItems = 16;
+constexpr double kHostOne = 6, kHostTwo = 8.7;     // a call's host time with one launch and with two: what bounds the short ones
 bool convert_in_kernel(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, bool wide) {
   const AttnParams& p = plan->p;
   const double es = d.bias_dtype == AF3K_F32 ? 4 : 2, elements = (double)d.B2 * d.Sq * d.Sk, width = p.kw / (double)kTile;
@@ -436,8 +439,9 @@ bool convert_in_kernel(const af3k_attention_desc& d, const DeviceInfo& dev, Plan
   Plan lone;
   if (d.rows_per_item > 1 || make_plan(d, dev, &lone, true, true) != AF3K_OK || lone.p.mixed) return false;
   const int rounds = (lone.p.n_items + lone.grid - 1) / lone.grid;
-  const double here = rounds * (lone.p.n_kt * (wide ? 1.65 : 2.2) * width + 1.3), reads = d.B1 * elements * es / 5e6;   // each pair row reads the whole bias
-  if ((here > reads ? here : reads) >= 0.95 * (plan->cost * 1.6 * width + pass)) return false;
+  const double reads = d.B1 * elements * es / 5e6;      // each pair row reads the whole bias
+  const double here = std::max(rounds * (lone.p.n_kt * (wide ? 1.65 : 2.2) * width + 1.2), reads), there = plan->cost * 1.6 * width + pass;
+  if (std::max(here + 1.5, kHostOne) >= 0.98 * std::max(there + 1.5, kHostTwo)) return false;
   *plan = lone;
   return true;
 }
