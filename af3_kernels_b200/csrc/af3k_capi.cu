@@ -423,7 +423,8 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
 // 1.65 (rows on vectors) or, where rows start anywhere, 2.2, which is 0.75 more than in place, and 1.2 for each such item.
 // Measured, us, pass before -> here: 16 heads, rows anywhere: 129 tokens 7.1 -> 6.3, 389 bf16 12.0 -> 10.5, 1001 bf16 26.8 -> 19.5,
 // fp32 34.4 -> 19.5; 5 heads of 385 9.5 (here 10.4).  In place of pairs of query tiles: 1300 tokens bf16 43.7 -> 38.1, fp32 53.8 -> 43.7;
-// 1536 fp32 61 -> 46; 2047 bf16 89 -> 79, fp32 118 -> 79; 2048 fp32 96 -> 63; 1301 bf16 43.9 and 1537 bf16 57.4 keep the pass.  In place of
+// 1536 fp32 61 -> 46; 2047 bf16 89 -> 79, fp32 118 -> 79; 2048 fp32 96 -> 63; 1301 fp32 54.1 -> 52.2; 1301 bf16 43.9 keeps the pass.  (fp32 in rows anywhere: 129, 1001
+// and 2047 tokens with a slower pass, 1301 with today's.)  In place of
 // several pair rows, us a call with its host: 45 rows, 4 heads 8.7 -> 7.1, 62 rows 8.7 -> 7.6; 75 rows 8.8 (here 9.5), 128 fp32 10.0 (13.2).
 // (Calls of a few items, bound by the host either way, keep it too.)
 constexpr int kFewItems = 16;
@@ -567,15 +568,18 @@ namespace {
 int launch_bias_staging(const af3k_attention_desc& d, const DeviceInfo& dev, const void* bias, const float* sq,
                         const float* sk, void* staged, cudaStream_t stream) {
   const int64_t pitch = staged_bias_pitch(d.Sk);
-  const long long total = (long long)d.B2 * d.Sq * (pitch / 8);
+  const bool f32 = d.bias_dtype == AF3K_F32;
+  const bool pieces = f32 && ((reinterpret_cast<uintptr_t>(bias) | (uintptr_t)d.bias_stride[0] * 4 | (uintptr_t)d.bias_stride[1] * 4) & 15u) != 0;
+  const long long total = (long long)d.B2 * d.Sq * (pieces ? (pitch + 255) / 256 * 32 : pitch / 8);      // threads
   long long blocks = (total + kBiasThreads - 1) / kBiasThreads;
   if (blocks > dev.sm_count * 8) blocks = dev.sm_count * 8;
   const auto launch = [&](auto kernel, auto* src) {
     launch_overlapped(kernel, dim3((unsigned)blocks), kBiasThreads, 0, stream, d.max_ctas <= 0, src, static_cast<__nv_bfloat16*>(staged), (int)d.B2,
                       (int)d.Sq, (int)d.Sk, (long long)d.bias_stride[0], (long long)d.bias_stride[1], (int)pitch, sq, sk, d.softmax_scale);
   };
-  if (d.bias_dtype == AF3K_F32) launch(bias_to_bf16_kernel<float>, static_cast<const float*>(bias));
-  else                          launch(bias_to_bf16_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(bias));
+  if (!f32)        launch(bias_to_bf16_kernel<__nv_bfloat16, false>, static_cast<const __nv_bfloat16*>(bias));
+  else if (pieces) launch(bias_to_bf16_kernel<float, true>, static_cast<const float*>(bias));
+  else             launch(bias_to_bf16_kernel<float, false>, static_cast<const float*>(bias));
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? AF3K_OK : cuda_fail("launch bias_to_bf16_kernel", e);
 }

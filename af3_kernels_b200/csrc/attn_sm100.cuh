@@ -1381,29 +1381,50 @@ __global__ void __launch_bounds__(kCastThreads) cast_kernel(const __grid_constan
 // and the softmax threads apply that scale to the sum.
 // (staged_pair says what becomes of values that bf16 cannot hold.)
 // One thread converts eight columns, two 16-byte loads where every row starts on a 16-byte boundary (else one by one) and one
-// 16-byte store, as many blocks as stay resident: it is bound by memory, and a call that converts pays it in full.
-// Two columns a thread, with two 64-bit divisions for each pair, against this, us: 16 heads of 512 x 512 fp32 11.3 -> 4.9 (5.2
+// 16-byte store, as many blocks as stay resident: it is bound by memory, and a call that converts pays it in full.  fp32 rows that
+// start anywhere (kPieces): a warp converts 256 columns of a row, a lane two next to one another in every 64, so that its loads are
+// whole pieces of the row and its stores whole lines (a thread's eight columns one by one touch every sector eight times).
+// Two columns a thread, with two 64-bit divisions for each pair, against eight, us: 16 heads of 512 x 512 fp32 11.3 -> 4.9 (5.2
 // TB/s), of 1536 x 1536 76.2 -> 35.2 (6.4 TB/s), 4 heads of 768 x 768 6.9 -> 3.0, of 2048 x 2048 bf16 with scales 40.9 -> 14.0.
+// Rows anywhere, eight columns one by one -> two in 64, 16 heads: fp32 389 tokens 4.4 -> 3.5, 1001 19.8 -> 13.4, 1537 43.1 -> 36.5, 2047 76.1
+// -> 62.4; but bf16 389 3.2 -> 3.8, 1301 23.1 -> 25.0, so that stays as it was.
 constexpr int kBiasThreads = 256;
-template <typename T>
+template <typename T, bool kPieces>
 __global__ void __launch_bounds__(kBiasThreads, 8)
 bias_to_bf16_kernel(const T* src, __nv_bfloat16* dst, int B2, int Sq, int Sk, long long src_stride_h, long long src_stride_r, int pitch,
                     const float* q_scale, const float* k_scale, float softmax_scale) {
   // (no __restrict__: it would allow loads of the read-only kind, which need not stay behind the wait)
   grid_wait_previous();
   grid_release_next();
-  const uint32_t chunks = (uint32_t)pitch / 8;
+  // a thread's eight columns, or a warp's 256
+  constexpr int kColumns = kPieces ? 256 : 8;
+  const uint32_t chunks = (uint32_t)(pitch + kColumns - 1) / kColumns;
   const long long total = (long long)B2 * Sq * chunks;
+  const int lane = threadIdx.x & 31, threads = kPieces ? kBiasThreads / 32 : kBiasThreads;
   const bool wide = ((reinterpret_cast<uintptr_t>(src) | (uintptr_t)(src_stride_h * sizeof(T)) | (uintptr_t)(src_stride_r * sizeof(T))) & 15u) == 0;
-  for (long long i = (long long)blockIdx.x * kBiasThreads + threadIdx.x; i < total; i += (long long)gridDim.x * kBiasThreads) {
+  for (long long i = (long long)blockIdx.x * threads + (kPieces ? threadIdx.x >> 5 : threadIdx.x); i < total; i += (long long)gridDim.x * threads) {
     long long t;             // row among all heads'
     if (total <= 0x7fffffff) t = (uint32_t)i / chunks; else t = i / chunks;
-    const int col = (int)(i - t * chunks) * 8;
+    const int col = (int)(i - t * chunks) * kColumns;
     int h, r;
     if (t <= 0x7fffffff) { h = (int)((uint32_t)t / (uint32_t)Sq); r = (int)((uint32_t)t % (uint32_t)Sq); }
     else                 { h = (int)(t / Sq); r = (int)(t % Sq); }
     const T* s = src + h * src_stride_h + r * src_stride_r + col;
+    const float mul = q_scale != nullptr ? 1.0f / (softmax_scale * q_scale[h] * k_scale[h]) : 1.0f;
     float x[8];
+    if constexpr (kPieces) {
+      const int left = Sk - col - 2 * lane;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int at = (e >> 1) * 64 + (e & 1);
+        x[e] = at < left ? (float)s[2 * lane + at] : 0.f;
+      }
+      uint32_t* d = reinterpret_cast<uint32_t*>(dst + t * pitch + col) + lane;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (col + 64 * e + 2 * lane < pitch) d[32 * e] = staged_pair(x[2 * e] * mul, x[2 * e + 1] * mul);
+      continue;
+    }
     if (wide && col + 8 <= Sk) {
       if constexpr (sizeof(T) == 4) {
         const float4 a = *reinterpret_cast<const float4*>(s), b = *reinterpret_cast<const float4*>(s + 4);
@@ -1418,7 +1439,6 @@ bias_to_bf16_kernel(const T* src, __nv_bfloat16* dst, int B2, int Sq, int Sk, lo
 #pragma unroll
       for (int e = 0; e < 8; ++e) x[e] = col + e < Sk ? (float)s[e] : 0.f;
     }
-    const float mul = q_scale != nullptr ? 1.0f / (softmax_scale * q_scale[h] * k_scale[h]) : 1.0f;
     uint32_t o[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[e] = staged_pair(x[2 * e] * mul, x[2 * e + 1] * mul);

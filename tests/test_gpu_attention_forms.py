@@ -460,3 +460,9 @@ def test_fp32_operands_give_the_bits_of_their_bf16_forms(cuda_device, form):
     out = A.dot_product_attention_cpp(q, k, v, None, bias)
     assert out.dtype == torch.float32
     assert torch.equal(out, A.dot_product_attention_cpp(*(t.to(torch.bfloat16) for t in (q, k, v)), None, bias).float())
+
+
+@pytest.mark.parametrize("Sk,pitch,offset", [(255, 255, 1), (256, 257, 0), (257, 257, 0), (263, 263, 2), (264, 268, 1), (513, 515, 0), (640, 641, 3)])
+def test_conversion_of_fp32_rows_that_start_anywhere(cuda_device, Sk, pitch, offset):
+    """A warp converts 256 columns of a row: lengths around whole pieces, rows of every remainder."""
+    test_conversion_of_the_bias(cuda_device, Sk, pitch, offset, torch.float32)
