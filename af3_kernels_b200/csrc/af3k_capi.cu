@@ -421,12 +421,12 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
 // Whether the attention kernel is to convert the bias itself (then *plan is one that can: one query tile of one pair row per item).
 // Estimates in us, for key tiles of 128: the pass 1.7 and 5 TB/s; a tile of a pair of streams 1.6; a lone tile whose bias is converted
 // 1.65 (rows on vectors) or, where rows start anywhere, 2.2, which is 0.75 more than in place, and 1.2 for each such item.
-// Measured, us, pass before -> here: 16 heads, rows anywhere: 129 tokens 7.1 -> 6.3, 389 bf16 12.0 -> 10.5, 1001 bf16 26.8 -> 19.5,
-// fp32 34.4 -> 19.5; 5 heads of 385 9.5 (here 10.4).  In place of pairs of query tiles: 1300 tokens bf16 43.7 -> 38.1, fp32 53.8 -> 43.7;
-// 1536 fp32 61 -> 46; 2047 bf16 89 -> 79, fp32 118 -> 79; 2048 fp32 96 -> 63; 1301 fp32 54.1 -> 52.2; 1301 bf16 43.9 keeps the pass.  (fp32 in rows anywhere: 129, 1001
-// and 2047 tokens with a slower pass, 1301 with today's.)  In place of
-// several pair rows, us a call with its host: 45 rows, 4 heads 8.7 -> 7.1, 62 rows 8.7 -> 7.6; 75 rows 8.8 (here 9.5), 128 fp32 10.0 (13.2).
-// (Calls of a few items, bound by the host either way, keep it too.)
+// Measured, us on the device, 16 heads, pass -> here (* against a slower pass over fp32 rows than today's):
+//   one query tile per item    129 tokens 7.1 -> 6.3, 389 bf16 12.0 -> 10.5, 1001 bf16 26.8 -> 19.5, fp32 34.4* -> 19.5; 5 heads of 385 9.5 (10.4)
+//   pairs of query tiles       1300 bf16 43.7 -> 38.1, fp32 53.8 -> 43.7, 1536 fp32 61 -> 46, 2048 fp32 96 -> 63, rows anywhere: 1301 fp32 54.1 -> 52.2,
+//                              2047 bf16 89 -> 79, fp32 118* -> 79; 1301 bf16 43.9 keeps the pass
+//   several pair rows          with the host, 4 heads: 45 rows 8.7 -> 7.1, 62 rows 8.7 -> 7.6; 75 rows 8.8 (9.5) and 128 fp32 10.0 (13.2) keep the pass
+// Calls of a few items, bound by the host either way, keep it too.
 constexpr int kFewItems = 16;
 constexpr double kHostOne = 6, kHostTwo = 8.7;     // a call's host time with one launch and with two: what bounds the short ones
 bool convert_in_kernel(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, bool wide) {
