@@ -515,6 +515,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
   // ring positions / barrier parities are carried incrementally: no division on this warp
   uint32_t st = 0, kv_par = 0, icount = 0, bst = 0, b_par = 0;
   uint32_t sfree_par = 0, used = 0;   // bit b: parity of buffer b's next release; buffer b has held a tile
+  grid_wait_previous();            // (nothing is there before; a wait's limit counts from here)
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {
     const Item it = decode_item<kMixed>(p, item);
@@ -621,6 +622,7 @@ __device__ void pv_issuer_role(const Ctx& c) {
   uint32_t tl_n = 0;
   uint32_t st = 0;
   uint32_t pready_par = 0;         // bit b: of warpgroup b's next P
+  grid_wait_previous();            // (a wait's limit counts from here)
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
     const Item it = decode_item<kMixed>(p, item);
@@ -984,8 +986,8 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
   const bool scales = kScalesQ && p.scale_q;
   const int scale_kt = !scales ? -1 : (p.q_buffers == 2 ? max(p.n_kt - 2, 0) : p.n_kt - 1);
   uint32_t icount = 0;
-  if (scales && (int)blockIdx.x < p.n_items && !scale_own_q<kMixed>(c, blockIdx.x, 0, wg, wq, lane)) return;
   grid_wait_previous();
+  if (scales && (int)blockIdx.x < p.n_items && !scale_own_q<kMixed>(c, blockIdx.x, 0, wg, wq, lane)) return;
 
 #pragma unroll 1
   for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++icount) {

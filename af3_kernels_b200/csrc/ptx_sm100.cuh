@@ -100,8 +100,9 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 // and loads behind it must not be of the read-only kind (__ldg), which may be moved or served across it.
 // release: the next kernel's blocks may come in as SMs become free (without it: as this kernel's blocks end).
 // A kernel's code that runs once is slow, its instructions and parameters being fetched for the first time: from the wait to the
-// first load it took 1.1 - 1.7 us with the wait at the end of the common set-up.  So each role waits where it first touches global
-// memory, its set-up behind it.  us on the device, before -> after: operator on 77 keys 5.3 -> 4.95, 512 8.6 -> 8.15, 1536 23.9 -> 23.2;
+// first load it took 1.1 - 1.7 us with the wait at the end of the common set-up.  So each role waits behind its set-up, where it first
+// touches global memory or waits on a barrier that others' loads complete: the limit of such a wait is for this kernel's own work and
+// must not run while the kernel before does, which may take any time on SMs that it does not share.  us on the device, before -> after: operator on 77 keys 5.3 -> 4.95, 512 8.6 -> 8.15, 1536 23.9 -> 23.2;
 // single block of 128 tokens 9.9 -> 8.9; grid module of 64 rows 17.2 -> 15.7, 192 rows 44.1 -> 41.7, 256 rows of 64 channels 48.5 -> 46.2.
 // (Overlap at all, us a call: 512 tokens 14.4 -> 11.7, 1536 tokens 30.8 -> 29.7, diffusion 5 x 1536 114.8 -> 112.0; grid module 64
 // rows 25.7 -> 22.2; single block of 1536 tokens 48.0 -> 43.3.  Calls of 0.6 ms and more: no difference beyond the runs' own.)

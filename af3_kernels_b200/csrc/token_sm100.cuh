@@ -110,6 +110,7 @@ token_proj_kernel(const __grid_constant__ TokParams p, const __grid_constant__ C
     const uint32_t lo = (uint32_t)d0, hi = (uint32_t)(d0 >> 32), b_lo = (uint32_t)b0, b_hi = (uint32_t)(b0 >> 32);
     const uint32_t b_step = mn ? (16 * 128) >> 4 : 2;
     bool ok = true;
+    grid_wait_previous();      // (a wait's limit counts from here)
     for (int kb = 0; kb < kblocks && ok; ++kb) {
       const int st = kb % Tile::kStages;
       ok = mbar_wait_bounded(bars + 8u * st, (kb / Tile::kStages) & 1, p.wait_limit, const_cast<volatile int*>(abort_flag));

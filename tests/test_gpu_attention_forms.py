@@ -6,7 +6,7 @@ import torch
 
 import af3_kernels_b200 as A
 from af3_kernels_b200 import _capi
-from af3_kernels_b200.dpa import dot_product_attention, stage_bias
+from af3_kernels_b200.dpa import dot_product_attention, read_status, stage_bias
 from oracle import attention_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -466,3 +466,54 @@ def test_fp32_operands_give_the_bits_of_their_bf16_forms(cuda_device, form):
 def test_conversion_of_fp32_rows_that_start_anywhere(cuda_device, Sk, pitch, offset):
     """A warp converts 256 columns of a row: lengths around whole pieces, rows of every remainder."""
     test_conversion_of_the_bias(cuda_device, Sk, pitch, offset, torch.float32)
+
+
+@pytest.mark.parametrize("form", ["bias_in_place", "converted", "converted_anywhere", "two_launches", "rows", "fp8", "single_block", "module"])
+def test_waits_are_counted_from_the_end_of_the_kernel_before(cuda_device, form):
+    """A call under a block limit lets the next kernel's blocks in on the SMs that it leaves free, and goes on for several times what a
+    single wait may take: the blocks that came in early must not have begun to count."""
+    g = torch.Generator().manual_seed(7)
+    lib = _capi.load()
+    S = 100 if form == "converted_anywhere" else 200
+    q, k, v, mask, bias = _inputs(64 if form == "rows" else 1, 4, S, 32, 7)
+    scales = {}
+    if form == "fp8":
+        q, k, scales = _quantised(q, k)
+        scales = {n: t.to(cuda_device) for n, t in scales.items()}
+    q, k, v, mask, bias = (t.to(cuda_device) for t in (q, k, v, mask, bias))
+    if form in ("converted", "two_launches"):
+        bias = bias.float()
+    if form == "converted_anywhere":
+        bias = torch.cat([bias, bias[..., :1]], -1)[..., 1:]
+    if form == "single_block":
+        x, qb = torch.randn(S, 128, generator=g).to(cuda_device, torch.bfloat16), torch.randn(128, generator=g).to(cuda_device)
+        w = [(torch.randn(128, 128, generator=g) * 0.1).to(cuda_device, torch.bfloat16) for _ in range(4)]
+        call = lambda: A.self_attention_cpp(x, mask[0], bias, w[0], qb, *w[1:], 4)
+    elif form == "module":
+        m = A.GridSelfAttentionCpp(64, 4).to(cuda_device, torch.bfloat16)
+        pair = torch.randn(40, 40, 64, generator=g).to(cuda_device, torch.bfloat16)
+        call = lambda: m(pair, mask[0, :40])
+    elif form in ("fp8", "two_launches"):
+        if form == "fp8":
+            bias = stage_bias(bias, 4, S, S, head_dim=32, **scales)
+        call = lambda: dot_product_attention(q, k, v, mask, bias, cache_bias=False, **scales)
+    else:
+        call = lambda: A.dot_product_attention_cpp(q, k, v, mask, bias)
+    with torch.no_grad():
+        want = call()
+        big = [t.to(cuda_device) for t in _inputs(192, 4, 512, 32, 8)]
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda.synchronize()
+        assert read_status(cuda_device)[0] == 0
+        lib.af3k_set_wait_limit_cycles(2_000_000)          # about a millisecond
+        try:
+            begin.record()
+            before = dot_product_attention(*big, max_ctas=1)
+            out = call()
+            end.record()
+            torch.cuda.synchronize()
+        finally:
+            lib.af3k_set_wait_limit_cycles(0)
+    assert begin.elapsed_time(end) > 4
+    assert read_status(cuda_device)[0] == 0
+    assert torch.equal(out, want) and torch.equal(before, dot_product_attention(*big))
