@@ -94,7 +94,9 @@ Tensor status_buffer(int64_t device) {
 
 // ------------------------------------------------------------------ conversions
 // Each of up to three tensors as bf16: those that are fp32, contiguous and aligned in one launch of the library's, others by torch.
-void to_bf16(std::initializer_list<Tensor*> tensors, cudaStream_t stream) {
+// block_limit: the call leaves SMs to another stream.  The library's conversions may be resident, waiting, while the kernel before
+// still runs, on those SMs too; torch's come in when it has ended, so they are taken there.
+void to_bf16(std::initializer_list<Tensor*> tensors, cudaStream_t stream, bool block_limit = false) {
   const void* src[3];
   void* dst[3];
   int64_t n[3];
@@ -102,7 +104,7 @@ void to_bf16(std::initializer_list<Tensor*> tensors, cudaStream_t stream) {
   std::vector<std::pair<Tensor*, Tensor>> made;
   for (Tensor* t : tensors) {
     if (t->scalar_type() == at::kBFloat16) continue;
-    if (t->scalar_type() != at::kFloat || !t->is_contiguous() || !t->is_cuda() || reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 != 0) {
+    if (block_limit || t->scalar_type() != at::kFloat || !t->is_contiguous() || !t->is_cuda() || reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 != 0) {
       *t = t->to(at::kBFloat16);
       continue;
     }
@@ -115,7 +117,8 @@ void to_bf16(std::initializer_list<Tensor*> tensors, cudaStream_t stream) {
 }
 
 // A contiguous bf16 result as fp32.
-Tensor to_float(const Tensor& t, cudaStream_t stream) {
+Tensor to_float(const Tensor& t, cudaStream_t stream, bool block_limit = false) {
+  if (block_limit) return t.to(at::kFloat);
   Tensor f = new_tensor(t.sizes(), at::kFloat, t.device());
   const void* src = t.data_ptr();
   void* dst = f.data_ptr();
@@ -269,7 +272,7 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
     }
     if (q.scalar_type() != at::kBFloat16 && !f32_result) type_error(std::string("q must be bfloat16, float32 or float8_e4m3fn, got ") + c10::toString(q.scalar_type()));
     if ((q_scale_in || k_scale_in) && !f32_result) type_error("q_scale / k_scale are only valid with fp8 q and k");
-    to_bf16({&q, &k, &v}, c10::cuda::getCurrentCUDAStream(dev.index()));
+    to_bf16({&q, &k, &v}, c10::cuda::getCurrentCUDAStream(dev.index()), max_ctas > 0);
   }
   if (v.scalar_type() != at::kBFloat16) v = v.to(at::kBFloat16);
   const float scale = softmax_scale ? (float)*softmax_scale : (float)(1.0 / std::sqrt((double)D));
@@ -335,7 +338,7 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
     const int rc = g_lib.attention_convert(&d, q.data_ptr(), k.data_ptr(), v.data_ptr(), bias.data_ptr(), mask_data, out.data_ptr(), status_data, stream);
     if (rc != AF3K_ERR_WORKSPACE) {
       check(rc);
-      return f32_result ? to_float(out, stream) : out;
+      return f32_result ? to_float(out, stream, max_ctas > 0) : out;
     }
   }
   Tensor ws;
@@ -346,7 +349,7 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const OptTensor& mask_in, Tensor 
   check(g_lib.attention(&d, q.data_ptr(), k.data_ptr(), v.data_ptr(), bias.data_ptr(), mask_data, out.data_ptr(), fp8 ? q_scale.data_ptr<float>() : nullptr, fp8 ? k_scale.data_ptr<float>() : nullptr,
                         ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? (size_t)ws.numel() : 0,
                         status_data, stream));
-  return f32_result ? to_float(out, stream) : out;
+  return f32_result ? to_float(out, stream, max_ctas > 0) : out;
 }
 
 // ------------------------------------------------------------------ block parameters

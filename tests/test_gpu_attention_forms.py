@@ -517,3 +517,16 @@ def test_waits_are_counted_from_the_end_of_the_kernel_before(cuda_device, form):
     assert begin.elapsed_time(end) > 4
     assert read_status(cuda_device)[0] == 0
     assert torch.equal(out, want) and torch.equal(before, dot_product_attention(*big))
+
+
+def test_fp32_operands_under_a_block_limit(cuda_device):
+    """The library's conversions overlap the kernel before, and would wait on the SMs that the limit leaves free: such a call launches
+    the pass over the bias and the attention kernel, and nothing of the library's behind them."""
+    q, k, v, mask, bias = (t.to(cuda_device) for t in _inputs(2, 4, 150, 32, 11))
+    bias = bias.float()
+    lib = _capi.load()
+    want = dot_product_attention(q, k, v, mask, bias, cache_bias=False, max_ctas=9)
+    out = dot_product_attention(q.float(), k.float(), v.float(), mask, bias, cache_bias=False, max_ctas=9, check_status=True)
+    assert lib.af3k_last_launch_count() == 2
+    assert out.dtype == torch.float32 and torch.equal(out, want.float())
+    assert torch.equal(out, A.dot_product_attention_cpp(q.float(), k.float(), v.float(), mask, bias))
