@@ -93,7 +93,8 @@ Tensor status_buffer(int64_t device) {
 }
 
 // ------------------------------------------------------------------ conversions
-// Each of up to three tensors as bf16: those that are fp32, contiguous and aligned in one launch of the library's, others by torch.
+// Each of up to three tensors as bf16: those that are fp32, contiguous, aligned and not lazily negated in one launch of the library's,
+// others by torch.
 // block_limit: the call leaves SMs to another stream.  The library's conversions may be resident, waiting, while the kernel before
 // still runs, on those SMs too; torch's come in when it has ended, so they are taken there.
 void to_bf16(std::initializer_list<Tensor*> tensors, cudaStream_t stream, bool block_limit = false) {
@@ -104,7 +105,7 @@ void to_bf16(std::initializer_list<Tensor*> tensors, cudaStream_t stream, bool b
   std::vector<std::pair<Tensor*, Tensor>> made;
   for (Tensor* t : tensors) {
     if (t->scalar_type() == at::kBFloat16) continue;
-    if (block_limit || t->scalar_type() != at::kFloat || !t->is_contiguous() || !t->is_cuda() || reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 != 0) {
+    if (block_limit || t->scalar_type() != at::kFloat || t->is_neg() || !t->is_contiguous() || !t->is_cuda() || reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 != 0) {
       *t = t->to(at::kBFloat16);
       continue;
     }
@@ -540,7 +541,7 @@ Tensor self_block(const Tensor& x_in, const OptTensor& mask_in, Tensor bias, con
                  (so == 1 || si == 1) && std::max(so, si) >= C && std::max(so, si) % 8 == 0;
   }
   // fp32 tokens are rounded in the same launch as weights that are packed
-  const bool with_tokens = !in_place_w && x_in.scalar_type() == at::kFloat && x_in.is_contiguous() && reinterpret_cast<uintptr_t>(x_in.data_ptr()) % 16 == 0;
+  const bool with_tokens = !in_place_w && x_in.scalar_type() == at::kFloat && !x_in.is_neg() && x_in.is_contiguous() && reinterpret_cast<uintptr_t>(x_in.data_ptr()) % 16 == 0;
   Tensor packed, x = x_in;
   if (!with_tokens) {
     to_bf16({&x}, stream);

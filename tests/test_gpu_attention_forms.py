@@ -530,3 +530,16 @@ def test_fp32_operands_under_a_block_limit(cuda_device):
     assert lib.af3k_last_launch_count() == 2
     assert out.dtype == torch.float32 and torch.equal(out, want.float())
     assert torch.equal(out, A.dot_product_attention_cpp(q.float(), k.float(), v.float(), mask, bias))
+
+
+def test_fp32_operands_that_are_lazily_negated(cuda_device):
+    """A tensor whose negative bit is set holds the values before the change of sign."""
+    g = torch.Generator().manual_seed(12)
+    q, k, v = (torch.randn(2, 4, 50, 24, generator=g).to(cuda_device) for _ in range(3))
+    bias = torch.randn(4, 50, 50, generator=g).to(cuda_device)
+    want = A.dot_product_attention_cpp(-q, k, -v, None, bias)
+    assert torch.equal(A.dot_product_attention_cpp(torch._neg_view(q), k, torch._neg_view(v), None, bias), want)
+    x, w = q[0].reshape(50, 96).contiguous(), [torch.randn(96, 96, generator=g).to(cuda_device) * 0.1 for _ in range(4)]
+    for ws in (w, [t.to(torch.bfloat16) for t in w]):       # packed in a launch that rounds the tokens too, and read in place
+        call = lambda t: A.self_attention_cpp(t, None, bias, ws[0], torch.zeros(96, device=cuda_device), *ws[1:], 4)
+        assert torch.equal(call(torch._neg_view(x)), call(-x))
