@@ -419,32 +419,46 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
 }
 
 // Whether the attention kernel is to convert the bias itself (then *plan is one that can: one query tile of one pair row per item).
-// Estimates in us, for key tiles of 128: the pass 1.7 and 5 TB/s; a tile of a pair of streams 1.6; a lone tile whose bias is converted
-// 1.65 (rows on vectors) or, where rows start anywhere, 2.2, which is 0.75 more than in place, and 1.2 for each such item.
-// Measured, us on the device, 16 heads, pass -> here (* against a slower pass over fp32 rows than today's):
-//   one query tile per item    129 tokens 7.1 -> 6.3, 389 bf16 12.0 -> 10.5, 1001 bf16 26.8 -> 19.5, fp32 34.4* -> 19.5; 5 heads of 385 9.5 (10.4)
-//   pairs of query tiles       1300 bf16 43.7 -> 38.1, fp32 53.8 -> 43.7, 1536 fp32 61 -> 46, 2048 fp32 96 -> 63, rows anywhere: 1301 fp32 54.1 -> 52.2,
-//                              2047 bf16 89 -> 79, fp32 118* -> 79; 1301 bf16 43.9 keeps the pass
-//   several pair rows          with the host, 4 heads: 45 rows 8.7 -> 7.1, 62 rows 8.7 -> 7.6; 75 rows 8.8 (9.5) and 128 fp32 10.0 (13.2) keep the pass
-// Calls of a few items, bound by the host either way, keep it too.
-constexpr int kFewItems = 16;
-constexpr double kHostOne = 6, kHostTwo = 8.7;     // a call's host time with one launch and with two: what bounds the short ones
-bool convert_in_kernel(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, bool wide) {
+// It is where that is no slower on the device by these estimates, in us: the pass 1.6 and, for fp32 whose copy stays in L2, 8 TB/s,
+// else 5; a lone tile of 128 keys 1.45, converted in place 1.65 (rows on vectors) or 2.2 (rows that start anywhere), and 1.2 for each such
+// item; a tile of a pair of streams 1.6, at least 1.1.  A single key tile or rows on vectors cost a lone item less than any pass.
+// Measured on the device, us, the way that is taken (the other); 16 heads, fp32 rows that start anywhere, unless said:
+//   one query tile per item   here 129 tokens 6.2 (7.0), 389 10.6 (12.0), 1001 22.8 (28.4), bf16 22.3 (27.5); 8 heads of 700 14.3 (15.2); 4 heads
+//                             of 129 6.1 (6.8), of 200 7.0 (7.4); the pass 4 heads of 1001 17.1 (18.3), 6 of 389 9.7 (10.4)
+//   pairs of query tiles      here on vectors 1200 40.0 (43.3), 1536 46.8 (60.8), 2048 66 (96), anywhere 1301 52.6 (54.0), 2047 81 (106), bf16
+//                             83 (89); the pass 1200 46.8 (48.3), 1301 bf16 44.0 (52.2), 1536 bf16 55.5 (57.3)
+//   several pair rows         nearly always the pass: 4 heads of 100 rows 9.6 (11.8), of 140 rows of 32 keys 7.8 (10.7), 3 rows of 1000 tokens on vectors
+//                             43.4 (46.6); in a graph 62 rows 6.7 (7.6)
+// Several pair rows to an item: a short call is bound by its launches, which take the host 8.6 us with the pass and 5.9 without, so
+// there up to kLaunchWorth us of the device's time are given for the one launch less (4 heads, 45 rows 9.2 -> 7.2 us a call, 62 rows 9.4 -> 7.6,
+// 40 rows of 100 on vectors 9.3 -> 7.6; most on the device: 74 rows of 64 keys 6.7 -> 8.0), and nothing is under capture, where launches are the graph's.
+// Below kFewItems ragged items the pass stays, although here would be faster up to 200 tokens (3 heads of 131: 6.8, here 6.1): no call in
+// use has fewer than four heads.
+constexpr int kFewItems = 8;
+constexpr double kLaunchWorth = 1.2, kShortCall = 5.5;
+constexpr double kL2Bytes = 126e6;
+bool convert_in_kernel(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, bool wide, cudaStream_t stream) {
   const AttnParams& p = plan->p;
-  const double es = d.bias_dtype == AF3K_F32 ? 4 : 2, elements = (double)d.B2 * d.Sq * d.Sk, width = p.kw / (double)kTile;
-  const double pass = 1.7 + elements * (es + 2) / 5e6;
-  if (p.n_streams == 1 && !p.mixed) {
-    const int rounds = (p.n_items + plan->grid - 1) / plan->grid;
-    return wide || p.n_kt == 1 || (p.n_items >= kFewItems && rounds * p.n_kt * 0.75 * width < pass);
-  }
-  Plan lone;
-  if (d.rows_per_item > 1 || make_plan(d, dev, &lone, true, true) != AF3K_OK || lone.p.mixed) return false;
-  const int rounds = (lone.p.n_items + lone.grid - 1) / lone.grid;
+  const bool lone = p.n_streams == 1 && !p.mixed;
+  if (lone && (wide || p.n_kt == 1)) return true;
+  if (lone && p.n_items < kFewItems) return false;
+  Plan other;
+  if (!lone && (d.rows_per_item > 1 || make_plan(d, dev, &other, true, true) != AF3K_OK || other.p.mixed)) return false;
+  const Plan& l = lone ? *plan : other;
+  const double es = d.bias_dtype == AF3K_F32 ? 4 : 2, elements = (double)d.B2 * d.Sq * d.Sk, bytes = elements * (es + 2);
+  const double pass = 1.6 + bytes / (es == 4 && bytes < kL2Bytes ? 8e6 : 5e6), width = p.kw / (double)kTile;
+  const auto lone_items = [&](double tile) { return ((l.p.n_items + l.grid - 1) / l.grid) * (l.p.n_kt * tile * std::max(width, 0.5) + 1.2); };
   const double reads = d.B1 * elements * es / 5e6;      // each pair row reads the whole bias
-  const double here = std::max(rounds * (lone.p.n_kt * (wide ? 1.65 : 2.2) * width + 1.2), reads), there = plan->cost * 1.6 * width + pass;
-  if (std::max(here + 1.5, kHostOne) >= 0.98 * std::max(there + 1.5, kHostTwo)) return false;
-  *plan = lone;
-  return true;
+  const double here = std::max(lone_items(wide ? 1.65 : 2.2), reads);
+  const double there = pass + (lone ? lone_items(1.45) : plan->cost * std::max(1.6 * width, 1.1));
+  bool convert = here < (lone ? 1.0 : 0.98) * there;      // (plans that are given up have to be beaten by this much)
+  if (!convert && p.G > 1 && there < kShortCall && here - there <= kLaunchWorth) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) (void)cudaGetLastError();
+    convert = capture == cudaStreamCaptureStatusNone;
+  }
+  if (convert && !lone) *plan = other;
+  return convert;
 }
 
 int encode_qkv_map(CUtensorMap* tm, const void* base, bool fp8, int64_t D, int64_t S, int64_t B2,
@@ -653,7 +667,7 @@ int attention_call(const af3k_attention_desc* desc, const void* q, const void* k
   // the kernel converts the bias itself: items of one query tile
   const uintptr_t bias_es = d.bias_dtype == AF3K_F32 ? 4 : 2;
   const bool wide = d.Sk % 4 == 0 && (reinterpret_cast<uintptr_t>(bias) | (uintptr_t)bias_sh * bias_es | (uintptr_t)bias_sr * bias_es) % (4 * bias_es) == 0;
-  const bool in_kernel = convert && must_stage && !fp8 && p.debug == nullptr && convert_in_kernel(d, *dev, &plan, wide);
+  const bool in_kernel = convert && must_stage && !fp8 && p.debug == nullptr && convert_in_kernel(d, *dev, &plan, wide, stream);
   p.bias_wide = wide ? 1 : 0;
   if ((must_stage && !in_kernel) || stage_fp8) {
     if (workspace == nullptr || workspace_bytes < stage_bytes) return AF3K_ERR_WORKSPACE;

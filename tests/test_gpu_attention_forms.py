@@ -401,11 +401,13 @@ def test_key_tiles_of_every_width(cuda_device, Sk, qk, D):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("B1,B2,Sq,Sk,D,pitch,offset,launches", [
-    (1, 16, 129, 129, 32, 129, 0, 1), (1, 16, 140, 161, 24, 161, 1, 1), (1, 16, 250, 225, 48, 231, 2, 1), (2, 16, 200, 257, 32, 257, 3, 1), (1, 6, 400, 389, 64, 389, 5, None),
-    (1, 5, 385, 385, 32, 385, 0, None), (1, 16, 1300, 1300, 24, 1300, 0, 1), (1, 16, 1290, 1301, 16, 1301, 1, None), (1, 20, 1100, 1030, 40, 1032, 4, None)])
+    (1, 16, 129, 129, 32, 129, 0, (1, 1)), (1, 16, 140, 161, 24, 161, 1, (1, 1)), (1, 16, 250, 225, 48, 231, 2, (1, 1)), (2, 16, 200, 257, 32, 257, 3, (1, 1)),
+    (1, 6, 400, 389, 64, 389, 5, (2, 2)), (1, 16, 400, 389, 64, 389, 5, (1, 1)), (1, 5, 385, 385, 32, 385, 0, (2, 2)), (1, 16, 385, 385, 32, 385, 0, (1, 1)),
+    (1, 16, 1300, 1300, 24, 1300, 0, (1, 1)), (1, 16, 1290, 1301, 16, 1301, 1, (1, 2)), (1, 16, 2000, 2001, 16, 2001, 1, (1, 1)), (1, 20, 1100, 1030, 40, 1032, 4, (1, 2))])
 def test_ragged_rows_of_several_key_tiles_converted_by_the_attention_kernel(cuda_device, dtype, B1, B2, Sq, Sk, D, pitch, offset, launches):
     """Rows that start anywhere, key tiles of 80 to 128 keys, more query tiles than SMs among them: the bits of the pass, whatever stands
-    in front of, between and behind the rows."""
+    in front of, between and behind the rows.  launches: with an fp32 and with a bf16 bias (two: the pass, by its estimate, so that
+    nothing is compared there but two ways into it)."""
     g = torch.Generator().manual_seed(Sk)
     q, k, v = (torch.randn(B1, B2, s, D, generator=g).to(cuda_device, torch.bfloat16) for s in (Sq, Sk, Sk))
     mask = (torch.rand(B1, Sk, generator=g) >= 0.1).to(cuda_device)
@@ -417,7 +419,7 @@ def test_ragged_rows_of_several_key_tiles_converted_by_the_attention_kernel(cuda
     bias[..., -1] = 1
     lib = _capi.load()
     out = A.dot_product_attention_cpp(q, k, v, mask, bias)
-    assert launches is None or lib.af3k_last_launch_count() == launches
+    assert lib.af3k_last_launch_count() == launches[dtype is torch.bfloat16]
     staged = dot_product_attention(q, k, v, mask, bias, cache_bias=False, check_status=True)
     assert lib.af3k_last_launch_count() == 2 and not out.isnan().any()
     assert torch.equal(out, staged)
@@ -543,3 +545,29 @@ def test_fp32_operands_that_are_lazily_negated(cuda_device):
     for ws in (w, [t.to(torch.bfloat16) for t in w]):       # packed in a launch that rounds the tokens too, and read in place
         call = lambda t: A.self_attention_cpp(t, None, bias, ws[0], torch.zeros(96, device=cuda_device), *ws[1:], 4)
         assert torch.equal(call(torch._neg_view(x)), call(-x))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B1,B2,S,pitch,offset,launches,captured", [
+    (45, 4, 45, 45, 0, 1, 2), (62, 4, 62, 62, 1, 1, 2), (64, 4, 64, 68, 4, 1, 2), (38, 8, 33, 33, 0, 2, 2), (75, 4, 75, 75, 0, 2, 2), (100, 4, 62, 62, 1, 2, 2), (140, 4, 24, 28, 4, 2, 2),
+    (140, 4, 31, 31, 0, 2, 2), (20, 16, 40, 44, 4, 2, 2), (1, 4, 129, 129, 0, 1, 1), (1, 4, 255, 255, 0, 1, 1), (1, 4, 1001, 1001, 0, 2, 2), (1, 3, 131, 131, 0, 2, 2)])
+def test_short_calls_convert_their_bias_where_the_device_loses_little(cuda_device, dtype, B1, B2, S, pitch, offset, launches, captured):
+    """Several pair rows per item, in place of which lone rows convert: only while that costs the device little, and not in a graph.
+    Lone items of four heads.  The same bits on every way."""
+    q, k, v, mask, _ = _inputs(B1, B2, S, 32, S)
+    mask[:, -1] = True
+    flat = torch.full((B2 * S * pitch + 16,), float("nan"), device=cuda_device, dtype=dtype)
+    bias = flat[offset:offset + B2 * S * pitch].view(B2, S, pitch)[:, :, :S]
+    bias.copy_(torch.randn(B2, S, S, generator=torch.Generator().manual_seed(S)))
+    q, k, v, mask = (t.to(cuda_device) for t in (q, k, v, mask))
+    lib = _capi.load()
+    out = A.dot_product_attention_cpp(q, k, v, mask, bias)
+    assert lib.af3k_last_launch_count() == launches
+    assert torch.equal(out, dot_product_attention(q, k, v, mask, bias, cache_bias=False, check_status=True))
+    assert lib.af3k_last_launch_count() == 2
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        replayed = A.dot_product_attention_cpp(q, k, v, mask, bias)
+        count = lib.af3k_last_launch_count()
+    graph.replay()
+    assert count == captured and torch.equal(replayed, out)
