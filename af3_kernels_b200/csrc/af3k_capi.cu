@@ -68,9 +68,16 @@ constexpr int kStaticSmemReserve = 1024;   // the kernels' few static bytes, pad
 // Key tiles come in these widths; every width is a kernel of its own, whose softmax warps have that many logits in registers.
 constexpr int kKeyWidths[] = {32, 64, 80, 96, 112, 128};
 
-// f(kernel) for the kernel of key tiles of kw keys.
+// f(kernel) for the kernel of key tiles of kw keys, the last of last_w.
 template <bool kFp8, bool kGate, bool kMixed, bool kConvert, typename F>
-void with_width(int kw, F&& f) {
+void with_width(int kw, int last_w, F&& f) {
+  if (last_w != kw) {
+    switch (last_w) {
+      case 32: return f(attention_kernel<false, true, kFp8, kGate, kMixed, kConvert, 128, 32>);
+      case 64: return f(attention_kernel<false, true, kFp8, kGate, kMixed, kConvert, 128, 64>);
+      default: return f(attention_kernel<false, true, kFp8, kGate, kMixed, kConvert, 128, 96>);
+    }
+  }
   switch (kw) {
     case 32: return f(attention_kernel<false, true, kFp8, kGate, kMixed, kConvert, 32>);
     case 64: return f(attention_kernel<false, true, kFp8, kGate, kMixed, kConvert, 64>);
@@ -117,12 +124,14 @@ int device_info(DeviceInfo** out) {
         (const void*)attention_kernel<true, false, true, false, true>,
     };
     const auto add = [&](auto kernel) { kernels.push_back((const void*)kernel); };
-    for (int kw : kKeyWidths) {
-      with_width<false, false, false, false>(kw, add); with_width<false, false, true, false>(kw, add);
-      with_width<false, true, false, false>(kw, add);  with_width<false, true, true, false>(kw, add);
-      with_width<false, false, false, true>(kw, add);  with_width<false, true, false, true>(kw, add);
-      with_width<true, false, false, false>(kw, add);  with_width<true, false, true, false>(kw, add);
-    }
+    const auto add_width = [&](int kw, int last_w) {
+      with_width<false, false, false, false>(kw, last_w, add); with_width<false, false, true, false>(kw, last_w, add);
+      with_width<false, true, false, false>(kw, last_w, add);  with_width<false, true, true, false>(kw, last_w, add);
+      with_width<false, false, false, true>(kw, last_w, add);  with_width<false, true, false, true>(kw, last_w, add);
+      with_width<true, false, false, false>(kw, last_w, add);  with_width<true, false, true, false>(kw, last_w, add);
+    };
+    for (int kw : kKeyWidths) add_width(kw, kw);
+    for (int last_w : {32, 64, 96}) add_width(kTile, last_w);
     e = cudaSuccess;
     for (const void* kfn : kernels)
       if (e == cudaSuccess) e = cudaFuncSetAttribute(kfn, attr, dyn);
@@ -228,6 +237,7 @@ void launch_overlapped(void (*kernel)(KArgs...), dim3 grid, int threads, size_t 
 
 struct Plan {
   AttnParams p;
+  int last_w;      // keys of the last key tile
   size_t smem_bytes;
   int grid;
   double cost;     // of the longest CTA, in logits-tile times of one warpgroup
@@ -255,19 +265,32 @@ constexpr double kLoneTile = 0.75;
 // Smaller items behind the last full round have to promise this much: the model is no better than that.
 constexpr double kTailGain = 0.98;
 
-// Keys per key tile: as many tiles as 128 keys each make, and of those the narrowest that hold the call's keys, because a
-// tile's loads from TMEM, maximum, exponentials, stores and MMAs go with its width while its waits and hand-overs do not.
-// (Depends on nothing but the keys and the kind of kernel, so that all plans of a call add up the same tiles.)  Attention kernel in
-// the grid module, us, tiles of 128 -> as wide as needed: 192 rows (96) 27.1 -> 24.3, 389 rows (112) 151 -> 139, 30 rows (32)
-// 6.3 -> 4.8; the operator on 77 keys (80) 5.6 -> 5.3.  With the width as a run-time value in the issuers' loops 1536 tokens took
-// 25.2 instead of 24.5, so it is a template argument of every role.
-int key_width(const af3k_attention_desc& d, bool tc_bias, bool debug) {
+// Keys per key tile, and of the last one.  A tile's loads from TMEM, maximum, exponentials, stores and MMAs go with its width
+// while its waits and hand-overs do not, so a single tile is the narrowest that holds the call's keys, and the last of several, behind
+// tiles of 128, the narrowest in steps of 32 where that leaves out at least a twelfth of the call's columns.  Its code beside the loop's costs
+// about what less than that gains: time with it over time without, 5 x 16 heads, rows of the operator, converted bias: 2 tiles, the last of 32 0.93
+// 0.88 0.92, of 96 0.97 0.93 1.00; 3 tiles, 96 0.97 0.97 1.01; 4 tiles, 32 0.98 0.93 0.94, 96 1.01 1.00 1.01; 6 tiles, 64 1.00 0.96 0.99; 8 tiles, 32
+// 0.99 0.96 0.98, 64 1.00 0.97 0.99; 13 tiles, 32 1.02 - 0.99, 64 1.01 - 1.01.
+// Where the borders between tiles lie is part of the result: they decide which key a row's weights are rounded against.  Tiles of one
+// width each (389 keys as four of 112) left results up to 1.5 % farther from 64 bits (192 rows of 192 keys 2.632e-3 -> 2.673e-3).
+// (Depends on nothing but the keys and the kind of kernel, so that all plans of a call add up the same tiles.)  Device time, us, all tiles
+// of 128 -> so: module call of 150 rows 46.2 -> 39.0, 192 48.9 -> 43.3, 389 216 -> 206; operator on 392 rows 151 -> 138, fp8 140 -> 131, on 77 keys
+// 5.6 -> 5.3.  With the width as a run-time value in the issuers' loops 1536 tokens took 25.2 instead of 24.5, so the widths
+// are template arguments of every role.
+void key_widths(const af3k_attention_desc& d, bool tc_bias, bool debug, Plan* plan) {
+  AttnParams* const p = &plan->p;
   const bool fp8 = d.qk_dtype == AF3K_FP8_E4M3;
-  if (!tc_bias || (fp8 && d.gate != nullptr) || debug) return kTile;   // kernels of one width
-  const int64_t tiles = (d.Sk + kTile - 1) / kTile, need = (d.Sk + tiles - 1) / tiles;
+  p->n_kt = (p->Sk + kTile - 1) / kTile;
+  p->kw = plan->last_w = kTile;
+  if (!tc_bias || (fp8 && d.gate != nullptr) || debug) return;   // kernels of one width
+  const int rest = p->Sk - (p->n_kt - 1) * kTile;
+  if (p->n_kt > 1) {
+    const int w = (rest + 31) / 32 * 32;
+    if (12 * (kTile - w) >= kTile * p->n_kt) plan->last_w = w;
+    return;
+  }
   for (int kw : kKeyWidths)
-    if (kw >= need) return kw;
-  return kTile;
+    if (kw >= rest) { p->kw = plan->last_w = kw; return; }
 }
 
 // Picks rows-per-item G and the K/V ring depth from a cost model of one CTA's time (below).
@@ -281,8 +304,7 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
   p.B1 = (int)d.B1; p.B2 = (int)d.B2; p.Sq = (int)d.Sq; p.Sk = (int)d.Sk; p.D = (int)d.D;
   p.n_qt = (p.Sq + kTile - 1) / kTile;
   p.debug = g_debug_dump.load();
-  p.kw = key_width(d, allow_q_split, p.debug != nullptr);
-  p.n_kt = (p.Sk + p.kw - 1) / p.kw;
+  key_widths(d, allow_q_split, p.debug != nullptr, plan);
   p.qk_row_bytes = row_bytes_for(d.D * es);
   p.v_row_bytes = row_bytes_for(d.D * 2);
   p.qk_ksteps = (int)((d.D * es + 31) / 32);
@@ -446,8 +468,9 @@ bool convert_in_kernel(const af3k_attention_desc& d, const DeviceInfo& dev, Plan
   if (!lone && (d.rows_per_item > 1 || make_plan(d, dev, &other, true, true) != AF3K_OK || other.p.mixed)) return false;
   const Plan& l = lone ? *plan : other;
   const double es = d.bias_dtype == AF3K_F32 ? 4 : 2, elements = (double)d.B2 * d.Sq * d.Sk, bytes = elements * (es + 2);
-  const double pass = 1.6 + bytes / (es == 4 && bytes < kL2Bytes ? 8e6 : 5e6), width = p.kw / (double)kTile;
-  const auto lone_items = [&](double tile) { return ((l.p.n_items + l.grid - 1) / l.grid) * (l.p.n_kt * tile * std::max(width, 0.5) + 1.2); };
+  const double pass = 1.6 + bytes / (es == 4 && bytes < kL2Bytes ? 8e6 : 5e6);
+  const double tiles = std::max(((p.n_kt - 1) * p.kw + plan->last_w) / (double)kTile, 0.5), width = tiles / p.n_kt;     // key tiles of 128
+  const auto lone_items = [&](double tile) { return ((l.p.n_items + l.grid - 1) / l.grid) * (tiles * tile + 1.2); };
   const double reads = d.B1 * elements * es / 5e6;      // each pair row reads the whole bias
   const double here = std::max(lone_items(wide ? 1.65 : 2.2), reads);
   const double there = pass + (lone ? lone_items(1.45) : plan->cost * std::max(1.6 * width, 1.1));
@@ -701,7 +724,7 @@ int attention_call(const af3k_attention_desc* desc, const void* q, const void* k
   p.k_scale = k_scale;
   p.mask = mask;
   p.mask_row_stride = d.mask_row_stride;
-  p.mask_col = (mask != nullptr || d.Sk % p.kw != 0) ? 1 : 0;
+  p.mask_col = (mask != nullptr || d.Sk != (int64_t)(p.n_kt - 1) * p.kw + plan.last_w) ? 1 : 0;
   p.out = static_cast<__nv_bfloat16*>(out);
   p.out_stride_b1 = d.out_stride[0];
   p.out_stride_b2 = d.out_stride[1];
@@ -722,20 +745,20 @@ int attention_call(const af3k_attention_desc* desc, const void* q, const void* k
     launch_overlapped(kernel, dim3(plan.grid), in_kernel ? kConvertThreads : kThreads, plan.smem_bytes, stream, d.max_ctas <= 0, p, tm_q, tm_k, tm_v, tm_b, tm_q2, tm_k2);
   };
   if (in_kernel) {
-    if (p.gate != nullptr) with_width<false, true, false, true>(p.kw, launch);
-    else                   with_width<false, false, false, true>(p.kw, launch);
+    if (p.gate != nullptr) with_width<false, true, false, true>(p.kw, plan.last_w, launch);
+    else                   with_width<false, false, false, true>(p.kw, plan.last_w, launch);
   } else if (dbg && p.gate == nullptr) {
     if (!fp8)         launch(attention_kernel<true, true, false, false, true>);
     else if (tc_bias) launch(attention_kernel<true, true, true, false, true>);
     else              launch(attention_kernel<true, false, true, false, true>);
   } else if (!fp8) {
-    if (p.gate != nullptr) { if (p.mixed) with_width<false, true, true, false>(p.kw, launch);  else with_width<false, true, false, false>(p.kw, launch); }
-    else                   { if (p.mixed) with_width<false, false, true, false>(p.kw, launch); else with_width<false, false, false, false>(p.kw, launch); }
+    if (p.gate != nullptr) { if (p.mixed) with_width<false, true, true, false>(p.kw, plan.last_w, launch);  else with_width<false, true, false, false>(p.kw, plan.last_w, launch); }
+    else                   { if (p.mixed) with_width<false, false, true, false>(p.kw, plan.last_w, launch); else with_width<false, false, false, false>(p.kw, plan.last_w, launch); }
   } else if (p.gate != nullptr) {
     if (tc_bias) { if (p.mixed) launch(attention_kernel<false, true, true, true, true>);  else launch(attention_kernel<false, true, true, true, false>); }
     else         { if (p.mixed) launch(attention_kernel<false, false, true, true, true>); else launch(attention_kernel<false, false, true, true, false>); }
   } else if (tc_bias) {
-    if (p.mixed) with_width<true, false, true, false>(p.kw, launch); else with_width<true, false, false, false>(p.kw, launch);
+    if (p.mixed) with_width<true, false, true, false>(p.kw, plan.last_w, launch); else with_width<true, false, false, false>(p.kw, plan.last_w, launch);
   } else {
     if (p.mixed) launch(attention_kernel<false, false, true, false, true>); else launch(attention_kernel<false, false, true, false, false>);
   }

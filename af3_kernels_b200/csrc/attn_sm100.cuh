@@ -111,7 +111,7 @@ __device__ __forceinline__ uint32_t divide(uint32_t x, const Divisor& v) { retur
 struct AttnParams {
   int B1, B2, Sq, Sk, D;
   int n_qt, n_kt;
-  int kw;                // keys per key tile (the kernel's kW)
+  int kw;                // keys per key tile (the kernel's kW; its kLast: of the last one)
   int G;                 // pair rows per work item
   int q_split;           // 1: the streams of an item are two neighbouring query tiles of ONE pair row (G == 1)
   int n_streams;         // streams per work item: G, or 2 with q_split
@@ -298,7 +298,7 @@ __device__ __forceinline__ uint32_t q_buf(const AttnParams& p, uint32_t j) { ret
 __device__ __forceinline__ uint32_t q_use(const AttnParams& p, uint32_t j) { return p.q_buffers == 2 ? (j >> 1) : j; }
 
 // ------------------------------------------------------------------ producer (one thread)
-template <bool kMixed, bool kConvert, int kW>
+template <bool kMixed, bool kConvert, int kW, int kLast>
 __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUtensorMap* tm_k,
                               const CUtensorMap* tm_v, const CUtensorMap* tm_bias, const CUtensorMap* tm_q2, const CUtensorMap* tm_k2) {
   const AttnParams& p = *c.p;
@@ -349,9 +349,10 @@ __device__ void producer_role(const Ctx& c, const CUtensorMap* tm_q, const CUten
           if (blap != 0) AF3K_WAIT(c, BarIdx::bias_empty + bst, (blap - 1) & 1);
           const uint32_t bfull = bar_addr(c, BarIdx::bias_full + bst);
           const uint32_t bdst = c.smem + p.off_bias + bst * kBiasTileBytes;
-          mbar_arrive_expect_tx(bfull, kW > 64 ? kBiasTileBytes : kBiasTileBytes / 2);
+          const bool both = kW > 64 && (kLast == kW || kLast > 64 || kt != p.n_kt - 1);      // boxes of 64 keys
+          mbar_arrive_expect_tx(bfull, both ? kBiasTileBytes : kBiasTileBytes / 2);
           tma_load_3d(bdst, tm_bias, bfull, kt * kW, stream_qt(p, it, s) * kTile, it.h);
-          if (kW > 64) tma_load_3d(bdst + kBiasTileBytes / 2, tm_bias, bfull, kt * kW + 64, stream_qt(p, it, s) * kTile, it.h);
+          if (both) tma_load_3d(bdst + kBiasTileBytes / 2, tm_bias, bfull, kt * kW + 64, stream_qt(p, it, s) * kTile, it.h);
           if (++bst == n_bias) { bst = 0; ++blap; }
         }
         if (lap != 0) AF3K_WAIT(c, BarIdx::kv_empty + st, (lap - 1) & 1);
@@ -473,7 +474,7 @@ __device__ void mask_writer_role(const Ctx& c, int lane) {
 // Logits of every tile, in order: Q K^T, then the mask column, then (bf16 q/k) the bias slices.
 // (The MMA loops are real loops and the fp8 / bf16 choice is a template argument: the warp pays an
 // instruction-cache miss for most lines of this loop on every pass, so the loop is kept small.)
-template <bool kDebug, bool kTcBias, bool kFp8, bool kMixed, int kW>
+template <bool kDebug, bool kTcBias, bool kFp8, bool kMixed, int kW, int kLast>
 __device__ void qk_issuer_role(const Ctx& c) {
   const AttnParams& p = *c.p;
   const WaitBlock* wait_block = wait_block_of(c.bars);
@@ -499,6 +500,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
   const uint32_t od_lo = (uint32_t)od0, od_hi = (uint32_t)(od0 >> 32);
   const uint32_t md_lo = (uint32_t)md0, md_hi = (uint32_t)(md0 >> 32);
   const uint32_t idesc_mask = make_idesc(1u, 1u, 0u, 0u, kW);
+  constexpr uint32_t idesc_short = make_idesc(0u, 0u, 0u, 0u, kW) - make_idesc(0u, 0u, 0u, 0u, kLast);
   const bool mask_col = p.mask_col != 0;
   // bias slices: A = 16 keys of the staged bias tile (K-major, 128-byte swizzled rows, two boxes
   // of 64 keys), B = the 16 x 16 identity (K-major, no swizzle: 8-key halves 256 bytes apart,
@@ -554,21 +556,23 @@ __device__ void qk_issuer_role(const Ctx& c) {
         const uint32_t bias_lo = bd_lo + bst * (kBiasTileBytes >> 4);
         if (leader) {
           const long long t0 = kDebug && tl != nullptr ? clock64() : 0;
+          const bool narrow = kLast != kW && kt == p.n_kt - 1;
+          const uint32_t fewer = narrow ? idesc_short : 0u;
 #pragma unroll 1
           for (int k = 0; k < ksteps; ++k) {     // one K step = 32 bytes of a tile row
             // (Q and K tiles have one layout, so one high descriptor word)
             const bool last16 = !fp8 && k >= wide_ksteps;
             const uint32_t off = last16 ? kNarrowOff >> 4 : 2 * k, hi = last16 ? narrow_hi : qd_hi;
-            if (fp8) mma_ss_f8(s_tmem, a_lo + off, hi, b_lo + off, hi, idesc_qk, k > 0 ? 1u : 0u);
-            else     mma_ss_f16(s_tmem, a_lo + off, hi, b_lo + off, hi, idesc_qk, k > 0 ? 1u : 0u);
+            if (fp8) mma_ss_f8(s_tmem, a_lo + off, hi, b_lo + off, hi, idesc_qk - fewer, k > 0 ? 1u : 0u);
+            else     mma_ss_f16(s_tmem, a_lo + off, hi, b_lo + off, hi, idesc_qk - fewer, k > 0 ? 1u : 0u);
           }
           // mask column: start address and leading offset both move with the ring slot (the
           // zero block stays put)
           if (mask_col)
-            mma_ss_f16(s_tmem, od_lo, od_hi, md_lo + slot16 - (slot16 << 16), md_hi, idesc_mask, 1u);
+            mma_ss_f16(s_tmem, od_lo, od_hi, md_lo + slot16 - (slot16 << 16), md_hi, idesc_mask - fewer, 1u);
           if (kTcBias) {
 #pragma unroll 1
-            for (int k = 0; k < kW / 16; ++k)   // keys 16k .. 16k + 15: box k / 4, 32 bytes per step
+            for (int k = 0; k < (narrow ? kLast : kW) / 16; ++k)   // keys 16k .. 16k + 15: box k / 4, 32 bytes per step
               mma_ss_f16(s_tmem + 16 * k, bias_lo + (k >> 2) * (kBiasTileBytes >> 5) + 2 * (k & 3), bd_hi,
                          id_lo, id_hi, idesc_bias, 1u);
           }
@@ -601,7 +605,7 @@ __device__ void qk_issuer_role(const Ctx& c) {
 }
 
 // O += P V for every tile, in order.
-template <bool kDebug, bool kMixed, int kW>
+template <bool kDebug, bool kMixed, int kW, int kLast>
 __device__ void pv_issuer_role(const Ctx& c) {
   const AttnParams& p = *c.p;
   const WaitBlock* wait_block = wait_block_of(c.bars);
@@ -642,7 +646,7 @@ __device__ void pv_issuer_role(const Ctx& c) {
           const long long t0 = kDebug && tl != nullptr ? clock64() : 0;
           mma_ts_f16(o_tmem, p_tmem, b_lo, vd_hi, idesc_pv, kt > 0 ? 1u : 0u);
 #pragma unroll 1
-          for (int k = 1; k < kW / 16; ++k)   // 16 keys per step: 8 TMEM columns of P
+          for (int k = 1; k < (kLast != kW && kt == p.n_kt - 1 ? kLast : kW) / 16; ++k)   // 16 keys per step: 8 TMEM columns of P
             mma_ts_f16(o_tmem, p_tmem + k * 8, b_lo + k * v_kstep, vd_hi, idesc_pv, 1u);
           tc_commit(bar_addr(c, BarIdx::pv_done + b));
           tc_commit(bar_addr(c, BarIdx::kv_empty + st));
@@ -964,7 +968,7 @@ __device__ __forceinline__ bool scale_own_q(const Ctx& c, int item, uint32_t j, 
   return true;
 }
 
-template <bool kDebug, bool kTcBias, bool kGate, bool kMixed, bool kScalesQ, int kW>
+template <bool kDebug, bool kTcBias, bool kGate, bool kMixed, bool kScalesQ, int kW, int kLast>
 __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
   const AttnParams& p = *c.p;
   const int row = wq * 32 + lane;                    // row of the 128-query tile == TMEM lane
@@ -998,8 +1002,10 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
     if (p.q_scale != nullptr) scale *= p.q_scale[it.h] * p.k_scale[it.h];
     if (kTcBias) scale = (p.scale_q ? 1.0f : scale) * kLog2e;
 
+    // A narrower last tile is taken behind the loop, so that the loop's code is as without: with the choice inside it, or inside the tile,
+    // 389 rows took longer than with four tiles of 128 (module call 216 us; inside 222 - 229, here 206).
 #pragma unroll 1
-    for (int kt = 0; kt < p.n_kt; ++kt) {
+    for (int kt = 0; kt < p.n_kt - (kLast != kW); ++kt) {
       // fp8 q/k: this thread adds the bias itself, from its row of the staged tile
       if (!kTcBias) AF3K_WAIT_WARP(c, BarIdx::bias_full + bst, b_par);
       const uint32_t bias_row = c.smem + p.off_bias + bst * kBiasTileBytes + row * 128;
@@ -1020,7 +1026,7 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
                                                   kt == 0, ts))
           return;
         st.swap = it.gv > wg + 2;
-        if (kt == p.n_kt - 1) {
+        if (kLast == kW && kt == p.n_kt - 1) {
           const int qrow = stream_qt(p, it, s) * kTile + row;
           st.done_o = c.tmem + lane_sel + kOCol + s * p.nv;
           st.done_row = qrow < p.Sq ? p.out + (long long)stream_row(p, it, s) * p.out_stride_b1 + (long long)it.h * p.out_stride_b2 +
@@ -1038,6 +1044,27 @@ __device__ void softmax_role(const Ctx& c, int wg, int wq, int lane) {
         if (++bst == (uint32_t)p.bias_stages) { bst = 0; b_par ^= 1; }
       }
       if (kScalesQ && kt == scale_kt && item + (int)gridDim.x < p.n_items &&
+          !scale_own_q<kMixed>(c, item + gridDim.x, icount + 1, wg, wq, lane))
+        return;
+    }
+    if constexpr (kLast != kW) {
+#pragma unroll 1
+      for (int s = wg; s < it.gv; s += 2) {
+        if (!softmax_tile<kDebug, kTcBias, kGate, kLast>(c, st, nullptr, wg, lane, s_taddr, p_taddr, c.tmem + lane_sel + kOCol + s * p.nv, 0, 0, scale, false,
+                                                     nullptr))
+          return;
+        st.swap = it.gv > wg + 2;
+        const int qrow = stream_qt(p, it, s) * kTile + row;
+        st.done_o = c.tmem + lane_sel + kOCol + s * p.nv;
+        st.done_row = qrow < p.Sq ? p.out + (long long)stream_row(p, it, s) * p.out_stride_b1 + (long long)it.h * p.out_stride_b2 +
+                                        (long long)qrow * p.out_stride_s
+                                  : nullptr;
+        if (kDebug) st.done_dbg = p.debug != nullptr && item == 0 && s == 0 ? p.debug + (size_t)row * kTile : nullptr;
+        if constexpr (kGate)
+          st.done_gate = p.gate + (long long)stream_row(p, it, s) * p.gate_stride_b1 + (long long)it.h * p.gate_stride_b2 +
+                         (long long)qrow * p.gate_stride_s;
+      }
+      if (kScalesQ && scale_kt == p.n_kt - 1 && item + (int)gridDim.x < p.n_items &&
           !scale_own_q<kMixed>(c, item + gridDim.x, icount + 1, wg, wq, lane))
         return;
     }
@@ -1220,8 +1247,8 @@ __device__ void bias_convert_ragged_role(const Ctx& c, int cw, int lane) {
 // tiles that leave a remainder), which takes slots and barriers that an item does not use through their phases and two sets
 // of constants to decode an item.  A plan of equal items runs without: 768 rows 645 -> 636 us.
 // kConvert: plans of one stream per item, bf16 q and k; see bias_convert_role.
-// kW: keys per key tile, 32 to 128 (chosen by key_width in the C API).
-template <bool kDebug, bool kTcBias, bool kFp8, bool kGate, bool kMixed, bool kConvert = false, int kW = kTile>
+// kW: keys per key tile, 32 to 128, kLast: of the last one, where it is narrower (chosen by key_widths in the C API).
+template <bool kDebug, bool kTcBias, bool kFp8, bool kGate, bool kMixed, bool kConvert = false, int kW = kTile, int kLast = kW>
 __global__ void __launch_bounds__(kConvert ? kConvertThreads : kThreads, 1)
 attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -1300,11 +1327,11 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     // warps 0-3 need few registers; the two softmax warpgroups take what they give up
     setmaxnreg_dec<kRegsMisc>();
     if (warp == 0) {
-      if (lane == 0) producer_role<kMixed, kConvert, kW>(c, &tm_q, &tm_k, &tm_v, &tm_bias, &tm_q2, &tm_k2);
+      if (lane == 0) producer_role<kMixed, kConvert, kW, kLast>(c, &tm_q, &tm_k, &tm_v, &tm_bias, &tm_q2, &tm_k2);
     } else if (warp == 1) {
-      qk_issuer_role<kDebug, kTcBias, kFp8, kMixed, kW>(c);
+      qk_issuer_role<kDebug, kTcBias, kFp8, kMixed, kW, kLast>(c);
     } else if (warp == 2) {
-      pv_issuer_role<kDebug, kMixed, kW>(c);
+      pv_issuer_role<kDebug, kMixed, kW, kLast>(c);
     } else if (warp == 3) {
       if (p.mask_col) mask_writer_role<kMixed, kW>(c, lane);
     }
@@ -1321,7 +1348,7 @@ attention_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ C
     }
   } else {
     setmaxnreg_inc<kRegsSoftmax>();
-    softmax_role<kDebug, kTcBias, kGate, kMixed, !kFp8, kW>(c, (warp - 4) >> 2, warp & 3, lane);
+    softmax_role<kDebug, kTcBias, kGate, kMixed, !kFp8, kW, kLast>(c, (warp - 4) >> 2, warp & 3, lane);
   }
 
   tc_fence_before();

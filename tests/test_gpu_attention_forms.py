@@ -571,3 +571,26 @@ def test_short_calls_convert_their_bias_where_the_device_loses_little(cuda_devic
         count = lib.af3k_last_launch_count()
     graph.replay()
     assert count == captured and torch.equal(replayed, out)
+
+
+@pytest.mark.parametrize("qk,D", [("bf16", 24), ("bf16", 48), ("fp8", 32)])
+@pytest.mark.parametrize("Sk", [1, 31, 77, 97, 128, 129, 160, 161, 192, 193, 224, 225, 256, 257, 300, 389, 512, 513])
+def test_results_do_not_depend_on_the_tiles_width(cuda_device, Sk, qk, D):
+    """Narrow tiles leave out keys that do not exist and nothing else: the same bits as all tiles of 128 keys give (the kernels that
+    write the debug dump have those only).  Several pair rows with a remainder, pairs of query tiles, a query tile of its own."""
+    lib = _capi.load()
+    dump = torch.empty(4 * 128 * 128 + 2 * (2 * 256 * 8 + 4 * 256), device=cuda_device)
+    for B1, Sq, kw in ((7, 140, {}), (1, 400, {"max_ctas": 2}), (1, 70, {}), (5, 90, {"rows_per_item": 4})):
+        q, k, v, mask, bias = _inputs(B1, 2, Sq, D, Sk + D, Sk)
+        mask[:, -1] = True
+        scales = {}
+        if qk == "fp8":
+            q, k, scales = _quantised(q, k)
+        scales = {n: t.to(cuda_device) for n, t in scales.items()}
+        out = _call(cuda_device, q, k, v, mask, bias, **kw, **scales)
+        lib.af3k_debug_set_dump(dump.data_ptr())
+        try:
+            wide = _call(cuda_device, q, k, v, mask, bias, **kw, **scales)
+        finally:
+            lib.af3k_debug_set_dump(None)
+        assert torch.equal(out, wide), (B1, Sq)
