@@ -445,16 +445,16 @@ int make_plan(const af3k_attention_desc& d, const DeviceInfo& dev, Plan* plan, b
 // else 5; a lone tile of 128 keys 1.45, converted in place 1.65 (rows on vectors) or 2.2 (rows that start anywhere), and 1.2 for each such
 // item; a tile of a pair of streams 1.6, at least 1.1.  A single key tile or rows on vectors cost a lone item less than any pass.
 // Measured on the device, us, the way that is taken (the other); 16 heads, fp32 rows that start anywhere, unless said:
-//   one query tile per item   here 129 tokens 6.2 (7.0), 389 10.6 (12.0), 1001 22.8 (28.4), bf16 22.3 (27.5); 8 heads of 700 14.3 (15.2); 4 heads
-//                             of 129 6.1 (6.8), of 200 7.0 (7.4); the pass 4 heads of 1001 17.1 (18.3), 6 of 389 9.7 (10.4)
-//   pairs of query tiles      here on vectors 1200 40.0 (43.3), 1536 46.8 (60.8), 2048 66 (96), anywhere 1301 52.6 (54.0), 2047 81 (106), bf16
-//                             83 (89); the pass 1200 46.8 (48.3), 1301 bf16 44.0 (52.2), 1536 bf16 55.5 (57.3)
-//   several pair rows         nearly always the pass: 4 heads of 100 rows 9.6 (11.8), of 140 rows of 32 keys 7.8 (10.7), 3 rows of 1000 tokens on vectors
-//                             43.4 (46.6); in a graph 62 rows 6.7 (7.6)
+//   one query tile per item   here 129 tokens 6.7 (7.2), 389 10.4 (12.1), 1001 22.7 (28.4), bf16 22.2 (27.5); 8 heads of 700 14.0 (15.0); 4 heads
+//                             of 129 6.5 (7.0), of 200 7.1 (7.5); the pass 4 heads of 1001 17.2 (18.2), 6 of 389 10.0 (10.3)
+//   pairs of query tiles      here on vectors 1200 39.6 (43.1), 1536 46.5 (60.7), 2048 66 (96), anywhere 1301 52.7 (54.0), 2047 81 (106), bf16
+//                             78 (89); the pass 1200 46.7 (48.3), 1301 bf16 43.7 (52.3), 1536 bf16 55.4 (57.5)
+//   several pair rows         nearly always the pass: 4 heads of 100 rows 9.5 (11.8), of 140 rows of 32 keys 7.8 (10.6), 3 rows of 1000 tokens on vectors
+//                             43.5 (46.3); in a graph 62 rows 6.7 (7.6)
 // Several pair rows to an item: a short call is bound by its launches, which take the host 8.6 us with the pass and 5.9 without, so
-// there up to kLaunchWorth us of the device's time are given for the one launch less (4 heads, 45 rows 9.2 -> 7.2 us a call, 62 rows 9.4 -> 7.6,
-// 40 rows of 100 on vectors 9.3 -> 7.6; most on the device: 74 rows of 64 keys 6.7 -> 8.0), and nothing is under capture, where launches are the graph's.
-// Below kFewItems ragged items the pass stays, although here would be faster up to 200 tokens (3 heads of 131: 6.8, here 6.1): no call in
+// there up to kLaunchWorth us of the device's time are given for the one launch less (4 heads, 45 rows 8.7 -> 7.4 us a call, 62 rows 8.7 -> 7.7,
+// 40 rows of 100 on vectors 8.7 -> 7.7; most on the device: 74 rows of 64 keys 6.7 -> 8.0), and nothing is under capture, where launches are the graph's.
+// Below kFewItems ragged items the pass stays, although here would be faster up to 200 tokens (3 heads of 131: 7.0, here 6.5): no call in
 // use has fewer than four heads.
 constexpr int kFewItems = 8;
 constexpr double kLaunchWorth = 1.2, kShortCall = 5.5;
@@ -570,7 +570,7 @@ int static_scratch_address(void** out) {
 
 extern "C" {
 
-int af3k_version(void) { return 1005; }
+int af3k_version(void) { return 1006; }
 
 const char* af3k_strerror(int code) {
   switch (code) {

@@ -1106,12 +1106,12 @@ __device__ __forceinline__ void store_bias4(uint32_t tile, int row, int lane, ui
 
 // kConvert: eight warps in place of the second softmax warpgroup, which has no stream in items of one, make the bias tiles, from fp32 or
 // from bf16 rows that TMA cannot address, in place of the producer's loads.  Otherwise such a call takes a launch more, and for a
-// short call that is a good part of it.  us, bias in place / converted here / in a pass before, 16 heads, fp32: 77 tokens 5.4 / 5.7
-// / 6.8, 512 9.0 / 10.1 / 13.5, 1000 14.4 / 17.3 / 26.6.  A warp takes 16 rows of a tile, a lane four keys of each.  What does
+// short call that is a good part of it.  us, converted here / in a pass before, 16 heads, fp32 on vectors: 100 tokens 4.7 / 6.3, 512 9.3 / 12.9,
+// 1152 20.4 / 33.2 (512 in place 8.2).  A warp takes 16 rows of a tile, a lane four keys of each.  What does
 // not exist takes the bias of a row or key that does, or anything: of such rows nothing is stored, such keys are at -inf.
 //
 // Rows that start on vectors (bias_wide): 8 rows' loads for the next tile follow directly on their store for this one, so that
-// 16 rows' are out nearly all the time.  The warp is alone on its scheduler beside a softmax warp that streams through its code, so the
+// 16 rows' are out nearly all the time.  Two such warps share a scheduler with a softmax warp that streams through its code, so the
 // loop is kept short: with a test for infinities and a second pass behind it 512 tokens took 11.4 us.
 template <bool kF32, int kW>
 __device__ void bias_convert_role(const Ctx& c, int cw, int lane) {
@@ -1174,7 +1174,7 @@ __device__ void bias_convert_role(const Ctx& c, int cw, int lane) {
 // Keys that do not exist get 0.  The fetch of instructions is what this kernel is short of, so the code is kept short.  Tried for 1001
 // tokens, us a tile (in place 1.4): aligned vectors of four elements stored in pieces that depend on where the row starts 8, put
 // together by shuffles 3.9, the same with eight warps 2.5, copied through shared memory in a rolled loop 3.3 - 3.9; this 2.2.
-// us, 16 heads, in place / here / pass before: 129 tokens 4.8 / 6.3 / 7.1, 389 bf16 7.7 / 10.5 / 12.0, 1001 fp32 13.5 / 19.5 / 34.4.
+// us, 16 heads, here / pass before: 129 tokens 6.7 / 7.2, 389 bf16 10.6 / 12.1, 1001 fp32 22.7 / 28.4.
 template <bool kF32, int kW>
 __device__ void bias_convert_ragged_role(const Ctx& c, int cw, int lane) {
   const AttnParams& p = *c.p;

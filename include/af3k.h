@@ -125,11 +125,13 @@ int af3k_dot_product_attention(const af3k_attention_desc* desc, const void* q, c
                                const float* q_scale, const float* k_scale, void* workspace,
                                size_t workspace_bytes, int* status_dev, void* stream);
 
-/* The same operation with bf16 q/k in one launch, without a workspace: where every work item has one query tile (small
- * calls), and Sk is at most 128 or the bias rows start and end on groups of four keys, the kernel converts an fp32 or
- * ragged bias itself, from where it is.  AF3K_ERR_WORKSPACE, and nothing is launched, where the bias needs converting and
- * that does not hold: then use af3k_dot_product_attention.  The results are the same bits.  No counterpart in the
- * reference. */
+/* The same operation with bf16 q/k in one launch, without a workspace: the kernel may convert an fp32 or ragged bias itself,
+ * from where it is.  Whether it does is the library's choice, by an estimate of which way is faster.  AF3K_ERR_WORKSPACE, and
+ * nothing is launched, where the bias needs converting and the library would rather have it converted first: then use
+ * af3k_dot_product_attention.  Any call whose bias needs converting may be answered so, but never one of equal items of one query
+ * tile (few enough tiles that each has an SM) with Sk at most 128 or bias rows that start and end on groups of four keys.  While
+ * `stream` is being captured a launch saved counts for nothing, so that the choice can be another one there.  The results are the
+ * same bits on every way.  No counterpart in the reference. */
 int af3k_dot_product_attention_convert(const af3k_attention_desc* desc, const void* q, const void* k, const void* v,
                                        const void* bias, const uint8_t* mask, void* out, int* status_dev, void* stream);
 
@@ -162,21 +164,22 @@ int af3k_dot_product_attention_noalloc(const af3k_attention_desc* desc, const vo
 /* Size in bytes of the built-in scratch array used by af3k_dot_product_attention_noalloc. */
 size_t af3k_static_scratch_bytes(void);
 
-/* Number of kernels the last successful af3k_dot_product_attention call on this thread
- * launched (1, or 2 when the bias staging pre-pass ran). */
+/* Number of kernels the last successful call on this thread that can launch any did launch (af3k_dot_product_attention: 1, or 2
+ * when the bias staging pre-pass ran; a call of the Python operator on fp32 tensors ends with af3k_cast's 1). */
 int af3k_last_launch_count(void);
 
 /* Upper bound, in SM clock cycles, for any single on-device wait (default 2e9, about a second).
- * A kernel whose wait runs out sets AF3K_STATUS_WAIT_TIMEOUT and returns. */
+ * Counted from the end of the kernel before on the stream.  A kernel whose wait runs out sets AF3K_STATUS_WAIT_TIMEOUT and returns. */
 void af3k_set_wait_limit_cycles(long long cycles);
 
-/* Launch plan the library would use for `desc` on the current device (a B200 with 148 SMs and
+/* Launch plan af3k_dot_product_attention would use for `desc` on the current device (a B200 with 148 SMs and
  * 227 KB of shared memory per block is assumed when no such device is present, so this also
  * works on a CPU-only host): out6 = {pair rows per work item, K/V ring stages, work items,
  * grid size, dynamic shared memory bytes, TMEM columns used}.  With one pair row per item an item is
  * one query tile while there is an SM for each, else two.  Where the pair rows behind the last full round go to smaller
- * items, there are more of them than rows, heads and query tiles make of the first size.  Diagnostic; no counterpart in
- * the reference. */
+ * items, there are more of them than rows, heads and query tiles make of the first size.  (af3k_dot_product_attention_convert
+ * gives this plan up for items of one query tile where it converts the bias of a call whose items have more.)  Diagnostic; no
+ * counterpart in the reference. */
 int af3k_describe_plan(const af3k_attention_desc* desc, int32_t* out6);
 
 /* The same plan's streams: out4 = {streams per work item, 1 if they are neighbouring query tiles of one pair row (0: pair
@@ -328,7 +331,8 @@ int af3k_token_pack(const af3k_matrix* w4, int64_t C, void* w4_bf16, const float
 
 /* Up to three contiguous arrays of n[i] elements, 16-byte aligned, fp32 -> bf16 (to_dtype AF3K_BF16, rounded to nearest) or
  * bf16 -> fp32 (AF3K_F32) in one launch: operands and results of fp32 callers (the reference's fp32 instantiation,
- * src/csrc/dot_product_attention.cpp:554-558). */
+ * src/csrc/dot_product_attention.cpp:554-558).  Its blocks may be resident, waiting, while the kernel before it on the stream still
+ * runs: not the way to convert behind a call under max_ctas, whose free SMs they would take. */
 int af3k_cast(const void* const* src, void* const* dst, const int64_t* n, int32_t count, int32_t to_dtype, void* stream);
 
 /* out = weighted * sigmoid(gate), elementwise over n bf16 elements (n a multiple of 8; all three

@@ -288,3 +288,8 @@ def test_ordinary_calls_leave_host_tensors_to_the_general_way():
     m = A.GridSelfAttentionCpp(64, 4)
     assert host.grid_forward(m, torch.zeros(8, 8, 64), torch.ones(8, 8, dtype=torch.bool), torch.nn.Linear, torch.nn.LayerNorm) is None
     assert host.grid_forward(object(), torch.zeros(8, 8, 64), None, torch.nn.Linear, torch.nn.LayerNorm) is None
+
+
+def test_version_is_that_of_the_documents():
+    text = open(os.path.join(ROOT, "INTEGRATION.md")).read()
+    assert f"`af3k_version()` is {_capi.load().af3k_version()} for this ABI" in text
