@@ -65,7 +65,8 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 constexpr int kStaticSmemReserve = 1024;   // the kernels' few static bytes, padded to the dynamic part's alignment
 
-// Key tiles come in these widths; every width is a kernel of its own, whose softmax warps have that many logits in registers.
+// Single key tiles come in these widths (48 was not tried: 33 to 48 keys run as 64); every width is a kernel of its own, whose softmax
+// warps have that many logits in registers.
 constexpr int kKeyWidths[] = {32, 64, 80, 96, 112, 128};
 
 // f(kernel) for the kernel of key tiles of kw keys, the last of last_w.

@@ -763,9 +763,13 @@ py::object operator_call(const Tensor& q, const Tensor& k, const Tensor& v, py::
 }
 
 // What attribute access finds in an instance's own dictionary (borrowed, null if nothing).
-PyObject* own(py::handle object, PyObject* name) {
-  const py::object d = py::reinterpret_steal<py::object>(PyObject_GenericGetDict(object.ptr(), nullptr));
+py::object own_dict(py::handle object) {
+  py::object d = py::reinterpret_steal<py::object>(PyObject_GenericGetDict(object.ptr(), nullptr));
   if (!d) PyErr_Clear();
+  return d;
+}
+PyObject* own(py::handle object, PyObject* name) {
+  const py::object d = own_dict(object);
   return d && PyDict_Check(d.ptr()) ? PyDict_GetItemWithError(d.ptr(), name) : nullptr;
 }
 PyObject* entry(PyObject* dict, PyObject* name) { return dict != nullptr && PyDict_Check(dict) ? PyDict_GetItemWithError(dict, name) : nullptr; }
@@ -786,11 +790,13 @@ py::object grid_forward(py::handle module, const Tensor& pair, py::handle mask, 
   if (head == nullptr || !PyLong_Check(head) || transpose == nullptr || !PyBool_Check(transpose) || mask.is_none() || !plain_mask(mask, 2)) return py::none();
   const int64_t H = PyLong_AsLongLong(head);
   if (!grid_fused(pair, H, H)) return py::none();
-  PyObject* const layers = own(module, modules);
+  const py::object of_module = own_dict(module);
+  PyObject* const layers = entry(of_module.ptr(), modules);
   std::vector<Tensor> params;
   params.reserve(8);
   double eps = 0;
   for (int i = 0; i < 8; ++i) {
+    if (entry(of_module.ptr(), names[i]) != nullptr) return py::none();                       // set past the module's layers
     PyObject* const layer = entry(layers, names[i]);
     const bool norm = i == 5 || i == 6;
     if (layer == nullptr || Py_TYPE(layer) != (PyTypeObject*)(norm ? layer_norm : linear).ptr()) return py::none();

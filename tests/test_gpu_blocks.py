@@ -609,7 +609,7 @@ class _Scaled(torch.nn.Linear):
 
 
 @pytest.mark.parametrize("C", [64, 128])
-@pytest.mark.parametrize("form", ["plain", "mask_1d", "mask_uint8", "mask_3d", "float32", "hook", "replaced", "weight_in_dict", "functional", "half_norm", "trains_output"])
+@pytest.mark.parametrize("form", ["plain", "mask_1d", "mask_uint8", "mask_3d", "float32", "hook", "replaced", "weight_in_dict", "layer_in_dict", "functional", "half_norm", "trains_output"])
 def test_module_call_straight_from_python(cuda_device, C, form):
     """Whatever parameters, layers, masks and modes a module is called with: the bits of the general way, and hooks run."""
     g = torch.Generator().manual_seed(C)
@@ -633,6 +633,11 @@ def test_module_call_straight_from_python(cuda_device, C, form):
     if form == "weight_in_dict":
         for m in (plain, general):
             m.v_projection.__dict__["weight"] = m.v_projection.weight.detach() * 3
+    if form == "layer_in_dict":
+        for m in (plain, general):
+            other = torch.nn.Linear(C, C, bias=False).to(cuda_device, torch.bfloat16)
+            other.weight.data.copy_(m.v_projection.weight.detach() * 3)
+            m.__dict__["v_projection"] = other
     pair = torch.randn(N, N, C, generator=g).to(cuda_device, torch.float32 if form == "float32" else torch.bfloat16)
     mask = (torch.rand(N, N, generator=g) >= 0.2).to(cuda_device)
     mask = {"mask_1d": mask[0], "mask_uint8": mask.to(torch.uint8), "mask_3d": mask[:, None, None, :]}.get(form, mask)
