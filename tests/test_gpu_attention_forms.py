@@ -381,7 +381,7 @@ def test_debug_dump_has_the_first_result(cuda_device, B1, B2, S, rows_per_item, 
                                 449, 560, 561])
 @pytest.mark.parametrize("qk,D", [("bf16", 24), ("bf16", 48), ("bf16", 64), ("fp8", 32)])
 def test_key_tiles_of_every_width(cuda_device, Sk, qk, D):
-    """Key tiles are as wide as the keys of a call need: first and last length of each width, with one to five tiles.  Several
+    """The last key tile is as wide as the keys of a call need: first and last length of each width, with one to five tiles.  Several
     pair rows per item with a remainder, two query tiles, and (fp32 bias, a single pair row) the bias converted on the way in."""
     for B1, Sq in ((5, 140), (1, 70)):
         q, k, v, mask, bias = _inputs(B1, 3, Sq, D, Sk + D, Sk)
